@@ -67,7 +67,7 @@ Model::~Model() {
     release_graphs();
     for (void* p : owned_) cudaFree(p);
     for (void* p : {(void*)hidden_, (void*)xnorm_, (void*)q_, (void*)k_, (void*)v_, (void*)attn_, (void*)act_, (void*)up_, (void*)part_,
-                    (void*)logits_, (void*)logits_l_, (void*)attn_scratch_, xq_h_, xq_a_, xq_i_, kc_, vc_, (void*)step_dev_,
+                    (void*)logits_, (void*)logits_l_, (void*)attn_scratch_, kc_, vc_, (void*)step_dev_,
                     (void*)attn_tickets_,
                     (void*)argmax_dev_, (void*)recent_dev_})
         if (p) cudaFree(p);
@@ -395,9 +395,6 @@ bool Model::finalize() {
     logits_ = dmalloc<float>((size_t)vocab_l_ * tp_size_);
     logits_l_ = dmalloc<float>(vocab_l_);
     attn_scratch_ = dmalloc<float>(attention_decode_dyn_scratch_floats(max_seq, nh_l_, nkv_l_, hd));
-    xq_h_ = dmalloc<uint8_t>(xq_bytes(hidden));
-    xq_a_ = dmalloc<uint8_t>(xq_bytes(nh_l_ * hd));
-    xq_i_ = dmalloc<uint8_t>(xq_bytes(inter_l_));
     attn_tickets_ = dmalloc<unsigned>((size_t)std::max(1, nh_l_));
     NT_CUDA_CHECK(cudaMemset(attn_tickets_, 0, (size_t)std::max(1, nh_l_) * sizeof(unsigned)));
     if (const char* fz = getenv("NT_B200_FUSE")) fuse_mask_ = atoi(fz);
@@ -482,7 +479,7 @@ size_t Model::bytes_per_token(int ctx) const {
 }
 
 // y_i = W_i . x' for n matrices sharing x' = norm_w ? rmsnorm(x, norm_w) : x.
-// When every matrix qualifies, one fused launch does (RMSNorm +) activation quantisation in its prologue, the TMA/dp4a
+// When every matrix qualifies, one fused launch does (RMSNorm +) activation quantisation in its prologue, the block
 // GEMV and the epilogue; otherwise the pieces run as separate launches like the reference's sequence.
 void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float* x, const float* norm_w, GemvEpilogue ep,
                    cudaStream_t s) {
@@ -490,13 +487,8 @@ void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float
     const int K = ws[0]->cols;
     for (int i = 0; i < n; i++) { mats[i].W = ws[i]->ptr; mats[i].y = ys[i]; mats[i].out = ws[i]->rows; mats[i].dtype = ws[i]->dtype; mats[i].row_pitch = ws[i]->pitch; }
     GemvInput in;
-    if (gemv_kq_supported(mats, n, K)) {
-        // (RMSNorm +) quantisation as one small multi-CTA launch: measured cheaper than redoing it in the prologue
-        // of each of the 148 GEMV CTAs (profiles/r01_*), and PDL overlaps it with the neighbouring kernels.
-        void* xq = (K == cfg_.hidden_size) ? xq_h_ : (K == inter_l_) ? xq_i_ : xq_a_;
-        if (norm_w) rmsnorm_xq(nullptr, xq, x, norm_w, K, cfg_.norm_eps, s);
-        else quantize_x(x, xq, K, s);
-        in.xq = xq;
+    if (gemv_kq_any_pitch(mats, n, K)) {
+        in.x = x; in.norm_w = norm_w; in.eps = cfg_.norm_eps;
         gemv_kq(mats, n, K, in, ep, s);
         return;
     }
@@ -510,14 +502,9 @@ void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float
         return;
     }
     for (int i = 0; i < n; i++) {
-        if (gemv_kq_supported(&mats[i], 1, K)) { in.x = xf; gemv_kq(&mats[i], 1, K, in, ep, s); }
+        if (gemv_kq_any_pitch(&mats[i], 1, K)) { in.x = xf; gemv_kq(&mats[i], 1, K, in, ep, s); }
         else gemv_generic(ys[i], ws[i]->ptr, xf, ws[i]->rows, K, ws[i]->dtype, ws[i]->pitch, ep, s);
     }
-}
-
-bool Model::o_xq_fusable(const Weight& wo) const {
-    GemvMat m; m.W = wo.ptr; m.y = nullptr; m.out = wo.rows; m.dtype = wo.dtype; m.row_pitch = wo.pitch;
-    return (nh_l_ * cfg_.head_dim) % 128 == 0 && gemv_kq_supported(&m, 1, wo.cols);
 }
 
 // hidden += all_reduce(partial)   (one exchange per sub-block)
@@ -553,13 +540,13 @@ bool Model::chain_ok() const {
     if (cfg_.hidden_size % 128 != 0 || inter_l_ % 128 != 0 || (nh_l_ * cfg_.head_dim) % 128 != 0) return false;
     auto kq = [&](const Weight& w, int K) {
         GemvMat m; m.W = w.ptr; m.y = nullptr; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch;
-        return w.cols == K && gemv_kq_supported(&m, 1, K);
+        return w.cols == K && gemv_kq_any_pitch(&m, 1, K);
     };
     for (const LayerWeights& L : layers_) {
         GemvMat qkv[3];
         const Weight* ws[3] = {&L.wq, &L.wk, &L.wv};
         for (int i = 0; i < 3; i++) { qkv[i].W = ws[i]->ptr; qkv[i].out = ws[i]->rows; qkv[i].dtype = ws[i]->dtype; qkv[i].row_pitch = ws[i]->pitch; }
-        if (!gemv_kq_supported(qkv, 3, cfg_.hidden_size)) return false;
+        if (!gemv_kq_any_pitch(qkv, 3, cfg_.hidden_size)) return false;
         if (!kq(L.wo, nh_l_ * cfg_.head_dim) || !kq(L.gate, cfg_.hidden_size) || !kq(L.up, cfg_.hidden_size) || !kq(L.down, inter_l_)) return false;
         if (L.gate.dtype != L.up.dtype) return false;
     }
@@ -568,11 +555,10 @@ bool Model::chain_ok() const {
 
 // One decoded token, all layers.  Two forms of the reference's launch sequence (Attention::forward attention.cpp:120-211,
 // FFN::forward ffn.cpp:85-134, 15 launches per layer there):
-//   short chain (one GPU, all projections on the TMA/dp4a GEMV) — 6 launches per layer:
-//     [RMSNorm + quantise + q/k/v GEMV] [RoPE + KV write + attention + merge] [quantise + o GEMV += residual]
-//     [RMSNorm + quantise + gate/up GEMV + SwiGLU] [quantise] [down GEMV += residual]
-//     The norms and the quantisers of hidden-sized vectors run in the consuming GEMV's prologue while its first weights are
-//     already in flight (gemv_kquant.cu); only the intermediate-sized activation vector keeps its own quantise launch;
+//   short chain (one GPU, all projections on the block GEMV) — 7 launches per layer:
+//     [RMSNorm + quantise + q/k/v GEMV] [RoPE + KV write] [attention] [merge] [quantise + o GEMV += residual]
+//     [RMSNorm + quantise + gate/up GEMV + SwiGLU] [quantise + down GEMV += residual]
+//     The norms and the quantisers run in the consuming GEMV's prologue while its first weights are already in flight (gemv_kquant.cu);
 //   unfused — 8-10 launches per layer (tensor parallel, mixed dtypes, NT_B200_FUSE=0).
 void Model::step_body(cudaStream_t s) {
     if (cfg_.layer_spec()) { step_body_spec(s); return; }
@@ -596,16 +582,15 @@ void Model::step_body(cudaStream_t s) {
         } else {
             const Weight* ws[3] = {&L.wq, &L.wk, &L.wv}; float* ys[3] = {q_, k_, v_}; matvec(ws, ys, 3, hidden_, L.attn_norm, GEMV_STORE, s);
         }
-        const bool o_xq = !chain && o_xq_fusable(L.wo);            // unfused path: attention emits xq for the o-projection
         if (attn1) {
             attention_decode_fused(attn_, q_, k_, v_, kc, vc, pos_dev, max_seq, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, scale,
-                                   attn_scratch_, attn_tickets_, o_xq ? xq_a_ : nullptr, s);
+                                   attn_scratch_, attn_tickets_, nullptr, s);
         } else if (fuse_mask_ & 4) {
             attention_decode_rope_dyn(attn_, q_, k_, v_, kc, vc, pos_dev, max_seq, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, scale,
-                                      attn_scratch_, o_xq ? xq_a_ : nullptr, s);
+                                      attn_scratch_, nullptr, s);
         } else {
             rope_kv_decode(q_, k_, v_, kc, vc, pos_dev, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, max_seq, s);
-            attention_decode_dyn(attn_, q_, kc, vc, pos_dev, max_seq, nh_l_, nkv_l_, hd, scale, attn_scratch_, o_xq ? xq_a_ : nullptr, s);
+            attention_decode_dyn(attn_, q_, kc, vc, pos_dev, max_seq, nh_l_, nkv_l_, hd, scale, attn_scratch_, nullptr, s);
         }
         if (chain) {
             GemvMat m = mat(L.wo, hidden_);
@@ -616,12 +601,7 @@ void Model::step_body(cudaStream_t s) {
             const Weight* ws[1] = {&L.wo};
             float* ys[1] = {tp_size_ == 1 ? hidden_ : part_};
             const GemvEpilogue ep = tp_size_ == 1 ? GEMV_ADD : GEMV_STORE;
-            if (o_xq) {
-                GemvMat m = mat(L.wo, ys[0]);
-                gemv_kq(&m, 1, L.wo.cols, xq_a_, ep, s);
-            } else {
-                matvec(ws, ys, 1, attn_, nullptr, ep, s);
-            }
+            matvec(ws, ys, 1, attn_, nullptr, ep, s);
             if (tp_size_ > 1) reduce_residual(part_, s);
         }
         // --- FFN sub-block ---
@@ -629,12 +609,8 @@ void Model::step_body(cudaStream_t s) {
             GemvMat m2[2] = {mat(L.gate, act_), mat(L.up, up_)};
             GemvInput in; in.x = hidden_; in.norm_w = L.ffn_norm; in.eps = cfg_.norm_eps;
             gemv_kq(m2, 2, hidden, in, GEMV_SWIGLU, s);
-            // The activation vector's quantiser: in the down GEMV's prologue when its staging (3.4 x inter bytes) fits over the ring
-            // (tensor-parallel shards: inter / tp <= 8192), as a launch of its own for the full 28672-wide vector.
             GemvMat md = mat(L.down, hidden_);
-            GemvInput ind;
-            if (inter_l_ <= 8192) ind.x = act_;
-            else { quantize_x(act_, xq_i_, inter_l_, s); ind.xq = xq_i_; }
+            GemvInput ind; ind.x = act_;
             if (tp_size_ == 1) gemv_kq(&md, 1, inter_l_, ind, GEMV_ADD, s);
             else { gemv_kq_peer(md, inter_l_, ind, xchg_->out(), s); xchg_->reduce_residual(hidden_, s); }
             continue;

@@ -294,7 +294,6 @@ private:
     bool f16_direct(const Weight& w) const;   // F16 rows usable by TMA in place
     // C[T, w.rows] (+)= split(A)[T, w.cols] . W^T for a weight of any GGUF dtype (quantised: dequantise to hi/lo, two GEMMs)
     void prefill_gemm(float* C, const void* ws, const Weight& w, int T, bool add, cudaStream_t s);
-    bool o_xq_fusable(const Weight& wo) const;
     void release_graphs();
 
     ModelConfig cfg_;
@@ -313,7 +312,6 @@ private:
     cudaStream_t stream_ = nullptr;
     float *hidden_ = nullptr, *xnorm_ = nullptr, *q_ = nullptr, *k_ = nullptr, *v_ = nullptr, *attn_ = nullptr;
     float *act_ = nullptr, *up_ = nullptr, *part_ = nullptr, *logits_ = nullptr, *logits_l_ = nullptr, *attn_scratch_ = nullptr;
-    void *xq_h_ = nullptr, *xq_a_ = nullptr, *xq_i_ = nullptr;
     unsigned* attn_tickets_ = nullptr;   // last-arriver tickets of the one-launch attention (zero between launches)
     int fuse_mask_ = 1;                  // bit 0: norm + quantiser in the GEMV prologues (default), bit 1: one-launch attention (opt-in: measured slower, profiles/r02_*), bit 2: RoPE + KV write inside the decode kernel, merge separate (NT_B200_FUSE)
     void *kc_ = nullptr, *vc_ = nullptr;

@@ -57,7 +57,8 @@ struct GemvInput {
     float eps = 0.f;
     const PeerOut* peer = nullptr;     // epilogue GEMV_PEER only
 };
-bool gemv_kq_supported(const GemvMat* mats, int n_mat, int K);
+bool gemv_kq_supported(const GemvMat* mats, int n_mat, int K);      // 16-byte aligned rows
+bool gemv_kq_any_pitch(const GemvMat* mats, int n_mat, int K);      // what gemv_kq takes: 16-byte aligned matrices, any even pitch for Q6_K
 void gemv_kq(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpilogue ep, cudaStream_t s);
 void gemv_kq(const GemvMat* mats, int n_mat, int K, const void* xq, GemvEpilogue ep, cudaStream_t s);
 // gemv_kquant_q.cu: the quarter-block kernel (lane <-> 64 weights, up to 16 warps); false = shape not covered, nothing launched

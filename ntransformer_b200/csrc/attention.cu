@@ -279,6 +279,12 @@ __global__ void __launch_bounds__(AW * 32) decode_kernel(float* __restrict__ out
         seq_len = *pos_dev + 1;
         split_len = max((seq_len + n_splits - 1) / n_splits, DYN_MIN_SPLIT);
     }
+    if (blockIdx.z) {                    // a run of tokens: query z attends one key more than the one before it (slices cut for the last)
+        seq_len += blockIdx.z;
+        q += (size_t)blockIdx.z * n_heads * HD;
+        out += (size_t)blockIdx.z * n_heads * HD;
+        scratch += (size_t)blockIdx.z * n_heads * n_splits * (HD + 2);
+    }
     const int head0 = blockIdx.x * GC, split = blockIdx.y;
     const int kv_head = head0 / (n_heads / n_kv);
     const int k_begin = split * split_len, k_end = min(seq_len, k_begin + split_len);
@@ -316,6 +322,9 @@ __global__ void decode_combine_kernel(float* __restrict__ out, const float* __re
     const int h = blockIdx.x;
     pdl_launch_dependents();
     pdl_wait();
+    seq_len += blockIdx.y;               // a run of tokens: blockIdx.y is the query
+    scratch += (size_t)blockIdx.y * n_heads * n_splits * (hd + 2);
+    out += (size_t)blockIdx.y * n_heads * hd;
     if (pos_dev) { seq_len = *pos_dev + 1; split_len = max((seq_len + n_splits - 1) / n_splits, DYN_MIN_SPLIT); }
     const float* ml = scratch + (size_t)n_heads * n_splits * hd + (size_t)h * n_splits * 2;
     const int used = (seq_len + split_len - 1) / split_len;
@@ -518,6 +527,36 @@ void launch_decode(float* out, const float* q, const __half* kc, const __half* v
     }
 }
 
+// Slices of a run of `tokens` queries: enough CTAs for the chip, at least 32 keys each, none longer than the shared memory of one holds.
+int rows_splits(int tokens, int total, int groups, int gc) {
+    int n = (2 * 148 + groups * tokens - 1) / (groups * tokens);
+    n = std::min(std::min(n, (total + 31) / 32), MAX_SPLITS);
+    n = std::max(n, (total + 16384 / gc - 1) / (16384 / gc));
+    return std::max(1, n);
+}
+// A few consecutive queries (start_pos ...), each with the arithmetic of a decoded token; scratch: attention_rows_scratch_floats().
+template <int DPL, int GC>
+void launch_rows(float* out, const float* q, const __half* kc, const __half* vc, int tokens, int start_pos, int n_heads, int n_kv, float scale, float* scratch,
+                 cudaStream_t s) {
+    constexpr int HD = DPL * 32;
+    const int groups = n_heads / GC, total = start_pos + tokens;
+    int n_splits = rows_splits(tokens, total, groups, GC);
+    const int split_len = (total + n_splits - 1) / n_splits;
+    n_splits = (total + split_len - 1) / split_len;
+    const size_t smem = ((size_t)GC * split_len + (size_t)AW * GC * HD + (size_t)GC * HD + 2 * GC) * sizeof(float);
+    static unsigned long long configured = 0;      // bit per device id
+    opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
+    NT_CHECK(smem <= (size_t)ATTN_MAX_DYN_SMEM && n_splits <= MAX_SPLITS, "attention over a run of tokens: context beyond the slices");
+    launch_k(decode_kernel<DPL, GC>, dim3(groups, n_splits, tokens), dim3(AW * 32), smem, s, out, q, kc, vc, start_pos + 1, n_heads, n_kv, scale, n_splits, split_len,
+             scratch, (const int*)nullptr);
+    count_launch();
+    if (n_splits > 1) {
+        launch_k(decode_combine_kernel, dim3(n_heads, tokens), dim3(128), 0, s, out, (const float*)scratch, n_heads, HD, n_splits, start_pos + 1, split_len,
+                 (const int*)nullptr, (int8_t*)nullptr);
+        count_launch();
+    }
+}
+
 // Graph-replayable decode: the context length (pos + 1) is read from device memory, the launch shape is fixed
 // by max_seq, partials always go through caller-owned scratch (n_heads * n_splits * (HD + 2) floats).
 template <int DPL, int GC>
@@ -611,6 +650,24 @@ void attention_decode(float* out, const float* q, const void* kc, const void* vc
     const __half* k = static_cast<const __half*>(kc);
     const __half* v = static_cast<const __half*>(vc);
     NT_DISPATCH_ATTN(launch_decode, out, q, k, v, seq_len, n_heads, n_kv, scale, s);
+}
+
+bool attention_rows_supported(int total, int n_heads, int n_kv) {
+    const int gc = pick_gc(n_heads / n_kv);
+    return rows_splits(1, total, n_heads / gc, gc) <= MAX_SPLITS;
+}
+size_t attention_rows_scratch_floats(int tokens, int max_seq, int n_heads, int n_kv, int hd) {
+    const int gc = pick_gc(n_heads / n_kv);
+    size_t most = 0;                     // fewer tokens are cut into more slices
+    for (int t = 1; t <= tokens; t++) most = std::max(most, (size_t)t * n_heads * rows_splits(t, max_seq, n_heads / gc, gc) * (hd + 2));
+    return most;
+}
+void attention_rows_f16(float* out, const float* q, const void* kc, const void* vc, int tokens, int start_pos, int n_heads, int n_kv, int hd, float scale,
+                        float* scratch, cudaStream_t s) {
+    if (tokens <= 0 || n_heads <= 0) return;
+    const __half* k = static_cast<const __half*>(kc);
+    const __half* v = static_cast<const __half*>(vc);
+    NT_DISPATCH_ATTN(launch_rows, out, q, k, v, tokens, start_pos, n_heads, n_kv, scale, scratch, s);
 }
 
 int attention_decode_dyn_splits(int max_seq, int n_heads, int n_kv) {

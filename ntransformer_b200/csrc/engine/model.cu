@@ -22,6 +22,7 @@ __global__ void iota_kernel(int* out, int first, int n) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = first + i;
 }
+constexpr int SHORT_CHUNK = 64;          // tokens of a pass through the kernels for a few tokens (bounds their buffers)
 constexpr int PREFILL_CHUNK = 4096;      // tokens per batched pass (bounds the activation buffers; weights re-read per chunk)
 
 // argmax over n floats, lowest index wins ties (reference Sampler::argmax, sampler.cpp:18-28)
@@ -72,7 +73,8 @@ Model::~Model() {
                     (void*)argmax_dev_, (void*)recent_dev_})
         if (p) cudaFree(p);
     for (void* p : {(void*)pf_.x, (void*)pf_.q, (void*)pf_.k, (void*)pf_.v, (void*)pf_.attn, pf_.ws, pf_.ws2, (void*)pf_.tok, (void*)pf_.pos,
-                    (void*)pf_.g, (void*)pf_.u, pf_.whi, pf_.wlo})
+                    (void*)pf_.g, (void*)pf_.u, pf_.whi, pf_.wlo, (void*)sb_.x, (void*)sb_.q, (void*)sb_.k, (void*)sb_.v, (void*)sb_.attn, (void*)sb_.act, sb_.xr,
+                    (void*)sb_.scratch, (void*)sb_.tok, (void*)sb_.pos})
         if (p) cudaFree(p);
     for (size_t i = 0; i < kcs_.size(); i++) if (kcs_[i] && (cache_owned_.empty() || cache_owned_[i])) { cudaFree(kcs_[i]); cudaFree(vcs_[i]); }
     for (void* p : {(void*)pf_.h, (void*)pf_.tmp, pf_.hws, (void*)want_out_, (void*)pf_.xs, (void*)pf_.maps, (void*)pf_.sel, (void*)pf_.work, (void*)pf_.wt,
@@ -758,6 +760,63 @@ bool Model::batched_prefill_ok(int seq_len, int start_pos) const {
     return true;
 }
 
+// A few tokens together through the decode step's arithmetic (gemv_rows.cu): every matrix on the block GEMV, one GPU.
+bool Model::short_batch_ok(int seq_len, int start_pos) const {
+    if (tp_size_ != 1 || seq_len < 2 || prefill_min_tokens_ <= 0 || getenv("NT_B200_NO_BATCHED_PREFILL") || (fuse_mask_ & 6)) return false;
+    const char* mk = getenv("NT_B200_MEGAKERNEL");
+    if (mk ? env_on("NT_B200_MEGAKERNEL") : use_mega_) return false;
+    return chain_ok() && attention_rows_supported(start_pos + seq_len, nh_l_, nkv_l_);
+}
+
+void Model::ensure_short_buffers() {
+    if (sb_.x) return;
+    const size_t T = SHORT_CHUNK, hidden = (size_t)cfg_.hidden_size, qdim = (size_t)nh_l_ * cfg_.head_dim, kvdim = (size_t)nkv_l_ * cfg_.head_dim;
+    sb_.x = dmalloc<float>(T * hidden);
+    sb_.q = dmalloc<float>(T * qdim); sb_.k = dmalloc<float>(T * kvdim); sb_.v = dmalloc<float>(T * kvdim); sb_.attn = dmalloc<float>(T * qdim);
+    sb_.act = dmalloc<float>(T * (size_t)inter_l_);
+    sb_.xr = dmalloc<uint8_t>(gemv_rows_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_)));
+    sb_.scratch = dmalloc<float>(attention_rows_scratch_floats((int)T, cfg_.max_seq_len, nh_l_, nkv_l_, cfg_.head_dim));
+    sb_.tok = dmalloc<int>(T); sb_.pos = dmalloc<int>(T);
+}
+
+void Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
+    cudaStream_t s = stream_;
+    const int hidden = cfg_.hidden_size, hd = cfg_.head_dim, max_seq = cfg_.max_seq_len, qdim = nh_l_ * hd;
+    const size_t kv_stride = (size_t)max_seq * nkv_l_ * hd;
+    ensure_short_buffers();
+    auto mat = [](const Weight& w, float* y) { GemvMat m; m.W = w.ptr; m.y = y; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch; return m; };
+    int T = 0;
+    for (int c0 = 0; c0 < seq_len; c0 += T) {
+        T = std::min(SHORT_CHUNK, seq_len - c0);
+        const int p0 = start_pos + c0;
+        NT_CUDA_CHECK(cudaMemcpyAsync(sb_.tok, tokens + c0, sizeof(int) * (size_t)T, cudaMemcpyHostToDevice, s));
+        iota_kernel<<<(T + 255) / 256, 256, 0, s>>>(sb_.pos, p0, T);
+        count_launch();
+        embed_rows(sb_.x, embd_.ptr, embd_.dtype, sb_.tok, T, hidden, s);
+        for (int i = 0; i < cfg_.n_layers; i++) {
+            const LayerWeights& L = layers_[(size_t)i];
+            uint16_t* kc = static_cast<uint16_t*>(kc_) + (size_t)i * kv_stride;
+            uint16_t* vc = static_cast<uint16_t*>(vc_) + (size_t)i * kv_stride;
+            const GemvMat qkv[3] = {mat(L.wq, sb_.q), mat(L.wk, sb_.k), mat(L.wv, sb_.v)}, gu[2] = {mat(L.gate, sb_.act), mat(L.up, nullptr)};
+            const GemvMat o = mat(L.wo, sb_.x), down = mat(L.down, sb_.x);
+            quantize_rows(sb_.xr, sb_.x, L.attn_norm, cfg_.norm_eps, T, hidden, s);
+            gemv_rows(qkv, 3, hidden, sb_.xr, T, GEMV_STORE, s);
+            rope(sb_.q, sb_.k, sb_.pos, T, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, false, s);
+            copy_to_kv_cache(kc, vc, sb_.k, sb_.v, T, nkv_l_, hd, p0, max_seq, s);
+            attention_rows_f16(sb_.attn, sb_.q, kc, vc, T, p0, nh_l_, nkv_l_, hd, 1.0f / sqrtf((float)hd), sb_.scratch, s);
+            quantize_rows(sb_.xr, sb_.attn, nullptr, 0.f, T, qdim, s);
+            gemv_rows(&o, 1, qdim, sb_.xr, T, GEMV_ADD, s);
+            quantize_rows(sb_.xr, sb_.x, L.ffn_norm, cfg_.norm_eps, T, hidden, s);
+            gemv_rows(gu, 2, hidden, sb_.xr, T, GEMV_SWIGLU, s);
+            quantize_rows(sb_.xr, sb_.act, nullptr, 0.f, T, inter_l_, s);
+            gemv_rows(&down, 1, inter_l_, sb_.xr, T, GEMV_ADD, s);
+        }
+        if (!want_.empty()) emit_wanted(sb_.x, c0, T, s);
+    }
+    copy(hidden_, sb_.x + (size_t)(T - 1) * hidden, hidden, s);
+    step_head(s, true);
+}
+
 bool Model::f16_direct(const Weight& w) const {
     return w.dtype == DType::F16 && gemm_f16_tc_supported(w.ptr, w.rows, w.cols, w.pitch);
 }
@@ -872,6 +931,7 @@ void Model::forward_async(const int* tokens, int seq_len, int start_pos) {
     if (cfg_.layer_spec()) {
         if (prefill_min_tokens_ > 0 && seq_len >= prefill_min_tokens_ && !getenv("NT_B200_NO_BATCHED_PREFILL")) { prefill_spec(tokens, seq_len, start_pos); return; }
     } else if (batched_prefill_ok(seq_len, start_pos)) { prefill_batched(tokens, seq_len, start_pos); return; }
+    else if (short_batch_ok(seq_len, start_pos)) { prefill_short(tokens, seq_len, start_pos); return; }
     size_t w = 0;
     for (int t = 0; t < seq_len; t++) {
         int tok = tokens[t];

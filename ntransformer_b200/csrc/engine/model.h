@@ -164,6 +164,11 @@ public:
     // Prompts of at least n tokens go through the batched tensor-core prefill when the weights allow it (0 = never).
     void set_prefill_min_tokens(int n) { prefill_min_tokens_ = n; }
     bool batched_prefill_ok(int seq_len, int start_pos) const;
+    bool short_batch_ok(int seq_len, int start_pos) const;
+    void ensure_short_buffers();
+    void prefill_short(const int* tokens, int seq_len, int start_pos);
+    struct { float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *act = nullptr, *scratch = nullptr; void* xr = nullptr;
+             int *tok = nullptr, *pos = nullptr; } sb_;       // a few tokens together
     void clear_kv();
     // Opt-in (also NT_B200_MEGAKERNEL=1): run the decode step as one persistent kernel (engine/decode_mega.h) instead of
     // the graph of fused launches.  Falls back to the graph path, with a note on stderr, when a shape is not covered.

@@ -52,36 +52,11 @@ struct KqParams {
     PeerOut peer;              // epilogue GEMV_PEER
 };
 
-__device__ unsigned wait_expired;      // a wait below gave up: the launch's results are wrong
-
-// Waits for the phase of a copy or of a reader in this CTA, both under way: microseconds.  A limit far above that keeps a broken launch from
-// hanging the GPU.
-__device__ __forceinline__ void wait_phase(uint64_t* bar, uint32_t parity) {
-    uint32_t done = 0;
-    for (uint32_t spin = 0; !done; spin++) {
-        if (spin == (1u << 24)) { wait_expired = 1u; return; }
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    }
-}
-__device__ __forceinline__ void arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
-template <int N> __device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
-
 // Shared memory: [barriers][zeros][norm][partials][digit planes][scales][sums][rings]
 constexpr size_t SM_ZERO = MAX_TEAMS * 16 * MAX_STAGES, SM_RED = SM_ZERO + 16, SM_PART = SM_RED + 112;
 constexpr size_t SM_X = (SM_PART + SM_WARPS * 2 * 2 * MROWS * 4 + 127) & ~(size_t)127;
 __host__ __device__ constexpr size_t x_bytes(int K) { return ((size_t)3 * (K + 64) + (size_t)(K / 32) * 8 + 127) & ~(size_t)127; }
 
-// Balanced base-256 digits of four integers, |T| <= 127 * 65536: with 128 added to each digit they are the bytes of one sum.
-__device__ __forceinline__ void digits4(const int (&T)[4], uint32_t& q1, uint32_t& q2, uint32_t& q3) {
-    uint32_t u[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) u[i] = (uint32_t)(T[i] + 0x808080);
-    const uint32_t a = __byte_perm(u[0], u[1], 0x5140), b = __byte_perm(u[2], u[3], 0x5140);      // bytes 0 0 1 1
-    q3 = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
-    q2 = __byte_perm(a, b, 0x7632) ^ 0x80808080u;
-    q1 = __byte_perm(__byte_perm(u[0], u[1], 0x0062), __byte_perm(u[2], u[3], 0x0062), 0x5410) ^ 0x80808080u;
-}
 // Eight consecutive elements (t8 = their index / 8), four threads to a 32-element block: digits, scale and sum into shared memory.
 __device__ __forceinline__ void quantize8(const float (&x)[8], int t8, uint8_t* planes, int plane, float* xs, float* sums) {
     float amax = 0.f, s = 0.f;
@@ -396,6 +371,8 @@ void launch_fmt(KqParams& p, cudaStream_t s) {
 }
 
 }  // namespace
+
+int gemv_kq_format(DType dt) { return fmt_of(dt); }
 
 // Rows of whole super-blocks that start on 16-byte boundaries: what the entries that answer with a code (nt_b200_gemv_fused*) accept.
 bool gemv_kq_supported(const GemvMat* mats, int n_mat, int K) {

@@ -38,6 +38,32 @@ __device__ __forceinline__ uint32_t xword_byte(int e) {
     return (uint32_t)((((e >> 7) * 8 + ((e >> 5) & 1) * 4 + ((e >> 2) & 3)) << 4) + ((((e >> 6) & 1) * 2 + ((e >> 4) & 1)) << 2));
 }
 
+__device__ unsigned wait_expired;      // a wait below gave up: the launch's results are wrong
+
+// Waits for the phase of a copy or of a reader in this CTA, both under way: microseconds.  A limit far above that keeps a broken launch from
+// hanging the GPU.
+__device__ __forceinline__ void wait_phase(uint64_t* bar, uint32_t parity) {
+    uint32_t done = 0;
+    for (uint32_t spin = 0; !done; spin++) {
+        if (spin == (1u << 24)) { wait_expired = 1u; return; }
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    }
+}
+__device__ __forceinline__ void arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
+template <int N> __device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
+
+// Balanced base-256 digits of four integers, |T| <= 127 * 65536: with 128 added to each digit they are the bytes of one sum.
+__device__ __forceinline__ void digits4(const int (&T)[4], uint32_t& q1, uint32_t& q2, uint32_t& q3) {
+    uint32_t u[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) u[i] = (uint32_t)(T[i] + 0x808080);
+    const uint32_t a = __byte_perm(u[0], u[1], 0x5140), b = __byte_perm(u[2], u[3], 0x5140);      // bytes 0 0 1 1
+    q3 = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
+    q2 = __byte_perm(a, b, 0x7632) ^ 0x80808080u;
+    q1 = __byte_perm(__byte_perm(u[0], u[1], 0x0062), __byte_perm(u[2], u[3], 0x0062), 0x5410) ^ 0x80808080u;
+}
+
 __device__ __forceinline__ float half_bits(uint32_t h16) { return __half2float(__ushort_as_half((unsigned short)h16)); }
 // float(byte of w that sel picks) by PRMT into a 2^23 mantissa (exact)
 __device__ __forceinline__ float magic_byte(uint32_t w, uint32_t sel) { return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)) - 8388608.0f; }

@@ -66,6 +66,13 @@ bool gemv_kq_quarter(const GemvMat* mats, int n_mat, int K, const GemvInput& in,
 // epilogue GEMV_PEER: one matrix, rows == peer.hidden
 void gemv_kq_peer(const GemvMat& mat, int K, const GemvInput& in, const PeerOut& peer, cudaStream_t s);
 
+int gemv_kq_format(DType dt);             // the block formats' numbers in the two kernels, -1: none
+// gemv_rows.cu: the same matrices times a few tokens.  quantize_rows: F32 rows [tokens, K] (norm_w: their RMSNorm) into xr (gemv_rows_bytes);
+// gemv_rows: y of matrix i is [tokens, out_i] (STORE, ADD, SWIGLU); gemv_kq_any_pitch says what is taken.
+size_t gemv_rows_bytes(int tokens, int K);
+void quantize_rows(void* xr, const float* x, const float* norm_w, float eps, int tokens, int K, cudaStream_t s);
+void gemv_rows(const GemvMat* mats, int n_mat, int K, const void* xr, int tokens, GemvEpilogue ep, cudaStream_t s);
+
 // Generic GEMV for every dtype / any alignment, F32 activations (Q8_0, Q4_0, F16, F32 and
 // unaligned K-quant shards).
 void gemv_generic(float* y, const void* W, const float* x, int out, int in, DType dt, size_t row_pitch,
@@ -98,6 +105,11 @@ void attention_prefill(float* out, const float* Q, const void* kc, const void* v
 bool attention_prefill_mma_supported(int seq_len, int n_heads, int n_kv, int hd);
 void attention_prefill_mma(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads,
                            int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
+// A run of a few tokens at start_pos ..., each query with the decode step's F32 arithmetic (slices of the context, merged).
+bool attention_rows_supported(int total, int n_heads, int n_kv);
+size_t attention_rows_scratch_floats(int tokens, int max_seq, int n_heads, int n_kv, int hd);
+void attention_rows_f16(float* out, const float* q, const void* kc, const void* vc, int tokens, int start_pos, int n_heads, int n_kv, int hd, float scale,
+                        float* scratch, cudaStream_t s);
 // CUDA-graph friendly decode attention: context length = *pos_dev + 1 is read on the device.
 int attention_decode_dyn_splits(int max_seq, int n_heads, int n_kv);
 size_t attention_decode_dyn_scratch_floats(int max_seq, int n_heads, int n_kv, int hd);

@@ -821,12 +821,35 @@ bool Model::f16_direct(const Weight& w) const {
     return w.dtype == DType::F16 && gemm_f16_tc_supported(w.ptr, w.rows, w.cols, w.pitch);
 }
 
+// matrices in GGUF blocks are expanded inside the GEMM; only F32 and unaligned F16 weights go through a scratch pair
+bool Model::blocks_direct(const Weight& w) const {
+    GemvMat m; m.W = w.ptr; m.y = nullptr; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch;
+    return gemm_blocks_supported(&m, 1, w.cols);
+}
+
+// C_i (+)= A . W_i^T for matrices over the same rows
+void Model::prefill_gemms(float* const* C, const void* ws, const Weight* const* w, int n, int T, bool add, cudaStream_t s) {
+    GemvMat m[3];
+    bool blocks = n <= 3;
+    for (int i = 0; i < n && blocks; i++) {
+        blocks = blocks_direct(*w[i]);
+        m[i].W = w[i]->ptr; m[i].y = C[i]; m[i].out = w[i]->rows; m[i].dtype = w[i]->dtype; m[i].row_pitch = w[i]->pitch;
+    }
+    if (blocks) NT_CHECK(gemm_blocks(m, n, w[0]->cols, ws, T, add, s), "prefill GEMM over blocks rejected");
+    else for (int i = 0; i < n; i++) prefill_gemm(C[i], ws, *w[i], T, add, s);
+}
+
 void Model::prefill_gemm(float* C, const void* ws, const Weight& w, int T, bool add, cudaStream_t s) {
+    if (blocks_direct(w)) {
+        GemvMat m; m.W = w.ptr; m.y = C; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch;
+        NT_CHECK(gemm_blocks(&m, 1, w.cols, ws, T, add, s), "prefill GEMM over blocks rejected");
+        return;
+    }
     if (f16_direct(w)) {
         NT_CHECK(gemm_f16_tc_ws(C, ws, w.ptr, T, w.rows, w.cols, add, s), "prefill GEMM rejected");
         return;
     }
-    // quantised (or unaligned F16 / F32) weights: expand once per prompt chunk, then C (+)= A.W_hi^T ; C += A.W_lo^T
+    // unaligned F16 / F32 weights: expand once per prompt chunk, then C (+)= A.W_hi^T ; C += A.W_lo^T
     dequant_split(pf_.whi, pf_.wlo, w.ptr, w.dtype, w.pitch, w.rows, w.cols, s);
     NT_CHECK(gemm_f16_tc_ws(C, ws, pf_.whi, T, w.rows, w.cols, add, s), "prefill GEMM (hi) rejected");
     NT_CHECK(gemm_f16_tc_ws(C, ws, pf_.wlo, T, w.rows, w.cols, true, s), "prefill GEMM (lo) rejected");
@@ -851,7 +874,7 @@ void Model::ensure_prefill_buffers(int tokens) {
     bool swiglu_unfused = false;
     for (const LayerWeights& L : layers_) {
         for (const Weight* w : {&L.wq, &L.wk, &L.wv, &L.wo, &L.gate, &L.up, &L.down})
-            if (!f16_direct(*w)) w_elems = std::max(w_elems, (size_t)w->rows * (size_t)w->cols);
+            if (!f16_direct(*w) && !blocks_direct(*w)) w_elems = std::max(w_elems, (size_t)w->rows * (size_t)w->cols);
         swiglu_unfused = swiglu_unfused || !f16_direct(L.gate) || !f16_direct(L.up);
     }
     if (w_elems) { pf_.whi = dmalloc<uint16_t>(w_elems); pf_.wlo = dmalloc<uint16_t>(w_elems); }
@@ -885,9 +908,11 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
             uint16_t* vc = static_cast<uint16_t*>(vc_) + (size_t)i * kv_stride;
             // --- attention sub-block (attention.cpp:120-211 for all T tokens at once) ---
             rmsnorm_split(pf_.ws, pf_.x, L.attn_norm, T, hidden, cfg_.norm_eps, s);
-            prefill_gemm(pf_.q, pf_.ws, L.wq, T, false, s);
-            prefill_gemm(pf_.k, pf_.ws, L.wk, T, false, s);
-            prefill_gemm(pf_.v, pf_.ws, L.wv, T, false, s);
+            {
+                const Weight* w[3] = {&L.wq, &L.wk, &L.wv};
+                float* c[3] = {pf_.q, pf_.k, pf_.v};
+                prefill_gemms(c, pf_.ws, w, 3, T, false, s);
+            }
             rope(pf_.q, pf_.k, pf_.pos, T, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, false, s);
             copy_to_kv_cache(kc, vc, pf_.k, pf_.v, T, nkv_l_, hd, p0, max_seq, s);
             attention_prefill(pf_.attn, pf_.q, kc, vc, T, p0, nh_l_, nkv_l_, hd, max_seq, scale, s);
@@ -897,11 +922,11 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
             rmsnorm_split(pf_.ws, pf_.x, L.ffn_norm, T, hidden, cfg_.norm_eps, s);
             if (f16_direct(L.gate) && f16_direct(L.up)) {
                 NT_CHECK(gemm_f16_tc_swiglu_ws(pf_.ws2, pf_.ws, L.gate.ptr, L.up.ptr, T, inter, hidden, s), "prefill GEMM (gate/up) rejected");
-            } else {                                   // quantised gate/up: plain GEMMs, then SwiGLU and split as separate passes
-                prefill_gemm(pf_.g, pf_.ws, L.gate, T, false, s);
-                prefill_gemm(pf_.u, pf_.ws, L.up, T, false, s);
-                silu_mul(pf_.g, pf_.g, pf_.u, T * inter, s);
-                split_activations(pf_.ws2, pf_.g, T, inter, s);
+            } else {                                   // quantised gate/up: one plain GEMM over both, then SwiGLU and split in a pass
+                const Weight* w[2] = {&L.gate, &L.up};
+                float* c[2] = {pf_.g, pf_.u};
+                prefill_gemms(c, pf_.ws, w, 2, T, false, s);
+                silu_mul_split(pf_.ws2, pf_.g, pf_.u, T, inter, s);
             }
             prefill_gemm(pf_.x, pf_.ws2, L.down, T, true, s);
         }

@@ -165,6 +165,8 @@ public:
     void set_prefill_min_tokens(int n) { prefill_min_tokens_ = n; }
     bool batched_prefill_ok(int seq_len, int start_pos) const;
     bool short_batch_ok(int seq_len, int start_pos) const;
+    bool blocks_direct(const Weight& w) const;
+    void prefill_gemms(float* const* C, const void* ws, const Weight* const* w, int n, int T, bool add, cudaStream_t s);
     void ensure_short_buffers();
     void prefill_short(const int* tokens, int seq_len, int start_pos);
     struct { float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *act = nullptr, *scratch = nullptr; void* xr = nullptr;

@@ -499,6 +499,10 @@ inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
     NT_CUDA_CHECK(rc);
 }
 
+// prefill_blocks.cu: C_i [T, rows_i] (+)= X . W_i^T for up to three matrices in GGUF blocks, X split into a workspace; false: nothing launched.
+bool gemm_blocks_supported(const GemvMat* mats, int n_mat, int K);
+bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const void* workspace, int T, bool add, cudaStream_t s);
+void silu_mul_split(void* workspace, const float* gate, const float* up, int rows, int cols, cudaStream_t s);
 // prefill_gemm.cu: tcgen05/TMEM GEMM, C[M,N] = A[M,K] (F32, split hi+lo F16) . W[N,K]^T (F16)
 size_t gemm_f16_tc_workspace_bytes(int M, int K);
 bool gemm_f16_tc(float* C, const float* A, const void* W_f16, int M, int N, int K, void* workspace, cudaStream_t s);

@@ -361,12 +361,12 @@ void launch_fmt(KqParams& p, cudaStream_t s) {
     for (int i = 0; i < p.n_mat; i++) { p.mat[i].groups = (p.mat[i].out + MROWS - 1) / MROWS; total += p.mat[i].groups; }
     p.total_groups = p.n_seg == 2 ? p.mat[0].groups : total;
     // How the 16 warps of an SM are dealt out.  Teams of 4 share one copy of the vector and pay the meeting at the end of 16 rows half as often, four of
-    // them hide one another's barriers: the rule for every launch that gives each SM more than a group.  Fewer groups than SMs: the 8 warps of a team
-    // of its own finish a group sooner (Q8_0 1024 x 4096: 4.8 us, 6.2 in teams of 4; Q4_K 4096 x 4096, 256 groups: 5.1 and 4.9).  Long rows of few groups
-    // likewise, in one CTA since the vector does not fit twice (Q4_K 4096 x 14336: 11.4 us, 12.3 in teams of 4; 8192 x 28672, 512 groups: 37 and 39, Q6_K
-    // 50 and 48).  Q4_K 57344 x 8192: 45.5 us in teams of 4, 58 in teams of 8; 53.4 with the dp4a kernel that this one replaced.
+    // them hide one another's barriers: the rule for every launch that gives each SM more than a group (Q4_K 57344 x 8192: 45.5 us, 58 in teams of 8, 53.4
+    // with the dp4a kernel that this one replaced).  Fewer groups than SMs: more warps finish a group sooner, 8 (Q8_0 1024 x 4096: 4.8 us, 6.2 in teams of 4;
+    // Q4_K 4096 x 4096, 256 groups: 5.1 and 4.9), for long rows 16 (Q6_K 1024 x 14336: 9.9 us, 11.0 in a team of 8, 12.2 before; Q8_0 2048 x 28672: 23.2, 29.7,
+    // 24.5); in between two teams of 8 in a CTA, since the vector does not fit twice (Q4_K 4096 x 14336: 11.4 us, 12.3 in teams of 4, 16.9 before).
     if (p.K > 8192 ? p.total_groups > 256 : p.total_groups > 148) launch_teams<MASK, 4, 4>(p, s);
-    else if (p.K > 8192) launch_teams<MASK, 8, 2>(p, s);
+    else if (p.K > 8192) { if (p.total_groups > 148) launch_teams<MASK, 8, 2>(p, s); else launch_teams<MASK, 16, 1>(p, s); }
     else launch_teams<MASK, 8, 1>(p, s);
 }
 

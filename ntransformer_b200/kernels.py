@@ -15,17 +15,22 @@ from .dtypes import DType
 
 
 def _p(t):
-    if t is None:
-        return None
-    if isinstance(t, int):
-        return t
-    assert t.is_cuda and t.is_contiguous(), "expected a contiguous CUDA tensor"
-    return t.data_ptr()
+    if isinstance(t, torch.Tensor):
+        assert t.is_cuda and t.is_contiguous(), "expected a contiguous CUDA tensor"
+        return t.data_ptr()
+    return t          # a raw device pointer, or None
+
+
+_raw_stream = None    # (raw stream of a device, current device): torch's stream object costs more than the launch itself
 
 
 def _s(stream):
     if stream is None:
-        return torch.cuda.current_stream().cuda_stream
+        global _raw_stream
+        if _raw_stream is None:
+            torch.cuda.init()
+            _raw_stream = (torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice)
+        return _raw_stream[0](_raw_stream[1]())
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 

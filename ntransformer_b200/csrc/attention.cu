@@ -38,14 +38,6 @@ template <> struct HalfVec<2> { using T = uint32_t; };
 template <> struct HalfVec<4> { using T = uint2; };
 template <> struct HalfVec<8> { using T = uint4; };
 
-template <int DPL>
-__device__ __forceinline__ void load_row(const __half* p, float (&f)[DPL]) {
-    typename HalfVec<DPL>::T raw = __ldg(reinterpret_cast<const typename HalfVec<DPL>::T*>(p));
-    const __half2* h2 = reinterpret_cast<const __half2*>(&raw);
-#pragma unroll
-    for (int i = 0; i < DPL / 2; i++) { float2 t = __half22float2(h2[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
-}
-
 // Reduce GC per-lane partial sums across the warp. On return lane L holds (in v[0]) the full sum of
 // value index (L / (32 / GC)) ... valid in every lane of that group.
 template <int GC>
@@ -118,19 +110,39 @@ __device__ __forceinline__ void store_row_f16(__half* p, const __half (&h)[DPL])
 // One CTA: GC query heads of one KV head, keys [k_begin, k_end).
 // q_base: first of the GC heads' query vectors (contiguous [GC][hd]); out likewise.
 // If part_* != nullptr writes unnormalised partials, else the normalised output.
+// Bound by latency: a slice has few keys to a warp.  Each warp takes batches of KU consecutive keys with a running maximum of its own, so nothing waits for
+// another warp before the end, and the next batch's keys are on their way while the weights are formed, its values while the next scores are
+// (the form before it walked the slice three times, scores, softmax, values, with a barrier and a fetch in front of each: 64 heads, 8 key heads, 4000 keys
+// 12.6 + 5 us for the slices and their merge, 21 us a call).
+constexpr int P_LD = KU + 1;             // per warp: KU weights and the rescaling of what is summed so far, for each head
+template <int DPL, int GC> __host__ __device__ constexpr int attend_floats() { return AW * GC * P_LD + AW * GC * DPL * 32 + 2 * AW * GC; }
+
 template <int DPL, int GC>
 __device__ void attend_group(float* __restrict__ out, const float* __restrict__ q_base, const __half* __restrict__ kc,
                              const __half* __restrict__ vc, int kv_head, int n_kv, int k_begin, int k_end, float scale,
                              float* __restrict__ part_o, float* __restrict__ part_ml, float* smem, const NewToken nt = NewToken{}) {
-    constexpr int HD = DPL * 32;
+    constexpr int HD = DPL * 32, LG = 32 / GC;           // lanes that hold a head's score
+    using Raw = typename HalfVec<DPL>::T;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_keys = k_end - k_begin;
-    float* sc = smem;                                   // [GC][n_keys]
-    float* red = smem + (size_t)GC * n_keys;            // [AW][GC][HD]
-    __shared__ float s_max[GC], s_sum[GC];
+    float* pw = smem + (size_t)warp * GC * P_LD;         // this warp's weights [KU + 1][GC]
+    float* red = smem + (size_t)AW * GC * P_LD;          // [AW][GC][HD]
+    float* ml = red + (size_t)AW * GC * HD;              // [AW][GC][2]
     const size_t row_stride = (size_t)n_kv * HD;
     const __half* kbase = kc + (size_t)kv_head * HD + (size_t)lane * DPL;
     const __half* vbase = vc + (size_t)kv_head * HD + (size_t)lane * DPL;
+
+    Raw kr[KU], vr[KU];
+    auto fetch = [&](const __half* base, Raw (&r)[KU], int k0) {     // rows behind the slice are its last one: loaded, not used
+#pragma unroll
+        for (int u = 0; u < KU; u++) r[u] = __ldg(reinterpret_cast<const Raw*>(base + (size_t)min(k0 + u, k_end - 1) * row_stride));
+    };
+    auto to_float = [](const Raw& raw, float (&f)[DPL]) {
+        const __half2* h2 = reinterpret_cast<const __half2*>(&raw);
+#pragma unroll
+        for (int i = 0; i < DPL / 2; i++) { const float2 t = __half22float2(h2[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
+    };
+    int k0 = k_begin + warp * KU;
+    if (k0 < k_end) { fetch(kbase, kr, k0); fetch(vbase, vr, k0); }
 
     float qr[GC][DPL];
 #pragma unroll
@@ -143,130 +155,112 @@ __device__ void attend_group(float* __restrict__ out, const float* __restrict__ 
 #pragma unroll
         for (int g = 0; g < GC; g++) rope_rotate<DPL>(qr[g], rc, rs, lane);
     }
-
-    // ---- phase 1: scores (KU cache rows in flight per warp: one memory round trip per KU keys).  A slice of at most AW * KU
-    // keys is one batch: its V rows are fetched in the same round trip and wait in registers for phase 3. ----
-    const bool single = n_keys <= AW * KU;
-    float vpre[KU][DPL];
-    for (int p0 = warp; p0 < n_keys; p0 += AW * KU) {
-        float kf[KU][DPL];
-        if (single) {
-#pragma unroll
-            for (int u = 0; u < KU; u++) {
-                const int p = p0 + u * AW;
-                if (p >= n_keys) break;
-                if (k_begin + p != nt.pos) load_row<DPL>(vbase + (size_t)(k_begin + p) * row_stride, vpre[u]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < KU; u++) {
-            const int p = p0 + u * AW;
-            if (p >= n_keys) break;                          // warp-uniform
-            if (k_begin + p == nt.pos) {                     // warp-uniform: the new token's key, not in the cache yet
-#pragma unroll
-                for (int i = 0; i < DPL; i++) kf[u][i] = nt.k[(size_t)kv_head * HD + lane * DPL + i];
-                rope_rotate<DPL>(kf[u], rc, rs, lane);
-                __half kh[DPL];
-#pragma unroll
-                for (int i = 0; i < DPL; i++) { kh[i] = __float2half(kf[u][i]); kf[u][i] = __half2float(kh[i]); }
-                if (nt.kc_w) store_row_f16<DPL>(nt.kc_w + (size_t)nt.pos * row_stride + (size_t)kv_head * HD + (size_t)lane * DPL, kh);
-            } else {
-                load_row<DPL>(kbase + (size_t)(k_begin + p) * row_stride, kf[u]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < KU; u++) {
-            const int p = p0 + u * AW;
-            if (p >= n_keys) break;
-            float part[GC];
-#pragma unroll
-            for (int g = 0; g < GC; g++) {
-                float a = 0.f;
-#pragma unroll
-                for (int i = 0; i < DPL; i++) a = fmaf(qr[g][i], kf[u][i], a);
-                part[g] = a;
-            }
-            float tot = transpose_reduce<GC>(part, lane);
-            if ((lane & (32 / GC - 1)) == 0) sc[(size_t)(lane / (32 / GC)) * n_keys + p] = tot * scale;
-        }
-    }
-    __syncthreads();
-    // ---- phase 2: per-head max / exp / sum (warp g <-> head g) ----
-    for (int g = warp; g < GC; g += AW) {
-        float* s = sc + (size_t)g * n_keys;
-        float mx = -FLT_MAX;
-        for (int p = lane; p < n_keys; p += 32) mx = fmaxf(mx, s[p]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-        float sum = 0.f;
-        for (int p = lane; p < n_keys; p += 32) { float e = expf(s[p] - mx); s[p] = e; sum += e; }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-        if (lane == 0) { s_max[g] = mx; s_sum[g] = sum; }
-    }
-    __syncthreads();
-    // ---- phase 3: P.V (warp <-> keys, lane <-> DPL dims) ----
     float acc[GC][DPL];
 #pragma unroll
     for (int g = 0; g < GC; g++)
 #pragma unroll
         for (int i = 0; i < DPL; i++) acc[g][i] = 0.f;
-    for (int p0 = warp; p0 < n_keys; p0 += AW * KU) {
-        float vf[KU][DPL];
+    float mx = -FLT_MAX, sum = 0.f;                      // of head lane / LG
+    for (; k0 < k_end; k0 += AW * KU) {
+        float s[KU];
 #pragma unroll
         for (int u = 0; u < KU; u++) {
-            const int p = p0 + u * AW;
-            if (p >= n_keys) break;
-            if (k_begin + p == nt.pos) {                     // the new token's value: F16-rounded like the cache row it becomes
-                __half vh[DPL];
+            float kf[DPL];
+            to_float(kr[u], kf);
+            if (k0 + u == nt.pos) {                      // warp-uniform: the new token's key, not in the cache yet
 #pragma unroll
-                for (int i = 0; i < DPL; i++) { vh[i] = __float2half(nt.v[(size_t)kv_head * HD + lane * DPL + i]); vf[u][i] = __half2float(vh[i]); }
-                if (nt.vc_w) store_row_f16<DPL>(nt.vc_w + (size_t)nt.pos * row_stride + (size_t)kv_head * HD + (size_t)lane * DPL, vh);
-            } else if (single) {
+                for (int i = 0; i < DPL; i++) kf[i] = nt.k[(size_t)kv_head * HD + lane * DPL + i];
+                rope_rotate<DPL>(kf, rc, rs, lane);
+                __half kh[DPL];
 #pragma unroll
-                for (int i = 0; i < DPL; i++) vf[u][i] = vpre[u][i];
-            } else {
-                load_row<DPL>(vbase + (size_t)(k_begin + p) * row_stride, vf[u]);
+                for (int i = 0; i < DPL; i++) { kh[i] = __float2half(kf[i]); kf[i] = __half2float(kh[i]); }
+                if (nt.kc_w) store_row_f16<DPL>(nt.kc_w + (size_t)nt.pos * row_stride + (size_t)kv_head * HD + (size_t)lane * DPL, kh);
             }
-        }
-#pragma unroll
-        for (int u = 0; u < KU; u++) {
-            const int p = p0 + u * AW;
-            if (p >= n_keys) break;
+            float part[GC];
 #pragma unroll
             for (int g = 0; g < GC; g++) {
-                float w = sc[(size_t)g * n_keys + p];
+                float a = 0.f;
 #pragma unroll
-                for (int i = 0; i < DPL; i++) acc[g][i] = fmaf(w, vf[u][i], acc[g][i]);
+                for (int i = 0; i < DPL; i++) a = fmaf(qr[g][i], kf[i], a);
+                part[g] = a;
+            }
+            const float tot = transpose_reduce<GC>(part, lane) * scale;
+            s[u] = k0 + u < k_end ? tot : -FLT_MAX;
+        }
+        if (k0 + AW * KU < k_end) fetch(kbase, kr, k0 + AW * KU);
+        float m2 = mx;
+#pragma unroll
+        for (int u = 0; u < KU; u++) m2 = fmaxf(m2, s[u]);
+        const float corr = expf(mx - m2);                // the first batch: 0, or 1 where no score lies above -FLT_MAX (then the sums are 0)
+        mx = m2;
+        sum *= corr;
+#pragma unroll
+        for (int u = 0; u < KU; u++) {
+            s[u] = k0 + u < k_end ? expf(s[u] - m2) : 0.f;
+            sum += s[u];
+        }
+        __syncwarp();                                    // the weights of the batch before have been read
+        if ((lane & (LG - 1)) == 0) {
+#pragma unroll
+            for (int u = 0; u < KU; u++) pw[u * GC + lane / LG] = s[u];
+            pw[KU * GC + lane / LG] = corr;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < GC; g++) {
+            const float c = pw[KU * GC + g];
+#pragma unroll
+            for (int i = 0; i < DPL; i++) acc[g][i] *= c;
+        }
+#pragma unroll
+        for (int u = 0; u < KU; u++) {
+            if (k0 + u >= k_end) break;
+            float vf[DPL];
+            to_float(vr[u], vf);
+            if (k0 + u == nt.pos) {                      // the new token's value: F16-rounded like the cache row it becomes
+                __half vh[DPL];
+#pragma unroll
+                for (int i = 0; i < DPL; i++) { vh[i] = __float2half(nt.v[(size_t)kv_head * HD + lane * DPL + i]); vf[i] = __half2float(vh[i]); }
+                if (nt.vc_w) store_row_f16<DPL>(nt.vc_w + (size_t)nt.pos * row_stride + (size_t)kv_head * HD + (size_t)lane * DPL, vh);
+            }
+#pragma unroll
+            for (int g = 0; g < GC; g++) {
+                const float w = pw[u * GC + g];
+#pragma unroll
+                for (int i = 0; i < DPL; i++) acc[g][i] = fmaf(w, vf[i], acc[g][i]);
             }
         }
+        if (k0 + AW * KU < k_end) fetch(vbase, vr, k0 + AW * KU);
     }
 #pragma unroll
     for (int g = 0; g < GC; g++)
 #pragma unroll
         for (int i = 0; i < DPL; i++) red[((size_t)warp * GC + g) * HD + lane * DPL + i] = acc[g][i];
+    if ((lane & (LG - 1)) == 0) { ml[(warp * GC + lane / LG) * 2] = mx; ml[(warp * GC + lane / LG) * 2 + 1] = sum; }
     __syncthreads();
     for (int idx = threadIdx.x; idx < GC * HD; idx += AW * 32) {
-        float t = 0.f;
-#pragma unroll
-        for (int w = 0; w < AW; w++) t += red[(size_t)w * GC * HD + idx];
         const int g = idx / HD, d = idx - g * HD;
+        float m = -FLT_MAX, l = 0.f, t = 0.f;
+#pragma unroll
+        for (int w = 0; w < AW; w++) m = fmaxf(m, ml[(w * GC + g) * 2]);
+#pragma unroll
+        for (int w = 0; w < AW; w++) {                   // a warp without keys has sums of 0
+            const float f = expf(ml[(w * GC + g) * 2] - m);
+            l = fmaf(ml[(w * GC + g) * 2 + 1], f, l);
+            t = fmaf(red[(size_t)w * GC * HD + idx], f, t);
+        }
         if (part_o) {
             part_o[(size_t)g * HD + d] = t;             // caller strides heads by HD inside its split slot
+            if (d == 0) { part_ml[2 * g] = m; part_ml[2 * g + 1] = l; }
         } else {
-            float l = s_sum[g];
             out[(size_t)g * HD + d] = t * ((l > 0.f) ? 1.0f / l : 0.f);
         }
-    }
-    if (part_ml && threadIdx.x < GC) {
-        part_ml[2 * threadIdx.x] = s_max[threadIdx.x];
-        part_ml[2 * threadIdx.x + 1] = s_sum[threadIdx.x];
     }
 }
 
 // Scratch layout for split decode: [head][split][HD] floats then [head][split][2] (max, sum).
 template <int DPL, int GC>
-__global__ void __launch_bounds__(AW * 32) decode_kernel(float* __restrict__ out, const float* __restrict__ q,
+__global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) decode_kernel(float* __restrict__ out, const float* __restrict__ q,
                                                          const __half* __restrict__ kc, const __half* __restrict__ vc,
                                                          int seq_len, int n_heads, int n_kv, float scale, int n_splits,
                                                          int split_len, float* __restrict__ scratch,
@@ -295,7 +289,7 @@ __global__ void __launch_bounds__(AW * 32) decode_kernel(float* __restrict__ out
     } else {
         // partials for head (head0+g) live at scratch[((head0+g) * n_splits + split) * HD]; attend_group strides
         // heads by HD, so hand it a staging area in shared memory and scatter afterwards.
-        float* stage = smem_dyn + (size_t)GC * (k_end - k_begin) + (size_t)AW * GC * HD;   // [GC][HD] + [GC][2]
+        float* stage = smem_dyn + attend_floats<DPL, GC>();   // [GC][HD] + [GC][2]
         attend_group<DPL, GC>(nullptr, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale, stage,
                               stage + GC * HD, smem_dyn);
         __syncthreads();
@@ -384,7 +378,7 @@ __global__ void decode_combine_kernel(float* __restrict__ out, const float* __re
 // K16 attention.cu:108-202); the merge keeps decode_combine_kernel's arithmetic and order, so both paths agree bit for bit
 // whenever they cut the context at the same places.
 template <int DPL, int GC>
-__global__ void __launch_bounds__(AW * 32) decode_fused_kernel(float* __restrict__ out, const float* __restrict__ q,
+__global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) decode_fused_kernel(float* __restrict__ out, const float* __restrict__ q,
                                                                const float* __restrict__ k_new, const float* __restrict__ v_new,
                                                                __half* __restrict__ kc, __half* __restrict__ vc,
                                                                const int* __restrict__ pos_dev, int n_heads, int n_kv, float scale,
@@ -412,7 +406,7 @@ __global__ void __launch_bounds__(AW * 32) decode_fused_kernel(float* __restrict
                               smem_dyn, nt);
         return;
     }
-    float* stage = smem_dyn + (size_t)GC * (k_end - k_begin) + (size_t)AW * GC * HD;   // [GC][HD] + [GC][2]
+    float* stage = smem_dyn + attend_floats<DPL, GC>();   // [GC][HD] + [GC][2]
     attend_group<DPL, GC>(nullptr, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale, stage, stage + GC * HD,
                           smem_dyn, nt);
     __syncthreads();
@@ -469,7 +463,7 @@ __global__ void __launch_bounds__(AW * 32) decode_fused_kernel(float* __restrict
 }
 
 template <int DPL, int GC>
-__global__ void __launch_bounds__(AW * 32) prefill_kernel(float* __restrict__ out, const float* __restrict__ Q,
+__global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) prefill_kernel(float* __restrict__ out, const float* __restrict__ Q,
                                                           const __half* __restrict__ kc, const __half* __restrict__ vc,
                                                           int start_pos, int n_heads, int n_kv, float scale) {
     constexpr int HD = DPL * 32;
@@ -512,10 +506,9 @@ void launch_decode(float* out, const float* q, const __half* kc, const __half* v
     }
     int split_len = (seq_len + n_splits - 1) / n_splits;
     n_splits = (seq_len + split_len - 1) / split_len;
-    size_t smem = ((size_t)GC * split_len + (size_t)AW * GC * HD + (size_t)GC * HD + 2 * GC) * sizeof(float);
+    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
-    NT_CHECK(smem <= (size_t)ATTN_MAX_DYN_SMEM, "attention_decode: context slice does not fit shared memory");
     float* scratch = nullptr;
     if (n_splits > 1) scratch = attn_scratch((size_t)n_heads * n_splits * (HD + 2));
     decode_kernel<DPL, GC><<<dim3(groups, n_splits), AW * 32, smem, s>>>(out, q, kc, vc, seq_len, n_heads, n_kv, scale,
@@ -527,11 +520,10 @@ void launch_decode(float* out, const float* q, const __half* kc, const __half* v
     }
 }
 
-// Slices of a run of `tokens` queries: enough CTAs for the chip, at least 32 keys each, none longer than the shared memory of one holds.
-int rows_splits(int tokens, int total, int groups, int gc) {
+// Slices of a run of `tokens` queries: enough CTAs for the chip, at least 32 keys each.
+int rows_splits(int tokens, int total, int groups) {
     int n = (2 * 148 + groups * tokens - 1) / (groups * tokens);
     n = std::min(std::min(n, (total + 31) / 32), MAX_SPLITS);
-    n = std::max(n, (total + 16384 / gc - 1) / (16384 / gc));
     return std::max(1, n);
 }
 // A few consecutive queries (start_pos ...), each with the arithmetic of a decoded token; scratch: attention_rows_scratch_floats().
@@ -540,13 +532,13 @@ void launch_rows(float* out, const float* q, const __half* kc, const __half* vc,
                  cudaStream_t s) {
     constexpr int HD = DPL * 32;
     const int groups = n_heads / GC, total = start_pos + tokens;
-    int n_splits = rows_splits(tokens, total, groups, GC);
+    int n_splits = rows_splits(tokens, total, groups);
     const int split_len = (total + n_splits - 1) / n_splits;
     n_splits = (total + split_len - 1) / split_len;
-    const size_t smem = ((size_t)GC * split_len + (size_t)AW * GC * HD + (size_t)GC * HD + 2 * GC) * sizeof(float);
+    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
-    NT_CHECK(smem <= (size_t)ATTN_MAX_DYN_SMEM && n_splits <= MAX_SPLITS, "attention over a run of tokens: context beyond the slices");
+    NT_CHECK(n_splits <= MAX_SPLITS, "attention over a run of tokens: context beyond the slices");
     launch_k(decode_kernel<DPL, GC>, dim3(groups, n_splits, tokens), dim3(AW * 32), smem, s, out, q, kc, vc, start_pos + 1, n_heads, n_kv, scale, n_splits, split_len,
              scratch, (const int*)nullptr);
     count_launch();
@@ -564,9 +556,7 @@ void launch_decode_dyn(float* out, const float* q, const __half* kc, const __hal
                        int n_heads, int n_kv, float scale, float* scratch, int n_splits, int8_t* xq_out, cudaStream_t s) {
     constexpr int HD = DPL * 32;
     const int groups = n_heads / GC;
-    const int max_split_len = std::max((max_seq + n_splits - 1) / n_splits, DYN_MIN_SPLIT);
-    size_t smem = ((size_t)GC * max_split_len + (size_t)AW * GC * HD + (size_t)GC * HD + 2 * GC) * sizeof(float);
-    NT_CHECK(smem <= (size_t)ATTN_MAX_DYN_SMEM, "attention_decode_dyn: context slice does not fit shared memory");
+    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     launch_k(decode_kernel<DPL, GC>, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, kc, vc, 0, n_heads, n_kv, scale,
@@ -581,10 +571,7 @@ void launch_decode_fused(float* out, const float* q, const float* k_new, const f
                          unsigned* tickets, int8_t* xq_out, cudaStream_t s) {
     constexpr int HD = DPL * 32;
     const int groups = n_heads / GC;
-    int max_split_len = (max_seq + n_splits - 1) / n_splits;
-    if (max_split_len < FUSED_MIN_SPLIT) max_split_len = FUSED_MIN_SPLIT;
-    size_t smem = ((size_t)GC * max_split_len + (size_t)AW * GC * HD + (size_t)GC * HD + 2 * GC) * sizeof(float);
-    NT_CHECK(smem <= (size_t)ATTN_MAX_DYN_SMEM, "attention_decode_fused: context slice does not fit shared memory");
+    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_fused_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     launch_k(decode_fused_kernel<DPL, GC>, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, k_new, v_new, kc, vc, pos_dev, n_heads,
@@ -600,9 +587,7 @@ void launch_decode_rope_dyn(float* out, const float* q, const float* k_new, cons
                             int8_t* xq_out, cudaStream_t s) {
     constexpr int HD = DPL * 32;
     const int groups = n_heads / GC;
-    const int max_split_len = std::max((max_seq + n_splits - 1) / n_splits, DYN_MIN_SPLIT);
-    size_t smem = ((size_t)GC * max_split_len + (size_t)AW * GC * HD + (size_t)GC * HD + 2 * GC) * sizeof(float);
-    NT_CHECK(smem <= (size_t)ATTN_MAX_DYN_SMEM, "attention_decode_rope_dyn: context slice does not fit shared memory");
+    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_fused_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     launch_k(decode_fused_kernel<DPL, GC>, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, k_new, v_new, kc, vc, pos_dev, n_heads,
@@ -614,9 +599,7 @@ void launch_decode_rope_dyn(float* out, const float* q, const float* k_new, cons
 template <int DPL, int GC>
 void launch_prefill(float* out, const float* Q, const __half* kc, const __half* vc, int seq_len, int start_pos, int n_heads,
                     int n_kv, float scale, cudaStream_t s) {
-    constexpr int HD = DPL * 32;
-    size_t smem = ((size_t)GC * (start_pos + seq_len) + (size_t)AW * GC * HD) * sizeof(float);
-    NT_CHECK(smem <= (size_t)ATTN_MAX_DYN_SMEM, "attention_prefill: context does not fit shared memory");
+    const size_t smem = (size_t)attend_floats<DPL, GC>() * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(prefill_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     prefill_kernel<DPL, GC><<<dim3(n_heads / GC, seq_len), AW * 32, smem, s>>>(out, Q, kc, vc, start_pos, n_heads, n_kv, scale);
@@ -652,14 +635,10 @@ void attention_decode(float* out, const float* q, const void* kc, const void* vc
     NT_DISPATCH_ATTN(launch_decode, out, q, k, v, seq_len, n_heads, n_kv, scale, s);
 }
 
-bool attention_rows_supported(int total, int n_heads, int n_kv) {
-    const int gc = pick_gc(n_heads / n_kv);
-    return rows_splits(1, total, n_heads / gc, gc) <= MAX_SPLITS;
-}
 size_t attention_rows_scratch_floats(int tokens, int max_seq, int n_heads, int n_kv, int hd) {
     const int gc = pick_gc(n_heads / n_kv);
     size_t most = 0;                     // fewer tokens are cut into more slices
-    for (int t = 1; t <= tokens; t++) most = std::max(most, (size_t)t * n_heads * rows_splits(t, max_seq, n_heads / gc, gc) * (hd + 2));
+    for (int t = 1; t <= tokens; t++) most = std::max(most, (size_t)t * n_heads * rows_splits(t, max_seq, n_heads / gc) * (hd + 2));
     return most;
 }
 void attention_rows_f16(float* out, const float* q, const void* kc, const void* vc, int tokens, int start_pos, int n_heads, int n_kv, int hd, float scale,

@@ -765,7 +765,7 @@ bool Model::short_batch_ok(int seq_len, int start_pos) const {
     if (tp_size_ != 1 || seq_len < 2 || prefill_min_tokens_ <= 0 || getenv("NT_B200_NO_BATCHED_PREFILL") || (fuse_mask_ & 6)) return false;
     const char* mk = getenv("NT_B200_MEGAKERNEL");
     if (mk ? env_on("NT_B200_MEGAKERNEL") : use_mega_) return false;
-    return chain_ok() && attention_rows_supported(start_pos + seq_len, nh_l_, nkv_l_);
+    return chain_ok();
 }
 
 void Model::ensure_short_buffers() {

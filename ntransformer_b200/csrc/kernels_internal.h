@@ -106,7 +106,6 @@ bool attention_prefill_mma_supported(int seq_len, int n_heads, int n_kv, int hd)
 void attention_prefill_mma(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads,
                            int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
 // A run of a few tokens at start_pos ..., each query with the decode step's F32 arithmetic (slices of the context, merged).
-bool attention_rows_supported(int total, int n_heads, int n_kv);
 size_t attention_rows_scratch_floats(int tokens, int max_seq, int n_heads, int n_kv, int hd);
 void attention_rows_f16(float* out, const float* q, const void* kc, const void* vc, int tokens, int start_pos, int n_heads, int n_kv, int hd, float scale,
                         float* scratch, cudaStream_t s);

@@ -835,8 +835,11 @@ void Model::prefill_gemms(float* const* C, const void* ws, const Weight* const* 
         blocks = blocks_direct(*w[i]);
         m[i].W = w[i]->ptr; m[i].y = C[i]; m[i].out = w[i]->rows; m[i].dtype = w[i]->dtype; m[i].row_pitch = w[i]->pitch;
     }
-    if (blocks) NT_CHECK(gemm_blocks(m, n, w[0]->cols, ws, T, add, s), "prefill GEMM over blocks rejected");
-    else for (int i = 0; i < n; i++) prefill_gemm(C[i], ws, *w[i], T, add, s);
+    if (blocks) { NT_CHECK(gemm_blocks(m, n, w[0]->cols, ws, T, add, s), "prefill GEMM over blocks rejected"); return; }
+    bool f16 = !add && n > 1 && n <= TC_MULTI_MAX;                 // F16 in place: narrow matrices fill the SMs together
+    const void* W[TC_MULTI_MAX]; int N[TC_MULTI_MAX];
+    for (int i = 0; i < n && f16; i++) { f16 = f16_direct(*w[i]) && w[i]->rows >= 256; W[i] = w[i]->ptr; N[i] = w[i]->rows; }
+    if (!f16 || !gemm_f16_tc_multi_ws(C, ws, W, N, n, T, w[0]->cols, s)) for (int i = 0; i < n; i++) prefill_gemm(C[i], ws, *w[i], T, add, s);
 }
 
 void Model::prefill_gemm(float* C, const void* ws, const Weight& w, int T, bool add, cudaStream_t s) {

@@ -206,24 +206,27 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                               // ---- MMA issuer ----
-            uint32_t it = 0, lt = 0;
-            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x)
-            for (int kc = 0; kc < n_kc; kc++, lt++) {
-                const uint32_t acc = lt & 1, acc_phase = (lt >> 1) & 1;
-                wait_or_trap(&tmem_empty_bar[acc], acc_phase ^ 1);         // epilogue drained this accumulator
+        // ---- MMA: the whole warp walks the loop, so that addresses and descriptors stay in uniform registers, and one lane issues (a loop of lane 0 alone
+        // moves every operand of every MMA there) ----
+        const bool leader = elect_lane();
+        const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);
+        const uint64_t desc0 = make_desc(smem);
+        constexpr uint64_t LO = TILE_A >> 4, B = (2 * TILE_A) >> 4, B2 = (2 * TILE_A + 128 * BK * 2) >> 4;
+        uint32_t s = 0, par = 0, lt = 0;
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x)
+        for (int kc = 0; kc < n_kc; kc++, lt++) {
+            const uint32_t acc = lt & 1, acc_phase = (lt >> 1) & 1;
+            wait_or_trap(&tmem_empty_bar[acc], acc_phase ^ 1);             // epilogue drained this accumulator
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t d = tm + acc * BN;
+            const int kb0 = ONE_CHUNK ? 0 : kc * kc_blocks, kb1 = ONE_CHUNK ? num_kb : min(num_kb, kb0 + kc_blocks);
+            for (int kb = kb0; kb < kb1; kb++) {
+                wait_or_trap(&full_bar[s], par);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem_base + acc * BN;
-                const int kb0 = ONE_CHUNK ? 0 : kc * kc_blocks, kb1 = ONE_CHUNK ? num_kb : min(num_kb, kb0 + kc_blocks);
-                for (int kb = kb0; kb < kb1; kb++, it++) {
-                    const uint32_t s = it % STAGES;
-                    wait_or_trap(&full_bar[s], (it / STAGES) & 1);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint8_t* st = smem + (size_t)s * STAGE_BYTES;
-                    const uint64_t da_hi = make_desc(st), da_lo = make_desc(st + TILE_A), db = make_desc(st + 2 * TILE_A);
-                    const uint64_t db2 = make_desc(st + 2 * TILE_A + 128 * BK * 2);
+                const uint64_t da_hi = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), da_lo = da_hi + LO, db = da_hi + B, db2 = da_hi + B2;
+                if (leader) {
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; k++) {  // advance 32 bytes (>> 4 = 2) inside the 128-byte swizzle row
+                    for (int k = 0; k < BK / UMMA_K; k++) {      // advance 32 bytes (>> 4 = 2) inside the 128-byte swizzle row
                         umma_f16(d, da_hi + 2 * k, db + 2 * k, IDESC, ((kb - kb0) | k) ? 1u : 0u);
                         if (MODE == MODE_SWIGLU) umma_f16(d + 128, da_hi + 2 * k, db2 + 2 * k, IDESC, (kb | k) ? 1u : 0u);
                     }
@@ -232,9 +235,11 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
                         umma_f16(d, da_lo + 2 * k, db + 2 * k, IDESC, 1u);
                         if (MODE == MODE_SWIGLU) umma_f16(d + 128, da_lo + 2 * k, db2 + 2 * k, IDESC, 1u);
                     }
-                    umma_commit(&empty_bar[s]);        // smem slot reusable once these MMAs retire
+                    umma_commit(&empty_bar[s]);            // smem slot reusable once these MMAs retire
+                    if (kb + 1 == kb1) umma_commit(&tmem_full_bar[acc]);      // accumulator complete
                 }
-                umma_commit(&tmem_full_bar[acc]);      // accumulator complete
+                __syncwarp();
+                if (++s == STAGES) { s = 0; par ^= 1; }
             }
         }
     } else {

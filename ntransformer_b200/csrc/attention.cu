@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) decode_kernel
                                                          const int* __restrict__ pos_dev) {
     constexpr int HD = DPL * 32;
     extern __shared__ float smem_dyn[];
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();
     if (pos_dev) {                       // CUDA-graph replay: context length lives in device memory
         seq_len = *pos_dev + 1;
         split_len = max((seq_len + n_splits - 1) / n_splits, DYN_MIN_SPLIT);
@@ -314,8 +314,8 @@ __global__ void decode_combine_kernel(float* __restrict__ out, const float* __re
     __shared__ float w_s[MAX_SPLITS];                // e^{m_i - m} per slice
     __shared__ float inv_s;
     const int h = blockIdx.x;
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();
     seq_len += blockIdx.y;               // a run of tokens: blockIdx.y is the query
     scratch += (size_t)blockIdx.y * n_heads * n_splits * (hd + 2);
     out += (size_t)blockIdx.y * n_heads * hd;
@@ -388,8 +388,8 @@ __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) decode_fused_
     constexpr int HD = DPL * 32;
     extern __shared__ float smem_dyn[];
     __shared__ int s_last;
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();
     const int pos = *pos_dev, seq_len = pos + 1;
     int split_len = (seq_len + n_splits - 1) / n_splits;
     if (split_len < min_split) split_len = min_split;      // short contexts: few, reasonably long slices
@@ -511,11 +511,13 @@ void launch_decode(float* out, const float* q, const __half* kc, const __half* v
     opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     float* scratch = nullptr;
     if (n_splits > 1) scratch = attn_scratch((size_t)n_heads * n_splits * (HD + 2));
-    decode_kernel<DPL, GC><<<dim3(groups, n_splits), AW * 32, smem, s>>>(out, q, kc, vc, seq_len, n_heads, n_kv, scale,
-                                                                        n_splits, split_len, scratch, nullptr);
+    // Programmatic launches outside graphs too: neither kernel reads or writes before its wait, so the merge's launch hides behind the slices
+    launch_k_pdl(true, decode_kernel<DPL, GC>, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, kc, vc, seq_len, n_heads, n_kv, scale, n_splits, split_len,
+                 scratch, (const int*)nullptr);
     count_launch();
     if (n_splits > 1) {
-        decode_combine_kernel<<<n_heads, 128, 0, s>>>(out, scratch, n_heads, HD, n_splits, seq_len, split_len, nullptr, nullptr);
+        launch_k_pdl(true, decode_combine_kernel, dim3(n_heads), dim3(128), 0, s, out, (const float*)scratch, n_heads, HD, n_splits, seq_len, split_len, (const int*)nullptr,
+                     (int8_t*)nullptr);
         count_launch();
     }
 }

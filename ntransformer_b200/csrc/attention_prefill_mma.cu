@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(128, 2) prefill_mma_kernel(float* __restrict__
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
+    const bool plain = window <= 0 && chunk <= 0 && softcap <= 0.f && !slopes;
     load_tile(0, 0);
     for (int j = 0; j < n_tiles; j++) {
         const int st = j & 1;
@@ -132,17 +133,32 @@ __global__ void __launch_bounds__(128, 2) prefill_mma_kernel(float* __restrict__
         for (int n = 0; n < 8; n++) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
 #pragma unroll
         for (int ks = 0; ks < KS; ks++) {
+            // all eight blocks of keys with the high half, then with the low: a product waits for the one eight before it, not for its neighbour
+            uint32_t kb[4][4];
 #pragma unroll
-            for (int n = 0; n < 8; n++) {
-                const __half* kp = tK + (size_t)(n * 8 + g) * LD + ks * 16 + 2 * t;
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(kp), b1 = *reinterpret_cast<const uint32_t*>(kp + 8);
-                mma16816<BF>(s[n], qhi[ks], b0, b1);
-                mma16816<BF>(s[n], qlo[ks], b0, b1);
+            for (int n2 = 0; n2 < 4; n2++) {             // four 8x8 blocks of K: (keys +0..7 | +8..15) x (dims +0..7 | +8..15)
+                const __half* kp = tK + (size_t)(n2 * 16 + (lane & 7) + (lane >> 4) * 8) * LD + ks * 16 + ((lane >> 3) & 1) * 8;
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(kb[n2][0]), "=r"(kb[n2][1]), "=r"(kb[n2][2]), "=r"(kb[n2][3]) : "r"((uint32_t)__cvta_generic_to_shared(kp)));
             }
+#pragma unroll
+            for (int n = 0; n < 8; n++) mma16816<BF>(s[n], qhi[ks], kb[n >> 1][2 * (n & 1)], kb[n >> 1][2 * (n & 1) + 1]);
+#pragma unroll
+            for (int n = 0; n < 8; n++) mma16816<BF>(s[n], qlo[ks], kb[n >> 1][2 * (n & 1)], kb[n >> 1][2 * (n & 1) + 1]);
         }
         // ---- scale, causal mask, online softmax ----
         const int key0 = tile_of(j) * BKV;
         float mx0 = -INFINITY, mx1 = -INFINITY;
+        // a tile that every row of the warp sees whole, without cap or slope, needs no per-score rule
+        if (plain && key0 + BKV - 1 <= start_pos + qb * BQ + warp * 16) {
+#pragma unroll
+            for (int n = 0; n < 8; n++) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) s[n][i] *= scale;
+                mx0 = fmaxf(mx0, fmaxf(s[n][0], s[n][1]));
+                mx1 = fmaxf(mx1, fmaxf(s[n][2], s[n][3]));
+            }
+        } else
 #pragma unroll
         for (int n = 0; n < 8; n++) {
 #pragma unroll
@@ -185,17 +201,21 @@ __global__ void __launch_bounds__(128, 2) prefill_mma_kernel(float* __restrict__
             split2<BF>(s[2 * kt][2], s[2 * kt][3], phi[1], plo[1]);
             split2<BF>(s[2 * kt + 1][0], s[2 * kt + 1][1], phi[2], plo[2]);
             split2<BF>(s[2 * kt + 1][2], s[2 * kt + 1][3], phi[3], plo[3]);
+            constexpr int G = HDV % 64 == 0 ? 4 : HDV % 32 == 0 ? 2 : 1;     // blocks of 16 columns whose products are interleaved
 #pragma unroll
-            for (int np = 0; np < HDV / 16; np++) {
+            for (int np = 0; np < HDV / 16; np += G) {
                 // four 8x8 blocks of V^T: (keys +0..7 | +8..15) x (hd +0..7 | +8..15)
-                const __half* vp = tV + (size_t)(kt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDV + np * 16 + (lane >> 4) * 8;
-                uint32_t v0, v1, v2, v3;
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3) : "r"((uint32_t)__cvta_generic_to_shared(vp)));
-                mma16816<BF>(o[2 * np], phi, v0, v1);
-                mma16816<BF>(o[2 * np], plo, v0, v1);
-                mma16816<BF>(o[2 * np + 1], phi, v2, v3);
-                mma16816<BF>(o[2 * np + 1], plo, v2, v3);
+                uint32_t v[G][4];
+#pragma unroll
+                for (int q = 0; q < G; q++) {
+                    const __half* vp = tV + (size_t)(kt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDV + (np + q) * 16 + (lane >> 4) * 8;
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(v[q][0]), "=r"(v[q][1]), "=r"(v[q][2]), "=r"(v[q][3]) : "r"((uint32_t)__cvta_generic_to_shared(vp)));
+                }
+#pragma unroll
+                for (int q = 0; q < G; q++) { mma16816<BF>(o[2 * (np + q)], phi, v[q][0], v[q][1]); mma16816<BF>(o[2 * (np + q) + 1], phi, v[q][2], v[q][3]); }
+#pragma unroll
+                for (int q = 0; q < G; q++) { mma16816<BF>(o[2 * (np + q)], plo, v[q][0], v[q][1]); mma16816<BF>(o[2 * (np + q) + 1], plo, v[q][2], v[q][3]); }
             }
         }
         __syncthreads();                                             // this stage is overwritten by the prefetch of tile j + 2

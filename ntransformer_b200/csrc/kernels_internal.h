@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 #include "nt_types.h"
 
 namespace nt { namespace b200 {
@@ -486,16 +487,20 @@ void mlstm_token(float* out, const float* q, const float* k, const float* v, con
 void set_pdl(bool on);
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>
-inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+inline void launch_k_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    at[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
     cfg.attrs = at; cfg.numAttrs = 1;
     const cudaError_t rc = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
     if (rc != cudaSuccess) fprintf(stderr, "launch of grid (%u, %u, %u), block %u, %zu bytes of shared memory:\n", grid.x, grid.y, grid.z, block.x, smem);
     NT_CUDA_CHECK(rc);
+}
+template <typename... KArgs, typename... Args>
+inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+    launch_k_pdl(pdl_enabled(), kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
 // prefill_blocks.cu: C_i [T, rows_i] (+)= X . W_i^T for up to three matrices in GGUF blocks, X split into a workspace; false: nothing launched.

@@ -6,7 +6,7 @@
 // Keys and values come from the per-layer cache ([max_seq, kv_heads * dim] and [max_seq, kv_heads * vdim], F32 or BF16 storage):
 // the caller writes the step's rows first (qk_norm_kv_write), so a prompt portion, a whole prompt and a decoded token all take the
 // same kernel and see the same stored values.  Softmax, score and the weighted sum are F32.
-//   one CTA per (query token, head); its warps stride over the visible keys (the kept prefix, then the window) in groups of 32
+//   one CTA per (query token, head); its warps stride over the visible keys (the kept prefix, then the window) in groups
 //   with a running (max, sum, acc) each, merged through shared memory at the end; for a single decoded token the keys of a head
 //   are further split over the CTAs of a thread-block cluster and merged through the leader's distributed shared memory.  Prompts over a BF16 cache with equal key and
 //   value width go to the tiled tensor-core form in attention_prefill_mma.cu instead.
@@ -68,10 +68,92 @@ __device__ __forceinline__ float dot_row(const __nv_bfloat16* row, const float* 
     return d;
 }
 
-// Warps take groups of 32 visible keys.  Scoring is lane-per-key (each lane walks one key row against q in shared memory: no
-// cross-lane reduction per key); the group's maximum and the rescale are one warp reduction; the weighted value sum is
-// lane-per-channel (the 32 probabilities are broadcast one by one, value rows are read coalesced).
-template <typename KT, int AW_MAXV>       // AW_MAXV: value elements per lane (vdim <= 32 * AW_MAXV)
+// BF16 rows whose pieces of 8 numbers start on 16 bytes: LPK lanes read a row together (8 numbers each: rows of up to 8 * LPK), so a warp reads
+// 32 / LPK rows at a time and takes 8 such turns at once.  Every key and value load of a group is under way before the first score is formed:
+// one trip to memory per group, where a lane per key row takes a chain of them (rows of 256 bytes walked by a lane each, then 32 value rows two
+// bytes to a lane).  The 8 scores of a lane group are reduced together: each exchange halves the scores a lane still holds, so a score costs one
+// shuffle, and ends on the lanes that then form its weight.
+// Decoded token, 32 heads over 8 key heads, width 128, 601 visible keys 21.2 -> 6.3 us, 1028 of 1500 21.5 -> 8.0; 16 / 4 heads, values 64 wide, 600 queries 379
+// -> 205; 8 heads of 64 over 2000 keys 14.6 -> 5.0; width 256, values 192, 259 keys 23.4 -> 7.4; 5 keys 9.4 -> 5.0 us.
+template <int LPK>
+__device__ __forceinline__ void walk_rows(float& m, float& l, float (&acc)[8], const __nv_bfloat16* __restrict__ kh, const __nv_bfloat16* __restrict__ vh, const float* qs,
+                                          size_t kstride, size_t vstride, int dim, int vdim, int first, int stride, int n_keys, int n_first, int lo, int pos,
+                                          float scale, float softcap, float slope, int lane) {
+    constexpr int ROWS = 32 / LPK, G = 8 * ROWS;
+    const int sub = lane % LPK, grp = lane / LPK, ch = sub * 8;
+    float q[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) q[e] = ch < dim ? qs[ch + e] : 0.f;
+    // the exchanges leave the score of turn `mine` (key mine * ROWS + grp) on this lane, and on the LPK / 8 lanes that differ in sub's lower bits
+    constexpr int DUP = LPK / 8;
+    const int mine = sub / DUP;
+    for (int n0 = first * G; n0 < n_keys; n0 += stride * G) {
+        uint4 kw[8], vw[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            const int n = n0 + t * ROWS + grp, j = n < n_first ? n : lo + (n - n_first);
+            kw[t] = n < n_keys && ch < dim ? *reinterpret_cast<const uint4*>(kh + (size_t)j * kstride + ch) : make_uint4(0u, 0u, 0u, 0u);
+            vw[t] = n < n_keys && ch < vdim ? *reinterpret_cast<const uint4*>(vh + (size_t)j * vstride + ch) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        float s[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            const unsigned u[4] = {kw[t].x, kw[t].y, kw[t].z, kw[t].w};
+            s[t] = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                s[t] = fmaf(q[2 * e], __uint_as_float(u[e] << 16), s[t]);
+                s[t] = fmaf(q[2 * e + 1], __uint_as_float(u[e] & 0xFFFF0000u), s[t]);
+            }
+        }
+#pragma unroll
+        for (int w = 4; w > 0; w >>= 1) {          // lanes w * DUP apart: the upper one keeps the upper half of the scores
+            const bool up = (sub & (w * DUP)) != 0;
+#pragma unroll
+            for (int t = 0; t < w; t++) {
+                const float keep = up ? s[t + w] : s[t], give = up ? s[t] : s[t + w];
+                s[t] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, w * DUP);
+            }
+        }
+        float sc = s[0];
+#pragma unroll
+        for (int o = DUP / 2; o > 0; o >>= 1) sc += __shfl_xor_sync(0xFFFFFFFFu, sc, o);
+        const int n = n0 + mine * ROWS + grp;
+        const bool valid = n < n_keys;
+        sc *= scale;
+        if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
+        sc = valid ? sc - slope * (float)(pos - (n < n_first ? n : lo + (n - n_first))) : -FLT_MAX;
+        float mn = sc;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mn = fmaxf(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, o));
+        mn = fmaxf(m, mn);
+        const float corr = expf(m - mn), p = valid ? expf(sc - mn) : 0.f;
+        l = l * corr + (sub % DUP == 0 ? p : 0.f);
+        m = mn;
+#pragma unroll
+        for (int e = 0; e < 8; e++) acc[e] *= corr;
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            const float pk = __shfl_sync(0xFFFFFFFFu, p, grp * LPK + t * DUP);
+            const unsigned u[4] = {vw[t].x, vw[t].y, vw[t].z, vw[t].w};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                acc[2 * e] = fmaf(pk, __uint_as_float(u[e] << 16), acc[2 * e]);
+                acc[2 * e + 1] = fmaf(pk, __uint_as_float(u[e] & 0xFFFF0000u), acc[2 * e + 1]);
+            }
+        }
+    }
+#pragma unroll
+    for (int o = LPK; o < 32; o <<= 1)             // the lane groups' rows together
+#pragma unroll
+        for (int e = 0; e < 8; e++) acc[e] += __shfl_xor_sync(0xFFFFFFFFu, acc[e], o);
+}
+
+// Warps take groups of visible keys with a running maximum each.  LPK > 0: walk_rows above.  LPK == 0 (F32 rows, rows wider than 256, pieces off
+// 16 bytes): groups of 32, scoring is lane-per-key (each lane walks one key row against q in shared memory: no cross-lane reduction per key);
+// the group's maximum and the rescale are one warp reduction; the weighted value sum is lane-per-channel (the 32 probabilities are broadcast one
+// by one, value rows are read coalesced).
+template <typename KT, int AW_MAXV, int LPK>       // AW_MAXV: value elements per lane (vdim <= 32 * AW_MAXV; LPK > 0: 8)
 __global__ void __launch_bounds__(AW_WARPS * 32) attention_window_kernel(float* __restrict__ out, const float* __restrict__ Q, const KT* __restrict__ kc,
                                                                          const KT* __restrict__ vc, const int* __restrict__ pos_dev, int p0,
                                                                          WindowAttn a) {
@@ -108,36 +190,41 @@ __global__ void __launch_bounds__(AW_WARPS * 32) attention_window_kernel(float* 
     float m = -FLT_MAX, l = 0.f, acc[AW_MAXV];
 #pragma unroll
     for (int e = 0; e < AW_MAXV; e++) acc[e] = 0.f;
-    for (int n0 = (rank * AW_WARPS + warp) * 32; n0 < n_keys; n0 += splits * AW_WARPS * 32) {
-        const int n = n0 + lane;
-        const bool valid = n < n_keys;
-        const int j = valid ? (n < n_first ? n : lo + (n - n_first)) : 0;
-        float sc = -FLT_MAX;
-        if (valid) {
-            sc = dot_row(kc + (size_t)j * kstride + (size_t)gk * a.dim, qs, a.dim, vec) * a.scale;
-            if (a.softcap > 0.f) sc = a.softcap * tanhf(sc / a.softcap);
-            sc -= slope * (float)(pos - j);
-        }
-        float gmax = sc;
+    if constexpr (LPK > 0) {
+        walk_rows<LPK>(m, l, acc, kc + (size_t)gk * a.dim, vc + (a.joint_v ? 0 : (size_t)g * a.vdim), qs, kstride, vstride, a.dim, a.vdim, rank * AW_WARPS + warp,
+                       splits * AW_WARPS, n_keys, n_first, lo, pos, a.scale, a.softcap, slope, lane);
+    } else {
+        for (int n0 = (rank * AW_WARPS + warp) * 32; n0 < n_keys; n0 += splits * AW_WARPS * 32) {
+            const int n = n0 + lane;
+            const bool valid = n < n_keys;
+            const int j = valid ? (n < n_first ? n : lo + (n - n_first)) : 0;
+            float sc = -FLT_MAX;
+            if (valid) {
+                sc = dot_row(kc + (size_t)j * kstride + (size_t)gk * a.dim, qs, a.dim, vec) * a.scale;
+                if (a.softcap > 0.f) sc = a.softcap * tanhf(sc / a.softcap);
+                sc -= slope * (float)(pos - j);
+            }
+            float gmax = sc;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) gmax = fmaxf(gmax, __shfl_xor_sync(0xFFFFFFFFu, gmax, o));
-        const float mn = fmaxf(m, gmax);
-        const float corr = expf(m - mn), p = valid ? expf(sc - mn) : 0.f;
-        l = l * corr + p;                                   // per-lane partial sums, reduced once at the end
-        m = mn;
+            for (int o = 16; o > 0; o >>= 1) gmax = fmaxf(gmax, __shfl_xor_sync(0xFFFFFFFFu, gmax, o));
+            const float mn = fmaxf(m, gmax);
+            const float corr = expf(m - mn), p = valid ? expf(sc - mn) : 0.f;
+            l = l * corr + p;                                   // per-lane partial sums, reduced once at the end
+            m = mn;
 #pragma unroll
-        for (int e = 0; e < AW_MAXV; e++) acc[e] *= corr;
-        // all 32 slots: lanes past the last key carry p == 0 and row 0, so the trip count is fixed and the loads of several
-        // keys are in flight together
+            for (int e = 0; e < AW_MAXV; e++) acc[e] *= corr;
+            // all 32 slots: lanes past the last key carry p == 0 and row 0, so the trip count is fixed and the loads of several
+            // keys are in flight together
 #pragma unroll 8
-        for (int kk = 0; kk < 32; kk++) {
-            const float pk = __shfl_sync(0xFFFFFFFFu, p, kk);
-            const int jk = __shfl_sync(0xFFFFFFFFu, j, kk);
-            const KT* vr = vc + (size_t)jk * vstride + (a.joint_v ? 0 : (size_t)g * a.vdim);
+            for (int kk = 0; kk < 32; kk++) {
+                const float pk = __shfl_sync(0xFFFFFFFFu, p, kk);
+                const int jk = __shfl_sync(0xFFFFFFFFu, j, kk);
+                const KT* vr = vc + (size_t)jk * vstride + (a.joint_v ? 0 : (size_t)g * a.vdim);
 #pragma unroll
-            for (int e = 0; e < AW_MAXV; e++) {
-                const int i = lane + 32 * e;
-                if (i < a.vdim) acc[e] = fmaf(pk, cache_ld(vr, i), acc[e]);
+                for (int e = 0; e < AW_MAXV; e++) {
+                    const int i = lane + 32 * e;
+                    if (i < a.vdim) acc[e] = fmaf(pk, cache_ld(vr, i), acc[e]);
+                }
             }
         }
     }
@@ -145,7 +232,10 @@ __global__ void __launch_bounds__(AW_WARPS * 32) attention_window_kernel(float* 
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, o);
     if (lane == 0) { ms[warp] = m; ls[warp] = l; }
 #pragma unroll
-    for (int e = 0; e < AW_MAXV; e++) { const int i = lane + 32 * e; if (i < a.vdim) accs[warp * a.vdim + i] = acc[e]; }
+    for (int e = 0; e < AW_MAXV; e++) {
+        const int i = LPK > 0 ? lane * 8 + e : lane + 32 * e;          // LPK > 0: every lane group holds the sums, the first one's lanes write them
+        if (i < a.vdim && (LPK == 0 || lane < LPK)) accs[warp * a.vdim + i] = acc[e];
+    }
     __syncthreads();
     float M = -FLT_MAX;
     for (int w = 0; w < AW_WARPS; w++) M = fmaxf(M, ms[w]);
@@ -262,11 +352,19 @@ void attention_window(float* out, const float* Q, const void* kc, const void* vc
     cfg.attrs = at; cfg.numAttrs = 2;
     NT_CHECK(smem <= 48 * 1024, "attention_window: the head does not fit in shared memory");
     const bool wide = a.vdim > 256;          // wide value rows (a latent as the value) keep 16 numbers per lane
-    if (cache_dt == DType::F32) {
-        auto* kern = wide ? attention_window_kernel<float, 16> : attention_window_kernel<float, 8>;
+    // whole 16-byte pieces of rows no wider than 256 go to walk_rows
+    const auto in8 = [&](long long n) { return n % 8 == 0; };
+    const bool pieces = cache_dt == DType::BF16 && in8(a.dim) && in8(a.vdim) && in8(a.k_stride) && in8(a.v_stride) && std::max(a.dim, a.vdim) <= 256 &&
+                        ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0;
+    if (pieces) {
+        const int width = std::max(a.dim, a.vdim);
+        auto* kern = width <= 64 ? attention_window_kernel<__nv_bfloat16, 8, 8> : width <= 128 ? attention_window_kernel<__nv_bfloat16, 8, 16> : attention_window_kernel<__nv_bfloat16, 8, 32>;
+        NT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, out, Q, static_cast<const __nv_bfloat16*>(kc), static_cast<const __nv_bfloat16*>(vc), pos_dev, p0, a));
+    } else if (cache_dt == DType::F32) {
+        auto* kern = wide ? attention_window_kernel<float, 16, 0> : attention_window_kernel<float, 8, 0>;
         NT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, out, Q, static_cast<const float*>(kc), static_cast<const float*>(vc), pos_dev, p0, a));
     } else {
-        auto* kern = wide ? attention_window_kernel<__nv_bfloat16, 16> : attention_window_kernel<__nv_bfloat16, 8>;
+        auto* kern = wide ? attention_window_kernel<__nv_bfloat16, 16, 0> : attention_window_kernel<__nv_bfloat16, 8, 0>;
         NT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, out, Q, static_cast<const __nv_bfloat16*>(kc), static_cast<const __nv_bfloat16*>(vc), pos_dev, p0, a));
     }
     count_launch();

@@ -517,7 +517,7 @@ void Model::reduce_residual(float* partial, cudaStream_t s) {
     add_inplace(hidden_, partial, cfg_.hidden_size, s);
 }
 
-// The short launch chain needs every projection on the TMA/dp4a GEMV (its prologue carries the norm + quantiser).
+// The short launch chain needs every projection on gemv_kquant.cu (its prologue carries the norm + quantiser).
 // Collective (every rank takes the same branch): map the peers' exchange buffers once, before any graph is captured.
 void Model::ensure_xchg() {
     if (tp_size_ == 1 || xchg_tried_) return;
@@ -768,22 +768,30 @@ bool Model::short_batch_ok(int seq_len, int start_pos) const {
     return chain_ok();
 }
 
-void Model::ensure_short_buffers() {
-    if (sb_.x) return;
-    const size_t T = SHORT_CHUNK, hidden = (size_t)cfg_.hidden_size, qdim = (size_t)nh_l_ * cfg_.head_dim, kvdim = (size_t)nkv_l_ * cfg_.head_dim;
-    sb_.x = dmalloc<float>(T * hidden);
-    sb_.q = dmalloc<float>(T * qdim); sb_.k = dmalloc<float>(T * kvdim); sb_.v = dmalloc<float>(T * kvdim); sb_.attn = dmalloc<float>(T * qdim);
-    sb_.act = dmalloc<float>(T * (size_t)inter_l_);
-    sb_.xr = dmalloc<uint8_t>(gemv_rows_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_)));
-    sb_.scratch = dmalloc<float>(attention_rows_scratch_floats((int)T, cfg_.max_seq_len, nh_l_, nkv_l_, cfg_.head_dim));
-    sb_.tok = dmalloc<int>(T); sb_.pos = dmalloc<int>(T);
+// false: no room for them; the caller takes the tokens one by one, which needs none
+bool Model::ensure_short_buffers() {
+    if (sb_.x) return true;
+    const size_t T = SHORT_CHUNK, hidden = (size_t)cfg_.hidden_size, qdim = (size_t)nh_l_ * cfg_.head_dim, kvdim = (size_t)nkv_l_ * cfg_.head_dim, f = sizeof(float);
+    const size_t bytes[10] = {T * hidden * f, T * qdim * f, T * kvdim * f, T * kvdim * f, T * qdim * f, T * (size_t)inter_l_ * f,
+                              gemv_rows_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_)),
+                              attention_rows_scratch_floats((int)T, cfg_.max_seq_len, nh_l_, nkv_l_, cfg_.head_dim) * f, T * sizeof(int), T * sizeof(int)};
+    void* got[10] = {};
+    for (int i = 0; i < 10; i++)
+        if (cudaMalloc(&got[i], std::max<size_t>(bytes[i], 1)) != cudaSuccess) {
+            cudaGetLastError();
+            for (int j = 0; j < i; j++) cudaFree(got[j]);
+            return false;
+        }
+    sb_.x = static_cast<float*>(got[0]); sb_.q = static_cast<float*>(got[1]); sb_.k = static_cast<float*>(got[2]); sb_.v = static_cast<float*>(got[3]);
+    sb_.attn = static_cast<float*>(got[4]); sb_.act = static_cast<float*>(got[5]); sb_.xr = static_cast<uint8_t*>(got[6]); sb_.scratch = static_cast<float*>(got[7]);
+    sb_.tok = static_cast<int*>(got[8]); sb_.pos = static_cast<int*>(got[9]);
+    return true;
 }
 
 void Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
     cudaStream_t s = stream_;
     const int hidden = cfg_.hidden_size, hd = cfg_.head_dim, max_seq = cfg_.max_seq_len, qdim = nh_l_ * hd;
     const size_t kv_stride = (size_t)max_seq * nkv_l_ * hd;
-    ensure_short_buffers();
     auto mat = [](const Weight& w, float* y) { GemvMat m; m.W = w.ptr; m.y = y; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch; return m; };
     int T = 0;
     for (int c0 = 0; c0 < seq_len; c0 += T) {
@@ -959,7 +967,7 @@ void Model::forward_async(const int* tokens, int seq_len, int start_pos) {
     if (cfg_.layer_spec()) {
         if (prefill_min_tokens_ > 0 && seq_len >= prefill_min_tokens_ && !getenv("NT_B200_NO_BATCHED_PREFILL")) { prefill_spec(tokens, seq_len, start_pos); return; }
     } else if (batched_prefill_ok(seq_len, start_pos)) { prefill_batched(tokens, seq_len, start_pos); return; }
-    else if (short_batch_ok(seq_len, start_pos)) { prefill_short(tokens, seq_len, start_pos); return; }
+    else if (short_batch_ok(seq_len, start_pos) && ensure_short_buffers()) { prefill_short(tokens, seq_len, start_pos); return; }
     size_t w = 0;
     for (int t = 0; t < seq_len; t++) {
         int tok = tokens[t];

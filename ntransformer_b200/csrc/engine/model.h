@@ -167,7 +167,7 @@ public:
     bool short_batch_ok(int seq_len, int start_pos) const;
     bool blocks_direct(const Weight& w) const;
     void prefill_gemms(float* const* C, const void* ws, const Weight* const* w, int n, int T, bool add, cudaStream_t s);
-    void ensure_short_buffers();
+    bool ensure_short_buffers();
     void prefill_short(const int* tokens, int seq_len, int start_pos);
     struct { float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *act = nullptr, *scratch = nullptr; void* xr = nullptr;
              int *tok = nullptr, *pos = nullptr; } sb_;       // a few tokens together
@@ -289,7 +289,7 @@ private:
     void run_step_mega(bool with_head);
     void step_body(cudaStream_t s);      // embedding + all layers for the token/position in step_dev_
     void step_head(cudaStream_t s, bool from_chain = false);   // final norm + LM head (+ all-gather under TP); from_chain: norm + quantiser in the GEMV prologue
-    bool chain_ok() const;               // every projection on the TMA/dp4a GEMV: the fused launch chain applies
+    bool chain_ok() const;               // every projection on gemv_kquant.cu: the fused launch chain applies
     void run_step(bool with_head);
     void matvec(const Weight* const* ws, float* const* ys, int n, const float* x, const float* norm_w, GemvEpilogue ep,
                 cudaStream_t s);

@@ -47,7 +47,7 @@ WORKLOADS = {
     "llama3-8b-q4_k_m-prefill-4096": ("8b", "Q4_K_M", 4096, 4096),
     "llama3-70b-q4_k_m-prefill-4096": ("70b", "Q4_K_M", 4096, 4096),
 }
-DTYPE_NOTE = "k-quant codes x block-scaled int8x3 activations via dp4a (s32 exact) + f32 scales/accumulate; KV f16"
+DTYPE_NOTE = "quantised codes x block-scaled 24-bit activations via integer matrix instructions (s32 exact) + f32 scales/accumulate; KV f16"
 
 
 def shape_cfg(shape: str, max_seq: int):
@@ -406,7 +406,7 @@ def measure_decode(args, rank, world, workload, with_cpu):
             dur_ms = float(np.mean([a.elapsed_time(b) for a, b in evs]))
             kbytes = 2 * model._keep[names[0][0]][0].numel()
             ach = kbytes / (dur_ms / 1e3) / 1e9
-            roof = {"bound": "hbm", "kernel": "gemv_kq_kernel (ffn gate+up fused, SwiGLU epilogue)", "achieved": round(ach, 1),
+            roof = {"bound": "hbm", "kernel": "gemv_mma_kernel (ffn gate+up fused, SwiGLU epilogue)", "achieved": round(ach, 1),
                     "peak": peak, "unit": "GB/s", "frac": round(ach / peak, 4), "traffic": ncu_traffic(workload, world),
                     "bytes_per_launch": kbytes, "avg_launch_us": round(dur_ms * 1e3, 2), "launches_timed": len(evs),
                     "peak_source": peak_src}

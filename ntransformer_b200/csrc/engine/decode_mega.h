@@ -17,8 +17,8 @@
 //     [norm+quantise] B [gate/up GEMV, SwiGLU] B [quantise] B [down GEMV -> slots] X         (x n_layers)
 //     [norm+quantise] B [LM head GEMV]
 // B = grid barrier (one atomic arrive per CTA + spin on an L2 word), X = grid barrier + tensor-parallel exchange.
-//   * the GEMV phases are the chunk-stationary TMA/dp4a data path of gemv_kquant.cu (same gemv_kq_device.cuh inner
-//     loops, same row-group schedule, same combine order => bit-identical outputs), but the per-warp TMA rings are primed
+//   * the GEMV phases are the chunk-stationary dp4a data path (gemv_kq_device.cuh inner
+//     loops), and the per-warp TMA rings are primed
 //     for the NEXT GEMV phase before the barrier that precedes it, so HBM keeps streaming weights across barriers and
 //     through the small phases;
 //   * the residual stream is never accumulated in place: o-proj / down-proj write their partial result into "slots"

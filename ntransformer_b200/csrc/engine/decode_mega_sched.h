@@ -12,7 +12,7 @@ constexpr size_t MEGA_STATIC_SMEM = 4096;                                   // u
 constexpr size_t MEGA_DYN_SMEM = 227 * 1024 - MEGA_STATIC_SMEM;             // TMA rings; aliased by the attention scratch
 constexpr int MEGA_NTHREADS = MEGA_WARPS * 32;
 
-// Identical schedule to gemv_kq_kernel: in round r CTA b handles row-groups (r * grid + b) * gpc + [0, gpc); warp w holds
+// The schedule: in round r CTA b handles row-groups (r * grid + b) * gpc + [0, gpc); warp w holds
 // chunk (w % NC) of row-group slot (w / NC).  Flattened stage index = round * n_seg + seg.
 struct Producer {
     int issued;        // stages issued so far in the phase (uniform across the warp)

@@ -4,7 +4,7 @@
 // path's split count the two paths can be compared bit for bit:
 //   MPH_NORM_XQ  <- rmsnorm_xq_kernel      (elementwise.cu; reference K12 rmsnorm.cu:17-70)
 //   MPH_QUANT    <- quantize_x_kernel      (elementwise.cu)
-//   MPH_GEMV     <- gemv_kq_kernel         (gemv_kquant.cu; reference K2-K5 gemm.cu:96-470)
+//   MPH_GEMV     <- gemv_kq_device.cuh     (reference K2-K5 gemm.cu:96-470)
 //   MPH_ATTN     <- rope_kv_decode_kernel + decode_kernel (elementwise.cu, attention.cu; reference K14/K15/K16
 //                   rotary.cu:16-62, attention.cu:316-342, attention.cu:108-202)
 //   MPH_COMBINE  <- decode_combine_kernel  (attention.cu)

@@ -1,8 +1,7 @@
 // gemv_generic.cu — GEMV for every dtype and any (2-byte) alignment with F32 activations.
 //
 // Covers reference kernels K1 (Q4_0), K2 (Q8_0), K6 (F16), K7 (F32) — src/cuda/gemm.cu:32-152, 546-671 —
-// and is the fallback for K-quant shapes the TMA kernel (gemv_kquant.cu) cannot take (rows whose pitch is
-// not a multiple of 16 bytes).  One warp per pair of rows, lanes stride over quantisation blocks, x is
+// and is the fallback for what gemv_kquant.cu cannot take (matrices or vectors off 16 bytes, rows of no whole super-blocks).  One warp per pair of rows, lanes stride over quantisation blocks, x is
 // read through L1 (ld.global.nc); 18/34/210-byte blocks are only 2-byte aligned so codes are fetched as
 // 16-bit words.  F32 accumulate, warp-shuffle reduction.
 #include "kernels_internal.h"

@@ -1,6 +1,6 @@
-// gemv_kq_device.cuh — per-lane data path of the K-quant / Q8_0 GEMV (see gemv_kquant.cu for the design notes): stage layout
-// constants, the lane's activation registers and the dp4a inner loops for one ring stage.  Shared by the stand-alone GEMV
-// kernel (gemv_kquant.cu) and the persistent decode-step kernel (engine/decode_megakernel.cu).
+// gemv_kq_device.cuh — per-lane dp4a data path of the persistent decode-step kernel (engine/decode_megakernel.cu): stage layout
+// constants, the lane's activation registers and the inner loops for one ring stage.  A lane holds 128 elements of the vector and
+// multiplies half a super-block of each row with them.
 #pragma once
 #include "kernels_internal.h"
 #include "ring.cuh"

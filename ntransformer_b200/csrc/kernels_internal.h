@@ -13,7 +13,7 @@ namespace nt { namespace b200 {
 // ---------------------------------------------------------------------------------------------
 // Block-scaled 3-term int8 activations ("xq").  x[e] ~= scale[e/32] * (q1*16384 + q2*128 + q3)
 // with q1 in [-127,127], q2,q3 in [-64,64]: |error| <= 2^-22 of the 32-block absmax, i.e. F32-class.
-// Integer dot products against the 4/5/6/8-bit weight codes are exact (IDP.4A), the float work is
+// Integer dot products against the 4/5/6/8-bit weight codes are exact, the float work is
 // one scale per 16/32 weights instead of one convert + FMA per weight.
 //   layout for K elements (K % 128 == 0): [q1: K][q2: K][q3: K][scale: K/32 f32][sum16: K/16 f32]; inside each plane
 //   element e lives at byte e ^ (((e >> 7) & 7) << 4)  (the GEMV's bank-conflict-free shared-memory order)
@@ -34,10 +34,10 @@ enum GemvEpilogue { GEMV_STORE = 0, GEMV_ADD = 1 /* y += W.x (residual) */, GEMV
                     GEMV_PEER = 3 /* tensor parallel: rows go to every rank's slot over NVLink (PeerOut), y is not written */ };
 
 
-// Fused K-quant GEMV over up to 3 matrices sharing one activation vector (already in xq form).
-// All matrices must be Q4_K / Q5_K / Q6_K with 16-byte aligned W and row pitch.
+// Fused GEMV over up to 3 matrices sharing one activation vector.
+// All matrices must be in GGUF blocks (gemv_kq_supported / gemv_kq_any_pitch).
 // Where the shared activation vector comes from: either pre-quantised `xq`, or an F32 vector `x` that the
-// kernel quantises in its prologue (staged over the not-yet-primed part of its TMA ring), optionally as
+// kernel quantises in its prologue, optionally as
 // RMSNorm(x) * norm_w: the prologue quantises x * norm_w, sums x^2 in the same pass and the scalar
 // rsqrt(mean(x^2) + eps) is applied to the results.
 // Where a tensor-parallel GEMV (o-projection / down-projection shard) delivers its partial rows (engine/peer_xchg.h): the slot

@@ -1,7 +1,7 @@
 // prefill_dequant.cu — GGUF block formats -> F16 hi/lo pair for the tensor-core prefill GEMM (csrc/prefill_gemm.cu).
 //
 // The reference only ever dequantises inside its per-token GEMV kernels (src/cuda/gemm.cu:32-470) and, for embeddings, on
-// the CPU (src/model/transformer.cpp:394-599).  For a prompt of T tokens the batched path instead expands one weight matrix
+// the CPU (src/model/transformer.cpp:394-599).  Matrices that prefill_blocks.cu does not take (F32, F16 off 16 bytes) are expanded one
 // at a time into a scratch pair W = W_hi + W_lo (both F16, ~22 mantissa bits together, so the F32 dequantised value
 // d*sc*q - dmin*m survives) and runs two tcgen05 GEMMs over it; the expansion costs ~12 B of traffic per weight once per
 // prompt chunk, against 2*T MMAs per weight.  Element formulas follow the reference's: Q8_0 gemm.cu:96-152, Q4_0 :32-90,

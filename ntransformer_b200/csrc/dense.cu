@@ -132,73 +132,6 @@ __device__ __forceinline__ float dense_row_dot(const unsigned char* row, const f
     return warp_sum(dense_row_part<T>(row, xs, K, lane, vec));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(DV_WARPS * 32) gemv_dense_kernel(DenseMats m, const float* __restrict__ x, int K, int ep,
-                                                                   const float* __restrict__ row_scale, float alpha, int vec,
-                                                                   const float* __restrict__ norm_w, float eps, StreamsIO sio, int norm_groups) {
-    extern __shared__ __align__(16) float xs[];
-    __shared__ float red[DV_WARPS];
-    __shared__ float inv_g[DENSE_MAX_NORM_GROUPS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_launch_dependents();
-    pdl_wait();
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < K; i += DV_WARPS * 32) {
-        float v;
-        if (sio.X_in) {                   // the blend of the token's residual streams
-            v = 0.f;
-            for (int st = 0; st < sio.S; st++) { const float xv = sio.X_in[(size_t)st * K + i]; v = sio.a ? fmaf(sio.a[st], xv, v) : v + xv; }
-        } else v = x[i];
-        xs[i] = v; ss = fmaf(v, v, ss);
-    }
-    if (norm_w && norm_groups > 1) {        // every run of K / norm_groups channels has its own root mean square: a warp per run
-        __syncthreads();
-        const int per = K / norm_groups;
-        for (int g = warp; g < norm_groups; g += DV_WARPS) {
-            float s2 = 0.f;
-            for (int i = lane; i < per; i += 32) { const float v = xs[g * per + i]; s2 = fmaf(v, v, s2); }
-            s2 = warp_sum(s2);
-            if (lane == 0) inv_g[g] = 1.0f / sqrtf(s2 / (float)per + eps);
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < K; i += DV_WARPS * 32) xs[i] = xs[i] * inv_g[i / per] * norm_w[i];
-    } else if (norm_w) {
-        // RMS norm of the staged vector: every CTA sums the squares in the same order, so all CTAs (and every launch that reads the
-        // same x) derive the bit-identical normalised vector
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-        if (lane == 0) red[warp] = ss;
-        __syncthreads();
-        float tot = 0.f;
-#pragma unroll
-        for (int w = 0; w < DV_WARPS; w++) tot += red[w];
-        const float inv = 1.0f / sqrtf(tot / (float)K + eps);
-        for (int i = threadIdx.x; i < K; i += DV_WARPS * 32) xs[i] = xs[i] * inv * norm_w[i];
-    }
-    __syncthreads();
-    const bool glu = ep == DENSE_SWIGLU || ep == DENSE_GEGLU || ep == DENSE_REGLU;
-    int total = m.out[0];
-    if (!glu) for (int i = 1; i < m.n; i++) total += m.out[i];
-    for (int r = blockIdx.x * DV_WARPS + warp; r < total; r += gridDim.x * DV_WARPS) {
-        if (glu) {
-            const float g = dense_row_dot<T>(m.W[0] + (size_t)r * m.pitch[0], xs, K, lane, vec);
-            const float u = dense_row_dot<T>(m.W[1] + (size_t)r * m.pitch[1], xs, K, lane, vec);
-            if (lane == 0) m.y[0][r] = (ep == DENSE_GEGLU ? gelu_tanh_f(g) : ep == DENSE_REGLU ? fmaxf(g, 0.f) : silu_f(g)) * u;
-            continue;
-        }
-        int mi = 0, row = r;
-        while (mi + 1 < m.n && row >= m.out[mi]) { row -= m.out[mi]; mi++; }
-        const float v = dense_row_dot<T>(m.W[mi] + (size_t)row * m.pitch[mi], xs, K, lane, vec);
-        if (lane == 0 && ep == DENSE_STREAMS) streams_update(sio, m.out[0], row, v);
-        else if (lane == 0) {
-            float* y = m.y[mi] + row;
-            if (ep == DENSE_ADD) *y += v;
-            else if (ep == DENSE_SCALED_ADD) *y = fmaf(alpha * (row_scale ? row_scale[row] : 1.f), v, *y);
-            else *y = v;
-        }
-    }
-}
-
 // n floats into shared memory by the whole CTA, 16 bytes at a time when the source is aligned.  planar (n % 8 == 0): the even and the odd
 // 16-byte pieces go to the first and the second half of dst, so that lanes holding consecutive 8-number pieces of a 16-bit weight row read
 // consecutive 16-byte words of either half (no bank conflicts).
@@ -236,6 +169,165 @@ __device__ __forceinline__ float piece_dot(const uint4& w, const float* xs, int 
     }
     return acc;
 }
+// where number i of the vector stands in its staged copy; half: n / 2 for the planar form, 0 for the plain one
+__device__ __forceinline__ int staged_at(int i, int half) { return half ? ((i & 4) ? half : 0) + (i >> 3) * 4 + (i & 3) : i; }
+
+// The decode GEMV is bound by HBM: every weight is read once.  VEC (16-bit rows in whole 16-byte pieces): a warp streams a row, a lane 4 pieces at a
+// time, and fetches its next pieces (of this row or its next one) before it multiplies the current ones; the staged vector is planar.  So neither the
+// reduction at a row's end nor bank conflicts hold the loads up.  64 registers, so that four CTAs share an SM.  KW = 2 warps share a row where that
+// fills the last round (host).  Before it waits for the producer's grid a warp asks L2 for its first pieces.
+// BF16 in a graph, before -> now: 14336 + 14336 rows of 4096, gated 49.1 -> 37.7 us (6.2 TB/s), 32000 x 4096 52.4 -> 39.4 (6.7), 4096 x 4096 11.1 -> 8.3,
+// 3000 x 3000 11.1 -> 6.3; F16 4096 x 11008 24.4 -> 17.5.  More warps to a row in general (4 at 4096, 8 at 14336) was slower: 32000 x 4096 55.4.
+template <typename T, bool VEC, bool STREAMS>          // STREAMS: the epilogue may be DENSE_STREAMS (its registers are the kernel's without it)
+__global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_dense_kernel(DenseMats m, const float* __restrict__ x, int K, int ep,
+                                                                      const float* __restrict__ row_scale, float alpha, int KW, int vec,
+                                                                      const float* __restrict__ norm_w, float eps, StreamsIO sio, int norm_groups) {
+    extern __shared__ __align__(16) float xs[];
+    __shared__ float red[DV_WARPS];
+    __shared__ float inv_g[DENSE_MAX_NORM_GROUPS];
+    __shared__ float2 part_s[2][DV_WARPS];
+    constexpr int P = Elem<T>::PER16;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int half = VEC && P == 8 ? K >> 1 : 0;
+    const bool glu = ep == DENSE_SWIGLU || ep == DENSE_GEGLU || ep == DENSE_REGLU;
+    int total = m.out[0];
+    if (!glu) for (int i = 1; i < m.n; i++) total += m.out[i];
+    // VEC: this warp's place in the work: unit r (a row, or a gate row then its up row), matrix row `sub` of the unit, chunk c of the row
+    const int nv = K / P, team = warp / KW, part = warp % KW, subs = glu ? 2 : 1, chunks = (nv + 128 * KW - 1) / (128 * KW), step = gridDim.x * (DV_WARPS / KW);
+    auto place = [&](int r, int& mi) { int row = r; mi = 0; while (mi + 1 < m.n && row >= m.out[mi]) { row -= m.out[mi]; mi++; } return row; };
+    auto row_ptr = [&](int r, int sub) -> const unsigned char* {
+        if (glu) return m.W[sub] + (size_t)r * m.pitch[sub];
+        int mi; const int row = place(r, mi);
+        return m.W[mi] + (size_t)row * m.pitch[mi];
+    };
+    int r = blockIdx.x + team * gridDim.x;
+    pdl_launch_dependents();
+    if constexpr (VEC) {
+        // lanes 0..15: the lines of the first chunk; lanes 16..31: those of the one after it
+        int r1 = r, sub1 = 0, c1 = 0;
+        if (lane >= 16 && ++c1 == chunks) { c1 = 0; if (++sub1 == subs) { sub1 = 0; r1 += step; } }
+        const int v = (c1 * KW + part) * 128 + (lane & 15) * 8;
+        if (r1 < total && v < nv) asm volatile("prefetch.global.L2 [%0];" ::"l"(row_ptr(r1, sub1) + (size_t)v * 16));
+    }
+    pdl_wait();
+    float ss = 0.f;
+    if (VEC && !sio.X_in && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < K >> 2; i += DV_WARPS * 32) {
+            const float4 v = *reinterpret_cast<const float4*>(x + 4 * i);
+            *reinterpret_cast<float4*>(xs + staged_at(4 * i, half)) = v;
+            ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
+        }
+    } else
+        for (int i = threadIdx.x; i < K; i += DV_WARPS * 32) {
+            float v;
+            if (sio.X_in) {                   // the blend of the token's residual streams
+                v = 0.f;
+                for (int st = 0; st < sio.S; st++) { const float xv = sio.X_in[(size_t)st * K + i]; v = sio.a ? fmaf(sio.a[st], xv, v) : v + xv; }
+            } else v = x[i];
+            xs[staged_at(i, half)] = v; ss = fmaf(v, v, ss);
+        }
+    if (norm_w && norm_groups > 1) {        // every run of K / norm_groups channels has its own root mean square: a warp per run
+        __syncthreads();
+        const int per = K / norm_groups;
+        for (int g = warp; g < norm_groups; g += DV_WARPS) {
+            float s2 = 0.f;
+            for (int i = lane; i < per; i += 32) { const float v = xs[staged_at(g * per + i, half)]; s2 = fmaf(v, v, s2); }
+            s2 = warp_sum(s2);
+            if (lane == 0) inv_g[g] = 1.0f / sqrtf(s2 / (float)per + eps);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < K; i += DV_WARPS * 32) { float* d = xs + staged_at(i, half); *d = *d * inv_g[i / per] * norm_w[i]; }
+    } else if (norm_w) {
+        // RMS norm of the staged vector: every CTA sums the squares in the same order, so all CTAs (and every launch that reads the
+        // same x) derive the bit-identical normalised vector
+        ss = warp_sum(ss);
+        if (lane == 0) red[warp] = ss;
+        __syncthreads();
+        float tot = 0.f;
+#pragma unroll
+        for (int w = 0; w < DV_WARPS; w++) tot += red[w];
+        const float inv = 1.0f / sqrtf(tot / (float)K + eps);
+        if (VEC && (reinterpret_cast<uintptr_t>(norm_w) & 15) == 0) {
+#pragma unroll 4
+            for (int i = threadIdx.x; i < K >> 2; i += DV_WARPS * 32) {
+                const float4 g = *reinterpret_cast<const float4*>(norm_w + 4 * i);
+                float4* d = reinterpret_cast<float4*>(xs + staged_at(4 * i, half));
+                const float4 v = *d;
+                *d = make_float4(v.x * inv * g.x, v.y * inv * g.y, v.z * inv * g.z, v.w * inv * g.w);
+            }
+        } else
+            for (int i = threadIdx.x; i < K; i += DV_WARPS * 32) { float* d = xs + staged_at(i, half); *d = *d * inv * norm_w[i]; }
+    }
+    __syncthreads();
+    // one lane ends a unit: v the row's product (g the gate's), y0 the old number and f its factor where the epilogue adds
+    auto finish = [&](int r, float g, float v, float y0, float f) {
+        if (glu) { m.y[0][r] = (ep == DENSE_GEGLU ? gelu_tanh_f(g) : ep == DENSE_REGLU ? fmaxf(g, 0.f) : silu_f(g)) * v; return; }
+        int mi; const int row = place(r, mi);
+        if constexpr (STREAMS) if (ep == DENSE_STREAMS) { streams_update(sio, m.out[0], row, v); return; }
+        m.y[mi][row] = ep == DENSE_ADD ? y0 + v : ep == DENSE_SCALED_ADD ? fmaf(f, v, y0) : v;
+    };
+    auto old_of = [&](int r, float& y0, float& f) {
+        if (ep != DENSE_ADD && ep != DENSE_SCALED_ADD) return;
+        int mi; const int row = place(r, mi);
+        y0 = m.y[mi][row];
+        f = alpha * (row_scale ? row_scale[row] : 1.f);
+    };
+    if constexpr (!VEC) {
+        for (r = blockIdx.x * DV_WARPS + warp; r < total; r += gridDim.x * DV_WARPS) {
+            float g = 0.f, y0 = 0.f, f = 0.f;
+            if (glu) g = dense_row_dot<T>(row_ptr(r, 0), xs, K, lane, vec);
+            const float v = dense_row_dot<T>(row_ptr(r, glu ? 1 : 0), xs, K, lane, vec);
+            if (lane == 0) { old_of(r, y0, f); finish(r, g, v, y0, f); }
+        }
+    } else {
+        const bool ends = part == 0 && lane == 0;
+        int sub = 0, c = 0, buf = 0;
+        float acc = 0.f, gate = 0.f, y0 = 0.f, f = 0.f;
+        const unsigned char* row = nullptr;
+        auto fetch = [&](uint4 (&w)[4], int c) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int v = (c * KW + part) * 128 + lane + 32 * u;
+                w[u] = row && v < nv ? ld_stream16(row + (size_t)v * 16) : make_uint4(0u, 0u, 0u, 0u);
+            }
+        };
+        // multiply `now` (chunk c of the unit's row sub) with the loads of the chunk after it, `next`, on their way
+        auto walk = [&](uint4 (&now)[4], uint4 (&next)[4]) {
+            const int rn = r, cn = c, sn = sub;
+            float y1 = 0.f, f1 = 0.f;
+            if (++c == chunks) {
+                c = 0;
+                if (++sub == subs) { sub = 0; r += step; if (ends && r < total) old_of(r, y1, f1); }
+                row = r < total ? row_ptr(r, sub) : nullptr;
+            }
+            fetch(next, c);
+#pragma unroll
+            for (int u = 0; u < 4; u++) acc = piece_dot<T>(now[u], xs, K, min((cn * KW + part) * 128 + lane + 32 * u, nv - 1), acc);   // past the end the weights are zeros
+            if (cn + 1 < chunks) return;
+            if (sn + 1 < subs) { gate = acc; acc = 0.f; return; }
+            float v = warp_sum(acc), g = glu ? warp_sum(gate) : 0.f;
+            acc = 0.f;
+            if (KW > 1) {
+                if (lane == 0) part_s[buf][warp] = make_float2(v, g);
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(32 * KW) : "memory");
+                if (ends) { v = g = 0.f; for (int w = 0; w < KW; w++) { v += part_s[buf][warp + w].x; g += part_s[buf][warp + w].y; } }
+                buf ^= 1;          // the other copy: a warp writes this one again only behind the next barrier, which warp 0 reaches after its reads
+            }
+            if (ends) finish(rn, g, v, y0, f);
+            y0 = y1; f = f1;
+        };
+        if (r < total) { row = row_ptr(r, 0); if (ends) old_of(r, y0, f); }
+        uint4 a[4], b[4];
+        fetch(a, 0);
+        while (r < total) {
+            walk(a, b);
+            if (r >= total) break;
+            walk(b, a);
+        }
+    }
+}
+
 // batch of up to 128 pieces from v0 on, four 16-byte loads in flight per lane
 template <typename T>
 __device__ __forceinline__ float batch_dot(const unsigned char* row, const float* xs, int K, int nv, int v0, int lane, float acc) {
@@ -478,7 +570,7 @@ void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpil
     DenseMats m{};
     m.n = n_mat;
     const int per16 = dt == DType::F32 ? 4 : 8;
-    int vec = (K % per16 == 0) ? 1 : 0, total = 0;
+    int vec = (K > 0 && K % per16 == 0) ? 1 : 0, total = 0;
     for (int i = 0; i < n_mat; i++) {
         NT_CHECK(mats[i].dtype == dt, "gemv_dense: one dtype per launch");
         m.W[i] = static_cast<const unsigned char*>(mats[i].W); m.y[i] = mats[i].y; m.out[i] = mats[i].out;
@@ -490,13 +582,20 @@ void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpil
     if (total <= 0) return;
     const size_t smem = (size_t)K * sizeof(float);
     NT_CHECK(smem <= 200 * 1024, "gemv_dense: the activation vector does not fit in shared memory");
-    int grid = (total + DV_WARPS - 1) / DV_WARPS;
-    const int resident = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)(220 * 1024) / (smem + 1024))) * 148;
-    grid = std::min(grid, resident);
-#define NT_DV(TY) { static unsigned long long done = 0; if (smem > 40 * 1024) opt_in_dynamic_smem(gemv_dense_kernel<TY>, 200 * 1024, done); \
-                    launch_k(gemv_dense_kernel<TY>, dim3(grid), dim3(DV_WARPS * 32), smem, s, m, x, K, (int)ep, row_scale, alpha, vec, norm_w, eps, sio, norm_groups); }
-    if (dt == DType::F32) NT_DV(float) else if (dt == DType::F16) NT_DV(__half) else NT_DV(__nv_bfloat16)
+    // 16-bit rows in whole pieces walk with their next pieces under way; F32 rows keep the plain walk, four loads to a lane and trip (1024 x 4096: 6.7 us,
+    // 7.4 in the other form).  Two warps share a row where one to a row would leave a second round nearly empty (4096 x
+    // 14336: 23.4 us, 27.0 with one; 6144 rows of 4096: 10.9 and 11.3).
+    const bool walk = vec && dt != DType::F32;
+    const int per_sm = !walk ? 8 : ep == DENSE_STREAMS ? 2 : 4;
+    const int resident = (int)std::max<size_t>(1, std::min<size_t>((size_t)per_sm, (size_t)(220 * 1024) / (smem + (walk ? 3 : 1) * 1024))) * 148;
+    const int kw = walk && total > resident * DV_WARPS && total <= resident * DV_WARPS * 3 / 2 ? 2 : 1, rows_at_once = DV_WARPS / kw;
+    const int grid = std::min((total + rows_at_once - 1) / rows_at_once, resident);
+#define NT_DVV(TY, VEC, ST) { static unsigned long long done = 0; if (smem > 40 * 1024) opt_in_dynamic_smem(gemv_dense_kernel<TY, VEC, ST>, 200 * 1024, done); \
+                              launch_k(gemv_dense_kernel<TY, VEC, ST>, dim3(grid), dim3(DV_WARPS * 32), smem, s, m, x, K, (int)ep, row_scale, alpha, kw, vec, norm_w, eps, sio, norm_groups); }
+#define NT_DV(TY) { if (!walk) NT_DVV(TY, false, true) else if (ep == DENSE_STREAMS) NT_DVV(TY, true, true) else NT_DVV(TY, true, false) }
+    if (dt == DType::F32) NT_DVV(float, false, true) else if (dt == DType::F16) NT_DV(__half) else NT_DV(__nv_bfloat16)
 #undef NT_DV
+#undef NT_DVV
     count_launch();
 }
 
@@ -557,7 +656,7 @@ void gemv_sum(float* y, const SumTerm* terms, int n, int out, DType dt, bool add
     const size_t smem = (size_t)at * sizeof(float);
     NT_CHECK(smem <= 200 * 1024, "gemv_sum: the input vectors do not fit in shared memory");
     // warps per row: as many as keep the grid within what is resident at once (64 warps per SM)
-    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(4, (size_t)(220 * 1024) / (smem + 1024)));
+    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(3, (size_t)(220 * 1024) / (smem + 1024)));
     sd.nw = 1;
     while (sd.nw < 4 && (long)out * sd.nw * 2 <= (long)148 * per_sm * SV_WARPS) sd.nw *= 2;
     const int rows = SV_WARPS / sd.nw, grid = std::min((out + rows - 1) / rows, 148 * per_sm);

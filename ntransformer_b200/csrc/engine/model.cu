@@ -68,7 +68,7 @@ Model::~Model() {
     release_graphs();
     for (void* p : owned_) cudaFree(p);
     for (void* p : {(void*)hidden_, (void*)xnorm_, (void*)q_, (void*)k_, (void*)v_, (void*)attn_, (void*)act_, (void*)up_, (void*)part_,
-                    (void*)logits_, (void*)logits_l_, (void*)attn_scratch_, kc_, vc_, (void*)step_dev_,
+                    (void*)logits_, (void*)logits_l_, (void*)attn_scratch_, xq_, kc_, vc_, (void*)step_dev_,
                     (void*)attn_tickets_,
                     (void*)argmax_dev_, (void*)recent_dev_})
         if (p) cudaFree(p);
@@ -400,6 +400,7 @@ bool Model::finalize() {
     attn_tickets_ = dmalloc<unsigned>((size_t)std::max(1, nh_l_));
     NT_CUDA_CHECK(cudaMemset(attn_tickets_, 0, (size_t)std::max(1, nh_l_) * sizeof(unsigned)));
     if (const char* fz = getenv("NT_B200_FUSE")) fuse_mask_ = atoi(fz);
+    if (!(fuse_mask_ & 1)) xq_ = dmalloc<uint8_t>(xq_bytes(std::max(std::max(hidden, inter_l_), nh_l_ * hd)));
     const size_t kv_elems = (size_t)cfg_.n_layers * max_seq * nkv_l_ * hd;     // F16 [L, max_seq, n_kv, hd], transformer.cpp:340-346
     kc_ = dmalloc<uint16_t>(kv_elems);
     vc_ = dmalloc<uint16_t>(kv_elems);
@@ -490,7 +491,11 @@ void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float
     for (int i = 0; i < n; i++) { mats[i].W = ws[i]->ptr; mats[i].y = ys[i]; mats[i].out = ws[i]->rows; mats[i].dtype = ws[i]->dtype; mats[i].row_pitch = ws[i]->pitch; }
     GemvInput in;
     if (gemv_kq_any_pitch(mats, n, K)) {
-        in.x = x; in.norm_w = norm_w; in.eps = cfg_.norm_eps;
+        if (xq_ && gemv_kq_supported(mats, n, K)) {        // the unfused form: norm and quantiser as a launch of their own
+            if (norm_w) rmsnorm_xq(nullptr, xq_, x, norm_w, K, cfg_.norm_eps, s);
+            else quantize_x(x, xq_, K, s);
+            in.xq = xq_;
+        } else { in.x = x; in.norm_w = norm_w; in.eps = cfg_.norm_eps; }
         gemv_kq(mats, n, K, in, ep, s);
         return;
     }

@@ -131,7 +131,7 @@ struct MegaParams {
     unsigned long long timeout_ns;
     int tp_rank, tp_size;
     // Optional timeline (null = off): CTAs 0..MEGA_TRACE_CTAS-1 store the SM clock at [cta][phase][0 start, 1 work done,
-    // 2 barrier passed] followed by 4 calibration values (clock and %globaltimer at kernel start / end).  tools/mega_trace.py turns it into time per phase kind and time spent waiting in barriers.
+    // 2 barrier passed] followed by 4 calibration values (clock and %globaltimer at kernel start / end).
     unsigned long long* trace;
     int trace_stride;               // values per CTA (3 x phases of the full program + 4)
     int pad2_;

@@ -1,7 +1,7 @@
-"""GPU tensor-parallel parity (needs >= 2 GPUs, run with `gpurun --gpus 2|4|8`): the TP engine must reproduce the single-GPU
+"""GPU tensor-parallel parity (needs >= 2 GPUs): the TP engine must reproduce the single-GPU
 engine's logits (<= 1e-3 relative; only the summation grouping of the o-proj / down-proj partials differs) and its greedy
 ids, with the partial sums exchanged through NVLink peer memory (default, engine/peer_xchg.h) and through ncclAllReduce
-(NT_B200_TP_NCCL=1).  8 KV heads so that 8-way sharding (one KV head per GPU, BASELINE configs[3]) is covered."""
+(NT_B200_TP_NCCL=1).  8 KV heads so that 8-way sharding (one KV head per GPU) is covered."""
 import os
 import socket
 import subprocess

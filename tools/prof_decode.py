@@ -3,7 +3,7 @@
     python tools/prof_decode.py --model 70b --layers 8 --mix Q4_K_M [--mega 1] [--ctx 2048] [--tokens 6]
 
 --ctx N starts decoding at position N-1 (the KV cache rows below are zeros: same traffic, same instruction stream).
-Prints nothing but a one-line summary; meant to be wrapped in `ncu ... python tools/prof_decode.py ...` under gpurun."""
+Prints nothing but a one-line summary; meant to be wrapped in `ncu ... python tools/prof_decode.py ...`."""
 import argparse
 import dataclasses
 import json

@@ -14,6 +14,7 @@
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "xquant.cuh"
+#include "attention_walk.cuh"
 #include <cuda_fp16.h>
 #include <algorithm>
 #include <cfloat>
@@ -23,47 +24,19 @@ namespace nt { namespace b200 {
 
 namespace {
 
-constexpr int AW = 8;                    // warps per CTA
+constexpr int AW = WALK_WARPS;           // warps per CTA
 constexpr int MAX_SPLITS = 64;
 // Graph-replayed decode (launch shape fixed by max_seq): a context slice holds at least this many keys.  Without the floor a short
 // context is cut into one-key slices (ctx 64 over 64 slices when a rank holds a single KV head) and the merge walks them all:
 // decode_combine took 13.9 us at tensor-parallel-8 shapes and 5.4 us at one GPU (profiles/r02_launches_tp8_shard.txt).
 constexpr int DYN_MIN_SPLIT = 32;
 constexpr int FUSED_MIN_SPLIT = 64;      // decode_fused_kernel: at least this many keys per context slice (one slice = no merge step)
-constexpr int KU = 8;                    // cache rows a warp keeps in flight in the score and P.V loops
-constexpr int ATTN_MAX_DYN_SMEM = 227 * 1024 - 1024;   // static __shared__ (s_max/s_sum) counts against the 227 KB cap
-
-template <int N> struct HalfVec;         // N halfs loaded as one vector
-template <> struct HalfVec<2> { using T = uint32_t; };
-template <> struct HalfVec<4> { using T = uint2; };
-template <> struct HalfVec<8> { using T = uint4; };
-
-// Reduce GC per-lane partial sums across the warp. On return lane L holds (in v[0]) the full sum of
-// value index (L / (32 / GC)) ... valid in every lane of that group.
-template <int GC>
-__device__ __forceinline__ float transpose_reduce(float (&v)[GC], int lane) {
-    // exchange phase: halve the number of live values per step
-#pragma unroll
-    for (int n = GC, off = 16; n > 1; n >>= 1, off >>= 1) {
-        const bool upper = lane & off;
-#pragma unroll
-        for (int i = 0; i < n / 2; i++) {
-            float send = upper ? v[i] : v[i + n / 2];
-            float keep = upper ? v[i + n / 2] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, off);
-        }
-    }
-    // plain butterfly over the remaining lanes of the group
-    float r = v[0];
-#pragma unroll
-    for (int off = 16 / GC; off > 0; off >>= 1) r += __shfl_xor_sync(0xFFFFFFFFu, r, off);
-    return r;
-}
+constexpr int ATTN_MAX_DYN_SMEM = 227 * 1024 - 1024;   // static __shared__ counts against the 227 KB cap
 
 // Decode-step fusion (decode_fused_kernel): the token at cache row `pos` is not in the cache yet.  Its key arrives unrotated
 // in F32 from the q/k/v GEMV; the warp that reaches row `pos` rotates it (reference rotary.cu:16-62, pairs (i, i + hd/2)), rounds
 // key and value to F16 exactly as the cache write does (attention.cu:338-339) and — in the one CTA per KV head that owns the
-// write — stores the row.  pos < 0: plain attention over the cache, queries used as given.
+// write — stores the row.  attend_group without NEW: plain attention over the cache, queries used as given.
 struct NewToken {
     const float* k = nullptr;      // [n_kv][HD]
     const float* v = nullptr;
@@ -107,148 +80,49 @@ __device__ __forceinline__ void store_row_f16(__half* p, const __half (&h)[DPL])
     *reinterpret_cast<typename HalfVec<DPL>::T*>(p) = raw;
 }
 
-// One CTA: GC query heads of one KV head, keys [k_begin, k_end).
+// One CTA: GC query heads of one KV head, keys [k_begin, k_end) (attention_walk.cuh).
 // q_base: first of the GC heads' query vectors (contiguous [GC][hd]); out likewise.
 // If part_* != nullptr writes unnormalised partials, else the normalised output.
-// Bound by latency: a slice has few keys to a warp.  Each warp takes batches of KU consecutive keys with a running maximum of its own, so nothing waits for
-// another warp before the end, and the next batch's keys are on their way while the weights are formed, its values while the next scores are
-// (the form before it walked the slice three times, scores, softmax, values, with a barrier and a fetch in front of each: 64 heads, 8 key heads, 4000 keys
-// 12.6 + 5 us for the slices and their merge, 21 us a call).
-constexpr int P_LD = KU + 1;             // per warp: KU weights and the rescaling of what is summed so far, for each head
-template <int DPL, int GC> __host__ __device__ constexpr int attend_floats() { return AW * GC * P_LD + AW * GC * DPL * 32 + 2 * AW * GC; }
-
-template <int DPL, int GC>
+template <int DPL, int GC, bool NEW = false>
 __device__ void attend_group(float* __restrict__ out, const float* __restrict__ q_base, const __half* __restrict__ kc,
                              const __half* __restrict__ vc, int kv_head, int n_kv, int k_begin, int k_end, float scale,
                              float* __restrict__ part_o, float* __restrict__ part_ml, float* smem, const NewToken nt = NewToken{}) {
-    constexpr int HD = DPL * 32, LG = 32 / GC;           // lanes that hold a head's score
-    using Raw = typename HalfVec<DPL>::T;
+    constexpr int HD = DPL * 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* pw = smem + (size_t)warp * GC * P_LD;         // this warp's weights [KU + 1][GC]
-    float* red = smem + (size_t)AW * GC * P_LD;          // [AW][GC][HD]
-    float* ml = red + (size_t)AW * GC * HD;              // [AW][GC][2]
-    const size_t row_stride = (size_t)n_kv * HD;
-    const __half* kbase = kc + (size_t)kv_head * HD + (size_t)lane * DPL;
-    const __half* vbase = vc + (size_t)kv_head * HD + (size_t)lane * DPL;
-
-    Raw kr[KU], vr[KU];
-    auto fetch = [&](const __half* base, Raw (&r)[KU], int k0) {     // rows behind the slice are its last one: loaded, not used
-#pragma unroll
-        for (int u = 0; u < KU; u++) r[u] = __ldg(reinterpret_cast<const Raw*>(base + (size_t)min(k0 + u, k_end - 1) * row_stride));
-    };
-    auto to_float = [](const Raw& raw, float (&f)[DPL]) {
-        const __half2* h2 = reinterpret_cast<const __half2*>(&raw);
-#pragma unroll
-        for (int i = 0; i < DPL / 2; i++) { const float2 t = __half22float2(h2[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
-    };
-    int k0 = k_begin + warp * KU;
-    if (k0 < k_end) { fetch(kbase, kr, k0); fetch(vbase, vr, k0); }
-
-    float qr[GC][DPL];
-#pragma unroll
-    for (int g = 0; g < GC; g++)
-#pragma unroll
-        for (int i = 0; i < DPL; i++) qr[g][i] = q_base[(size_t)g * HD + lane * DPL + i];
+    const size_t row_stride = (size_t)n_kv * HD, channel = (size_t)kv_head * HD + (size_t)lane * DPL;
     float rc[DPL], rs[DPL];
-    if (nt.pos >= 0) {                                   // fused decode step: the queries arrive unrotated
-        rope_angles<DPL>(rc, rs, lane, nt.pos, nt.theta, nt.freq_scale);
+    walk_slice<DPL, GC, NEW>(kc + channel, vc + channel, row_stride, k_begin, k_end, nt.pos, scale, smem, warp, lane,
+        [&](float (&qr)[GC][DPL]) {
 #pragma unroll
-        for (int g = 0; g < GC; g++) rope_rotate<DPL>(qr[g], rc, rs, lane);
-    }
-    float acc[GC][DPL];
+            for (int g = 0; g < GC; g++)
 #pragma unroll
-    for (int g = 0; g < GC; g++)
+                for (int i = 0; i < DPL; i++) qr[g][i] = q_base[(size_t)g * HD + lane * DPL + i];
+            if (NEW) {                                   // fused decode step: the queries arrive unrotated
+                rope_angles<DPL>(rc, rs, lane, nt.pos, nt.theta, nt.freq_scale);
 #pragma unroll
-        for (int i = 0; i < DPL; i++) acc[g][i] = 0.f;
-    float mx = -FLT_MAX, sum = 0.f;                      // of head lane / LG
-    for (; k0 < k_end; k0 += AW * KU) {
-        float s[KU];
-#pragma unroll
-        for (int u = 0; u < KU; u++) {
-            float kf[DPL];
-            to_float(kr[u], kf);
-            if (k0 + u == nt.pos) {                      // warp-uniform: the new token's key, not in the cache yet
-#pragma unroll
-                for (int i = 0; i < DPL; i++) kf[i] = nt.k[(size_t)kv_head * HD + lane * DPL + i];
-                rope_rotate<DPL>(kf, rc, rs, lane);
-                __half kh[DPL];
-#pragma unroll
-                for (int i = 0; i < DPL; i++) { kh[i] = __float2half(kf[i]); kf[i] = __half2float(kh[i]); }
-                if (nt.kc_w) store_row_f16<DPL>(nt.kc_w + (size_t)nt.pos * row_stride + (size_t)kv_head * HD + (size_t)lane * DPL, kh);
+                for (int g = 0; g < GC; g++) rope_rotate<DPL>(qr[g], rc, rs, lane);
             }
-            float part[GC];
+        },
+        [&](float (&kf)[DPL]) {                          // the new token's key, not in the cache yet
 #pragma unroll
-            for (int g = 0; g < GC; g++) {
-                float a = 0.f;
+            for (int i = 0; i < DPL; i++) kf[i] = nt.k[(size_t)kv_head * HD + lane * DPL + i];
+            rope_rotate<DPL>(kf, rc, rs, lane);
+            __half kh[DPL];
 #pragma unroll
-                for (int i = 0; i < DPL; i++) a = fmaf(qr[g][i], kf[i], a);
-                part[g] = a;
-            }
-            const float tot = transpose_reduce<GC>(part, lane) * scale;
-            s[u] = k0 + u < k_end ? tot : -FLT_MAX;
-        }
-        if (k0 + AW * KU < k_end) fetch(kbase, kr, k0 + AW * KU);
-        float m2 = mx;
+            for (int i = 0; i < DPL; i++) { kh[i] = __float2half(kf[i]); kf[i] = __half2float(kh[i]); }
+            if (nt.kc_w) store_row_f16<DPL>(nt.kc_w + (size_t)nt.pos * row_stride + channel, kh);
+        },
+        [&](float (&vf)[DPL]) {                          // the new token's value: F16-rounded like the cache row it becomes
+            __half vh[DPL];
 #pragma unroll
-        for (int u = 0; u < KU; u++) m2 = fmaxf(m2, s[u]);
-        const float corr = expf(mx - m2);                // the first batch: 0, or 1 where no score lies above -FLT_MAX (then the sums are 0)
-        mx = m2;
-        sum *= corr;
-#pragma unroll
-        for (int u = 0; u < KU; u++) {
-            s[u] = k0 + u < k_end ? expf(s[u] - m2) : 0.f;
-            sum += s[u];
-        }
-        __syncwarp();                                    // the weights of the batch before have been read
-        if ((lane & (LG - 1)) == 0) {
-#pragma unroll
-            for (int u = 0; u < KU; u++) pw[u * GC + lane / LG] = s[u];
-            pw[KU * GC + lane / LG] = corr;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int g = 0; g < GC; g++) {
-            const float c = pw[KU * GC + g];
-#pragma unroll
-            for (int i = 0; i < DPL; i++) acc[g][i] *= c;
-        }
-#pragma unroll
-        for (int u = 0; u < KU; u++) {
-            if (k0 + u >= k_end) break;
-            float vf[DPL];
-            to_float(vr[u], vf);
-            if (k0 + u == nt.pos) {                      // the new token's value: F16-rounded like the cache row it becomes
-                __half vh[DPL];
-#pragma unroll
-                for (int i = 0; i < DPL; i++) { vh[i] = __float2half(nt.v[(size_t)kv_head * HD + lane * DPL + i]); vf[i] = __half2float(vh[i]); }
-                if (nt.vc_w) store_row_f16<DPL>(nt.vc_w + (size_t)nt.pos * row_stride + (size_t)kv_head * HD + (size_t)lane * DPL, vh);
-            }
-#pragma unroll
-            for (int g = 0; g < GC; g++) {
-                const float w = pw[u * GC + g];
-#pragma unroll
-                for (int i = 0; i < DPL; i++) acc[g][i] = fmaf(w, vf[i], acc[g][i]);
-            }
-        }
-        if (k0 + AW * KU < k_end) fetch(vbase, vr, k0 + AW * KU);
-    }
-#pragma unroll
-    for (int g = 0; g < GC; g++)
-#pragma unroll
-        for (int i = 0; i < DPL; i++) red[((size_t)warp * GC + g) * HD + lane * DPL + i] = acc[g][i];
-    if ((lane & (LG - 1)) == 0) { ml[(warp * GC + lane / LG) * 2] = mx; ml[(warp * GC + lane / LG) * 2 + 1] = sum; }
+            for (int i = 0; i < DPL; i++) { vh[i] = __float2half(nt.v[(size_t)kv_head * HD + lane * DPL + i]); vf[i] = __half2float(vh[i]); }
+            if (nt.vc_w) store_row_f16<DPL>(nt.vc_w + (size_t)nt.pos * row_stride + channel, vh);
+        });
     __syncthreads();
     for (int idx = threadIdx.x; idx < GC * HD; idx += AW * 32) {
         const int g = idx / HD, d = idx - g * HD;
-        float m = -FLT_MAX, l = 0.f, t = 0.f;
-#pragma unroll
-        for (int w = 0; w < AW; w++) m = fmaxf(m, ml[(w * GC + g) * 2]);
-#pragma unroll
-        for (int w = 0; w < AW; w++) {                   // a warp without keys has sums of 0
-            const float f = expf(ml[(w * GC + g) * 2] - m);
-            l = fmaf(ml[(w * GC + g) * 2 + 1], f, l);
-            t = fmaf(red[(size_t)w * GC * HD + idx], f, t);
-        }
+        float m, l, t;
+        walk_merge<DPL, GC>(smem, idx, m, l, t);
         if (part_o) {
             part_o[(size_t)g * HD + d] = t;             // caller strides heads by HD inside its split slot
             if (d == 0) { part_ml[2 * g] = m; part_ml[2 * g + 1] = l; }
@@ -289,7 +163,7 @@ __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) decode_kernel
     } else {
         // partials for head (head0+g) live at scratch[((head0+g) * n_splits + split) * HD]; attend_group strides
         // heads by HD, so hand it a staging area in shared memory and scatter afterwards.
-        float* stage = smem_dyn + attend_floats<DPL, GC>();   // [GC][HD] + [GC][2]
+        float* stage = smem_dyn + walk_floats<DPL, GC>();   // [GC][HD] + [GC][2]
         attend_group<DPL, GC>(nullptr, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale, stage,
                               stage + GC * HD, smem_dyn);
         __syncthreads();
@@ -402,12 +276,12 @@ __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) decode_fused_
     nt.k = k_new; nt.v = v_new; nt.pos = pos; nt.theta = theta; nt.freq_scale = freq_scale;
     if (head0 % per_kv == 0) { nt.kc_w = kc; nt.vc_w = vc; }      // one CTA per KV head stores the new row (the split that holds pos)
     if (used == 1 && !xq_out && tickets) {                 // short context: one slice per head group, normalised output, no merge
-        attend_group<DPL, GC>(out + (size_t)head0 * HD, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale, nullptr, nullptr,
+        attend_group<DPL, GC, true>(out + (size_t)head0 * HD, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale, nullptr, nullptr,
                               smem_dyn, nt);
         return;
     }
-    float* stage = smem_dyn + attend_floats<DPL, GC>();   // [GC][HD] + [GC][2]
-    attend_group<DPL, GC>(nullptr, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale, stage, stage + GC * HD,
+    float* stage = smem_dyn + walk_floats<DPL, GC>();   // [GC][HD] + [GC][2]
+    attend_group<DPL, GC, true>(nullptr, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale, stage, stage + GC * HD,
                           smem_dyn, nt);
     __syncthreads();
     float* ml_all = scratch + (size_t)n_heads * n_splits * HD;
@@ -506,7 +380,7 @@ void launch_decode(float* out, const float* q, const __half* kc, const __half* v
     }
     int split_len = (seq_len + n_splits - 1) / n_splits;
     n_splits = (seq_len + split_len - 1) / split_len;
-    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
+    const size_t smem = ((size_t)walk_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     float* scratch = nullptr;
@@ -537,7 +411,7 @@ void launch_rows(float* out, const float* q, const __half* kc, const __half* vc,
     int n_splits = rows_splits(tokens, total, groups);
     const int split_len = (total + n_splits - 1) / n_splits;
     n_splits = (total + split_len - 1) / split_len;
-    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
+    const size_t smem = ((size_t)walk_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     NT_CHECK(n_splits <= MAX_SPLITS, "attention over a run of tokens: context beyond the slices");
@@ -558,7 +432,7 @@ void launch_decode_dyn(float* out, const float* q, const __half* kc, const __hal
                        int n_heads, int n_kv, float scale, float* scratch, int n_splits, int8_t* xq_out, cudaStream_t s) {
     constexpr int HD = DPL * 32;
     const int groups = n_heads / GC;
-    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
+    const size_t smem = ((size_t)walk_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     launch_k(decode_kernel<DPL, GC>, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, kc, vc, 0, n_heads, n_kv, scale,
@@ -573,7 +447,7 @@ void launch_decode_fused(float* out, const float* q, const float* k_new, const f
                          unsigned* tickets, int8_t* xq_out, cudaStream_t s) {
     constexpr int HD = DPL * 32;
     const int groups = n_heads / GC;
-    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
+    const size_t smem = ((size_t)walk_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_fused_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     launch_k(decode_fused_kernel<DPL, GC>, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, k_new, v_new, kc, vc, pos_dev, n_heads,
@@ -589,7 +463,7 @@ void launch_decode_rope_dyn(float* out, const float* q, const float* k_new, cons
                             int8_t* xq_out, cudaStream_t s) {
     constexpr int HD = DPL * 32;
     const int groups = n_heads / GC;
-    const size_t smem = ((size_t)attend_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
+    const size_t smem = ((size_t)walk_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_fused_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     launch_k(decode_fused_kernel<DPL, GC>, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, k_new, v_new, kc, vc, pos_dev, n_heads,
@@ -601,7 +475,7 @@ void launch_decode_rope_dyn(float* out, const float* q, const float* k_new, cons
 template <int DPL, int GC>
 void launch_prefill(float* out, const float* Q, const __half* kc, const __half* vc, int seq_len, int start_pos, int n_heads,
                     int n_kv, float scale, cudaStream_t s) {
-    const size_t smem = (size_t)attend_floats<DPL, GC>() * sizeof(float);
+    const size_t smem = (size_t)walk_floats<DPL, GC>() * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(prefill_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     prefill_kernel<DPL, GC><<<dim3(n_heads / GC, seq_len), AW * 32, smem, s>>>(out, Q, kc, vc, start_pos, n_heads, n_kv, scale);

@@ -17,8 +17,8 @@
 //     [norm+quantise] B [gate/up GEMV, SwiGLU] B [quantise] B [down GEMV -> slots] X         (x n_layers)
 //     [norm+quantise] B [LM head GEMV]
 // B = grid barrier (one atomic arrive per CTA + spin on an L2 word), X = grid barrier + tensor-parallel exchange.
-//   * the GEMV phases are the chunk-stationary dp4a data path (gemv_kq_device.cuh inner
-//     loops), and the per-warp TMA rings are primed
+//   * the GEMV phases are the chunk-stationary dp4a data path of gemv_xq.cu (gemv_kq_device.cuh inner
+//     loops, the same combine order), and the per-warp TMA rings are primed
 //     for the NEXT GEMV phase before the barrier that precedes it, so HBM keeps streaming weights across barriers and
 //     through the small phases;
 //   * the residual stream is never accumulated in place: o-proj / down-proj write their partial result into "slots"
@@ -124,7 +124,7 @@ struct MegaParams {
     int8_t* xq_a;               // attention output in xq form (input of the o-projection)
     int n_splits_max;           // stride of the split dimension in attn_scratch
     int split_fixed;            // > 0: the graph path's rule (ctx cut into this many splits); 0: adaptive
-    int min_split, max_split;   // adaptive rule: keys per split; max_split also sizes the score area in shared memory
+    int min_split, max_split;   // adaptive rule: keys per split
     int attn_smem_off;          // byte offset of the attention phase's scratch inside the dynamic shared memory (0 = aliases the rings)
     int xchg_direct;            // MEGA_XCHG_DIRECT: the exchange is one remote atomic per CTA and rank instead of a master round trip
     unsigned* sync;             // MEGA_SYNC_WORDS words
@@ -181,7 +181,7 @@ bool mega_make_plan(const MegaModelView& mv, const MegaBuffers& B, int grid, int
 std::string mega_check_gemv_schedule(const MegaPhase& d, int grid, size_t ring_bytes);   // "" = the schedule is consistent
 std::string mega_check_plan(const MegaPlan& pl, int grid, int tp_size);                  // "" = structural invariants hold
 
-// Host-side GEMV phase geometry (mirrors launch_fmt/pick_warps of gemv_kquant.cu).  Pure function: unit-tested on the CPU.
+// Host-side GEMV phase geometry (mirrors launch_fmt of gemv_xq.cu).  Pure function: unit-tested on the CPU.
 struct MegaGemvGeom { int NB, NC, warps, gpc, stages, slot_bytes, mask; bool ok; };
 MegaGemvGeom mega_gemv_geom(const int* fmts, int n_mat, int K, size_t ring_bytes);
 size_t mega_ring_bytes();       // dynamic shared memory of the kernel

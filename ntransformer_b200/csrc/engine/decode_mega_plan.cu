@@ -3,6 +3,7 @@
 // Pure host functions without CUDA calls: unit-tested on the CPU (tests/test_mega_plan.py) and reused by the CPU emulation
 // harness (tests/cusim/mega_sim.cpp).
 #include "decode_mega_sched.h"
+#include "../attention_walk.cuh"
 #include <cuda_fp16.h>
 #include <algorithm>
 #include <cstring>
@@ -10,7 +11,6 @@
 namespace nt { namespace b200 {
 
 namespace {
-constexpr int AW = MEGA_ATTN_WARPS;
 int fmt_of(DType dt) {
     return dt == DType::Q4_K_M ? 0 : dt == DType::Q5_K ? 1 : dt == DType::Q6_K ? 2 : dt == DType::Q8_0 ? 3 : dt == DType::Q4_0 ? 4 : -1;
 }
@@ -19,7 +19,7 @@ int fmt_of(DType dt) {
 
 size_t mega_ring_bytes() { return MEGA_DYN_SMEM; }
 
-// Mirrors launch_fmt / pick_warps of gemv_kquant.cu with the CTA width fixed at MEGA_WARPS: the widest multiple of NC that
+// Mirrors launch_fmt of gemv_xq.cu with the CTA width fixed at MEGA_WARPS: the widest multiple of NC that
 // affords two ring stages inside `ring_bytes`, ring depth up to MEGA_MAX_STAGES.
 MegaGemvGeom mega_gemv_geom(const int* fmts, int n_mat, int K, size_t ring_bytes) {
     MegaGemvGeom g{};
@@ -76,12 +76,13 @@ bool mega_make_plan(const MegaModelView& mv, const MegaBuffers& B, int grid, int
     // ---- attention split geometry ----
     const int n_groups = mv.nh / gc;
     pl.min_split = 64;
-    // score area + cross-warp reduction + rotated queries + the token's own k/v must fit the ring area
-    const size_t fixed = ((size_t)AW * gc * mv.hd + (size_t)gc * mv.hd) * sizeof(float) + 2 * (size_t)mv.hd * sizeof(__half);
-    int max_split = (int)std::min<size_t>(2048, (MEGA_DYN_SMEM - fixed) / ((size_t)gc * sizeof(float)));
+    // the walk's shared memory (attention_walk.cuh walk_floats) + rotated queries + the token's own k/v
+    const size_t walk = (size_t)WALK_WARPS * gc * (P_LD + mv.hd + 2);
+    const size_t attn_raw = (walk + (size_t)gc * mv.hd) * sizeof(float) + 2 * (size_t)mv.hd * sizeof(__half);
+    int max_split = 2048;
     if (split_fixed > 0) {
         const int need = std::max((mv.max_seq + split_fixed - 1) / split_fixed, MEGA_COMPAT_MIN_SPLIT);
-        if (need > max_split) return fail("split_fixed: context slice does not fit shared memory");
+        if (need > max_split) return fail("split_fixed: context slice too long");
         pl.n_splits_max = split_fixed;
     } else {
         max_split = std::min(max_split, 256);
@@ -92,7 +93,7 @@ bool mega_make_plan(const MegaModelView& mv, const MegaBuffers& B, int grid, int
     pl.split_fixed = split_fixed;
     // MEGA_OVERLAP_ATTN: keep the attention scratch out of the way of the o-projection's (smaller) rings, so that those can
     // be primed at the end of the q/k/v phase and HBM keeps streaming weights through the barrier and the attention phase.
-    const size_t attn_bytes = ((fixed + (size_t)gc * max_split * sizeof(float)) + 127) & ~(size_t)127;
+    const size_t attn_bytes = (attn_raw + 127) & ~(size_t)127;
     size_t o_ring = MEGA_DYN_SMEM;
     if ((fuse & MEGA_OVERLAP_ATTN) && (fuse & MEGA_FUSE_COMBINE) && attn_bytes + 4 * RG * BS * 144 <= MEGA_DYN_SMEM) {
         pl.attn_smem_off = (int)(MEGA_DYN_SMEM - attn_bytes);
@@ -120,7 +121,7 @@ bool mega_make_plan(const MegaModelView& mv, const MegaBuffers& B, int grid, int
             mats[i].W = ws[i]->ptr; mats[i].y = ys[i]; mats[i].out = ws[i]->rows; mats[i].dtype = ws[i]->dtype; mats[i].row_pitch = ws[i]->pitch;
             fmts[i] = fmt_of(ws[i]->dtype);
         }
-        // same alignment rules as gemv_kq_supported (gemv_kquant.cu), with Q4_0 admitted unconditionally on this opt-in path
+        // same alignment rules as gemv_xq_supported (gemv_xq.cu), with Q4_0 admitted unconditionally on this opt-in path
         if (K <= 0 || K % 256 != 0 || (K / 256 + BS - 1) / BS > MEGA_WARPS) return false;
         for (int i = 0; i < n; i++) {
             if (fmts[i] < 0 || mats[i].out <= 0) return false;

@@ -4,8 +4,8 @@
 // path's split count the two paths can be compared bit for bit:
 //   MPH_NORM_XQ  <- rmsnorm_xq_kernel      (elementwise.cu; reference K12 rmsnorm.cu:17-70)
 //   MPH_QUANT    <- quantize_x_kernel      (elementwise.cu)
-//   MPH_GEMV     <- gemv_kq_device.cuh     (reference K2-K5 gemm.cu:96-470)
-//   MPH_ATTN     <- rope_kv_decode_kernel + decode_kernel (elementwise.cu, attention.cu; reference K14/K15/K16
+//   MPH_GEMV     <- gemv_xq_kernel         (gemv_xq.cu; reference K2-K5 gemm.cu:96-470)
+//   MPH_ATTN     <- rope_kv_decode_kernel + decode_kernel (elementwise.cu, attention_walk.cuh; reference K14/K15/K16
 //                   rotary.cu:16-62, attention.cu:316-342, attention.cu:108-202)
 //   MPH_COMBINE  <- decode_combine_kernel  (attention.cu)
 // Compiled with --use_fast_math like those files so the transcendental expressions lower to the same instructions.
@@ -18,6 +18,7 @@
 #include "decode_mega_sched.h"
 #include "../ring.cuh"
 #include "../xquant.cuh"
+#include "../attention_walk.cuh"
 #include <cuda_fp16.h>
 #include <cfloat>
 #include <cstring>
@@ -35,7 +36,7 @@ namespace {
 
 constexpr int NTHREADS = MEGA_NTHREADS;
 constexpr int AW = MEGA_ATTN_WARPS;
-constexpr int KU = 4;                                                        // K / V rows in flight per warp in the attention phase
+static_assert(AW == WALK_WARPS, "the attention phase is attention_walk.cuh's walk");
 
 // ---- memory-model helpers -----------------------------------------------------------------------------------------
 #ifdef NT_CUSIM   // CPU emulation (tests/cusim): C++ atomics; the acquire loads yield so that spinning threads let others run
@@ -191,7 +192,6 @@ struct Shared {
     uint64_t bars[MEGA_WARPS * MEGA_MAX_STAGES];     // one mbarrier per (warp, ring stage)
     float partial[2][MEGA_WARPS][2][RG];             // [buffer][warp][segment][row] chunk partial sums
     float red[32];
-    float s_max[8], s_sum[8];
     unsigned bcast;                                  // CTA-wide broadcast of a last-arriver ticket
 };
 static_assert(sizeof(Shared) <= MEGA_STATIC_SMEM, "static shared memory budget");
@@ -466,37 +466,6 @@ __device__ void quant_phase(const MegaPhase& d, int warp, int lane) {
 }
 
 // ---- attention ------------------------------------------------------------------------------------------------------------------
-template <int N> struct HalfVec;
-template <> struct HalfVec<2> { using T = uint32_t; };
-template <> struct HalfVec<4> { using T = uint2; };
-template <> struct HalfVec<8> { using T = uint4; };
-
-template <int DPL>
-__device__ __forceinline__ void load_row(const __half* p, float (&f)[DPL]) {
-    typename HalfVec<DPL>::T raw = *reinterpret_cast<const typename HalfVec<DPL>::T*>(p);
-    const __half2* h2 = reinterpret_cast<const __half2*>(&raw);
-#pragma unroll
-    for (int i = 0; i < DPL / 2; i++) { float2 t = __half22float2(h2[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
-}
-
-template <int GC>
-__device__ __forceinline__ float transpose_reduce(float (&v)[GC], int lane) {
-#pragma unroll
-    for (int n = GC, off = 16; n > 1; n >>= 1, off >>= 1) {
-        const bool upper = lane & off;
-#pragma unroll
-        for (int i = 0; i < n / 2; i++) {
-            float send = upper ? v[i] : v[i + n / 2];
-            float keep = upper ? v[i + n / 2] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, off);
-        }
-    }
-    float r = v[0];
-#pragma unroll
-    for (int off = 16 / GC; off > 0; off >>= 1) r += __shfl_xor_sync(0xFFFFFFFFu, r, off);
-    return r;
-}
-
 struct SplitRule { int split_len, used; };
 __device__ __forceinline__ SplitRule split_rule(const MegaParams& P, int ctx, int n_groups) {
     SplitRule r;
@@ -516,16 +485,13 @@ __device__ __forceinline__ void combine_head(const MegaParams& P, int h, int use
 // One unit: GC query heads that share KV head `kv_head`, keys [k_begin, k_end) of a context of pos + 1 tokens.
 // RoPE of the unit's queries and of the token's own key (reference rotary.cu:16-62 expression), the F16 rounding of the
 // cache write (attention.cu:316-342) and, in the unit that owns the last split, the cache write itself happen here, so
-// no grid barrier is needed between the q/k/v projection and attention.  Scores / softmax / P.V as attend_group.
+// no grid barrier is needed between the q/k/v projection and attention.  Scores, softmax and P.V: attention_walk.cuh.
 template <int DPL, int GC>
 __device__ void attend_unit(const MegaParams& P, Shared& S, const MegaPhase& d, float* smf, int head0, int kv_head, int split,
                             int k_begin, int k_end, int pos, bool write_cache, int grp, int used) {
     constexpr int HD = DPL * 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_keys = k_end - k_begin;
-    float* sc = smf;                                         // [GC][max_split]
-    float* red = sc + (size_t)GC * P.max_split;              // [AW][GC][HD]
-    float* q_s = red + (size_t)AW * GC * HD;                 // [GC][HD] rotated queries
+    float* q_s = smf + walk_floats<DPL, GC>();               // [GC][HD] rotated queries
     __half* cur_k = reinterpret_cast<__half*>(q_s + GC * HD);   // [HD] the token's own key / value, rounded like the cache
     __half* cur_v = cur_k + HD;
     const int n_kv = P.nkv;
@@ -569,110 +535,32 @@ __device__ void attend_unit(const MegaParams& P, Shared& S, const MegaPhase& d, 
     __syncthreads();
 
     const size_t row_stride = (size_t)n_kv * HD;
-    const __half* kbase = kc + (size_t)kv_head * HD + (size_t)lane * DPL;
-    const __half* vbase = vc + (size_t)kv_head * HD + (size_t)lane * DPL;
-    if (warp < AW) {
-        float qr[GC][DPL];
+    const size_t channel = (size_t)kv_head * HD + (size_t)lane * DPL;
+    if (warp < AW)
+        walk_slice<DPL, GC, true>(kc + channel, vc + channel, row_stride, k_begin, k_end, pos, P.attn_scale, smf, warp, lane,
+            [&](float (&qr)[GC][DPL]) {
 #pragma unroll
-        for (int g = 0; g < GC; g++)
+                for (int g = 0; g < GC; g++)
 #pragma unroll
-            for (int i = 0; i < DPL; i++) qr[g][i] = q_s[g * HD + lane * DPL + i];
-        // ---- phase 1: scores.  KU key rows are fetched before any of them is used: one memory round trip per KU keys ----
-        for (int p0 = warp; p0 < n_keys; p0 += AW * KU) {
-            float kf[KU][DPL];
+                    for (int i = 0; i < DPL; i++) qr[g][i] = q_s[g * HD + lane * DPL + i];
+            },
+            [&](float (&kf)[DPL]) {
 #pragma unroll
-            for (int u = 0; u < KU; u++) {
-                const int p = p0 + u * AW;
-                if (p < n_keys) {
-                    if (k_begin + p == pos) load_row<DPL>(cur_k + lane * DPL, kf[u]);
-                    else {
-                        load_row<DPL>(kbase + (size_t)(k_begin + p) * row_stride, kf[u]);
-                        // the matching V row is needed two CTA barriers from now: start pulling it from HBM into L2
-                        if ((lane & (32 / DPL - 1)) == 0) prefetch_l2(vbase + (size_t)(k_begin + p) * row_stride);
-                    }
-                }
-            }
+                for (int i = 0; i < DPL; i++) kf[i] = __half2float(cur_k[lane * DPL + i]);
+            },
+            [&](float (&vf)[DPL]) {
 #pragma unroll
-            for (int u = 0; u < KU; u++) {
-                const int p = p0 + u * AW;
-                if (p < n_keys) {                            // warp-uniform
-                    float part[GC];
-#pragma unroll
-                    for (int g = 0; g < GC; g++) {
-                        float a = 0.f;
-#pragma unroll
-                        for (int i = 0; i < DPL; i++) a = fmaf(qr[g][i], kf[u][i], a);
-                        part[g] = a;
-                    }
-                    float tot = transpose_reduce<GC>(part, lane);
-                    if ((lane & (32 / GC - 1)) == 0) sc[(size_t)(lane / (32 / GC)) * P.max_split + p] = tot * P.attn_scale;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    // ---- phase 2: per-head max / exp / sum (warp g <-> head g) ----
-    if (warp < AW) {
-        for (int g = warp; g < GC; g += AW) {
-            float* s = sc + (size_t)g * P.max_split;
-            float mx = -FLT_MAX;
-            for (int p = lane; p < n_keys; p += 32) mx = fmaxf(mx, s[p]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-            float sum = 0.f;
-            for (int p = lane; p < n_keys; p += 32) { float e = expf(s[p] - mx); s[p] = e; sum += e; }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-            if (lane == 0) { S.s_max[g] = mx; S.s_sum[g] = sum; }
-        }
-    }
-    __syncthreads();
-    // ---- phase 3: P.V (warp <-> keys, lane <-> DPL dims) ----
-    if (warp < AW) {
-        float acc[GC][DPL];
-#pragma unroll
-        for (int g = 0; g < GC; g++)
-#pragma unroll
-            for (int i = 0; i < DPL; i++) acc[g][i] = 0.f;
-        for (int p0 = warp; p0 < n_keys; p0 += AW * KU) {    // same key order per warp as the one-at-a-time loop
-            float vf[KU][DPL];
-#pragma unroll
-            for (int u = 0; u < KU; u++) {
-                const int p = p0 + u * AW;
-                if (p < n_keys) {
-                    if (k_begin + p == pos) load_row<DPL>(cur_v + lane * DPL, vf[u]);
-                    else load_row<DPL>(vbase + (size_t)(k_begin + p) * row_stride, vf[u]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < KU; u++) {
-                const int p = p0 + u * AW;
-                if (p < n_keys) {
-#pragma unroll
-                    for (int g = 0; g < GC; g++) {
-                        float w = sc[(size_t)g * P.max_split + p];
-#pragma unroll
-                        for (int i = 0; i < DPL; i++) acc[g][i] = fmaf(w, vf[u][i], acc[g][i]);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int g = 0; g < GC; g++)
-#pragma unroll
-            for (int i = 0; i < DPL; i++) red[((size_t)warp * GC + g) * HD + lane * DPL + i] = acc[g][i];
-    }
+                for (int i = 0; i < DPL; i++) vf[i] = __half2float(cur_v[lane * DPL + i]);
+            });
     __syncthreads();
     if ((d.fuse & MEGA_FUSE_COMBINE) && used == 1) {
         // The only split of its head group: nothing to merge.  Normalise and quantise straight from shared memory — the values
         // the combine would produce (o = t * e^0, l = sum * e^0), without the round trip through the scratch buffer.
         if (threadIdx.x < AW * 32) {
             for (int idx = threadIdx.x; idx < GC * HD; idx += AW * 32) {      // 32 consecutive idx = one warp, one head
-                float t = 0.f;
-#pragma unroll
-                for (int w = 0; w < AW; w++) t += red[(size_t)w * GC * HD + idx];
                 const int g = idx / HD, dd = idx - g * HD;
-                const float l = S.s_sum[g];
+                float m, l, t;
+                walk_merge<DPL, GC>(smf, idx, m, l, t);
                 const float v = t * ((l > 0.f) ? 1.0f / l : 0.f);
                 const int e = (head0 + g) * HD + dd;
                 P.attn_out[e] = v;
@@ -687,15 +575,12 @@ __device__ void attend_unit(const MegaParams& P, Shared& S, const MegaPhase& d, 
     float* ml = P.attn_scratch + (size_t)P.nh * NS * HD;
     if (threadIdx.x < AW * 32) {
         for (int idx = threadIdx.x; idx < GC * HD; idx += AW * 32) {
-            float t = 0.f;
-#pragma unroll
-            for (int w = 0; w < AW; w++) t += red[(size_t)w * GC * HD + idx];
             const int g = idx / HD, dd = idx - g * HD;
-            P.attn_scratch[((size_t)(head0 + g) * NS + split) * HD + dd] = t;
-        }
-        if (threadIdx.x < 2 * GC) {
-            const int g = threadIdx.x >> 1;
-            ml[((size_t)(head0 + g) * NS + split) * 2 + (threadIdx.x & 1)] = (threadIdx.x & 1) ? S.s_sum[g] : S.s_max[g];
+            float m, l, t;
+            walk_merge<DPL, GC>(smf, idx, m, l, t);
+            const size_t slot = (size_t)(head0 + g) * NS + split;
+            P.attn_scratch[slot * HD + dd] = t;
+            if (dd == 0) { ml[2 * slot] = m; ml[2 * slot + 1] = l; }
         }
     }
     if (d.fuse & MEGA_FUSE_COMBINE) {

@@ -490,12 +490,14 @@ void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float
     const int K = ws[0]->cols;
     for (int i = 0; i < n; i++) { mats[i].W = ws[i]->ptr; mats[i].y = ys[i]; mats[i].out = ws[i]->rows; mats[i].dtype = ws[i]->dtype; mats[i].row_pitch = ws[i]->pitch; }
     GemvInput in;
+    if (xq_ && gemv_xq_supported(mats, n, K)) {            // the unfused form: norm and quantiser as a launch of their own
+        if (norm_w) rmsnorm_xq(nullptr, xq_, x, norm_w, K, cfg_.norm_eps, s);
+        else quantize_x(x, xq_, K, s);
+        gemv_xq(mats, n, K, xq_, ep, s);
+        return;
+    }
     if (gemv_kq_any_pitch(mats, n, K)) {
-        if (xq_ && gemv_kq_supported(mats, n, K)) {        // the unfused form: norm and quantiser as a launch of their own
-            if (norm_w) rmsnorm_xq(nullptr, xq_, x, norm_w, K, cfg_.norm_eps, s);
-            else quantize_x(x, xq_, K, s);
-            in.xq = xq_;
-        } else { in.x = x; in.norm_w = norm_w; in.eps = cfg_.norm_eps; }
+        in.x = x; in.norm_w = norm_w; in.eps = cfg_.norm_eps;
         gemv_kq(mats, n, K, in, ep, s);
         return;
     }

@@ -1,4 +1,5 @@
-// gemv_kq_device.cuh — per-lane dp4a data path of the persistent decode-step kernel (engine/decode_megakernel.cu): stage layout
+// gemv_kq_device.cuh — per-lane dp4a data path of the persistent decode-step kernel (engine/decode_megakernel.cu) and of the
+// decode step's unfused form (gemv_xq.cu): stage layout
 // constants, the lane's activation registers and the inner loops for one ring stage.  A lane holds 128 elements of the vector and
 // multiplies half a super-block of each row with them.
 #pragma once

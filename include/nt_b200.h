@@ -91,6 +91,9 @@ int    nt_b200_gemv_fused(int n_mat, float* const* y, const void* const* W, cons
 int    nt_b200_gemv_fused_f32(int n_mat, float* const* y, const void* const* W, const int* out_features,
                               const int* dtypes, int in_features, const float* x, const float* norm_w, float eps,
                               int epilogue, void* stream);
+/* How nt_b200_gemv_fused* would deal out an SM's shared memory for these matrices: plan[0] warps that share a row group, plan[1] such teams in a
+ * CTA, plan[2] stages of a team's ring.  Returns 0, or < 0 where the matrix-instruction kernel does not take them.  Needs no GPU. */
+int    nt_b200_gemv_fused_plan(int n_mat, const int* out_features, const int* dtypes, int in_features, int epilogue, int* plan);
 /* The decode step's attention sub-block in ONE launch: launch_rope (src/cuda/rotary.cu:113-140; q and k are read, not
  * modified) + launch_copy_to_kv_cache at row *pos_dev (src/cuda/attention.cu:405-425) + launch_attention_decode over
  * *pos_dev + 1 keys (src/cuda/attention.cu:348-375), context split over CTAs, merged by the last CTA of each head group.

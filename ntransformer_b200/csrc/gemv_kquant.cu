@@ -17,6 +17,7 @@
 #include "xquant.cuh"
 #include "gemv_mma_device.cuh"
 #include <cuda_fp16.h>
+#include <algorithm>
 #include <cstdlib>
 
 namespace nt { namespace b200 {
@@ -337,21 +338,44 @@ bool quarter_split_enabled() {    // NT_B200_GEMV_QB_SPLIT=0: launches that mix 
     return on;
 }
 
+// How the 16 warps of an SM are dealt out: CTAs of `teams` teams of `kw` warps, a ring of `stages` stages to a team.  stages == 0: no form fits.
+struct TeamPlan { int kw, teams, stages, slot; };
+int team_slot(int mask, int kw) {         // bytes of a stage
+    int slot = 0;
+    for (int f = 0; f < 5; f++) if ((mask >> f) & 1 && MROWS * stage_pitch(f, kw) > slot) slot = MROWS * stage_pitch(f, kw);
+    return slot;
+}
+TeamPlan plan_teams(int mask, int K, int groups) {
+    const size_t fixed = SM_X + x_bytes(K);
+    auto form = [&](int kw, int teams, size_t cap) {
+        TeamPlan t{kw, teams, 0, team_slot(mask, kw)};
+        if (cap > fixed) t.stages = (int)std::min<size_t>(MAX_STAGES, (cap - fixed) / ((size_t)t.slot * teams));
+        return t;
+    };
+    // Teams of 4 share one copy of the vector and pay the meeting at the end of 16 rows half as often, four of
+    // them hide one another's barriers: the rule for every launch that gives each SM more than a group (Q4_K 57344 x 8192: 45.5 us, 58 in teams of 8, 53.4
+    // with the dp4a kernel that this one replaced).  Fewer groups than SMs: more warps finish a group sooner, 8 (Q8_0 1024 x 4096: 4.8 us, 6.2 in teams of 4;
+    // Q4_K 4096 x 4096, 256 groups: 5.1 and 4.9), for long rows 16 (Q6_K 1024 x 14336: 9.9 us, 11.0 in a team of 8, 12.2 before; Q8_0 2048 x 28672: 23.2, 29.7,
+    // 24.5); in between two teams of 8 in a CTA, since the vector does not fit twice (Q4_K 4096 x 14336: 11.4 us, 12.3 in teams of 4, 16.9 before).
+    TeamPlan t = K > 8192 ? (groups > 256 ? form(4, 4, SMEM_CTA) : groups > 148 ? form(8, 2, SMEM_CTA) : form(16, 1, SMEM_CTA))
+                          : (groups > 148 ? form(4, 4, SMEM_CTA) : form(8, 1, SMEM_HALF));
+    // Very long rows (from 41984 on, by format): the vector leaves no room for a stage of every team.  One team of 8 always has one.
+    static const int ord[3][2] = {{8, 2}, {16, 1}, {8, 1}};
+    for (int i = 0; t.stages < 1 && i < 3; i++) t = form(ord[i][0], ord[i][1], SMEM_CTA);
+    return t;
+}
+
+// format mixes with a kernel of their own
+bool one_launch(int mask) { return mask == 1 || mask == 2 || mask == 4 || mask == 8 || mask == 3 || mask == 5 || mask == 16; }
+
 template <int MASK, int KW, int TEAMS>
 void launch_teams(KqParams& p, cudaStream_t s) {
-    constexpr int fmts[5] = {MASK & 1 ? 0 : -1, MASK & 2 ? 1 : -1, MASK & 4 ? 2 : -1, MASK & 8 ? 3 : -1, MASK & 16 ? 4 : -1}, ctas = SM_WARPS / (TEAMS * KW);
-    int slot = 0;
-    for (int f : fmts) if (f >= 0 && MROWS * stage_pitch(f, KW) > slot) slot = MROWS * stage_pitch(f, KW);
-    const size_t fixed = SM_X + x_bytes(p.K), cap = ctas == 1 ? SMEM_CTA : SMEM_HALF;
-    int stages = cap > fixed ? (int)((cap - fixed) / (slot * TEAMS)) : 0;
-    if (stages > MAX_STAGES) stages = MAX_STAGES;
-    NT_CHECK(stages >= 1, "gemv_kq: shared memory budget exceeded");
-    p.stages = stages; p.slot = slot;
+    constexpr int ctas = SM_WARPS / (TEAMS * KW);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(gemv_mma_kernel<MASK, KW, TEAMS>, (int)SMEM_CTA, configured);
-    const int places = num_sms() * ctas;
-    launch_k(gemv_mma_kernel<MASK, KW, TEAMS>, dim3(p.total_groups < places ? p.total_groups : places), dim3(TEAMS * (KW + 1) * 32),
-             fixed + (size_t)stages * slot * TEAMS, s, p);
+    const size_t smem = SM_X + x_bytes(p.K) + (size_t)p.stages * p.slot * TEAMS;
+    const int places = num_sms() * (smem > SMEM_HALF ? 1 : ctas);
+    launch_k(gemv_mma_kernel<MASK, KW, TEAMS>, dim3(p.total_groups < places ? p.total_groups : places), dim3(TEAMS * (KW + 1) * 32), smem, s, p);
     count_launch();
 }
 
@@ -360,13 +384,12 @@ void launch_fmt(KqParams& p, cudaStream_t s) {
     int total = 0;
     for (int i = 0; i < p.n_mat; i++) { p.mat[i].groups = (p.mat[i].out + MROWS - 1) / MROWS; total += p.mat[i].groups; }
     p.total_groups = p.n_seg == 2 ? p.mat[0].groups : total;
-    // How the 16 warps of an SM are dealt out.  Teams of 4 share one copy of the vector and pay the meeting at the end of 16 rows half as often, four of
-    // them hide one another's barriers: the rule for every launch that gives each SM more than a group (Q4_K 57344 x 8192: 45.5 us, 58 in teams of 8, 53.4
-    // with the dp4a kernel that this one replaced).  Fewer groups than SMs: more warps finish a group sooner, 8 (Q8_0 1024 x 4096: 4.8 us, 6.2 in teams of 4;
-    // Q4_K 4096 x 4096, 256 groups: 5.1 and 4.9), for long rows 16 (Q6_K 1024 x 14336: 9.9 us, 11.0 in a team of 8, 12.2 before; Q8_0 2048 x 28672: 23.2, 29.7,
-    // 24.5); in between two teams of 8 in a CTA, since the vector does not fit twice (Q4_K 4096 x 14336: 11.4 us, 12.3 in teams of 4, 16.9 before).
-    if (p.K > 8192 ? p.total_groups > 256 : p.total_groups > 148) launch_teams<MASK, 4, 4>(p, s);
-    else if (p.K > 8192) { if (p.total_groups > 148) launch_teams<MASK, 8, 2>(p, s); else launch_teams<MASK, 16, 1>(p, s); }
+    const TeamPlan t = plan_teams(MASK, p.K, p.total_groups);
+    NT_CHECK(t.stages >= 1, "gemv_kq: shared memory budget exceeded");
+    p.stages = t.stages; p.slot = t.slot;
+    if (t.kw == 4) launch_teams<MASK, 4, 4>(p, s);
+    else if (t.kw == 16) launch_teams<MASK, 16, 1>(p, s);
+    else if (t.teams == 2) launch_teams<MASK, 8, 2>(p, s);
     else launch_teams<MASK, 8, 1>(p, s);
 }
 
@@ -392,7 +415,21 @@ bool gemv_kq_any_pitch(const GemvMat* mats, int n_mat, int K) {
         const size_t row = dtype_row_size(mats[i].dtype, K), pitch = mats[i].row_pitch ? mats[i].row_pitch : row;
         if ((reinterpret_cast<uintptr_t>(mats[i].W) & 15) || pitch < row || (pitch & (f == 2 ? 1 : 15))) return false;
     }
-    return true;
+    int plan[3];
+    return gemv_kq_plan(mats, n_mat, K, false, plan);
+}
+
+// plan: warps of a team, teams of a CTA, stages of a team's ring (the first matrix's where every matrix has a launch of its own)
+bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, int* plan) {
+    int mask = 0, groups = 0;
+    for (int i = 0; i < n_mat; i++) { mask |= 1 << fmt_of(mats[i].dtype); groups += (mats[i].out + MROWS - 1) / MROWS; }
+    if (!one_launch(mask)) {
+        for (int i = n_mat - 1; i >= 0; i--) if (!gemv_kq_plan(&mats[i], 1, K, false, plan)) return false;
+        return true;
+    }
+    const TeamPlan t = plan_teams(mask, K, swiglu ? (mats[0].out + MROWS - 1) / MROWS : groups);
+    plan[0] = t.kw; plan[1] = t.teams; plan[2] = t.stages;
+    return t.stages >= 1;
 }
 
 void gemv_kq(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpilogue ep, cudaStream_t s) {
@@ -427,7 +464,7 @@ void gemv_kq(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpi
         NT_CHECK(n_mat == 2 && mats[0].out == mats[1].out, "gemv_kq: SWIGLU needs gate and up of equal rows");
     int mask = 0;
     for (int i = 0; i < n_mat; i++) mask |= 1 << fmt_of(mats[i].dtype);
-    const bool plain = mask == 1 || mask == 2 || mask == 4 || mask == 8 || mask == 3 || mask == 5 || mask == 16;
+    const bool plain = one_launch(mask);
     if (!plain && ep != GEMV_SWIGLU) {                         // rare mixes: one launch per matrix
         for (int i = 0; i < n_mat; i++) gemv_kq(&mats[i], 1, K, in, ep, s);
         return;

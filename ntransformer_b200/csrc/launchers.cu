@@ -136,6 +136,13 @@ int nt_b200_gemv_fused_f32(int n_mat, float* const* y, const void* const* W, con
     nt::b200::gemv_kq(m, n_mat, in_features, in, (nt::b200::GemvEpilogue)epilogue, static_cast<cudaStream_t>(stream));
     return 0;
 }
+int nt_b200_gemv_fused_plan(int n_mat, const int* out_features, const int* dtypes, int in_features, int epilogue, int* plan) {
+    if (n_mat < 1 || n_mat > 3) return -1;
+    nt::b200::GemvMat m[3];
+    for (int i = 0; i < n_mat; i++) { m[i].W = nullptr; m[i].y = nullptr; m[i].out = out_features[i]; m[i].dtype = (DType)dtypes[i]; m[i].row_pitch = 0; }
+    if (!nt::b200::gemv_kq_any_pitch(m, n_mat, in_features)) return -2;
+    return nt::b200::gemv_kq_plan(m, n_mat, in_features, epilogue == 2, plan) ? 0 : -2;
+}
 size_t nt_b200_attention_decode_scratch_floats(int ms, int nh, int nkv, int hd) { return nt::b200::attention_decode_dyn_scratch_floats(ms, nh, nkv, hd); }
 int nt_b200_attention_decode_tickets(int nh, int nkv) { return nt::b200::attention_decode_fused_tickets(nh, nkv); }
 void nt_b200_attention_decode_fused(float* o, const float* q, const float* k, const float* v, void* kc, void* vc, const int* pos_dev, int ms,

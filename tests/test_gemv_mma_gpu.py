@@ -35,6 +35,29 @@ def test_rows_and_stages(dt, rows, cols):
     close(got[:rows], raw, x, rows, cols, dt)
 
 
+# Rows as long as the kernel takes: what is left of shared memory beside the vector holds one to three stages.  More and fewer than 256 row groups.
+@pytest.mark.parametrize("dt,rows,cols", [(DType.Q4_K_M, 4113, 49152), (DType.Q4_K_M, 40, 49152), (DType.Q5_K, 4113, 42240), (DType.Q5_K, 2400, 49152),
+                                          (DType.Q6_K, 4113, 48896), (DType.Q8_0, 4113, 48384), (DType.Q8_0, 33, 49152), (DType.Q4_0, 4113, 49152)], ids=str)
+def test_longest_rows(dt, rows, cols):
+    rng = np.random.default_rng(cols + rows)
+    block = random_blocks_np(dt, 64, cols, rng)                        # rows repeat: the oracle walks 64 of them
+    raw = torch.from_numpy(block).cuda().reshape(64, -1).repeat((rows + 63) // 64, 1)[:rows].contiguous()
+    x = (rng.standard_normal(cols) * np.where(rng.random(cols) < 0.02, 10, 1)).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    ref = np.resize(O.gemv(block, x, 64, cols, int(dt)), rows)
+    ys = [torch.zeros(rows, device="cuda")]
+    K.launch_gemv(ys[0], raw, xd, rows, cols, dt)
+    if dtype_row_size(dt, cols) % 16 == 0:                             # the entry over a pre-quantised vector (22 bits: four times the rounding)
+        ys.append(torch.zeros(rows, device="cuda"))
+        xq = torch.zeros(K.xq_bytes(cols), dtype=torch.uint8, device="cuda")
+        K.quantize_x(xd, xq, cols)
+        K.gemv_fused([ys[1]], [raw], [rows], [dt], cols, xq)
+    torch.cuda.synchronize()
+    scale = np.abs(x).max() * np.sqrt(cols) * 0.02
+    for y, wide in zip(ys, (1, 4)):
+        assert np.abs(y.cpu().numpy() - ref).max() <= 4e-6 * wide * scale
+
+
 @pytest.mark.parametrize("special", ["zeros", "one", "tiny", "huge"])
 def test_vectors_at_the_ends_of_the_range(special):
     rng = np.random.default_rng(3)

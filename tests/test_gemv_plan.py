@@ -1,0 +1,42 @@
+"""The rule that deals an SM's shared memory out to the matrix-instruction GEMV (csrc/gemv_kquant.cu plan_teams): every shape that the kernel accepts has at
+least one stage for each team.  Host code only."""
+import ctypes as C
+
+import pytest
+
+from ntransformer_b200._lib import lib
+from ntransformer_b200.dtypes import DType
+
+FORMATS = [(DType.Q4_K_M,), (DType.Q5_K,), (DType.Q6_K,), (DType.Q8_0,), (DType.Q4_0,)]
+MIXES = [(DType.Q4_K_M, DType.Q4_K_M, DType.Q6_K), (DType.Q4_K_M, DType.Q5_K), (DType.Q4_0, DType.Q6_K), (DType.Q5_K, DType.Q6_K, DType.Q8_0)]
+# bytes of a 16-row stage for teams of 4, 8, 16 warps (two super-blocks to a warp in teams of 4 where the blocks are small), of an odd number of units
+BLOCK = {DType.Q4_K_M: 144, DType.Q5_K: 176, DType.Q6_K: 210, DType.Q8_0: 272, DType.Q4_0: 144}
+
+
+def stage(dt, kw):
+    blocks = 2 * kw if kw == 4 and dt not in (DType.Q6_K, DType.Q8_0) else kw
+    return 16 * ((((blocks * BLOCK[dt] + 15) // 16 + (dt == DType.Q6_K)) | 1) * 16)
+
+
+def plan(dts, rows, cols, epilogue=0):
+    n, out = len(dts), (C.c_int * 3)()
+    rc = lib().nt_b200_gemv_fused_plan(n, (C.c_int * n)(*[rows] * n), (C.c_int * n)(*map(int, dts)), cols, epilogue, out)
+    return rc, tuple(out)
+
+
+@pytest.mark.parametrize("dts", FORMATS + MIXES, ids=lambda d: "+".join(x.name for x in d))
+def test_every_accepted_shape_has_a_stage(dts):
+    one = dts if set(dts) != {DType.Q5_K, DType.Q6_K, DType.Q8_0} and set(dts) != {DType.Q4_0, DType.Q6_K} else dts[:1]      # mixes without a kernel: one launch each
+    for cols in range(256, 49152 + 1, 256):
+        for rows in (1, 16, 148 * 16, 148 * 16 + 1, 256 * 16, 256 * 16 + 1, 128256):
+            for epilogue in (0, 2) if len(dts) == 2 else (0,):
+                rc, (kw, teams, stages) = plan(dts, rows, cols, epilogue)
+                assert rc == 0 and (kw, teams) in ((4, 4), (8, 2), (16, 1), (8, 1)) and 1 <= stages <= 8, (dts, cols, rows)
+                # digit planes, scales and sums of the vector, and the rings, in the 227 KB of a CTA
+                assert 3 * (cols + 64) + cols // 4 + teams * stages * max(stage(d, kw) for d in one) <= 227 * 1024 - 4000, (dts, cols, rows)
+
+
+def test_longer_rows_are_refused():
+    assert plan((DType.Q4_K_M,), 4096, 49152 + 256)[0] == -2
+    assert plan((DType.Q4_K_M,), 4096, 128)[0] == -2
+    assert plan((DType.F16,), 4096, 4096)[0] == -2

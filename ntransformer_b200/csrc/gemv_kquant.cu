@@ -62,19 +62,18 @@ __host__ __device__ constexpr size_t x_bytes(int K) { return ((size_t)3 * (K + 6
 __device__ __forceinline__ void quantize8(const float (&x)[8], int t8, uint8_t* planes, int plane, float* xs, float* sums) {
     float amax = 0.f, s = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; i++) { amax = fmaxf(amax, fabsf(x[i])); s = __fadd_rn(s, x[i]); }
-    amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+    for (int i = 0; i < 8; i++) { amax = max_abs(amax, x[i]); s = __fadd_rn(s, x[i]); }
+    amax = max_abs(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+    amax = max_abs(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
     s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 1));
     s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 2));
-    constexpr float TOP = 127.0f * 65536.0f;
-    const float inv = (amax > 0.f) ? __fdiv_rn(TOP, amax) : 0.f;
+    const BlockScale scale(amax);
     uint32_t d[3][2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         int T[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) T[i] = __float2int_rn(__fmul_rn(x[4 * h + i], inv));
+        for (int i = 0; i < 4; i++) T[i] = scale(x[4 * h + i]);
         digits4(T, d[0][h], d[1][h], d[2][h]);
     }
     const uint32_t o = xword_byte(t8 * 8);                      // the two words are neighbours in t: 16 bytes apart
@@ -85,7 +84,7 @@ __device__ __forceinline__ void quantize8(const float (&x)[8], int t8, uint8_t* 
     }
     if ((t8 & 3) == 0) {
         const int b = t8 >> 2;                                  // 32-element block: 2 c + hi of its super-block
-        xs[(b & ~7) + (b & 1) * 4 + ((b & 7) >> 1)] = __fdiv_rn(amax, TOP);
+        xs[(b & ~7) + (b & 1) * 4 + ((b & 7) >> 1)] = scale.xs;
         sums[b] = s;
     }
 }

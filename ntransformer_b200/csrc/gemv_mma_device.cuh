@@ -53,6 +53,31 @@ __device__ __forceinline__ void wait_phase(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ void arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
 template <int N> __device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 
+// The largest magnitude, a NaN where there is one (its bits lie above infinity's; fmaxf would drop it)
+__device__ __forceinline__ float max_abs(float a, float b) {
+    const uint32_t u = __float_as_uint(a) & 0x7FFFFFFFu, v = __float_as_uint(b) & 0x7FFFFFFFu;
+    return __uint_as_float(u > v ? u : v);
+}
+// Scale and integers of a 32-block of activations whose largest magnitude is amax: x = xs * T.
+//   * below 2^-126 * 127 * 65536 (1e-31) the scale would be denormal and is flushed to 0, and its reciprocal overflows: 2^-126 then, and smaller integers;
+//   * a NaN is carried by the scale, so every row's product is one;
+//   * infinities are +-65537 beside zeros and the scale is infinite: both digits that a lane may hold (q1, q3) then multiply it by the same sum of codes, and
+//     the product is an infinity of the sum's sign, or NaN where the weight is 0.  (Q4_K and Q5_K subtract their offsets' infinity from it: NaN.)
+struct BlockScale {
+    float inv, xs;
+    bool infinite;
+    __device__ __forceinline__ explicit BlockScale(float amax) {
+        constexpr float TOP = 127.0f * 65536.0f, LEAST = TOP * 1.17549435e-38f;
+        inv = amax < LEAST ? 8.50705917e37f : __fdiv_rn(TOP, amax);
+        xs = amax < LEAST ? 1.17549435e-38f : __fdiv_rn(amax, TOP);
+        infinite = __float_as_uint(amax) == 0x7F800000u;
+    }
+    __device__ __forceinline__ int operator()(float x) const {
+        if (infinite) return (__float_as_uint(x) << 1) == 0xFF000000u ? (x > 0.f ? 65537 : -65537) : 0;
+        return __float2int_rn(__fmul_rn(x, inv));
+    }
+};
+
 // Balanced base-256 digits of four integers, |T| <= 127 * 65536: with 128 added to each digit they are the bytes of one sum.
 __device__ __forceinline__ void digits4(const int (&T)[4], uint32_t& q1, uint32_t& q2, uint32_t& q3) {
     uint32_t u[4];
@@ -260,7 +285,7 @@ __device__ __forceinline__ void tile_blocks(const uint8_t* sb, int mis, int sbi,
                     }
 #pragma unroll
                     for (int r = 0; r < 2; r++)
-                        acc[r] = fmaf(sum_of(s[2 * r], s[2 * r + 1]), half_bits(*reinterpret_cast<const uint16_t*>(p + B * (t >> 1) + r * 8 * PITCH)) * (c ? x2.y : x2.x), acc[r]);
+                        acc[r] = fmaf(sum_of(s[2 * r], s[2 * r + 1]) * (c ? x2.y : x2.x), half_bits(*reinterpret_cast<const uint16_t*>(p + B * (t >> 1) + r * 8 * PITCH)), acc[r]);
                 }
             }
         }

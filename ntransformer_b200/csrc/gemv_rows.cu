@@ -59,12 +59,12 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(uint8_t* __restrict_
             for (int i = 0; i < 8; i++) v[i] = __fmul_rn(v[i], __ldg(norm_w + 8 * t8 + i));
         float amax = 0.f, s = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; i++) { amax = fmaxf(amax, fabsf(v[i])); s = __fadd_rn(s, v[i]); }
-        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+        for (int i = 0; i < 8; i++) { amax = max_abs(amax, v[i]); s = __fadd_rn(s, v[i]); }
+        amax = max_abs(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+        amax = max_abs(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
         s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 1));
         s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 2));
-        const float inv = (amax > 0.f && live) ? __fdiv_rn(127.0f * 65536.0f, amax) : 0.f;
+        const BlockScale scale(live ? amax : 0.f);
         const int e = 8 * t8, sub = (e >> 5) & 7, seg = (e >> 4) & 1, t = (e >> 2) & 3, odd = sub & 1;
         uint8_t* blk = xr + ((size_t)pass * NB + (e >> 8)) * XB;
         uint8_t* pair = blk + (sub >> 1) * 1536;
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(uint8_t* __restrict_
         for (int h = 0; h < 2; h++) {
             int T[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) T[i] = __float2int_rn(__fmul_rn(v[4 * h + i], inv));
+            for (int i = 0; i < 4; i++) T[i] = live ? scale(v[4 * h + i]) : 0;
             uint32_t q1, q2, q3;
             digits4(T, q1, q2, q3);
             const int c = 2 * (tk & 3), w12 = ((tk >> 2) * 2 + seg) * 4, u12 = odd ? 1024 : 0;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(uint8_t* __restrict_
         }
         if ((t8 & 3) == 0) {
             float* f = reinterpret_cast<float*>(blk + XB_DIGITS);
-            f[tk * 8 + sub] = live ? __fmul_rn(__fdiv_rn(amax, 127.0f * 65536.0f), rms) : 0.f;
+            f[tk * 8 + sub] = live ? __fmul_rn(scale.xs, rms) : 0.f;
             f[64 + tk * 8 + sub] = live ? __fmul_rn(s, rms) : 0.f;
         }
     }
@@ -105,8 +105,8 @@ __device__ __forceinline__ void take(const int (&s12)[2][4], const int (&s3)[4],
     for (int r = 0; r < 2; r++)
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            a12[j][r] = fmaf(sum_of(s12[j][2 * r], s12[j][2 * r + 1]), sc[r] * x12[j], a12[j][r]);
-            a3[j][r] = fmaf((float)s3[2 * r + j], sc[r] * x3[j], a3[j][r]);
+            a12[j][r] = fmaf(sum_of(s12[j][2 * r], s12[j][2 * r + 1]) * x12[j], sc[r], a12[j][r]);
+            a3[j][r] = fmaf((float)s3[2 * r + j] * x3[j], sc[r], a3[j][r]);
         }
 }
 

@@ -6,12 +6,13 @@
 
 namespace nt { namespace b200 {
 
-// Quantises the 32 values held one per lane. Returns the three int8 terms of this lane; *scale_out is
+// Quantises the 32 values held one per lane (a NaN among them makes the scale one). Returns the three int8 terms of this lane; *scale_out is
 // absmax/127/16384 (valid in all lanes), *sum16_out the exact F32 sum of this lane's 16-element half.
 __device__ __forceinline__ void quantize_lane32(float v, int& q1, int& q2, int& q3, float& scale_out, float& sum16_out) {
-    float amax = fabsf(v);
+    uint32_t top = __float_as_uint(v) & 0x7FFFFFFFu;         // magnitudes as integers: a NaN is the largest
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+    for (int o = 16; o > 0; o >>= 1) { const uint32_t u = __shfl_xor_sync(0xFFFFFFFFu, top, o); top = u > top ? u : top; }
+    const float amax = __uint_as_float(top);
     const float s = __fdiv_rn(amax, 127.0f);
     const float t = (amax > 0.f) ? __fdiv_rn(v, s) : 0.f;
     const float f1 = rintf(t);

@@ -78,6 +78,57 @@ def test_vectors_at_the_ends_of_the_range(special):
     close(y.cpu().numpy(), raw, x, rows, cols, DType.Q4_K_M)
 
 
+# Rows of 3 super-blocks: in Q6_K they start at any even address, and were multiplied by the vector in F32 before there was this kernel (as Q4_0's)
+@pytest.mark.parametrize("dt", FORMATS, ids=lambda d: d.name)
+def test_nan_infinity_and_the_smallest_numbers(dt):
+    rows, cols = 70, 768
+    rng = np.random.default_rng(11)
+    raw = random_blocks_np(dt, rows, cols, rng)
+    W = np.stack([O.gemv(raw, e, rows, cols, int(dt)) for e in np.eye(cols, dtype=np.float32)], 1).astype(np.float64)
+
+    def run(x):
+        y = torch.zeros(rows, device="cuda")
+        K.launch_gemv(y, torch.from_numpy(raw).cuda(), torch.from_numpy(x).cuda(), rows, cols, dt)
+        torch.cuda.synchronize()
+        return y.cpu().numpy().astype(np.float64)
+
+    x = rng.standard_normal(cols).astype(np.float32)
+    for at in (0, 37, 750):
+        nan = x.copy()
+        nan[at] = np.nan
+        assert np.isnan(run(nan)).all()
+        for v in (np.inf, -np.inf):
+            inf = x.copy()
+            inf[at] = v
+            got = run(inf)
+            if dt in (DType.Q4_K_M, DType.Q5_K):          # the offset's infinity is taken off the codes': not a number
+                assert not np.isfinite(got).any()
+            else:                                          # as in 64 bits: the infinity of the weight's sign, not a number where the weight is 0
+                with np.errstate(invalid="ignore"):
+                    ref = W[:, at] * v
+                assert ((got == ref) | (np.isnan(got) & np.isnan(ref))).all()
+    # numbers whose scale would be denormal: integers of 2^-126, so an element is off by 2^-127 at most; and a lane's share of a super-block below 2^-126 is
+    # flushed before it counts 256
+    for size in (3e-32, 1e-32, 1e-33):
+        t = (x * np.float32(size)).astype(np.float32)
+        bound = 2.0 ** -126 * (np.abs(W).sum(1) + 256 * 4 * cols / 256) + 4e-6 * np.abs(W) @ np.abs(t).astype(np.float64)
+        assert (np.abs(run(t) - W @ t.astype(np.float64)) <= bound).all()
+
+
+def test_nan_in_a_vector_that_is_quantised_by_a_launch_of_its_own():
+    rng = np.random.default_rng(12)
+    rows, cols = 40, 1024
+    x = rng.standard_normal(cols).astype(np.float32)
+    x[500] = np.nan
+    for dt in FORMATS:
+        raw, y = random_blocks_np(dt, rows, cols, rng), torch.zeros(rows, device="cuda")
+        xq = torch.zeros(K.xq_bytes(cols), dtype=torch.uint8, device="cuda")
+        K.quantize_x(torch.from_numpy(x).cuda(), xq, cols)
+        K.gemv_fused([y], [torch.from_numpy(raw).cuda()], [rows], [dt], cols, xq)
+        torch.cuda.synchronize()
+        assert torch.isnan(y).all()
+
+
 def test_vector_that_is_not_16_byte_aligned_takes_the_general_path():
     rng = np.random.default_rng(4)
     rows, cols = 40, 512

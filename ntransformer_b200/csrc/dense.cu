@@ -303,7 +303,11 @@ __global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_d
             }
             fetch(next, c);
 #pragma unroll
-            for (int u = 0; u < 4; u++) acc = piece_dot<T>(now[u], xs, K, min((cn * KW + part) * 128 + lane + 32 * u, nv - 1), acc);   // past the end the weights are zeros
+            for (int u = 0; u < 4; u++) {
+                const int v = (cn * KW + part) * 128 + lane + 32 * u;
+                const float sum = piece_dot<T>(now[u], xs, K, min(v, nv - 1), acc);
+                acc = v < nv ? sum : acc;              // past the end: zeros times any piece, which may be infinite
+            }
             if (cn + 1 < chunks) return;
             if (sn + 1 < subs) { gate = acc; acc = 0.f; return; }
             float v = warp_sum(acc), g = glu ? warp_sum(gate) : 0.f;

@@ -131,6 +131,11 @@ void   nt_b200_rmsnorm_split(void* workspace, const float* x, const float* w, in
  * Reference dequant formulas: src/cuda/gemm.cu:32-470, src/model/transformer.cpp:394-599. */
 void   nt_b200_dequant_split(void* w_hi, void* w_lo, const void* W, int dtype, size_t row_pitch, int rows, int cols,
                              void* stream);
+/* Kernels that wait for copies or products of their own do so with a limit.  A wait that ran out sets a word (its launch's results are not to be used);
+ * nt_model_sync answers cudaErrorLaunchTimeout for it, nt_model_forward and its like end with that error.  Returns the word, 0 = none; set >= 0 also
+ * stores `set`.  nt_b200_wait_probe launches a wait of limit_ns for something that does not come (came_dev: device int, 0 afterwards). */
+int    nt_b200_wait_status(int set);
+void   nt_b200_wait_probe(unsigned limit_ns, int* came_dev, void* stream);
 unsigned long long nt_b200_launch_count(void);   /* kernels launched by this library so far */
 int    nt_b200_stream_sync(void* stream);        /* cudaStreamSynchronize; returns cudaError_t */
 const char* nt_b200_version(void);

@@ -1009,6 +1009,10 @@ int Model::sync() {
     if (mega_) mega_->enqueue_abort_read(stream_);
     if (xchg_) xchg_->enqueue_abort_read(stream_);
     const cudaError_t e = cudaStreamSynchronize(stream_);
+    if (e == cudaSuccess && wait_expired()) {
+        fprintf(stderr, "Error: a kernel's wait for its own copies or products ran out; the results are not usable\n");
+        return (int)cudaErrorLaunchTimeout;
+    }
     if (e == cudaSuccess && mega_) mega_->check_abort();
     if (e == cudaSuccess && xchg_) NT_CHECK(!xchg_->aborted(), "tensor-parallel peer exchange timed out (a rank never published its partial rows)");
     return (int)e;

@@ -50,6 +50,7 @@ struct KqParams {
     int n_seg;                 // segments (matrices) per group: 2 for SWIGLU else 1
     int epilogue;
     int stages, slot;          // depth of a team's ring and bytes of a stage
+    unsigned* status;          // wait_status.cuh
     PeerOut peer;              // epilogue GEMV_PEER
 };
 
@@ -134,7 +135,10 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
                     if (e16 > end) e16 -= 16;
                     const uint32_t bytes = lane < MROWS && row < m.out ? (uint32_t)(e16 - b16) : 0u;
                     const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, bytes);
-                    if (!ahead) wait_phase(empty + slot, parity);
+                    if (!ahead && !wait_warp(empty + slot, parity, p.status)) {
+                        for (int s = 0; s < stages; s++) wait_phase(full + s, s < slot ? parity ^ 1u : parity, p.status);      // the copies in flight
+                        return;
+                    }
                     uint8_t* dst = ring + (size_t)slot * slot_bytes + lane * stage_pitch(fmt, KW);
                     if (bytes && e16 < e)
                         for (const uint8_t* q = e16; q < e; q += 2) *reinterpret_cast<uint16_t*>(dst + (q - b16)) = *reinterpret_cast<const uint16_t*>(q);
@@ -234,6 +238,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
     float* part = reinterpret_cast<float*>(smem + SM_PART) + team * 2 * 2 * KW * MROWS;      // [buffer][segment][K share][row]
     int slot = 0, buf = 0, turn = 0;
     uint32_t parity = 0;
+    bool sound = true;                                          // no wait of this warp has run out
     for (int u = u0; u < p.total_groups; u += ustep) {
         for (int seg = 0; seg < p.n_seg; seg++) {
             int mi, gl;
@@ -243,8 +248,8 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
             float acc[2] = {}, mins[2] = {};
             for (int b0 = 0; b0 < p.NB; b0 += sblocks) {
                 const int sbi = b0 + warp, left = p.NB - sbi;   // super-blocks from this warp's first on
-                wait_phase(full + slot, parity);
-                if (left > 0) {
+                if (sound) sound = wait_warp(full + slot, parity, p.status);
+                if (left > 0 && sound) {
                     const uint8_t* sb = ring + (size_t)slot * slot_bytes + warp * blk;
                     const bool two = KW == 4 && left > KW;
                     if ((MASK & 1) && fmt == 0) { if (two) tile_blocks<0, 2, KW>(sb, 0, sbi, xv, lane, acc, mins); else tile_blocks<0, 1, KW>(sb, 0, sbi, xv, lane, acc, mins); }
@@ -255,7 +260,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
                     if ((MASK & 16) && fmt == 4) { if (two) tile_blocks<4, 2, KW>(sb, 0, sbi, xv, lane, acc, mins); else tile_blocks<4, 1, KW>(sb, 0, sbi, xv, lane, acc, mins); }
                 }
                 __syncwarp();
-                if (lane == 0) arrive(empty + slot);
+                if (lane == 0 && sound) arrive(empty + slot);
                 if (++slot == stages) { slot = 0; parity ^= 1u; }
             }
             const float f = lane_factor(fmt, t);
@@ -264,7 +269,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
             float v = (t & 1) ? v1 : v0;
             v += __shfl_xor_sync(0xFFFFFFFFu, (t & 1) ? v0 : v1, 1);
             v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
-            if (t < 2) part[((buf * 2 + seg) * KW + warp) * MROWS + g + 8 * t] = v;
+            if (t < 2) part[((buf * 2 + seg) * KW + warp) * MROWS + g + 8 * t] = sound ? v : __uint_as_float(0x7FFFFFFFu);      // NaN
         }
         named_sync<KW * 32>(2 + team);
         if (warp == turn && lane < MROWS) {                     // one warp in turn adds the shares and applies the epilogue
@@ -485,6 +490,7 @@ void gemv_kq(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpi
         m.row_pitch = (long long)(mats[i].row_pitch ? mats[i].row_pitch : dtype_row_size(mats[i].dtype, K));
     }
     p.n_seg = ep == GEMV_SWIGLU ? 2 : 1;
+    p.status = wait_status();
     switch (mask) {
         case 1: launch_fmt<1>(p, s); break;
         case 2: launch_fmt<2>(p, s); break;

@@ -10,6 +10,7 @@
 #pragma once
 #include "kernels_internal.h"
 #include "ring.cuh"
+#include "wait_status.cuh"
 #include <cuda_fp16.h>
 
 namespace nt { namespace b200 {
@@ -38,18 +39,6 @@ __device__ __forceinline__ uint32_t xword_byte(int e) {
     return (uint32_t)((((e >> 7) * 8 + ((e >> 5) & 1) * 4 + ((e >> 2) & 3)) << 4) + ((((e >> 6) & 1) * 2 + ((e >> 4) & 1)) << 2));
 }
 
-__device__ unsigned wait_expired;      // a wait below gave up: the launch's results are wrong
-
-// Waits for the phase of a copy or of a reader in this CTA, both under way: microseconds.  A limit far above that keeps a broken launch from
-// hanging the GPU.
-__device__ __forceinline__ void wait_phase(uint64_t* bar, uint32_t parity) {
-    uint32_t done = 0;
-    for (uint32_t spin = 0; !done; spin++) {
-        if (spin == (1u << 24)) { wait_expired = 1u; return; }
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    }
-}
 __device__ __forceinline__ void arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
 template <int N> __device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 

@@ -26,6 +26,7 @@ struct RowsParams {
     RowsMat mat[3];
     int n_mat, NB, passes, tokens, total_units, n_seg, epilogue, stages, slot;
     const uint8_t* xr;         // [pass][super-block][XB]
+    unsigned* status;          // wait_status.cuh
 };
 
 // One block: the token blockIdx.x (zeros beyond the last).  x: F32 rows of K, norm_w: RMSNorm's gains or null.
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
     pdl_launch_dependents();
     const int wslot = p.slot - RKW * XB;                           // bytes of the weights in a slot
     if (warp == RWARPS) {                                          // ---- producer: a lane for each row ----
-        int slot = 0;
+        int slot = 0, filled = 0;
         uint32_t parity = 1;
         for (int u = blockIdx.x; u < p.total_units; u += gridDim.x) {
             for (int seg = 0; seg < p.n_seg; seg++) {
@@ -297,7 +298,11 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
                     if (e16 > end) e16 -= 16;                      // what lies behind the matrix is not read: its last bytes go singly
                     const uint32_t bytes = row < m.out ? (uint32_t)(e16 - b16) : 0u;
                     const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, bytes) + (uint32_t)(nb * XB);
-                    wait_phase(empty + slot, parity);
+                    if (!wait_warp(empty + slot, parity, p.status)) {
+                        for (int s = 0; s < min(filled, p.stages); s++) wait_phase(full + s, s < slot ? parity ^ 1u : parity, p.status);      // the copies in flight
+                        return;
+                    }
+                    filled = min(filled + 1, p.stages);
                     uint8_t* st = ring + (size_t)slot * p.slot;
                     uint8_t* dst = st + lane * stage_pitch(fmt, RKW);
                     if (bytes && e16 < e)
@@ -317,6 +322,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
     float* part = reinterpret_cast<float*>(smem + R_PART) + tile * RKW * 128;       // + segment * RTILES * RKW * 128
     int slot = 0, turn = 0;
     uint32_t parity = 0;
+    bool sound = true;                                             // no wait of this warp has run out
     for (int u = blockIdx.x; u < p.total_units; u += gridDim.x) {
         for (int seg = 0; seg < p.n_seg; seg++) {
             int mi, gl, pass;
@@ -325,8 +331,8 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
             const int fmt = format(m), row = gl * RGROUP + tile * MROWS;
             float a12[2][2] = {}, a3[2][2] = {}, mins[2][2] = {};
             for (int b0 = 0; b0 < p.NB; b0 += RKW) {
-                wait_phase(full + slot, parity);
-                if (b0 + kw < p.NB && row < m.out) {
+                if (sound) sound = wait_warp(full + slot, parity, p.status);
+                if (b0 + kw < p.NB && row < m.out && sound) {
                     const uint8_t* st = ring + (size_t)slot * p.slot;
                     const uint8_t* sb = st + tile * MROWS * stage_pitch(fmt, RKW) + kw * fmt_bytes(fmt);
                     const uint8_t* xb = st + wslot + kw * XB;
@@ -337,7 +343,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
                     if ((MASK & 16) && fmt == 4) rows_block<4>(sb, 0, xb, lane, a12, a3, mins);
                 }
                 __syncwarp();
-                if (lane == 0) arrive(empty + slot);
+                if (lane == 0 && sound) arrive(empty + slot);
                 if (++slot == p.stages) { slot = 0; parity ^= 1u; }
             }
             // (q1, q2) counted 1 / 256 of their weight; codes were carried x4 (Q6_K) or x16 (Q4_0)
@@ -349,7 +355,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
                     const int src = (lane & ~3) + 2 * j + (t >> 1);
                     const float u0 = __shfl_sync(0xFFFFFFFFu, a3[0][r], src), u1 = __shfl_sync(0xFFFFFFFFu, a3[1][r], src);
                     const float v = fmaf(a12[j][r], f12, fmaf((t & 1) ? u1 : u0, f3, -mins[j][r]));
-                    part[(seg * RTILES * RKW + kw) * 128 + (4 * j + t) * MROWS + g + 8 * r] = v;
+                    part[(seg * RTILES * RKW + kw) * 128 + (4 * j + t) * MROWS + g + 8 * r] = sound ? v : __uint_as_float(0x7FFFFFFFu);      // NaN
                 }
         }
         named_sync<RKW * 32>(1 + tile);
@@ -424,6 +430,7 @@ void gemv_rows(const GemvMat* mats, int n_mat, int K, const void* xr, int tokens
     p.n_mat = n_mat; p.NB = K / 256; p.tokens = tokens; p.passes = (tokens + 7) / 8;
     p.xr = static_cast<const uint8_t*>(xr);
     p.epilogue = (int)ep; p.n_seg = ep == GEMV_SWIGLU ? 2 : 1;
+    p.status = wait_status();
     int groups = 0;
     for (int i = 0; i < n_mat; i++) {
         RowsMat& m = p.mat[i];

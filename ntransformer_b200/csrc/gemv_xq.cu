@@ -10,6 +10,7 @@
 // Bound by instruction issue (2.0 instructions a weight; 57344 x 8192 in Q4_K 53 us): gemv_kquant.cu is faster and is what every other caller takes.
 #include "kernels_internal.h"
 #include "ring.cuh"
+#include "wait_status.cuh"
 #include "xquant.cuh"
 #include "gemv_kq_device.cuh"
 #include <cuda_fp16.h>
@@ -42,6 +43,7 @@ struct XqParams {
     // Rounds over grid * gpc warp slots.  A last round that fills at most half (a quarter) of them deals its tail_groups row-groups out 2 (1) rows at a
     // time over all slots, so that it costs tail_nr / 4 of a round.  tail_nr == 4: no split.
     int full_rounds, tail_groups, tail_nr;
+    unsigned* status;          // wait_status.cuh
 };
 
 // MASK: bit f set <=> matrices of format f may appear in this launch (mixed Q4_K_M projections share one launch).
@@ -142,14 +144,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS <= 6 ? 2 : 1) gemv_xq_kernel
 
     int slot = 0;
     uint32_t parity = 0;
+    bool sound = true;                                       // no wait of this warp has run out
     for (int round = 0; round < n_rounds; round++) {
         int g, row_sub, nr;
         const bool live = slot_of(round, g, row_sub, nr);
         float res[2] = {0.f, 0.f};
         for (int seg = 0; seg < n_seg; seg++) {
             float acc[RG] = {0.f, 0.f, 0.f, 0.f};
-            mbar_wait(bars + slot, parity);
-            if (live && blk < nbc) {
+            if (sound) sound = wait_warp(bars + slot, parity, p.status);
+            if (live && blk < nbc && sound) {
                 int mi, gl;
                 locate(g, seg, mi, gl);
                 const uint8_t* slot_base = ring + (size_t)slot * STAGE_STRIDE;
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS <= 6 ? 2 : 1) gemv_xq_kernel
                 }
             }
             __syncwarp();
-            if (lane == 0 && issued < n_stages_total) issue_next(slot);
+            if (lane == 0 && issued < n_stages_total && sound) issue_next(slot);
             issued++;
             if (++slot == stages) { slot = 0; parity ^= 1u; }
             res[seg] = reduce4(acc, lane);
@@ -186,7 +189,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS <= 6 ? 2 : 1) gemv_xq_kernel
         const int buf = round & 1;
         if (live && (lane & 7) == 0) {
             const int r = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
-            partial[buf][warp][0][r] = res[0];
+            partial[buf][warp][0][r] = sound ? res[0] : __uint_as_float(0x7FFFFFFFu);      // NaN
             partial[buf][warp][1][r] = res[1];
         }
         __syncthreads();
@@ -301,6 +304,7 @@ void gemv_xq(const GemvMat* mats, int n_mat, int K, const void* xq, GemvEpilogue
     }
     p.n_seg = ep == GEMV_SWIGLU ? 2 : 1;
     p.total_groups = p.n_seg == 2 ? p.mat[0].groups : total;
+    p.status = wait_status();
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -71,6 +71,10 @@ bool gemv_kq_quarter(const GemvMat* mats, int n_mat, int K, const GemvInput& in,
 // epilogue GEMV_PEER: one matrix, rows == peer.hidden
 void gemv_kq_peer(const GemvMat& mat, int K, const GemvInput& in, const PeerOut& peer, cudaStream_t s);
 
+// wait_status.cu: the word that a kernel's wait sets where it ran out (wait_status.cuh), for kernels (null: no device) and for the host
+unsigned* wait_status();
+bool wait_expired();
+
 int gemv_kq_format(DType dt);             // the block formats' numbers in the two kernels, -1: none
 // gemv_rows.cu: the same matrices times a few tokens.  quantize_rows: F32 rows [tokens, K] (norm_w: their RMSNorm) into xr (gemv_rows_bytes);
 // gemv_rows: y of matrix i is [tokens, out_i] (STORE, ADD, SWIGLU); gemv_kq_any_pitch says what is taken.

@@ -35,6 +35,7 @@ struct BlkMat { const uint8_t* W; float* C; int rows, tiles, fmt; long long pitc
 struct BlkParams {
     BlkMat mat[3];
     int n_mat, T, NT, cols, n_tiles, Mp, K, add, b_stages, raw_depth, raw_slot, d_bufs;
+    unsigned* status;          // wait_status.cuh
 };
 
 // tcgen05.mma with A in tensor memory
@@ -191,12 +192,17 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
 
     if (warp == 0) {
         if (lane == 0) {                                           // ---- tokens by TMA ----
-            uint32_t st = 0, par = 1;
-            for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
+            uint32_t st = 0, par = 1, filled = 0;
+            bool sound = true;                                     // no wait of this thread has run out
+            for (int tile = blockIdx.x; tile < p.n_tiles && sound; tile += gridDim.x) {
                 int mi, row0, t0;
                 place(tile, mi, row0, t0);
                 for (int kb = 0; kb < num_kb; kb++) {
-                    wait_phase(b_empty + st, par);
+                    if (!(sound = wait_phase(b_empty + st, par, p.status))) {
+                        for (uint32_t s = 0; s < filled; s++) wait_phase(b_full + s, s < st ? par ^ 1u : par, p.status);      // the copies in flight
+                        break;
+                    }
+                    filled = min(filled + 1, (uint32_t)p.b_stages);
                     uint8_t* d = smem + (size_t)st * b_stage;
                     mbar_expect_tx(b_full + st, b_stage);
                     tma_load_2d(d, &map_x, kb * QBK, t0, b_full + st);
@@ -213,14 +219,15 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
         const uint64_t desc0 = make_desc(smem), lo_step = (uint64_t)(b_tile >> 4), stage_step = (uint64_t)(b_stage >> 4);
         uint32_t bs = 0, bpar = 0, as = 0, apar = 0, db = 0, dpar = 1;
-        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x)
-            for (int kc = 0; kc < n_kc; kc++) {
-                wait_phase(d_empty + db, dpar);
+        bool sound = true, issued = false;                         // no wait of this warp has run out
+        for (int tile = blockIdx.x; tile < p.n_tiles && sound; tile += gridDim.x)
+            for (int kc = 0; kc < n_kc && sound; kc++) {
+                if (!(sound = wait_warp(d_empty + db, dpar, p.status))) break;
                 const uint32_t d = tm + D_COL + db * NT;
                 const int kb0 = kc * KC, kb1 = min(num_kb, kb0 + KC);
                 for (int kb = kb0; kb < kb1; kb++) {
-                    wait_phase(b_full + bs, bpar);
-                    wait_phase(a_full + as, apar);
+                    if (!(sound = wait_warp(b_full + bs, bpar, p.status) && wait_warp(a_full + as, apar, p.status))) break;
+                    issued = true;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t bh = desc0 + bs * stage_step, bl = bh + lo_step;
                     const uint32_t ah = tm + as * A_COLS, al = ah + 32;
@@ -241,16 +248,19 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                 }
                 if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
             }
+        // a launch given up: the products in flight first (the last k-block's commit came after all of them)
+        if (!sound && issued) wait_warp(a_empty + (as + A_STAGES - 1) % A_STAGES, as == 0 ? apar ^ 1u : apar, p.status);
     } else if (warp < 6) {                                         // ---- epilogue: a lane is a row of W, so a warp stores 128 contiguous bytes for each token ----
         const int quarter = warp & 3;
         uint32_t db = 0, dpar = 0;
-        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
+        bool sound = true;
+        for (int tile = blockIdx.x; tile < p.n_tiles && sound; tile += gridDim.x) {
             int mi, row0, t0;
             place(tile, mi, row0, t0);
             const BlkMat& m = p.mat[mi];
             const int row = row0 + quarter * 32 + lane, live = min(NT, p.T - t0);
             for (int kc = 0; kc < n_kc; kc++) {
-                wait_phase(d_full + db, dpar);
+                if (!(sound = wait_warp(d_full + db, dpar, p.status))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem + ((uint32_t)(quarter * 32) << 16) + D_COL + db * NT;
                 const bool add = p.add || kc > 0;
@@ -303,6 +313,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         };
         for (int i = 0; i < depth - 1; i++) copy_next();
         int slot = 0, pending = -1;
+        bool sound = true;                                         // the four warps that share rows keep meeting at their barrier in any case
         auto stored = [&](int stage) {
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -334,7 +345,9 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     }
                     // the stores of the k-block before had this one's arithmetic to arrive in
                     if (pending >= 0) stored(pending);
-                    wait_phase(a_empty + as, apar);
+                    pending = -1;
+                    if (sound) sound = wait_warp(a_empty + as, apar, p.status);
+                    if (!sound) continue;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t a = tmem + ((uint32_t)(quarter * 32) << 16) + as * A_COLS + hf * 16;
                     tmem_st16(a, hi);
@@ -377,6 +390,7 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const void* workspace, i
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     BlkParams p{};
+    p.status = wait_status();
     p.n_mat = n_mat; p.T = T; p.K = K; p.add = add;
     p.Mp = (T + 127) / 128 * 128;
     int tiles = 0, slot = 0;

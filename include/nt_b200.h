@@ -94,6 +94,15 @@ int    nt_b200_gemv_fused_f32(int n_mat, float* const* y, const void* const* W, 
 /* How nt_b200_gemv_fused* would deal out an SM's shared memory for these matrices: plan[0] warps that share a row group, plan[1] such teams in a
  * CTA, plan[2] stages of a team's ring.  Returns 0, or < 0 where the matrix-instruction kernel does not take them.  Needs no GPU. */
 int    nt_b200_gemv_fused_plan(int n_mat, const int* out_features, const int* dtypes, int in_features, int epilogue, int* plan);
+/* The same products for a few tokens: x [tokens, in_features], y of matrix i [tokens, out_features[i]]; quantises the tokens (norm_w: their RMSNorm) into
+ * scratch (nt_b200_gemv_rows_bytes) and reads every weight once for 8 of them.  Returns 0, or < 0 when rejected (nothing launched). */
+size_t nt_b200_gemv_rows_bytes(int tokens, int K);
+int    nt_b200_gemv_rows(int n_mat, float* const* y, const void* const* W, const int* out_features, const int* dtypes, int in_features,
+                         const float* x, const float* norm_w, float eps, int tokens, void* scratch, int epilogue, void* stream);
+/* Prompts: C of matrix i [tokens, out_features[i]] (+)= X . W_i^T on the tcgen05 tensor cores, the blocks expanded on the way; X split into `workspace`
+ * (nt_b200_split_activations).  Returns 0, or < 0 when rejected (nothing launched). */
+int    nt_b200_gemm_blocks_ws(int n_mat, float* const* C, const void* const* W, const int* out_features, const int* dtypes, int in_features,
+                              const void* workspace, int tokens, int add, void* stream);
 /* The decode step's attention sub-block in ONE launch: launch_rope (src/cuda/rotary.cu:113-140; q and k are read, not
  * modified) + launch_copy_to_kv_cache at row *pos_dev (src/cuda/attention.cu:405-425) + launch_attention_decode over
  * *pos_dev + 1 keys (src/cuda/attention.cu:348-375), context split over CTAs, merged by the last CTA of each head group.

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
     float* part = reinterpret_cast<float*>(smem + SM_PART) + team * 2 * 2 * KW * MROWS;      // [buffer][segment][K share][row]
     int slot = 0, buf = 0, turn = 0;
     uint32_t parity = 0;
-    bool sound = true;                                          // no wait of this warp has run out
+    bool sound = true;                                          // no wait of this lane has run out
     for (int u = u0; u < p.total_groups; u += ustep) {
         for (int seg = 0; seg < p.n_seg; seg++) {
             int mi, gl;
@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
             float acc[2] = {}, mins[2] = {};
             for (int b0 = 0; b0 < p.NB; b0 += sblocks) {
                 const int sbi = b0 + warp, left = p.NB - sbi;   // super-blocks from this warp's first on
-                if (sound) sound = wait_warp(full + slot, parity, p.status);
-                if (left > 0 && sound) {
+                wait_sound(full + slot, parity, p.status, sound);
+                if (left > 0) {
                     const uint8_t* sb = ring + (size_t)slot * slot_bytes + warp * blk;
                     const bool two = KW == 4 && left > KW;
                     if ((MASK & 1) && fmt == 0) { if (two) tile_blocks<0, 2, KW>(sb, 0, sbi, xv, lane, acc, mins); else tile_blocks<0, 1, KW>(sb, 0, sbi, xv, lane, acc, mins); }

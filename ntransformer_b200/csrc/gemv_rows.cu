@@ -322,7 +322,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
     float* part = reinterpret_cast<float*>(smem + R_PART) + tile * RKW * 128;       // + segment * RTILES * RKW * 128
     int slot = 0, turn = 0;
     uint32_t parity = 0;
-    bool sound = true;                                             // no wait of this warp has run out
+    bool sound = true;                                             // no wait of this lane has run out
     for (int u = blockIdx.x; u < p.total_units; u += gridDim.x) {
         for (int seg = 0; seg < p.n_seg; seg++) {
             int mi, gl, pass;
@@ -331,8 +331,8 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
             const int fmt = format(m), row = gl * RGROUP + tile * MROWS;
             float a12[2][2] = {}, a3[2][2] = {}, mins[2][2] = {};
             for (int b0 = 0; b0 < p.NB; b0 += RKW) {
-                if (sound) sound = wait_warp(full + slot, parity, p.status);
-                if (b0 + kw < p.NB && row < m.out && sound) {
+                wait_sound(full + slot, parity, p.status, sound);
+                if (b0 + kw < p.NB && row < m.out) {
                     const uint8_t* st = ring + (size_t)slot * p.slot;
                     const uint8_t* sb = st + tile * MROWS * stage_pitch(fmt, RKW) + kw * fmt_bytes(fmt);
                     const uint8_t* xb = st + wslot + kw * XB;

@@ -144,15 +144,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS <= 6 ? 2 : 1) gemv_xq_kernel
 
     int slot = 0;
     uint32_t parity = 0;
-    bool sound = true;                                       // no wait of this warp has run out
+    bool sound = true;                                       // no wait of this lane has run out
     for (int round = 0; round < n_rounds; round++) {
         int g, row_sub, nr;
         const bool live = slot_of(round, g, row_sub, nr);
         float res[2] = {0.f, 0.f};
         for (int seg = 0; seg < n_seg; seg++) {
             float acc[RG] = {0.f, 0.f, 0.f, 0.f};
-            if (sound) sound = wait_warp(bars + slot, parity, p.status);
-            if (live && blk < nbc && sound) {
+            wait_sound(bars + slot, parity, p.status, sound);
+            if (live && blk < nbc) {
                 int mi, gl;
                 locate(g, seg, mi, gl);
                 const uint8_t* slot_base = ring + (size_t)slot * STAGE_STRIDE;

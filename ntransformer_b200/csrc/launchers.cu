@@ -143,6 +143,25 @@ int nt_b200_gemv_fused_plan(int n_mat, const int* out_features, const int* dtype
     if (!nt::b200::gemv_kq_any_pitch(m, n_mat, in_features)) return -2;
     return nt::b200::gemv_kq_plan(m, n_mat, in_features, epilogue == 2, plan) ? 0 : -2;
 }
+size_t nt_b200_gemv_rows_bytes(int tokens, int K) { return nt::b200::gemv_rows_bytes(tokens, K); }
+int nt_b200_gemv_rows(int n_mat, float* const* y, const void* const* W, const int* out_features, const int* dtypes, int in_features, const float* x,
+                      const float* norm_w, float eps, int tokens, void* scratch, int epilogue, void* stream) {
+    if (n_mat < 1 || n_mat > 3 || !x || tokens < 1) return -1;
+    nt::b200::GemvMat m[3];
+    for (int i = 0; i < n_mat; i++) { m[i].W = W[i]; m[i].y = y[i]; m[i].out = out_features[i]; m[i].dtype = (DType)dtypes[i]; m[i].row_pitch = 0; }
+    if (!nt::b200::gemv_kq_any_pitch(m, n_mat, in_features) || (reinterpret_cast<uintptr_t>(x) & 15)) return -2;
+    if (epilogue == 2 && (n_mat != 2 || out_features[0] != out_features[1] || dtypes[0] != dtypes[1])) return -3;
+    nt::b200::quantize_rows(scratch, x, norm_w, eps, tokens, in_features, static_cast<cudaStream_t>(stream));
+    nt::b200::gemv_rows(m, n_mat, in_features, scratch, tokens, (nt::b200::GemvEpilogue)epilogue, static_cast<cudaStream_t>(stream));
+    return 0;
+}
+int nt_b200_gemm_blocks_ws(int n_mat, float* const* C, const void* const* W, const int* out_features, const int* dtypes, int in_features,
+                           const void* workspace, int tokens, int add, void* stream) {
+    if (n_mat < 1 || n_mat > 3) return -1;
+    nt::b200::GemvMat m[3];
+    for (int i = 0; i < n_mat; i++) { m[i].W = W[i]; m[i].y = C[i]; m[i].out = out_features[i]; m[i].dtype = (DType)dtypes[i]; m[i].row_pitch = 0; }
+    return nt::b200::gemm_blocks(m, n_mat, in_features, workspace, tokens, add != 0, static_cast<cudaStream_t>(stream)) ? 0 : -2;
+}
 size_t nt_b200_attention_decode_scratch_floats(int ms, int nh, int nkv, int hd) { return nt::b200::attention_decode_dyn_scratch_floats(ms, nh, nkv, hd); }
 int nt_b200_attention_decode_tickets(int nh, int nkv) { return nt::b200::attention_decode_fused_tickets(nh, nkv); }
 void nt_b200_attention_decode_fused(float* o, const float* q, const float* k, const float* v, void* kc, void* vc, const int* pos_dev, int ms,

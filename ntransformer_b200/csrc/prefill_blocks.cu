@@ -219,19 +219,20 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
         const uint64_t desc0 = make_desc(smem), lo_step = (uint64_t)(b_tile >> 4), stage_step = (uint64_t)(b_stage >> 4);
         uint32_t bs = 0, bpar = 0, as = 0, apar = 0, db = 0, dpar = 1;
-        bool sound = true, issued = false;                         // no wait of this warp has run out
-        for (int tile = blockIdx.x; tile < p.n_tiles && sound; tile += gridDim.x)
-            for (int kc = 0; kc < n_kc && sound; kc++) {
-                if (!(sound = wait_warp(d_empty + db, dpar, p.status))) break;
+        bool sound = true;                                         // no wait of this lane has run out
+        int last = -1;                                             // stage and parity of the last commit
+        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x)
+            for (int kc = 0; kc < n_kc; kc++) {
+                wait_sound(d_empty + db, dpar, p.status, sound);
                 const uint32_t d = tm + D_COL + db * NT;
                 const int kb0 = kc * KC, kb1 = min(num_kb, kb0 + KC);
                 for (int kb = kb0; kb < kb1; kb++) {
-                    if (!(sound = wait_warp(b_full + bs, bpar, p.status) && wait_warp(a_full + as, apar, p.status))) break;
-                    issued = true;
+                    wait_sound(b_full + bs, bpar, p.status, sound);
+                    wait_sound(a_full + as, apar, p.status, sound);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t bh = desc0 + bs * stage_step, bl = bh + lo_step;
                     const uint32_t ah = tm + as * A_COLS, al = ah + 32;
-                    if (leader) {
+                    if (leader && sound) {
 #pragma unroll
                         for (int k = 0; k < 4; k++) umma_ts(d, al + 8 * k, bh + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);      // the small products first
 #pragma unroll
@@ -240,6 +241,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                         for (int k = 0; k < 4; k++) umma_ts(d, ah + 8 * k, bh + 2 * k, idesc, 1u);
                         umma_commit(b_empty + bs);
                         umma_commit(a_empty + as);
+                        last = (int)(as * 2 + apar);
                         if (kb + 1 == kb1) umma_commit(d_full + db);
                     }
                     __syncwarp();
@@ -248,19 +250,18 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                 }
                 if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
             }
-        // a launch given up: the products in flight first (the last k-block's commit came after all of them)
-        if (!sound && issued) wait_warp(a_empty + (as + A_STAGES - 1) % A_STAGES, as == 0 ? apar ^ 1u : apar, p.status);
+        if (!sound && last >= 0) wait_phase(a_empty + (last >> 1), last & 1, p.status);      // given up: the products in flight
     } else if (warp < 6) {                                         // ---- epilogue: a lane is a row of W, so a warp stores 128 contiguous bytes for each token ----
         const int quarter = warp & 3;
         uint32_t db = 0, dpar = 0;
         bool sound = true;
-        for (int tile = blockIdx.x; tile < p.n_tiles && sound; tile += gridDim.x) {
+        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
             int mi, row0, t0;
             place(tile, mi, row0, t0);
             const BlkMat& m = p.mat[mi];
             const int row = row0 + quarter * 32 + lane, live = min(NT, p.T - t0);
             for (int kc = 0; kc < n_kc; kc++) {
-                if (!(sound = wait_warp(d_full + db, dpar, p.status))) break;
+                wait_sound(d_full + db, dpar, p.status, sound);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem + ((uint32_t)(quarter * 32) << 16) + D_COL + db * NT;
                 const bool add = p.add || kc > 0;
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     uint32_t v[32];
                     tmem_ld32(d + (uint32_t)n, v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (row < m.rows) {
+                    if (row < m.rows && sound) {
                         // adds go to the memory's side (this lane is the element's only writer, so their order is fixed): nothing is waited for
 #pragma unroll
                         for (int j = 0; j < 32; j++) {
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(d_empty + db);
+                if (lane == 0 && sound) mbar_arrive(d_empty + db);
                 if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
             }
         }
@@ -313,12 +314,12 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         };
         for (int i = 0; i < depth - 1; i++) copy_next();
         int slot = 0, pending = -1;
-        bool sound = true;                                         // the four warps that share rows keep meeting at their barrier in any case
+        bool sound = true;
         auto stored = [&](int stage) {
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(a_full + stage);
+            if (lane == 0 && sound) mbar_arrive(a_full + stage);
         };
         for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
             int mi, row0, t0;
@@ -345,9 +346,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     }
                     // the stores of the k-block before had this one's arithmetic to arrive in
                     if (pending >= 0) stored(pending);
-                    pending = -1;
-                    if (sound) sound = wait_warp(a_empty + as, apar, p.status);
-                    if (!sound) continue;
+                    wait_sound(a_empty + as, apar, p.status, sound);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t a = tmem + ((uint32_t)(quarter * 32) << 16) + as * A_COLS + hf * 16;
                     tmem_st16(a, hi);

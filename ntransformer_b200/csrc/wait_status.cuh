@@ -1,9 +1,9 @@
 // wait_status.cuh — waits for the phase of a copy, a product or a reader in the same CTA, with a limit.
 //
 // What is waited for is under way and takes microseconds.  Where it does not come within the limit the launch is broken: the wait says so in a status word
-// that the host reads (kernels_internal.h wait_status), and returns false.  A warp that was told so waits for nothing more, uses no stage and arrives on
-// no barrier of the pipeline, so the others' waits run out as well; the CTA then leaves its loops as one, after the copies and products that it has in
-// flight (again with a limit).
+// that the host reads (kernels_internal.h wait_status).  Who was told so waits for nothing more and arrives on no barrier of the pipeline, so the others'
+// waits run out as well; the loops go to their end (on whatever the stages hold: results are NaN or not written), and whoever issued copies or products
+// waits for those in flight, again with a limit.
 #pragma once
 #include "ring.cuh"
 
@@ -33,7 +33,12 @@ __device__ __forceinline__ bool wait_phase(uint64_t* bar, uint32_t parity, unsig
         }
     return true;
 }
-// The same by a whole warp: one answer for all lanes.
+// In a loop whose instructions count: a lane that has once waited in vain (sound == false) goes on without waiting.
+__device__ __forceinline__ void wait_sound(uint64_t* bar, uint32_t parity, unsigned* status, bool& sound) {
+    if (phase_done(bar, parity) || !sound) return;
+    sound = wait_phase(bar, parity, status);
+}
+// By a whole warp that leaves where the wait runs out: one answer for all lanes.
 __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, unsigned* status) { return __all_sync(0xFFFFFFFFu, wait_phase(bar, parity, status)) != 0; }
 
 }  // namespace

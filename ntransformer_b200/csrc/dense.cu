@@ -659,8 +659,9 @@ void gemv_sum(float* y, const SumTerm* terms, int n, int out, DType dt, bool add
     }
     const size_t smem = (size_t)at * sizeof(float);
     NT_CHECK(smem <= 200 * 1024, "gemv_sum: the input vectors do not fit in shared memory");
-    // warps per row: as many as keep the grid within four CTAs to an SM (two are resident by their registers)
-    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(4, (size_t)(220 * 1024) / (smem + 1024)));
+    // Warps per row: as many as keep the grid within three CTAs to an SM (two are resident by their registers).  Four were slower: 4096 rows of 4096 + 4096
+    // 28.7 us against 24.6, 2048 of 2048 + 8192 24.6 against 20.5; 4096 + 14336, 8192 + 8192 and 3072 + 8192 the same.
+    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(3, (size_t)(220 * 1024) / (smem + 1024)));
     sd.nw = 1;
     while (sd.nw < 4 && (long)out * sd.nw * 2 <= (long)148 * per_sm * SV_WARPS) sd.nw *= 2;
     const int rows = SV_WARPS / sd.nw, grid = std::min((out + rows - 1) / rows, 148 * per_sm);

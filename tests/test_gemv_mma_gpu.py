@@ -117,7 +117,7 @@ def test_nan_infinity_and_the_smallest_numbers(dt):
 
 def test_nan_in_a_vector_that_is_quantised_by_a_launch_of_its_own():
     rng = np.random.default_rng(12)
-    rows, cols = 40, 1024
+    rows, cols = 40, 2048
     x = rng.standard_normal(cols).astype(np.float32)
     x[500] = np.nan
     for dt in FORMATS:

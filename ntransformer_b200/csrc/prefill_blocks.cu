@@ -6,17 +6,20 @@
 //   * the roles of the operands are exchanged: W is A (M = 128 rows), tokens are B (N = NT, any multiple of 16 up to 256, chosen so that the tiles
 //     fill whole waves of the SMs);
 //   * sixteen warps expand 64 columns of the 128 rows at a time (eight each of two k-blocks in turn), a row to a lane: blocks come into shared memory by cp.async, the F32 value of a weight is
-//     split into F16 hi + lo (W = hi + lo to 2^-22) and stored to TENSOR MEMORY, from where tcgen05.mma takes its A operand: shared memory's bandwidth
+//     split into F16 hi + lo (W = hi + lo to 2^-22 of it, or to 2^-25 where that is more: the least F16 halved) and stored to TENSOR MEMORY, from where tcgen05.mma takes its A operand: shared memory's bandwidth
 //     is left to B;
-//   * B is the split of the tokens (prefill_gemm.cu's workspace) by TMA; three products hi.hi, hi.lo, lo.hi (lo.lo is below the F32 rounding);
-//   * 2048 columns of K to an accumulator, partial sums added in F32 by the epilogue: the tensor cores truncate each addition, and three products a step
-//     would otherwise leave more error than two over 4096 columns did.
+//   * B is the split of the tokens (prefill_gemm.cu's workspace) by TMA; three products hi.hi, hi.lo, lo.hi (lo.lo, up to 2^-22 of a product and of either
+//     sign, leaves 4e-8 of a result; what follows is a hundred times that);
+//   * half of K, at most 2048 columns, to an accumulator, partial sums added in F32 by the epilogue: the tensor cores cut off each addition, which leaves
+//     1.86e-8 of the result for each.  The expanded form made 2 of them for 16 columns of up to 4096, this one makes 3 for 16 of half as many: error against 64 bits
+//     2.5e-6 -> 2.0e-6 at K = 1024, 9.7e-6 -> 7.1e-6 at 4096 (whole rows to 2048 left 3.6e-6 at 1024).
 // Llama-3 8B layer in Q4_K_M, 500 tokens: q/k/v 78 us (was 332 with the expansion), o 63 (173), gate + up 336 (604 and 40 for SwiGLU), down 201 (494); of
 // 1.9 us per 64 columns at first, 0.9 went into an epilogue that read C back before each addition (now red.add), 0.2 into an MMA loop of one lane.
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "tc_device.cuh"
 #include "gemv_mma_device.cuh"
+#include <algorithm>
 
 namespace nt { namespace b200 {
 
@@ -25,7 +28,7 @@ namespace {
 constexpr int QBK = 64;                                  // columns of a k-block: a 128-byte swizzle row of F16
 constexpr int A_STAGES = 4, A_COLS = 64;             // tensor-memory columns of an expanded k-block: 32 hi, 32 lo; the accumulators lie behind them
 constexpr int D_COL = A_STAGES * A_COLS;
-constexpr int KC = 2048 / QBK;                           // k-blocks to an accumulator
+constexpr int KC_MAX = 2048 / QBK;                       // k-blocks to an accumulator, at most
 constexpr int B_STAGES_MAX = 4;
 constexpr int Q_THREADS = 22 * 32;                       // warp 0 TMA, 1 MMA, 2-5 epilogue, 6-21 expansion
 
@@ -34,7 +37,7 @@ __host__ __device__ constexpr int raw_pitch(int fmt) { return fmt == 2 ? 240 : f
 struct BlkMat { const uint8_t* W; float* C; int rows, tiles, fmt; long long pitch; };
 struct BlkParams {
     BlkMat mat[3];
-    int n_mat, T, NT, cols, n_tiles, Mp, K, add, b_stages, raw_depth, raw_slot, d_bufs;
+    int n_mat, T, NT, cols, n_tiles, Mp, K, kc, add, b_stages, raw_depth, raw_slot, d_bufs;
     unsigned* status;          // wait_status.cuh
 };
 
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
     __shared__ uint64_t b_full[B_STAGES_MAX], b_empty[B_STAGES_MAX], a_full[A_STAGES], a_empty[A_STAGES], d_full[2], d_empty[2];
     __shared__ uint32_t tmem_base_smem;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int NB = p.K / 256, num_kb = p.K / QBK, n_kc = (num_kb + KC - 1) / KC, NT = p.NT;
+    const int NB = p.K / 256, num_kb = p.K / QBK, n_kc = (num_kb + p.kc - 1) / p.kc, NT = p.NT;
     const uint32_t b_tile = (uint32_t)NT * 128, b_stage = 2 * b_tile;
     uint8_t* raw = smem + (size_t)p.b_stages * b_stage;
     auto place = [&](int tile, int& mi, int& row0, int& t0) {      // tokens inside: the CTAs of a wave share rows
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
             for (int kc = 0; kc < n_kc; kc++) {
                 wait_sound(d_empty + db, dpar, p.status, sound);
                 const uint32_t d = tm + D_COL + db * NT;
-                const int kb0 = kc * KC, kb1 = min(num_kb, kb0 + KC);
+                const int kb0 = kc * p.kc, kb1 = min(num_kb, kb0 + p.kc);
                 for (int kb = kb0; kb < kb1; kb++) {
                     wait_sound(b_full + bs, bpar, p.status, sound);
                     wait_sound(a_full + as, apar, p.status, sound);
@@ -391,6 +394,7 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const void* workspace, i
     BlkParams p{};
     p.status = wait_status();
     p.n_mat = n_mat; p.T = T; p.K = K; p.add = add;
+    p.kc = std::min(KC_MAX, (K / QBK + 1) / 2);
     p.Mp = (T + 127) / 128 * 128;
     int tiles = 0, slot = 0;
     for (int i = 0; i < n_mat; i++) {

@@ -99,6 +99,12 @@ def test_few_tokens_swiglu_and_what_a_nan_reaches(dt):
     assert torch.isnan(y[3]).all() and torch.isfinite(y[:3]).all() and torch.isfinite(y[4:]).all()
 
 
+def cut(cols):
+    """Three products for 16 columns of half the row, at most 2048: each addition to an accumulator is cut by half a unit (2^-24 of the sum so far) on average and
+    always to one side, over sums that grow to the accumulator's: 2/3 of 2^-24 each; F32 additions of the partial sums and pairs of halves add 2^-21."""
+    return 3 * -(-min(2048, cols / 2) // 16) * 2.0 ** -24 * 2 / 3 + 2.0 ** -21
+
+
 # tokens around the tile widths (any multiple of 16 up to 256, two column tiles), rows around 128, K of one and of several accumulators of 2048
 @pytest.mark.parametrize("dt", FORMATS, ids=lambda d: d.name)
 @pytest.mark.parametrize("tokens,rows,cols", [(17, 100, 256), (113, 129, 2304), (256, 128, 4096), (300, 1000, 768), (500, 384, 11008)])
@@ -108,11 +114,9 @@ def test_prompt(dt, tokens, rows, cols):
     ref = x.double() @ W64.T
     y = torch.full((tokens + 1, rows), 7.0, device="cuda")
     blocks_product([y], [W], [rows], [dt], x)
-    # three products of halves: 16 * 8 * 3 additions to an accumulator, each cut at 2^-24 of it, and K / 2048 rounded additions behind them: below 1.2e-5 of a result's
-    # scale where every cut falls to one side (random signs leave a tenth of it); pairs of halves hold 2^-22
-    assert rel(y[:tokens], ref) <= 4e-6 and (y[tokens] == 7.0).all()
+    assert rel(y[:tokens], ref) <= cut(cols) and (y[tokens] == 7.0).all()
     blocks_product([y], [W], [rows], [dt], x, add=True)
-    assert rel(y[:tokens], 2 * ref) <= 4e-6 and (y[tokens] == 7.0).all()
+    assert rel(y[:tokens], 2 * ref) <= cut(cols) and (y[tokens] == 7.0).all()
 
 
 def test_prompt_several_matrices():
@@ -122,11 +126,12 @@ def test_prompt_several_matrices():
     ys = [torch.zeros(tokens, o, device="cuda") for o in outs]
     blocks_product(ys, [m[0] for m in mats], outs, dts, x)
     for y, (_, W64) in zip(ys, mats):
-        assert rel(y, x.double() @ W64.T) <= 4e-6
+        assert rel(y, x.double() @ W64.T) <= cut(cols)
 
 
 @pytest.mark.parametrize("dt", FORMATS, ids=lambda d: d.name)
-@pytest.mark.parametrize("tokens,rows,cols", [(64, 512, 1024), (500, 1024, 4096), (200, 512, 14336)])
+@pytest.mark.parametrize("tokens,rows,cols", [(64, 512, 256), (64, 512, 1024), (100, 512, 2048), (64, 512, 2304), (64, 512, 3072), (500, 1024, 4096),
+                                              (200, 512, 14336)])
 @pytest.mark.parametrize("scale", [1.0, 0.05])
 def test_prompt_is_no_further_from_64_bits_than_the_expanded_form(dt, tokens, rows, cols, scale):
     """Before: the matrix written out as two F16 matrices and two GEMMs over them, all four products of halves, 4096 columns to an accumulator."""

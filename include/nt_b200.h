@@ -92,7 +92,7 @@ int    nt_b200_gemv_fused_f32(int n_mat, float* const* y, const void* const* W, 
                               const int* dtypes, int in_features, const float* x, const float* norm_w, float eps,
                               int epilogue, void* stream);
 /* How nt_b200_gemv_fused* would deal out an SM's shared memory for these matrices: plan[0] warps that share a row group, plan[1] such teams in a
- * CTA, plan[2] stages of a team's ring.  Returns 0, or < 0 where the matrix-instruction kernel does not take them.  Needs no GPU. */
+ * CTA, plan[2] stages of a team's ring, plan[3] digits of an activation (3: 24 bits, 4: 32).  Returns 0, or < 0 where the matrix-instruction kernel does not take them.  Needs no GPU. */
 int    nt_b200_gemv_fused_plan(int n_mat, const int* out_features, const int* dtypes, int in_features, int epilogue, int* plan);
 /* The same products for a few tokens: x [tokens, in_features], y of matrix i [tokens, out_features[i]]; quantises the tokens (norm_w: their RMSNorm) into
  * scratch (nt_b200_gemv_rows_bytes) and reads every weight once for 8 of them.  Returns 0, or < 0 when rejected (nothing launched). */

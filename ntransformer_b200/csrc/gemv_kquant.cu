@@ -9,8 +9,8 @@
 //   * several teams on an SM, so that the barriers of one do not idle it.  Weights depend on no kernel in flight: under programmatic launch a
 //     kernel's first stages are fetched while the one before still runs, as far as it leaves room.  The activation vector is read after
 //     griddepcontrol.wait, and the dependants are released after it;
-//   * the prologue quantises the F32 vector (24-bit integers for each 32-block) into shared memory, with RMSNorm's gains multiplied in and its scalar
-//     applied to the results.
+//   * the prologue quantises the F32 vector (24-bit integers for each 32-block, 32-bit ones in front of Q4_0 and Q6_K) into shared memory, with RMSNorm's
+//     gains multiplied in and its scalar applied to the results.
 // Up to 3 matrices of mixed formats share a launch (q / k / v of a Q4_K_M file; gate + up with SwiGLU).
 #include "kernels_internal.h"
 #include "ring.cuh"
@@ -49,18 +49,23 @@ struct KqParams {
     int total_groups;          // SWIGLU: groups of mat[0]
     int n_seg;                 // segments (matrices) per group: 2 for SWIGLU else 1
     int epilogue;
-    int stages, slot;          // depth of a team's ring and bytes of a stage
+    int stages, slot, planes;  // depth of a team's ring and bytes of a stage; digits of an activation
     unsigned* status;          // wait_status.cuh
     PeerOut peer;              // epilogue GEMV_PEER
 };
 
-// Shared memory: [barriers][zeros][norm][partials][digit planes][scales][sums][rings]
+// Shared memory: [barriers][zeros][norm][partials][digit planes][scales(, those of the upper digits)][sums][rings]
 constexpr size_t SM_ZERO = MAX_TEAMS * 16 * MAX_STAGES, SM_RED = SM_ZERO + 16, SM_PART = SM_RED + 112;
 constexpr size_t SM_X = (SM_PART + SM_WARPS * 2 * 2 * MROWS * 4 + 127) & ~(size_t)127;
-__host__ __device__ constexpr size_t x_bytes(int K) { return ((size_t)3 * (K + 64) + (size_t)(K / 32) * 8 + 127) & ~(size_t)127; }
+__host__ __device__ constexpr size_t x_bytes(int K, int planes) { return ((size_t)planes * (K + 64) + (size_t)(K / 32) * (planes == 4 ? 12 : 8) + 127) & ~(size_t)127; }
+// Launches whose vector may have four digits (of Q4_0, and of Q6_K rows off 16 bytes, where there is room): these were multiplied in F32, and three digits left
+// more error than that (Q4_0 4096 wide, one element in a hundred ten times the others: 1.6e-7 of the result, 1.2e-7 in F32; a hundred times: 2.0e-7).  The
+// digit's column of the product was zeros, so only the prologue and the vector's place in shared memory grow.
+__host__ __device__ constexpr bool four_digits(int mask) { return mask == 4 || mask == 16; }
 
 // Eight consecutive elements (t8 = their index / 8), four threads to a 32-element block: digits, scale and sum into shared memory.
-__device__ __forceinline__ void quantize8(const float (&x)[8], int t8, uint8_t* planes, int plane, float* xs, float* sums) {
+template <bool FOUR>
+__device__ __forceinline__ void quantize8(const float (&x)[8], int t8, uint8_t* planes, int plane, int np, float* xs, float* xs_upper, float* sums) {
     float amax = 0.f, s = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; i++) { amax = max_abs(amax, x[i]); s = __fadd_rn(s, x[i]); }
@@ -68,24 +73,28 @@ __device__ __forceinline__ void quantize8(const float (&x)[8], int t8, uint8_t* 
     amax = max_abs(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
     s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 1));
     s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 2));
-    const BlockScale scale(amax);
-    uint32_t d[3][2];
+    const bool four = FOUR && np == 4;
+    const BlockScale scale(amax, four ? BlockScale::TOP4 : BlockScale::TOP3);
+    uint32_t d[4][2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         int T[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) T[i] = scale(x[4 * h + i]);
-        digits4(T, d[0][h], d[1][h], d[2][h]);
+        if (four) digits4(T, d[0][h], d[1][h], d[2][h], d[3][h]);
+        else { digits4(T, d[0][h], d[1][h], d[2][h]); d[3][h] = 0; }
     }
     const uint32_t o = xword_byte(t8 * 8);                      // the two words are neighbours in t: 16 bytes apart
 #pragma unroll
-    for (int p = 0; p < 3; p++) {
+    for (int p = 0; p < (FOUR ? 4 : 3); p++) {
+        if (p == 3 && !four) break;
         *reinterpret_cast<uint32_t*>(planes + p * plane + o) = d[p][0];
         *reinterpret_cast<uint32_t*>(planes + p * plane + o + 16) = d[p][1];
     }
     if ((t8 & 3) == 0) {
         const int b = t8 >> 2;                                  // 32-element block: 2 c + hi of its super-block
         xs[(b & ~7) + (b & 1) * 4 + ((b & 7) >> 1)] = scale.xs;
+        if (four) xs_upper[(b & ~7) + (b & 1) * 4 + ((b & 7) >> 1)] = scale.xs * 65536.0f;
         sums[b] = s;
     }
 }
@@ -100,7 +109,8 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
     const int stages = p.stages, slot_bytes = p.slot;
     uint64_t* full = reinterpret_cast<uint64_t*>(smem) + team * 2 * MAX_STAGES;
     uint64_t* empty = full + MAX_STAGES;
-    uint8_t* ring = smem + SM_X + x_bytes(p.K) + (size_t)team * stages * slot_bytes;
+    const int np = four_digits(MASK) ? p.planes : 3;
+    uint8_t* ring = smem + SM_X + x_bytes(p.K, np) + (size_t)team * stages * slot_bytes;
     const int u0 = (int)blockIdx.x + team * (int)gridDim.x, ustep = (int)gridDim.x * TEAMS;      // few groups: a team in each CTA first
     auto format = [&](const KqMat& m) { return (MASK == 1) ? 0 : (MASK == 2) ? 1 : (MASK == 4) ? 2 : (MASK == 8) ? 3 : (MASK == 16) ? 4 : m.fmt; };
     auto locate = [&](int u, int seg, int& mi, int& gl) {       // matrix and local group of group u
@@ -161,8 +171,9 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
     pdl_launch_dependents();
     const int K = p.K, plane = K + 64, tid = team * KW * 32 + warp * 32 + lane;
     uint8_t* planes = smem + SM_X;
-    float* xs = reinterpret_cast<float*>(planes + 3 * (size_t)plane);
-    float* sums = xs + K / 32;
+    float* xs = reinterpret_cast<float*>(planes + np * (size_t)plane);
+    float* xs_upper = xs + K / 32;                              // four digits
+    float* sums = np == 4 ? xs_upper + K / 32 : xs_upper;
     float* red = reinterpret_cast<float*>(smem + SM_RED);
     float rms_inv = 1.0f;
     if (p.x_f32) {
@@ -186,7 +197,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
 #pragma unroll
                     for (int i = 0; i < 8; i++) { ss = fmaf(x[i], x[i], ss); x[i] = __fmul_rn(x[i], w[i]); }
                 }
-                quantize8(x, t8, planes, plane, xs, sums);
+                quantize8<four_digits(MASK)>(x, t8, planes, plane, np, xs, xs_upper, sums);
             }
         }
         if (p.norm_w) {
@@ -207,13 +218,20 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
 #pragma unroll
             for (int i = 0; i < 4; i++)
                 T[i] = 4 * ((((int)(a << (24 - 8 * i)) >> 24) * 128 + ((int)(b << (24 - 8 * i)) >> 24)) * 128 + ((int)(c << (24 - 8 * i)) >> 24));
-            uint32_t d[3];
-            digits4(T, d[0], d[1], d[2]);
+            uint32_t d[4] = {};
+            const bool four = four_digits(MASK) && np == 4;
+            if (four) {
 #pragma unroll
-            for (int q = 0; q < 3; q++) *reinterpret_cast<uint32_t*>(planes + q * plane + xword_byte(e)) = d[q];
+                for (int i = 0; i < 4; i++) T[i] *= 256;
+                digits4(T, d[0], d[1], d[2], d[3]);
+            } else digits4(T, d[0], d[1], d[2]);
+#pragma unroll
+            for (int q = 0; q < (four_digits(MASK) ? 4 : 3); q++) if (q < 3 || four) *reinterpret_cast<uint32_t*>(planes + q * plane + xword_byte(e)) = d[q];
             if ((e & 31) == 0) {
                 const int blk = e >> 5;
-                xs[(blk & ~7) + (blk & 1) * 4 + ((blk & 7) >> 1)] = 0.25f * __ldg(fs + blk);
+                const int at = (blk & ~7) + (blk & 1) * 4 + ((blk & 7) >> 1);
+                xs[at] = (four ? 0.25f / 256.0f : 0.25f) * __ldg(fs + blk);
+                if (four) xs_upper[at] = 0.25f * 256.0f * __ldg(fs + blk);
                 sums[blk] = __ldg(fs + K / 32 + 2 * blk) + __ldg(fs + K / 32 + 2 * blk + 1);
             }
         }
@@ -229,11 +247,11 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
     }
     const int g = lane >> 2, t = lane & 3;
     XView xv;
-    const bool c0 = g < 3, c1 = g >= 4 && g < 7;
+    const bool c0 = g < np, c1 = g >= 4 && g < 4 + np;
     xv.b0 = c0 ? planes + g * plane + t * 16 : smem + SM_ZERO;
     xv.b1 = c1 ? planes + (g - 4) * plane + t * 16 : smem + SM_ZERO;
     xv.m0 = c0 ? ~0u : 0u; xv.m1 = c1 ? ~0u : 0u;
-    xv.xs = xs; xv.sums = sums;
+    xv.xs = np == 4 && !(t & 1) ? xs_upper : xs; xv.sums = sums;
 
     float* part = reinterpret_cast<float*>(smem + SM_PART) + team * 2 * 2 * KW * MROWS;      // [buffer][segment][K share][row]
     int slot = 0, buf = 0, turn = 0;
@@ -263,7 +281,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
                 if (lane == 0 && sound) arrive(empty + slot);
                 if (++slot == stages) { slot = 0; parity ^= 1u; }
             }
-            const float f = lane_factor(fmt, t);
+            const float f = lane_factor(fmt, t, np);
             // over the four lanes of a row pair: lane t = 0 ends with row g, t = 1 with row g + 8
             const float v0 = fmaf(acc[0], f, -mins[0]), v1 = fmaf(acc[1], f, -mins[1]);
             float v = (t & 1) ? v1 : v0;
@@ -343,17 +361,20 @@ bool quarter_split_enabled() {    // NT_B200_GEMV_QB_SPLIT=0: launches that mix 
 }
 
 // How the 16 warps of an SM are dealt out: CTAs of `teams` teams of `kw` warps, a ring of `stages` stages to a team.  stages == 0: no form fits.
-struct TeamPlan { int kw, teams, stages, slot; };
+struct TeamPlan { int kw, teams, stages, slot, planes; };
 int team_slot(int mask, int kw) {         // bytes of a stage
     int slot = 0;
     for (int f = 0; f < 5; f++) if ((mask >> f) & 1 && MROWS * stage_pitch(f, kw) > slot) slot = MROWS * stage_pitch(f, kw);
     return slot;
 }
-TeamPlan plan_teams(int mask, int K, int groups) {
-    const size_t fixed = SM_X + x_bytes(K);
+TeamPlan plan_teams(int mask, int K, int groups, bool four) {
     auto form = [&](int kw, int teams, size_t cap) {
-        TeamPlan t{kw, teams, 0, team_slot(mask, kw)};
-        if (cap > fixed) t.stages = (int)std::min<size_t>(MAX_STAGES, (cap - fixed) / ((size_t)t.slot * teams));
+        TeamPlan t{kw, teams, 0, team_slot(mask, kw), 3};
+        for (int planes = four ? 4 : 3; planes >= 3 && t.stages < 1; planes--) {      // four digits where that leaves a stage
+            const size_t fixed = SM_X + x_bytes(K, planes);
+            if (cap > fixed) t.stages = (int)std::min<size_t>(MAX_STAGES, (cap - fixed) / ((size_t)t.slot * teams));
+            t.planes = planes;
+        }
         return t;
     };
     // Teams of 4 share one copy of the vector and pay the meeting at the end of 16 rows half as often, four of
@@ -377,7 +398,7 @@ void launch_teams(KqParams& p, cudaStream_t s) {
     constexpr int ctas = SM_WARPS / (TEAMS * KW);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(gemv_mma_kernel<MASK, KW, TEAMS>, (int)SMEM_CTA, configured);
-    const size_t smem = SM_X + x_bytes(p.K) + (size_t)p.stages * p.slot * TEAMS;
+    const size_t smem = SM_X + x_bytes(p.K, p.planes) + (size_t)p.stages * p.slot * TEAMS;
     const int places = num_sms() * (smem > SMEM_HALF ? 1 : ctas);
     launch_k(gemv_mma_kernel<MASK, KW, TEAMS>, dim3(p.total_groups < places ? p.total_groups : places), dim3(TEAMS * (KW + 1) * 32), smem, s, p);
     count_launch();
@@ -388,9 +409,11 @@ void launch_fmt(KqParams& p, cudaStream_t s) {
     int total = 0;
     for (int i = 0; i < p.n_mat; i++) { p.mat[i].groups = (p.mat[i].out + MROWS - 1) / MROWS; total += p.mat[i].groups; }
     p.total_groups = p.n_seg == 2 ? p.mat[0].groups : total;
-    const TeamPlan t = plan_teams(MASK, p.K, p.total_groups);
+    bool four = MASK == 16;
+    for (int i = 0; i < p.n_mat; i++) four = four || (MASK == 4 && (p.mat[i].row_pitch & 15));
+    const TeamPlan t = plan_teams(MASK, p.K, p.total_groups, four);
     NT_CHECK(t.stages >= 1, "gemv_kq: shared memory budget exceeded");
-    p.stages = t.stages; p.slot = t.slot;
+    p.stages = t.stages; p.slot = t.slot; p.planes = t.planes;
     if (t.kw == 4) launch_teams<MASK, 4, 4>(p, s);
     else if (t.kw == 16) launch_teams<MASK, 16, 1>(p, s);
     else if (t.teams == 2) launch_teams<MASK, 8, 2>(p, s);
@@ -419,11 +442,11 @@ bool gemv_kq_any_pitch(const GemvMat* mats, int n_mat, int K) {
         const size_t row = dtype_row_size(mats[i].dtype, K), pitch = mats[i].row_pitch ? mats[i].row_pitch : row;
         if ((reinterpret_cast<uintptr_t>(mats[i].W) & 15) || pitch < row || (pitch & (f == 2 ? 1 : 15))) return false;
     }
-    int plan[3];
+    int plan[4];
     return gemv_kq_plan(mats, n_mat, K, false, plan);
 }
 
-// plan: warps of a team, teams of a CTA, stages of a team's ring (the first matrix's where every matrix has a launch of its own)
+// plan: warps of a team, teams of a CTA, stages of a team's ring, digits of an activation (the first matrix's where every matrix has a launch of its own)
 bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, int* plan) {
     int mask = 0, groups = 0;
     for (int i = 0; i < n_mat; i++) { mask |= 1 << fmt_of(mats[i].dtype); groups += (mats[i].out + MROWS - 1) / MROWS; }
@@ -431,8 +454,10 @@ bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, int* plan)
         for (int i = n_mat - 1; i >= 0; i--) if (!gemv_kq_plan(&mats[i], 1, K, false, plan)) return false;
         return true;
     }
-    const TeamPlan t = plan_teams(mask, K, swiglu ? (mats[0].out + MROWS - 1) / MROWS : groups);
-    plan[0] = t.kw; plan[1] = t.teams; plan[2] = t.stages;
+    bool four = mask == 16;
+    for (int i = 0; i < n_mat; i++) four = four || (mask == 4 && ((mats[i].row_pitch ? mats[i].row_pitch : dtype_row_size(mats[i].dtype, K)) & 15));
+    const TeamPlan t = plan_teams(mask, K, swiglu ? (mats[0].out + MROWS - 1) / MROWS : groups, four);
+    plan[0] = t.kw; plan[1] = t.teams; plan[2] = t.stages; plan[3] = t.planes;
     return t.stages >= 1;
 }
 

@@ -2,11 +2,11 @@
 // super-blocks held in shared memory by the activation vector.
 //
 // Activations: x[e] = xs[e / 32] * T[e] with a 24-bit integer T = q1 * 65536 + q2 * 256 + q3 (balanced digits, s8 each; |x - xs * T| <= 2^-24 of
-// the 32-block's absmax).  mma.sync m16n8k32 with s32 accumulators multiplies the weights' 4/5/6/8-bit codes by the digits exactly: A = 16 rows
-// of codes straight from the block layout, B = the digits of 32 elements.  A vector fills only three of B's eight columns, so B carries TWO
-// groups of elements: the k positions 0-15 meet columns 0-2 with group "lo", positions 16-31 meet columns 4-6 with group "hi", zeros
+// the 32-block's absmax), or a 32-bit one of four digits, as good as F32, where a vector was multiplied in F32 before.  mma.sync m16n8k32 with s32 accumulators multiplies the weights' 4/5/6/8-bit codes by the digits exactly: A = 16 rows
+// of codes straight from the block layout, B = the digits of 32 elements.  A vector fills only three or four of B's eight columns, so B carries TWO
+// groups of elements: the k positions 0-15 meet columns 0-2 (3) with group "lo", positions 16-31 meet columns 4-6 (7) with group "hi", zeros
 // elsewhere.  The groups are what one byte of codes holds (low and high nibble, or the q1/q3 and q2/q4 quarters of Q6_K), so a masked word IS the
-// operand, and each lane's two sums belong to one group of one row: (q1, q2) in lanes t = 0, 2, q3 in lanes t = 1, 3 of a row's four.
+// operand, and each lane's two sums belong to one group of one row: (q1, q2) in lanes t = 0, 2, q3 (q3, q4) in lanes t = 1, 3 of a row's four.
 #pragma once
 #include "kernels_internal.h"
 #include "ring.cuh"
@@ -29,10 +29,10 @@ __host__ __device__ constexpr int stage_pitch(int fmt, int KW) { return (((stage
 // that a lane's words of four (Q4_K) consecutive products are one 16-byte load: element e = 64 c + 32 hi + 16 s + 4 t + i is byte i of word
 // [c >> 1][hi][t][(c & 1) * 2 + s].
 struct XView {
-    const uint8_t* b0;          // this lane's words for columns 0-2 (group lo): its plane, its t; a lane of another column points at 16 zero bytes
-    const uint8_t* b1;          //   and has the offset mask 0.  b1, m1: columns 4-6 (group hi)
+    const uint8_t* b0;          // this lane's words for columns 0-2 (3) (group lo): its plane, its t; a lane of another column points at 16 zero bytes
+    const uint8_t* b1;          //   and has the offset mask 0.  b1, m1: columns 4-6 (7) (group hi)
     uint32_t m0, m1;
-    const float* xs;            // [super-block][hi][4]: scale of element block 2 c + hi of the super-block, c = 0..3
+    const float* xs;            // [super-block][hi][4]: scale of element block 2 c + hi of the super-block, c = 0..3 (four digits: for this lane's pair)
     const float* sums;          // [super-block][8]: F32 sums of the 32-element blocks
 };
 __device__ __forceinline__ uint32_t xword_byte(int e) {
@@ -48,15 +48,16 @@ __device__ __forceinline__ float max_abs(float a, float b) {
     return __uint_as_float(u > v ? u : v);
 }
 // Scale and integers of a 32-block of activations whose largest magnitude is amax: x = xs * T.
-//   * below 2^-126 * 127 * 65536 (1e-31) the scale would be denormal and is flushed to 0, and its reciprocal overflows: 2^-126 then, and smaller integers;
+//   * below 2^-126 * TOP (1e-31, 2.5e-29 for four digits) the scale would be denormal and is flushed to 0, and its reciprocal overflows: 2^-126 then, and smaller integers;
 //   * a NaN is carried by the scale, so every row's product is one;
-//   * infinities are +-65537 beside zeros and the scale is infinite: both digits that a lane may hold (q1, q3) then multiply it by the same sum of codes, and
+//   * infinities are +-65537 beside zeros and the scale is infinite: the lanes of the upper and of the lower digits then multiply it by the same sum of codes, and
 //     the product is an infinity of the sum's sign, or NaN where the weight is 0.  (Q4_K and Q5_K subtract their offsets' infinity from it: NaN.)
 struct BlockScale {
     float inv, xs;
     bool infinite;
-    __device__ __forceinline__ explicit BlockScale(float amax) {
-        constexpr float TOP = 127.0f * 65536.0f, LEAST = TOP * 1.17549435e-38f;
+    static constexpr float TOP3 = 127.0f * 65536.0f, TOP4 = 127.0f * 16777216.0f;       // the largest integer of three and of four digits
+    __device__ __forceinline__ explicit BlockScale(float amax, float TOP = TOP3) {
+        const float LEAST = TOP * 1.17549435e-38f;
         inv = amax < LEAST ? 8.50705917e37f : __fdiv_rn(TOP, amax);
         xs = amax < LEAST ? 1.17549435e-38f : __fdiv_rn(amax, TOP);
         infinite = __float_as_uint(amax) == 0x7F800000u;
@@ -76,6 +77,19 @@ __device__ __forceinline__ void digits4(const int (&T)[4], uint32_t& q1, uint32_
     q3 = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
     q2 = __byte_perm(a, b, 0x7632) ^ 0x80808080u;
     q1 = __byte_perm(__byte_perm(u[0], u[1], 0x0062), __byte_perm(u[2], u[3], 0x0062), 0x5410) ^ 0x80808080u;
+}
+
+// the same for four digits, |T| <= 127 * 2^24
+__device__ __forceinline__ void digits4(const int (&T)[4], uint32_t& q1, uint32_t& q2, uint32_t& q3, uint32_t& q4) {
+    uint32_t u[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) u[i] = (uint32_t)T[i] + 0x80808080u;
+    const uint32_t a = __byte_perm(u[0], u[1], 0x5140), b = __byte_perm(u[2], u[3], 0x5140);      // bytes 0 0 1 1
+    const uint32_t c = __byte_perm(u[0], u[1], 0x7362), d = __byte_perm(u[2], u[3], 0x7362);      // bytes 2 2 3 3
+    q4 = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
+    q3 = __byte_perm(a, b, 0x7632) ^ 0x80808080u;
+    q2 = __byte_perm(c, d, 0x5410) ^ 0x80808080u;
+    q1 = __byte_perm(c, d, 0x7632) ^ 0x80808080u;
 }
 
 __device__ __forceinline__ float half_bits(uint32_t h16) { return __half2float(__ushort_as_half((unsigned short)h16)); }
@@ -110,10 +124,10 @@ __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
 __device__ __forceinline__ uint4 lds128(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ float sum_of(int hi, int lo) { return (float)(hi * 256 + lo); }
 
-// What lane t's sums are multiplied by at the end: digits (q1, q2) count 256 (lanes 0, 2), q3 1 / 256 (lanes 1, 3: sum_of took it for a q1);
-// codes that the operands carry x16 (Q4_K's high nibbles, Q4_0) or x4 (Q6_K).
-__device__ __forceinline__ float lane_factor(int fmt, int t) {
-    const float digit = (t & 1) ? 1.0f / 256.0f : 256.0f;
+// What lane t's sums are multiplied by at the end: digits (q1, q2) count 256 (lanes 0, 2), q3 1 / 256 (lanes 1, 3: sum_of took it for a q1), four digits 1
+// (the scales of lanes 0, 2 carry 65536); codes that the operands carry x16 (Q4_K's high nibbles, Q4_0) or x4 (Q6_K).
+__device__ __forceinline__ float lane_factor(int fmt, int t, int planes) {
+    const float digit = planes == 4 ? 1.0f : (t & 1) ? 1.0f / 256.0f : 256.0f;
     if (fmt == 0) return t >= 2 ? digit * (1.0f / 16.0f) : digit;
     return fmt == 2 ? digit * 0.25f : fmt == 4 ? digit * (1.0f / 16.0f) : digit;
 }

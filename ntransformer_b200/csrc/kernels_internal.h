@@ -60,12 +60,13 @@ struct GemvInput {
 };
 bool gemv_kq_supported(const GemvMat* mats, int n_mat, int K);      // 16-byte aligned rows
 bool gemv_kq_any_pitch(const GemvMat* mats, int n_mat, int K);      // what gemv_kq takes: 16-byte aligned matrices, any even pitch for Q6_K
-bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, int* plan);      // plan[3]: how a launch deals out an SM; false: nothing fits
+bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, int* plan);      // plan[4]: how a launch deals out an SM; false: nothing fits
 void gemv_kq(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpilogue ep, cudaStream_t s);
 void gemv_kq(const GemvMat* mats, int n_mat, int K, const void* xq, GemvEpilogue ep, cudaStream_t s);
 // gemv_xq.cu: the same product over a vector in xq form, with the persistent decode-step kernel's arithmetic (the decode step's unfused form); no PEER
 bool gemv_xq_supported(const GemvMat* mats, int n_mat, int K);
 void gemv_xq(const GemvMat* mats, int n_mat, int K, const void* xq, GemvEpilogue ep, cudaStream_t s);
+bool gemv_xq_faster(const GemvMat& m, int K);      // than gemv_kq over the F32 vector, its quantise launch included
 // gemv_kquant_q.cu: the quarter-block kernel (lane <-> 64 weights, up to 16 warps); false = shape not covered, nothing launched
 bool gemv_kq_quarter(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpilogue ep, const PeerOut* peer, cudaStream_t s);
 // epilogue GEMV_PEER: one matrix, rows == peer.hidden

@@ -13,7 +13,10 @@ static void gemv_dispatch(float* y, const void* W, const float* x, int out, int 
     if (out <= 0 || in <= 0) return;
     GemvMat m;
     m.W = W; m.y = y; m.out = out; m.dtype = dt; m.row_pitch = 0;
-    if (gemv_kq_any_pitch(&m, 1, in) && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {      // 16-byte loads of x
+    // 16-byte loads of x.  Q4_0, and Q6_K rows off 16 bytes, take F32 activations or integers as good (four digits); very long rows leave no room for those.
+    int plan[4];
+    const bool whole = dt == DType::Q4_0 || (dt == DType::Q6_K && (dtype_row_size(dt, in) & 15));
+    if (gemv_kq_any_pitch(&m, 1, in) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && !(whole && gemv_kq_plan(&m, 1, in, false, plan) && plan[3] < 4)) {
         GemvInput gi;                 // F32 activations are quantised inside the kernel prologue: one launch, no state
         gi.x = x;
         gemv_kq(&m, 1, in, gi, ep, s);

@@ -92,8 +92,8 @@ int    nt_b200_gemv_fused_f32(int n_mat, float* const* y, const void* const* W, 
                               const int* dtypes, int in_features, const float* x, const float* norm_w, float eps,
                               int epilogue, void* stream);
 /* How nt_b200_gemv_fused* would deal out an SM's shared memory for these matrices: plan[0] warps that share a row group, plan[1] such teams in a
- * CTA, plan[2] stages of a team's ring, plan[3] digits of an activation (3: 24 bits, 4: 32).  Returns 0, or < 0 where the matrix-instruction kernel does not take them.  Needs no GPU. */
-int    nt_b200_gemv_fused_plan(int n_mat, const int* out_features, const int* dtypes, int in_features, int epilogue, int* plan);
+ * CTA, plan[2] stages of a team's ring, plan[3] digits of an activation (3: 24 bits; 4: 32, what nt_b200_gemv asks for in front of Q4_0: whole).  Returns 0, or < 0 where the matrix-instruction kernel does not take them.  Needs no GPU. */
+int    nt_b200_gemv_fused_plan(int n_mat, const int* out_features, const int* dtypes, int in_features, int epilogue, int whole, int* plan);
 /* The same products for a few tokens: x [tokens, in_features], y of matrix i [tokens, out_features[i]]; quantises the tokens (norm_w: their RMSNorm) into
  * scratch (nt_b200_gemv_rows_bytes) and reads every weight once for 8 of them.  Returns 0, or < 0 when rejected (nothing launched). */
 size_t nt_b200_gemv_rows_bytes(int tokens, int K);
@@ -142,9 +142,9 @@ void   nt_b200_dequant_split(void* w_hi, void* w_lo, const void* W, int dtype, s
                              void* stream);
 /* Kernels that wait for copies or products of their own do so with a limit.  A wait that ran out sets a word (its launch's results are not to be used);
  * nt_model_sync answers cudaErrorLaunchTimeout for it, nt_model_forward and its like end with that error.  Returns the word, 0 = none; set >= 0 also
- * stores `set`.  nt_b200_wait_probe launches a wait of limit_ns for something that does not come (came_dev: device int, 0 afterwards). */
+ * stores `set`.  nt_b200_wait_probe launches a wait that asks `tries` times for something that does not come (came_dev: device int, 0 afterwards). */
 int    nt_b200_wait_status(int set);
-void   nt_b200_wait_probe(unsigned limit_ns, int* came_dev, void* stream);
+void   nt_b200_wait_probe(unsigned tries, int* came_dev, void* stream);
 unsigned long long nt_b200_launch_count(void);   /* kernels launched by this library so far */
 int    nt_b200_stream_sync(void* stream);        /* cudaStreamSynchronize; returns cudaError_t */
 const char* nt_b200_version(void);

@@ -9,7 +9,7 @@
 //   * several teams on an SM, so that the barriers of one do not idle it.  Weights depend on no kernel in flight: under programmatic launch a
 //     kernel's first stages are fetched while the one before still runs, as far as it leaves room.  The activation vector is read after
 //     griddepcontrol.wait, and the dependants are released after it;
-//   * the prologue quantises the F32 vector (24-bit integers for each 32-block, 32-bit ones in front of Q4_0 and Q6_K) into shared memory, with RMSNorm's
+//   * the prologue quantises the F32 vector (24-bit integers for each 32-block, 32-bit ones on request in front of Q4_0) into shared memory, with RMSNorm's
 //     gains multiplied in and its scalar applied to the results.
 // Up to 3 matrices of mixed formats share a launch (q / k / v of a Q4_K_M file; gate + up with SwiGLU).
 #include "kernels_internal.h"
@@ -49,52 +49,52 @@ struct KqParams {
     int total_groups;          // SWIGLU: groups of mat[0]
     int n_seg;                 // segments (matrices) per group: 2 for SWIGLU else 1
     int epilogue;
-    int stages, slot, planes;  // depth of a team's ring and bytes of a stage; digits of an activation
+    int stages, slot;          // depth of a team's ring and bytes of a stage
     unsigned* status;          // wait_status.cuh
     PeerOut peer;              // epilogue GEMV_PEER
 };
 
-// Shared memory: [barriers][zeros][norm][partials][digit planes][scales(, those of the upper digits)][sums][rings]
-constexpr size_t SM_ZERO = MAX_TEAMS * 16 * MAX_STAGES, SM_RED = SM_ZERO + 16, SM_PART = SM_RED + 112;
+// Shared memory: [barriers][zeros][norm][a wait has run out][partials][digit planes][scales(, those of the upper digits)][sums][rings]
+constexpr size_t SM_ZERO = MAX_TEAMS * 16 * MAX_STAGES, SM_RED = SM_ZERO + 16, SM_DEAD = SM_RED + 64, SM_PART = SM_RED + 112;
 constexpr size_t SM_X = (SM_PART + SM_WARPS * 2 * 2 * MROWS * 4 + 127) & ~(size_t)127;
 __host__ __device__ constexpr size_t x_bytes(int K, int planes) { return ((size_t)planes * (K + 64) + (size_t)(K / 32) * (planes == 4 ? 12 : 8) + 127) & ~(size_t)127; }
-// Launches whose vector may have four digits (of Q4_0, and of Q6_K rows off 16 bytes, where there is room): these were multiplied in F32, and three digits left
-// more error than that (Q4_0 4096 wide, one element in a hundred ten times the others: 1.6e-7 of the result, 1.2e-7 in F32; a hundred times: 2.0e-7).  The
-// digit's column of the product was zeros, so only the prologue and the vector's place in shared memory grow.
-__host__ __device__ constexpr bool four_digits(int mask) { return mask == 4 || mask == 16; }
+// Kernels whose vector may have four digits (GemvInput::whole, where there is room): launch_gemv multiplied Q4_0 in F32, and three digits left more error than that
+// (4096 wide, one element in a hundred ten times the others: 1.6e-7 of the result, 1.2e-7 in F32 and 1.0e-7 with four).  The digit's column of the product was
+// zeros, but the prologue and the vector's place in shared memory grow: decode step of four 8B layers in Q4_0 309 us with four, 302 with three.
+constexpr int WHOLE = 32;               // in a kernel's MASK, beside the format's bit
 
 // Eight consecutive elements (t8 = their index / 8), four threads to a 32-element block: digits, scale and sum into shared memory.
-template <bool FOUR>
-__device__ __forceinline__ void quantize8(const float (&x)[8], int t8, uint8_t* planes, int plane, int np, float* xs, float* xs_upper, float* sums) {
+template <int MASK>
+__device__ __forceinline__ void quantize8(const float (&x)[8], int t8, uint8_t* planes, int plane, float* xs, float* xs_upper, float* sums) {
+    constexpr bool FOUR = MASK & WHOLE;
     float amax = 0.f, s = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; i++) { amax = max_abs(amax, x[i]); s = __fadd_rn(s, x[i]); }
-    amax = max_abs(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-    amax = max_abs(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+    for (int i = 0; i < 8; i++) { amax = fmaxf(amax, fabsf(x[i])); s = __fadd_rn(s, x[i]); }
+    amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
     s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 1));
     s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 2));
-    const bool four = FOUR && np == 4;
-    const BlockScale scale(amax, four ? BlockScale::TOP4 : BlockScale::TOP3);
+    constexpr float top = FOUR ? BlockScale::TOP4 : BlockScale::TOP3;
+    const BlockScale scale(amax, top);
     uint32_t d[4][2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         int T[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) T[i] = scale(x[4 * h + i]);
-        if (four) digits4(T, d[0][h], d[1][h], d[2][h], d[3][h]);
+        scale.integers<(MASK & (4 | 16)) != 0>(x + 4 * h, T);
+        if (FOUR) digits4(T, d[0][h], d[1][h], d[2][h], d[3][h]);
         else { digits4(T, d[0][h], d[1][h], d[2][h]); d[3][h] = 0; }
     }
     const uint32_t o = xword_byte(t8 * 8);                      // the two words are neighbours in t: 16 bytes apart
 #pragma unroll
     for (int p = 0; p < (FOUR ? 4 : 3); p++) {
-        if (p == 3 && !four) break;
         *reinterpret_cast<uint32_t*>(planes + p * plane + o) = d[p][0];
         *reinterpret_cast<uint32_t*>(planes + p * plane + o + 16) = d[p][1];
     }
     if ((t8 & 3) == 0) {
         const int b = t8 >> 2;                                  // 32-element block: 2 c + hi of its super-block
-        xs[(b & ~7) + (b & 1) * 4 + ((b & 7) >> 1)] = scale.xs;
-        if (four) xs_upper[(b & ~7) + (b & 1) * 4 + ((b & 7) >> 1)] = scale.xs * 65536.0f;
+        const float f = BlockScale::of(amax, s, top);
+        xs[(b & ~7) + (b & 1) * 4 + ((b & 7) >> 1)] = f;
+        if (FOUR) xs_upper[(b & ~7) + (b & 1) * 4 + ((b & 7) >> 1)] = f * 65536.0f;
         sums[b] = s;
     }
 }
@@ -102,17 +102,16 @@ __device__ __forceinline__ void quantize8(const float (&x)[8], int t8, uint8_t* 
 // MASK: bit f set <=> matrices of format f may appear in this launch (mixed Q4_K_M projections share one launch).
 template <int MASK, int KW, int TEAMS>
 __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)) gemv_mma_kernel(const __grid_constant__ KqParams p) {
-    constexpr int CTHREADS = TEAMS * KW * 32;
+    constexpr int CTHREADS = TEAMS * KW * 32, np = MASK & WHOLE ? 4 : 3;      // np: digits of an activation
     extern __shared__ __align__(128) uint8_t smem[];
     const int team = (int)threadIdx.x / ((KW + 1) * 32);
     const int warp = (threadIdx.x >> 5) - team * (KW + 1), lane = threadIdx.x & 31;
     const int stages = p.stages, slot_bytes = p.slot;
     uint64_t* full = reinterpret_cast<uint64_t*>(smem) + team * 2 * MAX_STAGES;
     uint64_t* empty = full + MAX_STAGES;
-    const int np = four_digits(MASK) ? p.planes : 3;
     uint8_t* ring = smem + SM_X + x_bytes(p.K, np) + (size_t)team * stages * slot_bytes;
     const int u0 = (int)blockIdx.x + team * (int)gridDim.x, ustep = (int)gridDim.x * TEAMS;      // few groups: a team in each CTA first
-    auto format = [&](const KqMat& m) { return (MASK == 1) ? 0 : (MASK == 2) ? 1 : (MASK == 4) ? 2 : (MASK == 8) ? 3 : (MASK == 16) ? 4 : m.fmt; };
+    auto format = [&](const KqMat& m) { return (MASK == 1) ? 0 : (MASK == 2) ? 1 : (MASK == 4) ? 2 : (MASK == 8) ? 3 : (MASK & 16) ? 4 : m.fmt; };
     auto locate = [&](int u, int seg, int& mi, int& gl) {       // matrix and local group of group u
         if (p.n_seg == 2) { mi = seg; gl = u; return; }
         mi = 0; gl = u;
@@ -123,6 +122,8 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
         mbar_fence_init();
     }
     if (threadIdx.x < 4) reinterpret_cast<uint32_t*>(smem + SM_ZERO)[threadIdx.x] = 0;
+    const uint32_t dead = smem_u32(smem + SM_DEAD);
+    if (threadIdx.x == 4) set_word(dead, 0u);
     __syncthreads();
 
     if (warp == KW) {                                           // ---- producer: lane r < 16 copies row r of each stage ----
@@ -145,10 +146,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
                     if (e16 > end) e16 -= 16;
                     const uint32_t bytes = lane < MROWS && row < m.out ? (uint32_t)(e16 - b16) : 0u;
                     const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, bytes);
-                    if (!ahead && !wait_warp(empty + slot, parity, p.status)) {
-                        for (int s = 0; s < stages; s++) wait_phase(full + s, s < slot ? parity ^ 1u : parity, p.status);      // the copies in flight
-                        return;
-                    }
+                    if (!ahead) wait_cta(empty + slot, parity, dead);
                     uint8_t* dst = ring + (size_t)slot * slot_bytes + lane * stage_pitch(fmt, KW);
                     if (bytes && e16 < e)
                         for (const uint8_t* q = e16; q < e; q += 2) *reinterpret_cast<uint16_t*>(dst + (q - b16)) = *reinterpret_cast<const uint16_t*>(q);
@@ -163,6 +161,8 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
                 }
             }
         }
+        if (word_set(dead))                                     // given up: the copies in flight (parity counts for slots yet to be filled in this round)
+            for (int s = 0; s < (ahead ? slot : stages); s++) wait_flight(full + s, s < slot ? parity ^ 1u : parity);
         return;
     }
 
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
 #pragma unroll
                     for (int i = 0; i < 8; i++) { ss = fmaf(x[i], x[i], ss); x[i] = __fmul_rn(x[i], w[i]); }
                 }
-                quantize8<four_digits(MASK)>(x, t8, planes, plane, np, xs, xs_upper, sums);
+                quantize8<MASK>(x, t8, planes, plane, xs, xs_upper, sums);
             }
         }
         if (p.norm_w) {
@@ -219,19 +219,18 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
             for (int i = 0; i < 4; i++)
                 T[i] = 4 * ((((int)(a << (24 - 8 * i)) >> 24) * 128 + ((int)(b << (24 - 8 * i)) >> 24)) * 128 + ((int)(c << (24 - 8 * i)) >> 24));
             uint32_t d[4] = {};
-            const bool four = four_digits(MASK) && np == 4;
-            if (four) {
+            if (np == 4) {
 #pragma unroll
                 for (int i = 0; i < 4; i++) T[i] *= 256;
                 digits4(T, d[0], d[1], d[2], d[3]);
             } else digits4(T, d[0], d[1], d[2]);
 #pragma unroll
-            for (int q = 0; q < (four_digits(MASK) ? 4 : 3); q++) if (q < 3 || four) *reinterpret_cast<uint32_t*>(planes + q * plane + xword_byte(e)) = d[q];
+            for (int q = 0; q < np; q++) *reinterpret_cast<uint32_t*>(planes + q * plane + xword_byte(e)) = d[q];
             if ((e & 31) == 0) {
                 const int blk = e >> 5;
                 const int at = (blk & ~7) + (blk & 1) * 4 + ((blk & 7) >> 1);
-                xs[at] = (four ? 0.25f / 256.0f : 0.25f) * __ldg(fs + blk);
-                if (four) xs_upper[at] = 0.25f * 256.0f * __ldg(fs + blk);
+                xs[at] = (np == 4 ? 0.25f / 256.0f : 0.25f) * __ldg(fs + blk);
+                if (np == 4) xs_upper[at] = 0.25f * 256.0f * __ldg(fs + blk);
                 sums[blk] = __ldg(fs + K / 32 + 2 * blk) + __ldg(fs + K / 32 + 2 * blk + 1);
             }
         }
@@ -256,7 +255,6 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
     float* part = reinterpret_cast<float*>(smem + SM_PART) + team * 2 * 2 * KW * MROWS;      // [buffer][segment][K share][row]
     int slot = 0, buf = 0, turn = 0;
     uint32_t parity = 0;
-    bool sound = true;                                          // no wait of this lane has run out
     for (int u = u0; u < p.total_groups; u += ustep) {
         for (int seg = 0; seg < p.n_seg; seg++) {
             int mi, gl;
@@ -266,7 +264,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
             float acc[2] = {}, mins[2] = {};
             for (int b0 = 0; b0 < p.NB; b0 += sblocks) {
                 const int sbi = b0 + warp, left = p.NB - sbi;   // super-blocks from this warp's first on
-                wait_sound(full + slot, parity, p.status, sound);
+                wait_cta(full + slot, parity, dead);
                 if (left > 0) {
                     const uint8_t* sb = ring + (size_t)slot * slot_bytes + warp * blk;
                     const bool two = KW == 4 && left > KW;
@@ -278,7 +276,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
                     if ((MASK & 16) && fmt == 4) { if (two) tile_blocks<4, 2, KW>(sb, 0, sbi, xv, lane, acc, mins); else tile_blocks<4, 1, KW>(sb, 0, sbi, xv, lane, acc, mins); }
                 }
                 __syncwarp();
-                if (lane == 0 && sound) arrive(empty + slot);
+                if (lane == 0) arrive(empty + slot);
                 if (++slot == stages) { slot = 0; parity ^= 1u; }
             }
             const float f = lane_factor(fmt, t, np);
@@ -287,7 +285,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
             float v = (t & 1) ? v1 : v0;
             v += __shfl_xor_sync(0xFFFFFFFFu, (t & 1) ? v0 : v1, 1);
             v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
-            if (t < 2) part[((buf * 2 + seg) * KW + warp) * MROWS + g + 8 * t] = sound ? v : __uint_as_float(0x7FFFFFFFu);      // NaN
+            if (t < 2) part[((buf * 2 + seg) * KW + warp) * MROWS + g + 8 * t] = v;
         }
         named_sync<KW * 32>(2 + team);
         if (warp == turn && lane < MROWS) {                     // one warp in turn adds the shares and applies the epilogue
@@ -324,6 +322,14 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
         }
         buf ^= 1;
         if (++turn == KW) turn = 0;
+    }
+    if (word_set(dead)) {                                       // a wait ran out: no results
+        report(p.status);
+        for (int u = u0; u < p.total_groups && p.epilogue != GEMV_PEER; u += ustep) {
+            int mi, gl;
+            locate(u, 0, mi, gl);
+            if (lane < MROWS && gl * MROWS + lane < p.mat[mi].out) p.mat[mi].y[gl * MROWS + lane] = __uint_as_float(0x7FFFFFFFu);      // NaN
+        }
     }
 }
 
@@ -398,7 +404,7 @@ void launch_teams(KqParams& p, cudaStream_t s) {
     constexpr int ctas = SM_WARPS / (TEAMS * KW);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(gemv_mma_kernel<MASK, KW, TEAMS>, (int)SMEM_CTA, configured);
-    const size_t smem = SM_X + x_bytes(p.K, p.planes) + (size_t)p.stages * p.slot * TEAMS;
+    const size_t smem = SM_X + x_bytes(p.K, MASK & WHOLE ? 4 : 3) + (size_t)p.stages * p.slot * TEAMS;
     const int places = num_sms() * (smem > SMEM_HALF ? 1 : ctas);
     launch_k(gemv_mma_kernel<MASK, KW, TEAMS>, dim3(p.total_groups < places ? p.total_groups : places), dim3(TEAMS * (KW + 1) * 32), smem, s, p);
     count_launch();
@@ -406,14 +412,14 @@ void launch_teams(KqParams& p, cudaStream_t s) {
 
 template <int MASK>
 void launch_fmt(KqParams& p, cudaStream_t s) {
+    constexpr int formats = MASK & ~WHOLE;
     int total = 0;
     for (int i = 0; i < p.n_mat; i++) { p.mat[i].groups = (p.mat[i].out + MROWS - 1) / MROWS; total += p.mat[i].groups; }
     p.total_groups = p.n_seg == 2 ? p.mat[0].groups : total;
-    bool four = MASK == 16;
-    for (int i = 0; i < p.n_mat; i++) four = four || (MASK == 4 && (p.mat[i].row_pitch & 15));
-    const TeamPlan t = plan_teams(MASK, p.K, p.total_groups, four);
+    const TeamPlan t = plan_teams(formats, p.K, p.total_groups, MASK != formats);
     NT_CHECK(t.stages >= 1, "gemv_kq: shared memory budget exceeded");
-    p.stages = t.stages; p.slot = t.slot; p.planes = t.planes;
+    p.stages = t.stages; p.slot = t.slot;
+    if constexpr (MASK != formats) if (t.planes == 3) { launch_fmt<formats>(p, s); return; }
     if (t.kw == 4) launch_teams<MASK, 4, 4>(p, s);
     else if (t.kw == 16) launch_teams<MASK, 16, 1>(p, s);
     else if (t.teams == 2) launch_teams<MASK, 8, 2>(p, s);
@@ -443,20 +449,18 @@ bool gemv_kq_any_pitch(const GemvMat* mats, int n_mat, int K) {
         if ((reinterpret_cast<uintptr_t>(mats[i].W) & 15) || pitch < row || (pitch & (f == 2 ? 1 : 15))) return false;
     }
     int plan[4];
-    return gemv_kq_plan(mats, n_mat, K, false, plan);
+    return K <= 32768 || gemv_kq_plan(mats, n_mat, K, false, false, plan);      // up to there every form fits
 }
 
 // plan: warps of a team, teams of a CTA, stages of a team's ring, digits of an activation (the first matrix's where every matrix has a launch of its own)
-bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, int* plan) {
+bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, bool whole, int* plan) {
     int mask = 0, groups = 0;
     for (int i = 0; i < n_mat; i++) { mask |= 1 << fmt_of(mats[i].dtype); groups += (mats[i].out + MROWS - 1) / MROWS; }
     if (!one_launch(mask)) {
-        for (int i = n_mat - 1; i >= 0; i--) if (!gemv_kq_plan(&mats[i], 1, K, false, plan)) return false;
+        for (int i = n_mat - 1; i >= 0; i--) if (!gemv_kq_plan(&mats[i], 1, K, false, whole, plan)) return false;
         return true;
     }
-    bool four = mask == 16;
-    for (int i = 0; i < n_mat; i++) four = four || (mask == 4 && ((mats[i].row_pitch ? mats[i].row_pitch : dtype_row_size(mats[i].dtype, K)) & 15));
-    const TeamPlan t = plan_teams(mask, K, swiglu ? (mats[0].out + MROWS - 1) / MROWS : groups, four);
+    const TeamPlan t = plan_teams(mask, K, swiglu ? (mats[0].out + MROWS - 1) / MROWS : groups, whole && mask == 16);
     plan[0] = t.kw; plan[1] = t.teams; plan[2] = t.stages; plan[3] = t.planes;
     return t.stages >= 1;
 }
@@ -522,7 +526,7 @@ void gemv_kq(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpi
         case 4: launch_fmt<4>(p, s); break;
         case 3: launch_fmt<3>(p, s); break;
         case 8: launch_fmt<8>(p, s); break;
-        case 16: launch_fmt<16>(p, s); break;
+        case 16: if (in.whole) launch_fmt<16 | WHOLE>(p, s); else launch_fmt<16>(p, s); break;
         default: launch_fmt<5>(p, s); break;
     }
 }
@@ -535,6 +539,9 @@ void gemv_kq_peer(const GemvMat& mat, int K, const GemvInput& in, const PeerOut&
 }
 
 void gemv_kq(const GemvMat* mats, int n_mat, int K, const void* xq, GemvEpilogue ep, cudaStream_t s) {
+    bool longer = ep != GEMV_PEER;
+    for (int i = 0; i < n_mat; i++) longer = longer && gemv_xq_faster(mats[i], K);
+    if (longer) { gemv_xq(mats, n_mat, K, xq, ep, s); return; }
     GemvInput in;
     in.xq = xq;
     gemv_kq(mats, n_mat, K, in, ep, s);

@@ -42,29 +42,29 @@ __device__ __forceinline__ uint32_t xword_byte(int e) {
 __device__ __forceinline__ void arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory"); }
 template <int N> __device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 
-// The largest magnitude, a NaN where there is one (its bits lie above infinity's; fmaxf would drop it)
-__device__ __forceinline__ float max_abs(float a, float b) {
-    const uint32_t u = __float_as_uint(a) & 0x7FFFFFFFu, v = __float_as_uint(b) & 0x7FFFFFFFu;
-    return __uint_as_float(u > v ? u : v);
-}
-// Scale and integers of a 32-block of activations whose largest magnitude is amax: x = xs * T.
+// Scale and integers of a 32-block of activations: x = xs * T.  amax: the largest magnitude (fmaxf: without a NaN), s: the block's sum.
 //   * below 2^-126 * TOP (1e-31, 2.5e-29 for four digits) the scale would be denormal and is flushed to 0, and its reciprocal overflows: 2^-126 then, and smaller integers;
-//   * a NaN is carried by the scale, so every row's product is one;
+//   * a NaN (and infinities of both signs) shows in the sum and is carried by the scale, so every row's product is one;
 //   * infinities are +-65537 beside zeros and the scale is infinite: the lanes of the upper and of the lower digits then multiply it by the same sum of codes, and
-//     the product is an infinity of the sum's sign, or NaN where the weight is 0.  (Q4_K and Q5_K subtract their offsets' infinity from it: NaN.)
+//     the product is an infinity of the sum's sign, or NaN where the weight is 0.  (Only for Q4_0 and Q6_K, whose vectors were F32 once; NaN for the others.)
 struct BlockScale {
-    float inv, xs;
+    float inv;
     bool infinite;
     static constexpr float TOP3 = 127.0f * 65536.0f, TOP4 = 127.0f * 16777216.0f;       // the largest integer of three and of four digits
-    __device__ __forceinline__ explicit BlockScale(float amax, float TOP = TOP3) {
-        const float LEAST = TOP * 1.17549435e-38f;
-        inv = amax < LEAST ? 8.50705917e37f : __fdiv_rn(TOP, amax);
-        xs = amax < LEAST ? 1.17549435e-38f : __fdiv_rn(amax, TOP);
-        infinite = __float_as_uint(amax) == 0x7F800000u;
+    __device__ __forceinline__ BlockScale(float amax, float top) {
+        inv = amax < top * 1.17549435e-38f ? 8.50705917e37f : __fdiv_rn(top, amax);
+        infinite = amax > 3.40282347e38f;
     }
-    __device__ __forceinline__ int operator()(float x) const {
-        if (infinite) return (__float_as_uint(x) << 1) == 0xFF000000u ? (x > 0.f ? 65537 : -65537) : 0;
-        return __float2int_rn(__fmul_rn(x, inv));
+    static __device__ __forceinline__ float of(float amax, float s, float top) {       // xs
+        return s != s ? s : amax < top * 1.17549435e-38f ? 1.17549435e-38f : __fdiv_rn(amax, top);
+    }
+    template <bool INF>                   // INF: infinities count (Q4_0, Q6_K); otherwise they are zeros under their infinite scale, NaN
+    __device__ __forceinline__ void integers(const float* x, int (&T)[4]) const {
+#pragma unroll
+        for (int i = 0; i < 4; i++) T[i] = __float2int_rn(__fmul_rn(x[i], inv));
+        if (INF && infinite)
+#pragma unroll
+            for (int i = 0; i < 4; i++) T[i] = fabsf(x[i]) > 3.40282347e38f ? (x[i] > 0.f ? 65537 : -65537) : 0;
     }
 };
 

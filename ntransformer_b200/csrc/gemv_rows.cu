@@ -60,20 +60,19 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(uint8_t* __restrict_
             for (int i = 0; i < 8; i++) v[i] = __fmul_rn(v[i], __ldg(norm_w + 8 * t8 + i));
         float amax = 0.f, s = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; i++) { amax = max_abs(amax, v[i]); s = __fadd_rn(s, v[i]); }
-        amax = max_abs(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-        amax = max_abs(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+        for (int i = 0; i < 8; i++) { amax = fmaxf(amax, fabsf(v[i])); s = __fadd_rn(s, v[i]); }
+        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
         s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 1));
         s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, 2));
-        const BlockScale scale(live ? amax : 0.f);
+        const BlockScale scale(amax, BlockScale::TOP3);
         const int e = 8 * t8, sub = (e >> 5) & 7, seg = (e >> 4) & 1, t = (e >> 2) & 3, odd = sub & 1;
         uint8_t* blk = xr + ((size_t)pass * NB + (e >> 8)) * XB;
         uint8_t* pair = blk + (sub >> 1) * 1536;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             int T[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) T[i] = live ? scale(v[4 * h + i]) : 0;
+            scale.integers<false>(v + 4 * h, T);
             uint32_t q1, q2, q3;
             digits4(T, q1, q2, q3);
             const int c = 2 * (tk & 3), w12 = ((tk >> 2) * 2 + seg) * 4, u12 = odd ? 1024 : 0;
@@ -83,7 +82,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(uint8_t* __restrict_
         }
         if ((t8 & 3) == 0) {
             float* f = reinterpret_cast<float*>(blk + XB_DIGITS);
-            f[tk * 8 + sub] = live ? __fmul_rn(scale.xs, rms) : 0.f;
+            f[tk * 8 + sub] = live ? __fmul_rn(BlockScale::of(amax, s, BlockScale::TOP3), rms) : 0.f;
             f[64 + tk * 8 + sub] = live ? __fmul_rn(s, rms) : 0.f;
         }
     }
@@ -299,7 +298,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
                     const uint32_t bytes = row < m.out ? (uint32_t)(e16 - b16) : 0u;
                     const uint32_t total = __reduce_add_sync(0xFFFFFFFFu, bytes) + (uint32_t)(nb * XB);
                     if (!wait_warp(empty + slot, parity, p.status)) {
-                        for (int s = 0; s < min(filled, p.stages); s++) wait_phase(full + s, s < slot ? parity ^ 1u : parity, p.status);      // the copies in flight
+                        for (int s = 0; s < min(filled, p.stages); s++) wait_flight(full + s, s < slot ? parity ^ 1u : parity);      // the copies in flight
                         return;
                     }
                     filled = min(filled + 1, p.stages);
@@ -322,7 +321,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
     float* part = reinterpret_cast<float*>(smem + R_PART) + tile * RKW * 128;       // + segment * RTILES * RKW * 128
     int slot = 0, turn = 0;
     uint32_t parity = 0;
-    bool sound = true;                                             // no wait of this lane has run out
+    uint32_t tries = WAIT_TRIES;                                             // 0: a wait of this lane has run out
     for (int u = blockIdx.x; u < p.total_units; u += gridDim.x) {
         for (int seg = 0; seg < p.n_seg; seg++) {
             int mi, gl, pass;
@@ -331,7 +330,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
             const int fmt = format(m), row = gl * RGROUP + tile * MROWS;
             float a12[2][2] = {}, a3[2][2] = {}, mins[2][2] = {};
             for (int b0 = 0; b0 < p.NB; b0 += RKW) {
-                wait_sound(full + slot, parity, p.status, sound);
+                wait_phase(full + slot, parity, p.status, tries);
                 if (b0 + kw < p.NB && row < m.out) {
                     const uint8_t* st = ring + (size_t)slot * p.slot;
                     const uint8_t* sb = st + tile * MROWS * stage_pitch(fmt, RKW) + kw * fmt_bytes(fmt);
@@ -343,7 +342,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
                     if ((MASK & 16) && fmt == 4) rows_block<4>(sb, 0, xb, lane, a12, a3, mins);
                 }
                 __syncwarp();
-                if (lane == 0 && sound) arrive(empty + slot);
+                if (lane == 0 && tries) arrive(empty + slot);
                 if (++slot == p.stages) { slot = 0; parity ^= 1u; }
             }
             // (q1, q2) counted 1 / 256 of their weight; codes were carried x4 (Q6_K) or x16 (Q4_0)
@@ -355,7 +354,7 @@ __global__ void __launch_bounds__((RWARPS + 1) * 32, 1) gemv_rows_kernel(const _
                     const int src = (lane & ~3) + 2 * j + (t >> 1);
                     const float u0 = __shfl_sync(0xFFFFFFFFu, a3[0][r], src), u1 = __shfl_sync(0xFFFFFFFFu, a3[1][r], src);
                     const float v = fmaf(a12[j][r], f12, fmaf((t & 1) ? u1 : u0, f3, -mins[j][r]));
-                    part[(seg * RTILES * RKW + kw) * 128 + (4 * j + t) * MROWS + g + 8 * r] = sound ? v : __uint_as_float(0x7FFFFFFFu);      // NaN
+                    part[(seg * RTILES * RKW + kw) * 128 + (4 * j + t) * MROWS + g + 8 * r] = tries ? v : __uint_as_float(0x7FFFFFFFu);      // NaN
                 }
         }
         named_sync<RKW * 32>(1 + tile);

@@ -1,13 +1,13 @@
 // gemv_xq.cu — GEMV over GGUF Q4_K / Q5_K / Q6_K / Q8_0 / Q4_0 blocks times an activation vector in pre-quantised form (kernels_internal.h "xq").
 //
-// Replaces reference kernels K2-K5 (src/cuda/gemm.cu:96-470) where the vector is quantised by a launch of its own: the decode step's unfused form.  Its
+// Replaces reference kernels K2-K5 (src/cuda/gemm.cu:96-470) where the vector is quantised by a launch of its own: the decode step's unfused form, and long rows.  Its
 // arithmetic, lane by lane and sum by sum, is the persistent decode-step kernel's GEMV phase (gemv_kq_device.cuh, engine/decode_megakernel.cu), so that
 // the two forms of a decoded token can be compared: 22-bit activations, IDP.4A products, one F32 scale for 16 or 32 weights, chunks added in order.
 //   * chunk-stationary warps: a row is cut into chunks of 16 super-blocks (4096 weights); warp w of a CTA owns chunk (w % NC) for the whole kernel, lane <->
 //     one 128-weight half super-block, whose slice of the vector sits in registers;
 //   * each warp streams its rows through a private ring of bulk copies: one stage = 4 rows x 16 super-blocks;
 //   * the NC warps that hold the chunks of a row-group meet once per row-group and one of them adds the partial sums in a fixed order.
-// Bound by instruction issue (2.0 instructions a weight; 57344 x 8192 in Q4_K 53 us): gemv_kquant.cu is faster and is what every other caller takes.
+// Bound by instruction issue (2.0 instructions a weight; 57344 x 8192 in Q4_K 53 us): gemv_kquant.cu is faster but for long rows (gemv_xq_faster).
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "wait_status.cuh"
@@ -144,14 +144,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS <= 6 ? 2 : 1) gemv_xq_kernel
 
     int slot = 0;
     uint32_t parity = 0;
-    bool sound = true;                                       // no wait of this lane has run out
+    uint32_t tries = WAIT_TRIES;                                       // 0: a wait of this lane has run out
     for (int round = 0; round < n_rounds; round++) {
         int g, row_sub, nr;
         const bool live = slot_of(round, g, row_sub, nr);
         float res[2] = {0.f, 0.f};
         for (int seg = 0; seg < n_seg; seg++) {
             float acc[RG] = {0.f, 0.f, 0.f, 0.f};
-            wait_sound(bars + slot, parity, p.status, sound);
+            wait_phase(bars + slot, parity, p.status, tries);
             if (live && blk < nbc) {
                 int mi, gl;
                 locate(g, seg, mi, gl);
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS <= 6 ? 2 : 1) gemv_xq_kernel
                 }
             }
             __syncwarp();
-            if (lane == 0 && issued < n_stages_total && sound) issue_next(slot);
+            if (lane == 0 && issued < n_stages_total && tries) issue_next(slot);
             issued++;
             if (++slot == stages) { slot = 0; parity ^= 1u; }
             res[seg] = reduce4(acc, lane);
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS <= 6 ? 2 : 1) gemv_xq_kernel
         const int buf = round & 1;
         if (live && (lane & 7) == 0) {
             const int r = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
-            partial[buf][warp][0][r] = sound ? res[0] : __uint_as_float(0x7FFFFFFFu);      // NaN
+            partial[buf][warp][0][r] = tries ? res[0] : __uint_as_float(0x7FFFFFFFu);      // NaN
             partial[buf][warp][1][r] = res[1];
         }
         __syncthreads();
@@ -274,6 +274,11 @@ bool gemv_xq_supported(const GemvMat* mats, int n_mat, int K) {
     }
     return true;
 }
+
+// Long rows: beside the vector (3.25 bytes an element) gemv_kquant.cu has one or two ring stages to a team, this kernel all of shared memory.  Decode steps, the
+// down projection here against there (its quantise launch included): 70B shapes, 28672 wide, three layers in Q8_0 756 us against 807, four in Q4_K_M 759 / 765,
+// three in Q6_K 764 / 766; in Q4_K 49152 wide, three layers, 673 / 808; 24576 488 / 507; 20480 428 / 433; 18944 326 / 325; 14336 (8B, six layers) 468 / 442.
+bool gemv_xq_faster(const GemvMat& m, int K) { return K >= 20480 && gemv_xq_supported(&m, 1, K); }
 
 void gemv_xq(const GemvMat* mats, int n_mat, int K, const void* xq, GemvEpilogue ep, cudaStream_t s) {
     NT_CHECK(gemv_xq_supported(mats, n_mat, K) && ep != GEMV_PEER, "gemv_xq: unsupported shape/dtype/alignment");

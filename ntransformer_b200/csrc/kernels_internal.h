@@ -57,10 +57,11 @@ struct GemvInput {
     const float* norm_w = nullptr;
     float eps = 0.f;
     const PeerOut* peer = nullptr;     // epilogue GEMV_PEER only
+    bool whole = false;                // Q4_0 alone: 32-bit integers of the activations, as good as F32, where there is room
 };
 bool gemv_kq_supported(const GemvMat* mats, int n_mat, int K);      // 16-byte aligned rows
 bool gemv_kq_any_pitch(const GemvMat* mats, int n_mat, int K);      // what gemv_kq takes: 16-byte aligned matrices, any even pitch for Q6_K
-bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, int* plan);      // plan[4]: how a launch deals out an SM; false: nothing fits
+bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, bool whole, int* plan);      // plan[4]: how a launch deals out an SM; false: nothing fits
 void gemv_kq(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpilogue ep, cudaStream_t s);
 void gemv_kq(const GemvMat* mats, int n_mat, int K, const void* xq, GemvEpilogue ep, cudaStream_t s);
 // gemv_xq.cu: the same product over a vector in xq form, with the persistent decode-step kernel's arithmetic (the decode step's unfused form); no PEER

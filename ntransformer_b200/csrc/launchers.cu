@@ -13,12 +13,13 @@ static void gemv_dispatch(float* y, const void* W, const float* x, int out, int 
     if (out <= 0 || in <= 0) return;
     GemvMat m;
     m.W = W; m.y = y; m.out = out; m.dtype = dt; m.row_pitch = 0;
-    // 16-byte loads of x.  Q4_0, and Q6_K rows off 16 bytes, take F32 activations or integers as good (four digits); very long rows leave no room for those.
+    // 16-byte loads of x.  Q4_0 takes F32 activations or integers as good (four digits); very long rows leave no room for those.
     int plan[4];
-    const bool whole = dt == DType::Q4_0 || (dt == DType::Q6_K && (dtype_row_size(dt, in) & 15));
-    if (gemv_kq_any_pitch(&m, 1, in) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && !(whole && gemv_kq_plan(&m, 1, in, false, plan) && plan[3] < 4)) {
+    const bool whole = dt == DType::Q4_0;
+    if (gemv_kq_any_pitch(&m, 1, in) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && !(whole && gemv_kq_plan(&m, 1, in, false, true, plan) && plan[3] < 4)) {
         GemvInput gi;                 // F32 activations are quantised inside the kernel prologue: one launch, no state
         gi.x = x;
+        gi.whole = whole;
         gemv_kq(&m, 1, in, gi, ep, s);
     } else {
         gemv_generic(y, W, x, out, in, dt, 0, ep, s);
@@ -139,12 +140,12 @@ int nt_b200_gemv_fused_f32(int n_mat, float* const* y, const void* const* W, con
     nt::b200::gemv_kq(m, n_mat, in_features, in, (nt::b200::GemvEpilogue)epilogue, static_cast<cudaStream_t>(stream));
     return 0;
 }
-int nt_b200_gemv_fused_plan(int n_mat, const int* out_features, const int* dtypes, int in_features, int epilogue, int* plan) {
+int nt_b200_gemv_fused_plan(int n_mat, const int* out_features, const int* dtypes, int in_features, int epilogue, int whole, int* plan) {
     if (n_mat < 1 || n_mat > 3) return -1;
     nt::b200::GemvMat m[3];
     for (int i = 0; i < n_mat; i++) { m[i].W = nullptr; m[i].y = nullptr; m[i].out = out_features[i]; m[i].dtype = (DType)dtypes[i]; m[i].row_pitch = 0; }
     if (!nt::b200::gemv_kq_any_pitch(m, n_mat, in_features)) return -2;
-    return nt::b200::gemv_kq_plan(m, n_mat, in_features, epilogue == 2, plan) ? 0 : -2;
+    return nt::b200::gemv_kq_plan(m, n_mat, in_features, epilogue == 2, whole != 0, plan) ? 0 : -2;
 }
 size_t nt_b200_gemv_rows_bytes(int tokens, int K) { return nt::b200::gemv_rows_bytes(tokens, K); }
 int nt_b200_gemv_rows(int n_mat, float* const* y, const void* const* W, const int* out_features, const int* dtypes, int in_features, const float* x,

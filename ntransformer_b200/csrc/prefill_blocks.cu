@@ -196,13 +196,14 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
     if (warp == 0) {
         if (lane == 0) {                                           // ---- tokens by TMA ----
             uint32_t st = 0, par = 1, filled = 0;
-            bool sound = true;                                     // no wait of this thread has run out
-            for (int tile = blockIdx.x; tile < p.n_tiles && sound; tile += gridDim.x) {
+            uint32_t tries = WAIT_TRIES;                                     // 0: a wait of this thread has run out
+            for (int tile = blockIdx.x; tile < p.n_tiles && tries; tile += gridDim.x) {
                 int mi, row0, t0;
                 place(tile, mi, row0, t0);
                 for (int kb = 0; kb < num_kb; kb++) {
-                    if (!(sound = wait_phase(b_empty + st, par, p.status))) {
-                        for (uint32_t s = 0; s < filled; s++) wait_phase(b_full + s, s < st ? par ^ 1u : par, p.status);      // the copies in flight
+                    wait_phase(b_empty + st, par, p.status, tries);
+                    if (!tries) {
+                        for (uint32_t s = 0; s < filled; s++) wait_flight(b_full + s, s < st ? par ^ 1u : par);      // the copies in flight
                         break;
                     }
                     filled = min(filled + 1, (uint32_t)p.b_stages);
@@ -222,20 +223,20 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
         const uint64_t desc0 = make_desc(smem), lo_step = (uint64_t)(b_tile >> 4), stage_step = (uint64_t)(b_stage >> 4);
         uint32_t bs = 0, bpar = 0, as = 0, apar = 0, db = 0, dpar = 1;
-        bool sound = true;                                         // no wait of this lane has run out
+        uint32_t tries = WAIT_TRIES;                                         // 0: a wait of this lane has run out
         int last = -1;                                             // stage and parity of the last commit
         for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x)
             for (int kc = 0; kc < n_kc; kc++) {
-                wait_sound(d_empty + db, dpar, p.status, sound);
+                wait_phase(d_empty + db, dpar, p.status, tries);
                 const uint32_t d = tm + D_COL + db * NT;
                 const int kb0 = kc * p.kc, kb1 = min(num_kb, kb0 + p.kc);
                 for (int kb = kb0; kb < kb1; kb++) {
-                    wait_sound(b_full + bs, bpar, p.status, sound);
-                    wait_sound(a_full + as, apar, p.status, sound);
+                    wait_phase(b_full + bs, bpar, p.status, tries);
+                    wait_phase(a_full + as, apar, p.status, tries);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t bh = desc0 + bs * stage_step, bl = bh + lo_step;
                     const uint32_t ah = tm + as * A_COLS, al = ah + 32;
-                    if (leader && sound) {
+                    if (leader && tries) {
 #pragma unroll
                         for (int k = 0; k < 4; k++) umma_ts(d, al + 8 * k, bh + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);      // the small products first
 #pragma unroll
@@ -253,18 +254,18 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                 }
                 if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
             }
-        if (!sound && last >= 0) wait_phase(a_empty + (last >> 1), last & 1, p.status);      // given up: the products in flight
+        if (!tries && last >= 0) wait_flight(a_empty + (last >> 1), last & 1);      // given up: the products in flight
     } else if (warp < 6) {                                         // ---- epilogue: a lane is a row of W, so a warp stores 128 contiguous bytes for each token ----
         const int quarter = warp & 3;
         uint32_t db = 0, dpar = 0;
-        bool sound = true;
+        uint32_t tries = WAIT_TRIES;
         for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
             int mi, row0, t0;
             place(tile, mi, row0, t0);
             const BlkMat& m = p.mat[mi];
             const int row = row0 + quarter * 32 + lane, live = min(NT, p.T - t0);
             for (int kc = 0; kc < n_kc; kc++) {
-                wait_sound(d_full + db, dpar, p.status, sound);
+                wait_phase(d_full + db, dpar, p.status, tries);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem + ((uint32_t)(quarter * 32) << 16) + D_COL + db * NT;
                 const bool add = p.add || kc > 0;
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     uint32_t v[32];
                     tmem_ld32(d + (uint32_t)n, v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (row < m.rows && sound) {
+                    if (row < m.rows && tries) {
                         // adds go to the memory's side (this lane is the element's only writer, so their order is fixed): nothing is waited for
 #pragma unroll
                         for (int j = 0; j < 32; j++) {
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0 && sound) mbar_arrive(d_empty + db);
+                if (lane == 0 && tries) mbar_arrive(d_empty + db);
                 if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
             }
         }
@@ -317,12 +318,12 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         };
         for (int i = 0; i < depth - 1; i++) copy_next();
         int slot = 0, pending = -1;
-        bool sound = true;
+        uint32_t tries = WAIT_TRIES;
         auto stored = [&](int stage) {
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0 && sound) mbar_arrive(a_full + stage);
+            if (lane == 0 && tries) mbar_arrive(a_full + stage);
         };
         for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
             int mi, row0, t0;
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     }
                     // the stores of the k-block before had this one's arithmetic to arrive in
                     if (pending >= 0) stored(pending);
-                    wait_sound(a_empty + as, apar, p.status, sound);
+                    wait_phase(a_empty + as, apar, p.status, tries);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t a = tmem + ((uint32_t)(quarter * 32) << 16) + as * A_COLS + hf * 16;
                     tmem_st16(a, hi);

@@ -24,12 +24,12 @@ struct Word {
 Word& word() { static Word w; return w; }
 
 // waits for a phase that nothing completes
-__global__ void wait_probe_kernel(unsigned* status, unsigned limit_ns, int* came) {
+__global__ void wait_probe_kernel(unsigned* status, unsigned tries, int* came) {
     __shared__ uint64_t bar;
     if (threadIdx.x == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
     __syncthreads();
-    const bool ok = wait_phase(&bar, 0, status, limit_ns);
-    if (threadIdx.x == 0) *came = ok;
+    wait_phase(&bar, 0, status, tries);
+    if (threadIdx.x == 0) *came = tries != 0;
 }
 
 }  // namespace
@@ -46,8 +46,8 @@ int nt_b200_wait_status(int set) {
     if (set >= 0) *w = (unsigned)set;
     return was;
 }
-void nt_b200_wait_probe(unsigned limit_ns, int* came_dev, void* stream) {
-    nt::b200::wait_probe_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(nt::b200::wait_status(), limit_ns, came_dev);
+void nt_b200_wait_probe(unsigned tries, int* came_dev, void* stream) {
+    nt::b200::wait_probe_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(nt::b200::wait_status(), tries, came_dev);
     nt::b200::count_launch();
 }
 }

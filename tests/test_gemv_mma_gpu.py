@@ -101,7 +101,7 @@ def test_nan_infinity_and_the_smallest_numbers(dt):
             inf = x.copy()
             inf[at] = v
             got = run(inf)
-            if dt in (DType.Q4_K_M, DType.Q5_K):          # the offset's infinity is taken off the codes': not a number
+            if dt not in (DType.Q4_0, DType.Q6_K):         # an infinite scale over zeros, or the offset's infinity taken off the codes': not a number
                 assert not np.isfinite(got).any()
             else:                                          # as in 64 bits: the infinity of the weight's sign, not a number where the weight is 0
                 with np.errstate(invalid="ignore"):

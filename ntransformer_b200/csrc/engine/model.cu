@@ -400,7 +400,9 @@ bool Model::finalize() {
     attn_tickets_ = dmalloc<unsigned>((size_t)std::max(1, nh_l_));
     NT_CUDA_CHECK(cudaMemset(attn_tickets_, 0, (size_t)std::max(1, nh_l_) * sizeof(unsigned)));
     if (const char* fz = getenv("NT_B200_FUSE")) fuse_mask_ = atoi(fz);
-    if (!(fuse_mask_ & 1)) xq_ = dmalloc<uint8_t>(xq_bytes(std::max(std::max(hidden, inter_l_), nh_l_ * hd)));
+    bool xq = !(fuse_mask_ & 1);
+    for (const LayerWeights& L : layers_) xq = xq || down_over_xq(L.down);
+    if (xq) xq_ = dmalloc<uint8_t>(xq_bytes(std::max(std::max(hidden, inter_l_), nh_l_ * hd)));
     const size_t kv_elems = (size_t)cfg_.n_layers * max_seq * nkv_l_ * hd;     // F16 [L, max_seq, n_kv, hd], transformer.cpp:340-346
     kc_ = dmalloc<uint16_t>(kv_elems);
     vc_ = dmalloc<uint16_t>(kv_elems);
@@ -490,7 +492,7 @@ void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float
     const int K = ws[0]->cols;
     for (int i = 0; i < n; i++) { mats[i].W = ws[i]->ptr; mats[i].y = ys[i]; mats[i].out = ws[i]->rows; mats[i].dtype = ws[i]->dtype; mats[i].row_pitch = ws[i]->pitch; }
     GemvInput in;
-    if (xq_ && gemv_xq_supported(mats, n, K)) {            // the unfused form: norm and quantiser as a launch of their own
+    if (!(fuse_mask_ & 1) && gemv_xq_supported(mats, n, K)) {      // the unfused form: norm and quantiser as a launch of their own
         if (norm_w) rmsnorm_xq(nullptr, xq_, x, norm_w, K, cfg_.norm_eps, s);
         else quantize_x(x, xq_, K, s);
         gemv_xq(mats, n, K, xq_, ep, s);
@@ -522,6 +524,12 @@ void Model::reduce_residual(float* partial, cudaStream_t s) {
     // (the unfused path; with the peer exchange mapped the short chain sums through NVLink stores instead, see step_body)
     comm_->all_reduce_sum(partial, (size_t)cfg_.hidden_size, s);
     add_inplace(hidden_, partial, cfg_.hidden_size, s);
+}
+
+// Very long rows: the vector takes the shared memory that gemv_kquant.cu's rings live on, so a quantise launch and gemv_xq.cu are faster.
+bool Model::down_over_xq(const Weight& w) const {
+    GemvMat m; m.W = w.ptr; m.y = nullptr; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch;
+    return tp_size_ == 1 && !cfg_.layer_spec() && gemv_xq_faster(m, w.cols);
 }
 
 // The short launch chain needs every projection on gemv_kquant.cu (its prologue carries the norm + quantiser).
@@ -620,7 +628,8 @@ void Model::step_body(cudaStream_t s) {
             gemv_kq(m2, 2, hidden, in, GEMV_SWIGLU, s);
             GemvMat md = mat(L.down, hidden_);
             GemvInput ind; ind.x = act_;
-            if (tp_size_ == 1) gemv_kq(&md, 1, inter_l_, ind, GEMV_ADD, s);
+            if (down_over_xq(L.down)) { quantize_x(act_, xq_, inter_l_, s); gemv_xq(&md, 1, inter_l_, xq_, GEMV_ADD, s); }
+            else if (tp_size_ == 1) gemv_kq(&md, 1, inter_l_, ind, GEMV_ADD, s);
             else { gemv_kq_peer(md, inter_l_, ind, xchg_->out(), s); xchg_->reduce_residual(hidden_, s); }
             continue;
         }

@@ -289,6 +289,7 @@ private:
     void run_step_mega(bool with_head);
     void step_body(cudaStream_t s);      // embedding + all layers for the token/position in step_dev_
     void step_head(cudaStream_t s, bool from_chain = false);   // final norm + LM head (+ all-gather under TP); from_chain: norm + quantiser in the GEMV prologue
+    bool down_over_xq(const Weight& w) const;   // the decode step's down projection over a vector quantised by a launch of its own
     bool chain_ok() const;               // every projection on gemv_kquant.cu: the fused launch chain applies
     void run_step(bool with_head);
     void matvec(const Weight* const* ws, float* const* ys, int n, const float* x, const float* norm_w, GemvEpilogue ep,
@@ -321,7 +322,7 @@ private:
     float *act_ = nullptr, *up_ = nullptr, *part_ = nullptr, *logits_ = nullptr, *logits_l_ = nullptr, *attn_scratch_ = nullptr;
     unsigned* attn_tickets_ = nullptr;   // last-arriver tickets of the one-launch attention (zero between launches)
     int fuse_mask_ = 1;                  // bit 0: norm + quantiser in the GEMV prologues (default), bit 1: one-launch attention (opt-in: measured slower, profiles/r02_*), bit 2: RoPE + KV write inside the decode kernel, merge separate (NT_B200_FUSE)
-    void* xq_ = nullptr;                 // pre-quantised activations of the unfused form (fuse_mask_ bit 0 off)
+    void* xq_ = nullptr;                 // pre-quantised activations (fuse_mask_ bit 0 off, or down_over_xq)
     void *kc_ = nullptr, *vc_ = nullptr;
     int* step_dev_ = nullptr;            // [0] token, [1] position, [2] the token before it (sequence state of the pair embedding)
     int* argmax_dev_ = nullptr;

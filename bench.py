@@ -104,8 +104,8 @@ class ClockSampler:
                 "reasons": sorted(reasons)}
 
 
-def ncu_traffic(workload: str, world: int, name: str = "r01_gemv_gateup_ncu.json"):
-    """dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the committed ncu --set full
+def ncu_traffic(workload: str, world: int, name: str = "gemv_mma_gateup_ncu.json"):
+    """dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the committed ncu
     capture of the same shape (profiles/<name>); None when no capture exists for this workload."""
     p = ROOT / "profiles" / name
     if world != 1 or not p.exists():
@@ -231,10 +231,10 @@ def run_prefill(args, rank, world):
                 "note": "algorithmic flops 2MNK; the kernel issues 2x that (F32 activations split into F16 hi+lo to keep parity <= 1e-3)",
                 "step_achieved": round(step_tf, 1), "step_frac": round(step_tf / peak, 4)}
     else:
-        roof = {"bound": "tensor", "kernel": "whole prefill step (gemm_f16_tc_kernel over dequantised F16 hi/lo weights, 2 launches per matrix)",
+        roof = {"bound": "tensor", "kernel": "whole prefill step (gemm_blocks_kernel: blocks expanded to F16 hi + lo on the way into tensor memory)",
                 "achieved": round(step_tf, 1), "peak": peak, "unit": "TFLOP/s", "frac": round(step_tf / peak, 4), "traffic": None,
                 "peak_source": peak_src,
-                "note": "algorithmic flops; the path issues 4x that (activations and dequantised weights both as F16 hi+lo)",
+                "note": "algorithmic flops; the path issues 3x that (activations and expanded weights both as F16 hi+lo, lo.lo left out)",
                 "step_achieved": round(step_tf, 1), "step_frac": round(step_tf / peak, 4)}
     line = {
         "metric": "prefill_tok_s", "value": round(tok_s, 1), "unit": "tok/s", "n_gpus": 1, "steps": steps, "warmup": args.warmup,

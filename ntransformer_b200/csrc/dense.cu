@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_d
         __syncthreads();
         for (int i = threadIdx.x; i < K; i += DV_WARPS * 32) { float* d = xs + staged_at(i, half); *d = *d * inv_g[i / per] * norm_w[i]; }
     } else if (norm_w) {
-        // RMS norm of the staged vector: every CTA sums the squares in the same order, so all CTAs (and every launch that reads the
-        // same x) derive the bit-identical normalised vector
+        // RMS norm of the staged vector: every CTA sums the squares in the same order, so all CTAs (and every launch of the same form, 16 bytes of x at a
+        // time or number by number, that reads the same x) derive the bit-identical normalised vector
         ss = warp_sum(ss);
         if (lane == 0) red[warp] = ss;
         __syncthreads();

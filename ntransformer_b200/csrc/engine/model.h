@@ -300,7 +300,7 @@ private:
     void prefill_batched(const int* tokens, int seq_len, int start_pos);
     void ensure_prefill_buffers(int tokens);
     bool f16_direct(const Weight& w) const;   // F16 rows usable by TMA in place
-    // C[T, w.rows] (+)= split(A)[T, w.cols] . W^T for a weight of any GGUF dtype (quantised: dequantise to hi/lo, two GEMMs)
+    // C[T, w.rows] (+)= split(A)[T, w.cols] . W^T for a weight of any GGUF dtype (blocks: prefill_blocks.cu; F32 and unaligned F16: expanded to hi/lo, two GEMMs)
     void prefill_gemm(float* C, const void* ws, const Weight& w, int T, bool add, cudaStream_t s);
     void release_graphs();
 

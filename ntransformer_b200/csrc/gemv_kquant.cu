@@ -383,11 +383,12 @@ TeamPlan plan_teams(int mask, int K, int groups, bool four) {
         }
         return t;
     };
-    // Teams of 4 share one copy of the vector and pay the meeting at the end of 16 rows half as often, four of
-    // them hide one another's barriers: the rule for every launch that gives each SM more than a group (Q4_K 57344 x 8192: 45.5 us, 58 in teams of 8, 53.4
-    // with the dp4a kernel that this one replaced).  Fewer groups than SMs: more warps finish a group sooner, 8 (Q8_0 1024 x 4096: 4.8 us, 6.2 in teams of 4;
-    // Q4_K 4096 x 4096, 256 groups: 5.1 and 4.9), for long rows 16 (Q6_K 1024 x 14336: 9.9 us, 11.0 in a team of 8, 12.2 before; Q8_0 2048 x 28672: 23.2, 29.7,
-    // 24.5); in between two teams of 8 in a CTA, since the vector does not fit twice (Q4_K 4096 x 14336: 11.4 us, 12.3 in teams of 4, 16.9 before).
+    // Teams of 4 share one copy of the vector and pay the meeting at the end of 16 rows half as often, four of them hide one another's barriers: the rule for
+    // every launch that gives each SM more than a group (Q4_K 57344 x 8192 in a graph of its own: 45.5 us, 58 in teams of 8, 53.4 with the dp4a kernel that this
+    // one replaced; cold and alone 50.6; as gate and up with SwiGLU in the 70B step 55.9, 54.4 before: 1792 groups over 592 teams are 3.03 rounds and cost four).
+    // Fewer groups than SMs: more warps finish a group sooner, 8 (Q8_0 1024 x 4096: 4.8 us, 6.2 in teams of 4; Q4_K 4096 x 4096, 256 groups: 5.1 and 4.9), for
+    // long rows 16 (Q6_K 1024 x 14336: 9.9 us, 11.0 in a team of 8, 12.2 before; Q8_0 2048 x 28672: 23.2, 29.7, 24.5); in between two teams of 8 in a CTA, since
+    // the vector does not fit twice (Q4_K 4096 x 14336: 11.4 us, 12.3 in teams of 4, 16.9 before).
     TeamPlan t = K > 8192 ? (groups > 256 ? form(4, 4, SMEM_CTA) : groups > 148 ? form(8, 2, SMEM_CTA) : form(16, 1, SMEM_CTA))
                           : (groups > 148 ? form(4, 4, SMEM_CTA) : form(8, 1, SMEM_HALF));
     // Very long rows (from 41984 on, by format): the vector leaves no room for a stage of every team.  One team of 8 always has one.

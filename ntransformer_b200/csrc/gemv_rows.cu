@@ -6,7 +6,8 @@
 //   * one launch quantises all tokens (optionally RMSNorm) into the order in which mma.sync's B operand wants them: 8 tokens fill the operand's columns,
 //     (q1, q2) of four tokens in one product, q3 of eight in another;
 //   * a CTA takes 32 rows x 8 tokens.  A producer warp streams stages of 8 super-blocks of the rows and of the tokens; 16 warps share them, a
-//     super-block of 16 rows each.  Bound by the instruction issue of the per-block scales (about 450 instructions for 16 rows x 256 weights x 8 tokens).
+//     super-block of 16 rows each.  Bound by the instruction issue of the per-block scales (about 450 instructions for 16 rows x 256 weights x 8 tokens) where the
+//     ring has two stages (Q4_K, Q4_0, Q5_K); a stage of Q6_K, of Q4_K mixed with it and of Q8_0 leaves no room for a second, so that copies and products take turns.
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "gemv_mma_device.cuh"
@@ -19,7 +20,7 @@ namespace {
 constexpr int RKW = 8, RTILES = 2, RGROUP = RTILES * MROWS;      // super-blocks of a stage, row tiles, rows of a CTA
 constexpr int RWARPS = RKW * RTILES;
 constexpr int XB_DIGITS = 4 * 3 * 512, XB = XB_DIGITS + 512;     // bytes of 8 tokens' super-block: digits, scales [token][8], sums [token][8]
-constexpr int R_STAGES = 4;
+constexpr int R_STAGES = 2;                                      // what 227 KB hold at most
 
 struct RowsMat { const uint8_t* W; float* y; int out, groups, fmt; long long pitch; };
 struct RowsParams {

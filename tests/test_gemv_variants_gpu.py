@@ -1,7 +1,6 @@
 """Opt-in GEMV kernel variants against the oracle (their switches are read once per process, hence the subprocesses):
-  NT_B200_GEMV_QB=1      the quarter-block kernel (csrc/gemv_kquant_q.cu: lane <-> 64 weights, 16 warps) — measured slower than the
-                         default half-block kernel (profiles/r02_qb_layer_ncu_summary.txt), kept as an A/B aid;
-  NT_B200_TAIL_SPLIT=0   whole 4-row stages in a partly filled last round (the earlier schedule)."""
+  NT_B200_GEMV_QB=1        the quarter-block dp4a kernel (csrc/gemv_kquant_q.cu: lane <-> 64 weights, 16 warps), kept as an A/B aid;
+  NT_B200_GEMV_QB_SPLIT=0  with it: launches that mix Q6_K with another format stay one launch of the default kernel."""
 import os
 import subprocess
 import sys
@@ -55,7 +54,7 @@ print("ok")
 ''' % str(ROOT)
 
 
-@pytest.mark.parametrize("env", [{"NT_B200_GEMV_QB": "1"}, {"NT_B200_TAIL_SPLIT": "0"}, {"NT_B200_GEMV_QB": "1", "NT_B200_GEMV_QB_SPLIT": "0"}])
+@pytest.mark.parametrize("env", [{"NT_B200_GEMV_QB": "1"}, {"NT_B200_GEMV_QB": "1", "NT_B200_GEMV_QB_SPLIT": "0"}])
 def test_gemv_variant_matches_the_oracle(env):
     r = subprocess.run([sys.executable, "-c", SCRIPT], capture_output=True, text=True, env=dict(os.environ, **env), timeout=900)
     assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-3000:]

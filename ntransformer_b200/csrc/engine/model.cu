@@ -492,7 +492,9 @@ void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float
     const int K = ws[0]->cols;
     for (int i = 0; i < n; i++) { mats[i].W = ws[i]->ptr; mats[i].y = ys[i]; mats[i].out = ws[i]->rows; mats[i].dtype = ws[i]->dtype; mats[i].row_pitch = ws[i]->pitch; }
     GemvInput in;
-    if (!(fuse_mask_ & 1) && gemv_xq_supported(mats, n, K)) {      // the unfused form: norm and quantiser as a launch of their own
+    bool over_xq = xq_ != nullptr;                         // long rows, or the unfused form: norm and quantiser as a launch of their own
+    for (int i = 0; i < n && (fuse_mask_ & 1); i++) over_xq = over_xq && gemv_xq_faster(mats[i], K);
+    if (over_xq && gemv_xq_supported(mats, n, K)) {
         if (norm_w) rmsnorm_xq(nullptr, xq_, x, norm_w, K, cfg_.norm_eps, s);
         else quantize_x(x, xq_, K, s);
         gemv_xq(mats, n, K, xq_, ep, s);

@@ -14,10 +14,14 @@ from oracle import oracle as O  # noqa: E402
 pytestmark = [pytest.mark.gpu]
 
 
-@pytest.mark.parametrize("mix,inter", [("Q4_K", 20224), ("Q4_K", 20480), ("Q8_0", 20480), ("Q6_K", 20480), ("Q6_K", 20736), ("Q4_0", 28672), ("Q5_K", 49152), ("Q8_0", 49152)])
-def test_wide_feed_forward(tmp_path, mix, inter):
+# mixed: attention in F16, so that the step is not the short chain of launches
+@pytest.mark.parametrize("mix,inter,mixed", [("Q4_K", 20224, False), ("Q4_K", 20480, False), ("Q8_0", 20480, False), ("Q6_K", 20480, False), ("Q6_K", 20736, False),
+                                             ("Q4_0", 28672, False), ("Q5_K", 49152, False), ("Q8_0", 49152, False), ("Q4_K", 28672, True)])
+def test_wide_feed_forward(tmp_path, mix, inter, mixed):
     cfg = dataclasses.replace(TINY, intermediate_size=inter, n_layers=2)
     tensors = synthetic_tensors_np(cfg, mix, seed=7)
+    if mixed:
+        tensors.update({n: t for n, t in synthetic_tensors_np(cfg, "F16", seed=8).items() if "attn_" in n})
     write_gguf(tmp_path / "m.gguf", cfg, tensors)
     m = Model.load(tmp_path / "m.gguf", cfg.max_seq_len)
     om = O.Model(cfg.dict(), {n: (np.ascontiguousarray(a), int(dt)) for n, (a, dt, r, c) in tensors.items()})

@@ -275,10 +275,17 @@ bool gemv_xq_supported(const GemvMat* mats, int n_mat, int K) {
     return true;
 }
 
-// Long rows: beside the vector (3.25 bytes an element) gemv_kquant.cu has one or two ring stages to a team, this kernel all of shared memory.  Decode steps, the
-// down projection here against there (its quantise launch included): 70B shapes, 28672 wide, three layers in Q8_0 756 us against 807, four in Q4_K_M 759 / 765,
-// three in Q6_K 764 / 766; in Q4_K 49152 wide, three layers, 673 / 808; 24576 488 / 507; 20480 428 / 433; 18944 326 / 325; 14336 (8B, six layers) 468 / 442.
-bool gemv_xq_faster(const GemvMat& m, int K) { return K >= 20480 && gemv_xq_supported(&m, 1, K); }
+// Long rows: beside the vector (3.25 bytes an element) gemv_kquant.cu has one or two ring stages to a team, this kernel all of shared memory.  The line lies where
+// that kernel is down to one stage of one super-block to a warp (Q8_0 from 26624 columns, Q6_K from 35328), and at 32768 for the formats whose stage holds two.
+// Decode steps of three layers, the down projection here against there (its quantise launch included): Q8_0 20480 wide 457 us against 460, 24576 550 / 545, 28672
+// 760 / 807; Q6_K 24576 557 / 547, 28672 757 / 755, 32768 781 / 788, 36864 835 / 896; Q4_K 18944 (four layers) 326 / 320, 24576 496 / 506, 28672 554 / 557, 32768
+// 564 / 573, 36864 829 / 877, 40960 608 / 635, 49152 666 / 802; Q5_K 24576 469 / 462, 28672 611 / 616, 40960 701 / 718.  70B in Q4_K_M (28672) 94.8 tok/s against 95.4.
+bool gemv_xq_faster(const GemvMat& m, int K) {
+    if (K < 20480 || !gemv_xq_supported(&m, 1, K)) return false;
+    int plan[4];
+    const bool single = m.dtype == DType::Q6_K || m.dtype == DType::Q8_0;
+    return K >= 32768 || !gemv_kq_any_pitch(&m, 1, K) || (single && gemv_kq_plan(&m, 1, K, false, false, plan) && plan[2] == 1);
+}
 
 void gemv_xq(const GemvMat* mats, int n_mat, int K, const void* xq, GemvEpilogue ep, cudaStream_t s) {
     NT_CHECK(gemv_xq_supported(mats, n_mat, K) && ep != GEMV_PEER, "gemv_xq: unsupported shape/dtype/alignment");

@@ -15,8 +15,8 @@ pytestmark = [pytest.mark.gpu]
 
 
 # mixed: attention in F16, so that the step is not the short chain of launches
-@pytest.mark.parametrize("mix,inter,mixed", [("Q4_K", 20224, False), ("Q4_K", 20480, False), ("Q8_0", 20480, False), ("Q6_K", 20480, False), ("Q6_K", 20736, False),
-                                             ("Q4_0", 28672, False), ("Q5_K", 49152, False), ("Q8_0", 49152, False), ("Q4_K", 28672, True)])
+@pytest.mark.parametrize("mix,inter,mixed", [("Q4_K", 28672, False), ("Q4_K", 32768, False), ("Q8_0", 26368, False), ("Q8_0", 28672, False), ("Q6_K", 32768, False),
+                                             ("Q6_K", 33024, False), ("Q4_0", 36864, False), ("Q5_K", 49152, False), ("Q8_0", 49152, False), ("Q4_K", 32768, True)])
 def test_wide_feed_forward(tmp_path, mix, inter, mixed):
     cfg = dataclasses.replace(TINY, intermediate_size=inter, n_layers=2)
     tensors = synthetic_tensors_np(cfg, mix, seed=7)

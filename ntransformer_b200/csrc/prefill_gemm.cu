@@ -13,6 +13,7 @@
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "tc_device.cuh"
+#include "wait_status.cuh"
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
@@ -68,19 +69,6 @@ __global__ void split_f32_kernel(__half2* __restrict__ hi, __half2* __restrict__
     }
 }
 
-// bounded mbarrier wait: a mis-programmed pipeline traps instead of hanging the GPU
-__device__ __forceinline__ void wait_or_trap(uint64_t* bar, uint32_t parity) {
-    uint32_t done = 0;
-    for (uint32_t spin = 0; spin < (1u << 24); spin++) {
-        asm volatile(
-            "{\n .reg .pred p;\n"
-            " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            " selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-        if (done) return;
-    }
-    __trap();
-}
 __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* map) {
     asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
 }
@@ -125,7 +113,7 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
                                                              float* __restrict__ C, __half* __restrict__ split_out,
                                                              int M, int Mp, int N, int K, int tiles_m, int tiles_n, int n_tiles, int n_outer,
                                                              int kc_blocks, int bf16, int gelu, const float* __restrict__ col_scale, float alpha,
-                                                             const float* __restrict__ act_p, const __grid_constant__ typename KindArg<KIND>::type grp) {
+                                                             const float* __restrict__ act_p, const __grid_constant__ typename KindArg<KIND>::type grp, unsigned* status) {
     constexpr bool GROUPED = KIND == KIND_GROUPED, MULTI = KIND == KIND_MULTI;
     static_assert(!MULTI || MODE == MODE_STORE, "several matrices: plain stores");
     constexpr bool ONE_CHUNK = MODE == MODE_SWIGLU || MODE == MODE_XIELU || MODE == MODE_RELU2;       // the epilogue needs the whole sum
@@ -180,8 +168,9 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
     if (warp == 0) {
         if (lane == 0) {                               // ---- TMA producer ----
             uint32_t it = 0;                           // k-block counter across all of this CTA's tiles
+            uint32_t tries = WAIT_TRIES;               // 0: a wait of this thread has run out
             int run = 0, m0 = 0, n0 = 0, m_end = 0, fenced = -1;
-            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            for (int tile = blockIdx.x; tile < n_tiles && tries; tile += gridDim.x) {
                 place(tile, run, m0, n0, m_end);
                 const CUtensorMap *mb = &map_b, *mb2 = &map_b2;
                 if constexpr (GROUPED) {
@@ -195,7 +184,11 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
                 if constexpr (MULTI) mb = &grp.map[run];
                 for (int kb = 0; kb < num_kb; kb++, it++) {         // chunk boundaries do not matter to the producer
                     const uint32_t s = it % STAGES;
-                    wait_or_trap(&empty_bar[s], ((it / STAGES) & 1) ^ 1);
+                    wait_phase(&empty_bar[s], ((it / STAGES) & 1) ^ 1, status, tries);
+                    if (!tries) {                                   // given up: the copies in flight
+                        for (uint32_t j = it > STAGES ? it - STAGES : 0; j < it; j++) wait_flight(&full_bar[j % STAGES], (j / STAGES) & 1);
+                        break;
+                    }
                     uint8_t* st = smem + (size_t)s * STAGE_BYTES;
                     mbar_expect_tx(&full_bar[s], STAGE_BYTES);
                     tma_load_2d(st, &map_a, kb * BK, m0, &full_bar[s]);                 // A_hi rows [m0, m0+128)
@@ -212,19 +205,20 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
         const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);
         const uint64_t desc0 = make_desc(smem);
         constexpr uint64_t LO = TILE_A >> 4, B = (2 * TILE_A) >> 4, B2 = (2 * TILE_A + 128 * BK * 2) >> 4;
-        uint32_t s = 0, par = 0, lt = 0;
+        uint32_t s = 0, par = 0, lt = 0, tries = WAIT_TRIES;               // tries 0: a wait of this lane has run out
+        int last = -1;                                                     // stage and parity of the last commit
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x)
         for (int kc = 0; kc < n_kc; kc++, lt++) {
             const uint32_t acc = lt & 1, acc_phase = (lt >> 1) & 1;
-            wait_or_trap(&tmem_empty_bar[acc], acc_phase ^ 1);             // epilogue drained this accumulator
+            wait_phase(&tmem_empty_bar[acc], acc_phase ^ 1, status, tries);      // epilogue drained this accumulator
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t d = tm + acc * BN;
             const int kb0 = ONE_CHUNK ? 0 : kc * kc_blocks, kb1 = ONE_CHUNK ? num_kb : min(num_kb, kb0 + kc_blocks);
             for (int kb = kb0; kb < kb1; kb++) {
-                wait_or_trap(&full_bar[s], par);
+                wait_phase(&full_bar[s], par, status, tries);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da_hi = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4)), da_lo = da_hi + LO, db = da_hi + B, db2 = da_hi + B2;
-                if (leader) {
+                if (leader && tries) {
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; k++) {      // advance 32 bytes (>> 4 = 2) inside the 128-byte swizzle row
                         umma_f16(d, da_hi + 2 * k, db + 2 * k, IDESC, ((kb - kb0) | k) ? 1u : 0u);
@@ -236,16 +230,18 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
                         if (MODE == MODE_SWIGLU) umma_f16(d + 128, da_lo + 2 * k, db2 + 2 * k, IDESC, 1u);
                     }
                     umma_commit(&empty_bar[s]);            // smem slot reusable once these MMAs retire
+                    last = (int)(s * 2 + par);
                     if (kb + 1 == kb1) umma_commit(&tmem_full_bar[acc]);      // accumulator complete
                 }
                 __syncwarp();
                 if (++s == STAGES) { s = 0; par ^= 1; }
             }
         }
+        if (!tries && last >= 0) wait_flight(&empty_bar[last >> 1], last & 1);      // given up: the products in flight
     } else {
         // ---- epilogue: TMEM -> registers -> global (warp w may only touch TMEM lanes [32 * (w % 4), +32)) ----
         const int quarter = warp & 3;
-        uint32_t lt = 0;
+        uint32_t lt = 0, tries = WAIT_TRIES;
         int run = 0, m0 = 0, n0 = 0, m_end = 0;
         float act_a = 0.f, act_b = 0.f;
         if (MODE == MODE_XIELU) { act_a = softplus_f(act_p[0]); act_b = softplus_f(act_p[1]); }
@@ -254,8 +250,8 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
             const uint32_t acc = lt & 1, acc_phase = (lt >> 1) & 1;
             const bool add_c = MODE == MODE_ADD || kc > 0;           // later chunks add their partial sums to what is in C
             if (kc == 0) place(tile, run, m0, n0, m_end);
-            const int row = m0 + quarter * 32 + lane;
-            wait_or_trap(&tmem_full_bar[acc], acc_phase);
+            wait_phase(&tmem_full_bar[acc], acc_phase, status, tries);
+            const int row = tries ? m0 + quarter * 32 + lane : m_end;      // given up: nothing is stored
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
 #pragma unroll 1
@@ -326,7 +322,7 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty_bar[acc]);             // this warp's quarter of the accumulator is free
+            if (lane == 0 && tries) mbar_arrive(&tmem_empty_bar[acc]);    // this warp's quarter of the accumulator is free
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -460,7 +456,7 @@ bool launch_gemm(float* C, __half* split_out, const void* workspace, const void*
     const int kc_blocks = kc_env > 0 ? kc_env : K / BK;
     gemm_f16_tc_kernel<BN, MODE, KIND_PLAIN><<<grid, 192, Cfg<BN>::SMEM, s>>>(map_a, map_b, map_b2, C, split_out, M, (int)Mp, N, K, tiles_m, tiles_n,
                                                                         n_tiles, n_outer, kc_blocks, o.bf16 ? 1 : 0, o.relu ? 2 : (o.gelu ? 1 : 0), o.col_scale, o.alpha, o.act_p,
-                                                                        Plain{});
+                                                                        Plain{}, wait_status());
     count_launch();
     return true;
 }
@@ -477,7 +473,7 @@ bool launch_grouped(float* C, __half* split_out, const void* workspace, const Gr
     const int tiles_n = (N + TN - 1) / TN;
     const int grid = (int)std::min<size_t>((size_t)sm_count(), Mp / BM * tiles_n);
     gemm_f16_tc_kernel<BN, MODE, KIND_GROUPED><<<grid, 192, Cfg<BN>::SMEM, s>>>(map_a, map_a, map_a, C, split_out, 0, (int)Mp, N, K, 0, tiles_n, 0, 0, 64, o.bf16 ? 1 : 0,
-                                                                       o.relu ? 2 : (o.gelu ? 1 : 0), nullptr, 1.0f, nullptr, grp);
+                                                                       o.relu ? 2 : (o.gelu ? 1 : 0), nullptr, 1.0f, nullptr, grp, wait_status());
     NT_LAUNCH_CHECK();
     count_launch();
     return true;
@@ -519,7 +515,7 @@ bool gemm_f16_tc_multi_ws(float* const* C, const void* workspace, const void* co
     opt_in_dynamic_smem(gemm_f16_tc_kernel<BN, MODE_STORE, KIND_MULTI>, (int)(Cfg<BN>::SMEM), configured);
     const int kc_blocks = 64;                      // accumulation chunk, as for one matrix
     gemm_f16_tc_kernel<BN, MODE_STORE, KIND_MULTI><<<std::min(tiles, sm_count()), 192, Cfg<BN>::SMEM, s>>>(map_a, map_a, map_a, nullptr, nullptr, M, (int)Mp, 0, K, tiles_m, 0, tiles, 0,
-                                                                                                          kc_blocks, o.bf16 ? 1 : 0, 0, nullptr, 1.0f, nullptr, mu);
+                                                                                                          kc_blocks, o.bf16 ? 1 : 0, 0, nullptr, 1.0f, nullptr, mu, wait_status());
     NT_LAUNCH_CHECK();
     count_launch();
     return true;

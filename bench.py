@@ -1,5 +1,5 @@
 #!/usr/bin/env python3
-"""bench.py — resident decode throughput of the B200-native engine on BASELINE.json's metric.
+"""bench.py — resident decode throughput of the B200-native engine (decoded tokens per second).
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--workload NAME] [--impl ours|reference]
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N ... bench.py --gpus N ...
@@ -11,7 +11,7 @@ device-side step state; e2e = tok/s through the C-ABI with HOST token ids in and
 
 --impl reference times the UNMODIFIED reference (its own CUDA kernels and Transformer::forward, compiled for
 sm_100 into oracle/_ref by oracle/Makefile) on the same synthetic model on one GPU of this box.  The reference
-has no CPU path (SURVEY §0), so its own implementation of this path IS a CUDA implementation; the CPU figure
+has no CPU path, so its own implementation of this path IS a CUDA implementation; the CPU figure
 reported next to it (cpu_baseline, kind "port") is the oracle's C restatement on the host cores.
 """
 from __future__ import annotations
@@ -33,14 +33,14 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 WORKLOADS = {
-    # name: (shape, mix, prompt_len, max_seq)          BASELINE.json configs[2] is the metric's own config
+    # name: (shape, mix, prompt_len, max_seq)          the 70B decode is the metric's own workload
     "llama3-70b-q4_k_m-decode": ("70b", "Q4_K_M", 16, 4096),
     "llama3-8b-q4_k_m-decode-ctx2048": ("8b", "Q4_K_M", 2047, 4096),
     "llama3-8b-q8_0-decode": ("8b", "Q8_0", 16, 4096),
     "llama3-70b-q6_k-decode": ("70b", "Q6_K", 16, 4096),
     "llama3-8b-q4_k_m-decode": ("8b", "Q4_K_M", 16, 4096),
     "tiny-q4_k_m-decode": ("tiny", "Q4_K_M", 8, 128),
-    # BASELINE.json configs[4]: the step is one whole 4096-token prompt (metric prefill_tok_s); see run_prefill
+    # the step is one whole 4096-token prompt (metric prefill_tok_s); see run_prefill
     "llama3-8b-f16-prefill-4096": ("8b", "F16", 4096, 4096),
     "tiny-f16-prefill-96": ("tiny", "F16", 96, 128),
     # quantised weights on the tensor-core prefill path (dequantised to an F16 hi/lo pair per matrix, two GEMMs each)
@@ -139,7 +139,7 @@ def measured_peak_tensor():
 
 # ------------------------------------------------------------------------------------------------
 def run_prefill(args, rank, world):
-    """BASELINE.json configs[4]: F16 prefill of a whole prompt through the batched tcgen05 path.  One step = one prompt;
+    """F16 prefill of a whole prompt through the batched tcgen05 path.  One step = one prompt;
     value = prompt tokens / s with the prompt ids already on the host side of the C-ABI call but no logits read-back,
     e2e = the same through nt_model_forward (token ids H2D + logits D2H inside the timed region)."""
     import torch
@@ -273,7 +273,7 @@ def run_ours(args, rank, world):
     if world > 1:
         dist.init_process_group("nccl", device_id=torch.device("cuda", local))
     line = measure_decode(args, rank, world, args.workload, with_cpu=not args.no_cpu_baseline)
-    # BASELINE.json configs[3] (70B Q6_K, 8-way tensor parallel) rides along with the 8-GPU run of the metric's own config
+    # 70B Q6_K, 8-way tensor parallel, rides along with the 8-GPU run of the metric's own config
     # (Q4_K_M at every N, so that the 1/2/4/8 series stays one workload): reported under "configs3".
     if world == 8 and args.workload == "llama3-70b-q4_k_m-decode" and not args.no_configs3:
         extra = measure_decode(args, rank, world, "llama3-70b-q6_k-decode", with_cpu=False)
@@ -592,7 +592,7 @@ def run_reference(args, rank, world):
                 "e2e": {"value": round(tok_s, 2), "unit": "tok/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
                 "setup_s": round(t_gen, 1)}), flush=True)
             return
-        # bounded prefill: the reference prefills with per-token GEMVs (SURVEY §3.2), so keep the prompt short
+        # bounded prefill: the reference prefills with per-token GEMVs, so keep the prompt short
         p_len = min(prompt_len, 16)
         toks = np.array([token_at(i, vocab) for i in range(p_len)], np.int32)
         logits = np.empty(vocab, np.float32)

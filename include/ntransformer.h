@@ -2,7 +2,7 @@
  * ntransformer.h — public C API of the engine.
  *
  * Same declarations as the reference's include/ntransformer.h:11-38, which the reference declares but never
- * defines (SURVEY §0); libnt_b200.so implements them over the resident B200 engine.  Strings returned by
+ * defines; libnt_b200.so implements them over the resident B200 engine.  Strings returned by
  * nt_engine_generate are malloc'ed and must be released with nt_free.
  */
 #ifndef NTRANSFORMER_H

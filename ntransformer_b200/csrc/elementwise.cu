@@ -4,7 +4,7 @@
 //
 // This file is compiled with --use_fast_math like the reference (CMakeLists.txt:20) and writes the
 // transcendental expressions in the same form (1.0f / powf, cosf/sinf, g / (1 + expf(-g)), rsqrtf) so they
-// lower to the same approximate instructions: greedy-token parity depends on it (SURVEY quirk Q2).
+// lower to the same approximate instructions: greedy-token parity depends on it.
 // Anything that must stay IEEE uses explicit *_rn intrinsics.
 #include "kernels_internal.h"
 #include "xquant.cuh"

@@ -147,7 +147,7 @@ __device__ void mega_barrier(const MegaParams& P, int kind, SyncState& st) {
         if (xchg) { __threadfence_system(); red_relaxed_gpu_add(counter, 1u); }
         else red_release_gpu_add(counter, 1u);
         if (xchg && P.xchg_direct) {
-            // Experiment (off by default; KNOWN GAP): with tp_size >= 3 a rank that has already passed exchange n can post
+            // Experiment (off by default; known gap): with tp_size >= 3 a rank that has already passed exchange n can post
             // its exchange-(n+1) arrivals into a slower rank's counter while another rank's exchange-n arrival is still in flight
             // (relaxed reds to different destinations are unordered), so the counter can reach n * tp * grid early.  Needs one
             // counter per exchange parity (or per source rank) before it may be used; the stand-alone exchange of

@@ -20,7 +20,7 @@ struct ModelConfig {                       // reference src/model/config.h:16-58
     int vocab_size = 32000, hidden_size = 4096, intermediate_size = 11008, n_layers = 32;
     int n_heads = 32, n_kv_heads = 32, head_dim = 128;
     float norm_eps = 1e-5f, rope_theta = 10000.0f, rope_freq_scale = 1.0f;
-    bool rope_interleaved = false;         // never set from GGUF by the reference (SURVEY quirk Q1)
+    bool rope_interleaved = false;         // never set from GGUF by the reference
     int max_seq_len = 4096;
     int bos_token_id = 1, eos_token_id = 2;
     // Families described layer by layer (a model folder, engine/model_registry.h): one entry per layer; empty for the GGUF Llama block.

@@ -520,7 +520,7 @@ void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float
     }
 }
 
-// hidden += all_reduce(partial)   (one exchange per sub-block; SURVEY §8e)
+// hidden += all_reduce(partial)   (one exchange per sub-block)
 void Model::reduce_residual(float* partial, cudaStream_t s) {
     NT_CHECK(comm_ != nullptr, "tensor-parallel model without a communicator");
     // (the unfused path; with the peer exchange mapped the short chain sums through NVLink stores instead, see step_body)

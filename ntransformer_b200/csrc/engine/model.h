@@ -6,7 +6,7 @@
 // (src/model/ffn.cpp:85-134) re-expressed as fused sm_100a launches captured in a CUDA graph:
 //   reference: 15 launches / layer / token, CPU embedding dequant, 2 sync H2D + 1 sync D2H per token;
 //   here:      10 launches / layer / token in one graph replay, embedding gathered on the GPU.
-// The streaming / tiered / speculative branches of the reference are out of scope (SURVEY §8).
+// The streaming / tiered / speculative branches of the reference are out of scope.
 #pragma once
 #include <cuda_runtime.h>
 #include <string>
@@ -155,7 +155,7 @@ public:
     float* logits_device() const { return logits_; }
     int tp_rank() const { return tp_rank_; }
     int tp_size() const { return tp_size_; }
-    // Algorithmic bytes this rank reads per decoded token at context length ctx (SURVEY §8d B_tok).
+    // Algorithmic bytes this rank reads per decoded token at context length ctx.
     size_t bytes_per_token(int ctx) const;
     size_t weight_bytes() const;
     double load_seconds() const { return load_seconds_; }     // wall time of load_gguf (parse + plan + pipelined upload + buffers)

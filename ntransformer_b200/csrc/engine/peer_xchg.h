@@ -1,6 +1,6 @@
 // peer_xchg.h — tensor-parallel sum of the o-projection / down-projection partials over NVLink peer memory, without NCCL.
 //
-// New relative to the single-GPU reference ("one all-reduce per sub-block").  One-shot all-reduce in two kernels:
+// New relative to the single-GPU reference (one all-reduce per sub-block).  One-shot all-reduce in two kernels:
 //   * the producing GEMV (gemv_kquant.cu, epilogue GEMV_PEER) stores each finished row of its partial result straight into the
 //     "slot" [parity][source rank][hidden] of EVERY rank (stores to cudaIpc-mapped peer memory, i.e. NVLink writes issued from
 //     the GEMV's epilogue while other CTAs are still streaming weights).  A slot element is one 64-bit word {sequence : value}

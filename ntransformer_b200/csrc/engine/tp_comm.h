@@ -1,5 +1,5 @@
 // tp_comm.h — tensor-parallel collectives over NCCL (NVLink 5 / NVSwitch).
-// New work relative to the reference, which is single-GPU (SURVEY §2.3, §8e).  One process per GPU: the
+// New work relative to the reference, which is single-GPU.  One process per GPU: the
 // 128-byte ncclUniqueId is created on rank 0 and handed to the other ranks by the host plumbing
 // (torch.distributed in bench.py); libnccl.so.2 is resolved at run time (it is already in the process when
 // torch is imported) so libnt_b200.so has no link-time NCCL dependency on single-GPU boxes.

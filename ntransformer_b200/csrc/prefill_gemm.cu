@@ -2,8 +2,8 @@
 //
 // The reference has no batched matmul on its forward path: prefill is a host loop of per-token GEMVs that re-reads
 // every weight matrix once per prompt token (src/model/attention.cpp:144-162, src/model/ffn.cpp:96-133; its
-// launch_gemm_f32, src/cuda/gemm.cu:677-694, is dead code).  This is the dense contraction BASELINE.json config 5
-// names, written for Blackwell's 5th-generation tensor cores:
+// launch_gemm_f32, src/cuda/gemm.cu:677-694, is dead code).  This is the dense contraction of a long prompt
+// into an F16 model, written for Blackwell's 5th-generation tensor cores:
 //   * operands staged by TMA (cp.async.bulk.tensor.2d, SWIZZLE_128B) into a 4-stage shared-memory ring,
 //   * tcgen05.mma.cta_group::1.kind::f16 issued by one elected thread, 128x128 F32 accumulator in TMEM,
 //   * tcgen05.commit -> mbarrier hand-offs (smem slot free / accumulator ready), epilogue via tcgen05.ld.

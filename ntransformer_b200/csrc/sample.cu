@@ -2,7 +2,7 @@
 //
 // Replaces, for 0 < top_k <= 1024 < vocab, the reference's CPU sampler (Sampler::apply_repeat_penalty + Sampler::sample,
 // src/inference/sampler.cpp:30-117), which copies 513 KB of logits to the host and runs a partial_sort over 128 k candidates
-// per token (0.1-1 ms: comparable to a whole 8B token on a B200, SURVEY §8f rank 1).  Here the token id is the only thing that
+// per token (0.1-1 ms: comparable to a whole 8B token on a B200).  Here the token id is the only thing that
 // leaves the GPU.  The arithmetic follows the reference step by step so that the draw is reproducible against it:
 //   * penalty: sequential over the window (a token that occurs twice is penalised twice), IEEE division;
 //   * candidates: logit / temperature (IEEE), the k largest (radix select on order-preserving keys, ties at the threshold

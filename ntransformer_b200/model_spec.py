@@ -1,6 +1,6 @@
-"""Llama-3 shapes and per-tensor quantisation mixes of the benchmark configs.
+"""Llama-3 shapes and per-tensor quantisation mixes of the benchmark workloads.
 
-The Q4_K_M recipe follows llama.cpp ftype 15 as SURVEY §8d states it: everything Q4_K except attn_v and
+The Q4_K_M recipe follows llama.cpp ftype 15: everything Q4_K except attn_v and
 ffn_down, which are Q6_K on layers with  i < L/8  or  i >= 7L/8  or  (i - L/8) % 3 == 2 ;  on the 70B shape the
 remaining attn_v are Q5_K ; output.weight is Q6_K, token_embd Q4_K, norms F32."""
 from __future__ import annotations
@@ -80,7 +80,7 @@ def tensor_table(cfg: LlamaConfig, mix: str, tp_rank: int = 0, tp_size: int = 1)
 
 
 def bytes_per_token(cfg: LlamaConfig, mix: str, ctx: int, tp_size: int = 1) -> int:
-    """Algorithmic bytes read per decoded token (SURVEY §8d): 7 projections x L + output.weight + norms + KV."""
+    """Algorithmic bytes read per decoded token: 7 projections x L + output.weight + norms + KV."""
     b = 0
     for name, dt, r, c in tensor_table(cfg, mix, 0, tp_size):
         if name == "token_embd.weight":

@@ -1,7 +1,7 @@
 """Synthetic GGUF-layout weights: random *valid* quantisation blocks (numpy on the host, torch on the GPU).
 
 Any byte pattern with finite fp16 scales is a valid block of every GGUF format used here, so blocks are
-drawn directly (SURVEY §8d): codes uniform, 6-bit scales/mins uniform, fp16 super-block scales chosen so
+drawn directly: codes uniform, 6-bit scales/mins uniform, fp16 super-block scales chosen so
 the dequantised weights have std ~ `std` and mean ~ 0.
 """
 from __future__ import annotations

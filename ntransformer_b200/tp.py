@@ -1,4 +1,4 @@
-"""Tensor-parallel shard plan for GGUF block-quantised weights (new relative to the single-GPU reference; SURVEY §8e).
+"""Tensor-parallel shard plan for GGUF block-quantised weights (new relative to the single-GPU reference).
 
 Row split (attn_q/k/v by heads, ffn_gate/up by FFN columns, output.weight by vocab rows) needs no communication;
 column split (attn_output, ffn_down: slices of the *input* dimension at quantisation-block boundaries) produces

@@ -1,4 +1,4 @@
-"""Loader throughput (SURVEY §8 f3): writes the workload's seeded GGUF to /dev/shm, then times our pipelined loader
+"""Loader throughput: writes the workload's seeded GGUF to /dev/shm, then times our pipelined loader
 (nt_model_load_gguf: reader threads -> pinned staging -> cudaMemcpyAsync) and the reference's own loader (oracle/_ref:
 Transformer::load, one synchronous cudaMemcpy per tensor from the mmap) on the same file.  Prints one JSON line.
 

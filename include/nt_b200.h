@@ -103,6 +103,10 @@ int    nt_b200_gemv_rows(int n_mat, float* const* y, const void* const* W, const
  * (nt_b200_split_activations).  Returns 0, or < 0 when rejected (nothing launched). */
 int    nt_b200_gemm_blocks_ws(int n_mat, float* const* C, const void* const* W, const int* out_features, const int* dtypes, int in_features,
                               const void* workspace, int tokens, int add, void* stream);
+/* The same over F32 tokens x [tokens, in_features] (norm_w: their RMSNorm), each under a power of two of its own; fine: 64 columns to an accumulator of the
+ * tensor cores instead of 256.  What it needs beside its arguments is stream-ordered memory of the call.  Returns 0, or < 0 when rejected. */
+int    nt_b200_gemm_blocks(int n_mat, float* const* C, const void* const* W, const int* out_features, const int* dtypes, int in_features,
+                           const float* x, const float* norm_w, float eps, int tokens, int fine, int add, void* stream);
 /* The decode step's attention sub-block in ONE launch: launch_rope (src/cuda/rotary.cu:113-140; q and k are read, not
  * modified) + launch_copy_to_kv_cache at row *pos_dev (src/cuda/attention.cu:405-425) + launch_attention_decode over
  * *pos_dev + 1 keys (src/cuda/attention.cu:348-375), context split over CTAs, merged by the last CTA of each head group.

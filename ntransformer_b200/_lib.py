@@ -46,6 +46,7 @@ SIGNATURES = {
     "nt_b200_gemv_fused_plan": (_i, [_i, C.POINTER(_i), C.POINTER(_i), _i, _i, _i, C.POINTER(_i)]),
     "nt_b200_gemv_rows_bytes": (_sz, [_i, _i]),
     "nt_b200_gemv_rows": (_i, [_i, C.POINTER(_vp), C.POINTER(_vp), C.POINTER(_i), C.POINTER(_i), _i, _vp, _vp, _f, _i, _vp, _i, _vp]),
+    "nt_b200_gemm_blocks": (_i, [_i, C.POINTER(_vp), C.POINTER(_vp), C.POINTER(_i), C.POINTER(_i), _i, _vp, _vp, _f, _i, _i, _i, _vp]),
     "nt_b200_gemm_blocks_ws": (_i, [_i, C.POINTER(_vp), C.POINTER(_vp), C.POINTER(_i), C.POINTER(_i), _i, _vp, _i, _i, _vp]),
     "nt_b200_attention_decode_scratch_floats": (_sz, [_i, _i, _i, _i]),
     "nt_b200_attention_decode_tickets": (_i, [_i, _i]),

@@ -73,8 +73,8 @@ Model::~Model() {
                     (void*)argmax_dev_, (void*)recent_dev_})
         if (p) cudaFree(p);
     for (void* p : {(void*)pf_.x, (void*)pf_.q, (void*)pf_.k, (void*)pf_.v, (void*)pf_.attn, pf_.ws, pf_.ws2, (void*)pf_.tok, (void*)pf_.pos,
-                    (void*)pf_.g, (void*)pf_.u, pf_.whi, pf_.wlo, (void*)sb_.x, (void*)sb_.q, (void*)sb_.k, (void*)sb_.v, (void*)sb_.attn, (void*)sb_.act, sb_.xr,
-                    (void*)sb_.scratch, (void*)sb_.tok, (void*)sb_.pos})
+                    (void*)pf_.g, (void*)pf_.u, pf_.whi, pf_.wlo, (void*)sb_.x, (void*)sb_.q, (void*)sb_.k, (void*)sb_.v, (void*)sb_.attn, (void*)sb_.g, (void*)sb_.u, sb_.ws,
+                    block_scratch_, (void*)sb_.scratch, (void*)sb_.tok, (void*)sb_.pos})
         if (p) cudaFree(p);
     for (size_t i = 0; i < kcs_.size(); i++) if (kcs_[i] && (cache_owned_.empty() || cache_owned_[i])) { cudaFree(kcs_[i]); cudaFree(vcs_[i]); }
     for (void* p : {(void*)pf_.h, (void*)pf_.tmp, pf_.hws, (void*)want_out_, (void*)pf_.xs, (void*)pf_.maps, (void*)pf_.sel, (void*)pf_.work, (void*)pf_.wt,
@@ -786,23 +786,35 @@ bool Model::short_batch_ok(int seq_len, int start_pos) const {
     return chain_ok();
 }
 
+// What the GEMM over blocks keeps shared tiles in, for every caller on this model's stream; false: no room
+bool Model::ensure_block_scratch() {
+    if (block_scratch_) return true;
+    void* p = nullptr;
+    if (cudaMalloc(&p, block_scratch_bytes()) != cudaSuccess) { cudaGetLastError(); return false; }
+    zero_block_scratch(p, stream_);
+    block_scratch_ = p;
+    return true;
+}
+
 // false: no room for them; the caller takes the tokens one by one, which needs none
 bool Model::ensure_short_buffers() {
     if (sb_.x) return true;
+    if (!ensure_block_scratch()) return false;
     const size_t T = SHORT_CHUNK, hidden = (size_t)cfg_.hidden_size, qdim = (size_t)nh_l_ * cfg_.head_dim, kvdim = (size_t)nkv_l_ * cfg_.head_dim, f = sizeof(float);
-    const size_t bytes[10] = {T * hidden * f, T * qdim * f, T * kvdim * f, T * kvdim * f, T * qdim * f, T * (size_t)inter_l_ * f,
-                              gemv_rows_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_)),
+    const size_t bytes[11] = {T * hidden * f, T * qdim * f, T * kvdim * f, T * kvdim * f, T * qdim * f, T * (size_t)inter_l_ * f, T * (size_t)inter_l_ * f,
+                              std::max(block_tokens_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_)),
+                                       gemv_rows_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_))),
                               attention_rows_scratch_floats((int)T, cfg_.max_seq_len, nh_l_, nkv_l_, cfg_.head_dim) * f, T * sizeof(int), T * sizeof(int)};
-    void* got[10] = {};
-    for (int i = 0; i < 10; i++)
+    void* got[11] = {};
+    for (int i = 0; i < 11; i++)
         if (cudaMalloc(&got[i], std::max<size_t>(bytes[i], 1)) != cudaSuccess) {
             cudaGetLastError();
             for (int j = 0; j < i; j++) cudaFree(got[j]);
             return false;
         }
     sb_.x = static_cast<float*>(got[0]); sb_.q = static_cast<float*>(got[1]); sb_.k = static_cast<float*>(got[2]); sb_.v = static_cast<float*>(got[3]);
-    sb_.attn = static_cast<float*>(got[4]); sb_.act = static_cast<float*>(got[5]); sb_.xr = static_cast<uint8_t*>(got[6]); sb_.scratch = static_cast<float*>(got[7]);
-    sb_.tok = static_cast<int*>(got[8]); sb_.pos = static_cast<int*>(got[9]);
+    sb_.attn = static_cast<float*>(got[4]); sb_.g = static_cast<float*>(got[5]); sb_.u = static_cast<float*>(got[6]); sb_.ws = got[7]; sb_.scratch = static_cast<float*>(got[8]);
+    sb_.tok = static_cast<int*>(got[9]); sb_.pos = static_cast<int*>(got[10]);
     return true;
 }
 
@@ -810,8 +822,23 @@ void Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
     cudaStream_t s = stream_;
     const int hidden = cfg_.hidden_size, hd = cfg_.head_dim, max_seq = cfg_.max_seq_len, qdim = nh_l_ * hd;
     const size_t kv_stride = (size_t)max_seq * nkv_l_ * hd;
-    auto mat = [](const Weight& w, float* y) { GemvMat m; m.W = w.ptr; m.y = y; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch; return m; };
     int T = 0;
+    // Rows x (norm: their RMSNorm; up: silu(x) * up) times a group of matrices, in the form that is better for them.  Returns whether GEMV_SWIGLU is still to be taken:
+    // gate and up then lie in the two y, otherwise their product in the first.
+    auto product = [&](const float* x, const float* norm, int K, std::initializer_list<std::pair<const Weight*, float*>> list, GemvEpilogue ep, const float* up) {
+        GemvMat m[3];
+        int n = 0;
+        for (auto& [w, y] : list) { m[n].W = w->ptr; m[n].y = y; m[n].out = w->rows; m[n].dtype = w->dtype; m[n++].row_pitch = w->pitch; }
+        if (!gemm_blocks_for_few(m, n, T)) {
+            if (up) silu_mul(const_cast<float*>(x), x, up, T * K, s);
+            quantize_rows(sb_.ws, x, norm, cfg_.norm_eps, T, K, s);
+            gemv_rows(m, n, K, sb_.ws, T, ep, s);
+            return false;
+        }
+        const BlockTokens t = up ? silu_split_tokens(sb_.ws, x, up, T, K, s) : split_tokens(sb_.ws, x, norm, cfg_.norm_eps, T, K, s);
+        NT_CHECK(gemm_blocks(m, n, K, t, block_scratch_, true, T, ep == GEMV_ADD, s), "GEMM of a few tokens over blocks rejected");
+        return ep == GEMV_SWIGLU;
+    };
     for (int c0 = 0; c0 < seq_len; c0 += T) {
         T = std::min(SHORT_CHUNK, seq_len - c0);
         const int p0 = start_pos + c0;
@@ -823,19 +850,13 @@ void Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
             const LayerWeights& L = layers_[(size_t)i];
             uint16_t* kc = static_cast<uint16_t*>(kc_) + (size_t)i * kv_stride;
             uint16_t* vc = static_cast<uint16_t*>(vc_) + (size_t)i * kv_stride;
-            const GemvMat qkv[3] = {mat(L.wq, sb_.q), mat(L.wk, sb_.k), mat(L.wv, sb_.v)}, gu[2] = {mat(L.gate, sb_.act), mat(L.up, nullptr)};
-            const GemvMat o = mat(L.wo, sb_.x), down = mat(L.down, sb_.x);
-            quantize_rows(sb_.xr, sb_.x, L.attn_norm, cfg_.norm_eps, T, hidden, s);
-            gemv_rows(qkv, 3, hidden, sb_.xr, T, GEMV_STORE, s);
+            product(sb_.x, L.attn_norm, hidden, {{&L.wq, sb_.q}, {&L.wk, sb_.k}, {&L.wv, sb_.v}}, GEMV_STORE, nullptr);
             rope(sb_.q, sb_.k, sb_.pos, T, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, false, s);
             copy_to_kv_cache(kc, vc, sb_.k, sb_.v, T, nkv_l_, hd, p0, max_seq, s);
             attention_rows_f16(sb_.attn, sb_.q, kc, vc, T, p0, nh_l_, nkv_l_, hd, 1.0f / sqrtf((float)hd), sb_.scratch, s);
-            quantize_rows(sb_.xr, sb_.attn, nullptr, 0.f, T, qdim, s);
-            gemv_rows(&o, 1, qdim, sb_.xr, T, GEMV_ADD, s);
-            quantize_rows(sb_.xr, sb_.x, L.ffn_norm, cfg_.norm_eps, T, hidden, s);
-            gemv_rows(gu, 2, hidden, sb_.xr, T, GEMV_SWIGLU, s);
-            quantize_rows(sb_.xr, sb_.act, nullptr, 0.f, T, inter_l_, s);
-            gemv_rows(&down, 1, inter_l_, sb_.xr, T, GEMV_ADD, s);
+            product(sb_.attn, nullptr, qdim, {{&L.wo, sb_.x}}, GEMV_ADD, nullptr);
+            const bool open = product(sb_.x, L.ffn_norm, hidden, {{&L.gate, sb_.g}, {&L.up, sb_.u}}, GEMV_SWIGLU, nullptr);
+            product(sb_.g, nullptr, inter_l_, {{&L.down, sb_.x}}, GEMV_ADD, open ? sb_.u : nullptr);
         }
         if (!want_.empty()) emit_wanted(sb_.x, c0, T, s);
     }
@@ -853,27 +874,34 @@ bool Model::blocks_direct(const Weight& w) const {
     return gemm_blocks_supported(&m, 1, w.cols);
 }
 
-// C_i (+)= A . W_i^T for matrices over the same rows
-void Model::prefill_gemms(float* const* C, const void* ws, const Weight* const* w, int n, int T, bool add, cudaStream_t s) {
+// C_i (+)= A . W_i^T for matrices over the same rows: x (norm_w: their RMSNorm), or (x null) a plain split that lies in ws.  Matrices in blocks and the
+// others take different splits, one after the other in ws; where a group has both (rare) the rows are split twice.
+void Model::prefill_gemms(float* const* C, void* ws, const float* x, const float* norm_w, const Weight* const* w, int n, int T, bool add, cudaStream_t s) {
+    const int K = w[0]->cols;
+    const Weight* plain[3];
     GemvMat m[3];
-    bool blocks = n <= 3;
-    for (int i = 0; i < n && blocks; i++) {
-        blocks = blocks_direct(*w[i]);
-        m[i].W = w[i]->ptr; m[i].y = C[i]; m[i].out = w[i]->rows; m[i].dtype = w[i]->dtype; m[i].row_pitch = w[i]->pitch;
+    float* c[3];
+    int n_blocks = 0, n_plain = 0;
+    for (int i = 0; i < n; i++) {
+        if (!blocks_direct(*w[i])) { c[n_plain] = C[i]; plain[n_plain++] = w[i]; continue; }
+        GemvMat& b = m[n_blocks++];
+        b.W = w[i]->ptr; b.y = C[i]; b.out = w[i]->rows; b.dtype = w[i]->dtype; b.row_pitch = w[i]->pitch;
     }
-    if (blocks) { NT_CHECK(gemm_blocks(m, n, w[0]->cols, ws, T, add, s), "prefill GEMM over blocks rejected"); return; }
-    bool f16 = !add && n > 1 && n <= TC_MULTI_MAX;                 // F16 in place: narrow matrices fill the SMs together
+    if (n_plain && x) {
+        if (norm_w) rmsnorm_split(ws, x, norm_w, T, K, cfg_.norm_eps, s);
+        else split_activations(ws, x, T, K, s);
+    }
+    bool together = !add && n_plain > 1;                           // F16 in place: narrow matrices fill the SMs together
     const void* W[TC_MULTI_MAX]; int N[TC_MULTI_MAX];
-    for (int i = 0; i < n && f16; i++) { f16 = f16_direct(*w[i]) && w[i]->rows >= 256; W[i] = w[i]->ptr; N[i] = w[i]->rows; }
-    if (!f16 || !gemm_f16_tc_multi_ws(C, ws, W, N, n, T, w[0]->cols, s)) for (int i = 0; i < n; i++) prefill_gemm(C[i], ws, *w[i], T, add, s);
+    for (int i = 0; i < n_plain && together; i++) { together = f16_direct(*plain[i]) && plain[i]->rows >= 256; W[i] = plain[i]->ptr; N[i] = plain[i]->rows; }
+    if (!together || !gemm_f16_tc_multi_ws(c, ws, W, N, n_plain, T, K, s)) for (int i = 0; i < n_plain; i++) prefill_gemm(c[i], ws, *plain[i], T, add, s);
+    if (n_blocks) {
+        const BlockTokens t = x ? split_tokens(ws, x, norm_w, cfg_.norm_eps, T, K, s) : resplit_tokens(ws, ws, T, K, s);
+        NT_CHECK(gemm_blocks(m, n_blocks, K, t, block_scratch_, false, T, add, s), "prefill GEMM over blocks rejected");
+    }
 }
 
 void Model::prefill_gemm(float* C, const void* ws, const Weight& w, int T, bool add, cudaStream_t s) {
-    if (blocks_direct(w)) {
-        GemvMat m; m.W = w.ptr; m.y = C; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch;
-        NT_CHECK(gemm_blocks(&m, 1, w.cols, ws, T, add, s), "prefill GEMM over blocks rejected");
-        return;
-    }
     if (f16_direct(w)) {
         NT_CHECK(gemm_f16_tc_ws(C, ws, w.ptr, T, w.rows, w.cols, add, s), "prefill GEMM rejected");
         return;
@@ -896,16 +924,18 @@ void Model::ensure_prefill_buffers(int tokens) {
     pf_.x = dmalloc<float>(T * hidden);
     pf_.q = dmalloc<float>(T * qdim);    pf_.k = dmalloc<float>(T * kvdim);   pf_.v = dmalloc<float>(T * kvdim);
     pf_.attn = dmalloc<float>(T * qdim);
-    pf_.ws = dmalloc<uint8_t>(gemm_f16_tc_workspace_bytes((int)T, (int)std::max(hidden, qdim)));
-    pf_.ws2 = dmalloc<uint8_t>(gemm_f16_tc_workspace_bytes((int)T, inter_l_));
+    pf_.ws = dmalloc<uint8_t>(block_tokens_bytes((int)T, (int)std::max(hidden, qdim)));
+    pf_.ws2 = dmalloc<uint8_t>(block_tokens_bytes((int)T, inter_l_));
     pf_.tok = dmalloc<int>(T);           pf_.pos = dmalloc<int>(T);
     size_t w_elems = 0;                  // largest matrix that needs the dequantised scratch pair
-    bool swiglu_unfused = false;
+    bool swiglu_unfused = false, any_blocks = false;
     for (const LayerWeights& L : layers_) {
         for (const Weight* w : {&L.wq, &L.wk, &L.wv, &L.wo, &L.gate, &L.up, &L.down})
-            if (!f16_direct(*w) && !blocks_direct(*w)) w_elems = std::max(w_elems, (size_t)w->rows * (size_t)w->cols);
+            if (blocks_direct(*w)) any_blocks = true;
+            else if (!f16_direct(*w)) w_elems = std::max(w_elems, (size_t)w->rows * (size_t)w->cols);
         swiglu_unfused = swiglu_unfused || !f16_direct(L.gate) || !f16_direct(L.up);
     }
+    if (any_blocks) NT_CHECK(ensure_block_scratch(), "no room for the scratch of the prompt GEMM over blocks");
     if (w_elems) { pf_.whi = dmalloc<uint16_t>(w_elems); pf_.wlo = dmalloc<uint16_t>(w_elems); }
     if (swiglu_unfused) { pf_.g = dmalloc<float>(T * (size_t)inter_l_); pf_.u = dmalloc<float>(T * (size_t)inter_l_); }
     pf_.cap = (int)T;
@@ -936,28 +966,28 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
             uint16_t* kc = static_cast<uint16_t*>(kc_) + (size_t)i * kv_stride;
             uint16_t* vc = static_cast<uint16_t*>(vc_) + (size_t)i * kv_stride;
             // --- attention sub-block (attention.cpp:120-211 for all T tokens at once) ---
-            rmsnorm_split(pf_.ws, pf_.x, L.attn_norm, T, hidden, cfg_.norm_eps, s);
-            {
-                const Weight* w[3] = {&L.wq, &L.wk, &L.wv};
-                float* c[3] = {pf_.q, pf_.k, pf_.v};
-                prefill_gemms(c, pf_.ws, w, 3, T, false, s);
-            }
+            const Weight *qkv[3] = {&L.wq, &L.wk, &L.wv}, *wo = &L.wo, *gu[2] = {&L.gate, &L.up}, *down = &L.down;
+            float *qkv_out[3] = {pf_.q, pf_.k, pf_.v}, *gu_out[2] = {pf_.g, pf_.u};
+            prefill_gemms(qkv_out, pf_.ws, pf_.x, L.attn_norm, qkv, 3, T, false, s);
             rope(pf_.q, pf_.k, pf_.pos, T, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, false, s);
             copy_to_kv_cache(kc, vc, pf_.k, pf_.v, T, nkv_l_, hd, p0, max_seq, s);
             attention_prefill(pf_.attn, pf_.q, kc, vc, T, p0, nh_l_, nkv_l_, hd, max_seq, scale, s);
-            split_activations(pf_.ws, pf_.attn, T, qdim, s);
-            prefill_gemm(pf_.x, pf_.ws, L.wo, T, true, s);
+            prefill_gemms(&pf_.x, pf_.ws, pf_.attn, nullptr, &wo, 1, T, true, s);
             // --- FFN sub-block (ffn.cpp:85-134) ---
-            rmsnorm_split(pf_.ws, pf_.x, L.ffn_norm, T, hidden, cfg_.norm_eps, s);
             if (f16_direct(L.gate) && f16_direct(L.up)) {
+                rmsnorm_split(pf_.ws, pf_.x, L.ffn_norm, T, hidden, cfg_.norm_eps, s);
                 NT_CHECK(gemm_f16_tc_swiglu_ws(pf_.ws2, pf_.ws, L.gate.ptr, L.up.ptr, T, inter, hidden, s), "prefill GEMM (gate/up) rejected");
+                prefill_gemms(&pf_.x, pf_.ws2, nullptr, nullptr, &down, 1, T, true, s);
             } else {                                   // quantised gate/up: one plain GEMM over both, then SwiGLU and split in a pass
-                const Weight* w[2] = {&L.gate, &L.up};
-                float* c[2] = {pf_.g, pf_.u};
-                prefill_gemms(c, pf_.ws, w, 2, T, false, s);
-                silu_mul_split(pf_.ws2, pf_.g, pf_.u, T, inter, s);
+                prefill_gemms(gu_out, pf_.ws, pf_.x, L.ffn_norm, gu, 2, T, false, s);
+                if (blocks_direct(L.down)) {
+                    GemvMat m; m.W = down->ptr; m.y = pf_.x; m.out = down->rows; m.dtype = down->dtype; m.row_pitch = down->pitch;
+                    NT_CHECK(gemm_blocks(&m, 1, inter, silu_split_tokens(pf_.ws2, pf_.g, pf_.u, T, inter, s), block_scratch_, false, T, true, s), "prefill GEMM over blocks rejected");
+                } else {
+                    silu_mul_split(pf_.ws2, pf_.g, pf_.u, T, inter, s);
+                    prefill_gemm(pf_.x, pf_.ws2, L.down, T, true, s);
+                }
             }
-            prefill_gemm(pf_.x, pf_.ws2, L.down, T, true, s);
         }
         if (!want_.empty()) emit_wanted(pf_.x, c0, T, s);
     }

@@ -166,10 +166,12 @@ public:
     bool batched_prefill_ok(int seq_len, int start_pos) const;
     bool short_batch_ok(int seq_len, int start_pos) const;
     bool blocks_direct(const Weight& w) const;
-    void prefill_gemms(float* const* C, const void* ws, const Weight* const* w, int n, int T, bool add, cudaStream_t s);
+    void prefill_gemms(float* const* C, void* ws, const float* x, const float* norm_w, const Weight* const* w, int n, int T, bool add, cudaStream_t s);
+    bool ensure_block_scratch();
+    void* block_scratch_ = nullptr;
     bool ensure_short_buffers();
     void prefill_short(const int* tokens, int seq_len, int start_pos);
-    struct { float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *act = nullptr, *scratch = nullptr; void* xr = nullptr;
+    struct { float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *g = nullptr, *u = nullptr, *scratch = nullptr; void* ws = nullptr;
              int *tok = nullptr, *pos = nullptr; } sb_;       // a few tokens together
     void clear_kv();
     // Opt-in (also NT_B200_MEGAKERNEL=1): run the decode step as one persistent kernel (engine/decode_mega.h) instead of

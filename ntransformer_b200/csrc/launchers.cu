@@ -164,7 +164,14 @@ int nt_b200_gemm_blocks_ws(int n_mat, float* const* C, const void* const* W, con
     if (n_mat < 1 || n_mat > 3) return -1;
     nt::b200::GemvMat m[3];
     for (int i = 0; i < n_mat; i++) { m[i].W = W[i]; m[i].y = C[i]; m[i].out = out_features[i]; m[i].dtype = (DType)dtypes[i]; m[i].row_pitch = 0; }
-    return nt::b200::gemm_blocks(m, n_mat, in_features, workspace, tokens, add != 0, static_cast<cudaStream_t>(stream)) ? 0 : -2;
+    return nt::b200::gemm_blocks(m, n_mat, in_features, nullptr, nullptr, 0.f, workspace, false, tokens, add != 0, static_cast<cudaStream_t>(stream)) ? 0 : -2;
+}
+int nt_b200_gemm_blocks(int n_mat, float* const* C, const void* const* W, const int* out_features, const int* dtypes, int in_features, const float* x,
+                        const float* norm_w, float eps, int tokens, int fine, int add, void* stream) {
+    if (n_mat < 1 || n_mat > 3 || !x) return -1;
+    nt::b200::GemvMat m[3];
+    for (int i = 0; i < n_mat; i++) { m[i].W = W[i]; m[i].y = C[i]; m[i].out = out_features[i]; m[i].dtype = (DType)dtypes[i]; m[i].row_pitch = 0; }
+    return nt::b200::gemm_blocks(m, n_mat, in_features, x, norm_w, eps, nullptr, fine != 0, tokens, add != 0, static_cast<cudaStream_t>(stream)) ? 0 : -2;
 }
 size_t nt_b200_attention_decode_scratch_floats(int ms, int nh, int nkv, int hd) { return nt::b200::attention_decode_dyn_scratch_floats(ms, nh, nkv, hd); }
 int nt_b200_attention_decode_tickets(int nh, int nkv) { return nt::b200::attention_decode_fused_tickets(nh, nkv); }

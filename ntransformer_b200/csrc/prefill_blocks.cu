@@ -1,24 +1,29 @@
-// prefill_blocks.cu — tensor-core GEMM of prompts over matrices in GGUF blocks: Y[T, N] (+)= X[T, K] . W[N, K]^T, W expanded on the way to the MMA.
+// prefill_blocks.cu — tensor-core GEMM of several tokens over matrices in GGUF blocks: Y[T, N] (+)= X[T, K] . W[N, K]^T, W expanded on the way to the MMA.
 //
-// The reference has no batched product (prefill loops its GEMV over the tokens, src/model/attention.cpp:144-162, ffn.cpp:96-133).  The form this
-// replaces wrote each matrix out as a pair of F16 matrices W_hi + W_lo (12 bytes of traffic for a 0.6-byte weight) and ran two GEMMs over it, four
-// products of halves in all, on 128 x 256 tiles of which a narrow matrix fills few.  Here a CTA owns 128 rows of W and NT tokens:
-//   * the roles of the operands are exchanged: W is A (M = 128 rows), tokens are B (N = NT, any multiple of 16 up to 256, chosen so that the tiles
-//     fill whole waves of the SMs);
-//   * sixteen warps expand 64 columns of the 128 rows at a time (eight each of two k-blocks in turn), a row to a lane: blocks come into shared memory by cp.async, the F32 value of a weight is
-//     split into F16 hi + lo (W = hi + lo to 2^-22 of it, or to 2^-25 where that is more: the least F16 halved) and stored to TENSOR MEMORY, from where tcgen05.mma takes its A operand: shared memory's bandwidth
-//     is left to B;
-//   * B is the split of the tokens (prefill_gemm.cu's workspace) by TMA; three products hi.hi, hi.lo, lo.hi (lo.lo, up to 2^-22 of a product and of either
-//     sign, leaves 4e-8 of a result; what follows is a hundred times that);
-//   * half of K, at most 2048 columns, to an accumulator, partial sums added in F32 by the epilogue: the tensor cores cut off each addition, which leaves
-//     1.86e-8 of the result for each.  The expanded form made 2 of them for 16 columns of up to 4096, this one makes 3 for 16 of half as many: error against 64 bits
-//     2.5e-6 -> 2.0e-6 at K = 1024, 9.7e-6 -> 7.1e-6 at 4096 (whole rows to 2048 left 3.6e-6 at 1024).
-// Llama-3 8B layer in Q4_K_M, 500 tokens: q/k/v 78 us (was 332 with the expansion), o 63 (173), gate + up 336 (604 and 40 for SwiGLU), down 201 (494); of
-// 1.9 us per 64 columns at first, 0.9 went into an epilogue that read C back before each addition (now red.add), 0.2 into an MMA loop of one lane.
+// The reference has no batched product (prefill loops its GEMV over the tokens, src/model/attention.cpp:144-162, ffn.cpp:96-133).  Here a CTA owns 128 rows of W
+// and NT tokens:
+//   * the roles of the operands are exchanged: W is A (M = 128 rows), tokens are B (N = NT, a multiple of 16 up to 128);
+//   * A holds INTEGERS.  A weight of Q4_K is d * (sc * q) - dmin * m, of Q5_K the same: sc * q <= 63 * 31 is exact in F16, so one F16 operand carries the weight
+//     and d joins when the epilogue takes a super-block's sum out of tensor memory.  The minima are a product of their own, m (8 for a super-block) times the sums
+//     of 32 activations.  Q6_K's sc * (q - 32) has up to 14 bits: a pair of halves, the second -1, 0 or 1.  Q8_0 and Q4_0 have a scale for 32 weights: d_i * q as
+//     a pair of halves, exact, under a power of two for the super-block;
+//   * eight warps expand 64 columns of 128 rows at a time, a row to a lane: blocks come into shared memory by cp.async, two halves cost a PRMT and an HFMA2,
+//     and go to TENSOR MEMORY, from where tcgen05.mma takes its A operand: shared memory's bandwidth is left to B;
+//   * B is the split of the tokens x = hi + lo by TMA: two products for 16 columns (hi, lo), a third with the low half of a pair;
+//   * a super-block (256 columns; half of one where a row has no more, 64 where the caller asks for it) to an accumulator: the tensor cores cut off each addition, which leaves 1.86e-8 of a sum for
+//     each.  The epilogue's eight warps add the sums in F32 registers, times d, and write C once;
+//   * the work, tiles times super-blocks, is dealt out evenly: a CTA takes a run of super-blocks, whichever tiles it touches.  A tile that several CTAs share goes
+//     to a scratch, and whoever comes last adds the shares in their order (nothing waits for another CTA, the sums do not depend on who was last).
+// Measured (gate and up of an 8B layer, 28672 x 4096 Q4_K; the form before, which expanded each weight to a pair of halves, beside it): 500 tokens 341 -> 218 us, bound by
+// the tokens' way from L2 (49 bytes a clock and SM, 128 x 128 tiles with two halves of each token ask for 64); 21 tokens 100 (24-bit integers, three passes) -> 58 us,
+// bound by the chain of barriers and instructions that a k-block takes (700 cycles, whatever the tokens).
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "tc_device.cuh"
+#include "wait_status.cuh"
 #include "gemv_mma_device.cuh"
+#include <cuda.h>
+#include <cuda_fp16.h>
 #include <algorithm>
 
 namespace nt { namespace b200 {
@@ -26,162 +31,223 @@ namespace nt { namespace b200 {
 namespace {
 
 constexpr int QBK = 64;                                  // columns of a k-block: a 128-byte swizzle row of F16
-constexpr int A_STAGES = 4, A_COLS = 64;             // tensor-memory columns of an expanded k-block: 32 hi, 32 lo; the accumulators lie behind them
-constexpr int D_COL = A_STAGES * A_COLS;
-constexpr int KC_MAX = 2048 / QBK;                       // k-blocks to an accumulator, at most
-constexpr int B_STAGES_MAX = 4;
-constexpr int Q_THREADS = 22 * 32;                       // warp 0 TMA, 1 MMA, 2-5 epilogue, 6-21 expansion
+constexpr int NT_MAX = 128;                              // tokens of a tile
+constexpr int STAGES_MAX = 4, D_BUFS_MAX = 4, RAW_MAX = 8, SCALE_RING = 8;
+constexpr int EPI_WARP = 4, EXP_WARP = 12, Q_THREADS = 20 * 32;      // warp 0 tokens, 1 MMA, 2 blocks (2, 3: off 16 bytes), 4-11 epilogue, 12-19 expansion
 
-__host__ __device__ constexpr int raw_pitch(int fmt) { return fmt == 2 ? 240 : fmt_bytes(fmt); }       // odd 16-byte units; Q6_K: the 14 units around a block
+// Bytes between rows of a super-block in shared memory: an odd number of 16-byte units.  Q6_K lies at any even address: the units around it.
+__host__ __device__ constexpr int raw_pitch(int fmt) { return fmt == 2 ? 240 : fmt_bytes(fmt); }
+__host__ __device__ constexpr bool has_mins(int fmt) { return fmt <= 1; }      // otherwise A is a pair of halves
 
 struct BlkMat { const uint8_t* W; float* C; int rows, tiles, fmt; long long pitch; };
+struct alignas(64) BlkMaps { CUtensorMap x, sums, w[3]; };      // tokens, their sums, matrices as 32-bit words
 struct BlkParams {
     BlkMat mat[3];
-    int n_mat, T, NT, cols, n_tiles, Mp, K, kc, add, b_stages, raw_depth, raw_slot, d_bufs;
+    int n_mat, T, NT, cols, Mp, NB, kc, add, grain, stages, b_stage, raw_depth, raw_slot, a_cols, d_bufs;
+    int tma;                   // a matrix's rows come by TMA (bits)
+    int units;                 // tiles * super-blocks
+    const float* scale;        // of a token's products
+    float* part;               // two tiles to a CTA
+    unsigned* count;           // one to a CTA
     unsigned* status;          // wait_status.cuh
 };
 
-// tcgen05.mma with A in tensor memory
-__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-                 ::"r"(d), "r"(a), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+// tcgen05.mma with A in tensor memory, and its commit, by the lane that `lead` marks.  Predicated, no branch: the operands stay in uniform registers.
+__device__ __forceinline__ void umma_ts(uint32_t lead, uint32_t d, uint32_t a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                 ::"r"(d), "r"(a), "l"(db), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
 }
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
+__device__ __forceinline__ void umma_commit_by(uint32_t lead, uint64_t* bar) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
+                 ::"r"(smem_u32(bar)), "r"(lead) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
                  ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
                  "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
-__device__ __forceinline__ void copy16(uint32_t dst, const uint8_t* src, int bytes) {       // the first `bytes`, zeros behind them
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+__device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&v)[4]) {      // the four words twice
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
-// 8 rows of super-block b into a slot: four lanes to a row, 64 contiguous bytes an instruction; rows behind the matrix are its last one, and nothing
-// behind the matrix's end is read
-template <int FMT>
+// 16 accumulator columns as pairs
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+                   "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(addr));
+}
+// K-major rows of 32 bytes under SWIZZLE_32B: eight rows are 256 bytes (make_desc's layout with type 6)
+__device__ __forceinline__ uint64_t make_desc32(const void* smem_ptr) {
+    const uint64_t addr = (uint64_t)(smem_u32(smem_ptr) & 0x3FFFFu) >> 4;
+    return addr | (1ull << 16) | ((uint64_t)(256 >> 4) << 32) | (1ull << 46) | (6ull << 61);
+}
+__device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+
+// Q6_K rows that do not lie 16 bytes apart, which TMA does not take: 64 rows of super-block b into a slot by units, four lanes to a row.  Rows behind the matrix are
+// its last one, and nothing behind the matrix's end is read.
 __device__ __forceinline__ void copy_rows(uint32_t slot, const BlkMat& m, int row, int b, int NB, int lane) {
-    constexpr int PITCH = raw_pitch(FMT), UNITS = FMT == 2 ? 14 : fmt_bytes(FMT) / 16;
-    const uint8_t* end = m.W + (long long)(m.rows - 1) * m.pitch + (long long)NB * fmt_bytes(FMT);
-    {
-        const int r = lane >> 2;
-        const uint8_t* p = m.W + (long long)min(row + r, m.rows - 1) * m.pitch + (long long)b * fmt_bytes(FMT);
-        if (FMT == 2) p = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)15);
+    constexpr int PITCH = raw_pitch(2), UNITS = 14;
+    const uint8_t* end = m.W + (long long)(m.rows - 1) * m.pitch + (long long)NB * fmt_bytes(2);
+#pragma unroll 2
+    for (int r = lane >> 2; r < 64; r += 8) {
+        const uint8_t* p = m.W + (long long)min(row + r, m.rows - 1) * m.pitch + (long long)b * fmt_bytes(2);
+        p = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)15);
+        const int left = (int)min((long long)(end - p), 256ll);
 #pragma unroll
         for (int i = 0; i < (UNITS + 3) / 4; i++) {
-            const int u = 4 * i + (lane & 3);
-            if (u >= UNITS) break;
-            const long long left = end - (p + 16 * u);
-            copy16(slot + r * PITCH + 16 * u, left > 0 ? p + 16 * u : m.W, FMT == 2 ? (int)max(0ll, min(16ll, left)) : 16);
+            const int u = 4 * i + (lane & 3), n = min(16, left - 16 * u);
+            if (u < UNITS && n > 0) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(slot + r * PITCH + 16 * u), "l"(p + 16 * u), "r"(n) : "memory");
         }
     }
 }
 
-__device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
-__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-// 32 consecutive weights of this lane's row — half hf of k-block c (0..3) of the super-block — as F16 pairs hi and lo, two columns of K to a word.
-// blk: the block in shared memory.
+__device__ __forceinline__ __half2 h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+__device__ __forceinline__ uint32_t bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+// bytes i, j of w as halves 1024 + byte
+template <int I, int J> __device__ __forceinline__ __half2 half_pair(uint32_t w) { return h2(__byte_perm(w, 0x64646464u, 0x4040u | I | (J << 8))); }
+__device__ __forceinline__ __half2 half_twice(uint32_t w, int i) { return h2(__byte_perm(w, 0x64646464u, 0x4040u + 0x0101u * i)); }
+
+// The scales and minima of a Q4_K / Q5_K super-block as bytes: sub-blocks 0-3 or 4-7
+__device__ __forceinline__ uint32_t kq_scales(const uint4& h, bool upper) { return upper ? (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u) : h.y & 0x3F3F3F3Fu; }
+__device__ __forceinline__ uint32_t kq_mins(const uint4& h, bool upper) { return upper ? ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u) : h.z & 0x3F3F3F3Fu; }
+
+// k-block c (64 columns) of a Q4_K / Q5_K super-block: sc * q, two columns to a word
 template <int FMT>
-__device__ __forceinline__ void expand32(const uint8_t* blk, int c, int hf, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
-    uint32_t q[8];                                                 // codes, four to a word, unsigned
-    float off, D[2], M;                                            // weight = D (code - off) - M, D of the first and the second 16
-    M = 0.f;
-    if (FMT <= 1) {
-        const uint4 h = lds128(blk), a = lds128(blk + (FMT == 0 ? 16 : 48) + 32 * c), b = lds128(blk + (FMT == 0 ? 32 : 64) + 32 * c);
-        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        const int sub = 2 * c + hf;
-        const uint32_t ss = sub < 4 ? h.y & 0x3F3F3F3Fu : (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
-        const uint32_t mm = sub < 4 ? h.z & 0x3F3F3F3Fu : ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
-        D[0] = D[1] = half_bits(h.x & 0xFFFFu) * magic_byte(ss, 0x7440u + (sub & 3));
-        M = half_bits(h.x >> 16) * magic_byte(mm, 0x7440u + (sub & 3));
-        off = 8388608.0f;
+__device__ __forceinline__ void expand_k(const uint8_t* blk, const uint4& h, int c, uint32_t (&out)[32]) {
+    const uint4 a = lds128(blk + (FMT == 0 ? 16 : 48) + 32 * c), b = lds128(blk + (FMT == 0 ? 32 : 64) + 32 * c);
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t v[8];
+    if (FMT == 1) {
+        const uint4 e = lds128(blk + 16), f = lds128(blk + 32);
+        const uint32_t u[8] = {e.x, e.y, e.z, e.w, f.x, f.y, f.z, f.w};
 #pragma unroll
-        for (int i = 0; i < 8; i++) q[i] = (w[i] >> (4 * hf)) & 0x0F0F0F0Fu;
-        if (FMT == 1) {
-            const uint4 e = lds128(blk + 16), f = lds128(blk + 32);
-            const uint32_t v[8] = {e.x, e.y, e.z, e.w, f.x, f.y, f.z, f.w};
+        for (int i = 0; i < 8; i++) v[i] = u[i] >> (2 * c);        // bits 0 and 1: the fifth bits of the two sub-blocks
+    }
+    const uint32_t ss = kq_scales(h, c >= 2);
+    const __half2 k = __float2half2_rn(1024.0f), neg = __float2half2_rn(-1024.0f);
 #pragma unroll
-            for (int i = 0; i < 8; i++) q[i] |= ((v[i] >> sub) & 0x01010101u) << 4;
+    for (int s = 0; s < 2; s++) {
+        const __half2 sc = __hsub2(half_twice(ss, 2 * (c & 1) + s), k), off = __hmul2(sc, neg);      // -1024 sc: exact, up to 64512
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            uint32_t q = (s ? w[i] >> 4 : w[i]) & 0x0F0F0F0Fu;
+            if (FMT == 1) q |= (s ? v[i] << 3 : v[i] << 4) & 0x10101010u;
+            out[16 * s + 2 * i] = bits(__hfma2(half_pair<0, 1>(q), sc, off));
+            out[16 * s + 2 * i + 1] = bits(__hfma2(half_pair<2, 3>(q), sc, off));
         }
+    }
+}
+
+// N words from any even address, by whole units (32-bit loads of rows an odd number of units apart would meet four to a bank)
+template <int N> __device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t (&w)[N]) {
+    constexpr int UNITS = (N + 7) / 4;
+    const uint32_t at = smem_u32(p), sel = (at & 2u) ? 0x5432u : 0x3210u;
+    const uint8_t* a = p - (at & 15u);
+    uint32_t u[4 * UNITS];
+#pragma unroll
+    for (int i = 0; i < UNITS; i++) { const uint4 v = lds128(a + 16 * i); u[4 * i] = v.x; u[4 * i + 1] = v.y; u[4 * i + 2] = v.z; u[4 * i + 3] = v.w; }
+#pragma unroll
+    for (int i = 0; i < N + 2; i++) u[i] = (at & 8u) ? u[i + 2] : u[i];
+#pragma unroll
+    for (int i = 0; i < N + 1; i++) u[i] = (at & 4u) ? u[i + 1] : u[i];
+#pragma unroll
+    for (int i = 0; i < N; i++) w[i] = __byte_perm(u[i], u[i + 1], sel);
+}
+// Half hf of k-block c of the other formats as pairs of halves.  codes: what has to be taken off 1024 + code; D: the scale of the first and the second 16 columns
+__device__ __forceinline__ void pairs(const uint32_t (&q)[8], __half2 off, const __half2 (&D)[2], uint32_t (&hi)[16], uint32_t (&lo)[16]) {
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const __half2 v = __hsub2(j ? half_pair<2, 3>(q[i]) : half_pair<0, 1>(q[i]), off), p = __hmul2_rn(v, D[i >> 2]);
+            hi[2 * i + j] = bits(p);
+            lo[2 * i + j] = bits(__hfma2(v, D[i >> 2], __hneg2(p)));      // what the product's rounding left, exact
+        }
+}
+template <int FMT>
+__device__ __forceinline__ void expand_pair(const uint8_t* blk, int c, int hf, float up, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
+    uint32_t q[8];
+    __half2 D[2];
+    if (FMT == 2) {
+        // half h of the super-block, quarters q1 (codes in the low nibbles of the first 32 bytes, bits 0-1 of the pairs), q2 (second 32, bits 2-3), q3, q4
+        const int h = c >> 1, qt = 2 * (c & 1) + hf;
+        uint32_t w[8], v[8];
+        lds_words(blk + 64 * h + 32 * hf, w);
+        lds_words(blk + 128 + 32 * h, v);
+        const int8_t* sc = reinterpret_cast<const int8_t*>(blk + 192 + 8 * h + 2 * qt);
+        D[0] = __half2half2(__int2half_rn(sc[0])); D[1] = __half2half2(__int2half_rn(sc[1]));
+#pragma unroll
+        for (int i = 0; i < 8; i++) q[i] = ((w[i] >> (4 * (c & 1))) & 0x0F0F0F0Fu) | (((v[i] >> (2 * qt)) & 0x03030303u) << 4);
+        pairs(q, __float2half2_rn(1056.0f), D, hi, lo);
     } else {
-        auto words = [&](const uint8_t* p, uint32_t (&w)[8]) {     // 32 bytes from any even address
-            const uint32_t mis = smem_u32(p) & 2u, sel = mis ? 0x5432u : 0x3210u;
-            const uint32_t* a = reinterpret_cast<const uint32_t*>(p - mis);
-            uint32_t u = a[0];
-#pragma unroll
-            for (int i = 0; i < 8; i++) { const uint32_t n = (i < 7 || mis) ? a[i + 1] : 0u; w[i] = __byte_perm(u, n, sel); u = n; }
-        };
-        if (FMT == 2) {
-            // half h of the super-block, quarters q1 (codes in the low nibbles of the first 32 bytes, bits 0-1 of the pairs), q2 (second 32, bits 2-3), q3, q4
-            const int h = c >> 1, qt = 2 * (c & 1) + hf;
-            uint32_t w[8], v[8];
-            words(blk + 64 * h + 32 * hf, w);
-            words(blk + 128 + 32 * h, v);
-            const float d = half_bits(*reinterpret_cast<const uint16_t*>(blk + 208));
-            const int8_t* sc = reinterpret_cast<const int8_t*>(blk + 192 + 8 * h + 2 * qt);
-            D[0] = d * (float)sc[0]; D[1] = d * (float)sc[1];
-            off = 8388608.0f + 32.0f;
-#pragma unroll
-            for (int i = 0; i < 8; i++) q[i] = ((w[i] >> (4 * (c & 1))) & 0x0F0F0F0Fu) | (((v[i] >> (2 * qt)) & 0x03030303u) << 4);
-        } else if (FMT == 3) {
-            const uint8_t* b = blk + 34 * (2 * c + hf);
-            words(b + 2, q);
-            D[0] = D[1] = half_bits(*reinterpret_cast<const uint16_t*>(b));
-            off = 8388608.0f + 128.0f;
+        const uint8_t* b = blk + (FMT == 3 ? 34 : 18) * (2 * c + hf);
+        D[0] = D[1] = __float2half2_rn(half_bits(*reinterpret_cast<const uint16_t*>(b)) * up);
+        if (FMT == 3) {
+            lds_words(b + 2, q);
 #pragma unroll
             for (int i = 0; i < 8; i++) q[i] ^= 0x80808080u;
         } else {
-            const uint8_t* b = blk + 18 * (2 * c + hf);
-            const uint32_t mis = smem_u32(b + 2) & 2u, sel = mis ? 0x5432u : 0x3210u;
-            const uint32_t* a = reinterpret_cast<const uint32_t*>(b + 2 - mis);
-            D[0] = D[1] = half_bits(*reinterpret_cast<const uint16_t*>(b));
-            off = 8388608.0f + 8.0f;
+            uint32_t w[4];
+            lds_words(b + 2, w);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint32_t n = __byte_perm(a[i], (i < 3 || mis) ? a[i + 1] : 0u, sel);
-                q[i] = n & 0x0F0F0F0Fu;
-                q[4 + i] = (n >> 4) & 0x0F0F0F0Fu;
-            }
+            for (int i = 0; i < 4; i++) { q[i] = w[i] & 0x0F0F0F0Fu; q[4 + i] = (w[i] >> 4) & 0x0F0F0F0Fu; }
         }
-    }
-    const uint64_t off2 = pack2(-off, -off), m2 = pack2(-M, -M), one2 = pack2(-1.0f, -1.0f);
-#pragma unroll
-    for (int i = 0; i < 16; i++) {                                 // two weights at a time in packed F32 arithmetic
-        const float d = D[i >> 3];
-        const uint32_t w4 = q[i >> 1];
-        uint64_t w = add2(pack2(__uint_as_float(__byte_perm(w4, 0x4B000000u, 0x7440u + 2 * (i & 1))), __uint_as_float(__byte_perm(w4, 0x4B000000u, 0x7441u + 2 * (i & 1)))), off2);
-        w = fma2(w, pack2(d, d), m2);
-        float a, b;
-        unpack2(w, a, b);
-        const __half2 h = __floats2half2_rn(a, b);
-        const float2 f = __half22float2(h);
-        unpack2(fma2(pack2(f.x, f.y), one2, w), a, b);             // w - hi, exact
-        const __half2 l = __floats2half2_rn(a, b);
-        hi[i] = *reinterpret_cast<const uint32_t*>(&h);
-        lo[i] = *reinterpret_cast<const uint32_t*>(&l);
+        pairs(q, __float2half2_rn(FMT == 3 ? 1152.0f : 1032.0f), D, hi, lo);
     }
 }
+// Q8_0, Q4_0: the power of two that takes a super-block's largest scale to 16 .. 32 (the product's low half then lies far above the least F16 number), and its
+// inverse.  Scales that are zero, or not finite: 1.
+template <int FMT>
+__device__ __forceinline__ float block_power(const uint8_t* blk, float& inverse) {
+    int e = 0;
+    uint32_t top = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) top = max(top, (uint32_t)*reinterpret_cast<const uint16_t*>(blk + (FMT == 3 ? 34 : 18) * i) & 0x7FFFu);
+    if (top && top < 0x7C00u) e = (int)(__float_as_uint(half_bits(top)) >> 23) - 127 - 4;
+    inverse = __uint_as_float((uint32_t)(127 + e) << 23);
+    return __uint_as_float((uint32_t)(127 - e) << 23);
+}
 
-__global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ BlkParams p) {
+// MASK: the formats that a launch's matrices have (bits)
+template <int MASK>
+__global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_constant__ BlkMaps maps, const __grid_constant__ BlkParams p) {
+    constexpr bool ONE = (MASK & (MASK - 1)) == 0, MINS = (MASK & 3) != 0, PAIRS = (MASK & 28) != 0;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t b_full[B_STAGES_MAX], b_empty[B_STAGES_MAX], a_full[A_STAGES], a_empty[A_STAGES], d_full[2], d_empty[2];
-    __shared__ uint32_t tmem_base_smem;
+    // a stage is a k-block of the tokens (shared memory) and of W (tensor memory) under one pair of barriers
+    __shared__ uint64_t full[STAGES_MAX], empty[STAGES_MAX], d_full[D_BUFS_MAX], d_empty[D_BUFS_MAX];
+    __shared__ uint64_t raw_full[RAW_MAX], raw_empty[RAW_MAX], s_full[SCALE_RING];
+    __shared__ float2 scales[SCALE_RING][128];                     // of a super-block's rows: what its sum and what its minima's sum are multiplied by
+    __shared__ uint32_t tmem_base_smem, last_smem, dead_smem;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int NB = p.K / 256, num_kb = p.K / QBK, n_kc = (num_kb + p.kc - 1) / p.kc, NT = p.NT;
-    const uint32_t b_tile = (uint32_t)NT * 128, b_stage = 2 * b_tile;
-    uint8_t* raw = smem + (size_t)p.b_stages * b_stage;
-    auto place = [&](int tile, int& mi, int& row0, int& t0) {      // tokens inside: the CTAs of a wave share rows
-        const int rt = tile / p.cols;
-        t0 = (tile - rt * p.cols) * NT;
-        mi = 0;
-        int r = rt;
-        while (mi + 1 < p.n_mat && r >= p.mat[mi].tiles) { r -= p.mat[mi].tiles; mi++; }
-        row0 = r * 128;
+    const int NB = p.NB, NT = p.NT;
+    const uint32_t b_tile = (uint32_t)NT * 128, b_stage = (uint32_t)p.b_stage, dead = smem_u32(&dead_smem);
+    uint8_t* raw = smem + (size_t)p.stages * b_stage;
+    // this CTA's super-blocks: units [u0, u1), unit = tile * NB + super-block
+    auto first_unit = [&](int cta) { return (int)((long long)(p.units / p.grain) * cta / (int)gridDim.x) * p.grain; };
+    const int u0 = first_unit(blockIdx.x), u1 = first_unit(blockIdx.x + 1);
+    auto format = [&](int fmt) { return MASK == 1 ? 0 : MASK == 2 ? 1 : MASK == 4 ? 2 : MASK == 8 ? 3 : MASK == 16 ? 4 : fmt; };
+    auto mins_of = [&](int mi) { return ONE ? MINS : MINS && has_mins(p.mat[mi].fmt); };
+    const bool by_tma = !(MASK & 4) || p.tma == (1 << p.n_mat) - 1;      // all of W
+    // where a tile lies: tokens inside, so that the CTAs of a wave share rows
+    struct Place { int tile, b, mi, row0, t0; };
+    auto place = [&](Place& q) {
+        const int rt = q.tile / p.cols;
+        q.t0 = (q.tile - rt * p.cols) * NT;
+        int r = rt, mi = 0;
+        if (p.n_mat > 1 && r >= p.mat[0].tiles) { r -= p.mat[0].tiles; mi = 1; }
+        if (p.n_mat > 2 && mi == 1 && r >= p.mat[1].tiles) { r -= p.mat[1].tiles; mi = 2; }
+        q.mi = mi; q.row0 = r * 128;
     };
+    auto start = [&] { Place q; q.tile = u0 / NB; q.b = u0 - q.tile * NB; place(q); return q; };
+    auto next = [&](Place& q) { if (++q.b == NB) { q.b = 0; q.tile++; place(q); } };
     if (threadIdx.x == 0) {
-        for (int i = 0; i < p.b_stages; i++) { mbar_init(b_full + i, 1); mbar_init(b_empty + i, 1); }
-        for (int i = 0; i < A_STAGES; i++) { mbar_init(a_full + i, 8); mbar_init(a_empty + i, 1); }
-        for (int i = 0; i < 2; i++) { mbar_init(d_full + i, 1); mbar_init(d_empty + i, 4); }
+        for (int i = 0; i < p.stages; i++) { mbar_init(full + i, 5); mbar_init(empty + i, 1); }      // the tokens' producer and four warps of the expansion
+        for (int i = 0; i < p.d_bufs; i++) { mbar_init(d_full + i, 1); mbar_init(d_empty + i, 8); }
+        for (int i = 0; i < p.raw_depth; i++) { mbar_init(raw_full + i, by_tma ? 1 : 65); mbar_init(raw_empty + i, 8); }
+        for (int i = 0; i < SCALE_RING; i++) mbar_init(s_full + i, 4);
+        dead_smem = 0;
         mbar_fence_init();
     }
     if (warp == 1) {
@@ -191,185 +257,383 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_base_smem;
+    // tensor memory is this CTA's whole (its address is 0): sums, expanded k-blocks, minima
+    const uint32_t a_base = (uint32_t)(p.d_bufs * NT), m_base = a_base + (uint32_t)(p.stages * p.a_cols);
 
+    // registers: 640 threads x 96 at launch; 56 + 2 x 120 + 2 x 88 for the five warpgroups are no more
+    if (warp < EPI_WARP) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 0) {
         if (lane == 0) {                                           // ---- tokens by TMA ----
             uint32_t st = 0, par = 1, filled = 0;
-            uint32_t tries = WAIT_TRIES;                                     // 0: a wait of this thread has run out
-            for (int tile = blockIdx.x; tile < p.n_tiles && tries; tile += gridDim.x) {
-                int mi, row0, t0;
-                place(tile, mi, row0, t0);
-                for (int kb = 0; kb < num_kb; kb++) {
-                    wait_phase(b_empty + st, par, p.status, tries);
-                    if (!tries) {
-                        for (uint32_t s = 0; s < filled; s++) wait_flight(b_full + s, s < st ? par ^ 1u : par);      // the copies in flight
+            Place q = start();
+            for (int u = u0; u < u1; u++, next(q)) {
+                const bool mins = mins_of(q.mi);
+                for (int kb = 0; kb < 4; kb++) {
+                    wait_cta(empty + st, par, dead);
+                    if (word_set(dead)) {
+                        for (uint32_t s = 0; s < filled; s++) wait_flight(full + s, s < st ? par ^ 1u : par);      // the copies in flight
+                        u = u1;
                         break;
                     }
-                    filled = min(filled + 1, (uint32_t)p.b_stages);
+                    filled = min(filled + 1, (uint32_t)p.stages);
                     uint8_t* d = smem + (size_t)st * b_stage;
-                    mbar_expect_tx(b_full + st, b_stage);
-                    tma_load_2d(d, &map_x, kb * QBK, t0, b_full + st);
-                    tma_load_2d(d + b_tile, &map_x, kb * QBK, p.Mp + t0, b_full + st);      // the lo halves lie Mp rows below
-                    if (++st == (uint32_t)p.b_stages) { st = 0; par ^= 1; }
+                    mbar_expect_tx(full + st, 2 * b_tile + (mins && kb == 3 ? NT * 32u : 0u));
+                    tma_load_2d(d, &maps.x, q.b * 256 + kb * QBK, q.t0, full + st);
+                    tma_load_2d(d + b_tile, &maps.x, q.b * 256 + kb * QBK, p.Mp + q.t0, full + st);      // the lo halves lie Mp rows below
+                    if (mins && kb == 3) tma_load_2d(d + 2 * b_tile, &maps.sums, q.b * 16, q.t0, full + st);
+                    if (++st == (uint32_t)p.stages) { st = 0; par ^= 1; }
                 }
             }
         }
     } else if (warp == 1) {
         // ---- MMA: the whole warp walks the loop, so that addresses and descriptors stay in uniform registers, and one lane issues (a loop of lane 0
         // alone moved every operand of every MMA there: about 100 cycles an instruction) ----
-        const bool leader = elect_lane();
+        const uint32_t lead = elect_lane();
         const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | (8u << 24);      // D F32, A and B F16 K-major, N, M = 128
-        const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
-        const uint64_t desc0 = make_desc(smem), lo_step = (uint64_t)(b_tile >> 4), stage_step = (uint64_t)(b_stage >> 4);
-        uint32_t bs = 0, bpar = 0, as = 0, apar = 0, db = 0, dpar = 1;
-        uint32_t tries = WAIT_TRIES;                                         // 0: a wait of this lane has run out
+        const uint64_t desc0 = make_desc(smem), desc32 = make_desc32(smem), lo_step = (uint64_t)(b_tile >> 4), stage_step = (uint64_t)(b_stage >> 4);
+        uint32_t st = 0, par = 0, db = 0, dpar = 1;
         int last = -1;                                             // stage and parity of the last commit
-        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x)
-            for (int kc = 0; kc < n_kc; kc++) {
-                wait_phase(d_empty + db, dpar, p.status, tries);
-                const uint32_t d = tm + D_COL + db * NT;
-                const int kb0 = kc * p.kc, kb1 = min(num_kb, kb0 + p.kc);
-                for (int kb = kb0; kb < kb1; kb++) {
-                    wait_phase(b_full + bs, bpar, p.status, tries);
-                    wait_phase(a_full + as, apar, p.status, tries);
+        Place q = start();
+        for (int u = u0; u < u1; u++, next(q)) {
+            const bool mins = mins_of(q.mi);
+#pragma unroll 1
+            for (int k0 = 0; k0 < 4; k0 += p.kc) {
+                wait_cta(d_empty + db, dpar, dead);
+                const uint32_t d = db * NT;
+#pragma unroll 1
+                for (int kb = k0; kb < k0 + p.kc; kb++) {
+                    wait_cta(full + st, par, dead);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t bh = desc0 + bs * stage_step, bl = bh + lo_step;
-                    const uint32_t ah = tm + as * A_COLS, al = ah + 32;
-                    if (leader && tries) {
+                    const uint64_t bh = desc0 + st * stage_step, bl = bh + lo_step;
+                    const uint32_t ah = a_base + st * p.a_cols, al = ah + 32, acc = kb != k0;
+                    if (PAIRS && (ONE || !mins)) {                 // the small products first
+                        umma_ts(lead, d, al, bh, idesc, acc);
 #pragma unroll
-                        for (int k = 0; k < 4; k++) umma_ts(d, al + 8 * k, bh + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);      // the small products first
+                        for (int k = 1; k < 4; k++) umma_ts(lead, d, al + 8 * k, bh + 2 * k, idesc, 1u);
+                        umma_ts(lead, d, ah, bl, idesc, 1u);
+                    } else umma_ts(lead, d, ah, bl, idesc, acc);
 #pragma unroll
-                        for (int k = 0; k < 4; k++) umma_ts(d, ah + 8 * k, bl + 2 * k, idesc, 1u);
+                    for (int k = 1; k < 4; k++) umma_ts(lead, d, ah + 8 * k, bl + 2 * k, idesc, 1u);
 #pragma unroll
-                        for (int k = 0; k < 4; k++) umma_ts(d, ah + 8 * k, bh + 2 * k, idesc, 1u);
-                        umma_commit(b_empty + bs);
-                        umma_commit(a_empty + as);
-                        last = (int)(as * 2 + apar);
-                        if (kb + 1 == kb1) umma_commit(d_full + db);
-                    }
-                    __syncwarp();
-                    if (++bs == (uint32_t)p.b_stages) { bs = 0; bpar ^= 1; }
-                    if (++as == A_STAGES) { as = 0; apar ^= 1; }
+                    for (int k = 0; k < 4; k++) umma_ts(lead, d, ah + 8 * k, bh + 2 * k, idesc, 1u);
+                    last = (int)(st * 2 + par);
+                    if (kb == 3 && mins) break;                    // its stage is free after the minima
+                    umma_commit_by(lead, empty + st);
+                    if (++st == (uint32_t)p.stages) { st = 0; par ^= 1; }
                 }
+                umma_commit_by(lead, d_full + db);
                 if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
             }
-        if (!tries && last >= 0) wait_flight(a_empty + (last >> 1), last & 1);      // given up: the products in flight
-    } else if (warp < 6) {                                         // ---- epilogue: a lane is a row of W, so a warp stores 128 contiguous bytes for each token ----
-        const int quarter = warp & 3;
-        uint32_t db = 0, dpar = 0;
-        uint32_t tries = WAIT_TRIES;
-        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
-            int mi, row0, t0;
-            place(tile, mi, row0, t0);
-            const BlkMat& m = p.mat[mi];
-            const int row = row0 + quarter * 32 + lane, live = min(NT, p.T - t0);
-            for (int kc = 0; kc < n_kc; kc++) {
-                wait_phase(d_full + db, dpar, p.status, tries);
+            if (MINS && mins) {                                    // minima: 8 of them times the halves of 8 sums, twice
+                wait_cta(d_empty + db, dpar, dead);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem + ((uint32_t)(quarter * 32) << 16) + D_COL + db * NT;
-                const bool add = p.add || kc > 0;
-                float* c = m.C + (size_t)t0 * m.rows + row;
+                umma_ts(lead, db * NT, m_base, desc32 + st * stage_step + 2 * lo_step, idesc, 0u);
+                umma_commit_by(lead, empty + st);                  // (the minima's place is free with this stage)
+                umma_commit_by(lead, d_full + db);
+                if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
+                if (++st == (uint32_t)p.stages) { st = 0; par ^= 1; }
+            }
+        }
+        if (word_set(dead) && last >= 0) wait_flight(empty + (last >> 1), last & 1);      // given up: the products in flight
+    } else if (by_tma ? threadIdx.x == 64 : true) {
+        // ---- blocks of W: the 16-byte units around a super-block of 128 rows, by TMA; Q6_K rows off 16 bytes by cp.async from both warps ----
+        uint32_t st = 0, par = 1, filled = 0;
+        Place q = start();
+        for (int u = u0; u < u1; u++, next(q)) {
+            const BlkMat& m = p.mat[q.mi];
+            const int fmt = format(m.fmt);
+            wait_cta(raw_empty + st, par, dead);
+            if (word_set(dead)) {
+                for (uint32_t s = 0; s < filled && by_tma; s++) wait_flight(raw_full + s, s < st ? par ^ 1u : par);      // the copies in flight
+                break;
+            }
+            filled = min(filled + 1, (uint32_t)p.raw_depth);
+            uint8_t* d = raw + (size_t)st * p.raw_slot;
+            if (by_tma || (p.tma >> q.mi & 1)) {
+                if (threadIdx.x == 64) {
+                    mbar_expect_tx(raw_full + st, 128u * raw_pitch(fmt));
+                    tma_load_2d(d, &maps.w[q.mi], (q.b * fmt_bytes(fmt) & ~15) >> 2, q.row0, raw_full + st);
+                }
+                if (!by_tma) mbar_arrive(raw_full + st);
+            } else {
+                copy_rows(smem_u32(d) + (warp - 2) * 64 * raw_pitch(2), m, q.row0 + (warp - 2) * 64, q.b, NB, lane);
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(raw_full + st)) : "memory");
+                if (threadIdx.x == 64) mbar_arrive(raw_full + st);
+            }
+            if (++st == (uint32_t)p.raw_depth) { st = 0; par ^= 1; }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    } else if (warp < EXP_WARP) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
+        // ---- epilogue: a lane is a row of W; two warps share a quarter's rows, every other 16 tokens to each ----
+        const int quarter = warp & 3, half = (warp - EPI_WARP) >> 2, r = quarter * 32 + lane;
+        const uint32_t tq = ((uint32_t)(quarter * 32) << 16) + half * 16;
+        uint32_t db = 0, dpar = 0, slot = 0, spar = 0;
+        Place q = start();
+        for (int u = u0; u < u1;) {
+            const int sums = 4 / p.kc, chunks = sums + (MINS && mins_of(q.mi) ? 1 : 0);
+            const int seg0 = u, end = min(u1, u + (NB - q.b));
+            uint64_t acc[4][8] = {};                               // pairs of tokens
 #pragma unroll 1
-                for (int n = 0; n < live; n += 32) {               // an odd multiple of 16: the last 16 columns read are not this tile's (nor beyond the 512), and not used
-                    uint32_t v[32];
-                    tmem_ld32(d + (uint32_t)n, v);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (row < m.rows && tries) {
-                        // adds go to the memory's side (this lane is the element's only writer, so their order is fixed): nothing is waited for
+            for (; u < end; u++) {
+                wait_cta(s_full + slot, spar, dead);
+                const float2 s = scales[slot][r];
+                if (++slot == SCALE_RING) { slot = 0; spar ^= 1; }
+#pragma unroll 1
+                for (int c = 0; c < chunks; c++) {
+                    const float f = c == sums ? s.y : s.x;
+                    const uint64_t ff = pack2(f, f);
+                    wait_cta(d_full + db, dpar, dead);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                        for (int j = 0; j < 32; j++) {
-                            if (n + j >= live) break;
-                            float* o = c + (size_t)(n + j) * m.rows;
-                            if (add) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o), "f"(__uint_as_float(v[j])) : "memory");
-                            else *o = __uint_as_float(v[j]);
+                    for (int i = 0; i < 4; i++) {
+                        if (32 * i + 16 * half >= NT) break;
+                        uint32_t v[16];
+                        tmem_ld16(tq + db * NT + 32 * i, v);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int j = 0; j < 8; j++) acc[i][j] = fma2(pack2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), ff, acc[i][j]);
+                    }
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(d_empty + db);
+                    if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
+                }
+            }
+            const int live = min(NT, p.T - q.t0), rows = p.mat[q.mi].rows, row = q.row0 + r;
+            bool write = true;
+            if (end - seg0 < NB) {                                 // shared: to the scratch; whoever comes last adds
+                write = false;
+                const int tu = q.tile * NB, G = gridDim.x;
+                const int c0 = (int)(((long long)(tu + 1) * G - 1) / p.units), c1 = (int)(((long long)(tu + NB) * G - 1) / p.units);      // (grain 1 wherever tiles are shared)
+                float* mine = p.part + (size_t)(2 * blockIdx.x + (seg0 == u0 ? 0 : 1)) * 128 * NT + r;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int n = 32 * i + 16 * half;
+                    if (n >= live) break;
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        float x, y;
+                        unpack2(acc[i][j], x, y);
+                        __stcg(mine + (n + 2 * j) * 128, x);
+                        __stcg(mine + (n + 2 * j + 1) * 128, y);
+                    }
+                }
+                __threadfence();
+                named_sync<256>(5);
+                if (threadIdx.x == EPI_WARP * 32) {
+                    const bool alive = !word_set(dead);
+                    const bool is_last = alive && atomicAdd(p.count + c0, 1u) == (unsigned)(c1 - c0);
+                    if (is_last) p.count[c0] = 0;
+                    __threadfence();
+                    last_smem = is_last;
+                }
+                named_sync<256>(5);
+                if (last_smem) {
+                    write = true;
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+#pragma unroll
+                        for (int j = 0; j < 8; j++) acc[i][j] = 0;
+#pragma unroll 1
+                    for (int c = c0; c <= c1; c++) {
+                        const float* o = p.part + (size_t)(2 * c + (first_unit(c) >= tu ? 0 : 1)) * 128 * NT + r;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            const int n = 32 * i + 16 * half;
+                            if (n >= live) break;
+                            float v[16];
+#pragma unroll
+                            for (int j = 0; j < 16; j++) v[j] = __ldcg(o + (n + j) * 128);
+#pragma unroll
+                            for (int j = 0; j < 8; j++) {
+                                float x, y;
+                                unpack2(acc[i][j], x, y);
+                                acc[i][j] = pack2(x + v[2 * j], y + v[2 * j + 1]);
+                            }
                         }
                     }
                 }
+            }
+            if (write && row < rows && !word_set(dead)) {          // a warp stores 128 contiguous bytes for each token
+                float* o = p.mat[q.mi].C + (size_t)(q.t0 + 16 * half) * rows + row;
+                const float* ts = p.scale + q.t0 + 16 * half;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++) {
+                        if (32 * i + 16 * half + j >= live) break;
+                        float x, y;
+                        unpack2(acc[i][j >> 1], x, y);
+                        const float v = ((j & 1) ? y : x) * __ldg(ts + 32 * i + j);
+                        // adds go to the memory's side (this lane is the element's only writer): nothing is waited for
+                        if (p.add) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + (size_t)j * rows), "f"(v) : "memory");
+                        else o[(size_t)j * rows] = v;
+                    }
+                    o += (size_t)32 * rows;
+                }
+            }
+            q.b = 0; q.tile++;
+            place(q);
+        }
+        if (word_set(dead)) report(p.status);
+    } else {                                                       // ---- expansion: two warps share 32 rows; k-blocks 0, 2 or 1, 3 of a super-block to each ----
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+        const int quarter = warp & 3, odd = (warp - EXP_WARP) >> 2;
+        const uint32_t tq = (uint32_t)(quarter * 32) << 16;
+        int slot = 0, sslot = 0;
+        uint32_t st = odd, par = 1, rpar = 0;
+        Place q = start();
+        for (int u = u0; u < u1; u++, next(q)) {
+            const BlkMat& m = p.mat[q.mi];
+            const int fmt = format(m.fmt);
+            wait_cta(raw_full + slot, rpar, dead);
+            const uint8_t* blk = raw + (size_t)slot * p.raw_slot + (quarter * 32 + lane) * raw_pitch(fmt);
+            if ((MASK & 4) && fmt == 2) blk += ((uint32_t)min(q.row0 + quarter * 32 + lane, m.rows - 1) * (uint32_t)m.pitch + (uint32_t)q.b * 210u) & 15u;      // (W on 16 bytes)
+            float up = 1.f, down = 1.f;
+            if ((MASK & 8) && fmt == 3) up = block_power<3>(blk, down);
+            if ((MASK & 16) && fmt == 4) up = block_power<4>(blk, down);
+            if (!odd) {
+                float2 s = make_float2(down, 0.f);
+                if (MINS && fmt <= 1) { const uint32_t h = *reinterpret_cast<const uint32_t*>(blk); s = make_float2(half_bits(h & 0xFFFFu), -32.0f * half_bits(h >> 16)); }
+                if ((MASK & 4) && fmt == 2) s.x = half_bits(*reinterpret_cast<const uint16_t*>(blk + 208));
+                scales[sslot][quarter * 32 + lane] = s;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_full + sslot);
+            }
+            if (++sslot == SCALE_RING) sslot = 0;
+#pragma unroll 1
+            for (int c = odd; c < 4; c += 2) {
+                const uint32_t a = tq + a_base + st * p.a_cols;
+                if (MINS && fmt <= 1) {
+                    uint32_t v[32];
+                    const uint4 h = lds128(blk);
+                    if ((MASK & 1) && fmt == 0) expand_k<0>(blk, h, c, v);
+                    if ((MASK & 2) && fmt == 1) expand_k<1>(blk, h, c, v);
+                    wait_cta(empty + st, par, dead);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    tmem_st16(a, v);
+                    tmem_st16(a + 16, v + 16);
+                    if (c == 3) {                                  // (the product of the minima before came ahead of the commit that freed a stage of k-block 3 or later)
+                        uint32_t w[4];
+                        const __half2 k = __float2half2_rn(1024.0f);
+#pragma unroll
+                        for (int i = 0; i < 2; i++) {
+                            const uint32_t mm = kq_mins(h, i != 0);
+                            w[2 * i] = bits(__hsub2(half_pair<0, 1>(mm), k));
+                            w[2 * i + 1] = bits(__hsub2(half_pair<2, 3>(mm), k));
+                        }
+                        tmem_st8(tq + m_base, w);
+                    }
+                } else if (PAIRS) {
+#pragma unroll 1
+                    for (int hf = 0; hf < 2; hf++) {
+                        uint32_t hi[16], lo[16];
+                        if ((MASK & 4) && fmt == 2) expand_pair<2>(blk, c, hf, up, hi, lo);
+                        if ((MASK & 8) && fmt == 3) expand_pair<3>(blk, c, hf, up, hi, lo);
+                        if ((MASK & 16) && fmt == 4) expand_pair<4>(blk, c, hf, up, hi, lo);
+                        if (hf == 0) {
+                            wait_cta(empty + st, par, dead);
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        }
+                        tmem_st16(a + 16 * hf, hi);
+                        tmem_st16(a + 32 + 16 * hf, lo);
+                    }
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0 && tries) mbar_arrive(d_empty + db);
-                if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
+                if (lane == 0) mbar_arrive(full + st);
+                st += 2;
+                if (st >= (uint32_t)p.stages) { st -= p.stages; par ^= 1; }
             }
+            if (lane == 0) mbar_arrive(raw_empty + slot);          // (every lane has read what it stored)
+            if (++slot == p.raw_depth) { slot = 0; rpar ^= 1; }
         }
-    } else {                                                       // ---- expansion: four warps share 32 rows; half hf of the k-blocks 0, 2 or 1, 3 of a super-block to each ----
-        const int quarter = warp & 3, share = (warp - 6) >> 2, hf = share & 1, odd = share >> 1, depth = p.raw_depth;
-        uint8_t* ring = raw + (size_t)quarter * depth * p.raw_slot;
-        uint32_t as = odd, apar = 1;
-        // the sequence of super-blocks over this CTA's tiles, `depth - 1` copied ahead
-        int ct = blockIdx.x, cb = 0, cslot = 0, cmi = 0, crow = 0, ct0 = 0;
-        if (ct < p.n_tiles) place(ct, cmi, crow, ct0);
-        auto copy_next = [&]() {
-            if (ct < p.n_tiles) {
-                const BlkMat& m = p.mat[cmi];
-                const uint32_t dst = smem_u32(ring + (size_t)cslot * p.raw_slot) + (uint32_t)(share * 8 * raw_pitch(m.fmt));
-                const int row = crow + quarter * 32 + share * 8;
-                switch (m.fmt) {
-                    case 0: copy_rows<0>(dst, m, row, cb, NB, lane); break;
-                    case 1: copy_rows<1>(dst, m, row, cb, NB, lane); break;
-                    case 2: copy_rows<2>(dst, m, row, cb, NB, lane); break;
-                    case 3: copy_rows<3>(dst, m, row, cb, NB, lane); break;
-                    default: copy_rows<4>(dst, m, row, cb, NB, lane); break;
-                }
-                if (++cb == NB) { cb = 0; ct += gridDim.x; if (ct < p.n_tiles) place(ct, cmi, crow, ct0); }
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            if (++cslot == depth) cslot = 0;
-        };
-        for (int i = 0; i < depth - 1; i++) copy_next();
-        int slot = 0, pending = -1;
-        uint32_t tries = WAIT_TRIES;
-        auto stored = [&](int stage) {
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0 && tries) mbar_arrive(a_full + stage);
-        };
-        for (int tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x) {
-            int mi, row0, t0;
-            place(tile, mi, row0, t0);
-            const BlkMat& m = p.mat[mi];
-            const int fmt = m.fmt, row = min(row0 + quarter * 32 + lane, m.rows - 1);
-            for (int b = 0; b < NB; b++) {
-                if (depth == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
-                else asm volatile("cp.async.wait_group 0;" ::: "memory");
-                named_sync<128>(1 + quarter);                      // all rows have arrived, and all four warps are done with the slot copied into next
-                copy_next();
-                const uint8_t* blk = ring + (size_t)slot * p.raw_slot + lane * raw_pitch(fmt);
-                if (fmt == 2) blk += (int)(((uint64_t)row * (uint64_t)m.pitch + (uint64_t)b * 210u) & 15u);
-                if (++slot == depth) slot = 0;
-#pragma unroll 1
-                for (int c = odd; c < 4; c += 2) {
-                    uint32_t hi[16], lo[16];
-                    switch (fmt) {
-                        case 0: expand32<0>(blk, c, hf, hi, lo); break;
-                        case 1: expand32<1>(blk, c, hf, hi, lo); break;
-                        case 2: expand32<2>(blk, c, hf, hi, lo); break;
-                        case 3: expand32<3>(blk, c, hf, hi, lo); break;
-                        default: expand32<4>(blk, c, hf, hi, lo); break;
-                    }
-                    // the stores of the k-block before had this one's arithmetic to arrive in
-                    if (pending >= 0) stored(pending);
-                    wait_phase(a_empty + as, apar, p.status, tries);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a = tmem + ((uint32_t)(quarter * 32) << 16) + as * A_COLS + hf * 16;
-                    tmem_st16(a, hi);
-                    tmem_st16(a + 32, lo);
-                    pending = (int)as;
-                    as += 2;
-                    if (as >= A_STAGES) { as = odd; apar ^= 1; }
-                }
-            }
-        }
-        if (pending >= 0) stored(pending);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     __syncwarp();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512));
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_smem), "n"(512));
 }
 
+// ---- tokens ----
+// One block to a token: x (MODE 1: RMSNorm(x) * w, rmsnorm.cu:17-70's math; 2: silu(x) * w, gemm.cu:713-725's expression; 3: hi x and lo w of
+// a plain split, which may be the one written to) as F16 hi + lo, the sums of 32 of them
+// (a 32nd part, so that they stay within F16) as hi + lo, and the factor that undoes the token's power of two.  That power takes the largest to 2^13 .. 2^14, where the
+// low halves keep their bits.
+enum : int { TOK_PLAIN = 0, TOK_NORM = 1, TOK_SILU = 2, TOK_SPLIT = 3 };
+template <int MODE>
+__global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* lo, __half* __restrict__ sums, float* __restrict__ scale, const float* xin, const float* w,
+                                                           float eps, int K) {
+    constexpr int KEEP = 7;                                        // chunks of 2048 held in registers: rows to 14336
+    __shared__ float red[2][16];
+    const int tid = threadIdx.x;
+    const size_t at = (size_t)blockIdx.x * K;
+    const float* x = xin + at;
+    const float* y = MODE == TOK_SILU ? w + at : w;
+    auto value = [&](int i, float& ss) {                           // before the norm's factor
+        if (MODE == TOK_SPLIT) {
+            const uint2 a = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(xin) + at + i), b = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(w) + at + i);
+            const float2 a0 = __half22float2(h2(a.x)), a1 = __half22float2(h2(a.y)), b0 = __half22float2(h2(b.x)), b1 = __half22float2(h2(b.y));
+            return make_float4(a0.x + b0.x, a0.y + b0.y, a1.x + b1.x, a1.y + b1.y);
+        }
+        float4 a = *reinterpret_cast<const float4*>(x + i);
+        if (MODE == TOK_NORM) {
+            const float4 g = *reinterpret_cast<const float4*>(y + i);
+            ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+            a.x *= g.x; a.y *= g.y; a.z *= g.z; a.w *= g.w;
+        }
+        if (MODE == TOK_SILU) {
+            const float4 u = *reinterpret_cast<const float4*>(y + i);
+            auto f = [](float p, float q) { return p / (1.0f + expf(-p)) * q; };
+            a = make_float4(f(a.x, u.x), f(a.y, u.y), f(a.z, u.z), f(a.w, u.w));
+        }
+        return a;
+    };
+    float4 keep[KEEP];
+    float ss = 0.f, amax = 0.f, none = 0.f;
+    auto most = [&](const float4& a) { amax = fmaxf(amax, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w)))); };
+#pragma unroll
+    for (int c = 0; c < KEEP; c++) { const int i = c * 2048 + 4 * tid; if (i < K) { keep[c] = value(i, ss); most(keep[c]); } }
+    for (int i = KEEP * 2048 + 4 * tid; i < K; i += 2048) most(value(i, ss));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o); amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o)); }
+    if ((tid & 31) == 0) { red[0][tid >> 5] = ss; red[1][tid >> 5] = amax; }
+    __syncthreads();
+    float tot = 0.f, f = 1.f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) { tot += red[0][i]; amax = fmaxf(amax, red[1][i]); }
+    if (MODE == TOK_NORM) f = rsqrtf(tot / K + eps);
+    const uint32_t e = __float_as_uint(amax * f) >> 23 & 255u;     // not finite, or zero: as it is
+    const uint32_t up = e == 255u || e == 0u ? 127u : min(227u, max(27u, 267u - e));
+    f *= __uint_as_float(up << 23);
+    if (tid == 0) scale[blockIdx.x] = __uint_as_float((254u - up) << 23);
+    __half* h = hi + (size_t)blockIdx.x * K;
+    __half* l = lo + (size_t)blockIdx.x * K;
+    __half* sm = sums + (size_t)blockIdx.x * (K / 16);
+    auto put = [&](int i, float4 a) {
+        a.x *= f; a.y *= f; a.z *= f; a.w *= f;
+        uint2 ph, pl;
+        split_pair(a.x, a.y, 0, ph.x, pl.x);
+        split_pair(a.z, a.w, 0, ph.y, pl.y);
+        *reinterpret_cast<uint2*>(h + i) = ph;
+        *reinterpret_cast<uint2*>(l + i) = pl;
+        float s = (a.x + a.y) + (a.z + a.w);                       // K is a multiple of 256: whole warps
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, 1); s += __shfl_xor_sync(0xFFFFFFFFu, s, 2); s += __shfl_xor_sync(0xFFFFFFFFu, s, 4);
+        if ((tid & 7) == 0) {
+            s *= 1.0f / 32.0f;
+            const __half sh = __float2half_rn(s);
+            __half* q = sm + (i >> 8) * 16 + ((i >> 5) & 7);
+            q[0] = sh; q[8] = __float2half_rn(s - __half2float(sh));
+        }
+    };
+#pragma unroll
+    for (int c = 0; c < KEEP; c++) { const int i = c * 2048 + 4 * tid; if (i < K) put(i, keep[c]); }
+    for (int i = KEEP * 2048 + 4 * tid; i < K; i += 2048) put(i, value(i, none));
+}
 // silu(g) * u (gemm.cu:713-725's expression) straight into the split of the next product
 __global__ void __launch_bounds__(256) silu_split_kernel(uint2* __restrict__ hi, uint2* __restrict__ lo, const float4* __restrict__ g, const float4* __restrict__ u, size_t n4) {
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
@@ -382,53 +646,152 @@ __global__ void __launch_bounds__(256) silu_split_kernel(uint2* __restrict__ hi,
     hi[i] = h; lo[i] = l;
 }
 
+template <int MASK>
+void launch_blocks(const BlkMaps& maps, const BlkParams& p, int grid, size_t smem, cudaStream_t s) {
+    static unsigned long long configured = 0;      // bit per device id
+    opt_in_dynamic_smem(gemm_blocks_kernel<MASK>, 214 * 1024, configured);
+    launch_k(gemm_blocks_kernel<MASK>, dim3(grid), dim3(Q_THREADS), smem, s, maps, p);
+    count_launch();
+}
+
+size_t padded(int T) { return ((size_t)T + 127) / 128 * 128; }
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 148;
+}
+
 }  // namespace
 
 bool gemm_blocks_supported(const GemvMat* mats, int n_mat, int K) { return gemv_kq_any_pitch(mats, n_mat, K); }
 
-// C_i [T, rows_i] (+)= X . W_i^T with X split into `workspace` (split_activations / rmsnorm_split: hi rows, then lo rows Mp below)
-bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const void* workspace, int T, bool add, cudaStream_t s) {
+// [hi rows, lo rows (gemm_f16_tc_workspace_bytes)][sums][scales], rows padded to 128
+size_t block_tokens_bytes(int T, int K) { return gemm_f16_tc_workspace_bytes(T, K) + padded(T) * ((size_t)K / 8 + sizeof(float)); }
+size_t block_scratch_bytes() { const size_t n = (size_t)sm_count(); return n * (2 * 128 * NT_MAX * sizeof(float) + sizeof(unsigned)); }
+
+void zero_block_scratch(void* scratch, cudaStream_t s) {      // its counts
+    const size_t n = (size_t)sm_count() * sizeof(unsigned);
+    NT_CUDA_CHECK(cudaMemsetAsync(static_cast<uint8_t*>(scratch) + block_scratch_bytes() - n, 0, n, s));
+}
+
+BlockTokens block_tokens(void* workspace, int T, int K) {
+    BlockTokens t;
+    uint8_t* p = static_cast<uint8_t*>(workspace);
+    t.split = p;
+    t.sums = p + gemm_f16_tc_workspace_bytes(T, K);
+    t.scale = reinterpret_cast<float*>(p + gemm_f16_tc_workspace_bytes(T, K) + padded(T) * ((size_t)K / 8));
+    return t;
+}
+
+BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, float eps, int T, int K, cudaStream_t s) {
+    const BlockTokens t = block_tokens(workspace, T, K);
+    __half* hi = static_cast<__half*>(t.split);
+    __half* lo = hi + padded(T) * (size_t)K;
+    launch_k(norm_w ? split_tokens_kernel<TOK_NORM> : split_tokens_kernel<TOK_PLAIN>, dim3(T), dim3(512), 0, s, hi, lo, static_cast<__half*>(t.sums), t.scale, x, norm_w, eps, K);
+    count_launch();
+    return t;
+}
+BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, cudaStream_t s) {
+    const BlockTokens t = block_tokens(workspace, T, K);
+    __half* hi = static_cast<__half*>(t.split);
+    launch_k(split_tokens_kernel<TOK_SILU>, dim3(T), dim3(512), 0, s, hi, hi + padded(T) * (size_t)K, static_cast<__half*>(t.sums), t.scale, gate, up, 0.f, K);
+    count_launch();
+    return t;
+}
+BlockTokens resplit_tokens(void* workspace, const void* split, int T, int K, cudaStream_t s) {
+    const BlockTokens t = block_tokens(workspace, T, K);
+    __half* hi = static_cast<__half*>(t.split);
+    const size_t lo = padded(T) * (size_t)K;
+    launch_k(split_tokens_kernel<TOK_SPLIT>, dim3(T), dim3(512), 0, s, hi, hi + lo, static_cast<__half*>(t.sums), t.scale, static_cast<const float*>(split),
+             reinterpret_cast<const float*>(static_cast<const __half*>(split) + lo), 0.f, K);
+    count_launch();
+    return t;
+}
+
+bool gemm_blocks_for_few(const GemvMat* mats, int n_mat, int tokens) {
+    bool exact = true;
+    for (int i = 0; i < n_mat; i++) exact = exact && mats[i].dtype != DType::Q8_0 && mats[i].dtype != DType::Q4_0;
+    return tokens > 8 && exact;
+}
+
+bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, bool fine, int T, bool add, cudaStream_t s) {
     if (T <= 0 || !gemm_blocks_supported(mats, n_mat, K)) return false;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     BlkParams p{};
     p.status = wait_status();
-    p.n_mat = n_mat; p.T = T; p.K = K; p.add = add;
-    p.kc = std::min(KC_MAX, (K / QBK + 1) / 2);
-    p.Mp = (T + 127) / 128 * 128;
-    int tiles = 0, slot = 0;
+    p.n_mat = n_mat; p.T = T; p.NB = K / 256; p.add = add;
+    p.Mp = (int)padded(T);
+    p.scale = x.scale;
+    p.kc = fine ? 1 : p.NB == 1 ? 2 : 4;
+    int tiles = 0, slot = 0, mask = 0;
     for (int i = 0; i < n_mat; i++) {
         BlkMat& m = p.mat[i];
         m.W = static_cast<const uint8_t*>(mats[i].W); m.C = mats[i].y; m.rows = mats[i].out; m.tiles = (m.rows + 127) / 128;
         m.fmt = gemv_kq_format(mats[i].dtype);
         m.pitch = (long long)(mats[i].row_pitch ? mats[i].row_pitch : dtype_row_size(mats[i].dtype, K));
         tiles += m.tiles;
-        if (32 * raw_pitch(m.fmt) > slot) slot = 32 * raw_pitch(m.fmt);
+        slot = std::max(slot, 128 * raw_pitch(m.fmt));
+        mask |= 1 << m.fmt;
     }
-    // Tokens of a tile: the split of T that costs least in waves of the SMs times a tile's cycles for 64 columns, measured as 1050 + 5.7 NT (0.79, 0.98, 1.1
-    // and 1.3 us at 64, 128, 176 and 256 tokens: the expansion's instructions up to about 100 tokens, then MMA and the tokens' loads).
-    long long best = -1;
-    for (int cols = (T + 255) / 256; cols <= (T + 31) / 32; cols++) {
-        const int NT = ((T + cols - 1) / cols + 15) / 16 * 16, n = (T + NT - 1) / NT;
-        const long long cost = ((long long)tiles * n + sms - 1) / sms * (10500 + 57 * NT);
-        if (best < 0 || cost < best) { best = cost; p.NT = NT; p.cols = n; }
-    }
-    p.n_tiles = tiles * p.cols;
-    p.d_bufs = 2 * p.NT <= 512 - A_STAGES * A_COLS ? 2 : 1;
+    const bool mins = mask & 3, pairs = mask & 28;
+    p.cols = (T + NT_MAX - 1) / NT_MAX;
+    p.NT = ((T + p.cols - 1) / p.cols + 15) / 16 * 16;
+    p.units = tiles * p.cols * p.NB;
+    // tensor memory: buffers of sums, expanded k-blocks, 8 columns of minima.  Shared memory: the same stages of tokens, and blocks of W behind them (the deeper the
+    // fewer tokens there are: weights from HBM are then what bounds)
+    p.a_cols = pairs ? 64 : 32;
     p.raw_slot = slot;
-    const size_t cap = 226 * 1024 - 1024, b_stage = (size_t)p.NT * 256;
-    p.raw_depth = 2 * b_stage + 4 * 3 * (size_t)slot <= cap ? 3 : 2;
-    p.b_stages = (int)((cap - 4 * (size_t)p.raw_depth * slot) / b_stage);
-    if (p.b_stages > B_STAGES_MAX) p.b_stages = B_STAGES_MAX;
-    if (p.b_stages < 1) return false;
-    CUtensorMap map;
-    if (!tc_map_f16(&map, workspace, 2 * (uint64_t)p.Mp, (uint64_t)K, (uint32_t)p.NT)) return false;
-    static unsigned long long configured = 0;      // bit per device id
-    opt_in_dynamic_smem(gemm_blocks_kernel, 226 * 1024, configured);
-    gemm_blocks_kernel<<<p.n_tiles < sms ? p.n_tiles : sms, Q_THREADS, p.b_stages * b_stage + 4 * (size_t)p.raw_depth * slot + 1024, s>>>(map, p);
-    count_launch();
+    p.b_stage = (p.NT * (256 + (mins ? 32 : 0)) + 1023) / 1024 * 1024;
+    const size_t cap = 213 * 1024;
+    for (p.stages = STAGES_MAX; p.stages > 2; p.stages--) {
+        p.d_bufs = std::min(D_BUFS_MAX, (512 - p.stages * p.a_cols - (mins ? 8 : 0)) / p.NT);
+        if (p.d_bufs >= (mins ? 3 : 2) && (size_t)p.stages * p.b_stage + 2 * (size_t)slot <= cap) break;
+    }
+    p.d_bufs = std::min(D_BUFS_MAX, (512 - p.stages * p.a_cols - (mins ? 8 : 0)) / p.NT);
+    p.raw_depth = (int)std::min<size_t>(RAW_MAX, (cap - (size_t)p.stages * p.b_stage) / slot);
+    if (p.raw_depth < 1 || p.d_bufs < 2) return false;
+    // a run of super-blocks to a CTA; without a scratch whole tiles
+    p.grain = scratch ? 1 : p.NB;
+    const int grid = std::min(sms, p.units / p.grain);
+    if (scratch) {
+        p.part = static_cast<float*>(scratch);
+        p.count = reinterpret_cast<unsigned*>(p.part + (size_t)sms * 2 * 128 * NT_MAX);
+    }
+    BlkMaps maps;
+    if (!tc_map_f16(&maps.x, x.split, 2 * (uint64_t)p.Mp, (uint64_t)K, (uint32_t)p.NT) || !tc_map_f16_rows32(&maps.sums, x.sums, (uint64_t)p.Mp, (uint64_t)K / 16, (uint32_t)p.NT))
+        return false;
+    for (int i = 0; i < n_mat; i++) {
+        const BlkMat& m = p.mat[i];
+        if (m.pitch & 15) continue;
+        if (!tc_map_words(&maps.w[i], m.W, (uint64_t)m.rows, (uint64_t)p.NB * fmt_bytes(m.fmt), (uint64_t)m.pitch, (uint32_t)raw_pitch(m.fmt))) return false;
+        p.tma |= 1 << i;
+    }
+    const size_t smem = p.stages * (size_t)p.b_stage + (size_t)p.raw_depth * slot + 1024;
+    switch (mask) {
+        case 1: launch_blocks<1>(maps, p, grid, smem, s); break;
+        case 2: launch_blocks<2>(maps, p, grid, smem, s); break;
+        case 4: launch_blocks<4>(maps, p, grid, smem, s); break;
+        case 5: launch_blocks<5>(maps, p, grid, smem, s); break;
+        case 8: launch_blocks<8>(maps, p, grid, smem, s); break;
+        case 16: launch_blocks<16>(maps, p, grid, smem, s); break;
+        default: launch_blocks<31>(maps, p, grid, smem, s); break;
+    }
     return true;
+}
+
+// The same over F32 tokens, or (x null) over tokens that split_activations laid out; what it needs beside them lies in memory of this call's
+bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const float* norm_w, float eps, const void* split, bool fine, int T, bool add, cudaStream_t s) {
+    if (T <= 0 || !gemm_blocks_supported(mats, n_mat, K) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(norm_w) & 15)) return false;
+    const size_t tokens = (block_tokens_bytes(T, K) + 255) / 256 * 256;
+    void* mem = nullptr;
+    if (cudaMallocAsync(&mem, tokens + block_scratch_bytes(), s) != cudaSuccess) { cudaGetLastError(); return false; }
+    uint8_t* scratch = static_cast<uint8_t*>(mem) + tokens;
+    zero_block_scratch(scratch, s);
+    const BlockTokens t = x ? split_tokens(mem, x, norm_w, eps, T, K, s) : resplit_tokens(mem, split, T, K, s);
+    const bool ok = gemm_blocks(mats, n_mat, K, t, scratch, fine, T, add, s);
+    NT_CUDA_CHECK(cudaFreeAsync(mem, s));
+    return ok;
 }
 
 void silu_mul_split(void* workspace, const float* gate, const float* up, int rows, int cols, cudaStream_t s) {

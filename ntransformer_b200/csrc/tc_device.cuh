@@ -9,6 +9,10 @@ namespace nt { namespace b200 {
 
 // prefill_gemm.cu: 2-D F16 tensor [rows][cols] (cols contiguous), box = 64 cols x box_rows rows (<= 256), 128-byte swizzle
 bool tc_map_f16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+// rows of `bytes`, `pitch` (a multiple of 16) apart, as 32-bit words: box = box_bytes x 128 rows, no swizzle
+bool tc_map_words(CUtensorMap* map, const void* base, uint64_t rows, uint64_t bytes, uint64_t pitch, uint32_t box_bytes);
+// F16 with 16 cols to a box, 32-byte swizzle
+bool tc_map_f16_rows32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
 namespace {
 

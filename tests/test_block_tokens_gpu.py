@@ -1,0 +1,88 @@
+"""Tokens over GGUF blocks on the tensor cores (csrc/prefill_blocks.cu) through nt_b200_gemm_blocks: the dealing out of tiles, formats side by side, wide ranges of
+activations, and the precision of the form that takes a few tokens' place (csrc/gemv_rows.cu, 24-bit integers)."""
+import ctypes as C
+
+import pytest
+
+torch = pytest.importorskip("torch")
+from ntransformer_b200._lib import lib  # noqa: E402
+from ntransformer_b200.dtypes import DType  # noqa: E402
+from test_block_products_gpu import FORMATS, activations, arrays, matrix, rel, rows_product, stream  # noqa: E402
+
+pytestmark = [pytest.mark.gpu]
+
+
+def product(ys, Ws, outs, dts, x, fine=False, add=False, norm_w=None):
+    y, w, o, d = arrays(ys, Ws, outs, dts)
+    assert lib().nt_b200_gemm_blocks(len(Ws), y, w, o, d, x.shape[1], x.data_ptr(), norm_w.data_ptr() if norm_w is not None else None, 1e-5, x.shape[0], int(fine),
+                                     int(add), stream()) == 0
+    torch.cuda.synchronize()
+
+
+def bound(dt, columns):
+    """An addition to an accumulator leaves 2/3 of 2^-24 of it: one for 16 columns, twice (two halves of the tokens; a third product's are small), of sums that may
+    be twice the result's size where minima are taken off (codes are not centred); pairs of halves and F32 additions leave 2^-22."""
+    return 2 * columns // 16 * 2.0 ** -24 * 2 / 3 * (2 if dt in (DType.Q4_K_M, DType.Q5_K) else 1) + 2.0 ** -22
+
+
+# one tile shared by as many CTAs as it has super-blocks; tiles that start and end inside a CTA's run; more tiles than CTAs; several tiles of tokens; ragged Q6_K
+@pytest.mark.parametrize("dt", FORMATS, ids=lambda d: d.name)
+@pytest.mark.parametrize("tokens,rows,cols", [(2, 5, 256), (16, 128, 4096), (33, 300, 2816), (129, 257, 4096), (257, 20000, 512), (21, 4096, 14336), (384, 640, 1280)])
+@pytest.mark.parametrize("fine", [False, True])
+def test_products(dt, tokens, rows, cols, fine):
+    W, W64 = matrix(dt, rows, cols, rows)
+    x = activations(tokens, cols, cols)
+    ref = x.double() @ W64.T
+    y = torch.full((tokens + 1, rows), 7.0, device="cuda")
+    product([y], [W], [rows], [dt], x, fine)
+    assert rel(y[:tokens], ref) <= bound(dt, 64 if fine else 256) and (y[tokens] == 7.0).all()
+    again = torch.zeros_like(y)
+    product([again], [W], [rows], [dt], x, fine)
+    assert torch.equal(again[:tokens], y[:tokens])                 # the shares of a tile are added in one order
+    product([y], [W], [rows], [dt], x, fine, add=True)
+    assert rel(y[:tokens], 2 * ref) <= bound(dt, 64 if fine else 256) and (y[tokens] == 7.0).all()
+
+
+@pytest.mark.parametrize("dts", [(DType.Q4_K_M, DType.Q4_K_M, DType.Q6_K), (DType.Q5_K, DType.Q8_0, DType.Q6_K), (DType.Q4_0, DType.Q6_K), (DType.Q6_K, DType.Q5_K)])
+@pytest.mark.parametrize("cols", [2048, 1280])
+def test_formats_side_by_side_and_norm(dts, cols):
+    tokens, outs = 70, [300, 33, 128][: len(dts)]
+    mats = [matrix(d, o, cols, o) for d, o in zip(dts, outs)]
+    x, g = activations(tokens, cols, 3), 1 + 0.1 * activations(1, cols, 4)[0]
+    u = x.double() / (x.double().pow(2).mean(1, keepdim=True) + 1e-5).sqrt() * g.double()
+    ys = [torch.zeros(tokens, o, device="cuda") for o in outs]
+    product(ys, [m[0] for m in mats], outs, dts, x, norm_w=g)
+    for y, d, (_, W64) in zip(ys, dts, mats):
+        assert rel(y, u @ W64.T) <= bound(d, 256)
+
+
+@pytest.mark.parametrize("dt", FORMATS, ids=lambda d: d.name)
+def test_activations_of_any_size_and_what_a_nan_reaches(dt):
+    tokens, rows, cols = 9, 130, 1024
+    W, W64 = matrix(dt, rows, cols, 1)
+    x = activations(tokens, cols, 5)
+    for t, by in enumerate((1e-20, 1e-6, 0.01, 1.0, 3e4, 1e6, 1e12)):
+        x[t] *= by
+    x[7] = 0
+    x[8, 500] = float("nan")
+    y = torch.zeros(tokens, rows, device="cuda")
+    product([y], [W], [rows], [dt], x)
+    ref = x.double() @ W64.T
+    for t in range(7):
+        assert rel(y[t], ref[t]) <= bound(dt, 256), t
+    assert (y[7] == 0).all() and torch.isnan(y[8]).all()
+
+
+@pytest.mark.parametrize("dt", [DType.Q4_K_M, DType.Q5_K, DType.Q6_K], ids=lambda d: d.name)      # (Q8_0 and Q4_0 stay with the integers)
+@pytest.mark.parametrize("cols", [1024, 4096, 14336])
+@pytest.mark.parametrize("wild,by", [(0.0, 1.0), (0.01, 10.0)])
+def test_a_few_tokens_are_no_further_from_64_bits_than_24_bit_integers(dt, cols, wild, by):
+    tokens, rows = 21, 1024
+    W, W64 = matrix(dt, rows, cols, 9)
+    x = activations(tokens, cols, 10, wild, by) * 0.3
+    ref = x.double() @ W64.T
+    y, old = torch.zeros(tokens, rows, device="cuda"), torch.zeros(tokens, rows, device="cuda")
+    product([y], [W], [rows], [dt], x, fine=True)
+    rows_product([old], [W], [rows], [dt], x)
+    print("%s %d, %g of them x %g: %.2e here, %.2e integers" % (dt.name, cols, wild, by, rel(y, ref), rel(old, ref)))
+    assert rel(y, ref) <= 1.02 * rel(old, ref)

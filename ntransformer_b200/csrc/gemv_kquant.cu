@@ -46,8 +46,9 @@ struct KqParams {
     const float* x_f32;        //   F32 activations quantised in the prologue,
     const float* norm_w;       //   optionally as RMSNorm(x) * norm_w: the prologue quantises x * norm_w and sums x^2 in the same
     float eps;                 //   pass; the scalar rsqrt(mean(x^2) + eps) is applied to the results (exact up to round-off)
-    int total_groups;          // SWIGLU: groups of mat[0]
-    int n_seg;                 // segments (matrices) per group: 2 for SWIGLU else 1
+    int total_groups;          // groups of 16 rows of a matrix; SWIGLU: pairs of them, gate and up (two segments), or 8 rows of gate and the same 8 of up (halves)
+    int n_seg;                 // segments (matrices) per group
+    int halves;
     int epilogue;
     int stages, slot;          // depth of a team's ring and bytes of a stage
     unsigned* status;          // wait_status.cuh
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
     const int u0 = (int)blockIdx.x + team * (int)gridDim.x, ustep = (int)gridDim.x * TEAMS;      // few groups: a team in each CTA first
     auto format = [&](const KqMat& m) { return (MASK == 1) ? 0 : (MASK == 2) ? 1 : (MASK == 4) ? 2 : (MASK == 8) ? 3 : (MASK & 16) ? 4 : m.fmt; };
     auto locate = [&](int u, int seg, int& mi, int& gl) {       // matrix and local group of group u
-        if (p.n_seg == 2) { mi = seg; gl = u; return; }
+        if (p.n_seg == 2 || p.halves) { mi = seg; gl = u; return; }
         mi = 0; gl = u;
         while (mi + 1 < p.n_mat && gl >= p.mat[mi].groups) { gl -= p.mat[mi].groups; mi++; }
     };
@@ -134,8 +135,9 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
             for (int seg = 0; seg < p.n_seg; seg++) {
                 int mi, gl;
                 locate(u, seg, mi, gl);
+                if (p.halves) mi = (lane >> 3) & 1;
                 const KqMat& m = p.mat[mi];
-                const int fmt = format(m), blk = fmt_bytes(fmt), sblocks = stage_blocks(fmt, KW), row = gl * MROWS + lane;
+                const int fmt = format(p.mat[p.halves ? 0 : mi]), blk = fmt_bytes(fmt), sblocks = stage_blocks(fmt, KW), row = p.halves ? gl * 8 + (lane & 7) : gl * MROWS + lane;
                 const uint8_t* end = m.W + (long long)(m.out - 1) * m.row_pitch + (long long)p.NB * blk;       // of the matrix
                 for (int b0 = 0; b0 < p.NB; b0 += sblocks) {
                     // whole 16-byte units around the row's bytes; what of the last one lies behind the matrix is left out and copied singly
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
                     if ((MASK & 1) && fmt == 0) { if (two) tile_blocks<0, 2, KW>(sb, 0, sbi, xv, lane, acc, mins); else tile_blocks<0, 1, KW>(sb, 0, sbi, xv, lane, acc, mins); }
                     if ((MASK & 2) && fmt == 1) { if (two) tile_blocks<1, 2, KW>(sb, 0, sbi, xv, lane, acc, mins); else tile_blocks<1, 1, KW>(sb, 0, sbi, xv, lane, acc, mins); }
                     if ((MASK & 4) && fmt == 2)
-                        tile_blocks<2, 1, KW>(sb, (int)((uint64_t)(gl * MROWS + g) * (uint64_t)m.row_pitch + (uint32_t)(b0 * 210) & 15u), sbi, xv, lane, acc, mins);
+                        tile_blocks<2, 1, KW>(sb, (int)((uint64_t)(gl * (p.halves ? 8 : MROWS) + g) * (uint64_t)m.row_pitch + (uint32_t)(b0 * 210) & 15u), sbi, xv, lane, acc, mins);
                     if ((MASK & 8) && fmt == 3) tile_blocks<3, 1, KW>(sb, 0, sbi, xv, lane, acc, mins);
                     if ((MASK & 16) && fmt == 4) { if (two) tile_blocks<4, 2, KW>(sb, 0, sbi, xv, lane, acc, mins); else tile_blocks<4, 1, KW>(sb, 0, sbi, xv, lane, acc, mins); }
                 }
@@ -297,12 +299,14 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
 #pragma unroll
                 for (int w = 0; w < KW; w++) v1 += pw[(KW + w) * MROWS];
             }
+            const float other = __shfl_down_sync(0xFFFFu, v0, 8);
+            if (p.halves) v1 = other;                           // up's row, eight lanes on
             v0 *= rms_inv; v1 *= rms_inv;                       // 1.0 unless the prologue normalised (RMSNorm's scalar factor)
             int mi, gl;
             locate(u, 0, mi, gl);
             const KqMat& m = p.mat[mi];
-            const int row = gl * MROWS + lane;
-            if (row < m.out) {
+            const int row = p.halves ? gl * 8 + lane : gl * MROWS + lane;
+            if (row < m.out && !(p.halves && lane >= 8)) {
                 if (p.epilogue == GEMV_SWIGLU) {
                     // silu(g) * u with the reference's fast-math expression (gemm.cu:713-725)
                     m.y[row] = __fdividef(v0, 1.0f + __expf(-v0)) * v1;
@@ -328,7 +332,8 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
         for (int u = u0; u < p.total_groups && p.epilogue != GEMV_PEER; u += ustep) {
             int mi, gl;
             locate(u, 0, mi, gl);
-            if (lane < MROWS && gl * MROWS + lane < p.mat[mi].out) p.mat[mi].y[gl * MROWS + lane] = __uint_as_float(0x7FFFFFFFu);      // NaN
+            const int row = p.halves ? gl * 8 + lane : gl * MROWS + lane;
+            if (lane < (p.halves ? 8 : MROWS) && row < p.mat[mi].out) p.mat[mi].y[row] = __uint_as_float(0x7FFFFFFFu);      // NaN
         }
     }
 }
@@ -385,16 +390,29 @@ TeamPlan plan_teams(int mask, int K, int groups, bool four) {
     };
     // Teams of 4 share one copy of the vector and pay the meeting at the end of 16 rows half as often, four of them hide one another's barriers: the rule for
     // every launch that gives each SM more than a group (Q4_K 57344 x 8192 in a graph of its own: 45.5 us, 58 in teams of 8, 53.4 with the dp4a kernel that this
-    // one replaced; cold and alone 50.6; as gate and up with SwiGLU in the 70B step 55.9, 54.4 before: 1792 groups over 592 teams are 3.03 rounds and cost four).
+    // one replaced; cold and alone 50.6).
     // Fewer groups than SMs: more warps finish a group sooner, 8 (Q8_0 1024 x 4096: 4.8 us, 6.2 in teams of 4; Q4_K 4096 x 4096, 256 groups: 5.1 and 4.9), for
     // long rows 16 (Q6_K 1024 x 14336: 9.9 us, 11.0 in a team of 8, 12.2 before; Q8_0 2048 x 28672: 23.2, 29.7, 24.5); in between two teams of 8 in a CTA, since
     // the vector does not fit twice (Q4_K 4096 x 14336: 11.4 us, 12.3 in teams of 4, 16.9 before).
     TeamPlan t = K > 8192 ? (groups > 256 ? form(4, 4, SMEM_CTA) : groups > 148 ? form(8, 2, SMEM_CTA) : form(16, 1, SMEM_CTA))
                           : (groups > 148 ? form(4, 4, SMEM_CTA) : form(8, 1, SMEM_HALF));
+    // Rings of one stage in four teams: two teams of 8 have the same bytes under way in stages of twice the columns, and half as many barriers (Q4_K 8192 x 28672:
+    // 36.3 us, 39.2 in teams of 4).  Two stages in teams of 4 are the better of the two (Q6_K 8192 x 28672: 46.6 us, 49.4 in teams of 8).
+    if (t.kw == 4 && t.stages < 2 && K > 8192) t = form(8, 2, SMEM_CTA);
     // Very long rows (from 41984 on, by format): the vector leaves no room for a stage of every team.  One team of 8 always has one.
     static const int ord[3][2] = {{8, 2}, {16, 1}, {8, 1}};
     for (int i = 0; t.stages < 1 && i < 3; i++) t = form(ord[i][0], ord[i][1], SMEM_CTA);
     return t;
+}
+
+// Gate and up as 8 rows of each to a group instead of two groups, where their rows can lie side by side in a stage and the last round then leaves fewer teams idle:
+// 70B, 1792 pairs of groups over 592 teams are 3.03 rounds and cost four, 3584 groups of half the work 6.05 and cost seven (48.8 -> 45.9 us).  Where the number of rounds
+// stays (8B: two, or four halves) pairs are no slower: 14.5 us, 14.9 in halves.
+bool halves_of(const GemvMat& a, const GemvMat& b, int K) {
+    auto pitch = [&](const GemvMat& m) { return m.row_pitch ? m.row_pitch : dtype_row_size(m.dtype, K); };
+    const int pairs = (a.out + MROWS - 1) / MROWS, teams = MAX_TEAMS * std::max(1, num_sms());
+    auto rounds = [&](int n) { return (n + teams - 1) / teams; };
+    return fmt_of(a.dtype) == fmt_of(b.dtype) && pitch(a) == pitch(b) && rounds((a.out + 7) / 8) < 2 * rounds(pairs);
 }
 
 // format mixes with a kernel of their own
@@ -416,7 +434,7 @@ void launch_fmt(KqParams& p, cudaStream_t s) {
     constexpr int formats = MASK & ~WHOLE;
     int total = 0;
     for (int i = 0; i < p.n_mat; i++) { p.mat[i].groups = (p.mat[i].out + MROWS - 1) / MROWS; total += p.mat[i].groups; }
-    p.total_groups = p.n_seg == 2 ? p.mat[0].groups : total;
+    p.total_groups = p.halves ? (p.mat[0].out + 7) / 8 : p.n_seg == 2 ? p.mat[0].groups : total;
     const TeamPlan t = plan_teams(formats, p.K, p.total_groups, MASK != formats);
     NT_CHECK(t.stages >= 1, "gemv_kq: shared memory budget exceeded");
     p.stages = t.stages; p.slot = t.slot;
@@ -461,7 +479,8 @@ bool gemv_kq_plan(const GemvMat* mats, int n_mat, int K, bool swiglu, bool whole
         for (int i = n_mat - 1; i >= 0; i--) if (!gemv_kq_plan(&mats[i], 1, K, false, whole, plan)) return false;
         return true;
     }
-    const TeamPlan t = plan_teams(mask, K, swiglu ? (mats[0].out + MROWS - 1) / MROWS : groups, whole && mask == 16);
+    if (swiglu) groups = halves_of(mats[0], mats[1], K) ? (mats[0].out + 7) / 8 : (mats[0].out + MROWS - 1) / MROWS;
+    const TeamPlan t = plan_teams(mask, K, groups, whole && mask == 16);
     plan[0] = t.kw; plan[1] = t.teams; plan[2] = t.stages; plan[3] = t.planes;
     return t.stages >= 1;
 }
@@ -519,7 +538,8 @@ void gemv_kq(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpi
         m.fmt = fmt_of(mats[i].dtype);
         m.row_pitch = (long long)(mats[i].row_pitch ? mats[i].row_pitch : dtype_row_size(mats[i].dtype, K));
     }
-    p.n_seg = ep == GEMV_SWIGLU ? 2 : 1;
+    p.halves = ep == GEMV_SWIGLU && halves_of(mats[0], mats[1], K);
+    p.n_seg = ep == GEMV_SWIGLU && !p.halves ? 2 : 1;
     p.status = wait_status();
     switch (mask) {
         case 1: launch_fmt<1>(p, s); break;

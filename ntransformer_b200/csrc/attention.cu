@@ -415,11 +415,11 @@ void launch_rows(float* out, const float* q, const __half* kc, const __half* vc,
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
     NT_CHECK(n_splits <= MAX_SPLITS, "attention over a run of tokens: context beyond the slices");
-    launch_k(decode_kernel<DPL, GC>, dim3(groups, n_splits, tokens), dim3(AW * 32), smem, s, out, q, kc, vc, start_pos + 1, n_heads, n_kv, scale, n_splits, split_len,
+    launch_k_pdl(true, decode_kernel<DPL, GC>, dim3(groups, n_splits, tokens), dim3(AW * 32), smem, s, out, q, kc, vc, start_pos + 1, n_heads, n_kv, scale, n_splits, split_len,
              scratch, (const int*)nullptr);
     count_launch();
     if (n_splits > 1) {
-        launch_k(decode_combine_kernel, dim3(n_heads, tokens), dim3(128), 0, s, out, (const float*)scratch, n_heads, HD, n_splits, start_pos + 1, split_len,
+        launch_k_pdl(true, decode_combine_kernel, dim3(n_heads, tokens), dim3(128), 0, s, out, (const float*)scratch, n_heads, HD, n_splits, start_pos + 1, split_len,
                  (const int*)nullptr, (int8_t*)nullptr);
         count_launch();
     }

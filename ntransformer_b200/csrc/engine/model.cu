@@ -851,8 +851,10 @@ void Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
             uint16_t* kc = static_cast<uint16_t*>(kc_) + (size_t)i * kv_stride;
             uint16_t* vc = static_cast<uint16_t*>(vc_) + (size_t)i * kv_stride;
             product(sb_.x, L.attn_norm, hidden, {{&L.wq, sb_.q}, {&L.wk, sb_.k}, {&L.wv, sb_.v}}, GEMV_STORE, nullptr);
-            rope(sb_.q, sb_.k, sb_.pos, T, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, false, s);
-            copy_to_kv_cache(kc, vc, sb_.k, sb_.v, T, nkv_l_, hd, p0, max_seq, s);
+            if (!rope_kv_rows(sb_.q, sb_.k, sb_.v, kc, vc, T, p0, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, max_seq, s)) {
+                rope(sb_.q, sb_.k, sb_.pos, T, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, false, s);
+                copy_to_kv_cache(kc, vc, sb_.k, sb_.v, T, nkv_l_, hd, p0, max_seq, s);
+            }
             attention_rows_f16(sb_.attn, sb_.q, kc, vc, T, p0, nh_l_, nkv_l_, hd, 1.0f / sqrtf((float)hd), sb_.scratch, s);
             product(sb_.attn, nullptr, qdim, {{&L.wo, sb_.x}}, GEMV_ADD, nullptr);
             const bool open = product(sb_.x, L.ffn_norm, hidden, {{&L.gate, sb_.g}, {&L.up, sb_.u}}, GEMV_SWIGLU, nullptr);
@@ -969,8 +971,10 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
             const Weight *qkv[3] = {&L.wq, &L.wk, &L.wv}, *wo = &L.wo, *gu[2] = {&L.gate, &L.up}, *down = &L.down;
             float *qkv_out[3] = {pf_.q, pf_.k, pf_.v}, *gu_out[2] = {pf_.g, pf_.u};
             prefill_gemms(qkv_out, pf_.ws, pf_.x, L.attn_norm, qkv, 3, T, false, s);
-            rope(pf_.q, pf_.k, pf_.pos, T, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, false, s);
-            copy_to_kv_cache(kc, vc, pf_.k, pf_.v, T, nkv_l_, hd, p0, max_seq, s);
+            if (!rope_kv_rows(pf_.q, pf_.k, pf_.v, kc, vc, T, p0, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, max_seq, s)) {
+                rope(pf_.q, pf_.k, pf_.pos, T, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, false, s);
+                copy_to_kv_cache(kc, vc, pf_.k, pf_.v, T, nkv_l_, hd, p0, max_seq, s);
+            }
             attention_prefill(pf_.attn, pf_.q, kc, vc, T, p0, nh_l_, nkv_l_, hd, max_seq, scale, s);
             prefill_gemms(&pf_.x, pf_.ws, pf_.attn, nullptr, &wo, 1, T, true, s);
             // --- FFN sub-block (ffn.cpp:85-134) ---

@@ -99,6 +99,9 @@ void rope(float* q, float* k, const int* positions, int seq_len, int n_heads, in
           float theta, float freq_scale, bool interleaved, cudaStream_t s);
 void copy_to_kv_cache(void* kc, void* vc, const float* k, const float* v, int seq_len, int n_kv, int hd,
                       int start_pos, int max_seq, cudaStream_t s);
+// rope (half-split pairs) and copy_to_kv_cache of consecutive tokens in one launch, k itself left as it was; false (nothing launched): heads other than 64, 128, 256 wide
+bool rope_kv_rows(float* q, const float* k, const float* v, void* kc, void* vc, int tokens, int start_pos, int n_heads, int n_kv, int hd, float theta, float freq_scale,
+                  int max_seq, cudaStream_t s);
 void silu_mul(float* out, const float* gate, const float* up, int n, cudaStream_t s);
 void add_bias(float* y, const float* b, int n, cudaStream_t s);
 void add(float* out, const float* a, const float* b, int n, cudaStream_t s);

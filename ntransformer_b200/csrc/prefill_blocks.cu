@@ -52,20 +52,6 @@ struct BlkParams {
     unsigned* status;          // wait_status.cuh
 };
 
-// tcgen05.mma with A in tensor memory, and its commit, by the lane that `lead` marks.  Predicated, no branch: the operands stay in uniform registers.
-__device__ __forceinline__ void umma_ts(uint32_t lead, uint32_t d, uint32_t a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-                 ::"r"(d), "r"(a), "l"(db), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
-}
-__device__ __forceinline__ void umma_commit_by(uint32_t lead, uint64_t* bar) {
-    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
-                 ::"r"(smem_u32(bar)), "r"(lead) : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
-                 "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
-}
 __device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&v)[4]) {      // the four words twice
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
@@ -257,6 +243,8 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // Weights depend on no launch in flight: their copies and expansion start at once, tokens and everything written wait for the launch before
+    pdl_launch_dependents();
     // tensor memory is this CTA's whole (its address is 0): sums, expanded k-blocks, minima
     const uint32_t a_base = (uint32_t)(p.d_bufs * NT), m_base = a_base + (uint32_t)(p.stages * p.a_cols);
 
@@ -267,6 +255,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         if (lane == 0) {                                           // ---- tokens by TMA ----
             uint32_t st = 0, par = 1, filled = 0;
             Place q = start();
+            pdl_wait();
             for (int u = u0; u < u1; u++, next(q)) {
                 const bool mins = mins_of(q.mi);
                 for (int kb = 0; kb < 4; kb++) {
@@ -308,15 +297,15 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     const uint64_t bh = desc0 + st * stage_step, bl = bh + lo_step;
                     const uint32_t ah = a_base + st * p.a_cols, al = ah + 32, acc = kb != k0;
                     if (PAIRS && (ONE || !mins)) {                 // the small products first
-                        umma_ts(lead, d, al, bh, idesc, acc);
+                        umma_ts_by(lead, d, al, bh, idesc, acc);
 #pragma unroll
-                        for (int k = 1; k < 4; k++) umma_ts(lead, d, al + 8 * k, bh + 2 * k, idesc, 1u);
-                        umma_ts(lead, d, ah, bl, idesc, 1u);
-                    } else umma_ts(lead, d, ah, bl, idesc, acc);
+                        for (int k = 1; k < 4; k++) umma_ts_by(lead, d, al + 8 * k, bh + 2 * k, idesc, 1u);
+                        umma_ts_by(lead, d, ah, bl, idesc, 1u);
+                    } else umma_ts_by(lead, d, ah, bl, idesc, acc);
 #pragma unroll
-                    for (int k = 1; k < 4; k++) umma_ts(lead, d, ah + 8 * k, bl + 2 * k, idesc, 1u);
+                    for (int k = 1; k < 4; k++) umma_ts_by(lead, d, ah + 8 * k, bl + 2 * k, idesc, 1u);
 #pragma unroll
-                    for (int k = 0; k < 4; k++) umma_ts(lead, d, ah + 8 * k, bh + 2 * k, idesc, 1u);
+                    for (int k = 0; k < 4; k++) umma_ts_by(lead, d, ah + 8 * k, bh + 2 * k, idesc, 1u);
                     last = (int)(st * 2 + par);
                     if (kb == 3 && mins) break;                    // its stage is free after the minima
                     umma_commit_by(lead, empty + st);
@@ -328,7 +317,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
             if (MINS && mins) {                                    // minima: 8 of them times the halves of 8 sums, twice
                 wait_cta(d_empty + db, dpar, dead);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                umma_ts(lead, db * NT, m_base, desc32 + st * stage_step + 2 * lo_step, idesc, 0u);
+                umma_ts_by(lead, db * NT, m_base, desc32 + st * stage_step + 2 * lo_step, idesc, 0u);
                 umma_commit_by(lead, empty + st);                  // (the minima's place is free with this stage)
                 umma_commit_by(lead, d_full + db);
                 if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
@@ -372,6 +361,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         const uint32_t tq = ((uint32_t)(quarter * 32) << 16) + half * 16;
         uint32_t db = 0, dpar = 0, slot = 0, spar = 0;
         Place q = start();
+        pdl_wait();
         for (int u = u0; u < u1;) {
             const int sums = 4 / p.kc, chunks = sums + (MINS && mins_of(q.mi) ? 1 : 0);
             const int seg0 = u, end = min(u1, u + (NB - q.b));
@@ -571,6 +561,8 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
     constexpr int KEEP = 7;                                        // chunks of 2048 held in registers: rows to 14336
     __shared__ float red[2][16];
     const int tid = threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t at = (size_t)blockIdx.x * K;
     const float* x = xin + at;
     const float* y = MODE == TOK_SILU ? w + at : w;
@@ -650,7 +642,7 @@ template <int MASK>
 void launch_blocks(const BlkMaps& maps, const BlkParams& p, int grid, size_t smem, cudaStream_t s) {
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(gemm_blocks_kernel<MASK>, 214 * 1024, configured);
-    launch_k(gemm_blocks_kernel<MASK>, dim3(grid), dim3(Q_THREADS), smem, s, maps, p);
+    launch_k_pdl(true, gemm_blocks_kernel<MASK>, dim3(grid), dim3(Q_THREADS), smem, s, maps, p);
     count_launch();
 }
 
@@ -688,14 +680,14 @@ BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, f
     const BlockTokens t = block_tokens(workspace, T, K);
     __half* hi = static_cast<__half*>(t.split);
     __half* lo = hi + padded(T) * (size_t)K;
-    launch_k(norm_w ? split_tokens_kernel<TOK_NORM> : split_tokens_kernel<TOK_PLAIN>, dim3(T), dim3(512), 0, s, hi, lo, static_cast<__half*>(t.sums), t.scale, x, norm_w, eps, K);
+    launch_k_pdl(true, norm_w ? split_tokens_kernel<TOK_NORM> : split_tokens_kernel<TOK_PLAIN>, dim3(T), dim3(512), 0, s, hi, lo, static_cast<__half*>(t.sums), t.scale, x, norm_w, eps, K);
     count_launch();
     return t;
 }
 BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, cudaStream_t s) {
     const BlockTokens t = block_tokens(workspace, T, K);
     __half* hi = static_cast<__half*>(t.split);
-    launch_k(split_tokens_kernel<TOK_SILU>, dim3(T), dim3(512), 0, s, hi, hi + padded(T) * (size_t)K, static_cast<__half*>(t.sums), t.scale, gate, up, 0.f, K);
+    launch_k_pdl(true, split_tokens_kernel<TOK_SILU>, dim3(T), dim3(512), 0, s, hi, hi + padded(T) * (size_t)K, static_cast<__half*>(t.sums), t.scale, gate, up, 0.f, K);
     count_launch();
     return t;
 }
@@ -703,7 +695,7 @@ BlockTokens resplit_tokens(void* workspace, const void* split, int T, int K, cud
     const BlockTokens t = block_tokens(workspace, T, K);
     __half* hi = static_cast<__half*>(t.split);
     const size_t lo = padded(T) * (size_t)K;
-    launch_k(split_tokens_kernel<TOK_SPLIT>, dim3(T), dim3(512), 0, s, hi, hi + lo, static_cast<__half*>(t.sums), t.scale, static_cast<const float*>(split),
+    launch_k_pdl(true, split_tokens_kernel<TOK_SPLIT>, dim3(T), dim3(512), 0, s, hi, hi + lo, static_cast<__half*>(t.sums), t.scale, static_cast<const float*>(split),
              reinterpret_cast<const float*>(static_cast<const __half*>(split) + lo), 0.f, K);
     count_launch();
     return t;

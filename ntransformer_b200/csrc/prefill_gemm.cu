@@ -331,9 +331,45 @@ __global__ void __launch_bounds__(192, 1) gemm_f16_tc_kernel(const __grid_consta
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TMEM_COLS));
 }
 
-// RMSNorm (rmsnorm.cu:17-70 math) writing the F16 hi/lo split the GEMM consumes: one CTA per row
+// RMSNorm (rmsnorm.cu:17-70 math) writing the F16 hi/lo split the GEMM consumes: one CTA per row, its first 8192 columns in registers between the sum and the
+// split, 16 bytes a load (2048 x 4096, scalar loads and a second trip to L2 before: 25 us)
 __global__ void __launch_bounds__(512) rmsnorm_split_kernel(__half* __restrict__ hi, __half* __restrict__ lo, const float* __restrict__ xin,
                                                             const float* __restrict__ w, int hidden, float eps, int bf16) {
+    constexpr int KEEP = 4;
+    __shared__ float red[16];
+    const float* x = xin + (size_t)blockIdx.x * hidden;
+    __half* h = hi + (size_t)blockIdx.x * hidden;
+    __half* l = lo + (size_t)blockIdx.x * hidden;
+    float4 keep[KEEP];
+    float ss = 0.f;
+    auto square = [&](const float4& v) { ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; };
+#pragma unroll
+    for (int c = 0; c < KEEP; c++) { const int i = c * 2048 + 4 * threadIdx.x; if (i < hidden) keep[c] = *reinterpret_cast<const float4*>(x + i); }
+#pragma unroll
+    for (int c = 0; c < KEEP; c++) if (c * 2048 + 4 * (int)threadIdx.x < hidden) square(keep[c]);
+    for (int i = KEEP * 2048 + 4 * threadIdx.x; i < hidden; i += 2048) square(*reinterpret_cast<const float4*>(x + i));
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float tot = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) tot += red[i];
+    const float rms_inv = rsqrtf(tot / hidden + eps);
+    auto put = [&](int i, const float4& v) {
+        const float4 g = *reinterpret_cast<const float4*>(w + i);
+        uint2 ph, pl;
+        split_pair(v.x * rms_inv * g.x, v.y * rms_inv * g.y, bf16, ph.x, pl.x);
+        split_pair(v.z * rms_inv * g.z, v.w * rms_inv * g.w, bf16, ph.y, pl.y);
+        *reinterpret_cast<uint2*>(h + i) = ph;
+        *reinterpret_cast<uint2*>(l + i) = pl;
+    };
+#pragma unroll
+    for (int c = 0; c < KEEP; c++) { const int i = c * 2048 + 4 * threadIdx.x; if (i < hidden) put(i, keep[c]); }
+    for (int i = KEEP * 2048 + 4 * threadIdx.x; i < hidden; i += 2048) put(i, *reinterpret_cast<const float4*>(x + i));
+}
+// the same over widths or pointers that 16-byte loads do not take
+__global__ void __launch_bounds__(512) rmsnorm_split_any_kernel(__half* __restrict__ hi, __half* __restrict__ lo, const float* __restrict__ xin,
+                                                                const float* __restrict__ w, int hidden, float eps, int bf16) {
     __shared__ float red[16];
     const float* x = xin + (size_t)blockIdx.x * hidden;
     float ss = 0.f;
@@ -348,9 +384,8 @@ __global__ void __launch_bounds__(512) rmsnorm_split_kernel(__half* __restrict__
     __half2* l2 = reinterpret_cast<__half2*>(lo + (size_t)blockIdx.x * hidden);
     for (int i = threadIdx.x; i < hidden / 2; i += blockDim.x) {
         const float2 xv = reinterpret_cast<const float2*>(x)[i], wv = reinterpret_cast<const float2*>(w)[i];
-        const float a = xv.x * rms_inv * wv.x, b = xv.y * rms_inv * wv.y;
         uint32_t ph, pl;
-        split_pair(a, b, bf16, ph, pl);
+        split_pair(xv.x * rms_inv * wv.x, xv.y * rms_inv * wv.y, bf16, ph, pl);
         reinterpret_cast<uint32_t*>(h2)[i] = ph;
         reinterpret_cast<uint32_t*>(l2)[i] = pl;
     }
@@ -429,7 +464,8 @@ void split_activations(void* workspace, const float* A, int M, int K, cudaStream
 void rmsnorm_split(void* workspace, const float* x, const float* w, int rows, int hidden, float eps, cudaStream_t s, bool bf16) {
     const size_t Mp = ((size_t)rows + BM - 1) / BM * BM;
     __half* hi = static_cast<__half*>(workspace);
-    rmsnorm_split_kernel<<<rows, 512, 0, s>>>(hi, hi + Mp * (size_t)hidden, x, w, hidden, eps, bf16 ? 1 : 0);
+    const bool wide = hidden % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(workspace)) & 15) == 0;
+    (wide ? rmsnorm_split_kernel : rmsnorm_split_any_kernel)<<<rows, 512, 0, s>>>(hi, hi + Mp * (size_t)hidden, x, w, hidden, eps, bf16 ? 1 : 0);
     count_launch();
 }
 

@@ -571,7 +571,8 @@ void attention_decode_rope_dyn(float* out, const float* q, const float* k, const
 void attention_prefill(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads,
                        int n_kv, int hd, int max_seq, float scale, cudaStream_t s) {
     if (seq_len <= 0 || n_heads <= 0) return;
-    if (attention_prefill_mma_supported(seq_len, n_heads, n_kv, hd)) {       // prompt-sized chunks: tiled tensor-core kernel
+    if (attention_prefill_mma_supported(seq_len, n_heads, n_kv, hd)) {       // prompt-sized chunks: tiled tensor-core kernels
+        if (attention_prefill_tc(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, scale, s)) return;
         attention_prefill_mma(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq, scale, s);
         return;
     }

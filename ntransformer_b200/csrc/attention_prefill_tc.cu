@@ -1,0 +1,296 @@
+// attention_prefill_tc.cu — causal GQA attention of a run of prompt tokens over the F16 cache on the 5th-generation tensor cores (tcgen05), sm_100a.
+//
+// Same contract as the reference's attention_prefill_kernel (src/cuda/attention.cu:216-311): F32 queries [seq][n_heads][hd], F16 cache [max_seq][n_kv][hd], query i
+// attends keys 0..start_pos + i.  The form on mma.sync (attention_prefill_mma.cu), which windows and BF16 caches still take, is bound by that instruction: two halves
+// of each query and of each weight make four products where one is counted.  Here:
+//   * a CTA owns two tiles of 128 queries that share their keys (two heads of a key head; two runs of queries where it has an odd number): while the tensor cores
+//     multiply for one, eight warps, a row to a lane, form the weights of the other;
+//   * scores S = (q_hi + q_lo) . K^T: queries split in shared memory, each row under a power of two that keeps its low halves' bits, keys by TMA, 128 at a time, two
+//     buffers; the sums of 128 x 128 scores in tensor memory;
+//   * weights exp2(f S - m) as F16 hi + lo take the scores' place in tensor memory, which is the A operand of (p_hi + p_lo) . V;
+//   * that product of 128 keys starts at zero in tensor memory; the rows' sums are kept in F32 registers, rescaled there where the maximum moves.
+#include "kernels_internal.h"
+#include "ring.cuh"
+#include "tc_device.cuh"
+#include "wait_status.cuh"
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+namespace nt { namespace b200 {
+
+namespace {
+
+constexpr int TQ = 128, TK = 128;                        // queries of a tile, keys of a step
+constexpr int TC_THREADS = 12 * 32;                      // warps 0-3 and 4-7: softmax of the two tiles, 8: TMA, 9: MMA; registers 2 x 216 + 72 = 3 x 168 at launch
+template <int HD> struct TcSmem {
+    static constexpr int Q = TQ * HD * 2, KV = TK * HD * 2;              // bytes of a tile's half of the queries; of a step's keys or values
+    static constexpr int K0 = 4 * Q, V0 = K0 + 2 * KV, ALL = V0 + KV + 1024;
+};
+
+__device__ __forceinline__ void umma_ss_by(uint32_t lead, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
+// Values as the B operand: N (channels) contiguous, SWIZZLE_128B: 64 channels x 8 keys to an atom of 1024 bytes, the next 8 keys 1024 bytes on (stride offset), the
+// next 64 channels a whole box on (leading offset)
+__device__ __forceinline__ uint64_t make_desc_mn(const void* smem_ptr, uint32_t box_bytes) {
+    const uint64_t addr = (uint64_t)(smem_u32(smem_ptr) & 0x3FFFFu) >> 4;
+    return addr | ((uint64_t)(box_bytes >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+
+struct TcAttn {
+    float* out;
+    const float* Q;
+    int seq_len, start_pos, n_heads, n_kv, pairs_of_queries;      // pairs_of_queries: a key head has an odd number of heads
+    float scale;
+    unsigned* status;
+};
+
+template <int HD>
+__global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ TcAttn p) {
+    using S = TcSmem<HD>;
+    constexpr int BOXES = HD / 64, BOX = TK * 128;                // boxes of 64 channels
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t k_full[2], k_empty[2], v_full, v_empty, q_full, s_full[2], p_full[2], o_full[2];
+    __shared__ uint32_t tmem_base_smem, dead_smem;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t dead = smem_u32(&dead_smem);
+    // the longest runs of keys first
+    const int qt = (int)gridDim.x - 1 - (int)blockIdx.x, h0 = p.pairs_of_queries ? (int)blockIdx.y : 2 * (int)blockIdx.y, kvh = h0 / (p.n_heads / p.n_kv);
+    const int first_q = qt * (p.pairs_of_queries ? 2 * TQ : TQ), last_q = min(first_q + (p.pairs_of_queries ? 2 * TQ : TQ), p.seq_len) - 1;
+    const int n = (p.start_pos + last_q) / TK + 1;               // steps
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; i++) { mbar_init(k_full + i, 1); mbar_init(k_empty + i, 1); mbar_init(s_full + i, 1); mbar_init(p_full + i, 4); mbar_init(o_full + i, 1); }
+        mbar_init(&v_full, 1); mbar_init(&v_empty, 1); mbar_init(&q_full, 8);
+        dead_smem = 0;
+        mbar_fence_init();
+    }
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_smem)), "n"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    pdl_launch_dependents();
+    pdl_wait();
+    // tensor memory is this CTA's whole: scores, then weights, of the two tiles at columns 0 and 128, the products with V at 256 and 384
+
+    if (warp < 8) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+        const int t = warp >> 2, r = (warp & 3) * 32 + lane, head = p.pairs_of_queries ? h0 : h0 + t, q0 = first_q + (p.pairs_of_queries ? t * TQ : 0), row = q0 + r;
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, ts = lanes + t * 128, to = lanes + 256 + t * 128;
+        float f;                                                  // of a row's scores: log2 e * scale, and the power of two taken back
+        {
+            const float4* src = reinterpret_cast<const float4*>(p.Q + ((size_t)min(row, p.seq_len - 1) * p.n_heads + head) * HD);
+            float amax = 0.f;
+#pragma unroll 8
+            for (int i = 0; i < HD / 4; i++) { const float4 x = __ldg(src + i); amax = fmaxf(fmaxf(amax, fmaxf(fabsf(x.x), fabsf(x.y))), fmaxf(fabsf(x.z), fabsf(x.w))); }
+            const uint32_t e = __float_as_uint(amax) >> 23 & 255u;       // not finite, or zero: as it is
+            const uint32_t up = e == 255u || e == 0u ? 127u : min(227u, max(27u, 264u - e));       // to 2^10 .. 2^11
+            const float g = __uint_as_float(up << 23);
+            f = p.scale * 1.4426950408889634f * __uint_as_float((254u - up) << 23);
+            uint8_t* hi = smem + 2 * t * S::Q + r * 128;
+#pragma unroll 4
+            for (int c = 0; c < HD / 8; c++) {                    // 16 bytes of a 128-byte swizzle row at a time
+                const float4 x = __ldg(src + 2 * c), y = __ldg(src + 2 * c + 1);
+                uint4 h, l;
+                split_pair(x.x * g, x.y * g, 0, h.x, l.x); split_pair(x.z * g, x.w * g, 0, h.y, l.y);
+                split_pair(y.x * g, y.y * g, 0, h.z, l.z); split_pair(y.z * g, y.w * g, 0, h.w, l.w);
+                const int at = (c >> 3) * (TQ * 128) + (((c & 7) ^ (r & 7)) << 4);
+                *reinterpret_cast<uint4*>(hi + at) = h;
+                *reinterpret_cast<uint4*>(hi + S::Q + at) = l;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&q_full);
+        }
+        uint64_t o[HD / 2];                                       // pairs of channels
+#pragma unroll
+        for (int i = 0; i < HD / 2; i++) o[i] = 0;
+        float m = -INFINITY, l = 0.f, before = 0.f;              // before: the rescaling of what was summed ahead of the step before
+        auto drain = [&](int j) {                                 // the product of step j joins the sums
+            wait_cta(o_full + t, j & 1, dead);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t a = pack2(before, before);
+#pragma unroll
+            for (int c = 0; c < HD / 32; c++) {
+                uint32_t v[32];
+                tmem_ld32(to + 32 * c, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 16; i++) o[16 * c + i] = fma2(o[16 * c + i], a, pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+            }
+        };
+#pragma unroll 1
+        for (int j = 0; j < n; j++) {
+            const int seen = p.start_pos + row - j * TK;          // this step's keys up to here are seen
+            const bool whole = j * TK + TK - 1 <= p.start_pos + q0;      // by every row of the tile
+            wait_cta(s_full + t, j & 1, dead);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float mx = -INFINITY;
+#pragma unroll
+            for (int c = 0; c < TK / 32; c++) {
+                uint32_t v[32];
+                tmem_ld32(ts + 32 * c, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (whole) {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) mx = fmaxf(mx, __uint_as_float(v[i]));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) mx = fmaxf(mx, 32 * c + i <= seen ? __uint_as_float(v[i]) : -INFINITY);
+                }
+            }
+            const float mn = fmaxf(m, mx * f), base = mn == -INFINITY ? 0.f : mn, alpha = exp2f(m - base);      // (a run of keys wholly unseen leaves the maximum; step 0 has key 0)
+            m = mn;
+            float sum = 0.f;
+#pragma unroll
+            for (int c = 0; c < TK / 32; c++) {
+                uint32_t v[32];
+                tmem_ld32(ts + 32 * c, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (!whole)
+#pragma unroll
+                    for (int i = 0; i < 32; i++) v[i] = 32 * c + i <= seen ? v[i] : 0xFF800000u;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {                     // 16 keys: 8 columns hi, 8 lo, where their scores were
+                    uint32_t w[16];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const float a = exp2f(fmaf(__uint_as_float(v[16 * h + 2 * i]), f, -base)), b = exp2f(fmaf(__uint_as_float(v[16 * h + 2 * i + 1]), f, -base));
+                        sum += a + b;
+                        split_pair(a, b, 0, w[i], w[8 + i]);
+                    }
+                    tmem_st16(ts + 32 * c + 16 * h, w);
+                }
+            }
+            l = fmaf(l, alpha, sum);
+            if (j > 0) drain(j - 1);
+            before = alpha;
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_full + t);
+        }
+        drain(n - 1);
+        if (word_set(dead)) report(p.status);
+        else if (row < p.seq_len) {
+            const float inv = 1.0f / l;
+            float4* dst = reinterpret_cast<float4*>(p.out + ((size_t)row * p.n_heads + head) * HD);
+#pragma unroll
+            for (int i = 0; i < HD / 4; i++) {
+                float4 x;
+                unpack2(o[2 * i], x.x, x.y); unpack2(o[2 * i + 1], x.z, x.w);
+                dst[i] = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
+            }
+        }
+    } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp == 8) {
+        if (lane == 0) {                                          // ---- keys and values by TMA: keys a step ahead ----
+            auto load = [&](uint8_t* d, const CUtensorMap* map, int j, uint64_t* full) {
+                mbar_expect_tx(full, S::KV);
+#pragma unroll
+                for (int i = 0; i < BOXES; i++) tma_load_2d(d + i * BOX, map, kvh * HD + 64 * i, j * TK, full);
+            };
+            int keys = 1, values = 0;                             // steps whose keys, whose values are under way
+            bool gone = false;
+            load(smem + S::K0, &map_k, 0, k_full);
+            for (int j = 0; j < n && !gone; j++) {
+                if (j + 1 < n) {
+                    wait_cta(k_empty + ((j + 1) & 1), (((j + 1) >> 1) & 1) ^ 1, dead);
+                    if (!(gone = word_set(dead))) { load(smem + S::K0 + ((j + 1) & 1) * S::KV, &map_k, j + 1, k_full + ((j + 1) & 1)); keys = j + 2; }
+                }
+                wait_cta(&v_empty, (j & 1) ^ 1, dead);
+                if (!(gone = gone || word_set(dead))) { load(smem + S::V0, &map_v, j, &v_full); values = j + 1; }
+            }
+            if (gone) {                                           // given up: the copies in flight
+                for (int j = max(0, keys - 2); j < keys; j++) wait_flight(k_full + (j & 1), (j >> 1) & 1);
+                if (values) wait_flight(&v_full, (values - 1) & 1);
+            }
+        }
+    } else if (warp == 9) {
+        // ---- MMA: the whole warp walks the loop and one lane issues by predicate, so that operands stay in uniform registers ----
+        const uint32_t lead = elect_lane();
+        constexpr uint32_t F32_M128 = (1u << 4) | (8u << 24);
+        constexpr uint32_t IDESC_S = F32_M128 | ((uint32_t)(TK >> 3) << 17), IDESC_O = F32_M128 | ((uint32_t)(HD >> 3) << 17) | (1u << 16);      // V: N-major
+        const uint64_t dq = make_desc(smem), dk = make_desc(smem + S::K0), dv = make_desc_mn(smem + S::V0, BOX);
+        auto commit = [&](uint64_t* bar) { umma_commit_by(lead, bar); };
+        auto scores = [&](int t, int j) {
+            const uint64_t a = dq + (uint64_t)((2 * t * S::Q) >> 4), b = dk + (uint64_t)(((j & 1) * S::KV) >> 4);
+#pragma unroll
+            for (int part = 1; part >= 0; part--)                 // the low halves first
+#pragma unroll
+                for (int s = 0; s < HD / 16; s++) {
+                    const uint64_t at = (uint64_t)((s >> 2) * (TQ * 128 >> 4) + 2 * (s & 3));
+                    umma_ss_by(lead, t * 128, a + (uint64_t)((part * S::Q) >> 4) + at, b + at, IDESC_S, part == 0 || s > 0);
+                }
+            commit(s_full + t);
+        };
+        wait_cta(&q_full, 0, dead);
+        wait_cta(k_full, 0, dead);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        scores(0, 0);
+        scores(1, 0);
+        commit(k_empty);
+#pragma unroll 1
+        for (int j = 0; j < n; j++) {
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
+                wait_cta(p_full + t, j & 1, dead);
+                if (t == 0) wait_cta(&v_full, j & 1, dead);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int part = 1; part >= 0; part--)
+#pragma unroll
+                    for (int s = 0; s < TK / 16; s++)
+                        umma_ts_by(lead, 256 + t * 128, t * 128 + 16 * s + 8 * part, dv + (uint64_t)(s * (2048 >> 4)), IDESC_O, part == 0 || s > 0);
+                commit(o_full + t);
+                if (t == 1) commit(&v_empty);
+                if (j + 1 < n) {
+                    if (t == 0) { wait_cta(k_full + ((j + 1) & 1), ((j + 1) >> 1) & 1, dead); asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+                    scores(t, j + 1);
+                    if (t == 1) commit(k_empty + ((j + 1) & 1));
+                }
+            }
+        }
+        wait_flight(&v_empty, (n - 1) & 1);                       // the last commit: nothing of this CTA is in flight behind its end
+    }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    __syncwarp();
+    if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_smem), "n"(512));
+}
+
+template <int HD>
+void launch_tc(const CUtensorMap& map_k, const CUtensorMap& map_v, const TcAttn& p, cudaStream_t s) {
+    static unsigned long long configured = 0;      // bit per device id
+    opt_in_dynamic_smem(prefill_tc_kernel<HD>, TcSmem<HD>::ALL, configured);
+    const int rows = p.pairs_of_queries ? 2 * TQ : TQ;
+    launch_k_pdl(true, prefill_tc_kernel<HD>, dim3((p.seq_len + rows - 1) / rows, p.pairs_of_queries ? p.n_heads : p.n_heads / 2), dim3(TC_THREADS), TcSmem<HD>::ALL, s, map_k, map_v, p);
+    count_launch();
+}
+
+}  // namespace
+
+// false: nothing launched (pointers off 16 bytes; other widths)
+bool attention_prefill_tc(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, float scale, cudaStream_t s) {
+    if (seq_len < 1 || (hd != 64 && hd != 128) || n_kv < 1 || n_heads % n_kv || n_heads > 65535 ||
+        ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15)) return false;
+    // the maps end with the last key: rows of the cache behind it are zeros, whatever they hold
+    CUtensorMap map_k, map_v;
+    const uint64_t keys = (uint64_t)start_pos + seq_len, row = (uint64_t)n_kv * hd;
+    if (!tc_map_f16(&map_k, kc, keys, row, TK) || !tc_map_f16(&map_v, vc, keys, row, TK)) return false;
+    TcAttn p{out, Q, seq_len, start_pos, n_heads, n_kv, (n_heads / n_kv) % 2, scale, wait_status()};
+    if (hd == 128) launch_tc<128>(map_k, map_v, p, s);
+    else launch_tc<64>(map_k, map_v, p, s);
+    return true;
+}
+
+}}  // namespace nt::b200

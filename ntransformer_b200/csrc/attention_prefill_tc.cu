@@ -6,9 +6,10 @@
 //   * a CTA owns two tiles of 128 queries that share their keys (two heads of a key head; two runs of queries where it has an odd number): while the tensor cores
 //     multiply for one, eight warps, a row to a lane, form the weights of the other;
 //   * scores S = (q_hi + q_lo) . K^T: queries split in shared memory, each row under a power of two that keeps its low halves' bits, keys by TMA, 128 at a time, two
-//     buffers; the sums of 128 x 128 scores in tensor memory;
+//     buffers; 128 x 128 scores in tensor memory, three buffers that the tiles use in turn, so that a tile's next scores are there when its weights are handed over;
 //   * weights exp2(f S - m) as F16 hi + lo take the scores' place in tensor memory, which is the A operand of (p_hi + p_lo) . V;
-//   * that product of 128 keys starts at zero in tensor memory; the rows' sums are kept in F32 registers, rescaled there where the maximum moves.
+//   * that product of 128 keys starts at zero in the fourth quarter of tensor memory and is taken from there at once; the rows' sums are kept in F32 registers,
+//     rescaled there where the maximum moves.
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "tc_device.cuh"
@@ -55,7 +56,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
     constexpr int BOXES = HD / 64, BOX = TK * 128;                // boxes of 64 channels
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t k_full[2], k_empty[2], v_full, v_empty, q_full, s_full[2], p_full[2], o_full[2];
+    __shared__ uint64_t k_full[2], k_empty[2], v_full, v_empty, q_full, s_full[3], p_full[2], o_full[2], o_empty;
+    __shared__ float factor[2 * TQ];                              // of a row's scores: log2 e * scale, and the power of two taken back
     __shared__ uint32_t tmem_base_smem, dead_smem;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t dead = smem_u32(&dead_smem);
@@ -64,8 +66,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
     const int first_q = qt * (p.pairs_of_queries ? 2 * TQ : TQ), last_q = min(first_q + (p.pairs_of_queries ? 2 * TQ : TQ), p.seq_len) - 1;
     const int n = (p.start_pos + last_q) / TK + 1;               // steps
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; i++) { mbar_init(k_full + i, 1); mbar_init(k_empty + i, 1); mbar_init(s_full + i, 1); mbar_init(p_full + i, 4); mbar_init(o_full + i, 1); }
-        mbar_init(&v_full, 1); mbar_init(&v_empty, 1); mbar_init(&q_full, 8);
+        for (int i = 0; i < 2; i++) { mbar_init(k_full + i, 1); mbar_init(k_empty + i, 1); mbar_init(p_full + i, 4); mbar_init(o_full + i, 1); }
+        for (int i = 0; i < 3; i++) mbar_init(s_full + i, 1);
+        mbar_init(&v_full, 1); mbar_init(&v_empty, 1); mbar_init(&q_full, 8); mbar_init(&o_empty, 4);
         dead_smem = 0;
         mbar_fence_init();
     }
@@ -78,45 +81,49 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     pdl_launch_dependents();
     pdl_wait();
-    // tensor memory is this CTA's whole: scores, then weights, of the two tiles at columns 0 and 128, the products with V at 256 and 384
+    // Step j of tile t is item 2 j + t.  Tensor memory is this CTA's whole: an item's scores, then weights, at column 128 (item mod 3), its product with V at 384.
 
     if (warp < 8) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
         const int t = warp >> 2, r = (warp & 3) * 32 + lane, head = p.pairs_of_queries ? h0 : h0 + t, q0 = first_q + (p.pairs_of_queries ? t * TQ : 0), row = q0 + r;
-        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, ts = lanes + t * 128, to = lanes + 256 + t * 128;
-        float f;                                                  // of a row's scores: log2 e * scale, and the power of two taken back
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, to = lanes + 384;
+        uint8_t* mine = smem + 2 * t * S::Q;                      // the tile's queries
         {
-            const float4* src = reinterpret_cast<const float4*>(p.Q + ((size_t)min(row, p.seq_len - 1) * p.n_heads + head) * HD);
-            float amax = 0.f;
+            // a row to LR lanes, so that loads are whole lines; 4 channels to a lane
+            constexpr int LR = HD / 4, RI = 32 / LR;              // lanes of a row, rows of an instruction
+            const int c = lane % LR;
 #pragma unroll 8
-            for (int i = 0; i < HD / 4; i++) { const float4 x = __ldg(src + i); amax = fmaxf(fmaxf(amax, fmaxf(fabsf(x.x), fabsf(x.y))), fmaxf(fabsf(x.z), fabsf(x.w))); }
-            const uint32_t e = __float_as_uint(amax) >> 23 & 255u;       // not finite, or zero: as it is
-            const uint32_t up = e == 255u || e == 0u ? 127u : min(227u, max(27u, 264u - e));       // to 2^10 .. 2^11
-            const float g = __uint_as_float(up << 23);
-            f = p.scale * 1.4426950408889634f * __uint_as_float((254u - up) << 23);
-            uint8_t* hi = smem + 2 * t * S::Q + r * 128;
-#pragma unroll 4
-            for (int c = 0; c < HD / 8; c++) {                    // 16 bytes of a 128-byte swizzle row at a time
-                const float4 x = __ldg(src + 2 * c), y = __ldg(src + 2 * c + 1);
-                uint4 h, l;
-                split_pair(x.x * g, x.y * g, 0, h.x, l.x); split_pair(x.z * g, x.w * g, 0, h.y, l.y);
-                split_pair(y.x * g, y.y * g, 0, h.z, l.z); split_pair(y.z * g, y.w * g, 0, h.w, l.w);
-                const int at = (c >> 3) * (TQ * 128) + (((c & 7) ^ (r & 7)) << 4);
-                *reinterpret_cast<uint4*>(hi + at) = h;
-                *reinterpret_cast<uint4*>(hi + S::Q + at) = l;
+            for (int i = 0; i < 32 / RI; i++) {
+                const int rr = (warp & 3) * 32 + i * RI + lane / LR;
+                const float4 x = __ldg(reinterpret_cast<const float4*>(p.Q + ((size_t)min(q0 + rr, p.seq_len - 1) * p.n_heads + head) * HD) + c);
+                float amax = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
+#pragma unroll
+                for (int s = LR / 2; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, s));
+                const uint32_t e = __float_as_uint(amax) >> 23 & 255u;       // not finite, or zero: as it is
+                const uint32_t up = e == 255u || e == 0u ? 127u : min(227u, max(27u, 264u - e));       // to 2^10 .. 2^11
+                const float g = __uint_as_float(up << 23);
+                if (c == 0) factor[t * TQ + rr] = p.scale * 1.4426950408889634f * __uint_as_float((254u - up) << 23);
+                uint2 h, l;
+                split_pair(x.x * g, x.y * g, 0, h.x, l.x);
+                split_pair(x.z * g, x.w * g, 0, h.y, l.y);
+                // 64 channels to a 128-byte swizzle row
+                uint8_t* d = mine + (c >> 4) * (TQ * 128) + rr * 128 + ((((c & 15) >> 1) ^ (rr & 7)) << 4) + (c & 1) * 8;
+                *reinterpret_cast<uint2*>(d) = h;
+                *reinterpret_cast<uint2*>(d + S::Q) = l;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&q_full);
         }
+        const float f = factor[t * TQ + r];
         uint64_t o[HD / 2];                                       // pairs of channels
 #pragma unroll
         for (int i = 0; i < HD / 2; i++) o[i] = 0;
-        float m = -INFINITY, l = 0.f, before = 0.f;              // before: the rescaling of what was summed ahead of the step before
-        auto drain = [&](int j) {                                 // the product of step j joins the sums
+        float m = -INFINITY, l = 0.f;
+        auto drain = [&](int j, float alpha) {                    // the product of step j joins the sums
             wait_cta(o_full + t, j & 1, dead);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t a = pack2(before, before);
+            const uint64_t a = pack2(alpha, alpha);
 #pragma unroll
             for (int c = 0; c < HD / 32; c++) {
                 uint32_t v[32];
@@ -125,12 +132,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
 #pragma unroll
                 for (int i = 0; i < 16; i++) o[16 * c + i] = fma2(o[16 * c + i], a, pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
             }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&o_empty);
         };
+        uint32_t ts = lanes + t * 128;                            // of the step's scores
 #pragma unroll 1
         for (int j = 0; j < n; j++) {
             const int seen = p.start_pos + row - j * TK;          // this step's keys up to here are seen
             const bool whole = j * TK + TK - 1 <= p.start_pos + q0;      // by every row of the tile
-            wait_cta(s_full + t, j & 1, dead);
+            wait_cta(s_full + ((2 * j + t) % 3), ((2 * j + t) / 3) & 1, dead);      // (of the buffer: a tile's next scores may come before these are looked at)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float mx = -INFINITY;
 #pragma unroll
@@ -170,23 +181,36 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 }
             }
             l = fmaf(l, alpha, sum);
-            if (j > 0) drain(j - 1);
-            before = alpha;
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full + t);
+            drain(j, alpha);
+            ts = ts == lanes ? lanes + 256 : ts - 128;            // two items on
         }
-        drain(n - 1);
         if (word_set(dead)) report(p.status);
-        else if (row < p.seq_len) {
+        else {
+            // 16 rows at a time over the tile's queries (no product reads them any more), then whole rows to memory
             const float inv = 1.0f / l;
-            float4* dst = reinterpret_cast<float4*>(p.out + ((size_t)row * p.n_heads + head) * HD);
+            constexpr int PITCH = HD + 4, LR = HD / 4, RI = 32 / LR;
+            float* stage = reinterpret_cast<float*>(mine) + (warp & 3) * 16 * PITCH;
 #pragma unroll
-            for (int i = 0; i < HD / 4; i++) {
-                float4 x;
-                unpack2(o[2 * i], x.x, x.y); unpack2(o[2 * i + 1], x.z, x.w);
-                dst[i] = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
+            for (int half = 0; half < 2; half++) {
+                if ((lane >> 4) == half)
+#pragma unroll
+                    for (int i = 0; i < HD / 4; i++) {
+                        float4 x;
+                        unpack2(o[2 * i], x.x, x.y); unpack2(o[2 * i + 1], x.z, x.w);
+                        *reinterpret_cast<float4*>(stage + (lane & 15) * PITCH + 4 * i) = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
+                    }
+                __syncwarp();
+#pragma unroll 4
+                for (int i = 0; i < 16 / RI; i++) {
+                    const int rr = i * RI + lane / LR, at = q0 + (warp & 3) * 32 + half * 16 + rr;
+                    if (at < p.seq_len)
+                        *(reinterpret_cast<float4*>(p.out + ((size_t)at * p.n_heads + head) * HD) + lane % LR) = *reinterpret_cast<const float4*>(stage + rr * PITCH + 4 * (lane % LR));
+                }
+                __syncwarp();
             }
         }
     } else {
@@ -220,44 +244,44 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
         constexpr uint32_t F32_M128 = (1u << 4) | (8u << 24);
         constexpr uint32_t IDESC_S = F32_M128 | ((uint32_t)(TK >> 3) << 17), IDESC_O = F32_M128 | ((uint32_t)(HD >> 3) << 17) | (1u << 16);      // V: N-major
         const uint64_t dq = make_desc(smem), dk = make_desc(smem + S::K0), dv = make_desc_mn(smem + S::V0, BOX);
-        auto commit = [&](uint64_t* bar) { umma_commit_by(lead, bar); };
-        auto scores = [&](int t, int j) {
-            const uint64_t a = dq + (uint64_t)((2 * t * S::Q) >> 4), b = dk + (uint64_t)(((j & 1) * S::KV) >> 4);
+        uint32_t sb = 0;                                          // columns of the next item's scores
+        auto scores = [&](int item) {
+            const int t = item & 1, j = item >> 1;
+            if (t == 0) { wait_cta(k_full + (j & 1), (j >> 1) & 1, dead); asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+            const uint64_t a = dq + (uint64_t)(t * (2 * S::Q >> 4)), b = dk + (uint64_t)((j & 1) * (S::KV >> 4));
 #pragma unroll
             for (int part = 1; part >= 0; part--)                 // the low halves first
 #pragma unroll
                 for (int s = 0; s < HD / 16; s++) {
                     const uint64_t at = (uint64_t)((s >> 2) * (TQ * 128 >> 4) + 2 * (s & 3));
-                    umma_ss_by(lead, t * 128, a + (uint64_t)((part * S::Q) >> 4) + at, b + at, IDESC_S, part == 0 || s > 0);
+                    umma_ss_by(lead, sb, a + (uint64_t)((part * S::Q) >> 4) + at, b + at, IDESC_S, part == 0 || s > 0);
                 }
-            commit(s_full + t);
+            umma_commit_by(lead, s_full + (sb >> 7));
+            if (t == 1) umma_commit_by(lead, k_empty + (j & 1));
+            sb = sb == 256 ? 0 : sb + 128;
         };
         wait_cta(&q_full, 0, dead);
-        wait_cta(k_full, 0, dead);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        scores(0, 0);
-        scores(1, 0);
-        commit(k_empty);
+        scores(0);
+        scores(1);
+        if (n > 1) scores(2);
 #pragma unroll 1
-        for (int j = 0; j < n; j++) {
+        for (int item = 0; item < 2 * n; item++) {
+            const int t = item & 1, j = item >> 1;
+            const uint32_t pb = n > 1 ? sb : item * 128;          // the buffer used longest ago (three items are under way; with one step two)
+            wait_cta(p_full + t, j & 1, dead);
+            if (t == 0) wait_cta(&v_full, j & 1, dead);
+            if (item > 0) wait_cta(&o_empty, (item - 1) & 1, dead);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int t = 0; t < 2; t++) {
-                wait_cta(p_full + t, j & 1, dead);
-                if (t == 0) wait_cta(&v_full, j & 1, dead);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int part = 1; part >= 0; part--)
 #pragma unroll
-                for (int part = 1; part >= 0; part--)
-#pragma unroll
-                    for (int s = 0; s < TK / 16; s++)
-                        umma_ts_by(lead, 256 + t * 128, t * 128 + 16 * s + 8 * part, dv + (uint64_t)(s * (2048 >> 4)), IDESC_O, part == 0 || s > 0);
-                commit(o_full + t);
-                if (t == 1) commit(&v_empty);
-                if (j + 1 < n) {
-                    if (t == 0) { wait_cta(k_full + ((j + 1) & 1), ((j + 1) >> 1) & 1, dead); asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-                    scores(t, j + 1);
-                    if (t == 1) commit(k_empty + ((j + 1) & 1));
-                }
-            }
+                for (int s = 0; s < TK / 16; s++)
+                    umma_ts_by(lead, 384, pb + 16 * s + 8 * part, dv + (uint64_t)(s * (2048 >> 4)), IDESC_O, part == 0 || s > 0);
+            umma_commit_by(lead, o_full + t);
+            if (t == 1) umma_commit_by(lead, &v_empty);
+            if (item + 3 < 2 * n) scores(item + 3);               // (behind the product that read the buffer)
+            else sb = sb == 256 ? 0 : sb + 128;
         }
         wait_flight(&v_empty, (n - 1) & 1);                       // the last commit: nothing of this CTA is in flight behind its end
     }

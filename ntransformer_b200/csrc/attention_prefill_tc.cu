@@ -4,7 +4,7 @@
 // attends keys 0..start_pos + i.  The form on mma.sync (attention_prefill_mma.cu), which windows and BF16 caches still take, is bound by that instruction: two halves
 // of each query and of each weight make four products where one is counted.  Here:
 //   * a CTA owns two tiles of 128 queries that share their keys (two heads of a key head; two runs of queries where it has an odd number): while the tensor cores
-//     multiply for one, eight warps, a row to a lane, form the weights of the other;
+//     multiply for one, eight warps form the weights of the other;
 //   * scores S = (q_hi + q_lo) . K^T: queries split in shared memory, each row under a power of two that keeps its low halves' bits, keys by TMA, 128 at a time, two
 //     buffers; 128 x 128 scores in tensor memory, three buffers that the tiles use in turn, so that a tile's next scores are there when its weights are handed over;
 //   * weights exp2(f S - m) as F16 hi + lo take the scores' place in tensor memory, which is the A operand of (p_hi + p_lo) . V;
@@ -22,10 +22,10 @@ namespace nt { namespace b200 {
 namespace {
 
 constexpr int TQ = 128, TK = 128;                        // queries of a tile, keys of a step
-constexpr int TC_THREADS = 12 * 32;                      // warps 0-3 and 4-7: softmax of the two tiles, 8: TMA, 9: MMA; registers 2 x 216 + 72 = 3 x 168 at launch
+constexpr int TC_THREADS = 20 * 32;                      // warps 0-7 and 8-15: softmax of the two tiles, 16: TMA, 17: MMA; registers 4 x 104 + 64 = 5 x 96 at launch
 template <int HD> struct TcSmem {
     static constexpr int Q = TQ * HD * 2, KV = TK * HD * 2;              // bytes of a tile's half of the queries; of a step's keys or values
-    static constexpr int K0 = 4 * Q, V0 = K0 + 2 * KV, ALL = V0 + KV + 1024;
+    static constexpr int K0 = 4 * Q, V0 = K0 + 2 * KV, ALL = V0 + KV;
 };
 
 __device__ __forceinline__ void umma_ss_by(uint32_t lead, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
@@ -55,9 +55,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
     using S = TcSmem<HD>;
     constexpr int BOXES = HD / 64, BOX = TK * 128;                // boxes of 64 channels
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* smem = smem_raw;                                     // the declared alignment: there is no room to round up
+    if (smem_u32(smem) & 1023u) { if (threadIdx.x == 0) report(p.status); return; }
     __shared__ uint64_t k_full[2], k_empty[2], v_full, v_empty, q_full, s_full[3], p_full[2], o_full[2], o_empty;
-    __shared__ float factor[2 * TQ];                              // of a row's scores: log2 e * scale, and the power of two taken back
+    __shared__ float row_word[2][2 * TQ];                         // [half of the keys][row]: factors first, then a step's maxima, at the end the sums
     __shared__ uint32_t tmem_base_smem, dead_smem;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t dead = smem_u32(&dead_smem);
@@ -66,13 +67,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
     const int first_q = qt * (p.pairs_of_queries ? 2 * TQ : TQ), last_q = min(first_q + (p.pairs_of_queries ? 2 * TQ : TQ), p.seq_len) - 1;
     const int n = (p.start_pos + last_q) / TK + 1;               // steps
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; i++) { mbar_init(k_full + i, 1); mbar_init(k_empty + i, 1); mbar_init(p_full + i, 4); mbar_init(o_full + i, 1); }
+        for (int i = 0; i < 2; i++) { mbar_init(k_full + i, 1); mbar_init(k_empty + i, 1); mbar_init(p_full + i, 8); mbar_init(o_full + i, 1); }
         for (int i = 0; i < 3; i++) mbar_init(s_full + i, 1);
-        mbar_init(&v_full, 1); mbar_init(&v_empty, 1); mbar_init(&q_full, 8); mbar_init(&o_empty, 4);
+        mbar_init(&v_full, 1); mbar_init(&v_empty, 1); mbar_init(&q_full, 16); mbar_init(&o_empty, 8);
         dead_smem = 0;
         mbar_fence_init();
     }
-    if (warp == 9) {
+    if (warp == 17) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_smem)), "n"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
@@ -83,18 +84,21 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
     pdl_wait();
     // Step j of tile t is item 2 j + t.  Tensor memory is this CTA's whole: an item's scores, then weights, at column 128 (item mod 3), its product with V at 384.
 
-    if (warp < 8) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
-        const int t = warp >> 2, r = (warp & 3) * 32 + lane, head = p.pairs_of_queries ? h0 : h0 + t, q0 = first_q + (p.pairs_of_queries ? t * TQ : 0), row = q0 + r;
-        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16, to = lanes + 384;
+    if (warp < 16) {
+        // ---- softmax: a row to two lanes, each with half of a step's keys and half of the channels (four warps to a scheduler hide what one waits for) ----
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+        constexpr int HK = TK / 2, HC = HD / 2;
+        const int t = warp >> 3, quarter = warp & 3, half = (warp >> 2) & 1, r = quarter * 32 + lane, head = p.pairs_of_queries ? h0 : h0 + t;
+        const int q0 = first_q + (p.pairs_of_queries ? t * TQ : 0), row = q0 + r;
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16, to = lanes + 384 + half * HC;
         uint8_t* mine = smem + 2 * t * S::Q;                      // the tile's queries
         {
             // a row to LR lanes, so that loads are whole lines; 4 channels to a lane
             constexpr int LR = HD / 4, RI = 32 / LR;              // lanes of a row, rows of an instruction
             const int c = lane % LR;
 #pragma unroll 8
-            for (int i = 0; i < 32 / RI; i++) {
-                const int rr = (warp & 3) * 32 + i * RI + lane / LR;
+            for (int i = 0; i < 16 / RI; i++) {
+                const int rr = quarter * 32 + half * 16 + i * RI + lane / LR;
                 const float4 x = __ldg(reinterpret_cast<const float4*>(p.Q + ((size_t)min(q0 + rr, p.seq_len - 1) * p.n_heads + head) * HD) + c);
                 float amax = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
 #pragma unroll
@@ -102,7 +106,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 const uint32_t e = __float_as_uint(amax) >> 23 & 255u;       // not finite, or zero: as it is
                 const uint32_t up = e == 255u || e == 0u ? 127u : min(227u, max(27u, 264u - e));       // to 2^10 .. 2^11
                 const float g = __uint_as_float(up << 23);
-                if (c == 0) factor[t * TQ + rr] = p.scale * 1.4426950408889634f * __uint_as_float((254u - up) << 23);
+                if (c == 0) row_word[0][t * TQ + rr] = p.scale * 1.4426950408889634f * __uint_as_float((254u - up) << 23);
                 uint2 h, l;
                 split_pair(x.x * g, x.y * g, 0, h.x, l.x);
                 split_pair(x.z * g, x.w * g, 0, h.y, l.y);
@@ -115,90 +119,92 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
             __syncwarp();
             if (lane == 0) mbar_arrive(&q_full);
         }
-        const float f = factor[t * TQ + r];
-        uint64_t o[HD / 2];                                       // pairs of channels
+        auto meet = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + t * 4 + quarter) : "memory"); };      // the two warps of a quarter's rows
+        meet();
+        const float f = row_word[0][t * TQ + r];                  // of the row's scores: log2 e * scale, and the power of two taken back
+        meet();
+        uint64_t o[HC / 2];                                       // pairs of channels
 #pragma unroll
-        for (int i = 0; i < HD / 2; i++) o[i] = 0;
+        for (int i = 0; i < HC / 2; i++) o[i] = 0;
         float m = -INFINITY, l = 0.f;
-        auto drain = [&](int j, float alpha) {                    // the product of step j joins the sums
-            wait_cta(o_full + t, j & 1, dead);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t a = pack2(alpha, alpha);
-#pragma unroll
-            for (int c = 0; c < HD / 32; c++) {
-                uint32_t v[32];
-                tmem_ld32(to + 32 * c, v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 16; i++) o[16 * c + i] = fma2(o[16 * c + i], a, pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&o_empty);
-        };
         uint32_t ts = lanes + t * 128;                            // of the step's scores
 #pragma unroll 1
         for (int j = 0; j < n; j++) {
-            const int seen = p.start_pos + row - j * TK;          // this step's keys up to here are seen
+            const int seen = p.start_pos + row - j * TK - half * HK;     // of this lane's keys those up to here are seen
             const bool whole = j * TK + TK - 1 <= p.start_pos + q0;      // by every row of the tile
             wait_cta(s_full + ((2 * j + t) % 3), ((2 * j + t) / 3) & 1, dead);      // (of the buffer: a tile's next scores may come before these are looked at)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float mx = -INFINITY;
 #pragma unroll
-            for (int c = 0; c < TK / 32; c++) {
-                uint32_t v[32];
-                tmem_ld32(ts + 32 * c, v);
+            for (int c = 0; c < HK / 16; c++) {
+                uint32_t v[16];
+                tmem_ld16(ts + half * HK + 16 * c, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (whole) {
 #pragma unroll
-                    for (int i = 0; i < 32; i++) mx = fmaxf(mx, __uint_as_float(v[i]));
+                    for (int i = 0; i < 16; i++) mx = fmaxf(mx, __uint_as_float(v[i]));
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 32; i++) mx = fmaxf(mx, 32 * c + i <= seen ? __uint_as_float(v[i]) : -INFINITY);
+                    for (int i = 0; i < 16; i++) mx = fmaxf(mx, 16 * c + i <= seen ? __uint_as_float(v[i]) : -INFINITY);
                 }
             }
+            row_word[half][t * TQ + r] = mx;                      // (the other warp has read the step before: that step's product waited for its weights)
+            meet();
+            mx = fmaxf(mx, row_word[half ^ 1][t * TQ + r]);
             const float mn = fmaxf(m, mx * f), base = mn == -INFINITY ? 0.f : mn, alpha = exp2f(m - base);      // (a run of keys wholly unseen leaves the maximum; step 0 has key 0)
             m = mn;
             float sum = 0.f;
 #pragma unroll
-            for (int c = 0; c < TK / 32; c++) {
-                uint32_t v[32];
-                tmem_ld32(ts + 32 * c, v);
+            for (int c = 0; c < HK / 16; c++) {                   // 16 keys: 8 columns hi, 8 lo, where their scores were
+                uint32_t v[16], w[16];
+                tmem_ld16(ts + half * HK + 16 * c, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (!whole)
 #pragma unroll
-                    for (int i = 0; i < 32; i++) v[i] = 32 * c + i <= seen ? v[i] : 0xFF800000u;
+                    for (int i = 0; i < 16; i++) v[i] = 16 * c + i <= seen ? v[i] : 0xFF800000u;
 #pragma unroll
-                for (int h = 0; h < 2; h++) {                     // 16 keys: 8 columns hi, 8 lo, where their scores were
-                    uint32_t w[16];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const float a = exp2f(fmaf(__uint_as_float(v[16 * h + 2 * i]), f, -base)), b = exp2f(fmaf(__uint_as_float(v[16 * h + 2 * i + 1]), f, -base));
-                        sum += a + b;
-                        split_pair(a, b, 0, w[i], w[8 + i]);
-                    }
-                    tmem_st16(ts + 32 * c + 16 * h, w);
+                for (int i = 0; i < 8; i++) {
+                    const float a = exp2f(fmaf(__uint_as_float(v[2 * i]), f, -base)), b = exp2f(fmaf(__uint_as_float(v[2 * i + 1]), f, -base));
+                    sum += a + b;
+                    split_pair(a, b, 0, w[i], w[8 + i]);
                 }
+                tmem_st16(ts + half * HK + 16 * c, w);
             }
             l = fmaf(l, alpha, sum);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full + t);
-            drain(j, alpha);
+            // the step's product joins the sums
+            wait_cta(o_full + t, j & 1, dead);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t aa = pack2(alpha, alpha);
+#pragma unroll
+            for (int c = 0; c < HC / 16; c++) {
+                uint32_t v[16];
+                tmem_ld16(to + 16 * c, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 8; i++) o[8 * c + i] = fma2(o[8 * c + i], aa, pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&o_empty);
             ts = ts == lanes ? lanes + 256 : ts - 128;            // two items on
         }
+        row_word[half][t * TQ + r] = l;
+        meet();
         if (word_set(dead)) report(p.status);
         else {
-            // 16 rows at a time over the tile's queries (no product reads them any more), then whole rows to memory
-            const float inv = 1.0f / l;
-            constexpr int PITCH = HD + 4, LR = HD / 4, RI = 32 / LR;
-            float* stage = reinterpret_cast<float*>(mine) + (warp & 3) * 16 * PITCH;
+            // 16 rows at a time over the tile's queries (no product reads them any more), then whole lines to memory
+            const float inv = 1.0f / (l + row_word[half ^ 1][t * TQ + r]);
+            constexpr int PITCH = HC + 4, LR = HC / 4, RI = 32 / LR;
+            float* stage = reinterpret_cast<float*>(mine) + (warp & 7) * 16 * PITCH;
 #pragma unroll
-            for (int half = 0; half < 2; half++) {
-                if ((lane >> 4) == half)
+            for (int part = 0; part < 2; part++) {
+                if ((lane >> 4) == part)
 #pragma unroll
-                    for (int i = 0; i < HD / 4; i++) {
+                    for (int i = 0; i < HC / 4; i++) {
                         float4 x;
                         unpack2(o[2 * i], x.x, x.y); unpack2(o[2 * i + 1], x.z, x.w);
                         *reinterpret_cast<float4*>(stage + (lane & 15) * PITCH + 4 * i) = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
@@ -206,16 +212,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 __syncwarp();
 #pragma unroll 4
                 for (int i = 0; i < 16 / RI; i++) {
-                    const int rr = i * RI + lane / LR, at = q0 + (warp & 3) * 32 + half * 16 + rr;
+                    const int rr = i * RI + lane / LR, at = q0 + quarter * 32 + part * 16 + rr;
                     if (at < p.seq_len)
-                        *(reinterpret_cast<float4*>(p.out + ((size_t)at * p.n_heads + head) * HD) + lane % LR) = *reinterpret_cast<const float4*>(stage + rr * PITCH + 4 * (lane % LR));
+                        *(reinterpret_cast<float4*>(p.out + ((size_t)at * p.n_heads + head) * HD + half * HC) + lane % LR) = *reinterpret_cast<const float4*>(stage + rr * PITCH + 4 * (lane % LR));
                 }
                 __syncwarp();
             }
         }
     } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-    if (warp == 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    if (warp == 16) {
         if (lane == 0) {                                          // ---- keys and values by TMA: keys a step ahead ----
             auto load = [&](uint8_t* d, const CUtensorMap* map, int j, uint64_t* full) {
                 mbar_expect_tx(full, S::KV);
@@ -238,7 +244,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 if (values) wait_flight(&v_full, (values - 1) & 1);
             }
         }
-    } else if (warp == 9) {
+    } else if (warp == 17) {
         // ---- MMA: the whole warp walks the loop and one lane issues by predicate, so that operands stay in uniform registers ----
         const uint32_t lead = elect_lane();
         constexpr uint32_t F32_M128 = (1u << 4) | (8u << 24);
@@ -289,7 +295,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     __syncwarp();
-    if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_smem), "n"(512));
+    if (warp == 17) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_smem), "n"(512));
 }
 
 template <int HD>

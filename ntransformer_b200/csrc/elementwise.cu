@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(256) rmsnorm_xq_kernel(float* __restrict__ y, 
 template <bool INTERLEAVED>
 __global__ void rope_kernel(float* __restrict__ q, float* __restrict__ k, const int* __restrict__ positions, int seq_len,
                             int n_heads, int n_kv_heads, int head_dim, float theta_base, float freq_scale) {
+    pdl_launch_dependents();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int half_dim = head_dim / 2;
     const int total_q = seq_len * n_heads * half_dim, total_k = seq_len * n_kv_heads * half_dim;
@@ -114,8 +115,9 @@ __global__ void rope_kernel(float* __restrict__ q, float* __restrict__ k, const 
     const int li = is_key ? idx - total_q : idx;
     const int n_h = is_key ? n_kv_heads : n_heads;
     const int pair = li % half_dim, head = (li / half_dim) % n_h, sp = li / (half_dim * n_h);
+    const float freq = 1.0f / powf(theta_base, (2.0f * pair) / head_dim);
+    pdl_wait();
     const int pos = positions[sp];
-    float freq = 1.0f / powf(theta_base, (2.0f * pair) / head_dim);
     float angle = pos * freq * freq_scale;
     float c = cosf(angle), sn = sinf(angle);
     float* d = (is_key ? k : q) + (size_t)sp * n_h * head_dim + (size_t)head * head_dim;
@@ -128,6 +130,8 @@ __global__ void rope_kernel(float* __restrict__ q, float* __restrict__ k, const 
 // ---- KV-cache write: F32 -> F16 RN at [start_pos + s] (attention.cu:316-342) ----
 __global__ void kv_write_kernel(__half* __restrict__ kc, __half* __restrict__ vc, const float* __restrict__ k,
                                 const float* __restrict__ v, int seq_len, int row /* n_kv * hd */, int start_pos, int max_seq) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= seq_len * row) return;
     const int s = idx / row, c = idx - s * row;
@@ -228,6 +232,8 @@ __global__ void add_kernel(float* out, const float* a, const float* b, int n) {
     if (i < n) out[i] = a[i] + b[i];
 }
 __global__ void copy_kernel(float* __restrict__ dst, const float* __restrict__ src, int n) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = src[i];
 }
@@ -348,7 +354,7 @@ inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 void quantize_x(const float* x, void* xq, int K, cudaStream_t s) {
     NT_CHECK(K % 128 == 0, "quantize_x: K must be a multiple of 128");
-    launch_k(quantize_x_kernel, dim3(cdiv(K, 256)), dim3(256), 0, s, x, static_cast<int8_t*>(xq), K);
+    launch_k_pdl(true, quantize_x_kernel, dim3(cdiv(K, 256)), dim3(256), 0, s, x, static_cast<int8_t*>(xq), K);
     count_launch();
 }
 
@@ -356,12 +362,12 @@ static int norm_threads(int hidden) { return hidden <= 1024 ? 256 : hidden <= 40
 
 void rmsnorm(float* y, const float* x, const float* w, int rows, int hidden, float eps, cudaStream_t s) {
     if (rows <= 0) return;
-    launch_k(rmsnorm_kernel<false>, dim3(rows), dim3(norm_threads(hidden)), 0, s, (void*)y, x, w, hidden, eps);
+    launch_k_pdl(true, rmsnorm_kernel<false>, dim3(rows), dim3(norm_threads(hidden)), 0, s, (void*)y, x, w, hidden, eps);
     count_launch();
 }
 void rmsnorm_f16(void* y, const float* x, const float* w, int rows, int hidden, float eps, cudaStream_t s) {
     if (rows <= 0) return;
-    rmsnorm_kernel<true><<<rows, norm_threads(hidden), 0, s>>>(y, x, w, hidden, eps);
+    launch_k_pdl(true, rmsnorm_kernel<true>, dim3(rows), dim3(norm_threads(hidden)), 0, s, y, x, w, hidden, eps);
     count_launch();
 }
 void rmsnorm_xq(float* y, void* xq, const float* x, const float* w, int hidden, float eps, cudaStream_t s) {
@@ -373,16 +379,15 @@ void rope(float* q, float* k, const int* positions, int seq_len, int n_heads, in
           float theta, float freq_scale, bool interleaved, cudaStream_t s) {
     int total = seq_len * (n_heads + n_kv_heads) * (head_dim / 2);
     if (total <= 0) return;
-    if (interleaved) rope_kernel<true><<<cdiv(total, 256), 256, 0, s>>>(q, k, positions, seq_len, n_heads, n_kv_heads, head_dim, theta, freq_scale);
-    else rope_kernel<false><<<cdiv(total, 256), 256, 0, s>>>(q, k, positions, seq_len, n_heads, n_kv_heads, head_dim, theta, freq_scale);
+    launch_k_pdl(true, interleaved ? rope_kernel<true> : rope_kernel<false>, dim3(cdiv(total, 256)), dim3(256), 0, s, q, k, positions, seq_len, n_heads, n_kv_heads, head_dim,
+                 theta, freq_scale);
     count_launch();
 }
 void copy_to_kv_cache(void* kc, void* vc, const float* k, const float* v, int seq_len, int n_kv, int hd,
                       int start_pos, int max_seq, cudaStream_t s) {
     int total = seq_len * n_kv * hd;
     if (total <= 0) return;
-    kv_write_kernel<<<cdiv(total, 256), 256, 0, s>>>(static_cast<__half*>(kc), static_cast<__half*>(vc), k, v, seq_len,
-                                                     n_kv * hd, start_pos, max_seq);
+    launch_k_pdl(true, kv_write_kernel, dim3(cdiv(total, 256)), dim3(256), 0, s, static_cast<__half*>(kc), static_cast<__half*>(vc), k, v, seq_len, n_kv * hd, start_pos, max_seq);
     count_launch();
 }
 bool rope_kv_rows(float* q, const float* k, const float* v, void* kc, void* vc, int tokens, int start_pos, int n_heads, int n_kv, int hd, float theta, float freq_scale,
@@ -403,19 +408,19 @@ void rope_kv_decode(float* q, float* k, const float* v, void* kc, void* vc, cons
 }
 void silu_mul(float* out, const float* gate, const float* up, int n, cudaStream_t s) {
     if (n <= 0) return;
-    launch_k(silu_mul_kernel, dim3(cdiv(n, 256)), dim3(256), 0, s, out, gate, up, n);
+    launch_k_pdl(true, silu_mul_kernel, dim3(cdiv(n, 256)), dim3(256), 0, s, out, gate, up, n);
     count_launch();
 }
 void add(float* out, const float* a, const float* b, int n, cudaStream_t s) {
     if (n <= 0) return;
-    launch_k(add_kernel, dim3(cdiv(n, 256)), dim3(256), 0, s, out, a, b, n);
+    launch_k_pdl(true, add_kernel, dim3(cdiv(n, 256)), dim3(256), 0, s, out, a, b, n);
     count_launch();
 }
 void add_inplace(float* a, const float* b, int n, cudaStream_t s) { add(a, a, b, n, s); }
 void add_bias(float* y, const float* b, int n, cudaStream_t s) { add(y, y, b, n, s); }
 void copy(float* dst, const float* src, int n, cudaStream_t s) {
     if (n <= 0) return;
-    copy_kernel<<<cdiv(n, 256), 256, 0, s>>>(dst, src, n);
+    launch_k_pdl(true, copy_kernel, dim3(cdiv(n, 256)), dim3(256), 0, s, dst, src, n);
     count_launch();
 }
 void cosine_similarity(float* result, const float* a, const float* b, int n, cudaStream_t s) {

@@ -264,12 +264,12 @@ void gemv_generic(float* y, const void* W, const float* x, int out, int in, DTyp
         int grid16 = (pairs + F16_WARPS - 1) / F16_WARPS;
         const int resident = (int)std::min<size_t>(8, (size_t)(220 * 1024) / ((size_t)in * 4 + 1024)) * 148;   // CTAs the chip holds
         if (grid16 > resident && resident > 0) grid16 = resident;
-        launch_k(gemv_f16_kernel, dim3(grid16), dim3(F16_WARPS * 32), (size_t)in * 4, s, y, w, x, out, in, pitch, (int)ep);
+        launch_k_pdl(true, gemv_f16_kernel, dim3(grid16), dim3(F16_WARPS * 32), (size_t)in * 4, s, y, w, x, out, in, pitch, (int)ep);
         count_launch();
         return;
     }
     int grid = (out + GW * RPW - 1) / (GW * RPW);
-#define NT_LAUNCH(DTV) launch_k(gemv_generic_kernel<(int)DTV>, dim3(grid), dim3(GW * 32), 0, s, y, w, x, out, in, pitch, (int)ep)
+#define NT_LAUNCH(DTV) launch_k_pdl(true, gemv_generic_kernel<(int)DTV>, dim3(grid), dim3(GW * 32), 0, s, y, w, x, out, in, pitch, (int)ep)
     switch (dt) {
         case DType::F32: NT_LAUNCH(DType::F32); break;
         case DType::F16: NT_LAUNCH(DType::F16); break;

@@ -49,6 +49,7 @@ struct KqParams {
     int total_groups;          // groups of 16 rows of a matrix; SWIGLU: pairs of them, gate and up (two segments), or 8 rows of gate and the same 8 of up (halves)
     int n_seg;                 // segments (matrices) per group
     int halves;
+    int weights_settled;       // no launch still under way writes the weights: they are read ahead of the wait for the launch before
     int epilogue;
     int stages, slot;          // depth of a team's ring and bytes of a stage
     unsigned* status;          // wait_status.cuh
@@ -131,6 +132,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
         int slot = 0;
         uint32_t parity = 1;                                    // the first round finds every slot empty
         bool ahead = true;                                      // still in it
+        if (!p.weights_settled) pdl_wait();
         for (int u = u0; u < p.total_groups; u += ustep) {
             for (int seg = 0; seg < p.n_seg; seg++) {
                 int mi, gl;
@@ -425,7 +427,7 @@ void launch_teams(KqParams& p, cudaStream_t s) {
     opt_in_dynamic_smem(gemv_mma_kernel<MASK, KW, TEAMS>, (int)SMEM_CTA, configured);
     const size_t smem = SM_X + x_bytes(p.K, MASK & WHOLE ? 4 : 3) + (size_t)p.stages * p.slot * TEAMS;
     const int places = num_sms() * (smem > SMEM_HALF ? 1 : ctas);
-    launch_k(gemv_mma_kernel<MASK, KW, TEAMS>, dim3(p.total_groups < places ? p.total_groups : places), dim3(TEAMS * (KW + 1) * 32), smem, s, p);
+    launch_k_pdl(true, gemv_mma_kernel<MASK, KW, TEAMS>, dim3(p.total_groups < places ? p.total_groups : places), dim3(TEAMS * (KW + 1) * 32), smem, s, p);
     count_launch();
 }
 
@@ -540,6 +542,7 @@ void gemv_kq(const GemvMat* mats, int n_mat, int K, const GemvInput& in, GemvEpi
     }
     p.halves = ep == GEMV_SWIGLU && halves_of(mats[0], mats[1], K);
     p.n_seg = ep == GEMV_SWIGLU && !p.halves ? 2 : 1;
+    p.weights_settled = pdl_enabled();                         // a step of the engine; behind the launcher boundary the launch before may have written them
     p.status = wait_status();
     switch (mask) {
         case 1: launch_fmt<1>(p, s); break;

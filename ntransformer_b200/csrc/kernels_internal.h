@@ -498,7 +498,9 @@ void mlstm_token(float* out, const float* q, const float* k, const float* v, con
 // Programmatic dependent launch (PDL): when enabled, kernels are launched with
 // cudaLaunchAttributeProgrammaticStreamSerialization so that a kernel's prologue (barrier init, TMA weight
 // prefetch) overlaps the tail of its predecessor; every kernel executes griddepcontrol.wait before it touches
-// data produced upstream, so ordering is unchanged.  Off by default; the engine turns it on for decode graphs.
+// data produced upstream, so ordering is unchanged.  launch_k: off by default, the engine turns it on for decode graphs; there kernels may read weights ahead of the wait.
+// launch_k_pdl(true, ...): everywhere, for kernels that read nothing ahead of it then.  Behind the launcher boundary, call by call, a launch waits for the one before
+// to drain and then starts for 1.3 .. 2.3 us (one Q8_0 matrix of 1024 x 4096: 6.14 -> 3.87 us a call, a decoder layer's sixteen launches 112 -> 80.6 us).
 void set_pdl(bool on);
 bool pdl_enabled();
 template <typename... KArgs, typename... Args>

@@ -555,8 +555,8 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
     constexpr int KEEP = 7;                                        // chunks of 2048 held in registers: rows to 14336
     __shared__ float red[2][16];
     const int tid = threadIdx.x;
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();               // after the wait: the product reads weights before its own, and whatever wrote them came before this launch
     const size_t at = (size_t)blockIdx.x * K;
     const float* x = xin + at;
     const float* y = MODE == TOK_SILU ? w + at : w;

@@ -9,6 +9,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -17,6 +18,7 @@ CSRC = PKG / "csrc"
 OBJ = PKG / "_build"
 LIB = PKG / "libnt_b200.so"
 CLI = PKG / "ntransformer"
+FAST = PKG / "_fast.so"           # CPython extension of the launcher boundary (csrc/fast_call.cpp)
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "--use_fast_math", "-Xcompiler", "-fPIC,-Wall,-Wno-unused-function",
@@ -34,7 +36,7 @@ def _nvcc() -> str:
 
 
 def sources() -> list[Path]:
-    srcs = sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cpp"))
+    srcs = sorted(CSRC.glob("*.cu")) + sorted(p for p in CSRC.glob("*.cpp") if p.name != "fast_call.cpp")
     eng = CSRC / "engine"
     if eng.is_dir():
         srcs += sorted(p for p in eng.glob("*.cpp") if p.name != "main.cpp") + sorted(eng.glob("*.cu"))
@@ -78,6 +80,13 @@ def build(verbose: bool = False, force: bool = False) -> Path:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    fast = CSRC / "fast_call.cpp"
+    if not FAST.exists() or FAST.stat().st_mtime < max(fast.stat().st_mtime, hdr_m):
+        cmd = [shutil.which("g++") or "g++", "-std=c++17", "-O2", "-Wall", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], "-o", str(FAST), str(fast)]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("building the launcher extension failed")
     main = CSRC / "engine" / "main.cpp"
     if main.exists() and (not CLI.exists() or CLI.stat().st_mtime < max(LIB.stat().st_mtime, main.stat().st_mtime)):
         cmd = [_nvcc(), *COMMON, "-I", str(CSRC), "-I", str(PKG.parent / "include"), "-o", str(CLI), str(main),

@@ -10,7 +10,7 @@ import ctypes as C
 
 import torch
 
-from ._lib import lib
+from ._lib import SIGNATURES, lib
 from .dtypes import DType
 
 
@@ -34,79 +34,97 @@ def _s(stream):
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 
+def _launch(name, args):
+    """A launch through ctypes: the route of arguments that csrc/fast_call.cpp leaves alone (a c_void_p, a NumPy integer, ...)."""
+    types = SIGNATURES["nt_b200_" + name][1]
+    getattr(lib(), "nt_b200_" + name)(*(_p(a) if t is C.c_void_p else a for a, t in zip(args[:-1], types)), _s(args[-1]))
+
+
+_entries = None       # csrc/fast_call.cpp: takes tensors, raw pointers (ints) or None, and a stream (None: the current one)
+
+
+def _fast():
+    global _entries
+    if _entries is None:
+        try:
+            from . import _fast as m
+        except ImportError as e:
+            raise RuntimeError("ntransformer_b200/_fast.so is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`") from e
+        m.bind(torch.Tensor, torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice, torch.cuda.init, _launch,
+               {n: C.cast(getattr(lib(), "nt_b200_" + n), C.c_void_p).value for n in m.ENTRIES})
+        _entries = m
+    return _entries
+
+
 def launch_rmsnorm(output, input, weight, batch_size, hidden_size, eps, stream=None):
-    lib().nt_b200_rmsnorm(_p(output), _p(input), _p(weight), batch_size, hidden_size, eps, _s(stream))
+    _fast().rmsnorm(output, input, weight, batch_size, hidden_size, eps, stream)
 
 
 def launch_rmsnorm_f16(output, input, weight, batch_size, hidden_size, eps, stream=None):
-    lib().nt_b200_rmsnorm_f16(_p(output), _p(input), _p(weight), batch_size, hidden_size, eps, _s(stream))
+    _fast().rmsnorm_f16(output, input, weight, batch_size, hidden_size, eps, stream)
 
 
 def launch_rope(q, k, positions, batch_size, seq_len, n_heads, n_kv_heads, head_dim, theta_base, freq_scale,
                 interleaved, stream=None):
-    lib().nt_b200_rope(_p(q), _p(k), _p(positions), batch_size, seq_len, n_heads, n_kv_heads, head_dim, theta_base,
-                       freq_scale, int(bool(interleaved)), _s(stream))
+    _fast().rope(q, k, positions, batch_size, seq_len, n_heads, n_kv_heads, head_dim, theta_base, freq_scale, int(bool(interleaved)), stream)
 
 
 def launch_softmax(output, input, rows, cols, stream=None):
-    lib().nt_b200_softmax(_p(output), _p(input), rows, cols, _s(stream))
+    _fast().softmax(output, input, rows, cols, stream)
 
 
 def launch_masked_softmax(output, input, mask, rows, cols, stream=None):
-    lib().nt_b200_masked_softmax(_p(output), _p(input), _p(mask), rows, cols, _s(stream))
+    _fast().masked_softmax(output, input, mask, rows, cols, stream)
 
 
 def launch_gemv(y, W, x, out_features, in_features, weight_dtype, stream=None):
-    lib().nt_b200_gemv(_p(y), _p(W), _p(x), out_features, in_features, int(weight_dtype), _s(stream))
+    _fast().gemv(y, W, x, out_features, in_features, int(weight_dtype), stream)
 
 
 def launch_gemv_add(y, W, x, out_features, in_features, weight_dtype, stream=None):
-    lib().nt_b200_gemv_add(_p(y), _p(W), _p(x), out_features, in_features, int(weight_dtype), _s(stream))
+    _fast().gemv_add(y, W, x, out_features, in_features, int(weight_dtype), stream)
 
 
 def launch_gemm_f32(Cm, A, B, M, N, K, stream=None):
-    lib().nt_b200_gemm_f32(_p(Cm), _p(A), _p(B), M, N, K, _s(stream))
+    _fast().gemm_f32(Cm, A, B, M, N, K, stream)
 
 
 def launch_silu_mul(output, gate, up, size, stream=None):
-    lib().nt_b200_silu_mul(_p(output), _p(gate), _p(up), size, _s(stream))
+    _fast().silu_mul(output, gate, up, size, stream)
 
 
 def launch_add_bias(y, bias, size, stream=None):
-    lib().nt_b200_add_bias(_p(y), _p(bias), size, _s(stream))
+    _fast().add_bias(y, bias, size, stream)
 
 
 def launch_attention_decode(output, q, k_cache, v_cache, seq_len, n_heads, n_kv_heads, head_dim, max_seq, scale,
                             stream=None):
-    lib().nt_b200_attention_decode(_p(output), _p(q), _p(k_cache), _p(v_cache), seq_len, n_heads, n_kv_heads,
-                                   head_dim, max_seq, scale, _s(stream))
+    _fast().attention_decode(output, q, k_cache, v_cache, seq_len, n_heads, n_kv_heads, head_dim, max_seq, scale, stream)
 
 
 def launch_attention_prefill(output, Q, k_cache, v_cache, seq_len, start_pos, n_heads, n_kv_heads, head_dim,
                              max_seq, scale, stream=None):
-    lib().nt_b200_attention_prefill(_p(output), _p(Q), _p(k_cache), _p(v_cache), seq_len, start_pos, n_heads,
-                                    n_kv_heads, head_dim, max_seq, scale, _s(stream))
+    _fast().attention_prefill(output, Q, k_cache, v_cache, seq_len, start_pos, n_heads, n_kv_heads, head_dim, max_seq, scale, stream)
 
 
 def launch_copy_to_kv_cache(k_cache, v_cache, k, v, seq_len, n_kv_heads, head_dim, start_pos, max_seq, stream=None):
-    lib().nt_b200_copy_to_kv_cache(_p(k_cache), _p(v_cache), _p(k), _p(v), seq_len, n_kv_heads, head_dim, start_pos,
-                                   max_seq, _s(stream))
+    _fast().copy_to_kv_cache(k_cache, v_cache, k, v, seq_len, n_kv_heads, head_dim, start_pos, max_seq, stream)
 
 
 def launch_add(out, a, b, size, stream=None):
-    lib().nt_b200_add(_p(out), _p(a), _p(b), size, _s(stream))
+    _fast().add(out, a, b, size, stream)
 
 
 def launch_add_inplace(a, b, size, stream=None):
-    lib().nt_b200_add_inplace(_p(a), _p(b), size, _s(stream))
+    _fast().add_inplace(a, b, size, stream)
 
 
 def launch_copy(dst, src, size, stream=None):
-    lib().nt_b200_copy(_p(dst), _p(src), size, _s(stream))
+    _fast().copy(dst, src, size, stream)
 
 
 def launch_cosine_similarity(result, a, b, size, stream=None):
-    lib().nt_b200_cosine_similarity(_p(result), _p(a), _p(b), size, _s(stream))
+    _fast().cosine_similarity(result, a, b, size, stream)
 
 
 # ---- additions without a reference counterpart ----

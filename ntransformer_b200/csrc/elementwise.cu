@@ -63,23 +63,43 @@ __global__ void quantize_x_kernel(const float* __restrict__ x, int8_t* __restric
 }
 
 // ---- RMSNorm: y = x * rsqrtf(mean(x^2) + eps) * w, one CTA per row (rmsnorm.cu:17-70) ----
-template <bool HALF_OUT>
+// One row is all latency.  Up to KEEP elements to a thread, x and w are fetched once and together and stay in registers; longer rows read both again behind the sum.
+template <bool HALF_OUT, int KEEP>
 __global__ void __launch_bounds__(1024) rmsnorm_kernel(void* __restrict__ yv, const float* __restrict__ xin,
                                                        const float* __restrict__ w, int hidden, float eps) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float red[32];
     const float* x = xin + (size_t)blockIdx.x * hidden;
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) { float v = x[i]; ss += v * v; }
-    ss = block_sum(ss, red);
-    float mean_sq = ss / hidden;
-    float rms_inv = rsqrtf(mean_sq + eps);
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        const float v = x[i] * rms_inv * w[i];
+    auto store = [&](int i, float v) {
         if (HALF_OUT) reinterpret_cast<__half*>(yv)[(size_t)blockIdx.x * hidden + i] = __float2half(v);
         else reinterpret_cast<float*>(yv)[(size_t)blockIdx.x * hidden + i] = v;
+    };
+    float ss = 0.f;
+    if constexpr (KEEP > 0) {
+        float xs[KEEP], ws[KEEP];
+#pragma unroll
+        for (int j = 0; j < KEEP; j++) { const int i = threadIdx.x + j * blockDim.x; xs[j] = i < hidden ? x[i] : 0.f; }
+#pragma unroll
+        for (int j = 0; j < KEEP; j++) { const int i = threadIdx.x + j * blockDim.x; ws[j] = i < hidden ? w[i] : 0.f; }
+#pragma unroll
+        for (int j = 0; j < KEEP; j++) ss += xs[j] * xs[j];
+        const float rms_inv = rsqrtf(block_sum(ss, red) / hidden + eps);
+#pragma unroll
+        for (int j = 0; j < KEEP; j++) { const int i = threadIdx.x + j * blockDim.x; if (i < hidden) store(i, xs[j] * rms_inv * ws[j]); }
+    } else {
+        for (int i = threadIdx.x; i < hidden; i += blockDim.x) { float v = x[i]; ss += v * v; }
+        const float rms_inv = rsqrtf(block_sum(ss, red) / hidden + eps);
+        for (int i = threadIdx.x; i < hidden; i += blockDim.x) store(i, x[i] * rms_inv * w[i]);
     }
+}
+inline int norm_threads(int hidden) { return hidden <= 1024 ? 256 : hidden <= 4096 ? 512 : 1024; }
+template <bool HALF_OUT>
+void launch_rmsnorm_rows(void* y, const float* x, const float* w, int rows, int hidden, float eps, cudaStream_t s) {
+    constexpr int KEEP = 8;                                        // rows to 8192, the widest model's
+    const int threads = norm_threads(hidden);
+    launch_k_pdl(true, hidden <= KEEP * threads ? rmsnorm_kernel<HALF_OUT, KEEP> : rmsnorm_kernel<HALF_OUT, 0>, dim3(rows), dim3(threads), 0, s, y, x, w, hidden, eps);
+    count_launch();
 }
 
 // Multi-CTA RMSNorm + activation quantiser for the decode step: every CTA recomputes the (cheap, L2-resident)
@@ -358,17 +378,13 @@ void quantize_x(const float* x, void* xq, int K, cudaStream_t s) {
     count_launch();
 }
 
-static int norm_threads(int hidden) { return hidden <= 1024 ? 256 : hidden <= 4096 ? 512 : 1024; }
-
 void rmsnorm(float* y, const float* x, const float* w, int rows, int hidden, float eps, cudaStream_t s) {
     if (rows <= 0) return;
-    launch_k_pdl(true, rmsnorm_kernel<false>, dim3(rows), dim3(norm_threads(hidden)), 0, s, (void*)y, x, w, hidden, eps);
-    count_launch();
+    launch_rmsnorm_rows<false>(y, x, w, rows, hidden, eps, s);
 }
 void rmsnorm_f16(void* y, const float* x, const float* w, int rows, int hidden, float eps, cudaStream_t s) {
     if (rows <= 0) return;
-    launch_k_pdl(true, rmsnorm_kernel<true>, dim3(rows), dim3(norm_threads(hidden)), 0, s, y, x, w, hidden, eps);
-    count_launch();
+    launch_rmsnorm_rows<true>(y, x, w, rows, hidden, eps, s);
 }
 void rmsnorm_xq(float* y, void* xq, const float* x, const float* w, int hidden, float eps, cudaStream_t s) {
     NT_CHECK(hidden % 128 == 0, "rmsnorm_xq: hidden must be a multiple of 128");

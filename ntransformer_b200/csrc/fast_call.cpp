@@ -1,6 +1,6 @@
 // fast_call.cpp — the launcher boundary as a CPython extension (ntransformer_b200/_fast.so): what kernels.py's launch_* do with their arguments, without ctypes.
 //
-// Bound by the host: a call through ctypes took 6.1 us, of them 3 in the driver's launch, the rest in ctypes' conversions and the checks in Python.  A small matrix
+// Bound by the host: a call through ctypes takes 4.6 us, of them 2.5 in the driver's launch, the rest in ctypes' conversions and the checks in Python.  A small matrix
 // (Q8_0, 1024 x 4096) times a vector, call after call: 4.64 -> 3.87 us, the GPU's time; a decoder layer's sixteen launches on an idle GPU 112 -> 99 us.
 // The library's entries come as addresses from the library that is loaded (bind), so that an override of its path holds here too.  The GIL is let go
 // around the launch, as ctypes does.  Only the plain forms of an argument are taken here (a tensor, an int, a float, None, a stream object); a call with any

@@ -231,10 +231,10 @@ def run_prefill(args, rank, world):
                 "note": "algorithmic flops 2MNK; the kernel issues 2x that (F32 activations split into F16 hi+lo to keep parity <= 1e-3)",
                 "step_achieved": round(step_tf, 1), "step_frac": round(step_tf / peak, 4)}
     else:
-        roof = {"bound": "tensor", "kernel": "whole prefill step (gemm_blocks_kernel: blocks expanded to F16 hi + lo on the way into tensor memory)",
+        roof = {"bound": "tensor", "kernel": "whole prefill step (gemm_blocks_kernel: blocks expanded on the way into tensor memory)",
                 "achieved": round(step_tf, 1), "peak": peak, "unit": "TFLOP/s", "frac": round(step_tf / peak, 4), "traffic": None,
                 "peak_source": peak_src,
-                "note": "algorithmic flops; the path issues 3x that (activations and expanded weights both as F16 hi+lo, lo.lo left out)",
+                "note": "algorithmic flops; the path issues 2x that for Q4_K and Q5_K (activations as F16 hi+lo, weights as integers) and 3x for the other formats (weights as F16 hi+lo too, lo.lo left out)",
                 "step_achieved": round(step_tf, 1), "step_frac": round(step_tf / peak, 4)}
     line = {
         "metric": "prefill_tok_s", "value": round(tok_s, 1), "unit": "tok/s", "n_gpus": 1, "steps": steps, "warmup": args.warmup,

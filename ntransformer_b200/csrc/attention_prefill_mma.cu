@@ -8,6 +8,7 @@
 // registers (flash-attention-2 data flow).  F32 operands are split into two F16 terms (q = hi + lo, p = hi + lo) so
 // the result keeps ~22 mantissa bits and stays within the 2e-5 tolerance of the oracle.
 //
+// Prompts over an F16 cache take attention_prefill_tc.cu where their pointers start on 16 bytes; this form is for the others.
 // The same kernel serves windowed attention (csrc/attention_window.cu's rule: key j visible from position p iff j <= p and
 // (p - j < window or j < keep)), optionally with soft-capped scores cap * tanh(s / cap) and a BF16 cache (BF: both MMAs take
 // BF16 operands, the splits are BF16 pairs): a query block then walks only the key tiles of the kept prefix and of its window.

@@ -2,14 +2,16 @@
 //
 // Same contract as the reference's attention_prefill_kernel (src/cuda/attention.cu:216-311): F32 queries [seq][n_heads][hd], F16 cache [max_seq][n_kv][hd], query i
 // attends keys 0..start_pos + i.  The form on mma.sync (attention_prefill_mma.cu), which windows and BF16 caches still take, is bound by that instruction: two halves
-// of each query and of each weight make four products where one is counted.  Here:
+// of each query and of each weight make four products where two are counted.  Here:
 //   * a CTA owns two tiles of 128 queries that share their keys (two heads of a key head; two runs of queries where it has an odd number): while the tensor cores
-//     multiply for one, eight warps form the weights of the other;
+//     multiply for one, eight warps form the weights of the other (half of a row's keys each);
 //   * scores S = (q_hi + q_lo) . K^T: queries split in shared memory, each row under a power of two that keeps its low halves' bits, keys by TMA, 128 at a time, two
 //     buffers; 128 x 128 scores in tensor memory, three buffers that the tiles use in turn, so that a tile's next scores are there when its weights are handed over;
 //   * weights exp2(f S - m) as F16 hi + lo take the scores' place in tensor memory, which is the A operand of (p_hi + p_lo) . V;
 //   * that product of 128 keys starts at zero in the fourth quarter of tensor memory and is taken from there at once; the rows' sums are kept in F32 registers,
 //     rescaled there where the maximum moves.
+// 1000 tokens behind 1023, 32 heads of 128 over 8: 174 us on mma.sync, 62.2 here with eight warps for the weights, 56.9 with sixteen; 50 GFLOP issued in it, 0.9 PFLOP/s.
+// Bound by the forming of the weights, behind which the tensor cores wait.
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "tc_device.cuh"

@@ -778,7 +778,7 @@ bool Model::batched_prefill_ok(int seq_len, int start_pos) const {
     return true;
 }
 
-// A few tokens together through the decode step's arithmetic (gemv_rows.cu): every matrix on the block GEMV, one GPU.
+// A few tokens together, every matrix in blocks, one GPU: the decode step's arithmetic (gemv_rows.cu) or, where that takes two passes, the GEMM over blocks (prefill_blocks.cu).
 bool Model::short_batch_ok(int seq_len, int start_pos) const {
     if (tp_size_ != 1 || seq_len < 2 || prefill_min_tokens_ <= 0 || getenv("NT_B200_NO_BATCHED_PREFILL") || (fuse_mask_ & 6)) return false;
     const char* mk = getenv("NT_B200_MEGAKERNEL");

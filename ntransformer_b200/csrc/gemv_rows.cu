@@ -1,4 +1,4 @@
-// gemv_rows.cu — a few tokens (2 to 31) times matrices in GGUF blocks: Y[t, n] = sum_k W[n, k] X[t, k], every weight read once for 8 tokens.
+// gemv_rows.cu — a few tokens (the engine: to 8, Q8_0 and Q4_0 to 31) times matrices in GGUF blocks: Y[t, n] = sum_k W[n, k] X[t, k], every weight read once for 8 tokens.
 //
 // The reference runs its GEMV once for every prompt token (src/model/attention.cpp:144-162, ffn.cpp:96-133), and so did the engine below the length
 // where the tensor-core GEMM of prompts pays: 21 tokens cost 21 decode steps.  Here the arithmetic stays the decode step's — exact s32 products of the

@@ -117,7 +117,7 @@ void attention_prefill(float* out, const float* Q, const void* kc, const void* v
                        int n_heads, int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
 // attention_prefill_tc.cu: 128 x 128 tiles on tcgen05 (heads 64 and 128 wide, pointers on 16 bytes); false: nothing launched
 bool attention_prefill_tc(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, float scale, cudaStream_t s);
-// attention_prefill_mma.cu: 64-query x 64-key tiles on mma.sync (used by attention_prefill for seq_len >= 16, hd 64/128)
+// attention_prefill_mma.cu: 64-query x 64-key tiles on mma.sync (attention_prefill: seq_len >= 16, hd 64/128, pointers off 16 bytes; windows; BF16 caches)
 bool attention_prefill_mma_supported(int seq_len, int n_heads, int n_kv, int hd);
 void attention_prefill_mma(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads,
                            int n_kv, int hd, int max_seq, float scale, cudaStream_t s);

@@ -107,8 +107,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 for (int s = LR / 2; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, s));
                 const uint32_t e = __float_as_uint(amax) >> 23 & 255u;       // not finite, or zero: as it is
                 const uint32_t up = e == 255u || e == 0u ? 127u : min(227u, max(27u, 264u - e));       // to 2^10 .. 2^11
-                const float g = __uint_as_float(up << 23);
-                if (c == 0) row_word[0][t * TQ + rr] = p.scale * 1.4426950408889634f * __uint_as_float((254u - up) << 23);
+                const float g = copysignf(__uint_as_float(up << 23), p.scale);        // the scale's sign goes with the queries: the greatest score stays the greatest
+                if (c == 0) row_word[0][t * TQ + rr] = fabsf(p.scale) * 1.4426950408889634f * __uint_as_float((254u - up) << 23);
                 uint2 h, l;
                 split_pair(x.x * g, x.y * g, 0, h.x, l.x);
                 split_pair(x.z * g, x.w * g, 0, h.y, l.y);
@@ -161,12 +161,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 uint32_t v[16], w[16];
                 tmem_ld16(ts + half * HK + 16 * c, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (!whole)
+#pragma unroll
+                for (int i = 0; i < 16; i++) v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), f, -base));
+                if (!whole)                                       // behind the multiplication: f may be zero
 #pragma unroll
                     for (int i = 0; i < 16; i++) v[i] = 16 * c + i <= seen ? v[i] : 0xFF800000u;
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
-                    const float a = exp2f(fmaf(__uint_as_float(v[2 * i]), f, -base)), b = exp2f(fmaf(__uint_as_float(v[2 * i + 1]), f, -base));
+                    const float a = exp2f(__uint_as_float(v[2 * i])), b = exp2f(__uint_as_float(v[2 * i + 1]));
                     sum += a + b;
                     split_pair(a, b, 0, w[i], w[8 + i]);
                 }

@@ -74,3 +74,14 @@ def test_a_nan_stays_in_its_row_and_wide_scores():
     keep = torch.ones(200, 4, dtype=torch.bool, device="cuda")
     keep[7, 1] = False
     assert torch.isfinite(got[keep]).all() and rel(got[keep], want[keep]) <= 5e-5       # scores of up to 100: 2^-22 of them in the exponent
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("scale", [0.0, -0.0, -0.1, -1.0, 1e-30])
+@pytest.mark.parametrize("tokens,start", [(200, 50), (130, 0)])
+def test_a_scale_of_any_sign(dim, scale, tokens, start):
+    q, kc, vc = inputs(153, 51, dim, tokens, start)                # (three heads to a key head: runs of queries, whose first tile has whole steps behind it)
+    got, want = attend(q, kc, vc, start, scale), exact(q, kc, vc, start, scale)
+    # in the exponent: 2 * dim / 16 additions, each cut by 2/3 of 2^-24 of a score, and halves' pairs, 2^-22 of it; weights as above
+    most = abs(scale) * float((q.norm(dim=2).max() * kc[: start + tokens].float().norm(dim=2).max()).item())
+    assert torch.isfinite(got).all() and rel(got, want) <= 5e-6 + (dim / 8 * 2 / 3 * 2.0**-24 + 2.0**-22) * most

@@ -55,6 +55,10 @@ void nt_b200_attention_decode(float* output, const float* q, const void* k_cache
 void nt_b200_attention_prefill(float* output, const float* Q, const void* k_cache,
                                const void* v_cache, int seq_len, int start_pos, int n_heads,
                                int n_kv_heads, int head_dim, int max_seq, float scale, void* stream);
+/* The form that such a call takes (nothing is launched or read): 0 a query at a time, 1 tiles on mma.sync, 2 tiles on tcgen05. */
+int  nt_b200_attention_prefill_form(const float* output, const float* Q, const void* k_cache,
+                                    const void* v_cache, int seq_len, int start_pos, int n_heads,
+                                    int n_kv_heads, int head_dim, int max_seq);
 void nt_b200_copy_to_kv_cache(void* k_cache, void* v_cache, const float* k, const float* v,
                               int seq_len, int n_kv_heads, int head_dim, int start_pos,
                               int max_seq, void* stream);

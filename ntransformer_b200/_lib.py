@@ -26,6 +26,7 @@ SIGNATURES = {
     "nt_b200_add_bias": (None, [_vp, _vp, _i, _vp]),
     "nt_b200_attention_decode": (None, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _vp]),
     "nt_b200_attention_prefill": (None, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _vp]),
+    "nt_b200_attention_prefill_form": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i]),
     "nt_b200_copy_to_kv_cache": (None, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "nt_b200_add": (None, [_vp, _vp, _vp, _i, _vp]),
     "nt_b200_add_inplace": (None, [_vp, _vp, _i, _vp]),

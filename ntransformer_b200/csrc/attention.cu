@@ -578,11 +578,17 @@ void attention_decode_rope_dyn(float* out, const float* q, const float* k, const
                      static_cast<int8_t*>(xq_out), s);
 }
 
+// prompt-sized chunks: tiled tensor-core kernels
+int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq) {
+    if (!attention_prefill_mma_supported(seq_len, n_heads, n_kv, hd)) return PREFILL_QUERIES;
+    return attention_prefill_tc_takes(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq) ? PREFILL_TC : PREFILL_MMA;
+}
 void attention_prefill(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads,
                        int n_kv, int hd, int max_seq, float scale, cudaStream_t s) {
     if (seq_len <= 0 || n_heads <= 0) return;
-    if (attention_prefill_mma_supported(seq_len, n_heads, n_kv, hd)) {       // prompt-sized chunks: tiled tensor-core kernels
-        if (attention_prefill_tc(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, scale, s)) return;
+    const int form = attention_prefill_form(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq);
+    if (form != PREFILL_QUERIES) {
+        if (form == PREFILL_TC && attention_prefill_tc(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, scale, s)) return;
         attention_prefill_mma(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq, scale, s);
         return;
     }

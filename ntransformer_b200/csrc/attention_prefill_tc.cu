@@ -313,10 +313,15 @@ void launch_tc(const CUtensorMap& map_k, const CUtensorMap& map_v, const TcAttn&
 
 }  // namespace
 
-// false: nothing launched (pointers off 16 bytes; other widths)
+// Whether this form takes a call: widths, pointers on 16 bytes, and positions inside the cache (its maps have a row for every key; the form on mma.sync stays inside
+// a cache of max_seq rows whatever the positions)
+bool attention_prefill_tc_takes(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq) {
+    return seq_len >= 1 && (hd == 64 || hd == 128) && n_kv >= 1 && n_heads % n_kv == 0 && n_heads <= 65535 && start_pos >= 0 && (long long)start_pos + seq_len <= max_seq &&
+           ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0;
+}
+
+// A call that attention_prefill_tc_takes; false: nothing launched
 bool attention_prefill_tc(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, float scale, cudaStream_t s) {
-    if (seq_len < 1 || (hd != 64 && hd != 128) || n_kv < 1 || n_heads % n_kv || n_heads > 65535 ||
-        ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(Q) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15)) return false;
     // the maps end with the last key: rows of the cache behind it are zeros, whatever they hold
     CUtensorMap map_k, map_v;
     const uint64_t keys = (uint64_t)start_pos + seq_len, row = (uint64_t)n_kv * hd;

@@ -115,9 +115,13 @@ void attention_decode(float* out, const float* q, const void* kc, const void* vc
                       int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
 void attention_prefill(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos,
                        int n_heads, int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
-// attention_prefill_tc.cu: 128 x 128 tiles on tcgen05 (heads 64 and 128 wide, pointers on 16 bytes); false: nothing launched
+// the form that attention_prefill takes: a query at a time, mma.sync, tcgen05
+enum : int { PREFILL_QUERIES = 0, PREFILL_MMA = 1, PREFILL_TC = 2 };
+int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq);
+// attention_prefill_tc.cu: 128 x 128 tiles on tcgen05 (heads 64 and 128 wide, pointers on 16 bytes, positions inside the cache); false: nothing launched
+bool attention_prefill_tc_takes(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq);
 bool attention_prefill_tc(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, float scale, cudaStream_t s);
-// attention_prefill_mma.cu: 64-query x 64-key tiles on mma.sync (attention_prefill: seq_len >= 16, hd 64/128, pointers off 16 bytes; windows; BF16 caches)
+// attention_prefill_mma.cu: 64-query x 64-key tiles on mma.sync (attention_prefill: seq_len >= 16, hd 64/128, what the form above does not take; windows; BF16 caches)
 bool attention_prefill_mma_supported(int seq_len, int n_heads, int n_kv, int hd);
 void attention_prefill_mma(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads,
                            int n_kv, int hd, int max_seq, float scale, cudaStream_t s);

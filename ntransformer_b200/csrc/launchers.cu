@@ -109,6 +109,9 @@ void nt_b200_attention_decode(float* o, const float* q, const void* kc, const vo
 void nt_b200_attention_prefill(float* o, const float* Q, const void* kc, const void* vc, int sl, int sp, int nh, int nkv, int hd, int ms, float sc, void* s) {
     C::launch_attention_prefill(o, Q, kc, vc, sl, sp, nh, nkv, hd, ms, sc, s);
 }
+int nt_b200_attention_prefill_form(const float* o, const float* Q, const void* kc, const void* vc, int sl, int sp, int nh, int nkv, int hd, int ms) {
+    return nt::b200::attention_prefill_form(o, Q, kc, vc, sl, sp, nh, nkv, hd, ms);
+}
 void nt_b200_copy_to_kv_cache(void* kc, void* vc, const float* k, const float* v, int sl, int nkv, int hd, int sp, int ms, void* s) {
     C::launch_copy_to_kv_cache(kc, vc, k, v, sl, nkv, hd, sp, ms, s);
 }

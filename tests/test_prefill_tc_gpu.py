@@ -85,3 +85,15 @@ def test_a_scale_of_any_sign(dim, scale, tokens, start):
     # in the exponent: 2 * dim / 16 additions, each cut by 2/3 of 2^-24 of a score, and halves' pairs, 2^-22 of it; weights as above
     most = abs(scale) * float((q.norm(dim=2).max() * kc[: start + tokens].float().norm(dim=2).max()).item())
     assert torch.isfinite(got).all() and rel(got, want) <= 5e-6 + (dim / 8 * 2 / 3 * 2.0**-24 + 2.0**-22) * most
+
+
+@pytest.mark.parametrize("rows", [1, 250, 299])
+def test_positions_behind_the_cache_stay_inside_it(rows):
+    """Such keys are the cache's last row, as in the form on mma.sync; what lies behind the cache is not read."""
+    q, kc, vc = inputs(8, 2, 128, 200, 100)
+    kc[rows:], vc[rows:] = float("nan"), float("nan")              # (the allocation goes on)
+    inside = torch.arange(300, device="cuda").clamp(max=rows - 1)
+    out = torch.empty_like(q)
+    K.launch_attention_prefill(out, q, kc, vc, 200, 100, 8, 2, 128, rows, 128 ** -0.5)
+    torch.cuda.synchronize()
+    assert rel(out, exact(q, kc[inside], vc[inside], 100, 128 ** -0.5)) <= 2e-5      # the form on mma.sync: queries and weights as pairs of halves without a power of two

@@ -47,10 +47,53 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { u
 struct TcAttn {
     float* out;
     const float* Q;
+    const __half *kc, *vc;
     int seq_len, start_pos, n_heads, n_kv, pairs_of_queries;      // pairs_of_queries: a key head has an odd number of heads
     float scale;
     unsigned* status;
 };
+
+// A row by itself, HC of its channels, by a warp: keys 0 .. pos and no others, 32 at a time, a key to a lane and then HC / 32 channels to each.  For a row whose sums the
+// products left infinite or NaN: the weight of a key that the row does not see is zero, and zero times an infinite or NaN value, of a later token in the row's last
+// steps, is NaN.  Values that the row does see reach it here as well.
+template <int HD, int HC>
+__device__ __noinline__ void row_alone(const TcAttn& p, int row, int head, int kvh, int channel, int lane) {
+    constexpr int C = HC / 32;
+    const size_t pitch = (size_t)p.n_kv * HD, at = ((size_t)row * p.n_heads + head) * HD;
+    const int pos = p.start_pos + row;
+    const __half* k = p.kc + (size_t)kvh * HD;
+    const __half* v = p.vc + (size_t)kvh * HD + channel + lane * C;
+    float m = -INFINITY, l = 0.f, o[C] = {};
+#pragma unroll 1
+    for (int k0 = 0; k0 <= pos; k0 += 32) {
+        float s = 0.f;
+        const __half* kr = k + (size_t)min(k0 + lane, pos) * pitch;
+#pragma unroll 4
+        for (int d = 0; d < HD; d += 2) {
+            const float2 x = __half22float2(*reinterpret_cast<const __half2*>(kr + d)), q = __ldg(reinterpret_cast<const float2*>(p.Q + at + d));
+            s = fmaf(q.x, x.x, fmaf(q.y, x.y, s));
+        }
+        s = k0 + lane <= pos ? s * p.scale * 1.4426950408889634f : -INFINITY;
+        float mx = fmaxf(m, s);
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, i));
+        const float base = mx == -INFINITY ? 0.f : mx, alpha = exp2f(m - base), w = exp2f(s - base);
+        m = mx;
+        float sum = w;
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, i);
+        l = fmaf(l, alpha, sum);
+#pragma unroll
+        for (int i = 0; i < C; i++) o[i] *= alpha;
+        for (int j = 0; j < min(32, pos + 1 - k0); j++) {
+            const float wj = __shfl_sync(0xFFFFFFFFu, w, j);
+#pragma unroll
+            for (int i = 0; i < C; i++) o[i] = fmaf(wj, __half2float(v[(size_t)(k0 + j) * pitch + i]), o[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < C; i++) p.out[at + channel + lane * C + i] = o[i] / l;
+}
 
 template <int HD>
 __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ TcAttn p) {
@@ -201,7 +244,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
         if (word_set(dead)) report(p.status);
         else {
             // 16 rows at a time over the tile's queries (no product reads them any more), then whole lines to memory
-            const float inv = 1.0f / (l + row_word[half ^ 1][t * TQ + r]);
+            l += row_word[half ^ 1][t * TQ + r];
+            const float inv = 1.0f / l;
+            uint64_t odd = 0;                                     // NaN where a sum is infinite or NaN
+#pragma unroll
+            for (int i = 0; i < HC / 2; i++) odd = fma2(o[i], 0, odd);
+            float odd0, odd1;
+            unpack2(odd, odd0, odd1);
+            unsigned again = __ballot_sync(0xFFFFFFFFu, row < p.seq_len && !(odd0 + odd1 == 0.f) && l < INFINITY);      // (a row that sees a NaN or infinite score is NaN)
             constexpr int PITCH = HC + 4, LR = HC / 4, RI = 32 / LR;
             float* stage = reinterpret_cast<float*>(mine) + (warp & 7) * 16 * PITCH;
 #pragma unroll
@@ -222,6 +272,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 }
                 __syncwarp();
             }
+            for (; again; again &= again - 1) row_alone<HD, HC>(p, q0 + quarter * 32 + __ffs(again) - 1, head, kvh, half * HC, lane);
         }
     } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
@@ -326,7 +377,7 @@ bool attention_prefill_tc(float* out, const float* Q, const void* kc, const void
     CUtensorMap map_k, map_v;
     const uint64_t keys = (uint64_t)start_pos + seq_len, row = (uint64_t)n_kv * hd;
     if (!tc_map_f16(&map_k, kc, keys, row, TK) || !tc_map_f16(&map_v, vc, keys, row, TK)) return false;
-    TcAttn p{out, Q, seq_len, start_pos, n_heads, n_kv, (n_heads / n_kv) % 2, scale, wait_status()};
+    TcAttn p{out, Q, static_cast<const __half*>(kc), static_cast<const __half*>(vc), seq_len, start_pos, n_heads, n_kv, (n_heads / n_kv) % 2, scale, wait_status()};
     if (hd == 128) launch_tc<128>(map_k, map_v, p, s);
     else launch_tc<64>(map_k, map_v, p, s);
     return true;

@@ -97,3 +97,20 @@ def test_positions_behind_the_cache_stay_inside_it(rows):
     K.launch_attention_prefill(out, q, kc, vc, 200, 100, 8, 2, 128, rows, 128 ** -0.5)
     torch.cuda.synchronize()
     assert rel(out, exact(q, kc[inside], vc[inside], 100, 128 ** -0.5)) <= 2e-5      # the form on mma.sync: queries and weights as pairs of halves without a power of two
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("heads,kv,tokens,start", [(152, 76, 200, 70), (153, 51, 300, 0), (152, 76, 16, 1000)])
+def test_an_infinite_or_nan_value_reaches_the_queries_that_see_it_and_no_others(dim, heads, kv, tokens, start):
+    q, kc, vc = inputs(heads, kv, dim, tokens, start)
+    want = exact(q, kc, vc, start, dim ** -0.5)
+    last = start + tokens - 1
+    for head, key, channel, value in ((0, last - 9, 3, "inf"), (1, start + 7, dim - 1, "nan"), (2, last, 0, "-inf")):
+        vc[key, head, channel] = float(value)
+    got = attend(q, kc, vc, start, dim ** -0.5)
+    bad = torch.zeros(tokens, heads, dim, dtype=torch.bool, device="cuda")
+    for head, key, channel in ((0, last - 9, 3), (1, start + 7, dim - 1), (2, last, 0)):
+        bad[key - start:, head * (heads // kv):(head + 1) * (heads // kv), channel] = True
+    assert torch.equal(~torch.isfinite(got), bad)
+    keep = torch.where(bad, torch.zeros_like(got), got)
+    assert rel(keep, torch.where(bad, torch.zeros_like(want), want)) <= 5e-6

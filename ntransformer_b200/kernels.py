@@ -40,6 +40,13 @@ def _launch(name, args):
     getattr(lib(), "nt_b200_" + name)(*(_p(a) if t is C.c_void_p else a for a, t in zip(args[:-1], types)), _s(args[-1]))
 
 
+class _Through:
+    """The launches through ctypes: for an interpreter that the extension was not built for."""
+
+    def __getattr__(self, name):
+        return lambda *args: _launch(name, args)
+
+
 _entries = None       # csrc/fast_call.cpp: takes tensors, raw pointers (ints) or None, and a stream (None: the current one)
 
 
@@ -48,8 +55,9 @@ def _fast():
     if _entries is None:
         try:
             from . import _fast as m
-        except ImportError as e:
-            raise RuntimeError("ntransformer_b200/_fast.so is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`") from e
+        except ImportError:
+            _entries = _Through()
+            return _entries
         m.bind(torch.Tensor, torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice, torch.cuda.init, _launch,
                {n: C.cast(getattr(lib(), "nt_b200_" + n), C.c_void_p).value for n in m.ENTRIES})
         _entries = m

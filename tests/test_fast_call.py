@@ -1,10 +1,13 @@
 """The launcher boundary's extension (csrc/fast_call.cpp) hands every entry the arguments that ctypes hands it, and leaves to ctypes what it does not take."""
 import ctypes as C
+import sys
+import sysconfig
 
 import numpy as np
 import pytest
 import torch
 
+import ntransformer_b200
 from ntransformer_b200 import _fast, kernels
 from ntransformer_b200._lib import SIGNATURES, lib
 
@@ -75,6 +78,26 @@ def test_the_other_route_refuses_as_before():
     with pytest.raises(C.ArgumentError):
         kernels.launch_add(None, None, None, 4.5, 0)
     assert kernels._fast() is _fast and lib() is not None
+
+
+def test_without_the_extension_launches_go_through_ctypes(monkeypatch):
+    got = []
+
+    class Library:
+        def __getattr__(self, name):
+            return lambda *a: got.append((name, a))
+
+    monkeypatch.delattr(ntransformer_b200, "_fast")
+    monkeypatch.setitem(sys.modules, "ntransformer_b200._fast", None)         # an ImportError
+    monkeypatch.setattr(kernels, "_entries", None)
+    monkeypatch.setattr(kernels, "lib", Library)
+    kernels.launch_rope(8, None, 16, 1, 2, 3, 4, 64, 1e4, 1.0, True, stream=5)
+    kernels.launch_add(8, 16, 24, 7, Stream)
+    assert got == [("nt_b200_rope", (8, None, 16, 1, 2, 3, 4, 64, 1e4, 1.0, 1, 5)), ("nt_b200_add", (8, 16, 24, 7, Stream.cuda_stream))]
+
+
+def test_the_extension_is_of_this_interpreter_alone():
+    assert _fast.__file__.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
 
 
 @pytest.mark.gpu

@@ -578,10 +578,23 @@ void attention_decode_rope_dyn(float* out, const float* q, const float* k, const
                      static_cast<int8_t*>(xq_out), s);
 }
 
+// Whether a prompt is better served by the tiles of 128 queries x 128 keys on tcgen05 (one CTA to an SM and two of these tiles, which walk all keys in series, however few
+// of their rows are live) than by those of 64 x 64 on mma.sync.  Beyond a wave of the smaller tiles always (500 tokens, 24 heads of 128: 21.5 us, 31.8 on mma.sync; 1000
+// behind 1023, 32 heads: 57, 174).  Within one, each takes a start and its steps over the keys of the last query, heads of 128 (64): 8.4 us and 2.82 (5.8 and 2.1) for
+// 128 keys here, 5.6 us and 1.9 (4.5 and 1.22) for 64 keys there, and 0.7 (0.3) more here each time the queries' tiles double.  Measured (here, there): 17 tokens
+// behind 0, 300, 1000: 10.9, 16.8, 31.0; 8.4, 14.5, 36.1 (heads of 64: 7.8, 12.3, 22.9; 6.3, 10.5, 24.7); 200 behind 0, 300: 14.6, 21.9; 12.5, 22.7.  Of 720 pairs (17 to 1000 tokens, 4 to 64 heads,
+// 0 to 4000 keys before, both widths) none takes a form that is more than 3 % slower, but 12 of heads of 64, by up to 6 %, on mma.sync.
+bool attention_prefill_tc_pays(int seq_len, int start_pos, int n_heads, int hd) {
+    if ((long long)((seq_len + 63) / 64) * n_heads > 148) return true;
+    const int keys = start_pos + seq_len;
+    const float s64 = (float)((keys + 63) / 64), s128 = (float)((keys + 127) / 128), doubled = log2f((float)((seq_len + 127) / 128));
+    return hd == 128 ? 1.9f * s64 - 2.82f * s128 - 0.7f * doubled > 2.75f : 1.22f * s64 - 2.1f * s128 - 0.3f * doubled > 1.25f;
+}
 // prompt-sized chunks: tiled tensor-core kernels
 int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq) {
     if (!attention_prefill_mma_supported(seq_len, n_heads, n_kv, hd)) return PREFILL_QUERIES;
-    return attention_prefill_tc_takes(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq) ? PREFILL_TC : PREFILL_MMA;
+    return attention_prefill_tc_takes(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq) && attention_prefill_tc_pays(seq_len, start_pos, n_heads, hd)
+               ? PREFILL_TC : PREFILL_MMA;
 }
 void attention_prefill(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads,
                        int n_kv, int hd, int max_seq, float scale, cudaStream_t s) {

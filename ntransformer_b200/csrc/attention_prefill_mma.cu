@@ -8,13 +8,14 @@
 // registers (flash-attention-2 data flow).  F32 operands are split into two F16 terms (q = hi + lo, p = hi + lo) so
 // the result keeps ~22 mantissa bits and stays within the 2e-5 tolerance of the oracle.
 //
-// Prompts over an F16 cache take attention_prefill_tc.cu where their pointers start on 16 bytes; this form is for the others.
+// Prompts over an F16 cache take attention_prefill_tc.cu where that pays (attention.cu attention_prefill_tc_pays) and it takes them; this form is for the others.
 // The same kernel serves windowed attention (csrc/attention_window.cu's rule: key j visible from position p iff j <= p and
 // (p - j < window or j < keep)), optionally with soft-capped scores cap * tanh(s / cap) and a BF16 cache (BF: both MMAs take
 // BF16 operands, the splits are BF16 pairs): a query block then walks only the key tiles of the kept prefix and of its window.
 #include "kernels_internal.h"
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
+#include <algorithm>
 
 namespace nt { namespace b200 {
 
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(128, 2) prefill_mma_kernel(float* __restrict__
         constexpr int CH = HD / 8, CHV = HDV / 8;                     // 16-byte chunks per row
         for (int c = threadIdx.x; c < BKV * CH; c += 128) {
             const int row = c / CH, ch = c % CH;
-            const int key = min(tile_of(j) * BKV + row, max_seq - 1); // rows past the cache are masked by causality anyway
+            const int key = min(tile_of(j) * BKV + row, max_seq - 1); // rows past the last are masked by causality anyway
             cp_async16(sK + ((size_t)st * BKV + row) * LD + ch * 8, kc + ((size_t)key * n_k + kvh) * HD + ch * 8);
         }
         for (int c = threadIdx.x; c < BKV * CHV; c += 128) {
@@ -247,6 +248,9 @@ void launch(float* out, const float* Q, const __half* kc, const __half* vc, int 
     const int smem = 2 * BKV * (HD + PAD + HDV + PAD) * (int)sizeof(__half);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(prefill_mma_kernel<HD, HDV, BF>, (int)(smem), configured);
+    // The cache ends with the last query for it: what lies behind may be infinite or NaN, and a masked row's weight of zero times that would be NaN.
+    max_seq = std::min(max_seq, std::max(1, start_pos + seq_len));
+    // (not programmatic: CTAs that wait for the launch before would gather two to an SM where it is done; 64 heads, 128 tokens behind 4000: 131 us, 206)
     prefill_mma_kernel<HD, HDV, BF><<<dim3((seq_len + BQ - 1) / BQ, n_heads * maps), 128, smem, s>>>(out, Q, kc, vc, seq_len, start_pos, n_heads * maps, n_kv,
                                                                                                     max_seq, scale, window, keep, softcap, maps, chunk, sink, joint_v, slopes);
     NT_LAUNCH_CHECK();

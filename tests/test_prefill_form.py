@@ -23,3 +23,25 @@ def test_pointers_and_widths():
     assert form(1000, 0, dim=64) == TC and form(1000, 0, dim=96) == QUERIES and form(15, 0) == QUERIES and form(1000, 0, heads=30) == QUERIES
     for name in ("out", "q", "k", "v"):
         assert form(1000, 0, **{name: 0x1008}) == MMA
+
+
+# measured where the two forms take turns (us on tcgen05, on mma.sync): neither side of the line by more than a few per cent
+@pytest.mark.parametrize("dim,heads,kv,start,tokens,want", [
+    (128, 32, 8, 0, 17, MMA),          # 10.9, 8.4
+    (128, 64, 8, 0, 26, MMA),          # 10.9, 8.2
+    (128, 4, 2, 0, 167, MMA),          # 13.5, 10.8
+    (128, 32, 8, 300, 17, MMA),        # 16.8, 14.5
+    (128, 32, 8, 300, 40, TC),         # 16.9, 18.6
+    (128, 32, 8, 300, 100, MMA),       # 21.1, 18.8
+    (128, 32, 8, 0, 256, MMA),         # 15.5, 14.0
+    (128, 32, 8, 0, 500, TC),          # 21.3, 32.2: more than a wave there
+    (128, 4, 4, 1000, 17, TC),         # 30.1, 35.6
+    (128, 4, 4, 0, 1000, TC),          # 32.4, 35.7
+    (64, 8, 2, 24, 231, MMA),          # 12.7, 10.3
+    (64, 16, 4, 0, 115, MMA),          # 8.0, 7.2
+    (64, 32, 8, 1000, 17, TC),         # 22.9, 24.7
+    (64, 16, 16, 300, 500, MMA),       # 22.9, 20.8
+    (64, 64, 8, 0, 200, TC),           # 10.6, 12.5
+])
+def test_the_faster_form(dim, heads, kv, start, tokens, want):
+    assert form(tokens, start, heads, kv, dim) == want

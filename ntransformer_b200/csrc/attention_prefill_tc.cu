@@ -57,12 +57,13 @@ struct TcAttn {
 // products left infinite or NaN: the weight of a key that the row does not see is zero, and zero times an infinite or NaN value, of a later token in the row's last
 // steps, is NaN.  Values that the row does see reach it here as well.
 template <int HD, int HC>
-__device__ __noinline__ void row_alone(const TcAttn& p, int row, int head, int kvh, int channel, int lane) {
+__device__ __noinline__ void row_alone(const TcAttn& p, int row, int head, int channel, int lane) {
     constexpr int C = HC / 32;
     const size_t pitch = (size_t)p.n_kv * HD, at = ((size_t)row * p.n_heads + head) * HD;
     const int pos = p.start_pos + row;
-    const __half* k = p.kc + (size_t)kvh * HD;
-    const __half* v = p.vc + (size_t)kvh * HD + channel + lane * C;
+    const size_t kvh = (size_t)(head / (p.n_heads / p.n_kv));
+    const __half* k = p.kc + kvh * HD;
+    const __half* v = p.vc + kvh * HD + channel + lane * C;
     float m = -INFINITY, l = 0.f, o[C] = {};
 #pragma unroll 1
     for (int k0 = 0; k0 <= pos; k0 += 32) {
@@ -151,7 +152,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 const uint32_t e = __float_as_uint(amax) >> 23 & 255u;       // not finite, or zero: as it is
                 const uint32_t up = e == 255u || e == 0u ? 127u : min(227u, max(27u, 264u - e));       // to 2^10 .. 2^11
                 const float g = copysignf(__uint_as_float(up << 23), p.scale);        // the scale's sign goes with the queries: the greatest score stays the greatest
-                if (c == 0) row_word[0][t * TQ + rr] = fabsf(p.scale) * 1.4426950408889634f * __uint_as_float((254u - up) << 23);
+                // never zero: masked scores are -inf times it, and others as small as that have equal weights
+                const float fq = fabsf(p.scale) * 1.4426950408889634f * __uint_as_float((254u - up) << 23);
+                if (c == 0) row_word[0][t * TQ + rr] = fq == 0.f ? 1.1754944e-38f : fq;
                 uint2 h, l;
                 split_pair(x.x * g, x.y * g, 0, h.x, l.x);
                 split_pair(x.z * g, x.w * g, 0, h.y, l.y);
@@ -204,14 +207,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 uint32_t v[16], w[16];
                 tmem_ld16(ts + half * HK + 16 * c, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 16; i++) v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), f, -base));
-                if (!whole)                                       // behind the multiplication: f may be zero
+                if (!whole)
 #pragma unroll
                     for (int i = 0; i < 16; i++) v[i] = 16 * c + i <= seen ? v[i] : 0xFF800000u;
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
-                    const float a = exp2f(__uint_as_float(v[2 * i])), b = exp2f(__uint_as_float(v[2 * i + 1]));
+                    const float a = exp2f(fmaf(__uint_as_float(v[2 * i]), f, -base)), b = exp2f(fmaf(__uint_as_float(v[2 * i + 1]), f, -base));
                     sum += a + b;
                     split_pair(a, b, 0, w[i], w[8 + i]);
                 }
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
                 }
                 __syncwarp();
             }
-            for (; again; again &= again - 1) row_alone<HD, HC>(p, q0 + quarter * 32 + __ffs(again) - 1, head, kvh, half * HC, lane);
+            for (; again; again &= again - 1) row_alone<HD, HC>(p, q0 + quarter * 32 + __ffs(again) - 1, head, half * HC, lane);
         }
     } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");

@@ -791,7 +791,6 @@ bool Model::ensure_block_scratch() {
     if (block_scratch_) return true;
     void* p = nullptr;
     if (cudaMalloc(&p, block_scratch_bytes()) != cudaSuccess) { cudaGetLastError(); return false; }
-    zero_block_scratch(p, stream_);
     block_scratch_ = p;
     return true;
 }

@@ -48,7 +48,7 @@ struct BlkParams {
     int units;                 // tiles * super-blocks
     const float* scale;        // of a token's products
     float* part;               // two tiles to a CTA
-    unsigned* count;           // one to a CTA
+    unsigned* count;           // one to a CTA: shares of its last tile that have arrived; zeros at first
     unsigned* status;          // wait_status.cuh
 };
 
@@ -547,16 +547,17 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
 // One block to a token: x (MODE 1: RMSNorm(x) * w, rmsnorm.cu:17-70's math; 2: silu(x) * w, gemm.cu:713-725's expression; 3: hi x and lo w of
 // a plain split, which may be the one written to) as F16 hi + lo, the sums of 32 of them
 // (a 32nd part, so that they stay within F16) as hi + lo, and the factor that undoes the token's power of two.  That power takes the largest to 2^13 .. 2^14, where the
-// low halves keep their bits.
+// low halves keep their bits.  Block 0 also clears the product's counts: a launch whose wait ran out leaves some behind.
 enum : int { TOK_PLAIN = 0, TOK_NORM = 1, TOK_SILU = 2, TOK_SPLIT = 3 };
 template <int MODE>
-__global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* lo, __half* __restrict__ sums, float* __restrict__ scale, const float* xin, const float* w,
-                                                           float eps, int K) {
+__global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* lo, __half* __restrict__ sums, float* __restrict__ scale, unsigned* __restrict__ count, int counts,
+                                                           const float* xin, const float* w, float eps, int K) {
     constexpr int KEEP = 7;                                        // chunks of 2048 held in registers: rows to 14336
     __shared__ float red[2][16];
     const int tid = threadIdx.x;
     pdl_wait();
     pdl_launch_dependents();               // after the wait: the product reads weights before its own, and whatever wrote them came before this launch
+    if (blockIdx.x == 0) for (int i = tid; i < counts; i += 512) count[i] = 0;
     const size_t at = (size_t)blockIdx.x * K;
     const float* x = xin + at;
     const float* y = MODE == TOK_SILU ? w + at : w;
@@ -652,14 +653,9 @@ int sm_count() {
 
 bool gemm_blocks_supported(const GemvMat* mats, int n_mat, int K) { return gemv_kq_any_pitch(mats, n_mat, K); }
 
-// [hi rows, lo rows (gemm_f16_tc_workspace_bytes)][sums][scales], rows padded to 128
-size_t block_tokens_bytes(int T, int K) { return gemm_f16_tc_workspace_bytes(T, K) + padded(T) * ((size_t)K / 8 + sizeof(float)); }
-size_t block_scratch_bytes() { const size_t n = (size_t)sm_count(); return n * (2 * 128 * NT_MAX * sizeof(float) + sizeof(unsigned)); }
-
-void zero_block_scratch(void* scratch, cudaStream_t s) {      // its counts
-    const size_t n = (size_t)sm_count() * sizeof(unsigned);
-    NT_CUDA_CHECK(cudaMemsetAsync(static_cast<uint8_t*>(scratch) + block_scratch_bytes() - n, 0, n, s));
-}
+// [hi rows, lo rows (gemm_f16_tc_workspace_bytes)][sums][scales][counts], rows padded to 128
+size_t block_tokens_bytes(int T, int K) { return gemm_f16_tc_workspace_bytes(T, K) + padded(T) * ((size_t)K / 8 + sizeof(float)) + (size_t)sm_count() * sizeof(unsigned); }
+size_t block_scratch_bytes() { return (size_t)sm_count() * 2 * 128 * NT_MAX * sizeof(float); }
 
 BlockTokens block_tokens(void* workspace, int T, int K) {
     BlockTokens t;
@@ -667,6 +663,7 @@ BlockTokens block_tokens(void* workspace, int T, int K) {
     t.split = p;
     t.sums = p + gemm_f16_tc_workspace_bytes(T, K);
     t.scale = reinterpret_cast<float*>(p + gemm_f16_tc_workspace_bytes(T, K) + padded(T) * ((size_t)K / 8));
+    t.count = reinterpret_cast<unsigned*>(t.scale + padded(T));
     return t;
 }
 
@@ -674,14 +671,15 @@ BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, f
     const BlockTokens t = block_tokens(workspace, T, K);
     __half* hi = static_cast<__half*>(t.split);
     __half* lo = hi + padded(T) * (size_t)K;
-    launch_k_pdl(true, norm_w ? split_tokens_kernel<TOK_NORM> : split_tokens_kernel<TOK_PLAIN>, dim3(T), dim3(512), 0, s, hi, lo, static_cast<__half*>(t.sums), t.scale, x, norm_w, eps, K);
+    launch_k_pdl(true, norm_w ? split_tokens_kernel<TOK_NORM> : split_tokens_kernel<TOK_PLAIN>, dim3(T), dim3(512), 0, s, hi, lo, static_cast<__half*>(t.sums), t.scale, t.count, sm_count(), x, norm_w, eps, K);
     count_launch();
     return t;
 }
 BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, cudaStream_t s) {
     const BlockTokens t = block_tokens(workspace, T, K);
     __half* hi = static_cast<__half*>(t.split);
-    launch_k_pdl(true, split_tokens_kernel<TOK_SILU>, dim3(T), dim3(512), 0, s, hi, hi + padded(T) * (size_t)K, static_cast<__half*>(t.sums), t.scale, gate, up, 0.f, K);
+    launch_k_pdl(true, split_tokens_kernel<TOK_SILU>, dim3(T), dim3(512), 0, s, hi, hi + padded(T) * (size_t)K, static_cast<__half*>(t.sums), t.scale, t.count, sm_count(), gate,
+                 up, 0.f, K);
     count_launch();
     return t;
 }
@@ -689,8 +687,8 @@ BlockTokens resplit_tokens(void* workspace, const void* split, int T, int K, cud
     const BlockTokens t = block_tokens(workspace, T, K);
     __half* hi = static_cast<__half*>(t.split);
     const size_t lo = padded(T) * (size_t)K;
-    launch_k_pdl(true, split_tokens_kernel<TOK_SPLIT>, dim3(T), dim3(512), 0, s, hi, hi + lo, static_cast<__half*>(t.sums), t.scale, static_cast<const float*>(split),
-             reinterpret_cast<const float*>(static_cast<const __half*>(split) + lo), 0.f, K);
+    launch_k_pdl(true, split_tokens_kernel<TOK_SPLIT>, dim3(T), dim3(512), 0, s, hi, hi + lo, static_cast<__half*>(t.sums), t.scale, t.count, sm_count(),
+                 static_cast<const float*>(split), reinterpret_cast<const float*>(static_cast<const __half*>(split) + lo), 0.f, K);
     count_launch();
     return t;
 }
@@ -740,10 +738,8 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     // a run of super-blocks to a CTA; without a scratch whole tiles
     p.grain = scratch ? 1 : p.NB;
     const int grid = std::min(sms, p.units / p.grain);
-    if (scratch) {
-        p.part = static_cast<float*>(scratch);
-        p.count = reinterpret_cast<unsigned*>(p.part + (size_t)sms * 2 * 128 * NT_MAX);
-    }
+    p.part = static_cast<float*>(scratch);
+    p.count = x.count;
     BlkMaps maps;
     if (!tc_map_f16(&maps.x, x.split, 2 * (uint64_t)p.Mp, (uint64_t)K, (uint32_t)p.NT) || !tc_map_f16_rows32(&maps.sums, x.sums, (uint64_t)p.Mp, (uint64_t)K / 16, (uint32_t)p.NT))
         return false;
@@ -773,7 +769,6 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const fl
     void* mem = nullptr;
     if (cudaMallocAsync(&mem, tokens + block_scratch_bytes(), s) != cudaSuccess) { cudaGetLastError(); return false; }
     uint8_t* scratch = static_cast<uint8_t*>(mem) + tokens;
-    zero_block_scratch(scratch, s);
     const BlockTokens t = x ? split_tokens(mem, x, norm_w, eps, T, K, s) : resplit_tokens(mem, split, T, K, s);
     const bool ok = gemm_blocks(mats, n_mat, K, t, scratch, fine, T, add, s);
     NT_CUDA_CHECK(cudaFreeAsync(mem, s));

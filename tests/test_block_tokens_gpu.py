@@ -1,12 +1,16 @@
 """Tokens over GGUF blocks on the tensor cores (csrc/prefill_blocks.cu) through nt_b200_gemm_blocks: the dealing out of tiles, formats side by side, wide ranges of
 activations, and the precision of the form that takes a few tokens' place (csrc/gemv_rows.cu, 24-bit integers)."""
 import ctypes as C
+import dataclasses
 
+import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
 from ntransformer_b200._lib import lib  # noqa: E402
 from ntransformer_b200.dtypes import DType  # noqa: E402
+from ntransformer_b200.engine import Model  # noqa: E402
+from ntransformer_b200.model_spec import TINY  # noqa: E402
 from test_block_products_gpu import FORMATS, activations, arrays, matrix, rel, rows_product, stream  # noqa: E402
 
 pytestmark = [pytest.mark.gpu]
@@ -86,3 +90,16 @@ def test_a_few_tokens_are_no_further_from_64_bits_than_24_bit_integers(dt, cols,
     rows_product([old], [W], [rows], [dt], x)
     print("%s %d, %g of them x %g: %.2e here, %.2e integers" % (dt.name, cols, wild, by, rel(y, ref), rel(old, ref)))
     assert rel(y, ref) <= 1.02 * rel(old, ref)
+
+
+@pytest.mark.parametrize("mix", ["Q4_K_M", "Q8_0"])
+def test_prompts_of_other_lengths_before_leave_nothing_behind(mix):
+    """The counts of a product's shared tiles lie in the tokens' workspace, where other lengths have other numbers: each split clears them."""
+    cfg = dataclasses.replace(TINY, max_seq_len=1024)
+    toks = np.random.default_rng(4).integers(3, cfg.vocab_size, size=700).tolist()
+    m = Model.synthetic(cfg, mix, seed=6)
+    want = {}
+    for n in (130, 40, 11, 300, 33, 130, 20, 11, 700, 40, 300, 20, 33, 700):
+        got = m.forward(toks[:n], 0).copy()
+        assert np.array_equal(want.setdefault(n, got), got), n
+    m.close()

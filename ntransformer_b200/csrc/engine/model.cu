@@ -500,7 +500,7 @@ void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float
         gemv_xq(mats, n, K, xq_, ep, s);
         return;
     }
-    if (gemv_kq_any_pitch(mats, n, K)) {
+    if (gemv_kq_any_pitch(mats, n, K) && (reinterpret_cast<uintptr_t>(norm_w) & 15) == 0) {
         in.x = x; in.norm_w = norm_w; in.eps = cfg_.norm_eps;
         gemv_kq(mats, n, K, in, ep, s);
         return;
@@ -561,7 +561,10 @@ bool Model::chain_ok() const {
         GemvMat m; m.W = w.ptr; m.y = nullptr; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch;
         return w.cols == K && gemv_kq_any_pitch(&m, 1, K);
     };
+    auto wide = [](const float* w) { return (reinterpret_cast<uintptr_t>(w) & 15) == 0; };      // gains that the GEMVs' prologue and quantize_rows read 16 bytes at a time
+    if (!wide(out_norm_)) return false;
     for (const LayerWeights& L : layers_) {
+        if (!wide(L.attn_norm) || !wide(L.ffn_norm)) return false;
         GemvMat qkv[3];
         const Weight* ws[3] = {&L.wq, &L.wk, &L.wv};
         for (int i = 0; i < 3; i++) { qkv[i].W = ws[i]->ptr; qkv[i].out = ws[i]->rows; qkv[i].dtype = ws[i]->dtype; qkv[i].row_pitch = ws[i]->pitch; }

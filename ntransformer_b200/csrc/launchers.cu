@@ -137,7 +137,7 @@ int nt_b200_gemv_fused_f32(int n_mat, float* const* y, const void* const* W, con
     if (n_mat < 1 || n_mat > 3 || !x) return -1;
     nt::b200::GemvMat m[3];
     for (int i = 0; i < n_mat; i++) { m[i].W = W[i]; m[i].y = y[i]; m[i].out = out_features[i]; m[i].dtype = (DType)dtypes[i]; m[i].row_pitch = 0; }
-    if (!nt::b200::gemv_kq_supported(m, n_mat, in_features)) return -2;
+    if (!nt::b200::gemv_kq_supported(m, n_mat, in_features) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(norm_w)) & 15)) return -2;
     if (epilogue == 2 && (n_mat != 2 || out_features[0] != out_features[1])) return -3;
     nt::b200::GemvInput in; in.x = x; in.norm_w = norm_w; in.eps = eps;
     nt::b200::gemv_kq(m, n_mat, in_features, in, (nt::b200::GemvEpilogue)epilogue, static_cast<cudaStream_t>(stream));
@@ -156,7 +156,7 @@ int nt_b200_gemv_rows(int n_mat, float* const* y, const void* const* W, const in
     if (n_mat < 1 || n_mat > 3 || !x || tokens < 1) return -1;
     nt::b200::GemvMat m[3];
     for (int i = 0; i < n_mat; i++) { m[i].W = W[i]; m[i].y = y[i]; m[i].out = out_features[i]; m[i].dtype = (DType)dtypes[i]; m[i].row_pitch = 0; }
-    if (!nt::b200::gemv_kq_any_pitch(m, n_mat, in_features) || (reinterpret_cast<uintptr_t>(x) & 15)) return -2;
+    if (!nt::b200::gemv_kq_any_pitch(m, n_mat, in_features) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(norm_w)) & 15)) return -2;
     if (epilogue == 2 && (n_mat != 2 || out_features[0] != out_features[1] || dtypes[0] != dtypes[1])) return -3;
     nt::b200::quantize_rows(scratch, x, norm_w, eps, tokens, in_features, static_cast<cudaStream_t>(stream));
     nt::b200::gemv_rows(m, n_mat, in_features, scratch, tokens, (nt::b200::GemvEpilogue)epilogue, static_cast<cudaStream_t>(stream));

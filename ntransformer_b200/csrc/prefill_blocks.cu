@@ -548,7 +548,8 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
 // a plain split, which may be the one written to) as F16 hi + lo, the sums of 32 of them
 // (a 32nd part, so that they stay within F16) as hi + lo, and the factor that undoes the token's power of two.  That power takes the largest to 2^13 .. 2^14, where the
 // low halves keep their bits.  Block 0 also clears the product's counts: a launch whose wait ran out leaves some behind.
-enum : int { TOK_PLAIN = 0, TOK_NORM = 1, TOK_SILU = 2, TOK_SPLIT = 3 };
+// TOK_NORM_ANY: TOK_NORM whose gains do not lie on 16 bytes.
+enum : int { TOK_PLAIN = 0, TOK_NORM = 1, TOK_SILU = 2, TOK_SPLIT = 3, TOK_NORM_ANY = 4 };
 template <int MODE>
 __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* lo, __half* __restrict__ sums, float* __restrict__ scale, unsigned* __restrict__ count, int counts,
                                                            const float* xin, const float* w, float eps, int K) {
@@ -568,8 +569,8 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
             return make_float4(a0.x + b0.x, a0.y + b0.y, a1.x + b1.x, a1.y + b1.y);
         }
         float4 a = *reinterpret_cast<const float4*>(x + i);
-        if (MODE == TOK_NORM) {
-            const float4 g = *reinterpret_cast<const float4*>(y + i);
+        if (MODE == TOK_NORM || MODE == TOK_NORM_ANY) {
+            const float4 g = MODE == TOK_NORM ? *reinterpret_cast<const float4*>(y + i) : make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
             ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
             a.x *= g.x; a.y *= g.y; a.z *= g.z; a.w *= g.w;
         }
@@ -593,7 +594,7 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
     float tot = 0.f, f = 1.f;
 #pragma unroll
     for (int i = 0; i < 16; i++) { tot += red[0][i]; amax = fmaxf(amax, red[1][i]); }
-    if (MODE == TOK_NORM) f = rsqrtf(tot / K + eps);
+    if (MODE == TOK_NORM || MODE == TOK_NORM_ANY) f = rsqrtf(tot / K + eps);
     const uint32_t e = __float_as_uint(amax * f) >> 23 & 255u;     // not finite, or zero: as it is
     const uint32_t up = e == 255u || e == 0u ? 127u : min(227u, max(27u, 267u - e));
     f *= __uint_as_float(up << 23);
@@ -671,7 +672,8 @@ BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, f
     const BlockTokens t = block_tokens(workspace, T, K);
     __half* hi = static_cast<__half*>(t.split);
     __half* lo = hi + padded(T) * (size_t)K;
-    launch_k_pdl(true, norm_w ? split_tokens_kernel<TOK_NORM> : split_tokens_kernel<TOK_PLAIN>, dim3(T), dim3(512), 0, s, hi, lo, static_cast<__half*>(t.sums), t.scale, t.count, sm_count(), x, norm_w, eps, K);
+    const bool wide = (reinterpret_cast<uintptr_t>(norm_w) & 15) == 0;
+    launch_k_pdl(true, !norm_w ? split_tokens_kernel<TOK_PLAIN> : wide ? split_tokens_kernel<TOK_NORM> : split_tokens_kernel<TOK_NORM_ANY>, dim3(T), dim3(512), 0, s, hi, lo, static_cast<__half*>(t.sums), t.scale, t.count, sm_count(), x, norm_w, eps, K);
     count_launch();
     return t;
 }
@@ -764,7 +766,7 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
 
 // The same over F32 tokens, or (x null) over tokens that split_activations laid out; what it needs beside them lies in memory of this call's
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const float* norm_w, float eps, const void* split, bool fine, int T, bool add, cudaStream_t s) {
-    if (T <= 0 || !gemm_blocks_supported(mats, n_mat, K) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(norm_w) & 15)) return false;
+    if (T <= 0 || !gemm_blocks_supported(mats, n_mat, K) || (reinterpret_cast<uintptr_t>(x) & 15)) return false;
     const size_t tokens = (block_tokens_bytes(T, K) + 255) / 256 * 256;
     void* mem = nullptr;
     if (cudaMallocAsync(&mem, tokens + block_scratch_bytes(), s) != cudaSuccess) { cudaGetLastError(); return false; }

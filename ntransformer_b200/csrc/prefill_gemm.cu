@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(512) rmsnorm_split_any_kernel(__half* __restri
     __half2* h2 = reinterpret_cast<__half2*>(hi + (size_t)blockIdx.x * hidden);
     __half2* l2 = reinterpret_cast<__half2*>(lo + (size_t)blockIdx.x * hidden);
     for (int i = threadIdx.x; i < hidden / 2; i += blockDim.x) {
-        const float2 xv = reinterpret_cast<const float2*>(x)[i], wv = reinterpret_cast<const float2*>(w)[i];
+        const float2 xv = make_float2(x[2 * i], x[2 * i + 1]), wv = make_float2(w[2 * i], w[2 * i + 1]);
         uint32_t ph, pl;
         split_pair(xv.x * rms_inv * wv.x, xv.y * rms_inv * wv.y, bf16, ph, pl);
         reinterpret_cast<uint32_t*>(h2)[i] = ph;

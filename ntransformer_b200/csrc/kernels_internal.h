@@ -533,7 +533,7 @@ size_t block_tokens_bytes(int T, int K);
 BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w /* null: x itself */, float eps, int T, int K, cudaStream_t s);
 BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, cudaStream_t s);
 BlockTokens resplit_tokens(void* workspace, const void* split, int T, int K, cudaStream_t s);      // of a plain split (split_activations' layout), in place too
-// scratch: block_scratch_bytes(), whatever they hold, of one stream's; null: whole tiles to a CTA.  fine: 64 columns to an accumulator, as exact as
+// scratch: block_scratch_bytes(), whatever they hold, of one stream's.  fine: 64 columns to an accumulator, as exact as
 // the decode step's 24-bit integers, instead of 256
 size_t block_scratch_bytes();
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, bool fine, int T, bool add, cudaStream_t s);

@@ -43,7 +43,7 @@ struct BlkMat { const uint8_t* W; float* C; int rows, tiles, fmt; long long pitc
 struct alignas(64) BlkMaps { CUtensorMap x, sums, w[3]; };      // tokens, their sums, matrices as 32-bit words
 struct BlkParams {
     BlkMat mat[3];
-    int n_mat, T, NT, cols, Mp, NB, kc, add, grain, stages, b_stage, raw_depth, raw_slot, a_cols, d_bufs;
+    int n_mat, T, NT, cols, Mp, NB, kc, add, stages, b_stage, raw_depth, raw_slot, a_cols, d_bufs;
     int tma;                   // a matrix's rows come by TMA (bits)
     int units;                 // tiles * super-blocks
     const float* scale;        // of a token's products
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
     const uint32_t b_tile = (uint32_t)NT * 128, b_stage = (uint32_t)p.b_stage, dead = smem_u32(&dead_smem);
     uint8_t* raw = smem + (size_t)p.stages * b_stage;
     // this CTA's super-blocks: units [u0, u1), unit = tile * NB + super-block
-    auto first_unit = [&](int cta) { return (int)((long long)(p.units / p.grain) * cta / (int)gridDim.x) * p.grain; };
+    auto first_unit = [&](int cta) { return (int)((long long)p.units * cta / (int)gridDim.x); };
     const int u0 = first_unit(blockIdx.x), u1 = first_unit(blockIdx.x + 1);
     auto format = [&](int fmt) { return MASK == 1 ? 0 : MASK == 2 ? 1 : MASK == 4 ? 2 : MASK == 8 ? 3 : MASK == 16 ? 4 : fmt; };
     auto mins_of = [&](int mi) { return ONE ? MINS : MINS && has_mins(p.mat[mi].fmt); };
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
             if (end - seg0 < NB) {                                 // shared: to the scratch; whoever comes last adds
                 write = false;
                 const int tu = q.tile * NB, G = gridDim.x;
-                const int c0 = (int)(((long long)(tu + 1) * G - 1) / p.units), c1 = (int)(((long long)(tu + NB) * G - 1) / p.units);      // (grain 1 wherever tiles are shared)
+                const int c0 = (int)(((long long)(tu + 1) * G - 1) / p.units), c1 = (int)(((long long)(tu + NB) * G - 1) / p.units);
                 float* mine = p.part + (size_t)(2 * blockIdx.x + (seg0 == u0 ? 0 : 1)) * 128 * NT + r;
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
@@ -737,9 +737,7 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     p.d_bufs = std::min(D_BUFS_MAX, (512 - p.stages * p.a_cols - (mins ? 8 : 0)) / p.NT);
     p.raw_depth = (int)std::min<size_t>(RAW_MAX, (cap - (size_t)p.stages * p.b_stage) / slot);
     if (p.raw_depth < 1 || p.d_bufs < 2) return false;
-    // a run of super-blocks to a CTA; without a scratch whole tiles
-    p.grain = scratch ? 1 : p.NB;
-    const int grid = std::min(sms, p.units / p.grain);
+    const int grid = std::min(sms, p.units);
     p.part = static_cast<float*>(scratch);
     p.count = x.count;
     BlkMaps maps;

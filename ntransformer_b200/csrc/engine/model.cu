@@ -804,7 +804,7 @@ bool Model::ensure_short_buffers() {
     if (!ensure_block_scratch()) return false;
     const size_t T = SHORT_CHUNK, hidden = (size_t)cfg_.hidden_size, qdim = (size_t)nh_l_ * cfg_.head_dim, kvdim = (size_t)nkv_l_ * cfg_.head_dim, f = sizeof(float);
     const size_t bytes[11] = {T * hidden * f, T * qdim * f, T * kvdim * f, T * kvdim * f, T * qdim * f, T * (size_t)inter_l_ * f, T * (size_t)inter_l_ * f,
-                              std::max(block_tokens_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_)),
+                              std::max(block_tokens_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_), true),
                                        gemv_rows_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_))),
                               attention_rows_scratch_floats((int)T, cfg_.max_seq_len, nh_l_, nkv_l_, cfg_.head_dim) * f, T * sizeof(int), T * sizeof(int)};
     void* got[11] = {};
@@ -837,8 +837,8 @@ void Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
             gemv_rows(m, n, K, sb_.ws, T, ep, s);
             return false;
         }
-        const BlockTokens t = up ? silu_split_tokens(sb_.ws, x, up, T, K, s) : split_tokens(sb_.ws, x, norm, cfg_.norm_eps, T, K, s);
-        NT_CHECK(gemm_blocks(m, n, K, t, block_scratch_, true, T, ep == GEMV_ADD, s), "GEMM of a few tokens over blocks rejected");
+        const BlockTokens t = up ? silu_split_tokens(sb_.ws, x, up, T, K, true, s) : split_tokens(sb_.ws, x, norm, cfg_.norm_eps, T, K, true, s);
+        NT_CHECK(gemm_blocks(m, n, K, t, block_scratch_, T, ep == GEMV_ADD, s), "GEMM of a few tokens over blocks rejected");
         return ep == GEMV_SWIGLU;
     };
     for (int c0 = 0; c0 < seq_len; c0 += T) {
@@ -900,8 +900,8 @@ void Model::prefill_gemms(float* const* C, void* ws, const float* x, const float
     for (int i = 0; i < n_plain && together; i++) { together = f16_direct(*plain[i]) && plain[i]->rows >= 256; W[i] = plain[i]->ptr; N[i] = plain[i]->rows; }
     if (!together || !gemm_f16_tc_multi_ws(c, ws, W, N, n_plain, T, K, s)) for (int i = 0; i < n_plain; i++) prefill_gemm(c[i], ws, *plain[i], T, add, s);
     if (n_blocks) {
-        const BlockTokens t = x ? split_tokens(ws, x, norm_w, cfg_.norm_eps, T, K, s) : resplit_tokens(ws, ws, T, K, s);
-        NT_CHECK(gemm_blocks(m, n_blocks, K, t, block_scratch_, false, T, add, s), "prefill GEMM over blocks rejected");
+        const BlockTokens t = x ? split_tokens(ws, x, norm_w, cfg_.norm_eps, T, K, false, s) : resplit_tokens(ws, ws, T, K, s);
+        NT_CHECK(gemm_blocks(m, n_blocks, K, t, block_scratch_, T, add, s), "prefill GEMM over blocks rejected");
     }
 }
 
@@ -928,8 +928,8 @@ void Model::ensure_prefill_buffers(int tokens) {
     pf_.x = dmalloc<float>(T * hidden);
     pf_.q = dmalloc<float>(T * qdim);    pf_.k = dmalloc<float>(T * kvdim);   pf_.v = dmalloc<float>(T * kvdim);
     pf_.attn = dmalloc<float>(T * qdim);
-    pf_.ws = dmalloc<uint8_t>(block_tokens_bytes((int)T, (int)std::max(hidden, qdim)));
-    pf_.ws2 = dmalloc<uint8_t>(block_tokens_bytes((int)T, inter_l_));
+    pf_.ws = dmalloc<uint8_t>(block_tokens_bytes((int)T, (int)std::max(hidden, qdim), false));
+    pf_.ws2 = dmalloc<uint8_t>(block_tokens_bytes((int)T, inter_l_, false));
     pf_.tok = dmalloc<int>(T);           pf_.pos = dmalloc<int>(T);
     size_t w_elems = 0;                  // largest matrix that needs the dequantised scratch pair
     bool swiglu_unfused = false, any_blocks = false;
@@ -988,7 +988,7 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
                 prefill_gemms(gu_out, pf_.ws, pf_.x, L.ffn_norm, gu, 2, T, false, s);
                 if (blocks_direct(L.down)) {
                     GemvMat m; m.W = down->ptr; m.y = pf_.x; m.out = down->rows; m.dtype = down->dtype; m.row_pitch = down->pitch;
-                    NT_CHECK(gemm_blocks(&m, 1, inter, silu_split_tokens(pf_.ws2, pf_.g, pf_.u, T, inter, s), block_scratch_, false, T, true, s), "prefill GEMM over blocks rejected");
+                    NT_CHECK(gemm_blocks(&m, 1, inter, silu_split_tokens(pf_.ws2, pf_.g, pf_.u, T, inter, false, s), block_scratch_, T, true, s), "prefill GEMM over blocks rejected");
                 } else {
                     silu_mul_split(pf_.ws2, pf_.g, pf_.u, T, inter, s);
                     prefill_gemm(pf_.x, pf_.ws2, L.down, T, true, s);

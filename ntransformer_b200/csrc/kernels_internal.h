@@ -528,15 +528,15 @@ inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
 bool gemm_blocks_supported(const GemvMat* mats, int n_mat, int K);
 // T tokens as this product takes them, in one workspace (block_tokens_bytes; its front is split_activations' layout): F16 hi and lo rows, sums of 32 columns,
 // the power of two that each token was divided by, and the counts of the product that follows, cleared.
-struct BlockTokens { void* split = nullptr; void* sums = nullptr; float* scale = nullptr; unsigned* count = nullptr; };
-size_t block_tokens_bytes(int T, int K);
-BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w /* null: x itself */, float eps, int T, int K, cudaStream_t s);
-BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, cudaStream_t s);
+struct BlockTokens { void* split = nullptr; void* sums = nullptr; float* scale = nullptr; unsigned* count = nullptr; bool fine = false; };
+size_t block_tokens_bytes(int T, int K, bool fine);
+BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w /* null: x itself */, float eps, int T, int K, bool fine, cudaStream_t s);
+BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, bool fine, cudaStream_t s);
 BlockTokens resplit_tokens(void* workspace, const void* split, int T, int K, cudaStream_t s);      // of a plain split (split_activations' layout), in place too
 // scratch: block_scratch_bytes(), whatever they hold, of one stream's.  fine: 64 columns to an accumulator, as exact as
 // the decode step's 24-bit integers, instead of 256
 size_t block_scratch_bytes();
-bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, bool fine, int T, bool add, cudaStream_t s);
+bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, int T, bool add, cudaStream_t s);
 // Whether a few tokens are better served here (fine) than by gemv_rows: from two of its passes on (layers of an 8B model in Q4_K_M, 4 layers and head: 8 tokens
 // 771 us there, 900 here; 9 tokens 1025, 908; 31 tokens 1586, 973), and only where the error is no larger: not in Q8_0 and Q4_0, whose weights are pairs of halves here
 // (error against 64 bits 1.5e-7 of a result; 24-bit integers 1.3e-7.  K-quants: 1.3e-7 to 1.9e-7 here, 1.4e-7 to 2.3e-7 there)

@@ -189,8 +189,8 @@ __device__ __forceinline__ float block_power(const uint8_t* blk, float& inverse)
     return __uint_as_float((uint32_t)(127 - e) << 23);
 }
 
-// MASK: the formats that a launch's matrices have (bits)
-template <int MASK>
+// MASK: the formats that a launch's matrices have (bits).  PARTS: halves that a token's column is split into
+template <int MASK, int PARTS>
 __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_constant__ BlkMaps maps, const __grid_constant__ BlkParams p) {
     constexpr bool ONE = (MASK & (MASK - 1)) == 0, MINS = (MASK & 3) != 0, PAIRS = (MASK & 28) != 0;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -261,10 +261,12 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     }
                     filled = min(filled + 1, (uint32_t)p.stages);
                     uint8_t* d = smem + (size_t)st * b_stage;
-                    mbar_expect_tx(full + st, 2 * b_tile + (mins && kb == 3 ? NT * 32u : 0u));
-                    tma_load_2d(d, &maps.x, q.b * 256 + kb * QBK, q.t0, full + st);
-                    tma_load_2d(d + b_tile, &maps.x, q.b * 256 + kb * QBK, p.Mp + q.t0, full + st);      // the lo halves lie Mp rows below
-                    if (mins && kb == 3) tma_load_2d(d + 2 * b_tile, &maps.sums, q.b * 16, q.t0, full + st);
+                    mbar_expect_tx(full + st, PARTS * b_tile + (mins && kb == 3 ? (PARTS - 1) * NT * 32u : 0u));
+#pragma unroll
+                    for (int i = 0; i < PARTS; i++) tma_load_2d(d + i * b_tile, &maps.x, q.b * 256 + kb * QBK, i * p.Mp + q.t0, full + st);      // a part lies Mp rows below the one before
+                    if (mins && kb == 3)
+#pragma unroll
+                        for (int i = 0; i < PARTS - 1; i++) tma_load_2d(d + PARTS * b_tile + i * NT * 32, &maps.sums, q.b * 16, i * p.Mp + q.t0, full + st);
                     if (++st == (uint32_t)p.stages) { st = 0; par ^= 1; }
                 }
             }
@@ -289,17 +291,22 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     wait_cta(full + st, par, dead);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t bh = desc0 + st * stage_step, bl = bh + lo_step;
-                    const uint32_t ah = a_base + st * p.a_cols, al = ah + 32, acc = kb != k0;
-                    if (PAIRS && (ONE || !mins)) {                 // the small products first
-                        umma_ts_by(lead, d, al, bh, idesc, acc);
+                    const uint32_t ah = a_base + st * p.a_cols, al = ah + 32;
+                    uint32_t acc = kb != k0;
+                    auto product = [&](uint32_t a, uint64_t b) {
+                        umma_ts_by(lead, d, a, b, idesc, acc);
 #pragma unroll
-                        for (int k = 1; k < 4; k++) umma_ts_by(lead, d, al + 8 * k, bh + 2 * k, idesc, 1u);
-                        umma_ts_by(lead, d, ah, bl, idesc, 1u);
-                    } else umma_ts_by(lead, d, ah, bl, idesc, acc);
-#pragma unroll
-                    for (int k = 1; k < 4; k++) umma_ts_by(lead, d, ah + 8 * k, bl + 2 * k, idesc, 1u);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) umma_ts_by(lead, d, ah + 8 * k, bh + 2 * k, idesc, 1u);
+                        for (int k = 1; k < 4; k++) umma_ts_by(lead, d, a + 8 * k, b + 2 * k, idesc, 1u);
+                        acc = 1u;
+                    };
+                    // the small products first (what is left out is 2^-22 of a product with two parts, 2^-33 with three)
+                    if (PARTS == 3) {
+                        if (PAIRS && (ONE || !mins)) product(al, bl);
+                        product(ah, bl + lo_step);
+                    }
+                    if (PAIRS && (ONE || !mins)) product(al, bh);
+                    product(ah, bl);
+                    product(ah, bh);
                     last = (int)(st * 2 + par);
                     if (kb == 3 && mins) break;                    // its stage is free after the minima
                     umma_commit_by(lead, empty + st);
@@ -308,10 +315,12 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                 umma_commit_by(lead, d_full + db);
                 if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
             }
-            if (MINS && mins) {                                    // minima: 8 of them times the halves of 8 sums, twice
+            if (MINS && mins) {                                    // minima: 8 of them times the halves of 8 sums, twice (the third halves, and zeros, before)
                 wait_cta(d_empty + db, dpar, dead);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                umma_ts_by(lead, db * NT, m_base, desc32 + st * stage_step + 2 * lo_step, idesc, 0u);
+                const uint64_t sums = desc32 + st * stage_step + PARTS * lo_step;
+                if (PARTS == 3) umma_ts_by(lead, db * NT, m_base, sums + (NT * 32 >> 4), idesc, 0u);
+                umma_ts_by(lead, db * NT, m_base, sums, idesc, PARTS == 3);
                 umma_commit_by(lead, empty + st);                  // (the minima's place is free with this stage)
                 umma_commit_by(lead, d_full + db);
                 if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
@@ -546,12 +555,12 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
 // ---- tokens ----
 // One block to a token: x (MODE 1: RMSNorm(x) * w, rmsnorm.cu:17-70's math; 2: silu(x) * w, gemm.cu:713-725's expression; 3: hi x and lo w of
 // a plain split, which may be the one written to) as F16 hi + lo, the sums of 32 of them
-// (a 32nd part, so that they stay within F16) as hi + lo, and the factor that undoes the token's power of two.  That power takes the largest to 2^13 .. 2^14, where the
+// (a 32nd part, so that they stay within F16) as hi + lo, where `third` is given the halves that those two leave of both, and the factor that undoes the token's power of two.  That power takes the largest to 2^13 .. 2^14, where the
 // low halves keep their bits.  Block 0 also clears the product's counts: a launch whose wait ran out leaves some behind.
 // TOK_NORM_ANY: TOK_NORM whose gains do not lie on 16 bytes.
 enum : int { TOK_PLAIN = 0, TOK_NORM = 1, TOK_SILU = 2, TOK_SPLIT = 3, TOK_NORM_ANY = 4 };
 template <int MODE>
-__global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* lo, __half* __restrict__ sums, float* __restrict__ scale, unsigned* __restrict__ count, int counts,
+__global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* lo, __half* third, __half* __restrict__ sums, __half* __restrict__ third_sums, float* __restrict__ scale, unsigned* __restrict__ count, int counts,
                                                            const float* xin, const float* w, float eps, int K) {
     constexpr int KEEP = 7;                                        // chunks of 2048 held in registers: rows to 14336
     __shared__ float red[2][16];
@@ -601,7 +610,11 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
     if (tid == 0) scale[blockIdx.x] = __uint_as_float((254u - up) << 23);
     __half* h = hi + (size_t)blockIdx.x * K;
     __half* l = lo + (size_t)blockIdx.x * K;
-    __half* sm = sums + (size_t)blockIdx.x * (K / 16);
+    const size_t sm = (size_t)blockIdx.x * (K / 16);
+    auto rest = [](float v, uint32_t h, uint32_t l, bool upper) {  // what two halves leave of v: exact
+        const float2 fh = __half22float2(h2(h)), fl = __half22float2(h2(l));
+        return upper ? v - fh.y - fl.y : v - fh.x - fl.x;
+    };
     auto put = [&](int i, float4 a) {
         a.x *= f; a.y *= f; a.z *= f; a.w *= f;
         uint2 ph, pl;
@@ -609,13 +622,19 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
         split_pair(a.z, a.w, 0, ph.y, pl.y);
         *reinterpret_cast<uint2*>(h + i) = ph;
         *reinterpret_cast<uint2*>(l + i) = pl;
+        if (third)
+            *reinterpret_cast<uint2*>(third + (size_t)blockIdx.x * K + i) =
+                make_uint2(bits(__floats2half2_rn(rest(a.x, ph.x, pl.x, false), rest(a.y, ph.x, pl.x, true))), bits(__floats2half2_rn(rest(a.z, ph.y, pl.y, false), rest(a.w, ph.y, pl.y, true))));
         float s = (a.x + a.y) + (a.z + a.w);                       // K is a multiple of 256: whole warps
         s += __shfl_xor_sync(0xFFFFFFFFu, s, 1); s += __shfl_xor_sync(0xFFFFFFFFu, s, 2); s += __shfl_xor_sync(0xFFFFFFFFu, s, 4);
         if ((tid & 7) == 0) {
             s *= 1.0f / 32.0f;
             const __half sh = __float2half_rn(s);
-            __half* q = sm + (i >> 8) * 16 + ((i >> 5) & 7);
-            q[0] = sh; q[8] = __float2half_rn(s - __half2float(sh));
+            const float left = s - __half2float(sh);
+            const __half sl = __float2half_rn(left);
+            const size_t q = sm + (i >> 8) * 16 + ((i >> 5) & 7);
+            sums[q] = sh; sums[q + 8] = sl;
+            if (third) { third_sums[q] = __float2half_rn(left - __half2float(sl)); third_sums[q + 8] = __float2half_rn(0.f); }
         }
     };
 #pragma unroll
@@ -634,11 +653,11 @@ __global__ void __launch_bounds__(256) silu_split_kernel(uint2* __restrict__ hi,
     hi[i] = h; lo[i] = l;
 }
 
-template <int MASK>
+template <int MASK, int PARTS>
 void launch_blocks(const BlkMaps& maps, const BlkParams& p, int grid, size_t smem, cudaStream_t s) {
     static unsigned long long configured = 0;      // bit per device id
-    opt_in_dynamic_smem(gemm_blocks_kernel<MASK>, 214 * 1024, configured);
-    launch_k_pdl(true, gemm_blocks_kernel<MASK>, dim3(grid), dim3(Q_THREADS), smem, s, maps, p);
+    opt_in_dynamic_smem(gemm_blocks_kernel<MASK, PARTS>, 214 * 1024, configured);
+    launch_k_pdl(true, gemm_blocks_kernel<MASK, PARTS>, dim3(grid), dim3(Q_THREADS), smem, s, maps, p);
     count_launch();
 }
 
@@ -654,45 +673,44 @@ int sm_count() {
 
 bool gemm_blocks_supported(const GemvMat* mats, int n_mat, int K) { return gemv_kq_any_pitch(mats, n_mat, K); }
 
-// [hi rows, lo rows (gemm_f16_tc_workspace_bytes)][sums][scales][counts], rows padded to 128
-size_t block_tokens_bytes(int T, int K) { return gemm_f16_tc_workspace_bytes(T, K) + padded(T) * ((size_t)K / 8 + sizeof(float)) + (size_t)sm_count() * sizeof(unsigned); }
+// [hi rows][lo rows][third rows][their sums, part by part: fine has three, two of sums][scales][counts], rows padded to 128.  The front is gemm_f16_tc_workspace_bytes.
+static size_t parts_bytes(int T, int K, bool fine) { return gemm_f16_tc_workspace_bytes(T, K) / 2 * (fine ? 3 : 2); }
+static size_t sums_bytes(int T, int K, bool fine) { return padded(T) * ((size_t)K / 8) * (fine ? 2 : 1); }
+size_t block_tokens_bytes(int T, int K, bool fine) { return parts_bytes(T, K, fine) + sums_bytes(T, K, fine) + padded(T) * sizeof(float) + (size_t)sm_count() * sizeof(unsigned); }
 size_t block_scratch_bytes() { return (size_t)sm_count() * 2 * 128 * NT_MAX * sizeof(float); }
 
-BlockTokens block_tokens(void* workspace, int T, int K) {
+BlockTokens block_tokens(void* workspace, int T, int K, bool fine) {
     BlockTokens t;
     uint8_t* p = static_cast<uint8_t*>(workspace);
     t.split = p;
-    t.sums = p + gemm_f16_tc_workspace_bytes(T, K);
-    t.scale = reinterpret_cast<float*>(p + gemm_f16_tc_workspace_bytes(T, K) + padded(T) * ((size_t)K / 8));
+    t.sums = p + parts_bytes(T, K, fine);
+    t.scale = reinterpret_cast<float*>(p + parts_bytes(T, K, fine) + sums_bytes(T, K, fine));
     t.count = reinterpret_cast<unsigned*>(t.scale + padded(T));
+    t.fine = fine;
     return t;
 }
 
-BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, float eps, int T, int K, cudaStream_t s) {
-    const BlockTokens t = block_tokens(workspace, T, K);
-    __half* hi = static_cast<__half*>(t.split);
-    __half* lo = hi + padded(T) * (size_t)K;
-    const bool wide = (reinterpret_cast<uintptr_t>(norm_w) & 15) == 0;
-    launch_k_pdl(true, !norm_w ? split_tokens_kernel<TOK_PLAIN> : wide ? split_tokens_kernel<TOK_NORM> : split_tokens_kernel<TOK_NORM_ANY>, dim3(T), dim3(512), 0, s, hi, lo, static_cast<__half*>(t.sums), t.scale, t.count, sm_count(), x, norm_w, eps, K);
+namespace {
+template <int MODE>
+BlockTokens launch_split(void* workspace, const float* x, const float* w, float eps, int T, int K, bool fine, cudaStream_t s) {
+    const BlockTokens t = block_tokens(workspace, T, K, fine);
+    const size_t part = padded(T) * (size_t)K;
+    __half *hi = static_cast<__half*>(t.split), *sums = static_cast<__half*>(t.sums);
+    launch_k_pdl(true, split_tokens_kernel<MODE>, dim3(T), dim3(512), 0, s, hi, hi + part, fine ? hi + 2 * part : nullptr, sums, sums + part / 16, t.scale, t.count, sm_count(), x, w, eps, K);
     count_launch();
     return t;
 }
-BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, cudaStream_t s) {
-    const BlockTokens t = block_tokens(workspace, T, K);
-    __half* hi = static_cast<__half*>(t.split);
-    launch_k_pdl(true, split_tokens_kernel<TOK_SILU>, dim3(T), dim3(512), 0, s, hi, hi + padded(T) * (size_t)K, static_cast<__half*>(t.sums), t.scale, t.count, sm_count(), gate,
-                 up, 0.f, K);
-    count_launch();
-    return t;
+}  // namespace
+
+BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, float eps, int T, int K, bool fine, cudaStream_t s) {
+    if (!norm_w) return launch_split<TOK_PLAIN>(workspace, x, nullptr, 0.f, T, K, fine, s);
+    return (reinterpret_cast<uintptr_t>(norm_w) & 15) ? launch_split<TOK_NORM_ANY>(workspace, x, norm_w, eps, T, K, fine, s) : launch_split<TOK_NORM>(workspace, x, norm_w, eps, T, K, fine, s);
+}
+BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, bool fine, cudaStream_t s) {
+    return launch_split<TOK_SILU>(workspace, gate, up, 0.f, T, K, fine, s);
 }
 BlockTokens resplit_tokens(void* workspace, const void* split, int T, int K, cudaStream_t s) {
-    const BlockTokens t = block_tokens(workspace, T, K);
-    __half* hi = static_cast<__half*>(t.split);
-    const size_t lo = padded(T) * (size_t)K;
-    launch_k_pdl(true, split_tokens_kernel<TOK_SPLIT>, dim3(T), dim3(512), 0, s, hi, hi + lo, static_cast<__half*>(t.sums), t.scale, t.count, sm_count(),
-                 static_cast<const float*>(split), reinterpret_cast<const float*>(static_cast<const __half*>(split) + lo), 0.f, K);
-    count_launch();
-    return t;
+    return launch_split<TOK_SPLIT>(workspace, static_cast<const float*>(split), reinterpret_cast<const float*>(static_cast<const __half*>(split) + padded(T) * (size_t)K), 0.f, T, K, false, s);
 }
 
 bool gemm_blocks_for_few(const GemvMat* mats, int n_mat, int tokens) {
@@ -701,7 +719,7 @@ bool gemm_blocks_for_few(const GemvMat* mats, int n_mat, int tokens) {
     return tokens > 8 && exact;
 }
 
-bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, bool fine, int T, bool add, cudaStream_t s) {
+bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, int T, bool add, cudaStream_t s) {
     if (T <= 0 || !gemm_blocks_supported(mats, n_mat, K)) return false;
     const int sms = sm_count();
     BlkParams p{};
@@ -709,7 +727,8 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     p.n_mat = n_mat; p.T = T; p.NB = K / 256; p.add = add;
     p.Mp = (int)padded(T);
     p.scale = x.scale;
-    p.kc = fine ? 1 : p.NB == 1 ? 2 : 4;
+    p.kc = x.fine ? 1 : p.NB == 1 ? 2 : 4;
+    const int parts = x.fine ? 3 : 2;
     int tiles = 0, slot = 0, mask = 0;
     for (int i = 0; i < n_mat; i++) {
         BlkMat& m = p.mat[i];
@@ -728,7 +747,7 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     // fewer tokens there are: weights from HBM are then what bounds)
     p.a_cols = pairs ? 64 : 32;
     p.raw_slot = slot;
-    p.b_stage = (p.NT * (256 + (mins ? 32 : 0)) + 1023) / 1024 * 1024;
+    p.b_stage = (p.NT * (128 * parts + (mins ? 32 * (parts - 1) : 0)) + 1023) / 1024 * 1024;
     const size_t cap = 213 * 1024;
     for (p.stages = STAGES_MAX; p.stages > 2; p.stages--) {
         p.d_bufs = std::min(D_BUFS_MAX, (512 - p.stages * p.a_cols - (mins ? 8 : 0)) / p.NT);
@@ -741,7 +760,8 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     p.part = static_cast<float*>(scratch);
     p.count = x.count;
     BlkMaps maps;
-    if (!tc_map_f16(&maps.x, x.split, 2 * (uint64_t)p.Mp, (uint64_t)K, (uint32_t)p.NT) || !tc_map_f16_rows32(&maps.sums, x.sums, (uint64_t)p.Mp, (uint64_t)K / 16, (uint32_t)p.NT))
+    if (!tc_map_f16(&maps.x, x.split, parts * (uint64_t)p.Mp, (uint64_t)K, (uint32_t)p.NT) ||
+        !tc_map_f16_rows32(&maps.sums, x.sums, (parts - 1) * (uint64_t)p.Mp, (uint64_t)K / 16, (uint32_t)p.NT))
         return false;
     for (int i = 0; i < n_mat; i++) {
         const BlkMat& m = p.mat[i];
@@ -750,27 +770,24 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
         p.tma |= 1 << i;
     }
     const size_t smem = p.stages * (size_t)p.b_stage + (size_t)p.raw_depth * slot + 1024;
+#define NT_BLOCKS(M) case M: parts == 3 ? launch_blocks<M, 3>(maps, p, grid, smem, s) : launch_blocks<M, 2>(maps, p, grid, smem, s); break
     switch (mask) {
-        case 1: launch_blocks<1>(maps, p, grid, smem, s); break;
-        case 2: launch_blocks<2>(maps, p, grid, smem, s); break;
-        case 4: launch_blocks<4>(maps, p, grid, smem, s); break;
-        case 5: launch_blocks<5>(maps, p, grid, smem, s); break;
-        case 8: launch_blocks<8>(maps, p, grid, smem, s); break;
-        case 16: launch_blocks<16>(maps, p, grid, smem, s); break;
-        default: launch_blocks<31>(maps, p, grid, smem, s); break;
+        NT_BLOCKS(1); NT_BLOCKS(2); NT_BLOCKS(4); NT_BLOCKS(5); NT_BLOCKS(8); NT_BLOCKS(16);
+        default: parts == 3 ? launch_blocks<31, 3>(maps, p, grid, smem, s) : launch_blocks<31, 2>(maps, p, grid, smem, s); break;
     }
+#undef NT_BLOCKS
     return true;
 }
 
 // The same over F32 tokens, or (x null) over tokens that split_activations laid out; what it needs beside them lies in memory of this call's
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const float* norm_w, float eps, const void* split, bool fine, int T, bool add, cudaStream_t s) {
     if (T <= 0 || !gemm_blocks_supported(mats, n_mat, K) || (reinterpret_cast<uintptr_t>(x) & 15)) return false;
-    const size_t tokens = (block_tokens_bytes(T, K) + 255) / 256 * 256;
+    const size_t tokens = (block_tokens_bytes(T, K, fine && x) + 255) / 256 * 256;
     void* mem = nullptr;
     if (cudaMallocAsync(&mem, tokens + block_scratch_bytes(), s) != cudaSuccess) { cudaGetLastError(); return false; }
     uint8_t* scratch = static_cast<uint8_t*>(mem) + tokens;
-    const BlockTokens t = x ? split_tokens(mem, x, norm_w, eps, T, K, s) : resplit_tokens(mem, split, T, K, s);
-    const bool ok = gemm_blocks(mats, n_mat, K, t, scratch, fine, T, add, s);
+    const BlockTokens t = x ? split_tokens(mem, x, norm_w, eps, T, K, fine, s) : resplit_tokens(mem, split, T, K, s);
+    const bool ok = gemm_blocks(mats, n_mat, K, t, scratch, T, add, s);
     NT_CUDA_CHECK(cudaFreeAsync(mem, s));
     return ok;
 }

@@ -154,6 +154,7 @@ void   nt_b200_dequant_split(void* w_hi, void* w_lo, const void* W, int dtype, s
 int    nt_b200_wait_status(int set);
 void   nt_b200_wait_probe(unsigned tries, int* came_dev, void* stream);
 unsigned long long nt_b200_launch_count(void);   /* kernels launched by this library so far */
+unsigned long long nt_b200_programmatic_count(void);   /* those launched so that they may start while the one before ends (NT_B200_NO_PDL: none of a Model's) */
 int    nt_b200_stream_sync(void* stream);        /* cudaStreamSynchronize; returns cudaError_t */
 const char* nt_b200_version(void);
 

@@ -63,6 +63,7 @@ SIGNATURES = {
     "nt_b200_wait_status": (_i, [_i]),
     "nt_b200_wait_probe": (None, [C.c_uint, _vp, _vp]),
     "nt_b200_launch_count": (C.c_ulonglong, []),
+    "nt_b200_programmatic_count": (C.c_ulonglong, []),
     "nt_b200_stream_sync": (_i, [_vp]),
     "nt_b200_version": (C.c_char_p, []),
 }

@@ -18,9 +18,13 @@ namespace nt { namespace b200 {
 static std::atomic<unsigned long long> g_launches{0};
 unsigned long long launch_count() { return g_launches.load(); }
 void count_launch(int n) { g_launches.fetch_add((unsigned long long)n); }
-static std::atomic<bool> g_pdl{false};
-void set_pdl(bool on) { g_pdl.store(on); }
-bool pdl_enabled() { return g_pdl.load(); }
+static std::atomic<unsigned long long> g_programmatic{0};
+unsigned long long programmatic_count() { return g_programmatic.load(); }
+void count_programmatic() { g_programmatic.fetch_add(1); }
+static thread_local Launches t_launches = Launches::Boundary;
+Launches launches() { return t_launches; }
+LaunchScope::LaunchScope(Launches m) : was(t_launches) { t_launches = m; }
+LaunchScope::~LaunchScope() { t_launches = was; }
 
 namespace {
 

@@ -740,7 +740,10 @@ void Model::run_step_mega(bool with_head) {
     if (with_head && tp_size_ > 1) comm_->all_gather(logits_l_, logits_, (size_t)vocab_l_, stream_);
 }
 
+bool Model::programmatic() const { return use_pdl_ && !getenv("NT_B200_NO_PDL"); }
+
 void Model::run_step(bool with_head) {
+    const LaunchScope scope(programmatic() ? launches() : Launches::Plain);
     // NT_B200_MEGAKERNEL: unset -> the model's own setting (set_use_megakernel, off by default), "0" -> off, anything else -> on
     const char* mk = getenv("NT_B200_MEGAKERNEL");
     const bool want_mega = !cfg_.layer_spec() && (mk ? env_on("NT_B200_MEGAKERNEL") : use_mega_);
@@ -757,10 +760,11 @@ void Model::run_step(bool with_head) {
         cudaGraph_t graph = nullptr;
         const unsigned long long before = launch_count();
         NT_CUDA_CHECK(cudaStreamBeginCapture(stream_, tp_size_ > 1 ? cudaStreamCaptureModeRelaxed : cudaStreamCaptureModeThreadLocal));
-        set_pdl(use_pdl_ && !getenv("NT_B200_NO_PDL"));   // programmatic edges between the step's kernels
-        step_body(stream_);
-        if (with_head) step_head(stream_, chain_ok());
-        set_pdl(false);
+        {
+            const LaunchScope step(programmatic() ? Launches::Step : Launches::Plain);      // programmatic edges between the step's kernels
+            step_body(stream_);
+            if (with_head) step_head(stream_, chain_ok());
+        }
         NT_CUDA_CHECK(cudaStreamEndCapture(stream_, &graph));
         NT_CUDA_CHECK(cudaGraphInstantiate(&g, graph, 0));
         NT_CUDA_CHECK(cudaGraphDestroy(graph));
@@ -1018,6 +1022,7 @@ void Model::forward_async(const int* tokens, int seq_len, int start_pos) {
     NT_CHECK(seq_len >= 1, "forward: empty token list");
     NT_CHECK(start_pos >= 0 && start_pos + seq_len <= cfg_.max_seq_len, "forward: position beyond the KV cache (max_seq_len)");
     for (int t = 0; t < seq_len; t++) NT_CHECK(tokens[t] >= 0 && tokens[t] < cfg_.vocab_size, "token id out of range");
+    const LaunchScope scope(programmatic() ? launches() : Launches::Plain);
     if (cfg_.layer_spec()) {
         if (prefill_min_tokens_ > 0 && seq_len >= prefill_min_tokens_ && !getenv("NT_B200_NO_BATCHED_PREFILL")) { prefill_spec(tokens, seq_len, start_pos); return; }
     } else if (batched_prefill_ok(seq_len, start_pos)) { prefill_batched(tokens, seq_len, start_pos); return; }

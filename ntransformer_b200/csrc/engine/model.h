@@ -161,6 +161,7 @@ public:
     double load_seconds() const { return load_seconds_; }     // wall time of load_gguf (parse + plan + pipelined upload + buffers)
     void set_use_graph(bool on) { use_graph_ = on; }
     void set_use_pdl(bool on) { use_pdl_ = on; }
+    bool programmatic() const;
     // Prompts of at least n tokens go through the batched tensor-core prefill when the weights allow it (0 = never).
     void set_prefill_min_tokens(int n) { prefill_min_tokens_ = n; }
     bool batched_prefill_ok(int seq_len, int start_pos) const;

@@ -499,16 +499,30 @@ void mlstm_out_norm(float* out, void* split, const float* o, const float* den, c
 void mlstm_token(float* out, const float* q, const float* k, const float* v, const float* gate, const float* zi, const float* zf, const float* bi, const float* bf,
                  const float* norm, float* state, float* m, float cap, float q_scale, float eps, int heads, int dim, int vdim, const int* pos_dev, int p0, cudaStream_t s);
 
-// Programmatic dependent launch (PDL): when enabled, kernels are launched with
-// cudaLaunchAttributeProgrammaticStreamSerialization so that a kernel's prologue (barrier init, TMA weight
-// prefetch) overlaps the tail of its predecessor; every kernel executes griddepcontrol.wait before it touches
-// data produced upstream, so ordering is unchanged.  launch_k: off by default, the engine turns it on for decode graphs; there kernels may read weights ahead of the wait.
-// launch_k_pdl(true, ...): everywhere, for kernels that read nothing ahead of it then.  Behind the launcher boundary, call by call, a launch waits for the one before
-// to drain and then starts for 1.3 .. 2.3 us (one Q8_0 matrix of 1024 x 4096: 6.14 -> 3.87 us a call, a decoder layer's sixteen launches 112 -> 80.6 us).
-void set_pdl(bool on);
-bool pdl_enabled();
+// Programmatic dependent launch (PDL): kernels launched with cudaLaunchAttributeProgrammaticStreamSerialization have their prologue (barrier init, TMA weight
+// prefetch) overlap the tail of the launch before; every kernel executes griddepcontrol.wait before it touches data produced upstream, so ordering is unchanged.
+// This thread's launches:
+//   Boundary (as it is by itself)  launch_k_pdl(true, ...) is programmatic, launch_k is not, and no kernel reads weights ahead of its wait (the launch before may have
+//                                  written them; gemm_blocks does, and says why it may).  Call by call, a launch otherwise waits for the one before to drain and then starts
+//                                  for 1.3 .. 2.3 us (one Q8_0 matrix of 1024 x 4096: 6.14 -> 4.64 us a call, a decoder layer's sixteen launches 112 -> 80.6 us)
+//   Step                           a decode step that the engine captures: all of them are, and weights are settled: kernels may read them ahead of the wait
+//   Plain                          none is: a Model whose programmatic launches are switched off (set_use_pdl, NT_B200_NO_PDL)
+enum class Launches { Boundary, Step, Plain };
+Launches launches();
+struct LaunchScope {
+    Launches was;
+    explicit LaunchScope(Launches m);
+    ~LaunchScope();
+    LaunchScope(const LaunchScope&) = delete;
+    LaunchScope& operator=(const LaunchScope&) = delete;
+};
+inline bool pdl_enabled() { return launches() == Launches::Step; }
+unsigned long long programmatic_count();      // launches so far that were
+void count_programmatic();
 template <typename... KArgs, typename... Args>
 inline void launch_k_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+    pdl = pdl && launches() != Launches::Plain;
+    if (pdl) count_programmatic();
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -535,6 +549,8 @@ BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* u
 BlockTokens resplit_tokens(void* workspace, const void* split, int T, int K, cudaStream_t s);      // of a plain split (split_activations' layout), in place too
 // scratch: block_scratch_bytes(), whatever they hold, of one stream's.  fine: 64 columns to an accumulator, as exact as
 // the decode step's 24-bit integers, instead of 256
+// The matrices are read ahead of the wait for the launch before.  That is the one that laid the tokens out: it lets this one start only behind its own wait, when
+// whatever wrote the matrices is done.  No other launch comes between the two.
 size_t block_scratch_bytes();
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, int T, bool add, cudaStream_t s);
 // Whether a few tokens are better served here (fine) than by gemv_rows: from two of its passes on (layers of an 8B model in Q4_K_M, 4 layers and head: 8 tokens

@@ -207,6 +207,7 @@ void nt_b200_dequant_split(void* hi, void* lo, const void* W, int dt, size_t pit
     nt::b200::dequant_split(hi, lo, W, (DType)dt, pitch, rows, cols, static_cast<cudaStream_t>(s));
 }
 unsigned long long nt_b200_launch_count(void) { return nt::b200::launch_count(); }
+unsigned long long nt_b200_programmatic_count(void) { return nt::b200::programmatic_count(); }
 int nt_b200_stream_sync(void* s) { return (int)cudaStreamSynchronize(static_cast<cudaStream_t>(s)); }
 const char* nt_b200_version(void) { return "ntransformer_b200 0.1 (sm_100a)"; }
 

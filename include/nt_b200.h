@@ -153,6 +153,10 @@ void   nt_b200_dequant_split(void* w_hi, void* w_lo, const void* W, int dtype, s
  * stores `set`.  nt_b200_wait_probe launches a wait that asks `tries` times for something that does not come (came_dev: device int, 0 afterwards). */
 int    nt_b200_wait_status(int set);
 void   nt_b200_wait_probe(unsigned tries, int* came_dev, void* stream);
+/* Memory that calls need beside their arguments (nt_b200_attention_decode, nt_b200_gemm_blocks*) is theirs or their stream's, in its order (captured: memory nodes of
+ * the graph).  For each device up to 64 MB of it, and the buffers of up to 16 streams that decode, are kept for the next calls; this waits for the current device and
+ * gives its back, as the end of a Model does. */
+void   nt_b200_trim_memory(void);
 unsigned long long nt_b200_launch_count(void);   /* kernels launched by this library so far */
 unsigned long long nt_b200_programmatic_count(void);   /* those launched so that they may start while the one before ends (NT_B200_NO_PDL: none of a Model's) */
 int    nt_b200_stream_sync(void* stream);        /* cudaStreamSynchronize; returns cudaError_t */

@@ -18,7 +18,7 @@
 #include <cuda_fp16.h>
 #include <algorithm>
 #include <cfloat>
-#include <mutex>
+#include <optional>
 
 namespace nt { namespace b200 {
 
@@ -358,20 +358,6 @@ __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) prefill_kerne
     attend_group<DPL, GC>(out + qoff, Q + qoff, kc, vc, kv_head, n_kv, 0, start_pos + qi + 1, scale, nullptr, nullptr, smem_dyn);
 }
 
-float* g_scratch = nullptr;
-size_t g_scratch_floats = 0;
-std::mutex g_scratch_mu;
-float* attn_scratch(size_t floats) {
-    std::lock_guard<std::mutex> lk(g_scratch_mu);
-    if (floats > g_scratch_floats) {
-        if (g_scratch) { cudaDeviceSynchronize(); cudaFree(g_scratch); }
-        size_t want = floats < (1u << 20) ? (1u << 20) : floats;
-        NT_CUDA_CHECK(cudaMalloc(&g_scratch, want * sizeof(float)));
-        g_scratch_floats = want;
-    }
-    return g_scratch;
-}
-
 int pick_gc(int group) { return group % 8 == 0 ? 8 : group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1; }
 
 template <int DPL, int GC>
@@ -393,8 +379,11 @@ void launch_decode(float* out, const float* q, const __half* kc, const __half* v
     const size_t smem = ((size_t)walk_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
     opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
-    float* scratch = nullptr;
-    if (n_splits > 1) scratch = attn_scratch((size_t)n_heads * n_splits * (HD + 2));
+    // the slices' results: the stream's, so that calls on other streams and devices and by other threads have their own
+    std::optional<StreamMemory> memory;
+    if (n_splits > 1) memory.emplace((size_t)n_heads * n_splits * (HD + 2) * sizeof(float), s);
+    float* scratch = memory ? static_cast<float*>(memory->p) : nullptr;
+    if (!scratch) { n_splits = 1; split_len = seq_len; }          // no memory: one slice
     // Programmatic launches outside graphs too: neither kernel reads or writes before its wait, so the merge's launch hides behind the slices
     launch_k_pdl(true, decode_kernel<DPL, GC>, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, kc, vc, seq_len, n_heads, n_kv, scale, n_splits, split_len,
                  scratch, (const int*)nullptr);

@@ -97,6 +97,7 @@ Model::~Model() {
                     (void*)par_dec_.mix[4]}) if (p) cudaFree(p);
     if (argmax_host_) cudaFreeHost(argmax_host_);
     if (stream_) cudaStreamDestroy(stream_);
+    trim_call_memory();
 }
 
 void Model::release_graphs() {

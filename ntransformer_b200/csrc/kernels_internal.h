@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 #include <utility>
 #include "nt_types.h"
 
@@ -115,6 +116,28 @@ void attention_decode(float* out, const float* q, const void* kc, const void* vc
                       int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
 void attention_prefill(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos,
                        int n_heads, int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
+// call_memory.cu: memory that lasts for the launches of a call (the object's life), in the order of its stream; p null: there is none
+constexpr size_t CALL_MEMORY_KEPT = 64u << 20;        // of a device, between calls
+constexpr size_t STREAM_MEMORY_LEAST = 2u << 20;
+struct CallMemory {
+    void* p;
+    cudaStream_t stream;
+    CallMemory(size_t bytes, cudaStream_t s);
+    ~CallMemory();
+    CallMemory(const CallMemory&) = delete;
+    CallMemory& operator=(const CallMemory&) = delete;
+};
+struct StreamMemory {
+    void* p = nullptr;
+    cudaStream_t stream;
+    bool own = false;
+    std::unique_lock<std::mutex> lock;
+    StreamMemory(size_t bytes, cudaStream_t s);
+    ~StreamMemory();
+    StreamMemory(const StreamMemory&) = delete;
+    StreamMemory& operator=(const StreamMemory&) = delete;
+};
+void trim_call_memory();                              // what the current device keeps
 // the form that attention_prefill takes: a query at a time, mma.sync, tcgen05
 enum : int { PREFILL_QUERIES = 0, PREFILL_MMA = 1, PREFILL_TC = 2 };
 int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq);

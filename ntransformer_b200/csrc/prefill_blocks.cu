@@ -783,13 +783,12 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const float* norm_w, float eps, const void* split, bool fine, int T, bool add, cudaStream_t s) {
     if (T <= 0 || !gemm_blocks_supported(mats, n_mat, K) || (reinterpret_cast<uintptr_t>(x) & 15)) return false;
     const size_t tokens = (block_tokens_bytes(T, K, fine && x) + 255) / 256 * 256;
-    void* mem = nullptr;
-    if (cudaMallocAsync(&mem, tokens + block_scratch_bytes(), s) != cudaSuccess) { cudaGetLastError(); return false; }
-    uint8_t* scratch = static_cast<uint8_t*>(mem) + tokens;
+    CallMemory memory(tokens + block_scratch_bytes(), s);
+    uint8_t* mem = static_cast<uint8_t*>(memory.p);
+    if (!mem) return false;
+    uint8_t* scratch = mem + tokens;
     const BlockTokens t = x ? split_tokens(mem, x, norm_w, eps, T, K, fine, s) : resplit_tokens(mem, split, T, K, s);
-    const bool ok = gemm_blocks(mats, n_mat, K, t, scratch, T, add, s);
-    NT_CUDA_CHECK(cudaFreeAsync(mem, s));
-    return ok;
+    return gemm_blocks(mats, n_mat, K, t, scratch, T, add, s);
 }
 
 void silu_mul_split(void* workspace, const float* gate, const float* up, int rows, int cols, cudaStream_t s) {

@@ -905,7 +905,7 @@ void Model::prefill_gemms(float* const* C, void* ws, const float* x, const float
     for (int i = 0; i < n_plain && together; i++) { together = f16_direct(*plain[i]) && plain[i]->rows >= 256; W[i] = plain[i]->ptr; N[i] = plain[i]->rows; }
     if (!together || !gemm_f16_tc_multi_ws(c, ws, W, N, n_plain, T, K, s)) for (int i = 0; i < n_plain; i++) prefill_gemm(c[i], ws, *plain[i], T, add, s);
     if (n_blocks) {
-        const BlockTokens t = x ? split_tokens(ws, x, norm_w, cfg_.norm_eps, T, K, false, s) : resplit_tokens(ws, ws, T, K, s);
+        const BlockTokens t = x ? split_tokens(ws, x, norm_w, cfg_.norm_eps, T, K, false, s) : resplit_tokens(ws, ws, static_cast<uint8_t*>(ws) + gemm_f16_tc_workspace_bytes(T, K) / 2, T, K, s);
         NT_CHECK(gemm_blocks(m, n_blocks, K, t, block_scratch_, T, add, s), "prefill GEMM over blocks rejected");
     }
 }

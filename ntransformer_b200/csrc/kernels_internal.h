@@ -569,7 +569,7 @@ struct BlockTokens { void* split = nullptr; void* sums = nullptr; float* scale =
 size_t block_tokens_bytes(int T, int K, bool fine);
 BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w /* null: x itself */, float eps, int T, int K, bool fine, cudaStream_t s);
 BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, bool fine, cudaStream_t s);
-BlockTokens resplit_tokens(void* workspace, const void* split, int T, int K, cudaStream_t s);      // of a plain split (split_activations' layout), in place too
+BlockTokens resplit_tokens(void* workspace, const void* hi, const void* lo, int T, int K, cudaStream_t s);      // of a plain split's rows, in place too
 // scratch: block_scratch_bytes(), whatever they hold, of one stream's.  fine: 64 columns to an accumulator, as exact as
 // the decode step's 24-bit integers, instead of 256
 // The matrices are read ahead of the wait for the launch before.  That is the one that laid the tokens out: it lets this one start only behind its own wait, when

@@ -641,6 +641,12 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
     for (int c = 0; c < KEEP; c++) { const int i = c * 2048 + 4 * tid; if (i < K) put(i, keep[c]); }
     for (int i = KEEP * 2048 + 4 * tid; i < K; i += 2048) put(i, value(i, none));
 }
+__global__ void __launch_bounds__(512) plain_tokens_kernel(float* __restrict__ scale, int rows, unsigned* __restrict__ count, int counts) {
+    pdl_wait();
+    pdl_launch_dependents();               // after the wait, as above
+    for (int i = threadIdx.x; i < rows; i += 512) scale[i] = 1.0f;
+    for (int i = threadIdx.x; i < counts; i += 512) count[i] = 0;
+}
 // silu(g) * u (gemm.cu:713-725's expression) straight into the split of the next product
 __global__ void __launch_bounds__(256) silu_split_kernel(uint2* __restrict__ hi, uint2* __restrict__ lo, const float4* __restrict__ g, const float4* __restrict__ u, size_t n4) {
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
@@ -709,8 +715,19 @@ BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, f
 BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, bool fine, cudaStream_t s) {
     return launch_split<TOK_SILU>(workspace, gate, up, 0.f, T, K, fine, s);
 }
-BlockTokens resplit_tokens(void* workspace, const void* split, int T, int K, cudaStream_t s) {
-    return launch_split<TOK_SPLIT>(workspace, static_cast<const float*>(split), reinterpret_cast<const float*>(static_cast<const __half*>(split) + padded(T) * (size_t)K), 0.f, T, K, false, s);
+BlockTokens resplit_tokens(void* workspace, const void* hi, const void* lo, int T, int K, cudaStream_t s) {
+    return launch_split<TOK_SPLIT>(workspace, static_cast<const float*>(hi), static_cast<const float*>(lo), 0.f, T, K, false, s);
+}
+// A plain split as it lies, for matrices without minima: it has no sums, and powers of 2^0
+static size_t plain_tokens_bytes(int T) { return padded(T) * sizeof(float) + (size_t)sm_count() * sizeof(unsigned); }
+static BlockTokens plain_tokens(void* memory, const void* split, int T, cudaStream_t s) {
+    BlockTokens t;
+    t.split = t.sums = const_cast<void*>(split);
+    t.scale = static_cast<float*>(memory);
+    t.count = reinterpret_cast<unsigned*>(t.scale + padded(T));
+    launch_k_pdl(true, plain_tokens_kernel, dim3(1), dim3(512), 0, s, t.scale, (int)padded(T), t.count, sm_count());
+    count_launch();
+    return t;
 }
 
 bool gemm_blocks_for_few(const GemvMat* mats, int n_mat, int tokens) {
@@ -779,16 +796,36 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     return true;
 }
 
-// The same over F32 tokens, or (x null) over tokens that split_activations laid out; what it needs beside them lies in memory of this call's
+// The same over F32 tokens, or (x null) over tokens that split_activations laid out; what it needs beside them is memory of this call, at most what a device keeps between
+// calls: long runs of tokens go through it in portions
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const float* norm_w, float eps, const void* split, bool fine, int T, bool add, cudaStream_t s) {
     if (T <= 0 || !gemm_blocks_supported(mats, n_mat, K) || (reinterpret_cast<uintptr_t>(x) & 15)) return false;
-    const size_t tokens = (block_tokens_bytes(T, K, fine && x) + 255) / 256 * 256;
-    CallMemory memory(tokens + block_scratch_bytes(), s);
-    uint8_t* mem = static_cast<uint8_t*>(memory.p);
-    if (!mem) return false;
-    uint8_t* scratch = mem + tokens;
-    const BlockTokens t = x ? split_tokens(mem, x, norm_w, eps, T, K, fine, s) : resplit_tokens(mem, split, T, K, s);
-    return gemm_blocks(mats, n_mat, K, t, scratch, T, add, s);
+    fine = fine && x;
+    bool as_it_lies = !x;
+    for (int i = 0; i < n_mat; i++) as_it_lies = as_it_lies && !has_mins(gemv_kq_format(mats[i].dtype));
+    auto up256 = [](size_t n) { return (n + 255) / 256 * 256; };
+    if (as_it_lies) {
+        const size_t front = up256(plain_tokens_bytes(T));
+        CallMemory memory(front + block_scratch_bytes(), s);
+        if (!memory.p) return false;
+        return gemm_blocks(mats, n_mat, K, plain_tokens(memory.p, split, T, s), static_cast<uint8_t*>(memory.p) + front, T, add, s);
+    }
+    auto front_of = [&](int tokens) { return up256(block_tokens_bytes(tokens, K, fine)); };
+    int portion = (T + 127) / 128 * 128;
+    for (int n = 2; portion > 128 && front_of(portion) + block_scratch_bytes() > CALL_MEMORY_KEPT; n++) portion = ((T + n - 1) / n + 127) / 128 * 128;
+    portion = std::min(portion, T);
+    CallMemory memory(front_of(portion) + block_scratch_bytes(), s);
+    if (!memory.p) return false;
+    const __half *hi = static_cast<const __half*>(split), *lo = hi + padded(T) * (size_t)K;
+    GemvMat m[3];
+    for (int t0 = 0; t0 < T; t0 += portion) {
+        const int n = std::min(portion, T - t0);
+        const size_t at = (size_t)t0 * K;
+        for (int i = 0; i < n_mat; i++) { m[i] = mats[i]; m[i].y += (size_t)t0 * mats[i].out; }
+        const BlockTokens t = x ? split_tokens(memory.p, x + at, norm_w, eps, n, K, fine, s) : resplit_tokens(memory.p, hi + at, lo + at, n, K, s);
+        if (!gemm_blocks(m, n_mat, K, t, static_cast<uint8_t*>(memory.p) + front_of(portion), n, add, s)) return false;
+    }
+    return true;
 }
 
 void silu_mul_split(void* workspace, const float* gate, const float* up, int rows, int cols, cudaStream_t s) {

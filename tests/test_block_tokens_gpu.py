@@ -12,7 +12,7 @@ from ntransformer_b200.dtypes import DType  # noqa: E402
 from ntransformer_b200.engine import Model  # noqa: E402
 from ntransformer_b200.model_spec import TINY  # noqa: E402
 from oracle import oracle as O  # noqa: E402
-from test_block_products_gpu import FORMATS, activations, arrays, matrix, rel, rows_product, stream  # noqa: E402
+from test_block_products_gpu import FORMATS, activations, arrays, blocks_product, matrix, rel, rows_product, stream  # noqa: E402
 
 pytestmark = [pytest.mark.gpu]
 
@@ -131,6 +131,56 @@ def test_a_token_s_product_is_the_same_however_many_share_the_call(dt):
         product([y], [W], [rows], [dt], x[:tokens].contiguous(), fine=True)
         got.append(y)
     assert all(torch.equal(y[:9], got[0]) for y in got) and torch.equal(got[3][:31], got[2])
+
+
+@pytest.mark.parametrize("dt", [DType.Q4_K_M, DType.Q6_K], ids=lambda d: d.name)
+@pytest.mark.parametrize("tokens", [700, 1025])
+def test_long_runs_go_through_the_kept_memory_in_portions(dt, tokens):
+    """14336 columns: 700 tokens are the most that the memory a device keeps between calls takes, or two portions with the third halves."""
+    rows, cols = 130, 14336
+    W, W64 = matrix(dt, rows, cols, 11)
+    x = activations(tokens, cols, 12)
+    ref = x.double() @ W64.T
+    for fine in (False, True):
+        y = torch.full((tokens + 1, rows), 7.0, device="cuda")
+        product([y], [W], [rows], [dt], x, fine)
+        assert rel(y[:tokens], ref) <= bound(dt, 64 if fine else 256) and (y[tokens] == 7.0).all()
+    y = torch.full((tokens + 1, rows), 7.0, device="cuda")
+    blocks_product([y], [W], [rows], [dt], x)
+    blocks_product([y], [W], [rows], [dt], x, add=True)
+    assert rel(y[:tokens], 2 * ref) <= bound(dt, 256) and (y[tokens] == 7.0).all()
+
+
+@pytest.mark.parametrize("dt", [DType.Q4_K_M, DType.Q6_K], ids=lambda d: d.name)
+def test_captured(dt):
+    tokens, rows, cols = 40, 300, 2048
+    W, _ = matrix(dt, rows, cols, 1)
+    x = activations(tokens, cols, 2)
+    ws = torch.empty(lib().nt_b200_gemm_f16_tc_workspace_bytes(tokens, cols), dtype=torch.uint8, device="cuda")
+    lib().nt_b200_split_activations(ws.data_ptr(), x.data_ptr(), tokens, cols, stream())
+    ys = [torch.zeros(tokens, rows, device="cuda") for _ in range(4)]
+    want = [torch.zeros(tokens, rows, device="cuda") for _ in range(2)]
+
+    def calls(a, b):
+        for y, of_ws in ((a, False), (b, True)):
+            c, w, o, d = arrays([y], [W], [rows], [dt])
+            if of_ws:
+                assert lib().nt_b200_gemm_blocks_ws(1, c, w, o, d, cols, ws.data_ptr(), tokens, 0, stream()) == 0
+            else:
+                assert lib().nt_b200_gemm_blocks(1, c, w, o, d, cols, x.data_ptr(), None, 0.0, tokens, 1, 0, stream()) == 0
+
+    calls(*want)
+    torch.cuda.synchronize()
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=side):
+        calls(ys[0], ys[1])
+        calls(ys[2], ys[3])
+    for _ in range(3):
+        for y in ys:
+            y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, want[i & 1]) for i, y in enumerate(ys))
 
 
 @pytest.mark.parametrize("mix", ["Q4_K_M", "Q8_0"])

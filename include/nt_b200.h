@@ -153,6 +153,8 @@ void   nt_b200_dequant_split(void* w_hi, void* w_lo, const void* W, int dtype, s
  * stores `set`.  nt_b200_wait_probe launches a wait that asks `tries` times for something that does not come (came_dev: device int, 0 afterwards). */
 int    nt_b200_wait_status(int set);
 void   nt_b200_wait_probe(unsigned tries, int* came_dev, void* stream);
+/* dst = src (bytes: a multiple of 4), by a launch that lets the next one start at once and writes only `nanoseconds` later: what is launched behind it must wait. */
+void   nt_b200_late_copy(void* dst, const void* src, size_t bytes, unsigned nanoseconds, void* stream);
 /* Memory that calls need beside their arguments (nt_b200_attention_decode, nt_b200_gemm_blocks*) is theirs or their stream's, in its order (captured: memory nodes of
  * the graph).  For each device up to 64 MB of it, and the buffers of up to 16 streams that decode, are kept for the next calls; this waits for the current device and
  * gives its back, as the end of a Model does. */

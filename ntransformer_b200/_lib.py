@@ -61,6 +61,7 @@ SIGNATURES = {
     "nt_b200_rmsnorm_split": (None, [_vp, _vp, _vp, _i, _i, C.c_float, _vp]),
     "nt_b200_dequant_split": (None, [_vp, _vp, _vp, _i, _sz, _i, _i, _vp]),
     "nt_b200_wait_status": (_i, [_i]),
+    "nt_b200_late_copy": (None, [_vp, _vp, _sz, C.c_uint, _vp]),
     "nt_b200_wait_probe": (None, [C.c_uint, _vp, _vp]),
     "nt_b200_trim_memory": (None, []),
     "nt_b200_launch_count": (C.c_ulonglong, []),

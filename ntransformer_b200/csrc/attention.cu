@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) decode_kernel
     extern __shared__ float smem_dyn[];
     pdl_wait();
     pdl_launch_dependents();
+    q = behind_wait(q); kc = behind_wait(kc); vc = behind_wait(vc); pos_dev = behind_wait(pos_dev);
     if (pos_dev) {                       // CUDA-graph replay: context length lives in device memory
         seq_len = *pos_dev + 1;
         split_len = max((seq_len + n_splits - 1) / n_splits, DYN_MIN_SPLIT);
@@ -190,6 +191,7 @@ __global__ void __launch_bounds__(128) decode_combine_kernel(float* __restrict__
     const int h = blockIdx.x;
     pdl_wait();
     pdl_launch_dependents();
+    scratch = behind_wait(scratch); pos_dev = behind_wait(pos_dev);
     seq_len += blockIdx.y;               // a run of tokens: blockIdx.y is the query
     scratch += (size_t)blockIdx.y * n_heads * n_splits * (hd + 2);
     out += (size_t)blockIdx.y * n_heads * hd;

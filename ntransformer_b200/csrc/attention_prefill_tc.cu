@@ -71,7 +71,7 @@ __device__ __noinline__ void row_alone(const TcAttn& p, int row, int head, int c
         const __half* kr = k + (size_t)min(k0 + lane, pos) * pitch;
 #pragma unroll 4
         for (int d = 0; d < HD; d += 2) {
-            const float2 x = __half22float2(*reinterpret_cast<const __half2*>(kr + d)), q = __ldg(reinterpret_cast<const float2*>(p.Q + at + d));
+            const float2 x = __half22float2(*reinterpret_cast<const __half2*>(kr + d)), q = *reinterpret_cast<const float2*>(p.Q + at + d);
             s = fmaf(q.x, x.x, fmaf(q.y, x.y, s));
         }
         s = k0 + lane <= pos ? s * p.scale * 1.4426950408889634f : -INFINITY;
@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
         constexpr int HK = TK / 2, HC = HD / 2;
         const int t = warp >> 3, quarter = warp & 3, half = (warp >> 2) & 1, r = quarter * 32 + lane, head = p.pairs_of_queries ? h0 : h0 + t;
         const int q0 = first_q + (p.pairs_of_queries ? t * TQ : 0), row = q0 + r;
+        const float* queries = behind_wait(p.Q);
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16, to = lanes + 384 + half * HC;
         uint8_t* mine = smem + 2 * t * S::Q;                      // the tile's queries
         {
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) prefill_tc_kernel(const __grid_
 #pragma unroll 8
             for (int i = 0; i < 16 / RI; i++) {
                 const int rr = quarter * 32 + half * 16 + i * RI + lane / LR;
-                const float4 x = __ldg(reinterpret_cast<const float4*>(p.Q + ((size_t)min(q0 + rr, p.seq_len - 1) * p.n_heads + head) * HD) + c);
+                const float4 x = __ldg(reinterpret_cast<const float4*>(queries + ((size_t)min(q0 + rr, p.seq_len - 1) * p.n_heads + head) * HD) + c);
                 float amax = fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
 #pragma unroll
                 for (int s = LR / 2; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, s));

@@ -61,6 +61,7 @@ __device__ float block_max(float v, float* red) {
 __global__ void quantize_x_kernel(const float* __restrict__ x, int8_t* __restrict__ xq, int K) {
     pdl_launch_dependents();
     pdl_wait();
+    x = behind_wait(x);
     const int blk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (blk * 32 >= K) return;
     quantize_block32(x[blk * 32 + lane], blk, lane, xq, K);
@@ -74,7 +75,8 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(void* __restrict__ yv, co
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float red[32];
-    const float* x = xin + (size_t)blockIdx.x * hidden;
+    const float* x = behind_wait(xin) + (size_t)blockIdx.x * hidden;
+    w = behind_wait(w);
     auto store = [&](int i, float v) {
         if (HALF_OUT) reinterpret_cast<__half*>(yv)[(size_t)blockIdx.x * hidden + i] = __float2half(v);
         else reinterpret_cast<float*>(yv)[(size_t)blockIdx.x * hidden + i] = v;
@@ -141,7 +143,8 @@ __global__ void rope_kernel(float* __restrict__ q, float* __restrict__ k, const 
     const int pair = li % half_dim, head = (li / half_dim) % n_h, sp = li / (half_dim * n_h);
     const float freq = 1.0f / powf(theta_base, (2.0f * pair) / head_dim);
     pdl_wait();
-    const int pos = positions[sp];
+    q = behind_wait(q); k = behind_wait(k);
+    const int pos = behind_wait(positions)[sp];
     float angle = pos * freq * freq_scale;
     float c = cosf(angle), sn = sinf(angle);
     float* d = (is_key ? k : q) + (size_t)sp * n_h * head_dim + (size_t)head * head_dim;
@@ -156,6 +159,7 @@ __global__ void kv_write_kernel(__half* __restrict__ kc, __half* __restrict__ vc
                                 const float* __restrict__ v, int seq_len, int row /* n_kv * hd */, int start_pos, int max_seq) {
     pdl_launch_dependents();
     pdl_wait();
+    k = behind_wait(k); v = behind_wait(v);
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= seq_len * row) return;
     const int s = idx / row, c = idx - s * row;
@@ -172,6 +176,7 @@ __global__ void __launch_bounds__(256) rope_kv_rows_kernel(float* __restrict__ q
                                                            int max_seq) {
     pdl_launch_dependents();
     pdl_wait();
+    q = behind_wait(q); k = behind_wait(k); v = behind_wait(v);
     const int half_dim = head_dim / 2, per_head = half_dim / 4, pos = start_pos + blockIdx.x;
     const int pair = threadIdx.x % per_head * 4;                   // 256 is a multiple of per_head
     float c[4], sn[4];
@@ -246,6 +251,7 @@ __global__ void rope_kv_decode_kernel(float* __restrict__ q, float* __restrict__
 __global__ void silu_mul_kernel(float* __restrict__ out, const float* __restrict__ gate, const float* __restrict__ up, int n) {
     pdl_launch_dependents();
     pdl_wait();
+    gate = behind_wait(gate); up = behind_wait(up);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) { float g = gate[i]; float silu = g / (1.0f + expf(-g)); out[i] = silu * up[i]; }
 }
@@ -259,7 +265,7 @@ __global__ void copy_kernel(float* __restrict__ dst, const float* __restrict__ s
     pdl_launch_dependents();
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[i];
+    if (i < n) dst[i] = behind_wait(src)[i];
 }
 // single-block cosine similarity (elementwise.cu:46-84): dot / (|a||b|), 0 when the denominator is <= 1e-8
 __global__ void __launch_bounds__(1024) cosine_kernel(float* result, const float* __restrict__ a, const float* __restrict__ b, int n) {

@@ -180,6 +180,7 @@ __global__ void __launch_bounds__(GW * 32) gemv_generic_kernel(float* __restrict
     const int row0 = (blockIdx.x * GW + warp) * RPW;
     pdl_launch_dependents();
     pdl_wait();
+    W = behind_wait(W); x = behind_wait(x); y = behind_wait(y);
 #pragma unroll
     for (int r = 0; r < RPW; r++) {
         int row = row0 + r;
@@ -212,6 +213,7 @@ __global__ void __launch_bounds__(F16_WARPS * 32) gemv_f16_kernel(float* __restr
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     pdl_launch_dependents();
     pdl_wait();
+    x = behind_wait(x); y = behind_wait(y);                        // (W by volatile asm)
     for (int i = threadIdx.x * 4; i < in; i += F16_WARPS * 32 * 4) *reinterpret_cast<float4*>(xs + i) = *reinterpret_cast<const float4*>(x + i);
     __syncthreads();
     const int n8 = in / 8;

@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
     float* red = reinterpret_cast<float*>(smem + SM_RED);
     float rms_inv = 1.0f;
     if (p.x_f32) {
+        const float *x_f32 = behind_wait(p.x_f32), *norm_w = behind_wait(p.norm_w);
         float ss = 0.f;
         constexpr int AHEAD = 4;                                // vectors of 8 in flight for each thread
         for (int base = 0; base < K / 8; base += AHEAD * CTHREADS) {
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
 #pragma unroll
             for (int j = 0; j < AHEAD; j++) {
                 const int t8 = base + j * CTHREADS + tid;
-                if (t8 < K / 8) { v[j][0] = __ldcg(reinterpret_cast<const float4*>(p.x_f32) + 2 * t8); v[j][1] = __ldcg(reinterpret_cast<const float4*>(p.x_f32) + 2 * t8 + 1); }
+                if (t8 < K / 8) { v[j][0] = __ldcg(reinterpret_cast<const float4*>(x_f32) + 2 * t8); v[j][1] = __ldcg(reinterpret_cast<const float4*>(x_f32) + 2 * t8 + 1); }
             }
 #pragma unroll
             for (int j = 0; j < AHEAD; j++) {
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
                 if (t8 >= K / 8) break;                         // K / 8 is a multiple of 32: whole warps leave together
                 float x[8] = {v[j][0].x, v[j][0].y, v[j][0].z, v[j][0].w, v[j][1].x, v[j][1].y, v[j][1].z, v[j][1].w};
                 if (p.norm_w) {
-                    const float4 a = __ldg(reinterpret_cast<const float4*>(p.norm_w) + 2 * t8), b = __ldg(reinterpret_cast<const float4*>(p.norm_w) + 2 * t8 + 1);
+                    const float4 a = __ldg(reinterpret_cast<const float4*>(norm_w) + 2 * t8), b = __ldg(reinterpret_cast<const float4*>(norm_w) + 2 * t8 + 1);
                     const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
                     for (int i = 0; i < 8; i++) { ss = fmaf(x[i], x[i], ss); x[i] = __fmul_rn(x[i], w[i]); }
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(TEAMS * (KW + 1) * 32, SM_WARPS / (TEAMS * KW)
     } else {
         // the public xq form: x = scale * (q1 * 16384 + q2 * 128 + q3), planes in 16-byte columns swizzled as xquant.cuh has it.  Times 4 the
         // integer splits into balanced bytes without a loss.
-        const uint8_t* xq = reinterpret_cast<const uint8_t*>(p.xq);
+        const uint8_t* xq = reinterpret_cast<const uint8_t*>(behind_wait(p.xq));
         const float* fs = reinterpret_cast<const float*>(xq + 3 * (size_t)K);
         for (int e = 4 * tid; e < K; e += 4 * CTHREADS) {
             const uint32_t o = xq_swizzle((uint32_t)e);

@@ -523,7 +523,8 @@ void mlstm_token(float* out, const float* q, const float* k, const float* v, con
                  const float* norm, float* state, float* m, float cap, float q_scale, float eps, int heads, int dim, int vdim, const int* pos_dev, int p0, cudaStream_t s);
 
 // Programmatic dependent launch (PDL): kernels launched with cudaLaunchAttributeProgrammaticStreamSerialization have their prologue (barrier init, TMA weight
-// prefetch) overlap the tail of the launch before; every kernel executes griddepcontrol.wait before it touches data produced upstream, so ordering is unchanged.
+// prefetch) overlap the tail of the launch before; every kernel executes griddepcontrol.wait before it touches data produced upstream, so ordering is unchanged;
+// what it reads just behind the wait it reads through behind_wait (ring.cuh).
 // This thread's launches:
 //   Boundary (as it is by itself)  launch_k_pdl(true, ...) is programmatic, launch_k is not, and no kernel reads weights ahead of its wait (the launch before may have
 //                                  written them; gemm_blocks does, and says why it may).  Call by call, a launch otherwise waits for the one before to drain and then starts

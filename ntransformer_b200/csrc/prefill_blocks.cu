@@ -365,6 +365,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         uint32_t db = 0, dpar = 0, slot = 0, spar = 0;
         Place q = start();
         pdl_wait();
+        const float* token_scale = behind_wait(p.scale);
         for (int u = u0; u < u1;) {
             const int sums = 4 / p.kc, chunks = sums + (MINS && mins_of(q.mi) ? 1 : 0);
             const int seg0 = u, end = min(u1, u + (NB - q.b));
@@ -452,7 +453,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
             }
             if (write && row < rows && !word_set(dead)) {          // a warp stores 128 contiguous bytes for each token
                 float* o = p.mat[q.mi].C + (size_t)(q.t0 + 16 * half) * rows + row;
-                const float* ts = p.scale + q.t0 + 16 * half;
+                const float* ts = token_scale + q.t0 + 16 * half;
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
 #pragma unroll

@@ -49,6 +49,13 @@ __device__ __forceinline__ int dp4a_ss(int a_s8x4, int b_s8x4, int c) {
 }
 // Programmatic dependent launch: wait for the producer grid / let dependents start.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// p behind a pdl_wait(): loads through a const __restrict__ parameter count as loads of what nothing writes, and the compiler may take them ahead of the wait; those
+// through this pointer it may not.  (By way of the global address, so that they stay loads from global memory.)
+template <class T> __device__ __forceinline__ T* behind_wait(T* p) {
+    size_t at = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(at) : : "memory");
+    return static_cast<T*>(__cvta_global_to_generic(at));
+}
 // Hint: bring the 128-byte lines of [p, p + bytes) into L2, the lines shared out over `n` threads (this one is `i`).  Used in front of pdl_wait()
 // on data no kernel of the running step writes (weights, older state): the fetch from HBM overlaps the producer grid's tail.
 __device__ __forceinline__ void l2_prefetch(const void* p, size_t bytes, int i, int n) {

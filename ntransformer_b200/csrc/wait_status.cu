@@ -31,6 +31,13 @@ __global__ void wait_probe_kernel(unsigned* status, unsigned tries, int* came) {
     wait_phase(&bar, 0, status, tries);
     if (threadIdx.x == 0) *came = tries != 0;
 }
+// lets the next launch start, and writes only then
+__global__ void __launch_bounds__(1024) late_copy_kernel(uint32_t* dst, const uint32_t* src, size_t words, unsigned nanoseconds) {
+    pdl_launch_dependents();
+    pdl_wait();
+    for (unsigned t = 0; t < nanoseconds; t += 1000) __nanosleep(1000);
+    for (size_t i = threadIdx.x; i < words; i += 1024) dst[i] = src[i];
+}
 
 }  // namespace
 
@@ -45,6 +52,11 @@ int nt_b200_wait_status(int set) {
     const int was = (int)*w;
     if (set >= 0) *w = (unsigned)set;
     return was;
+}
+void nt_b200_late_copy(void* dst, const void* src, size_t bytes, unsigned nanoseconds, void* stream) {
+    nt::b200::launch_k_pdl(true, nt::b200::late_copy_kernel, dim3(1), dim3(1024), 0, static_cast<cudaStream_t>(stream), static_cast<uint32_t*>(dst), static_cast<const uint32_t*>(src),
+                           bytes / 4, nanoseconds);
+    nt::b200::count_launch();
 }
 void nt_b200_wait_probe(unsigned tries, int* came_dev, void* stream) {
     nt::b200::wait_probe_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(nt::b200::wait_status(), tries, came_dev);

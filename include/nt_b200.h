@@ -157,7 +157,7 @@ void   nt_b200_wait_probe(unsigned tries, int* came_dev, void* stream);
 void   nt_b200_late_copy(void* dst, const void* src, size_t bytes, unsigned nanoseconds, void* stream);
 /* Memory that calls need beside their arguments (nt_b200_attention_decode, nt_b200_gemm_blocks*) is theirs or their stream's, in its order (captured: memory nodes of
  * the graph).  For each device up to 64 MB of it, and the buffers of up to 16 streams that decode, are kept for the next calls; this waits for the current device and
- * gives its back, as the end of a Model does. */
+ * gives its back, as the end of the last Model does. */
 void   nt_b200_trim_memory(void);
 unsigned long long nt_b200_launch_count(void);   /* kernels launched by this library so far */
 unsigned long long nt_b200_programmatic_count(void);   /* those launched so that they may start while the one before ends (NT_B200_NO_PDL: none of a Model's) */

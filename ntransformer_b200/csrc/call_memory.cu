@@ -102,6 +102,10 @@ void trim_call_memory() {
     cudaGetLastError();
 }
 
+static std::atomic<int> g_users{0};
+CallMemoryUser::CallMemoryUser() { g_users.fetch_add(1); }
+CallMemoryUser::~CallMemoryUser() { if (g_users.fetch_sub(1) == 1) trim_call_memory(); }
+
 }}  // namespace nt::b200
 
 extern "C" void nt_b200_trim_memory(void) { nt::b200::trim_call_memory(); }

@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstring>
 #include <cstdlib>
+#include <optional>
 #include <atomic>
 #include <chrono>
 #include <thread>
@@ -72,10 +73,11 @@ Model::~Model() {
                     (void*)attn_tickets_,
                     (void*)argmax_dev_, (void*)recent_dev_})
         if (p) cudaFree(p);
-    for (void* p : {(void*)pf_.x, (void*)pf_.q, (void*)pf_.k, (void*)pf_.v, (void*)pf_.attn, pf_.ws, pf_.ws2, (void*)pf_.tok, (void*)pf_.pos,
-                    (void*)pf_.g, (void*)pf_.u, pf_.whi, pf_.wlo, (void*)sb_.x, (void*)sb_.q, (void*)sb_.k, (void*)sb_.v, (void*)sb_.attn, (void*)sb_.g, (void*)sb_.u, sb_.ws,
-                    block_scratch_, (void*)sb_.scratch, (void*)sb_.tok, (void*)sb_.pos})
-        if (p) cudaFree(p);
+    for (void* p : {pf_arena_, sb_arena_}) if (p) cudaFree(p);
+    if (!pf_arena_)                                                // a layer-spec model's
+        for (void* p : {(void*)pf_.x, (void*)pf_.q, (void*)pf_.k, (void*)pf_.v, (void*)pf_.attn, pf_.ws, pf_.ws2, (void*)pf_.tok, (void*)pf_.pos, (void*)pf_.g, (void*)pf_.u,
+                        pf_.whi, pf_.wlo})
+            if (p) cudaFree(p);
     for (size_t i = 0; i < kcs_.size(); i++) if (kcs_[i] && (cache_owned_.empty() || cache_owned_[i])) { cudaFree(kcs_[i]); cudaFree(vcs_[i]); }
     for (void* p : {(void*)pf_.h, (void*)pf_.tmp, pf_.hws, (void*)want_out_, (void*)pf_.xs, (void*)pf_.maps, (void*)pf_.sel, (void*)pf_.work, (void*)pf_.wt,
                     (void*)pf_.sgate, (void*)pf_.act_rows, (void*)pf_.y_rows, (void*)streams_, (void*)sub_y_, (void*)maps_out_, (void*)moe_sel_,
@@ -97,7 +99,6 @@ Model::~Model() {
                     (void*)par_dec_.mix[4]}) if (p) cudaFree(p);
     if (argmax_host_) cudaFreeHost(argmax_host_);
     if (stream_) cudaStreamDestroy(stream_);
-    trim_call_memory();
 }
 
 void Model::release_graphs() {
@@ -794,39 +795,39 @@ bool Model::short_batch_ok(int seq_len, int start_pos) const {
     return chain_ok();
 }
 
-// What the GEMM over blocks keeps shared tiles in, for every caller on this model's stream; false: no room
-bool Model::ensure_block_scratch() {
-    if (block_scratch_) return true;
-    void* p = nullptr;
-    if (cudaMalloc(&p, block_scratch_bytes()) != cudaSuccess) { cudaGetLastError(); return false; }
-    block_scratch_ = p;
-    return true;
-}
+// Buffers cut out of one allocation: each of a dozen of its own costs the first prompt of a model as much as a launch of it
+struct Cuts {
+    struct Cut { void** p; size_t bytes; };
+    std::vector<Cut> list;
+    template <class T> void want(T*& p, size_t bytes) { p = nullptr; list.push_back({reinterpret_cast<void**>(&p), bytes}); }
+    size_t total() const { size_t n = 0; for (const Cut& c : list) n += (c.bytes + 255) / 256 * 256; return n; }
+    void place(void* base) { uint8_t* at = static_cast<uint8_t*>(base); for (const Cut& c : list) { *c.p = at; at += (c.bytes + 255) / 256 * 256; } }
+};
 
 // false: no room for them; the caller takes the tokens one by one, which needs none
 bool Model::ensure_short_buffers() {
-    if (sb_.x) return true;
-    if (!ensure_block_scratch()) return false;
+    if (sb_arena_) return true;
     const size_t T = SHORT_CHUNK, hidden = (size_t)cfg_.hidden_size, qdim = (size_t)nh_l_ * cfg_.head_dim, kvdim = (size_t)nkv_l_ * cfg_.head_dim, f = sizeof(float);
-    const size_t bytes[11] = {T * hidden * f, T * qdim * f, T * kvdim * f, T * kvdim * f, T * qdim * f, T * (size_t)inter_l_ * f, T * (size_t)inter_l_ * f,
-                              std::max(block_tokens_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_), true),
-                                       gemv_rows_bytes((int)T, (int)std::max(std::max(hidden, qdim), (size_t)inter_l_))),
-                              attention_rows_scratch_floats((int)T, cfg_.max_seq_len, nh_l_, nkv_l_, cfg_.head_dim) * f, T * sizeof(int), T * sizeof(int)};
-    void* got[11] = {};
-    for (int i = 0; i < 11; i++)
-        if (cudaMalloc(&got[i], std::max<size_t>(bytes[i], 1)) != cudaSuccess) {
-            cudaGetLastError();
-            for (int j = 0; j < i; j++) cudaFree(got[j]);
-            return false;
-        }
-    sb_.x = static_cast<float*>(got[0]); sb_.q = static_cast<float*>(got[1]); sb_.k = static_cast<float*>(got[2]); sb_.v = static_cast<float*>(got[3]);
-    sb_.attn = static_cast<float*>(got[4]); sb_.g = static_cast<float*>(got[5]); sb_.u = static_cast<float*>(got[6]); sb_.ws = got[7]; sb_.scratch = static_cast<float*>(got[8]);
-    sb_.tok = static_cast<int*>(got[9]); sb_.pos = static_cast<int*>(got[10]);
+    const int widest = (int)std::max(std::max(hidden, qdim), (size_t)inter_l_);
+    Cuts c;
+    c.want(sb_.x, T * hidden * f); c.want(sb_.q, T * qdim * f); c.want(sb_.k, T * kvdim * f); c.want(sb_.v, T * kvdim * f); c.want(sb_.attn, T * qdim * f);
+    c.want(sb_.g, T * (size_t)inter_l_ * f); c.want(sb_.u, T * (size_t)inter_l_ * f);
+    c.want(sb_.ws, std::max(block_tokens_bytes((int)T, widest, true), gemv_rows_bytes((int)T, widest)));
+    c.want(sb_.scratch, attention_rows_scratch_floats((int)T, cfg_.max_seq_len, nh_l_, nkv_l_, cfg_.head_dim) * f);
+    c.want(sb_.tok, T * sizeof(int)); c.want(sb_.pos, T * sizeof(int));
+    if (cudaMalloc(&sb_arena_, c.total()) != cudaSuccess) { cudaGetLastError(); sb_arena_ = nullptr; return false; }
+    c.place(sb_arena_);
     return true;
 }
 
-void Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
+// false: no room for the GEMM's scratch; nothing launched
+bool Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
     cudaStream_t s = stream_;
+    std::optional<CallMemory> block_scratch;                       // where a chunk is more than a pass of gemv_rows
+    if (seq_len > 8) {
+        block_scratch.emplace(block_scratch_bytes(std::min(SHORT_CHUNK, seq_len)), s);
+        if (!block_scratch->p) return false;
+    }
     const int hidden = cfg_.hidden_size, hd = cfg_.head_dim, max_seq = cfg_.max_seq_len, qdim = nh_l_ * hd;
     const size_t kv_stride = (size_t)max_seq * nkv_l_ * hd;
     int T = 0;
@@ -843,7 +844,7 @@ void Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
             return false;
         }
         const BlockTokens t = up ? silu_split_tokens(sb_.ws, x, up, T, K, true, s) : split_tokens(sb_.ws, x, norm, cfg_.norm_eps, T, K, true, s);
-        NT_CHECK(gemm_blocks(m, n, K, t, block_scratch_, T, ep == GEMV_ADD, s), "GEMM of a few tokens over blocks rejected");
+        NT_CHECK(gemm_blocks(m, n, K, t, block_scratch->p, T, ep == GEMV_ADD, s), "GEMM of a few tokens over blocks rejected");
         return ep == GEMV_SWIGLU;
     };
     for (int c0 = 0; c0 < seq_len; c0 += T) {
@@ -871,6 +872,7 @@ void Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
     }
     copy(hidden_, sb_.x + (size_t)(T - 1) * hidden, hidden, s);
     step_head(s, true);
+    return true;
 }
 
 bool Model::f16_direct(const Weight& w) const {
@@ -906,7 +908,7 @@ void Model::prefill_gemms(float* const* C, void* ws, const float* x, const float
     if (!together || !gemm_f16_tc_multi_ws(c, ws, W, N, n_plain, T, K, s)) for (int i = 0; i < n_plain; i++) prefill_gemm(c[i], ws, *plain[i], T, add, s);
     if (n_blocks) {
         const BlockTokens t = x ? split_tokens(ws, x, norm_w, cfg_.norm_eps, T, K, false, s) : resplit_tokens(ws, ws, static_cast<uint8_t*>(ws) + gemm_f16_tc_workspace_bytes(T, K) / 2, T, K, s);
-        NT_CHECK(gemm_blocks(m, n_blocks, K, t, block_scratch_, T, add, s), "prefill GEMM over blocks rejected");
+        NT_CHECK(gemm_blocks(m, n_blocks, K, t, pf_scratch_, T, add, s), "prefill GEMM over blocks rejected");
     }
 }
 
@@ -924,29 +926,31 @@ void Model::prefill_gemm(float* C, const void* ws, const Weight& w, int T, bool 
 void Model::ensure_prefill_buffers(int tokens) {
     if (tokens <= pf_.cap) return;
     NT_CUDA_CHECK(cudaStreamSynchronize(stream_));
-    for (void* p : {(void*)pf_.x, (void*)pf_.q, (void*)pf_.k, (void*)pf_.v, (void*)pf_.attn, pf_.ws, pf_.ws2, (void*)pf_.tok, (void*)pf_.pos,
-                    (void*)pf_.g, (void*)pf_.u, pf_.whi, pf_.wlo})
-        if (p) cudaFree(p);
-    pf_.g = pf_.u = nullptr; pf_.whi = pf_.wlo = nullptr;
+    if (pf_arena_) cudaFree(pf_arena_);
+    pf_arena_ = nullptr;
     const size_t T = (size_t)((tokens + 127) / 128 * 128);
     const size_t hidden = (size_t)cfg_.hidden_size, qdim = (size_t)nh_l_ * cfg_.head_dim, kvdim = (size_t)nkv_l_ * cfg_.head_dim;
-    pf_.x = dmalloc<float>(T * hidden);
-    pf_.q = dmalloc<float>(T * qdim);    pf_.k = dmalloc<float>(T * kvdim);   pf_.v = dmalloc<float>(T * kvdim);
-    pf_.attn = dmalloc<float>(T * qdim);
-    pf_.ws = dmalloc<uint8_t>(block_tokens_bytes((int)T, (int)std::max(hidden, qdim), false));
-    pf_.ws2 = dmalloc<uint8_t>(block_tokens_bytes((int)T, inter_l_, false));
-    pf_.tok = dmalloc<int>(T);           pf_.pos = dmalloc<int>(T);
+    const size_t f = sizeof(float);
+    Cuts c;
+    c.want(pf_.x, T * hidden * f);
+    c.want(pf_.q, T * qdim * f); c.want(pf_.k, T * kvdim * f); c.want(pf_.v, T * kvdim * f);
+    c.want(pf_.attn, T * qdim * f);
+    c.want(pf_.ws, block_tokens_bytes((int)T, (int)std::max(hidden, qdim), false));
+    c.want(pf_.ws2, block_tokens_bytes((int)T, inter_l_, false));
+    c.want(pf_.tok, T * sizeof(int)); c.want(pf_.pos, T * sizeof(int));
     size_t w_elems = 0;                  // largest matrix that needs the dequantised scratch pair
-    bool swiglu_unfused = false, any_blocks = false;
+    bool swiglu_unfused = false;
+    any_blocks_ = false;
     for (const LayerWeights& L : layers_) {
         for (const Weight* w : {&L.wq, &L.wk, &L.wv, &L.wo, &L.gate, &L.up, &L.down})
-            if (blocks_direct(*w)) any_blocks = true;
+            if (blocks_direct(*w)) any_blocks_ = true;
             else if (!f16_direct(*w)) w_elems = std::max(w_elems, (size_t)w->rows * (size_t)w->cols);
         swiglu_unfused = swiglu_unfused || !f16_direct(L.gate) || !f16_direct(L.up);
     }
-    if (any_blocks) NT_CHECK(ensure_block_scratch(), "no room for the scratch of the prompt GEMM over blocks");
-    if (w_elems) { pf_.whi = dmalloc<uint16_t>(w_elems); pf_.wlo = dmalloc<uint16_t>(w_elems); }
-    if (swiglu_unfused) { pf_.g = dmalloc<float>(T * (size_t)inter_l_); pf_.u = dmalloc<float>(T * (size_t)inter_l_); }
+    if (w_elems) { c.want(pf_.whi, w_elems * sizeof(uint16_t)); c.want(pf_.wlo, w_elems * sizeof(uint16_t)); }
+    if (swiglu_unfused) { c.want(pf_.g, T * (size_t)inter_l_ * f); c.want(pf_.u, T * (size_t)inter_l_ * f); }
+    pf_arena_ = dmalloc<uint8_t>(c.total());
+    c.place(pf_arena_);
     pf_.cap = (int)T;
 }
 
@@ -957,6 +961,12 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
     const float scale = 1.0f / sqrtf((float)hd);
     const size_t kv_stride = (size_t)max_seq * nkv_l_ * hd;
     ensure_prefill_buffers(std::min(seq_len, PREFILL_CHUNK));
+    std::optional<CallMemory> scratch;
+    if (any_blocks_) {
+        scratch.emplace(block_scratch_bytes(std::min(seq_len, PREFILL_CHUNK)), s);
+        NT_CHECK(scratch->p, "no room for the scratch of the prompt GEMM over blocks");
+        pf_scratch_ = scratch->p;
+    }
     int last_rows = 0;
     for (int c0 = 0, T = 0; c0 < seq_len; c0 += T) {
         // A ragged tail of 1..15 tokens would miss the tiled attention kernel's 16-token minimum (and the per-query kernel it
@@ -993,7 +1003,7 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
                 prefill_gemms(gu_out, pf_.ws, pf_.x, L.ffn_norm, gu, 2, T, false, s);
                 if (blocks_direct(L.down)) {
                     GemvMat m; m.W = down->ptr; m.y = pf_.x; m.out = down->rows; m.dtype = down->dtype; m.row_pitch = down->pitch;
-                    NT_CHECK(gemm_blocks(&m, 1, inter, silu_split_tokens(pf_.ws2, pf_.g, pf_.u, T, inter, false, s), block_scratch_, T, true, s), "prefill GEMM over blocks rejected");
+                    NT_CHECK(gemm_blocks(&m, 1, inter, silu_split_tokens(pf_.ws2, pf_.g, pf_.u, T, inter, false, s), pf_scratch_, T, true, s), "prefill GEMM over blocks rejected");
                 } else {
                     silu_mul_split(pf_.ws2, pf_.g, pf_.u, T, inter, s);
                     prefill_gemm(pf_.x, pf_.ws2, L.down, T, true, s);
@@ -1027,7 +1037,7 @@ void Model::forward_async(const int* tokens, int seq_len, int start_pos) {
     if (cfg_.layer_spec()) {
         if (prefill_min_tokens_ > 0 && seq_len >= prefill_min_tokens_ && !getenv("NT_B200_NO_BATCHED_PREFILL")) { prefill_spec(tokens, seq_len, start_pos); return; }
     } else if (batched_prefill_ok(seq_len, start_pos)) { prefill_batched(tokens, seq_len, start_pos); return; }
-    else if (short_batch_ok(seq_len, start_pos) && ensure_short_buffers()) { prefill_short(tokens, seq_len, start_pos); return; }
+    else if (short_batch_ok(seq_len, start_pos) && ensure_short_buffers() && prefill_short(tokens, seq_len, start_pos)) return;
     size_t w = 0;
     for (int t = 0; t < seq_len; t++) {
         int tok = tokens[t];

@@ -168,10 +168,11 @@ public:
     bool short_batch_ok(int seq_len, int start_pos) const;
     bool blocks_direct(const Weight& w) const;
     void prefill_gemms(float* const* C, void* ws, const float* x, const float* norm_w, const Weight* const* w, int n, int T, bool add, cudaStream_t s);
-    bool ensure_block_scratch();
-    void* block_scratch_ = nullptr;
+    void *pf_arena_ = nullptr, *sb_arena_ = nullptr;               // pf_ (but a layer-spec model's) and sb_ lie in
+    bool any_blocks_ = false;                                     // prompts go through the GEMM over blocks
+    void* pf_scratch_ = nullptr;                                   // its scratch, for the length of a prompt
     bool ensure_short_buffers();
-    void prefill_short(const int* tokens, int seq_len, int start_pos);
+    bool prefill_short(const int* tokens, int seq_len, int start_pos);
     struct { float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *g = nullptr, *u = nullptr, *scratch = nullptr; void* ws = nullptr;
              int *tok = nullptr, *pos = nullptr; } sb_;       // a few tokens together
     void clear_kv();
@@ -356,6 +357,7 @@ private:
     int prefill_min_tokens_ = 32;
 
     bool use_graph_ = true;
+    CallMemoryUser call_memory_user_;
     bool use_pdl_ = true;
     cudaGraphExec_t g_full_ = nullptr, g_body_ = nullptr;
     int n_full_ = 0, n_body_ = 0;        // kernels per graph replay

@@ -138,6 +138,12 @@ struct StreamMemory {
     StreamMemory& operator=(const StreamMemory&) = delete;
 };
 void trim_call_memory();                              // what the current device keeps
+struct CallMemoryUser {                               // the last of these to go trims it
+    CallMemoryUser();
+    ~CallMemoryUser();
+    CallMemoryUser(const CallMemoryUser&) = delete;
+    CallMemoryUser& operator=(const CallMemoryUser&) = delete;
+};
 // the form that attention_prefill takes: a query at a time, mma.sync, tcgen05
 enum : int { PREFILL_QUERIES = 0, PREFILL_MMA = 1, PREFILL_TC = 2 };
 int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq);
@@ -571,11 +577,11 @@ size_t block_tokens_bytes(int T, int K, bool fine);
 BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w /* null: x itself */, float eps, int T, int K, bool fine, cudaStream_t s);
 BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, bool fine, cudaStream_t s);
 BlockTokens resplit_tokens(void* workspace, const void* hi, const void* lo, int T, int K, cudaStream_t s);      // of a plain split's rows, in place too
-// scratch: block_scratch_bytes(), whatever they hold, of one stream's.  fine: 64 columns to an accumulator, as exact as
+// scratch: block_scratch_bytes() for as many tokens or more, whatever they hold, of one stream's.  fine: 64 columns to an accumulator, as exact as
 // the decode step's 24-bit integers, instead of 256
 // The matrices are read ahead of the wait for the launch before.  That is the one that laid the tokens out: it lets this one start only behind its own wait, when
 // whatever wrote the matrices is done.  No other launch comes between the two.
-size_t block_scratch_bytes();
+size_t block_scratch_bytes(int T);
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, int T, bool add, cudaStream_t s);
 // Whether a few tokens are better served here (fine) than by gemv_rows: from two of its passes on (layers of an 8B model in Q4_K_M, 4 layers and head: 8 tokens
 // 771 us there, 900 here; 9 tokens 1025, 908; 31 tokens 1586, 973), and only where the error is no larger: not in Q8_0 and Q4_0, whose weights are pairs of halves here

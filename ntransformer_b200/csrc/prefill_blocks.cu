@@ -684,7 +684,9 @@ bool gemm_blocks_supported(const GemvMat* mats, int n_mat, int K) { return gemv_
 static size_t parts_bytes(int T, int K, bool fine) { return gemm_f16_tc_workspace_bytes(T, K) / 2 * (fine ? 3 : 2); }
 static size_t sums_bytes(int T, int K, bool fine) { return padded(T) * ((size_t)K / 8) * (fine ? 2 : 1); }
 size_t block_tokens_bytes(int T, int K, bool fine) { return parts_bytes(T, K, fine) + sums_bytes(T, K, fine) + padded(T) * sizeof(float) + (size_t)sm_count() * sizeof(unsigned); }
-size_t block_scratch_bytes() { return (size_t)sm_count() * 2 * 128 * NT_MAX * sizeof(float); }
+// tokens of a tile
+static int tile_tokens(int T) { const int cols = (T + NT_MAX - 1) / NT_MAX; return ((T + cols - 1) / cols + 15) / 16 * 16; }
+size_t block_scratch_bytes(int T) { return (size_t)sm_count() * 2 * 128 * (T > NT_MAX ? NT_MAX : tile_tokens(T)) * sizeof(float); }
 
 BlockTokens block_tokens(void* workspace, int T, int K, bool fine) {
     BlockTokens t;
@@ -759,7 +761,7 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     }
     const bool mins = mask & 3, pairs = mask & 28;
     p.cols = (T + NT_MAX - 1) / NT_MAX;
-    p.NT = ((T + p.cols - 1) / p.cols + 15) / 16 * 16;
+    p.NT = tile_tokens(T);
     p.units = tiles * p.cols * p.NB;
     // tensor memory: buffers of sums, expanded k-blocks, 8 columns of minima.  Shared memory: the same stages of tokens, and blocks of W behind them (the deeper the
     // fewer tokens there are: weights from HBM are then what bounds)
@@ -807,15 +809,15 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const fl
     auto up256 = [](size_t n) { return (n + 255) / 256 * 256; };
     if (as_it_lies) {
         const size_t front = up256(plain_tokens_bytes(T));
-        CallMemory memory(front + block_scratch_bytes(), s);
+        CallMemory memory(front + block_scratch_bytes(T), s);
         if (!memory.p) return false;
         return gemm_blocks(mats, n_mat, K, plain_tokens(memory.p, split, T, s), static_cast<uint8_t*>(memory.p) + front, T, add, s);
     }
     auto front_of = [&](int tokens) { return up256(block_tokens_bytes(tokens, K, fine)); };
     int portion = (T + 127) / 128 * 128;
-    for (int n = 2; portion > 128 && front_of(portion) + block_scratch_bytes() > CALL_MEMORY_KEPT; n++) portion = ((T + n - 1) / n + 127) / 128 * 128;
+    for (int n = 2; portion > 128 && front_of(portion) + block_scratch_bytes(portion) > CALL_MEMORY_KEPT; n++) portion = ((T + n - 1) / n + 127) / 128 * 128;
     portion = std::min(portion, T);
-    CallMemory memory(front_of(portion) + block_scratch_bytes(), s);
+    CallMemory memory(front_of(portion) + block_scratch_bytes(portion), s);
     if (!memory.p) return false;
     const __half *hi = static_cast<const __half*>(split), *lo = hi + padded(T) * (size_t)K;
     GemvMat m[3];

@@ -155,18 +155,28 @@ __global__ void rope_kernel(float* __restrict__ q, float* __restrict__ k, const 
 }
 
 // ---- KV-cache write: F32 -> F16 RN at [start_pos + s] (attention.cu:316-342) ----
-__global__ void kv_write_kernel(__half* __restrict__ kc, __half* __restrict__ vc, const float* __restrict__ k,
+// EACH elements to a thread, a block's width apart: a block costs its start and its wait, which long runs of one-element threads are bound by (copy of 64 M: 272 us, 184 without the
+// wait)
+template <int EACH>
+__global__ void __launch_bounds__(256) kv_write_kernel(__half* __restrict__ kc, __half* __restrict__ vc, const float* __restrict__ k,
                                 const float* __restrict__ v, int seq_len, int row /* n_kv * hd */, int start_pos, int max_seq) {
     pdl_launch_dependents();
     pdl_wait();
     k = behind_wait(k); v = behind_wait(v);
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= seq_len * row) return;
-    const int s = idx / row, c = idx - s * row;
-    const int cp = start_pos + s;
-    if (cp >= max_seq) return;                       // silently dropped, like attention.cu:336
-    kc[(size_t)cp * row + c] = __float2half(k[idx]);
-    vc[(size_t)cp * row + c] = __float2half(v[idx]);
+    const int i0 = blockIdx.x * (256 * EACH) + threadIdx.x;
+    // rows behind the cache are silently dropped, like attention.cu:336
+    const long long total = min((long long)seq_len * row, max(0ll, (long long)max_seq - start_pos) * row);
+    float a[EACH], b[EACH];
+#pragma unroll
+    for (int e = 0; e < EACH; e++) { const int idx = i0 + 256 * e; if (idx < total) { a[e] = k[idx]; b[e] = v[idx]; } }
+#pragma unroll
+    for (int e = 0; e < EACH; e++) {
+        const int idx = i0 + 256 * e;
+        if (idx >= total) return;
+        const int s = idx / row, c = idx - s * row;
+        kc[(size_t)(start_pos + s) * row + c] = __float2half(a[e]);
+        vc[(size_t)(start_pos + s) * row + c] = __float2half(b[e]);
+    }
 }
 
 // Both for a run of tokens from start_pos on, one block to a token: q in place, k and v to the cache (k itself stays as it was).  A thread keeps four pairs of a head
@@ -261,11 +271,17 @@ __global__ void add_kernel(float* out, const float* a, const float* b, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = a[i] + b[i];
 }
-__global__ void copy_kernel(float* __restrict__ dst, const float* __restrict__ src, int n) {
+template <int EACH>
+__global__ void __launch_bounds__(256) copy_kernel(float* __restrict__ dst, const float* __restrict__ src, int n) {
     pdl_launch_dependents();
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = behind_wait(src)[i];
+    src = behind_wait(src);
+    const int i0 = blockIdx.x * (256 * EACH) + threadIdx.x;
+    float a[EACH];
+#pragma unroll
+    for (int e = 0; e < EACH; e++) if (i0 + 256 * e < n) a[e] = src[i0 + 256 * e];
+#pragma unroll
+    for (int e = 0; e < EACH; e++) if (i0 + 256 * e < n) dst[i0 + 256 * e] = a[e];
 }
 // single-block cosine similarity (elementwise.cu:46-84): dot / (|a||b|), 0 when the denominator is <= 1e-8
 __global__ void __launch_bounds__(1024) cosine_kernel(float* result, const float* __restrict__ a, const float* __restrict__ b, int n) {
@@ -379,6 +395,7 @@ __global__ void __launch_bounds__(256) embed_kernel(float* __restrict__ out, con
 }
 
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
+constexpr int WIDE_RUN = 1 << 18;      // elements from which a thread takes four: 148 SMs have a block of each kind then
 
 }  // namespace
 
@@ -413,7 +430,8 @@ void copy_to_kv_cache(void* kc, void* vc, const float* k, const float* v, int se
                       int start_pos, int max_seq, cudaStream_t s) {
     int total = seq_len * n_kv * hd;
     if (total <= 0) return;
-    launch_k_pdl(true, kv_write_kernel, dim3(cdiv(total, 256)), dim3(256), 0, s, static_cast<__half*>(kc), static_cast<__half*>(vc), k, v, seq_len, n_kv * hd, start_pos, max_seq);
+    const int each = total >= WIDE_RUN ? 4 : 1;
+    launch_k_pdl(true, each == 4 ? kv_write_kernel<4> : kv_write_kernel<1>, dim3(cdiv(total, 256 * each)), dim3(256), 0, s, static_cast<__half*>(kc), static_cast<__half*>(vc), k, v, seq_len, n_kv * hd, start_pos, max_seq);
     count_launch();
 }
 bool rope_kv_rows(float* q, const float* k, const float* v, void* kc, void* vc, int tokens, int start_pos, int n_heads, int n_kv, int hd, float theta, float freq_scale,
@@ -446,7 +464,8 @@ void add_inplace(float* a, const float* b, int n, cudaStream_t s) { add(a, a, b,
 void add_bias(float* y, const float* b, int n, cudaStream_t s) { add(y, y, b, n, s); }
 void copy(float* dst, const float* src, int n, cudaStream_t s) {
     if (n <= 0) return;
-    launch_k_pdl(true, copy_kernel, dim3(cdiv(n, 256)), dim3(256), 0, s, dst, src, n);
+    const int each = n >= WIDE_RUN ? 4 : 1;
+    launch_k_pdl(true, each == 4 ? copy_kernel<4> : copy_kernel<1>, dim3(cdiv(n, 256 * each)), dim3(256), 0, s, dst, src, n);
     count_launch();
 }
 void cosine_similarity(float* result, const float* a, const float* b, int n, cudaStream_t s) {

@@ -208,10 +208,10 @@ __device__ __forceinline__ float dot8(const uint4& w, const float4& xa, const fl
     return acc;
 }
 __global__ void __launch_bounds__(F16_WARPS * 32) gemv_f16_kernel(float* __restrict__ y, const uint8_t* __restrict__ W,
-                                                                  const float* __restrict__ x, int out, int in, size_t pitch, int ep) {
+                                                                  const float* __restrict__ x, int out, int in, size_t pitch, int ep, int early) {
     extern __shared__ __align__(16) float xs[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_launch_dependents();
+    if (early) pdl_launch_dependents();
     pdl_wait();
     x = behind_wait(x); y = behind_wait(y);                        // (W by volatile asm)
     for (int i = threadIdx.x * 4; i < in; i += F16_WARPS * 32 * 4) *reinterpret_cast<float4*>(xs + i) = *reinterpret_cast<const float4*>(x + i);
@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(F16_WARPS * 32) gemv_f16_kernel(float* __restr
             else { y[r0] = a0; if (r0 + 1 < out) y[r0 + 1] = a1; }
         }
     }
+    pdl_launch_dependents();
 }
 constexpr int F16_MAX_SMEM = 200 * 1024;
 
@@ -266,12 +267,17 @@ void gemv_generic(float* y, const void* W, const float* x, int out, int in, DTyp
         int grid16 = (pairs + F16_WARPS - 1) / F16_WARPS;
         const int resident = (int)std::min<size_t>(8, (size_t)(220 * 1024) / ((size_t)in * 4 + 1024)) * 148;   // CTAs the chip holds
         if (grid16 > resident && resident > 0) grid16 = resident;
-        launch_k_pdl(true, gemv_f16_kernel, dim3(grid16), dim3(F16_WARPS * 32), (size_t)in * 4, s, y, w, x, out, in, pitch, (int)ep);
+        // Several CTAs fit on an SM: where this launch lets the next one start before it has done its part, that one's CTAs gather on the SMs that have room (4096 x 14336, call after
+        // call: 38 us, 23.6 launched plainly), where it does so at its end some still do (26.9, 23.7; 14336 x 4096 21.2, 20.4), which is more than the gap between launches
+        // but for small matrices (4096 x 4096 6.1, 8.35).  In a step the next launch is another kernel.
+        const bool small = (size_t)out * pitch <= (size_t)64 << 20;
+        launch_k_pdl(small || pdl_enabled(), gemv_f16_kernel, dim3(grid16), dim3(F16_WARPS * 32), (size_t)in * 4, s, y, w, x, out, in, pitch, (int)ep, pdl_enabled() ? 1 : 0);
         count_launch();
         return;
     }
     int grid = (out + GW * RPW - 1) / (GW * RPW);
-#define NT_LAUNCH(DTV) launch_k_pdl(true, gemv_generic_kernel<(int)DTV>, dim3(grid), dim3(GW * 32), 0, s, y, w, x, out, in, pitch, (int)ep)
+    // (programmatic in steps only: behind the boundary, call after call, the CTAs of the next launch gather on the SMs that are done first; F32 4096 x 4096 14.6 us, 26.8)
+#define NT_LAUNCH(DTV) launch_k(gemv_generic_kernel<(int)DTV>, dim3(grid), dim3(GW * 32), 0, s, y, w, x, out, in, pitch, (int)ep)
     switch (dt) {
         case DType::F32: NT_LAUNCH(DType::F32); break;
         case DType::F16: NT_LAUNCH(DType::F16); break;

@@ -399,9 +399,14 @@ TeamPlan plan_teams(int mask, int K, int groups, bool four) {
     // the vector does not fit twice (Q4_K 4096 x 14336: 11.4 us, 12.3 in teams of 4, 16.9 before).
     TeamPlan t = K > 8192 ? (groups > 256 ? form(4, 4, SMEM_CTA) : groups > 148 ? form(8, 2, SMEM_CTA) : form(16, 1, SMEM_CTA))
                           : (groups > 148 ? form(4, 4, SMEM_CTA) : form(8, 1, SMEM_HALF));
-    // Rings of one stage in four teams: two teams of 8 have the same bytes under way in stages of twice the columns, and half as many barriers (Q4_K 8192 x 28672:
-    // 36.3 us, 39.2 in teams of 4).  Two stages in teams of 4 are the better of the two (Q6_K 8192 x 28672: 46.6 us, 49.4 in teams of 8).
-    if (t.kw == 4 && t.stages < 2 && K > 8192) t = form(8, 2, SMEM_CTA);
+    // Rings of one stage in four teams: two teams of 8 have the same bytes under way in stages of twice the columns, and half as many barriers, where they have two stages
+    // (Q4_K 8192 x 28672: 36.3 us, 39.2 in teams of 4; Q5_K 8192 x 22016 call after call 31.9, 39.4) or are one round (Q8_0 4113 x 27904 35.6, 51.3); with one stage and more
+    // rounds they are the slower ones (Q8_0 14529 x 27904 112.9 us, 103.8; Q6_K 14529 x 48128 224.5, 207.6).  Two stages in teams of 4 are the better of the two
+    // (Q6_K 8192 x 28672: 46.6 us, 49.4 in teams of 8).
+    if (t.kw == 4 && t.stages < 2 && K > 8192) {
+        const TeamPlan u = form(8, 2, SMEM_CTA);
+        if (u.stages >= 2 || groups <= 2 * 148 || u.planes > t.planes) t = u;      // (four digits: Q4_0 8192 x 36096 72 us, 1217 where the generic form takes it)
+    }
     // Very long rows (from 41984 on, by format): the vector leaves no room for a stage of every team.  One team of 8 always has one.
     static const int ord[3][2] = {{8, 2}, {16, 1}, {8, 1}};
     for (int i = 0; t.stages < 1 && i < 3; i++) t = form(ord[i][0], ord[i][1], SMEM_CTA);

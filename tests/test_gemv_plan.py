@@ -51,3 +51,21 @@ def test_longer_rows_are_refused():
     assert plan((DType.Q4_K_M,), 4096, 49152 + 256)[0] == -2
     assert plan((DType.Q4_K_M,), 4096, 128)[0] == -2
     assert plan((DType.F16,), 4096, 4096)[0] == -2
+
+
+# us call after call in teams of 4 (one stage), in teams of 8
+@pytest.mark.parametrize("dt,rows,cols,whole,want", [
+    (DType.Q8_0, 14529, 27904, 0, (4, 4, 1)),       # 103.8, 112.9 with one stage
+    (DType.Q8_0, 6000, 36096, 0, (4, 4, 1)),        # 68.4, 74.1
+    (DType.Q6_K, 14529, 48128, 0, (4, 4, 1)),       # 207.6, 224.5
+    (DType.Q8_0, 4113, 27904, 0, (8, 2, 1)),        # 51.3, 35.6: one round
+    (DType.Q8_0, 14529, 26624, 0, (8, 2, 2)),       # 97.9, 74.0
+    (DType.Q6_K, 14529, 35840, 0, (8, 2, 2)),       # 157.1, 106.0
+    (DType.Q4_K_M, 8192, 28672, 0, (8, 2, 3)),      # 41.1, 35.5
+    (DType.Q5_K, 14529, 41472, 0, (8, 2, 2)),       # 112.9, 107.0
+    (DType.Q4_0, 8192, 36096, 1, (8, 2, 1)),        # 1217 in the generic form, for want of the fourth digit, 72
+    (DType.Q6_K, 8192, 28672, 0, (4, 4, 2)),
+])
+def test_long_rows_take_the_faster_teams(dt, rows, cols, whole, want):
+    rc, out = plan((dt,), rows, cols, whole=whole)
+    assert rc == 0 and out[:3] == want

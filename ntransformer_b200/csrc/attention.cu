@@ -582,15 +582,15 @@ bool attention_prefill_tc_pays(int seq_len, int start_pos, int n_heads, int hd) 
     return hd == 128 ? 1.9f * s64 - 2.82f * s128 - 0.7f * doubled > 2.75f : 1.22f * s64 - 2.1f * s128 - 0.3f * doubled > 1.25f;
 }
 // prompt-sized chunks: tiled tensor-core kernels
-int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq) {
+int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq, bool in_chain) {
     if (!attention_prefill_mma_supported(seq_len, n_heads, n_kv, hd)) return PREFILL_QUERIES;
-    return attention_prefill_tc_takes(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq) && attention_prefill_tc_pays(seq_len, start_pos, n_heads, hd)
+    return attention_prefill_tc_takes(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq) && (in_chain || attention_prefill_tc_pays(seq_len, start_pos, n_heads, hd))
                ? PREFILL_TC : PREFILL_MMA;
 }
 void attention_prefill(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads,
-                       int n_kv, int hd, int max_seq, float scale, cudaStream_t s) {
+                       int n_kv, int hd, int max_seq, float scale, cudaStream_t s, bool in_chain) {
     if (seq_len <= 0 || n_heads <= 0) return;
-    const int form = attention_prefill_form(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq);
+    const int form = attention_prefill_form(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq, in_chain);
     if (form != PREFILL_QUERIES) {
         if (form == PREFILL_TC && attention_prefill_tc(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, scale, s)) return;
         attention_prefill_mma(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq, scale, s);

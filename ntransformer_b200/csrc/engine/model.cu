@@ -992,7 +992,7 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
                 rope(pf_.q, pf_.k, pf_.pos, T, nh_l_, nkv_l_, hd, cfg_.rope_theta, cfg_.rope_freq_scale, false, s);
                 copy_to_kv_cache(kc, vc, pf_.k, pf_.v, T, nkv_l_, hd, p0, max_seq, s);
             }
-            attention_prefill(pf_.attn, pf_.q, kc, vc, T, p0, nh_l_, nkv_l_, hd, max_seq, scale, s);
+            attention_prefill(pf_.attn, pf_.q, kc, vc, T, p0, nh_l_, nkv_l_, hd, max_seq, scale, s, true);
             prefill_gemms(&pf_.x, pf_.ws, pf_.attn, nullptr, &wo, 1, T, true, s);
             // --- FFN sub-block (ffn.cpp:85-134) ---
             if (f16_direct(L.gate) && f16_direct(L.up)) {

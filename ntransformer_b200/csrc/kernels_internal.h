@@ -114,8 +114,10 @@ void masked_softmax(float* out, const float* in, const bool* mask, int rows, int
 void gemm_f32(float* C, const float* A, const float* B, int M, int N, int K, cudaStream_t s);
 void attention_decode(float* out, const float* q, const void* kc, const void* vc, int seq_len, int n_heads,
                       int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
+// in_chain: between programmatic launches, which the tcgen05 form joins.  The other, launched plainly, costs a prompt 3 to 4 us a layer beside its own time there (2 layers of 2048,
+// 64 tokens: 275 us, 281; 500: 456, 464), more than it saves anywhere
 void attention_prefill(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos,
-                       int n_heads, int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
+                       int n_heads, int n_kv, int hd, int max_seq, float scale, cudaStream_t s, bool in_chain = false);
 // call_memory.cu: memory that lasts for the launches of a call (the object's life), in the order of its stream; p null: there is none
 constexpr size_t CALL_MEMORY_KEPT = 64u << 20;        // of a device, between calls
 constexpr size_t STREAM_MEMORY_LEAST = 2u << 20;
@@ -146,7 +148,8 @@ struct CallMemoryUser {                               // the last of these to go
 };
 // the form that attention_prefill takes: a query at a time, mma.sync, tcgen05
 enum : int { PREFILL_QUERIES = 0, PREFILL_MMA = 1, PREFILL_TC = 2 };
-int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq);
+int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq,
+                           bool in_chain = false);
 // attention_prefill_tc.cu: 128 x 128 tiles on tcgen05 (heads 64 and 128 wide, pointers on 16 bytes, positions inside the cache); false: nothing launched
 bool attention_prefill_tc_takes(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq);
 bool attention_prefill_tc(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, float scale, cudaStream_t s);

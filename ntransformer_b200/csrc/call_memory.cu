@@ -53,7 +53,7 @@ void* take(size_t bytes, cudaStream_t s) {
     return m;
 }
 
-// Streams by the number that no later stream has again
+// Streams by the number that no other stream of the process has, then or later
 struct Kept { int dev = -1; unsigned long long stream = 0; void* p = nullptr; size_t bytes = 0; };
 Kept g_kept[STREAMS];
 std::mutex g_kept_mu;
@@ -66,11 +66,10 @@ CallMemory::~CallMemory() { if (p) NT_CUDA_CHECK(cudaFreeAsync(p, stream)); }
 StreamMemory::StreamMemory(size_t bytes, cudaStream_t s) : stream(s) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     unsigned long long id = 0;
-    const int dev = device();
-    if (cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone && dev >= 0 && cudaStreamGetId(s, &id) == cudaSuccess) {
+    if (cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone && cudaStreamGetId(s, &id) == cudaSuccess) {
         lock = std::unique_lock<std::mutex>(g_kept_mu);
         Kept* k = nullptr;
-        for (Kept& e : g_kept) if (e.p && e.dev == dev && e.stream == id) { k = &e; break; }
+        for (Kept& e : g_kept) if (e.p && e.stream == id) { k = &e; break; }
         if (k && k->bytes < bytes) {                               // behind the calls that use it
             NT_CUDA_CHECK(cudaFreeAsync(k->p, s));
             k->p = nullptr;
@@ -78,7 +77,7 @@ StreamMemory::StreamMemory(size_t bytes, cudaStream_t s) : stream(s) {
         for (Kept& e : g_kept) if (!k && !e.p) k = &e;
         if (k && !k->p) {
             const size_t room = bytes < STREAM_MEMORY_LEAST ? STREAM_MEMORY_LEAST : bytes;
-            if ((k->p = take(room, s))) { k->dev = dev; k->stream = id; k->bytes = room; }
+            if ((k->p = take(room, s))) { k->dev = device(); k->stream = id; k->bytes = room; }
         }
         if (k && k->p) { p = k->p; return; }
         lock.unlock();

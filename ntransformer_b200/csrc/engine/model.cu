@@ -8,7 +8,6 @@
 #include <cmath>
 #include <cstring>
 #include <cstdlib>
-#include <optional>
 #include <atomic>
 #include <chrono>
 #include <thread>
@@ -65,6 +64,7 @@ bool env_on(const char* name) { const char* e = getenv(name); return e && *e && 
 }  // namespace
 
 Model::~Model() {
+    block_scratch_.reset();
     if (stream_) cudaStreamSynchronize(stream_);
     release_graphs();
     for (void* p : owned_) cudaFree(p);
@@ -804,6 +804,18 @@ struct Cuts {
     void place(void* base) { uint8_t* at = static_cast<uint8_t*>(base); for (const Cut& c : list) { *c.p = at; at += (c.bytes + 255) / 256 * 256; } }
 };
 
+// What the GEMM over blocks keeps the shares of tiles in, for calls on this model's stream: of the pool, so that the next model finds it there.  false: no room
+bool Model::ensure_block_scratch(int tokens) {
+    const size_t bytes = block_scratch_bytes(tokens);
+    if (block_scratch_ && block_scratch_bytes_ >= bytes) return true;
+    block_scratch_.reset();
+    auto m = std::make_unique<CallMemory>(bytes, stream_);
+    if (!m->p) return false;
+    block_scratch_ = std::move(m);
+    block_scratch_bytes_ = bytes;
+    return true;
+}
+
 // false: no room for them; the caller takes the tokens one by one, which needs none
 bool Model::ensure_short_buffers() {
     if (sb_arena_) return true;
@@ -823,11 +835,7 @@ bool Model::ensure_short_buffers() {
 // false: no room for the GEMM's scratch; nothing launched
 bool Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
     cudaStream_t s = stream_;
-    std::optional<CallMemory> block_scratch;                       // where a chunk is more than a pass of gemv_rows
-    if (seq_len > 8) {
-        block_scratch.emplace(block_scratch_bytes(std::min(SHORT_CHUNK, seq_len)), s);
-        if (!block_scratch->p) return false;
-    }
+    if (seq_len > 8 && !ensure_block_scratch(std::min(SHORT_CHUNK, seq_len))) return false;      // where a chunk is more than a pass of gemv_rows
     const int hidden = cfg_.hidden_size, hd = cfg_.head_dim, max_seq = cfg_.max_seq_len, qdim = nh_l_ * hd;
     const size_t kv_stride = (size_t)max_seq * nkv_l_ * hd;
     int T = 0;
@@ -844,7 +852,7 @@ bool Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
             return false;
         }
         const BlockTokens t = up ? silu_split_tokens(sb_.ws, x, up, T, K, true, s) : split_tokens(sb_.ws, x, norm, cfg_.norm_eps, T, K, true, s);
-        NT_CHECK(gemm_blocks(m, n, K, t, block_scratch->p, T, ep == GEMV_ADD, s), "GEMM of a few tokens over blocks rejected");
+        NT_CHECK(gemm_blocks(m, n, K, t, block_scratch_->p, T, ep == GEMV_ADD, s), "GEMM of a few tokens over blocks rejected");
         return ep == GEMV_SWIGLU;
     };
     for (int c0 = 0; c0 < seq_len; c0 += T) {
@@ -908,7 +916,7 @@ void Model::prefill_gemms(float* const* C, void* ws, const float* x, const float
     if (!together || !gemm_f16_tc_multi_ws(c, ws, W, N, n_plain, T, K, s)) for (int i = 0; i < n_plain; i++) prefill_gemm(c[i], ws, *plain[i], T, add, s);
     if (n_blocks) {
         const BlockTokens t = x ? split_tokens(ws, x, norm_w, cfg_.norm_eps, T, K, false, s) : resplit_tokens(ws, ws, static_cast<uint8_t*>(ws) + gemm_f16_tc_workspace_bytes(T, K) / 2, T, K, s);
-        NT_CHECK(gemm_blocks(m, n_blocks, K, t, pf_scratch_, T, add, s), "prefill GEMM over blocks rejected");
+        NT_CHECK(gemm_blocks(m, n_blocks, K, t, block_scratch_->p, T, add, s), "prefill GEMM over blocks rejected");
     }
 }
 
@@ -961,12 +969,7 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
     const float scale = 1.0f / sqrtf((float)hd);
     const size_t kv_stride = (size_t)max_seq * nkv_l_ * hd;
     ensure_prefill_buffers(std::min(seq_len, PREFILL_CHUNK));
-    std::optional<CallMemory> scratch;
-    if (any_blocks_) {
-        scratch.emplace(block_scratch_bytes(std::min(seq_len, PREFILL_CHUNK)), s);
-        NT_CHECK(scratch->p, "no room for the scratch of the prompt GEMM over blocks");
-        pf_scratch_ = scratch->p;
-    }
+    if (any_blocks_) NT_CHECK(ensure_block_scratch(std::min(seq_len, PREFILL_CHUNK)), "no room for the scratch of the prompt GEMM over blocks");
     int last_rows = 0;
     for (int c0 = 0, T = 0; c0 < seq_len; c0 += T) {
         // A ragged tail of 1..15 tokens would miss the tiled attention kernel's 16-token minimum (and the per-query kernel it
@@ -1003,7 +1006,7 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
                 prefill_gemms(gu_out, pf_.ws, pf_.x, L.ffn_norm, gu, 2, T, false, s);
                 if (blocks_direct(L.down)) {
                     GemvMat m; m.W = down->ptr; m.y = pf_.x; m.out = down->rows; m.dtype = down->dtype; m.row_pitch = down->pitch;
-                    NT_CHECK(gemm_blocks(&m, 1, inter, silu_split_tokens(pf_.ws2, pf_.g, pf_.u, T, inter, false, s), pf_scratch_, T, true, s), "prefill GEMM over blocks rejected");
+                    NT_CHECK(gemm_blocks(&m, 1, inter, silu_split_tokens(pf_.ws2, pf_.g, pf_.u, T, inter, false, s), block_scratch_->p, T, true, s), "prefill GEMM over blocks rejected");
                 } else {
                     silu_mul_split(pf_.ws2, pf_.g, pf_.u, T, inter, s);
                     prefill_gemm(pf_.x, pf_.ws2, L.down, T, true, s);

@@ -170,7 +170,9 @@ public:
     void prefill_gemms(float* const* C, void* ws, const float* x, const float* norm_w, const Weight* const* w, int n, int T, bool add, cudaStream_t s);
     void *pf_arena_ = nullptr, *sb_arena_ = nullptr;               // pf_ (but a layer-spec model's) and sb_ lie in
     bool any_blocks_ = false;                                     // prompts go through the GEMM over blocks
-    void* pf_scratch_ = nullptr;                                   // its scratch, for the length of a prompt
+    bool ensure_block_scratch(int tokens);
+    std::unique_ptr<CallMemory> block_scratch_;
+    size_t block_scratch_bytes_ = 0;
     bool ensure_short_buffers();
     bool prefill_short(const int* tokens, int seq_len, int start_pos);
     struct { float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *g = nullptr, *u = nullptr, *scratch = nullptr; void* ws = nullptr;

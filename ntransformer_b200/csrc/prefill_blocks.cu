@@ -556,11 +556,11 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
 // ---- tokens ----
 // One block to a token: x (MODE 1: RMSNorm(x) * w, rmsnorm.cu:17-70's math; 2: silu(x) * w, gemm.cu:713-725's expression; 3: hi x and lo w of
 // a plain split, which may be the one written to) as F16 hi + lo, the sums of 32 of them
-// (a 32nd part, so that they stay within F16) as hi + lo, where `third` is given the halves that those two leave of both, and the factor that undoes the token's power of two.  That power takes the largest to 2^13 .. 2^14, where the
+// (a 32nd part, so that they stay within F16) as hi + lo, FINE: the halves that those two leave of both, and the factor that undoes the token's power of two.  That power takes the largest to 2^13 .. 2^14, where the
 // low halves keep their bits.  Block 0 also clears the product's counts: a launch whose wait ran out leaves some behind.
 // TOK_NORM_ANY: TOK_NORM whose gains do not lie on 16 bytes.
 enum : int { TOK_PLAIN = 0, TOK_NORM = 1, TOK_SILU = 2, TOK_SPLIT = 3, TOK_NORM_ANY = 4 };
-template <int MODE>
+template <int MODE, bool FINE>
 __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* lo, __half* third, __half* __restrict__ sums, __half* __restrict__ third_sums, float* __restrict__ scale, unsigned* __restrict__ count, int counts,
                                                            const float* xin, const float* w, float eps, int K) {
     constexpr int KEEP = 7;                                        // chunks of 2048 held in registers: rows to 14336
@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
         split_pair(a.z, a.w, 0, ph.y, pl.y);
         *reinterpret_cast<uint2*>(h + i) = ph;
         *reinterpret_cast<uint2*>(l + i) = pl;
-        if (third)
+        if (FINE)
             *reinterpret_cast<uint2*>(third + (size_t)blockIdx.x * K + i) =
                 make_uint2(bits(__floats2half2_rn(rest(a.x, ph.x, pl.x, false), rest(a.y, ph.x, pl.x, true))), bits(__floats2half2_rn(rest(a.z, ph.y, pl.y, false), rest(a.w, ph.y, pl.y, true))));
         float s = (a.x + a.y) + (a.z + a.w);                       // K is a multiple of 256: whole warps
@@ -635,7 +635,7 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
             const __half sl = __float2half_rn(left);
             const size_t q = sm + (i >> 8) * 16 + ((i >> 5) & 7);
             sums[q] = sh; sums[q + 8] = sl;
-            if (third) { third_sums[q] = __float2half_rn(left - __half2float(sl)); third_sums[q + 8] = __float2half_rn(0.f); }
+            if (FINE) { third_sums[q] = __float2half_rn(left - __half2float(sl)); third_sums[q + 8] = __float2half_rn(0.f); }
         }
     };
 #pragma unroll
@@ -705,7 +705,7 @@ BlockTokens launch_split(void* workspace, const float* x, const float* w, float 
     const BlockTokens t = block_tokens(workspace, T, K, fine);
     const size_t part = padded(T) * (size_t)K;
     __half *hi = static_cast<__half*>(t.split), *sums = static_cast<__half*>(t.sums);
-    launch_k_pdl(true, split_tokens_kernel<MODE>, dim3(T), dim3(512), 0, s, hi, hi + part, fine ? hi + 2 * part : nullptr, sums, sums + part / 16, t.scale, t.count, sm_count(), x, w, eps, K);
+    launch_k_pdl(true, fine ? split_tokens_kernel<MODE, true> : split_tokens_kernel<MODE, false>, dim3(T), dim3(512), 0, s, hi, hi + part, hi + 2 * part, sums, sums + part / 16, t.scale, t.count, sm_count(), x, w, eps, K);
     count_launch();
     return t;
 }

@@ -104,11 +104,12 @@ size_t nt_b200_gemv_rows_bytes(int tokens, int K);
 int    nt_b200_gemv_rows(int n_mat, float* const* y, const void* const* W, const int* out_features, const int* dtypes, int in_features,
                          const float* x, const float* norm_w, float eps, int tokens, void* scratch, int epilogue, void* stream);
 /* Prompts: C of matrix i [tokens, out_features[i]] (+)= X . W_i^T on the tcgen05 tensor cores, the blocks expanded on the way; X split into `workspace`
- * (nt_b200_split_activations).  Takes stream-ordered memory for the call.  Returns 0, or < 0 when rejected (nothing launched). */
+ * (nt_b200_split_activations).  Takes stream-ordered memory for the call, at most 64 MB (where a matrix has minima the tokens are laid out anew in it, in portions).
+ * Returns 0, or < 0 when rejected (nothing launched). */
 int    nt_b200_gemm_blocks_ws(int n_mat, float* const* C, const void* const* W, const int* out_features, const int* dtypes, int in_features,
                               const void* workspace, int tokens, int add, void* stream);
 /* The same over F32 tokens x [tokens, in_features] (norm_w: their RMSNorm), each under a power of two of its own; fine: 64 columns to an accumulator of the
- * tensor cores instead of 256.  What it needs beside its arguments is stream-ordered memory of the call.  Returns 0, or < 0 when rejected. */
+ * tensor cores instead of 256, and tokens in three halves instead of two.  What it needs beside its arguments is stream-ordered memory of the call.  Returns 0, or < 0 when rejected. */
 int    nt_b200_gemm_blocks(int n_mat, float* const* C, const void* const* W, const int* out_features, const int* dtypes, int in_features,
                            const float* x, const float* norm_w, float eps, int tokens, int fine, int add, void* stream);
 /* The decode step's attention sub-block in ONE launch: launch_rope (src/cuda/rotary.cu:113-140; q and k are read, not

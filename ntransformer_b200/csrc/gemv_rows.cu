@@ -2,7 +2,8 @@
 //
 // The reference runs its GEMV once for every prompt token (src/model/attention.cpp:144-162, ffn.cpp:96-133), and so did the engine below the length
 // where the tensor-core GEMM of prompts pays: 21 tokens cost 21 decode steps.  Here the arithmetic stays the decode step's — exact s32 products of the
-// weights' codes with 24-bit activations (gemv_mma_device.cuh), F32 sums — so a token's result does not depend on how many share the call:
+// weights' codes with 24-bit activations (gemv_mma_device.cuh), F32 sums — so a token's products here do not depend on how many share the
+// call (K-quants go to prefill_blocks.cu from 9 tokens on: other sums, with no larger error, which do not depend on it either):
 //   * one launch quantises all tokens (optionally RMSNorm) into the order in which mma.sync's B operand wants them: 8 tokens fill the operand's columns,
 //     (q1, q2) of four tokens in one product, q3 of eight in another;
 //   * a CTA takes 32 rows x 8 tokens.  A producer warp streams stages of 8 super-blocks of the rows and of the tokens; 16 warps share them, a

@@ -586,9 +586,9 @@ BlockTokens resplit_tokens(void* workspace, const void* hi, const void* lo, int 
 // whatever wrote the matrices is done.  No other launch comes between the two.
 size_t block_scratch_bytes(int T);
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, int T, bool add, cudaStream_t s);
-// Whether a few tokens are better served here (fine) than by gemv_rows: from two of its passes on (layers of an 8B model in Q4_K_M, 4 layers and head: 8 tokens
-// 771 us there, 900 here; 9 tokens 1025, 908; 31 tokens 1586, 973), and only where the error is no larger: not in Q8_0 and Q4_0, whose weights are pairs of halves here
-// (error against 64 bits 1.5e-7 of a result; 24-bit integers 1.3e-7.  K-quants: 1.3e-7 to 1.9e-7 here, 1.4e-7 to 2.3e-7 there)
+// Whether a few tokens are better served here (fine) than by gemv_rows: from two of its passes on (two layers of an 8B model in Q4_K_M and a head of 32000: 8 tokens
+// 342 us there, about 380 here; 9 tokens 497, 384; 31 tokens 778, 427), and not in Q8_0 and Q4_0, whose weights are pairs of halves here.  Error against 64 bits of a
+// result, K-quants: 1.0e-7 to 1.8e-7 here, 1.3e-7 to 2.6e-7 there
 bool gemm_blocks_for_few(const GemvMat* mats, int n_mat, int tokens);
 // over F32 tokens, or (x null) over split_activations' layout
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const float* norm_w, float eps, const void* split, bool fine, int T, bool add, cudaStream_t s);

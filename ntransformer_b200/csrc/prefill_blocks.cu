@@ -7,16 +7,17 @@
 //     and d joins when the epilogue takes a super-block's sum out of tensor memory.  The minima are a product of their own, m (8 for a super-block) times the sums
 //     of 32 activations.  Q6_K's sc * (q - 32) has up to 14 bits: a pair of halves, the second -1, 0 or 1.  Q8_0 and Q4_0 have a scale for 32 weights: d_i * q as
 //     a pair of halves, exact, under a power of two for the super-block;
-//   * eight warps expand 64 columns of 128 rows at a time, a row to a lane: blocks come into shared memory by cp.async, two halves cost a PRMT and an HFMA2,
+//   * eight warps expand 64 columns of 128 rows at a time, a row to a lane: blocks come into shared memory by TMA (Q6_K rows off 16 bytes by cp.async), two halves cost a PRMT and an HFMA2,
 //     and go to TENSOR MEMORY, from where tcgen05.mma takes its A operand: shared memory's bandwidth is left to B;
-//   * B is the split of the tokens x = hi + lo by TMA: two products for 16 columns (hi, lo), a third with the low half of a pair;
+//   * B is the split of the tokens x = hi + lo by TMA: two products for 16 columns (hi, lo), a third with the low half of a pair; in the fine form x = hi + lo + third,
+//     as many bits as the 24-bit integers hold and more (three products, five with a pair; a turn of 21 tokens 841 -> 864 us);
 //   * a super-block (256 columns; half of one where a row has no more, 64 where the caller asks for it) to an accumulator: the tensor cores cut off each addition, which leaves 1.86e-8 of a sum for
 //     each.  The epilogue's eight warps add the sums in F32 registers, times d, and write C once;
 //   * the work, tiles times super-blocks, is dealt out evenly: a CTA takes a run of super-blocks, whichever tiles it touches.  A tile that several CTAs share goes
 //     to a scratch, and whoever comes last adds the shares in their order (nothing waits for another CTA, the sums do not depend on who was last).
-// Measured (gate and up of an 8B layer, 28672 x 4096 Q4_K; the form before, which expanded each weight to a pair of halves, beside it): 500 tokens 341 -> 218 us, bound by
-// the tokens' way from L2 (49 bytes a clock and SM, 128 x 128 tiles with two halves of each token ask for 64); 21 tokens 100 (24-bit integers, three passes) -> 58 us,
-// bound by the chain of barriers and instructions that a k-block takes (700 cycles, whatever the tokens).
+// Measured (gate and up of an 8B layer, 28672 x 4096 Q4_K; the form before, which expanded each weight to a pair of halves, beside it): 500 tokens 341 -> 218 us, with 61 %
+// of the tensor cycles and 41 bytes a clock and SM from L2, where 128 x 128 tiles with two halves of each token ask for 64 at full rate; 21 tokens 100 (24-bit integers,
+// three passes) -> 63 us, bound by the chain of barriers and instructions that a k-block takes (1150 cycles, the tensor cores at a fifth).
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "tc_device.cuh"

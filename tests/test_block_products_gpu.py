@@ -105,7 +105,7 @@ def cut(cols):
     return 3 * -(-min(2048, cols / 2) // 16) * 2.0 ** -24 * 2 / 3 + 2.0 ** -21
 
 
-# tokens around the tile widths (any multiple of 16 up to 256, two column tiles), rows around 128, K of one and of several accumulators of 2048
+# tokens around the tile widths (multiples of 16 up to 128, several column tiles), rows around 128, K of one and of several super-blocks
 @pytest.mark.parametrize("dt", FORMATS, ids=lambda d: d.name)
 @pytest.mark.parametrize("tokens,rows,cols", [(17, 100, 256), (113, 129, 2304), (256, 128, 4096), (300, 1000, 768), (500, 384, 11008)])
 def test_prompt(dt, tokens, rows, cols):

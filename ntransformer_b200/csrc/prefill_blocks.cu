@@ -10,14 +10,14 @@
 //   * eight warps expand 64 columns of 128 rows at a time, a row to a lane: blocks come into shared memory by TMA (Q6_K rows off 16 bytes by cp.async), two halves cost a PRMT and an HFMA2,
 //     and go to TENSOR MEMORY, from where tcgen05.mma takes its A operand: shared memory's bandwidth is left to B;
 //   * B is the split of the tokens x = hi + lo by TMA: two products for 16 columns (hi, lo), a third with the low half of a pair; in the fine form x = hi + lo + third,
-//     as many bits as the 24-bit integers hold and more (three products, five with a pair; a turn of 21 tokens 841 -> 864 us);
+//     as many bits as the 24-bit integers hold and more (three products, five with a pair);
 //   * a super-block (256 columns; half of one where a row has no more, 64 where the caller asks for it) to an accumulator: the tensor cores cut off each addition, which leaves 1.86e-8 of a sum for
 //     each.  The epilogue's eight warps add the sums in F32 registers, times d, and write C once;
 //   * the work, tiles times super-blocks, is dealt out evenly: a CTA takes a run of super-blocks, whichever tiles it touches.  A tile that several CTAs share goes
 //     to a scratch, and whoever comes last adds the shares in their order (nothing waits for another CTA, the sums do not depend on who was last).
 // Measured (gate and up of an 8B layer, 28672 x 4096 Q4_K; the form before, which expanded each weight to a pair of halves, beside it): 500 tokens 341 -> 218 us, with 61 %
 // of the tensor cycles and 41 bytes a clock and SM from L2, where 128 x 128 tiles with two halves of each token ask for 64 at full rate; 21 tokens 100 (24-bit integers,
-// three passes) -> 63 us, bound by the chain of barriers and instructions that a k-block takes (1150 cycles, the tensor cores at a fifth).
+// three passes) -> 57 us, and 43 in the form for a few tokens below.
 #include "kernels_internal.h"
 #include "ring.cuh"
 #include "tc_device.cuh"
@@ -32,7 +32,7 @@ namespace nt { namespace b200 {
 namespace {
 
 constexpr int QBK = 64;                                  // columns of a k-block: a 128-byte swizzle row of F16
-constexpr int NT_MAX = 128;                              // tokens of a tile
+constexpr int NT_MAX = 128, FEW_TOKENS = 32;             // tokens of a tile; of a launch of the form for a few
 constexpr int STAGES_MAX = 4, D_BUFS_MAX = 4, RAW_MAX = 8, SCALE_RING = 8;
 constexpr int EPI_WARP = 4, EXP_WARP = 12, Q_THREADS = 20 * 32;      // warp 0 tokens, 1 MMA, 2 blocks (2, 3: off 16 bytes), 4-11 epilogue, 12-19 expansion
 
@@ -146,20 +146,24 @@ __device__ __forceinline__ void pairs(const uint32_t (&q)[8], __half2 off, const
             lo[2 * i + j] = bits(__hfma2(v, D[i >> 2], __hneg2(p)));      // what the product's rounding left, exact
         }
 }
+// Q6_K: the upper bits of a k-block's codes, the same words for its two halves
+__device__ __forceinline__ void upper_bits(const uint8_t* blk, int c, uint32_t (&v)[8]) { lds_words(blk + 128 + 32 * (c >> 1), v); }
 template <int FMT>
-__device__ __forceinline__ void expand_pair(const uint8_t* blk, int c, int hf, float up, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
+__device__ __forceinline__ void expand_pair(const uint8_t* blk, int c, int hf, float up, const uint32_t (&v)[8], uint32_t (&hi)[16], uint32_t (&lo)[16]) {
     uint32_t q[8];
     __half2 D[2];
     if (FMT == 2) {
         // half h of the super-block, quarters q1 (codes in the low nibbles of the first 32 bytes, bits 0-1 of the pairs), q2 (second 32, bits 2-3), q3, q4
         const int h = c >> 1, qt = 2 * (c & 1) + hf;
-        uint32_t w[8], v[8];
+        uint32_t w[8];
         lds_words(blk + 64 * h + 32 * hf, w);
-        lds_words(blk + 128 + 32 * h, v);
         const int8_t* sc = reinterpret_cast<const int8_t*>(blk + 192 + 8 * h + 2 * qt);
         D[0] = __half2half2(__int2half_rn(sc[0])); D[1] = __half2half2(__int2half_rn(sc[1]));
 #pragma unroll
-        for (int i = 0; i < 8; i++) q[i] = ((w[i] >> (4 * (c & 1))) & 0x0F0F0F0Fu) | (((v[i] >> (2 * qt)) & 0x03030303u) << 4);
+        for (int i = 0; i < 8; i++) {                              // bits 4 and 5 from the word whose bits 2 qt and 2 qt + 1 they are
+            const uint32_t a = w[i] >> (4 * (c & 1)), b = __funnelshift_l(v[i], v[i], 36 - 2 * qt);      // (what comes round is masked off)
+            q[i] = ((a & 0x0F0F0F0Fu) | (b & ~0x0F0F0F0Fu)) & 0x3F3F3F3Fu;
+        }
         pairs(q, __float2half2_rn(1056.0f), D, hi, lo);
     } else {
         const uint8_t* b = blk + (FMT == 3 ? 34 : 18) * (2 * c + hf);
@@ -190,6 +194,157 @@ __device__ __forceinline__ float block_power(const uint8_t* blk, float& inverse)
     return __uint_as_float((uint32_t)(127 - e) << 23);
 }
 
+// Where a CTA's run of units (tile * NB + super-block) stands; tokens inside, so that the CTAs of a wave share rows
+struct Place { int tile, b, mi, row0, t0; };
+__device__ __forceinline__ int first_unit(const BlkParams& p, int cta) { return (int)((long long)p.units * cta / (int)gridDim.x); }
+__device__ __forceinline__ void place(const BlkParams& p, Place& q) {
+    const int rt = q.tile / p.cols;
+    q.t0 = (q.tile - rt * p.cols) * p.NT;
+    int r = rt, mi = 0;
+    if (p.n_mat > 1 && r >= p.mat[0].tiles) { r -= p.mat[0].tiles; mi = 1; }
+    if (p.n_mat > 2 && mi == 1 && r >= p.mat[1].tiles) { r -= p.mat[1].tiles; mi = 2; }
+    q.mi = mi; q.row0 = r * 128;
+}
+__device__ __forceinline__ Place start(const BlkParams& p, int u0) { Place q; q.tile = u0 / p.NB; q.b = u0 - q.tile * p.NB; place(p, q); return q; }
+__device__ __forceinline__ void next(const BlkParams& p, Place& q) { if (++q.b == p.NB) { q.b = 0; q.tile++; place(p, q); } }
+template <int MASK> __device__ __forceinline__ int format(int fmt) { return MASK == 1 ? 0 : MASK == 2 ? 1 : MASK == 4 ? 2 : MASK == 8 ? 3 : MASK == 16 ? 4 : fmt; }
+template <int MASK> __device__ __forceinline__ bool mins_of(const BlkParams& p, int mi) { return (MASK & (MASK - 1)) == 0 ? (MASK & 3) != 0 : (MASK & 3) != 0 && has_mins(p.mat[mi].fmt); }
+
+// One thread, or (Q6_K rows off 16 bytes) both warps of the producer: blocks of W, the 16-byte units around a super-block of 128 rows, by TMA or by cp.async
+template <int MASK>
+__device__ __forceinline__ void load_blocks(const BlkMaps& maps, const BlkParams& p, int u0, int u1, uint8_t* raw, uint64_t* raw_full, uint64_t* raw_empty, bool by_tma, uint32_t dead, int warp, int lane) {
+    uint32_t st = 0, par = 1, filled = 0;
+    Place q = start(p, u0);
+    for (int u = u0; u < u1; u++, next(p, q)) {
+        const BlkMat& m = p.mat[q.mi];
+        const int fmt = format<MASK>(m.fmt);
+        wait_cta(raw_empty + st, par, dead);
+        if (word_set(dead)) {
+            for (uint32_t s = 0; s < filled && by_tma; s++) wait_flight(raw_full + s, s < st ? par ^ 1u : par);      // the copies in flight
+            break;
+        }
+        filled = min(filled + 1, (uint32_t)p.raw_depth);
+        uint8_t* d = raw + (size_t)st * p.raw_slot;
+        if (by_tma || (p.tma >> q.mi & 1)) {
+            if (threadIdx.x == 64) {
+                mbar_expect_tx(raw_full + st, 128u * raw_pitch(fmt));
+                tma_load_2d(d, &maps.w[q.mi], (q.b * fmt_bytes(fmt) & ~15) >> 2, q.row0, raw_full + st);
+            }
+            if (!by_tma) mbar_arrive(raw_full + st);
+        } else {
+            copy_rows(smem_u32(d) + (warp - 2) * 64 * raw_pitch(2), m, q.row0 + (warp - 2) * 64, q.b, p.NB, lane);
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(raw_full + st)) : "memory");
+            if (threadIdx.x == 64) mbar_arrive(raw_full + st);
+        }
+        if (++st == (uint32_t)p.raw_depth) { st = 0; par ^= 1; }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// The super-block that this lane's row has in a slot, the power of two that its codes are taken up by, and (first) what its sums are multiplied by
+template <int MASK>
+__device__ __forceinline__ const uint8_t* find_block(const BlkMat& m, const Place& q, int fmt, const uint8_t* slot, int r, float& up, float2& scale) {
+    const uint8_t* blk = slot + r * raw_pitch(fmt);
+    if ((MASK & 4) && fmt == 2) blk += ((uint32_t)min(q.row0 + r, m.rows - 1) * (uint32_t)m.pitch + (uint32_t)q.b * 210u) & 15u;      // (W on 16 bytes)
+    float down = 1.f;
+    up = 1.f;
+    if ((MASK & 8) && fmt == 3) up = block_power<3>(blk, down);
+    if ((MASK & 16) && fmt == 4) up = block_power<4>(blk, down);
+    scale = make_float2(down, 0.f);
+    if ((MASK & 3) && fmt <= 1) { const uint32_t h = *reinterpret_cast<const uint32_t*>(blk); scale = make_float2(half_bits(h & 0xFFFFu), -32.0f * half_bits(h >> 16)); }
+    if ((MASK & 4) && fmt == 2) scale.x = half_bits(*reinterpret_cast<const uint16_t*>(blk + 208));
+    return blk;
+}
+// the minima of a Q4_K / Q5_K super-block as halves
+__device__ __forceinline__ void expand_mins(const uint4& h, uint32_t (&w)[4]) {
+    const __half2 k = __float2half2_rn(1024.0f);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const uint32_t mm = kq_mins(h, i != 0);
+        w[2 * i] = bits(__hsub2(half_pair<0, 1>(mm), k));
+        w[2 * i + 1] = bits(__hsub2(half_pair<2, 3>(mm), k));
+    }
+}
+
+// The epilogue's end of a tile: this CTA's sums of units [seg0, end), 16 tokens of every STEP from `from` on.  A tile that other CTAs have a share of goes to the scratch, and
+// whoever comes last adds the shares in their order.  named barrier 5: the epilogue's threads, two warps to a row where STEP is 32.
+template <int N, int STEP>
+__device__ __forceinline__ void finish_tile(const BlkParams& p, const Place& q, uint64_t (&acc)[N][8], int u0, int seg0, int end, int from, int r, const float* token_scale, uint32_t* last_smem, uint32_t dead) {
+    const int NT = p.NT, live = min(NT, p.T - q.t0), rows = p.mat[q.mi].rows, row = q.row0 + r;
+    bool write = true;
+    if (end - seg0 < p.NB) {                                       // shared: to the scratch; whoever comes last adds
+        write = false;
+        const int tu = q.tile * p.NB, G = gridDim.x;
+        const int c0 = (int)(((long long)(tu + 1) * G - 1) / p.units), c1 = (int)(((long long)(tu + p.NB) * G - 1) / p.units);
+        float* mine = p.part + (size_t)(2 * blockIdx.x + (seg0 == u0 ? 0 : 1)) * 128 * NT + r;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int n = STEP * i + from;
+            if (n >= live) break;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                float x, y;
+                unpack2(acc[i][j], x, y);
+                __stcg(mine + (n + 2 * j) * 128, x);
+                __stcg(mine + (n + 2 * j + 1) * 128, y);
+            }
+        }
+        __threadfence();
+        named_sync<8 * STEP>(5);
+        if (threadIdx.x == EPI_WARP * 32) {
+            const bool alive = !word_set(dead);
+            const bool is_last = alive && atomicAdd(p.count + c0, 1u) == (unsigned)(c1 - c0);
+            if (is_last) p.count[c0] = 0;
+            __threadfence();
+            *last_smem = is_last;
+        }
+        named_sync<8 * STEP>(5);
+        if (*last_smem) {
+            write = true;
+#pragma unroll
+            for (int i = 0; i < N; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = 0;
+#pragma unroll 1
+            for (int c = c0; c <= c1; c++) {
+                const float* o = p.part + (size_t)(2 * c + (first_unit(p, c) >= tu ? 0 : 1)) * 128 * NT + r;
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    const int n = STEP * i + from;
+                    if (n >= live) break;
+                    float v[16];
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] = __ldcg(o + (n + j) * 128);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        float x, y;
+                        unpack2(acc[i][j], x, y);
+                        acc[i][j] = pack2(x + v[2 * j], y + v[2 * j + 1]);
+                    }
+                }
+            }
+        }
+    }
+    if (write && row < rows && !word_set(dead)) {                  // a warp stores 128 contiguous bytes for each token
+        float* o = p.mat[q.mi].C + (size_t)(q.t0 + from) * rows + row;
+        const float* ts = token_scale + q.t0 + from;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                if (STEP * i + from + j >= live) break;
+                float x, y;
+                unpack2(acc[i][j >> 1], x, y);
+                const float v = ((j & 1) ? y : x) * __ldg(ts + STEP * i + j);
+                // adds go to the memory's side (this lane is the element's only writer): nothing is waited for
+                if (p.add) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + (size_t)j * rows), "f"(v) : "memory");
+                else o[(size_t)j * rows] = v;
+            }
+            o += (size_t)STEP * rows;
+        }
+    }
+}
+
 // MASK: the formats that a launch's matrices have (bits).  PARTS: halves that a token's column is split into
 template <int MASK, int PARTS>
 __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_constant__ BlkMaps maps, const __grid_constant__ BlkParams p) {
@@ -202,27 +357,11 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
     __shared__ float2 scales[SCALE_RING][128];                     // of a super-block's rows: what its sum and what its minima's sum are multiplied by
     __shared__ uint32_t tmem_base_smem, last_smem, dead_smem;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int NB = p.NB, NT = p.NT;
+    const int NT = p.NT;
     const uint32_t b_tile = (uint32_t)NT * 128, b_stage = (uint32_t)p.b_stage, dead = smem_u32(&dead_smem);
     uint8_t* raw = smem + (size_t)p.stages * b_stage;
-    // this CTA's super-blocks: units [u0, u1), unit = tile * NB + super-block
-    auto first_unit = [&](int cta) { return (int)((long long)p.units * cta / (int)gridDim.x); };
-    const int u0 = first_unit(blockIdx.x), u1 = first_unit(blockIdx.x + 1);
-    auto format = [&](int fmt) { return MASK == 1 ? 0 : MASK == 2 ? 1 : MASK == 4 ? 2 : MASK == 8 ? 3 : MASK == 16 ? 4 : fmt; };
-    auto mins_of = [&](int mi) { return ONE ? MINS : MINS && has_mins(p.mat[mi].fmt); };
+    const int u0 = first_unit(p, blockIdx.x), u1 = first_unit(p, blockIdx.x + 1);      // this CTA's super-blocks
     const bool by_tma = !(MASK & 4) || p.tma == (1 << p.n_mat) - 1;      // all of W
-    // where a tile lies: tokens inside, so that the CTAs of a wave share rows
-    struct Place { int tile, b, mi, row0, t0; };
-    auto place = [&](Place& q) {
-        const int rt = q.tile / p.cols;
-        q.t0 = (q.tile - rt * p.cols) * NT;
-        int r = rt, mi = 0;
-        if (p.n_mat > 1 && r >= p.mat[0].tiles) { r -= p.mat[0].tiles; mi = 1; }
-        if (p.n_mat > 2 && mi == 1 && r >= p.mat[1].tiles) { r -= p.mat[1].tiles; mi = 2; }
-        q.mi = mi; q.row0 = r * 128;
-    };
-    auto start = [&] { Place q; q.tile = u0 / NB; q.b = u0 - q.tile * NB; place(q); return q; };
-    auto next = [&](Place& q) { if (++q.b == NB) { q.b = 0; q.tile++; place(q); } };
     if (threadIdx.x == 0) {
         for (int i = 0; i < p.stages; i++) { mbar_init(full + i, 5); mbar_init(empty + i, 1); }      // the tokens' producer and four warps of the expansion
         for (int i = 0; i < p.d_bufs; i++) { mbar_init(d_full + i, 1); mbar_init(d_empty + i, 8); }
@@ -249,10 +388,10 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
     if (warp == 0) {
         if (lane == 0) {                                           // ---- tokens by TMA ----
             uint32_t st = 0, par = 1, filled = 0;
-            Place q = start();
+            Place q = start(p, u0);
             pdl_wait();
-            for (int u = u0; u < u1; u++, next(q)) {
-                const bool mins = mins_of(q.mi);
+            for (int u = u0; u < u1; u++, next(p, q)) {
+                const bool mins = mins_of<MASK>(p, q.mi);
                 for (int kb = 0; kb < 4; kb++) {
                     wait_cta(empty + st, par, dead);
                     if (word_set(dead)) {
@@ -280,9 +419,9 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         const uint64_t desc0 = make_desc(smem), desc32 = make_desc32(smem), lo_step = (uint64_t)(b_tile >> 4), stage_step = (uint64_t)(b_stage >> 4);
         uint32_t st = 0, par = 0, db = 0, dpar = 1;
         int last = -1;                                             // stage and parity of the last commit
-        Place q = start();
-        for (int u = u0; u < u1; u++, next(q)) {
-            const bool mins = mins_of(q.mi);
+        Place q = start(p, u0);
+        for (int u = u0; u < u1; u++, next(p, q)) {
+            const bool mins = mins_of<MASK>(p, q.mi);
 #pragma unroll 1
             for (int k0 = 0; k0 < 4; k0 += p.kc) {
                 wait_cta(d_empty + db, dpar, dead);
@@ -330,33 +469,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         }
         if (word_set(dead) && last >= 0) wait_flight(empty + (last >> 1), last & 1);      // given up: the products in flight
     } else if (by_tma ? threadIdx.x == 64 : true) {
-        // ---- blocks of W: the 16-byte units around a super-block of 128 rows, by TMA; Q6_K rows off 16 bytes by cp.async from both warps ----
-        uint32_t st = 0, par = 1, filled = 0;
-        Place q = start();
-        for (int u = u0; u < u1; u++, next(q)) {
-            const BlkMat& m = p.mat[q.mi];
-            const int fmt = format(m.fmt);
-            wait_cta(raw_empty + st, par, dead);
-            if (word_set(dead)) {
-                for (uint32_t s = 0; s < filled && by_tma; s++) wait_flight(raw_full + s, s < st ? par ^ 1u : par);      // the copies in flight
-                break;
-            }
-            filled = min(filled + 1, (uint32_t)p.raw_depth);
-            uint8_t* d = raw + (size_t)st * p.raw_slot;
-            if (by_tma || (p.tma >> q.mi & 1)) {
-                if (threadIdx.x == 64) {
-                    mbar_expect_tx(raw_full + st, 128u * raw_pitch(fmt));
-                    tma_load_2d(d, &maps.w[q.mi], (q.b * fmt_bytes(fmt) & ~15) >> 2, q.row0, raw_full + st);
-                }
-                if (!by_tma) mbar_arrive(raw_full + st);
-            } else {
-                copy_rows(smem_u32(d) + (warp - 2) * 64 * raw_pitch(2), m, q.row0 + (warp - 2) * 64, q.b, NB, lane);
-                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(raw_full + st)) : "memory");
-                if (threadIdx.x == 64) mbar_arrive(raw_full + st);
-            }
-            if (++st == (uint32_t)p.raw_depth) { st = 0; par ^= 1; }
-        }
-        asm volatile("cp.async.wait_all;" ::: "memory");
+        load_blocks<MASK>(maps, p, u0, u1, raw, raw_full, raw_empty, by_tma, dead, warp, lane);      // ---- blocks of W ----
     }
     } else if (warp < EXP_WARP) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
@@ -364,12 +477,12 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         const int quarter = warp & 3, half = (warp - EPI_WARP) >> 2, r = quarter * 32 + lane;
         const uint32_t tq = ((uint32_t)(quarter * 32) << 16) + half * 16;
         uint32_t db = 0, dpar = 0, slot = 0, spar = 0;
-        Place q = start();
+        Place q = start(p, u0);
         pdl_wait();
         const float* token_scale = behind_wait(p.scale);
         for (int u = u0; u < u1;) {
-            const int sums = 4 / p.kc, chunks = sums + (MINS && mins_of(q.mi) ? 1 : 0);
-            const int seg0 = u, end = min(u1, u + (NB - q.b));
+            const int sums = 4 / p.kc, chunks = sums + (MINS && mins_of<MASK>(p, q.mi) ? 1 : 0);
+            const int seg0 = u, end = min(u1, u + (p.NB - q.b));
             uint64_t acc[4][8] = {};                               // pairs of tokens
 #pragma unroll 1
             for (; u < end; u++) {
@@ -397,81 +510,9 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     if (++db == (uint32_t)p.d_bufs) { db = 0; dpar ^= 1; }
                 }
             }
-            const int live = min(NT, p.T - q.t0), rows = p.mat[q.mi].rows, row = q.row0 + r;
-            bool write = true;
-            if (end - seg0 < NB) {                                 // shared: to the scratch; whoever comes last adds
-                write = false;
-                const int tu = q.tile * NB, G = gridDim.x;
-                const int c0 = (int)(((long long)(tu + 1) * G - 1) / p.units), c1 = (int)(((long long)(tu + NB) * G - 1) / p.units);
-                float* mine = p.part + (size_t)(2 * blockIdx.x + (seg0 == u0 ? 0 : 1)) * 128 * NT + r;
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int n = 32 * i + 16 * half;
-                    if (n >= live) break;
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        float x, y;
-                        unpack2(acc[i][j], x, y);
-                        __stcg(mine + (n + 2 * j) * 128, x);
-                        __stcg(mine + (n + 2 * j + 1) * 128, y);
-                    }
-                }
-                __threadfence();
-                named_sync<256>(5);
-                if (threadIdx.x == EPI_WARP * 32) {
-                    const bool alive = !word_set(dead);
-                    const bool is_last = alive && atomicAdd(p.count + c0, 1u) == (unsigned)(c1 - c0);
-                    if (is_last) p.count[c0] = 0;
-                    __threadfence();
-                    last_smem = is_last;
-                }
-                named_sync<256>(5);
-                if (last_smem) {
-                    write = true;
-#pragma unroll
-                    for (int i = 0; i < 4; i++)
-#pragma unroll
-                        for (int j = 0; j < 8; j++) acc[i][j] = 0;
-#pragma unroll 1
-                    for (int c = c0; c <= c1; c++) {
-                        const float* o = p.part + (size_t)(2 * c + (first_unit(c) >= tu ? 0 : 1)) * 128 * NT + r;
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const int n = 32 * i + 16 * half;
-                            if (n >= live) break;
-                            float v[16];
-#pragma unroll
-                            for (int j = 0; j < 16; j++) v[j] = __ldcg(o + (n + j) * 128);
-#pragma unroll
-                            for (int j = 0; j < 8; j++) {
-                                float x, y;
-                                unpack2(acc[i][j], x, y);
-                                acc[i][j] = pack2(x + v[2 * j], y + v[2 * j + 1]);
-                            }
-                        }
-                    }
-                }
-            }
-            if (write && row < rows && !word_set(dead)) {          // a warp stores 128 contiguous bytes for each token
-                float* o = p.mat[q.mi].C + (size_t)(q.t0 + 16 * half) * rows + row;
-                const float* ts = token_scale + q.t0 + 16 * half;
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-#pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        if (32 * i + 16 * half + j >= live) break;
-                        float x, y;
-                        unpack2(acc[i][j >> 1], x, y);
-                        const float v = ((j & 1) ? y : x) * __ldg(ts + 32 * i + j);
-                        // adds go to the memory's side (this lane is the element's only writer): nothing is waited for
-                        if (p.add) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + (size_t)j * rows), "f"(v) : "memory");
-                        else o[(size_t)j * rows] = v;
-                    }
-                    o += (size_t)32 * rows;
-                }
-            }
+            finish_tile<4, 32>(p, q, acc, u0, seg0, end, 16 * half, r, token_scale, &last_smem, dead);
             q.b = 0; q.tile++;
-            place(q);
+            place(p, q);
         }
         if (word_set(dead)) report(p.status);
     } else {                                                       // ---- expansion: two warps share 32 rows; k-blocks 0, 2 or 1, 3 of a super-block to each ----
@@ -480,21 +521,16 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         const uint32_t tq = (uint32_t)(quarter * 32) << 16;
         int slot = 0, sslot = 0;
         uint32_t st = odd, par = 1, rpar = 0;
-        Place q = start();
-        for (int u = u0; u < u1; u++, next(q)) {
+        Place q = start(p, u0);
+        for (int u = u0; u < u1; u++, next(p, q)) {
             const BlkMat& m = p.mat[q.mi];
-            const int fmt = format(m.fmt);
+            const int fmt = format<MASK>(m.fmt);
             wait_cta(raw_full + slot, rpar, dead);
-            const uint8_t* blk = raw + (size_t)slot * p.raw_slot + (quarter * 32 + lane) * raw_pitch(fmt);
-            if ((MASK & 4) && fmt == 2) blk += ((uint32_t)min(q.row0 + quarter * 32 + lane, m.rows - 1) * (uint32_t)m.pitch + (uint32_t)q.b * 210u) & 15u;      // (W on 16 bytes)
-            float up = 1.f, down = 1.f;
-            if ((MASK & 8) && fmt == 3) up = block_power<3>(blk, down);
-            if ((MASK & 16) && fmt == 4) up = block_power<4>(blk, down);
+            float up;
+            float2 scale;
+            const uint8_t* blk = find_block<MASK>(m, q, fmt, raw + (size_t)slot * p.raw_slot, quarter * 32 + lane, up, scale);
             if (!odd) {
-                float2 s = make_float2(down, 0.f);
-                if (MINS && fmt <= 1) { const uint32_t h = *reinterpret_cast<const uint32_t*>(blk); s = make_float2(half_bits(h & 0xFFFFu), -32.0f * half_bits(h >> 16)); }
-                if ((MASK & 4) && fmt == 2) s.x = half_bits(*reinterpret_cast<const uint16_t*>(blk + 208));
-                scales[sslot][quarter * 32 + lane] = s;
+                scales[sslot][quarter * 32 + lane] = scale;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(s_full + sslot);
             }
@@ -513,22 +549,18 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     tmem_st16(a + 16, v + 16);
                     if (c == 3) {                                  // (the product of the minima before came ahead of the commit that freed a stage of k-block 3 or later)
                         uint32_t w[4];
-                        const __half2 k = __float2half2_rn(1024.0f);
-#pragma unroll
-                        for (int i = 0; i < 2; i++) {
-                            const uint32_t mm = kq_mins(h, i != 0);
-                            w[2 * i] = bits(__hsub2(half_pair<0, 1>(mm), k));
-                            w[2 * i + 1] = bits(__hsub2(half_pair<2, 3>(mm), k));
-                        }
+                        expand_mins(h, w);
                         tmem_st8(tq + m_base, w);
                     }
                 } else if (PAIRS) {
+                    uint32_t v[8];
+                    if ((MASK & 4) && fmt == 2) upper_bits(blk, c, v);
 #pragma unroll 1
                     for (int hf = 0; hf < 2; hf++) {
                         uint32_t hi[16], lo[16];
-                        if ((MASK & 4) && fmt == 2) expand_pair<2>(blk, c, hf, up, hi, lo);
-                        if ((MASK & 8) && fmt == 3) expand_pair<3>(blk, c, hf, up, hi, lo);
-                        if ((MASK & 16) && fmt == 4) expand_pair<4>(blk, c, hf, up, hi, lo);
+                        if ((MASK & 4) && fmt == 2) expand_pair<2>(blk, c, hf, up, v, hi, lo);
+                        if ((MASK & 8) && fmt == 3) expand_pair<3>(blk, c, hf, up, v, hi, lo);
+                        if ((MASK & 16) && fmt == 4) expand_pair<4>(blk, c, hf, up, v, hi, lo);
                         if (hf == 0) {
                             wait_cta(empty + st, par, dead);
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -543,6 +575,242 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                 if (lane == 0) mbar_arrive(full + st);
                 st += 2;
                 if (st >= (uint32_t)p.stages) { st -= p.stages; par ^= 1; }
+            }
+            if (lane == 0) mbar_arrive(raw_empty + slot);          // (every lane has read what it stored)
+            if (++slot == p.raw_depth) { slot = 0; rpar ^= 1; }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    __syncwarp();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_smem), "n"(512));
+}
+
+// The same for up to 32 tokens in the fine form (64 columns to an accumulator, a token in three halves).  There the products take a fifth of a k-block's time, memory a sixth: what
+// bounds is that copies, expansion, products and sums hand each k-block on by barriers, two commits and five waits of a warp to each (the MMA warp's wait for a free accumulator
+// alone took 270 of 1050 cycles).  So a stage is half a super-block, with accumulators of its own, and one barrier (done) says that its products are finished, which frees its
+// tokens and weights and hands its sums over.  A super-block of Q4_K takes 2200 cycles where it took 3200; the expansion's instructions bound then, of Q6_K above all (5000).
+// 21 tokens, us with the split of the tokens, before and now: Q4_K 28672 x 4096 56.6, 43.1; 4096 x 14336 39.1, 31.1; 4096 x 4096 21.2, 18.3; Q5_K 14336 x 4096 37.1, 29.8; Q6_K
+// 4096 x 14336 48.5, 46.2.  Sixteen warps of expansion and four of sums in place of eight and eight: 57.6 (the four are then behind, and the issuing warp is starved).
+// Tiles of more than 32 tokens leave room for one stage of it: 40 tokens 60.8, 70.8.
+template <int MASK>
+__global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __grid_constant__ BlkMaps maps, const __grid_constant__ BlkParams p) {
+    constexpr bool ONE = (MASK & (MASK - 1)) == 0, MINS = (MASK & 3) != 0, PAIRS = (MASK & 28) != 0;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t full[STAGES_MAX], done[STAGES_MAX], d_empty[STAGES_MAX];
+    __shared__ uint64_t raw_full[RAW_MAX], raw_empty[RAW_MAX], s_full[SCALE_RING];
+    __shared__ float2 scales[SCALE_RING][128];
+    __shared__ uint32_t tmem_base_smem, last_smem, dead_smem;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int NT = p.NT;
+    const uint32_t b_tile = (uint32_t)NT * 128, b_stage = (uint32_t)p.b_stage, dead = smem_u32(&dead_smem);
+    uint8_t* raw = smem + (size_t)p.stages * b_stage;
+    const int u0 = first_unit(p, blockIdx.x), u1 = first_unit(p, blockIdx.x + 1);
+    const bool by_tma = !(MASK & 4) || p.tma == (1 << p.n_mat) - 1;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < p.stages; i++) { mbar_init(full + i, 9); mbar_init(done + i, 1); mbar_init(d_empty + i, 8); }      // the tokens' producer and eight warps of the expansion
+        for (int i = 0; i < p.raw_depth; i++) { mbar_init(raw_full + i, by_tma ? 1 : 65); mbar_init(raw_empty + i, 8); }
+        for (int i = 0; i < SCALE_RING; i++) mbar_init(s_full + i, 4);
+        dead_smem = 0;
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_smem)), "n"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    pdl_launch_dependents();
+    // tensor memory, stage by stage: sums (two k-blocks, minima), expanded k-blocks, minima
+    const uint32_t d_cols = (uint32_t)((MINS ? 3 : 2) * NT), a_base = (uint32_t)p.stages * d_cols, m_base = a_base + (uint32_t)(p.stages * 2 * p.a_cols);
+
+    if (warp < EPI_WARP) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == 0) {
+        if (lane == 0) {                                           // ---- tokens by TMA ----
+            uint32_t st = 0, par = 1, filled = 0;
+            Place q = start(p, u0);
+            pdl_wait();
+            for (int u = u0; u < u1; u++, next(p, q)) {
+                const bool mins = mins_of<MASK>(p, q.mi);
+                for (int h = 0; h < 2; h++) {
+                    wait_cta(done + st, par, dead);
+                    if (word_set(dead)) {
+                        for (uint32_t s = 0; s < filled; s++) wait_flight(full + s, s < st ? par ^ 1u : par);      // the copies in flight
+                        u = u1;
+                        break;
+                    }
+                    filled = min(filled + 1, (uint32_t)p.stages);
+                    uint8_t* d = smem + (size_t)st * b_stage;
+                    mbar_expect_tx(full + st, 6 * b_tile + (mins && h ? 64u * NT : 0u));
+#pragma unroll
+                    for (int i = 0; i < 6; i++) tma_load_2d(d + i * b_tile, &maps.x, q.b * 256 + (2 * h + i / 3) * QBK, (i % 3) * p.Mp + q.t0, full + st);      // a part lies Mp rows below the one before
+                    if (mins && h)
+#pragma unroll
+                        for (int i = 0; i < 2; i++) tma_load_2d(d + 6 * b_tile + i * NT * 32, &maps.sums, q.b * 16, i * p.Mp + q.t0, full + st);
+                    if (++st == (uint32_t)p.stages) { st = 0; par ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMA: the whole warp walks the loop, one lane issues ----
+        const uint32_t lead = elect_lane();
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | (8u << 24);
+        const uint64_t desc0 = make_desc(smem), desc32 = make_desc32(smem), part_step = (uint64_t)(b_tile >> 4), stage_step = (uint64_t)(b_stage >> 4);
+        uint32_t st = 0, par = 0;
+        int last = -1;
+        Place q = start(p, u0);
+        for (int u = u0; u < u1; u++, next(p, q)) {
+            const bool mins = mins_of<MASK>(p, q.mi);
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+                wait_cta(d_empty + st, par ^ 1u, dead);
+                wait_cta(full + st, par, dead);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t b0 = desc0 + st * stage_step;
+                const uint32_t d0 = st * d_cols, a0 = a_base + st * 2 * p.a_cols;
+#pragma unroll 1
+                for (int kb = 0; kb < 2; kb++) {
+                    const uint64_t bh = b0 + 3 * kb * part_step, bl = bh + part_step, b3 = bl + part_step;
+                    const uint32_t d = d0 + kb * NT, ah = a0 + kb * p.a_cols, al = ah + 32;
+                    uint32_t acc = 0u;
+                    auto product = [&](uint32_t a, uint64_t b) {
+                        umma_ts_by(lead, d, a, b, idesc, acc);
+#pragma unroll
+                        for (int k = 1; k < 4; k++) umma_ts_by(lead, d, a + 8 * k, b + 2 * k, idesc, 1u);
+                        acc = 1u;
+                    };
+                    // the small products first (what is left out is 2^-33 of a product)
+                    if (PAIRS && (ONE || !mins)) product(al, bl);
+                    product(ah, b3);
+                    if (PAIRS && (ONE || !mins)) product(al, bh);
+                    product(ah, bl);
+                    product(ah, bh);
+                }
+                if (MINS && mins && h) {                           // minima: 8 of them times the halves of 8 sums, twice (the third halves, and zeros, before)
+                    const uint64_t sums = desc32 + st * stage_step + 6 * part_step;
+                    umma_ts_by(lead, d0 + 2 * NT, m_base + 8 * st, sums + (NT * 32 >> 4), idesc, 0u);
+                    umma_ts_by(lead, d0 + 2 * NT, m_base + 8 * st, sums, idesc, 1u);
+                }
+                umma_commit_by(lead, done + st);
+                last = (int)(st * 2 + par);
+                if (++st == (uint32_t)p.stages) { st = 0; par ^= 1; }
+            }
+        }
+        if (word_set(dead) && last >= 0) wait_flight(done + (last >> 1), last & 1);      // given up: the products in flight
+    } else if (by_tma ? threadIdx.x == 64 : true) {
+        load_blocks<MASK>(maps, p, u0, u1, raw, raw_full, raw_empty, by_tma, dead, warp, lane);      // ---- blocks of W ----
+    }
+    } else if (warp < EXP_WARP) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
+        // ---- epilogue: a lane is a row of W; two warps share a quarter's rows, 16 tokens to each ----
+        const int quarter = warp & 3, half = (warp - EPI_WARP) >> 2, r = quarter * 32 + lane;
+        const uint32_t tq = ((uint32_t)(quarter * 32) << 16) + half * 16;
+        uint32_t st = 0, par = 0, slot = 0, spar = 0;
+        Place q = start(p, u0);
+        pdl_wait();
+        const float* token_scale = behind_wait(p.scale);
+        for (int u = u0; u < u1;) {
+            const bool mins = mins_of<MASK>(p, q.mi);
+            const int seg0 = u, end = min(u1, u + (p.NB - q.b));
+            uint64_t acc[1][8] = {};                               // pairs of tokens
+#pragma unroll 1
+            for (; u < end; u++) {
+                wait_cta(s_full + slot, spar, dead);
+                const float2 s = scales[slot][r];
+                const uint64_t fx = pack2(s.x, s.x), fy = pack2(s.y, s.y);
+                if (++slot == SCALE_RING) { slot = 0; spar ^= 1; }
+#pragma unroll 1
+                for (int h = 0; h < 2; h++) {
+                    wait_cta(done + st, par, dead);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (16 * half < NT) {
+                        uint32_t v[2][16], m[16];
+                        const uint32_t d = tq + st * d_cols;
+                        tmem_ld16(d, v[0]);
+                        tmem_ld16(d + NT, v[1]);
+                        if (MINS && mins && h) tmem_ld16(d + 2 * NT, m);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < 2; i++)
+#pragma unroll
+                            for (int j = 0; j < 8; j++) acc[0][j] = fma2(pack2(__uint_as_float(v[i][2 * j]), __uint_as_float(v[i][2 * j + 1])), fx, acc[0][j]);
+                        if (MINS && mins && h)
+#pragma unroll
+                            for (int j = 0; j < 8; j++) acc[0][j] = fma2(pack2(__uint_as_float(m[2 * j]), __uint_as_float(m[2 * j + 1])), fy, acc[0][j]);
+                    }
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(d_empty + st);
+                    if (++st == (uint32_t)p.stages) { st = 0; par ^= 1; }
+                }
+            }
+            finish_tile<1, 32>(p, q, acc, u0, seg0, end, 16 * half, r, token_scale, &last_smem, dead);
+            q.b = 0; q.tile++;
+            place(p, q);
+        }
+        if (word_set(dead)) report(p.status);
+    } else {                                                       // ---- expansion: two warps share 32 rows; a k-block of a stage to each ----
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+        const int quarter = warp & 3, odd = (warp - EXP_WARP) >> 2;
+        const uint32_t tq = (uint32_t)(quarter * 32) << 16;
+        int slot = 0, sslot = 0;
+        uint32_t st = 0, par = 1, rpar = 0;
+        Place q = start(p, u0);
+        for (int u = u0; u < u1; u++, next(p, q)) {
+            const BlkMat& m = p.mat[q.mi];
+            const int fmt = format<MASK>(m.fmt);
+            wait_cta(raw_full + slot, rpar, dead);
+            float up;
+            float2 scale;
+            const uint8_t* blk = find_block<MASK>(m, q, fmt, raw + (size_t)slot * p.raw_slot, quarter * 32 + lane, up, scale);
+            if (!odd) {
+                scales[sslot][quarter * 32 + lane] = scale;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_full + sslot);
+            }
+            if (++sslot == SCALE_RING) sslot = 0;
+#pragma unroll 1
+            for (int c = odd; c < 4; c += 2) {
+                const uint32_t a = tq + a_base + (2 * st + odd) * p.a_cols;
+                if (MINS && fmt <= 1) {
+                    uint32_t v[32];
+                    const uint4 h = lds128(blk);
+                    if ((MASK & 1) && fmt == 0) expand_k<0>(blk, h, c, v);
+                    if ((MASK & 2) && fmt == 1) expand_k<1>(blk, h, c, v);
+                    wait_cta(done + st, par, dead);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    tmem_st16(a, v);
+                    tmem_st16(a + 16, v + 16);
+                    if (c == 3) {
+                        uint32_t w[4];
+                        expand_mins(h, w);
+                        tmem_st8(tq + m_base + 8 * st, w);
+                    }
+                } else if (PAIRS) {
+                    uint32_t v[8];
+                    if ((MASK & 4) && fmt == 2) upper_bits(blk, c, v);
+#pragma unroll 1
+                    for (int hf = 0; hf < 2; hf++) {
+                        uint32_t hi[16], lo[16];
+                        if ((MASK & 4) && fmt == 2) expand_pair<2>(blk, c, hf, up, v, hi, lo);
+                        if ((MASK & 8) && fmt == 3) expand_pair<3>(blk, c, hf, up, v, hi, lo);
+                        if ((MASK & 16) && fmt == 4) expand_pair<4>(blk, c, hf, up, v, hi, lo);
+                        if (hf == 0) {
+                            wait_cta(done + st, par, dead);
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        }
+                        tmem_st16(a + 16 * hf, hi);
+                        tmem_st16(a + 32 + 16 * hf, lo);
+                    }
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full + st);
+                if (++st == (uint32_t)p.stages) { st = 0; par ^= 1; }
             }
             if (lane == 0) mbar_arrive(raw_empty + slot);          // (every lane has read what it stored)
             if (++slot == p.raw_depth) { slot = 0; rpar ^= 1; }
@@ -661,11 +929,16 @@ __global__ void __launch_bounds__(256) silu_split_kernel(uint2* __restrict__ hi,
     hi[i] = h; lo[i] = l;
 }
 
-template <int MASK, int PARTS>
-void launch_blocks(const BlkMaps& maps, const BlkParams& p, int grid, size_t smem, cudaStream_t s) {
-    static unsigned long long configured = 0;      // bit per device id
-    opt_in_dynamic_smem(gemm_blocks_kernel<MASK, PARTS>, 214 * 1024, configured);
-    launch_k_pdl(true, gemm_blocks_kernel<MASK, PARTS>, dim3(grid), dim3(Q_THREADS), smem, s, maps, p);
+template <int MASK>
+void launch_blocks(const BlkMaps& maps, const BlkParams& p, int parts, bool few, int grid, size_t smem, cudaStream_t s) {
+    static unsigned long long configured[3] = {};      // bit per device id
+    auto launch = [&](auto kernel, unsigned long long& done) {
+        opt_in_dynamic_smem(kernel, 214 * 1024, done);
+        launch_k_pdl(true, kernel, dim3(grid), dim3(Q_THREADS), smem, s, maps, p);
+    };
+    if (few) launch(gemm_blocks_few_kernel<MASK>, configured[0]);
+    else if (parts == 3) launch(gemm_blocks_kernel<MASK, 3>, configured[1]);
+    else launch(gemm_blocks_kernel<MASK, 2>, configured[2]);
     count_launch();
 }
 
@@ -685,7 +958,7 @@ bool gemm_blocks_supported(const GemvMat* mats, int n_mat, int K) { return gemv_
 static size_t parts_bytes(int T, int K, bool fine) { return gemm_f16_tc_workspace_bytes(T, K) / 2 * (fine ? 3 : 2); }
 static size_t sums_bytes(int T, int K, bool fine) { return padded(T) * ((size_t)K / 8) * (fine ? 2 : 1); }
 size_t block_tokens_bytes(int T, int K, bool fine) { return parts_bytes(T, K, fine) + sums_bytes(T, K, fine) + padded(T) * sizeof(float) + (size_t)sm_count() * sizeof(unsigned); }
-// tokens of a tile
+// tokens of a tile, as even as they come
 static int tile_tokens(int T) { const int cols = (T + NT_MAX - 1) / NT_MAX; return ((T + cols - 1) / cols + 15) / 16 * 16; }
 size_t block_scratch_bytes(int T) { return (size_t)sm_count() * 2 * 128 * (T > NT_MAX ? NT_MAX : tile_tokens(T)) * sizeof(float); }
 
@@ -750,6 +1023,7 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     p.scale = x.scale;
     p.kc = x.fine ? 1 : p.NB == 1 ? 2 : 4;
     const int parts = x.fine ? 3 : 2;
+    const bool few = x.fine && T <= FEW_TOKENS;
     int tiles = 0, slot = 0, mask = 0;
     for (int i = 0; i < n_mat; i++) {
         BlkMat& m = p.mat[i];
@@ -768,15 +1042,22 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     // fewer tokens there are: weights from HBM are then what bounds)
     p.a_cols = pairs ? 64 : 32;
     p.raw_slot = slot;
-    p.b_stage = (p.NT * (128 * parts + (mins ? 32 * (parts - 1) : 0)) + 1023) / 1024 * 1024;
     const size_t cap = 213 * 1024;
-    for (p.stages = STAGES_MAX; p.stages > 2; p.stages--) {
+    if (few) {                                                     // a stage is two k-blocks, with sums of its own
+        const int cols = (mins ? 3 : 2) * p.NT + 2 * p.a_cols + (mins ? 8 : 0);
+        p.b_stage = (p.NT * (6 * 128 + (mins ? 64 : 0)) + 1023) / 1024 * 1024;
+        p.stages = std::min(STAGES_MAX, 512 / cols);
+    } else {
+        p.b_stage = (p.NT * (128 * parts + (mins ? 32 * (parts - 1) : 0)) + 1023) / 1024 * 1024;
+        for (p.stages = STAGES_MAX; p.stages > 2; p.stages--) {
+            p.d_bufs = std::min(D_BUFS_MAX, (512 - p.stages * p.a_cols - (mins ? 8 : 0)) / p.NT);
+            if (p.d_bufs >= (mins ? 3 : 2) && (size_t)p.stages * p.b_stage + 2 * (size_t)slot <= cap) break;
+        }
         p.d_bufs = std::min(D_BUFS_MAX, (512 - p.stages * p.a_cols - (mins ? 8 : 0)) / p.NT);
-        if (p.d_bufs >= (mins ? 3 : 2) && (size_t)p.stages * p.b_stage + 2 * (size_t)slot <= cap) break;
+        if (p.d_bufs < 2) return false;
     }
-    p.d_bufs = std::min(D_BUFS_MAX, (512 - p.stages * p.a_cols - (mins ? 8 : 0)) / p.NT);
     p.raw_depth = (int)std::min<size_t>(RAW_MAX, (cap - (size_t)p.stages * p.b_stage) / slot);
-    if (p.raw_depth < 1 || p.d_bufs < 2) return false;
+    if (p.raw_depth < 1) return false;
     const int grid = std::min(sms, p.units);
     p.part = static_cast<float*>(scratch);
     p.count = x.count;
@@ -791,10 +1072,10 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
         p.tma |= 1 << i;
     }
     const size_t smem = p.stages * (size_t)p.b_stage + (size_t)p.raw_depth * slot + 1024;
-#define NT_BLOCKS(M) case M: parts == 3 ? launch_blocks<M, 3>(maps, p, grid, smem, s) : launch_blocks<M, 2>(maps, p, grid, smem, s); break
+#define NT_BLOCKS(M) case M: launch_blocks<M>(maps, p, parts, few, grid, smem, s); break
     switch (mask) {
         NT_BLOCKS(1); NT_BLOCKS(2); NT_BLOCKS(4); NT_BLOCKS(5); NT_BLOCKS(8); NT_BLOCKS(16);
-        default: parts == 3 ? launch_blocks<31, 3>(maps, p, grid, smem, s) : launch_blocks<31, 2>(maps, p, grid, smem, s); break;
+        default: launch_blocks<31>(maps, p, parts, few, grid, smem, s); break;
     }
 #undef NT_BLOCKS
     return true;

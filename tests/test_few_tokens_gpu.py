@@ -1,0 +1,24 @@
+"""The GEMM over blocks in its form for up to 32 tokens (csrc/prefill_blocks.cu, gemm_blocks_few_kernel): the edges of its token tiles, runs of a single super-block, tiles
+shared by several CTAs, and formats with and without minima in one launch."""
+import pytest
+
+torch = pytest.importorskip("torch")
+from ntransformer_b200.dtypes import DType  # noqa: E402
+from test_block_products_gpu import FORMATS, activations, matrix, rel  # noqa: E402
+from test_block_tokens_gpu import bound, product  # noqa: E402
+
+pytestmark = [pytest.mark.gpu]
+
+
+@pytest.mark.parametrize("dts", [(d,) for d in FORMATS] + [(DType.Q4_K_M, DType.Q4_K_M, DType.Q6_K), (DType.Q6_K, DType.Q5_K), (DType.Q8_0, DType.Q4_K_M, DType.Q4_0)],
+                         ids=lambda d: "+".join(t.name for t in d))
+@pytest.mark.parametrize("tokens", [1, 16, 17, 32, 33])
+@pytest.mark.parametrize("rows,cols", [(128, 256), (300, 512), (129, 7168), (20000, 512)])
+def test_products(dts, tokens, rows, cols):
+    outs = [rows, 33, 128][: len(dts)]
+    mats = [matrix(d, o, cols, o) for d, o in zip(dts, outs)]
+    x = activations(tokens, cols, cols + tokens)
+    ys = [torch.full((tokens + 1, o), 7.0, device="cuda") for o in outs]
+    product(ys, [m[0] for m in mats], outs, dts, x, fine=True)
+    for y, d, (_, W64) in zip(ys, dts, mats):
+        assert rel(y[:tokens], x.double() @ W64.T) <= bound(d, 64) and (y[tokens] == 7.0).all()

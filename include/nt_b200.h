@@ -112,6 +112,10 @@ int    nt_b200_gemm_blocks_ws(int n_mat, float* const* C, const void* const* W, 
  * tensor cores instead of 256, and tokens in three halves instead of two.  What it needs beside its arguments is stream-ordered memory of the call.  Returns 0, or < 0 when rejected. */
 int    nt_b200_gemm_blocks(int n_mat, float* const* C, const void* const* W, const int* out_features, const int* dtypes, int in_features,
                            const float* x, const float* norm_w, float eps, int tokens, int fine, int add, void* stream);
+/* The same over up to three F16 or BF16 matrices (dtype, one for all; dense rows on 16 bytes, in_features a multiple of 256): C_i (+)= alpha * col_scale[n] * X . W_i^T (col_scale may be
+ * NULL).  fine: tokens in three halves (BF16: three of its numbers) and 64 columns to an accumulator, otherwise two and 256.  Returns 0, or < 0 when rejected (nothing launched). */
+int    nt_b200_gemm_dense_tc(int n_mat, float* const* C, const void* const* W, const int* out_features, int dtype, int in_features, const float* x, const float* norm_w, float eps,
+                          int tokens, int fine, int add, const float* col_scale, float alpha, void* stream);
 /* The decode step's attention sub-block in ONE launch: launch_rope (src/cuda/rotary.cu:113-140; q and k are read, not
  * modified) + launch_copy_to_kv_cache at row *pos_dev (src/cuda/attention.cu:405-425) + launch_attention_decode over
  * *pos_dev + 1 keys (src/cuda/attention.cu:348-375), context split over CTAs, merged by the last CTA of each head group.

@@ -30,10 +30,6 @@ template <int HD> struct TcSmem {
     static constexpr int K0 = 4 * Q, V0 = K0 + 2 * KV, ALL = V0 + KV;
 };
 
-__device__ __forceinline__ void umma_ss_by(uint32_t lead, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
-}
 // Values as the B operand: N (channels) contiguous, SWIZZLE_128B: 64 channels x 8 keys to an atom of 1024 bytes, the next 8 keys 1024 bytes on (stride offset), the
 // next 64 channels a whole box on (leading offset)
 __device__ __forceinline__ uint64_t make_desc_mn(const void* smem_ptr, uint32_t box_bytes) {

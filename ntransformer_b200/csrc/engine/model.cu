@@ -787,12 +787,23 @@ bool Model::batched_prefill_ok(int seq_len, int start_pos) const {
     return true;
 }
 
-// A few tokens together, every matrix in blocks, one GPU: the decode step's arithmetic (gemv_rows.cu) or, where that takes two passes, the GEMM over blocks (prefill_blocks.cu).
+// A few tokens together, one GPU.  Every matrix in blocks: the decode step's arithmetic (gemv_rows.cu) or, where that takes two passes, the GEMM over blocks (prefill_blocks.cu).
+// Every matrix F16: prefill_dense.cu's fine form.
 bool Model::short_batch_ok(int seq_len, int start_pos) const {
     if (tp_size_ != 1 || seq_len < 2 || prefill_min_tokens_ <= 0 || getenv("NT_B200_NO_BATCHED_PREFILL") || (fuse_mask_ & 6)) return false;
     const char* mk = getenv("NT_B200_MEGAKERNEL");
     if (mk ? env_on("NT_B200_MEGAKERNEL") : use_mega_) return false;
-    return chain_ok();
+    return chain_ok() || dense_short_ok();
+}
+
+static GemvMat dense_mat(const Weight& w, float* y) { GemvMat m; m.W = w.ptr; m.y = y; m.out = w.rows; m.dtype = w.dtype; m.row_pitch = w.pitch; return m; }
+static bool f16_dense(const Weight& w) { const GemvMat m = dense_mat(w, nullptr); return w.dtype == DType::F16 && gemm_dense_tc_supported(&m, 1, w.cols); }
+bool Model::dense_short_ok() const {
+    if (cfg_.layer_spec()) return false;
+    for (const LayerWeights& L : layers_)
+        for (const Weight* w : {&L.wq, &L.wk, &L.wv, &L.wo, &L.gate, &L.up, &L.down})
+            if (!f16_dense(*w)) return false;
+    return true;
 }
 
 // Buffers cut out of one allocation: each of a dozen of its own costs the first prompt of a model as much as a launch of it
@@ -835,7 +846,8 @@ bool Model::ensure_short_buffers() {
 // false: no room for the GEMM's scratch; nothing launched
 bool Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
     cudaStream_t s = stream_;
-    if (seq_len > 8 && !ensure_block_scratch(std::min(SHORT_CHUNK, seq_len))) return false;      // where a chunk is more than a pass of gemv_rows
+    const bool dense = dense_short_ok();
+    if ((dense || seq_len > 8) && !ensure_block_scratch(std::min(SHORT_CHUNK, seq_len))) return false;      // where a chunk is more than a pass of gemv_rows
     const int hidden = cfg_.hidden_size, hd = cfg_.head_dim, max_seq = cfg_.max_seq_len, qdim = nh_l_ * hd;
     const size_t kv_stride = (size_t)max_seq * nkv_l_ * hd;
     int T = 0;
@@ -845,6 +857,11 @@ bool Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
         GemvMat m[3];
         int n = 0;
         for (auto& [w, y] : list) { m[n].W = w->ptr; m[n].y = y; m[n].out = w->rows; m[n].dtype = w->dtype; m[n++].row_pitch = w->pitch; }
+        if (dense) {
+            const BlockTokens t = up ? silu_split_tokens(sb_.ws, x, up, T, K, true, s) : split_tokens(sb_.ws, x, norm, cfg_.norm_eps, T, K, true, s);
+            NT_CHECK(gemm_dense_tc(m, n, K, t, block_scratch_->p, T, ep == GEMV_ADD, s), "GEMM of a few tokens over F16 rejected");
+            return ep == GEMV_SWIGLU;
+        }
         if (!gemm_blocks_for_few(m, n, T)) {
             if (up) silu_mul(const_cast<float*>(x), x, up, T * K, s);
             quantize_rows(sb_.ws, x, norm, cfg_.norm_eps, T, K, s);
@@ -879,7 +896,7 @@ bool Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
         if (!want_.empty()) emit_wanted(sb_.x, c0, T, s);
     }
     copy(hidden_, sb_.x + (size_t)(T - 1) * hidden, hidden, s);
-    step_head(s, true);
+    step_head(s, chain_ok());
     return true;
 }
 
@@ -906,13 +923,24 @@ void Model::prefill_gemms(float* const* C, void* ws, const float* x, const float
         GemvMat& b = m[n_blocks++];
         b.W = w[i]->ptr; b.y = C[i]; b.out = w[i]->rows; b.dtype = w[i]->dtype; b.row_pitch = w[i]->pitch;
     }
+    bool dense = n_plain && block_scratch_;
+    for (int i = 0; i < n_plain; i++) dense = dense && f16_dense(*plain[i]);
+    bool together = !add && n_plain > 1;                           // F16 in place: narrow matrices fill the SMs together
+    const void* W[TC_MULTI_MAX]; int N[TC_MULTI_MAX];
+    for (int i = 0; i < n_plain; i++) { together = together && f16_direct(*plain[i]) && plain[i]->rows >= 256; W[i] = plain[i]->ptr; N[i] = plain[i]->rows; }
+    if (dense && gemm_dense_tc_pays(N, n_plain, T, K, together)) {
+        GemvMat d[3];
+        for (int i = 0; i < n_plain; i++) d[i] = dense_mat(*plain[i], c[i]);
+        BlockTokens t;
+        t.split = ws; t.count = pf_.count;
+        if (x) t = split_tokens(ws, x, norm_w, cfg_.norm_eps, T, K, false, s);
+        NT_CHECK(gemm_dense_tc(d, n_plain, K, t, block_scratch_->p, T, add, s), "prefill GEMM over F16 rejected");
+        n_plain = 0;
+    }
     if (n_plain && x) {
         if (norm_w) rmsnorm_split(ws, x, norm_w, T, K, cfg_.norm_eps, s);
         else split_activations(ws, x, T, K, s);
     }
-    bool together = !add && n_plain > 1;                           // F16 in place: narrow matrices fill the SMs together
-    const void* W[TC_MULTI_MAX]; int N[TC_MULTI_MAX];
-    for (int i = 0; i < n_plain && together; i++) { together = f16_direct(*plain[i]) && plain[i]->rows >= 256; W[i] = plain[i]->ptr; N[i] = plain[i]->rows; }
     if (!together || !gemm_f16_tc_multi_ws(c, ws, W, N, n_plain, T, K, s)) for (int i = 0; i < n_plain; i++) prefill_gemm(c[i], ws, *plain[i], T, add, s);
     if (n_blocks) {
         const BlockTokens t = x ? split_tokens(ws, x, norm_w, cfg_.norm_eps, T, K, false, s) : resplit_tokens(ws, ws, static_cast<uint8_t*>(ws) + gemm_f16_tc_workspace_bytes(T, K) / 2, T, K, s);
@@ -946,12 +974,14 @@ void Model::ensure_prefill_buffers(int tokens) {
     c.want(pf_.ws, block_tokens_bytes((int)T, (int)std::max(hidden, qdim), false));
     c.want(pf_.ws2, block_tokens_bytes((int)T, inter_l_, false));
     c.want(pf_.tok, T * sizeof(int)); c.want(pf_.pos, T * sizeof(int));
+    c.want(pf_.count, dense_count_bytes());
     size_t w_elems = 0;                  // largest matrix that needs the dequantised scratch pair
     bool swiglu_unfused = false;
-    any_blocks_ = false;
+    any_blocks_ = any_f16_ = false;
     for (const LayerWeights& L : layers_) {
         for (const Weight* w : {&L.wq, &L.wk, &L.wv, &L.wo, &L.gate, &L.up, &L.down})
-            if (blocks_direct(*w)) any_blocks_ = true;
+            if (f16_dense(*w)) any_f16_ = true;
+            else if (blocks_direct(*w)) any_blocks_ = true;
             else if (!f16_direct(*w)) w_elems = std::max(w_elems, (size_t)w->rows * (size_t)w->cols);
         swiglu_unfused = swiglu_unfused || !f16_direct(L.gate) || !f16_direct(L.up);
     }
@@ -970,6 +1000,7 @@ void Model::prefill_batched(const int* tokens, int seq_len, int start_pos) {
     const size_t kv_stride = (size_t)max_seq * nkv_l_ * hd;
     ensure_prefill_buffers(std::min(seq_len, PREFILL_CHUNK));
     if (any_blocks_) NT_CHECK(ensure_block_scratch(std::min(seq_len, PREFILL_CHUNK)), "no room for the scratch of the prompt GEMM over blocks");
+    if (any_f16_ && ensure_block_scratch(std::min(seq_len, PREFILL_CHUNK))) NT_CUDA_CHECK(cudaMemsetAsync(pf_.count, 0, dense_count_bytes(), s));
     int last_rows = 0;
     for (int c0 = 0, T = 0; c0 < seq_len; c0 += T) {
         // A ragged tail of 1..15 tokens would miss the tiled attention kernel's 16-token minimum (and the per-query kernel it
@@ -1038,7 +1069,8 @@ void Model::forward_async(const int* tokens, int seq_len, int start_pos) {
     for (int t = 0; t < seq_len; t++) NT_CHECK(tokens[t] >= 0 && tokens[t] < cfg_.vocab_size, "token id out of range");
     const LaunchScope scope(programmatic() ? launches() : Launches::Plain);
     if (cfg_.layer_spec()) {
-        if (prefill_min_tokens_ > 0 && seq_len >= prefill_min_tokens_ && !getenv("NT_B200_NO_BATCHED_PREFILL")) { prefill_spec(tokens, seq_len, start_pos); return; }
+        const bool few = seq_len > 2 && seq_len < SPEC_FEW && spec_few_ready(seq_len);      // (two tokens, two layers of 4096: 305 us one by one, 337)
+        if (few || (prefill_min_tokens_ > 0 && seq_len >= prefill_min_tokens_ && !getenv("NT_B200_NO_BATCHED_PREFILL"))) { prefill_spec(tokens, seq_len, start_pos, few); return; }
     } else if (batched_prefill_ok(seq_len, start_pos)) { prefill_batched(tokens, seq_len, start_pos); return; }
     else if (short_batch_ok(seq_len, start_pos) && ensure_short_buffers() && prefill_short(tokens, seq_len, start_pos)) return;
     size_t w = 0;

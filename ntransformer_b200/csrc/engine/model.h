@@ -169,10 +169,12 @@ public:
     bool blocks_direct(const Weight& w) const;
     void prefill_gemms(float* const* C, void* ws, const float* x, const float* norm_w, const Weight* const* w, int n, int T, bool add, cudaStream_t s);
     void *pf_arena_ = nullptr, *sb_arena_ = nullptr;               // pf_ (but a layer-spec model's) and sb_ lie in
+    bool any_f16_ = false;                                        // some of their matrices are F16 that prefill_dense.cu takes
     bool any_blocks_ = false;                                     // prompts go through the GEMM over blocks
     bool ensure_block_scratch(int tokens);
     std::unique_ptr<CallMemory> block_scratch_;
     size_t block_scratch_bytes_ = 0;
+    bool dense_short_ok() const;                                  // every matrix F16 as the GEMM of a few tokens takes it
     bool ensure_short_buffers();
     bool prefill_short(const int* tokens, int seq_len, int start_pos);
     struct { float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *attn = nullptr, *g = nullptr, *u = nullptr, *scratch = nullptr; void* ws = nullptr;
@@ -253,9 +255,14 @@ private:
     bool finalize_spec();
     void step_body_spec(cudaStream_t s);
     void step_head_spec(cudaStream_t s);
-    void prefill_spec(const int* tokens, int seq_len, int start_pos);
+    void prefill_spec(const int* tokens, int seq_len, int start_pos, bool few);
     void ensure_prefill_buffers_spec(int tokens);
     bool spec_tc_ok(const Weight& w) const;
+    // Fewer tokens than SPEC_FEW together through gemm_dense_tc, as exact as one by one; ready: the buffers are there
+    static constexpr int SPEC_FEW = 16;
+    bool spec_dense_short_ok() const;
+    bool spec_few_ready(int tokens);
+    bool spec_dense(float* const* C, const void* A_split, const Weight* const* w, int n, int T, bool add, const float* row_scale, float alpha, cudaStream_t s);      // by gemm_dense_tc, where that pays
     void spec_gemm(float* C, const float* A, const void* A_split, const Weight& w, int T, DenseEpilogue ep, const float* row_scale, float alpha, cudaStream_t s);
     void emit_wanted(const float* x_rows, int c0, int T, cudaStream_t s);   // logits of the wanted places inside tokens [c0, c0 + T)
     const ModelFamily* family_ = nullptr;
@@ -343,6 +350,7 @@ private:
         float *g = nullptr, *u = nullptr;     // gate / up activations (only when those weights are not F16: unfused SwiGLU)
         void *whi = nullptr, *wlo = nullptr;  // dequantised weight matrix as an F16 hi/lo pair (quantised models)
         int *tok = nullptr, *pos = nullptr;
+        unsigned* count = nullptr;            // gemm_dense_tc's, for splits that other kernels than split_tokens laid out; zeros between launches
         float *h = nullptr, *tmp = nullptr;   // layer-spec families: the block's normed input (read by both branches), a GEMM result before its scaled add
         void *hws = nullptr;                  // ... and its F16 hi/lo split
         float *xs = nullptr, *maps = nullptr;     // STREAMS: the residual streams [T, S, width]; attention maps' outputs [T, heads * maps * vdim]

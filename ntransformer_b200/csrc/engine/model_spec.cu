@@ -510,7 +510,7 @@ void Model::ensure_prefill_buffers_spec(int tokens) {
     if (tokens <= pf_.cap) return;
     NT_CUDA_CHECK(cudaStreamSynchronize(stream_));
     for (void* p : {(void*)pf_.x, (void*)pf_.q, (void*)pf_.k, (void*)pf_.v, (void*)pf_.attn, (void*)pf_.g, (void*)pf_.u, (void*)pf_.h, (void*)pf_.tmp,
-                    pf_.ws, pf_.ws2, pf_.hws, (void*)pf_.tok, (void*)pf_.xs, (void*)pf_.maps, (void*)pf_.sel, (void*)pf_.work, (void*)pf_.wt, (void*)pf_.sgate,
+                    pf_.ws, pf_.ws2, pf_.hws, (void*)pf_.count, (void*)pf_.tok, (void*)pf_.xs, (void*)pf_.maps, (void*)pf_.sel, (void*)pf_.work, (void*)pf_.wt, (void*)pf_.sgate,
                     (void*)pf_.act_rows, (void*)pf_.y_rows, (void*)pf_.g2, pf_.moe_ws, pf_.moe_ws2, (void*)pf_.gate_rows, (void*)pf_.wide})
         if (p) cudaFree(p);
     pf_.moe_ws2 = nullptr; pf_.wide = nullptr;
@@ -553,7 +553,7 @@ void Model::ensure_prefill_buffers_spec(int tokens) {
     pf_.q = dmalloc<float>(T * qmax); pf_.k = dmalloc<float>(T * kmax); pf_.v = dmalloc<float>(T * vmax); pf_.attn = dmalloc<float>(T * omax);
     pf_.g = dmalloc<float>(T * ffmax); pf_.u = dmalloc<float>(T * ffmax);
     pf_.tok = dmalloc<int>(T);
-    pf_.ws = pf_.ws2 = pf_.hws = nullptr;
+    pf_.ws = pf_.ws2 = pf_.hws = nullptr; pf_.count = nullptr;
     if (post_form && topmax > 0) pf_.gate_rows = dmalloc<float>(T * topmax * effmax);      // the gate half of the gated experts' rows
     if (post_form && topmax > 0 && !exact32_) pf_.moe_ws2 = dmalloc<uint8_t>(gemm_f16_tc_workspace_bytes((int)(T * topmax + emax * 128), (int)effmax));
     bool any_tc = false;
@@ -587,9 +587,11 @@ void Model::ensure_prefill_buffers_spec(int tokens) {
         any_tc = false;
     }
     if (any_tc) {                         // BF16 hi/lo splits of the three GEMM inputs (normed block input, attention output, gated activation)
-        pf_.hws = dmalloc<uint8_t>(gemm_f16_tc_workspace_bytes((int)T, (int)hidden));
-        pf_.ws = dmalloc<uint8_t>(gemm_f16_tc_workspace_bytes((int)T, (int)omax));
-        pf_.ws2 = dmalloc<uint8_t>(gemm_f16_tc_workspace_bytes((int)T, (int)ffmax));
+        auto split = [&](size_t K) { return dmalloc<uint8_t>(std::max(gemm_f16_tc_workspace_bytes((int)T, (int)K), block_tokens_bytes(SPEC_FEW, (int)K, true))); };      // (a few tokens: in three parts)
+        pf_.hws = split(hidden);
+        pf_.ws = split(omax);
+        pf_.ws2 = split(ffmax);
+        pf_.count = reinterpret_cast<unsigned*>(dmalloc<uint8_t>(dense_count_bytes()));
     }
     pf_.cap = (int)T;
 }
@@ -600,9 +602,54 @@ bool Model::spec_tc_ok(const Weight& w) const {
     return !exact32_ && !off && w.dtype == DType::BF16 && gemm_f16_tc_ragged_supported(w.ptr, w.rows, w.cols, w.pitch);
 }
 
+static bool bf16_dense(const Weight& w) { const GemvMat m = mat_of(w, nullptr); return w.dtype == DType::BF16 && gemm_dense_tc_supported(&m, 1, w.cols); }
+// Zelunex' form alone: the other families' rows take other ways
+bool Model::spec_dense_short_ok() const {
+    if (exact32_ || prefill_min_tokens_ <= 0 || parallel_rows() || getenv("NT_B200_NO_TC_PREFILL") || getenv("NT_B200_NO_BATCHED_PREFILL")) return false;
+    const BlockForm f = cfg_.layers[0].form;
+    if (f == BlockForm::SANDWICH || f == BlockForm::STREAMS || f == BlockForm::POST_NORM || f == BlockForm::SUM_NORM) return false;
+    for (int i = 0; i < cfg_.n_layers; i++) {
+        const LayerWeights& L = layer_weights(i);
+        for (const Weight* w : {&L.wq, &L.wk, &L.wv, &L.wo, &L.gate, &L.up, &L.down})
+            if ((cfg_.layers[(size_t)i].ff > 0 || (w != &L.gate && w != &L.up && w != &L.down)) && !bf16_dense(*w)) return false;
+    }
+    return true;
+}
+// false: the caller takes the tokens one by one, which needs no buffers
+bool Model::spec_few_ready(int tokens) {
+    if (!spec_dense_short_ok()) return false;
+    if (!pf_.cap) {
+        size_t free_bytes = 0, total = 0, widest = (size_t)cfg_.hidden_size, rows = 4 * widest;
+        for (const LayerSpec& S : cfg_.layers) {
+            const size_t q = (size_t)S.heads * S.dim, k = (size_t)S.kv_heads * S.dim, v = (size_t)S.kv_heads * S.vdim, o = (size_t)S.heads * S.vdim;
+            widest = std::max({widest, o, (size_t)S.ff});
+            rows = std::max(rows, 4 * (size_t)cfg_.hidden_size + q + k + v + o + 2 * (size_t)S.ff);
+        }
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (free_bytes < 128 * rows * sizeof(float) + 3 * block_tokens_bytes(SPEC_FEW, (int)widest, true) + (64u << 20)) return false;
+    }
+    ensure_prefill_buffers_spec(tokens);
+    return pf_.count && ensure_block_scratch(tokens);
+}
+bool Model::spec_dense(float* const* C, const void* A_split, const Weight* const* w, int n, int T, bool add, const float* row_scale, float alpha, cudaStream_t s) {
+    if (!A_split || !block_scratch_ || !pf_.count) return false;
+    int N[3];
+    GemvMat m[3];
+    for (int i = 0; i < n; i++) {
+        if (!spec_tc_ok(*w[i]) || !bf16_dense(*w[i])) return false;
+        N[i] = w[i]->rows; m[i] = mat_of(*w[i], C[i]);
+    }
+    if (!gemm_dense_tc_pays(N, n, T, w[0]->cols, false)) return false;
+    BlockTokens t;
+    t.split = const_cast<void*>(A_split); t.count = pf_.count;
+    return gemm_dense_tc(m, n, w[0]->cols, t, block_scratch_->p, T, add, s, row_scale, alpha);
+}
+
 // C (ep)= A . W^T for T prompt rows: on the tensor cores from the BF16 hi/lo split of A when the matrix qualifies, else in FP32
 // on CUDA cores from A itself.  Either input may be null when the caller knows which path the matrix takes.
 void Model::spec_gemm(float* C, const float* A, const void* A_split, const Weight& w, int T, DenseEpilogue ep, const float* row_scale, float alpha, cudaStream_t s) {
+    const Weight* one = &w;
+    if (spec_dense(&C, A_split, &one, 1, T, ep != DENSE_STORE, ep == DENSE_SCALED_ADD ? row_scale : nullptr, ep == DENSE_SCALED_ADD ? alpha : 1.f, s)) return;
     if (A_split && spec_tc_ok(w)) {
         TcOpts o;
         o.bf16 = true;
@@ -617,11 +664,12 @@ void Model::spec_gemm(float* C, const float* A, const void* A_split, const Weigh
 // A prompt (or a portion of one: start_pos > 0) in chunks of up to SPEC_PREFILL_CHUNK tokens.  The chunk's key / value rows go to
 // the cache first, then the attention kernel reads cache rows only — earlier portions, the kept first tokens and the chunk itself
 // alike — so where a prompt is cut cannot change what a query sees.
-void Model::prefill_spec(const int* tokens, int seq_len, int start_pos) {
+void Model::prefill_spec(const int* tokens, int seq_len, int start_pos, bool few) {
     cudaStream_t s = stream_;
     const int hidden = cfg_.hidden_size;
     const float m = cfg_.residual_mult;
     ensure_prefill_buffers_spec(std::min(seq_len, SPEC_PREFILL_CHUNK));
+    if (pf_.count && ensure_block_scratch(std::min(seq_len, SPEC_PREFILL_CHUNK))) NT_CUDA_CHECK(cudaMemsetAsync(pf_.count, 0, dense_count_bytes(), s));
     int last_rows = 0;
     for (int c0 = 0; c0 < seq_len; c0 += SPEC_PREFILL_CHUNK) {
         const int T = std::min(SPEC_PREFILL_CHUNK, seq_len - c0), p0 = start_pos + c0;
@@ -649,6 +697,26 @@ void Model::prefill_spec(const int* tokens, int seq_len, int start_pos) {
             if (post_form) { layer_postnorm(i, T, pf_.tok, nullptr, p0, rb, s); continue; }
             const LayerSpec& S = cfg_.layers[(size_t)i];
             const LayerWeights& L = layer_weights(i);
+            if (few) {
+                const int odim = S.heads * S.vdim;
+                const BlockTokens h = split_tokens(pf_.hws, pf_.x, L.attn_norm, cfg_.norm_eps, T, hidden, true, s, true);
+                const GemvMat qkv[3] = {mat_of(L.wq, pf_.q), mat_of(L.wk, pf_.k), mat_of(L.wv, pf_.v)}, o = mat_of(L.wo, pf_.x), gu[2] = {mat_of(L.gate, pf_.g), mat_of(L.up, pf_.u)},
+                              down = mat_of(L.down, pf_.x);
+                auto gemm = [&](const GemvMat* mats, int n, int K, const BlockTokens& t, bool add, const float* ls) {
+                    NT_CHECK(gemm_dense_tc(mats, n, K, t, block_scratch_->p, T, add, s, ls, add ? m : 1.f), "GEMM of a few tokens over BF16 rejected");
+                };
+                gemm(qkv, 3, hidden, h, false, nullptr);
+                if (S.ff > 0) gemm(gu, 2, hidden, h, false, nullptr);      // (before x changes)
+                qk_norm_kv_write(pf_.q, pf_.k, pf_.v, L.q_norm, L.k_norm, cfg_.norm_eps, kcs_[(size_t)i], vcs_[(size_t)i], cache_dt_, T, nullptr, p0,
+                                 S.heads * S.dim, S.kv_heads * S.dim, S.kv_heads * S.vdim, s);
+                attention_window(pf_.attn, pf_.q, kcs_[(size_t)i], vcs_[(size_t)i], cache_dt_, T, nullptr, p0, cfg_.max_seq_len, attn_of(S), s);
+                gemm(&o, 1, odim, split_tokens(pf_.ws, pf_.attn, nullptr, 0.f, T, odim, true, s, true), true, L.ls1);
+                if (S.ff > 0) {
+                    glu_mul(pf_.g, pf_.g, pf_.u, (size_t)T * S.ff, S.act == GluAct::GELU_TANH, s);
+                    gemm(&down, 1, S.ff, split_tokens(pf_.ws2, pf_.g, nullptr, 0.f, T, S.ff, true, s, true), true, L.ls2);
+                }
+                continue;
+            }
             // the block's normed input feeds q, k, v, gate and up: as FP32 rows, as a BF16 split, or both, by what those matrices take
             bool h_f32 = false, h_split = false;
             auto reads_h = [&](const Weight& w) { if (spec_tc_ok(w)) h_split = true; else h_f32 = true; };
@@ -658,9 +726,10 @@ void Model::prefill_spec(const int* tokens, int seq_len, int start_pos) {
             if (h_split) rmsnorm_split(pf_.hws, pf_.x, L.attn_norm, T, hidden, cfg_.norm_eps, s, true);
             const float* hf = h_f32 ? pf_.h : nullptr;
             const void* hs = h_split ? pf_.hws : nullptr;
-            spec_gemm(pf_.q, hf, hs, L.wq, T, DENSE_STORE, nullptr, 1.f, s);
-            spec_gemm(pf_.k, hf, hs, L.wk, T, DENSE_STORE, nullptr, 1.f, s);
-            spec_gemm(pf_.v, hf, hs, L.wv, T, DENSE_STORE, nullptr, 1.f, s);
+            const Weight* qkv[3] = {&L.wq, &L.wk, &L.wv};
+            float* qkv_out[3] = {pf_.q, pf_.k, pf_.v};
+            if (!spec_dense(qkv_out, hs, qkv, 3, T, false, nullptr, 1.f, s))
+                for (int j = 0; j < 3; j++) spec_gemm(qkv_out[j], hf, hs, *qkv[j], T, DENSE_STORE, nullptr, 1.f, s);
             qk_norm_kv_write(pf_.q, pf_.k, pf_.v, L.q_norm, L.k_norm, cfg_.norm_eps, kcs_[(size_t)i], vcs_[(size_t)i], cache_dt_, T, nullptr, p0,
                              S.heads * S.dim, S.kv_heads * S.dim, S.kv_heads * S.vdim, s);
             attention_window(pf_.attn, pf_.q, kcs_[(size_t)i], vcs_[(size_t)i], cache_dt_, T, nullptr, p0, cfg_.max_seq_len, attn_of(S), s);

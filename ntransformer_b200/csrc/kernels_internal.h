@@ -577,7 +577,7 @@ bool gemm_blocks_supported(const GemvMat* mats, int n_mat, int K);
 // the power of two that each token was divided by, and the counts of the product that follows, cleared.
 struct BlockTokens { void* split = nullptr; void* sums = nullptr; float* scale = nullptr; unsigned* count = nullptr; bool fine = false; };
 size_t block_tokens_bytes(int T, int K, bool fine);
-BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w /* null: x itself */, float eps, int T, int K, bool fine, cudaStream_t s);
+BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w /* null: x itself */, float eps, int T, int K, bool fine, cudaStream_t s, bool bf16 = false);
 BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, bool fine, cudaStream_t s);
 BlockTokens resplit_tokens(void* workspace, const void* hi, const void* lo, int T, int K, cudaStream_t s);      // of a plain split's rows, in place too
 // scratch: block_scratch_bytes() for as many tokens or more, whatever they hold, of one stream's.  fine: 64 columns to an accumulator, as exact as
@@ -592,6 +592,16 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
 bool gemm_blocks_for_few(const GemvMat* mats, int n_mat, int tokens);
 // over F32 tokens, or (x null) over split_activations' layout
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const float* norm_w, float eps, const void* split, bool fine, int T, bool add, cudaStream_t s);
+// prefill_dense.cu: the same over up to three F16 or BF16 matrices (one type, dense rows on 16 bytes, K a multiple of 256): C_i (+)= alpha * col_scale[n] * X . W_i^T.  x as laid out by
+// split_tokens (fine: in three parts), or a plain split of split_activations / rmsnorm_split, BF16 for BF16 matrices (scale null; count: zeroed words, one to an SM, left zeroed).
+// Reads the matrices ahead of its wait, as gemm_blocks does.
+bool gemm_dense_tc_supported(const GemvMat* mats, int n_mat, int K);
+size_t dense_count_bytes();
+// Whether it is faster over n matrices of N[i] rows than prefill_gemm.cu's tiles (together: all in one launch there), tokens in two parts either way
+bool gemm_dense_tc_pays(const int* N, int n, int T, int K, bool together);
+bool gemm_dense_tc(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, int T, bool add, cudaStream_t s, const float* col_scale = nullptr, float alpha = 1.0f);
+bool gemm_dense_tc(const GemvMat* mats, int n_mat, int K, const float* x, const float* norm_w, float eps, bool fine, int T, bool add, cudaStream_t s, const float* col_scale = nullptr,
+                float alpha = 1.0f);      // over F32 tokens, in memory of the call
 void silu_mul_split(void* workspace, const float* gate, const float* up, int rows, int cols, cudaStream_t s);
 // prefill_gemm.cu: tcgen05/TMEM GEMM, C[M,N] = A[M,K] (F32, split hi+lo F16) . W[N,K]^T (F16)
 size_t gemm_f16_tc_workspace_bytes(int M, int K);

@@ -176,6 +176,13 @@ int nt_b200_gemm_blocks(int n_mat, float* const* C, const void* const* W, const 
     for (int i = 0; i < n_mat; i++) { m[i].W = W[i]; m[i].y = C[i]; m[i].out = out_features[i]; m[i].dtype = (DType)dtypes[i]; m[i].row_pitch = 0; }
     return nt::b200::gemm_blocks(m, n_mat, in_features, x, norm_w, eps, nullptr, fine != 0, tokens, add != 0, static_cast<cudaStream_t>(stream)) ? 0 : -2;
 }
+int nt_b200_gemm_dense_tc(int n_mat, float* const* C, const void* const* W, const int* out_features, int dtype, int in_features, const float* x, const float* norm_w, float eps, int tokens,
+                       int fine, int add, const float* col_scale, float alpha, void* stream) {
+    if (n_mat < 1 || n_mat > 3 || !x) return -1;
+    nt::b200::GemvMat m[3];
+    for (int i = 0; i < n_mat; i++) { m[i].W = W[i]; m[i].y = C[i]; m[i].out = out_features[i]; m[i].dtype = (DType)dtype; m[i].row_pitch = 0; }
+    return nt::b200::gemm_dense_tc(m, n_mat, in_features, x, norm_w, eps, fine != 0, tokens, add != 0, static_cast<cudaStream_t>(stream), col_scale, alpha) ? 0 : -2;
+}
 size_t nt_b200_attention_decode_scratch_floats(int ms, int nh, int nkv, int hd) { return nt::b200::attention_decode_dyn_scratch_floats(ms, nh, nkv, hd); }
 int nt_b200_attention_decode_tickets(int nh, int nkv) { return nt::b200::attention_decode_fused_tickets(nh, nkv); }
 void nt_b200_attention_decode_fused(float* o, const float* q, const float* k, const float* v, void* kc, void* vc, const int* pos_dev, int ms,

@@ -23,6 +23,7 @@
 #include "tc_device.cuh"
 #include "wait_status.cuh"
 #include "gemv_mma_device.cuh"
+#include "tile_deal.cuh"
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <algorithm>
@@ -34,22 +35,16 @@ namespace {
 constexpr int QBK = 64;                                  // columns of a k-block: a 128-byte swizzle row of F16
 constexpr int NT_MAX = 128, FEW_TOKENS = 32;             // tokens of a tile; of a launch of the form for a few
 constexpr int STAGES_MAX = 4, D_BUFS_MAX = 4, RAW_MAX = 8, SCALE_RING = 8;
-constexpr int EPI_WARP = 4, EXP_WARP = 12, Q_THREADS = 20 * 32;      // warp 0 tokens, 1 MMA, 2 blocks (2, 3: off 16 bytes), 4-11 epilogue, 12-19 expansion
+constexpr int EXP_WARP = 12, Q_THREADS = 20 * 32;      // warp 0 tokens, 1 MMA, 2 blocks (2, 3: off 16 bytes), 4-11 epilogue, 12-19 expansion
 
 // Bytes between rows of a super-block in shared memory: an odd number of 16-byte units.  Q6_K lies at any even address: the units around it.
 __host__ __device__ constexpr int raw_pitch(int fmt) { return fmt == 2 ? 240 : fmt_bytes(fmt); }
 __host__ __device__ constexpr bool has_mins(int fmt) { return fmt <= 1; }      // otherwise A is a pair of halves
 
-struct BlkMat { const uint8_t* W; float* C; int rows, tiles, fmt; long long pitch; };
 struct alignas(64) BlkMaps { CUtensorMap x, sums, w[3]; };      // tokens, their sums, matrices as 32-bit words
-struct BlkParams {
-    BlkMat mat[3];
-    int n_mat, T, NT, cols, Mp, NB, kc, add, stages, b_stage, raw_depth, raw_slot, a_cols, d_bufs;
+struct BlkParams : Deal {
+    int Mp, kc, stages, b_stage, raw_depth, raw_slot, a_cols, d_bufs;
     int tma;                   // a matrix's rows come by TMA (bits)
-    int units;                 // tiles * super-blocks
-    const float* scale;        // of a token's products
-    float* part;               // two tiles to a CTA
-    unsigned* count;           // one to a CTA: shares of its last tile that have arrived; zeros at first
     unsigned* status;          // wait_status.cuh
 };
 
@@ -61,13 +56,9 @@ __device__ __forceinline__ uint64_t make_desc32(const void* smem_ptr) {
     const uint64_t addr = (uint64_t)(smem_u32(smem_ptr) & 0x3FFFFu) >> 4;
     return addr | (1ull << 16) | ((uint64_t)(256 >> 4) << 32) | (1ull << 46) | (6ull << 61);
 }
-__device__ __forceinline__ uint64_t pack2(float a, float b) { uint64_t d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
-__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-
 // Q6_K rows that do not lie 16 bytes apart, which TMA does not take: 64 rows of super-block b into a slot by units, four lanes to a row.  Rows behind the matrix are
 // its last one, and nothing behind the matrix's end is read.
-__device__ __forceinline__ void copy_rows(uint32_t slot, const BlkMat& m, int row, int b, int NB, int lane) {
+__device__ __forceinline__ void copy_rows(uint32_t slot, const DealMat& m, int row, int b, int NB, int lane) {
     constexpr int PITCH = raw_pitch(2), UNITS = 14;
     const uint8_t* end = m.W + (long long)(m.rows - 1) * m.pitch + (long long)NB * fmt_bytes(2);
 #pragma unroll 2
@@ -194,19 +185,6 @@ __device__ __forceinline__ float block_power(const uint8_t* blk, float& inverse)
     return __uint_as_float((uint32_t)(127 - e) << 23);
 }
 
-// Where a CTA's run of units (tile * NB + super-block) stands; tokens inside, so that the CTAs of a wave share rows
-struct Place { int tile, b, mi, row0, t0; };
-__device__ __forceinline__ int first_unit(const BlkParams& p, int cta) { return (int)((long long)p.units * cta / (int)gridDim.x); }
-__device__ __forceinline__ void place(const BlkParams& p, Place& q) {
-    const int rt = q.tile / p.cols;
-    q.t0 = (q.tile - rt * p.cols) * p.NT;
-    int r = rt, mi = 0;
-    if (p.n_mat > 1 && r >= p.mat[0].tiles) { r -= p.mat[0].tiles; mi = 1; }
-    if (p.n_mat > 2 && mi == 1 && r >= p.mat[1].tiles) { r -= p.mat[1].tiles; mi = 2; }
-    q.mi = mi; q.row0 = r * 128;
-}
-__device__ __forceinline__ Place start(const BlkParams& p, int u0) { Place q; q.tile = u0 / p.NB; q.b = u0 - q.tile * p.NB; place(p, q); return q; }
-__device__ __forceinline__ void next(const BlkParams& p, Place& q) { if (++q.b == p.NB) { q.b = 0; q.tile++; place(p, q); } }
 template <int MASK> __device__ __forceinline__ int format(int fmt) { return MASK == 1 ? 0 : MASK == 2 ? 1 : MASK == 4 ? 2 : MASK == 8 ? 3 : MASK == 16 ? 4 : fmt; }
 template <int MASK> __device__ __forceinline__ bool mins_of(const BlkParams& p, int mi) { return (MASK & (MASK - 1)) == 0 ? (MASK & 3) != 0 : (MASK & 3) != 0 && has_mins(p.mat[mi].fmt); }
 
@@ -216,7 +194,7 @@ __device__ __forceinline__ void load_blocks(const BlkMaps& maps, const BlkParams
     uint32_t st = 0, par = 1, filled = 0;
     Place q = start(p, u0);
     for (int u = u0; u < u1; u++, next(p, q)) {
-        const BlkMat& m = p.mat[q.mi];
+        const DealMat& m = p.mat[q.mi];
         const int fmt = format<MASK>(m.fmt);
         wait_cta(raw_empty + st, par, dead);
         if (word_set(dead)) {
@@ -243,7 +221,7 @@ __device__ __forceinline__ void load_blocks(const BlkMaps& maps, const BlkParams
 
 // The super-block that this lane's row has in a slot, the power of two that its codes are taken up by, and (first) what its sums are multiplied by
 template <int MASK>
-__device__ __forceinline__ const uint8_t* find_block(const BlkMat& m, const Place& q, int fmt, const uint8_t* slot, int r, float& up, float2& scale) {
+__device__ __forceinline__ const uint8_t* find_block(const DealMat& m, const Place& q, int fmt, const uint8_t* slot, int r, float& up, float2& scale) {
     const uint8_t* blk = slot + r * raw_pitch(fmt);
     if ((MASK & 4) && fmt == 2) blk += ((uint32_t)min(q.row0 + r, m.rows - 1) * (uint32_t)m.pitch + (uint32_t)q.b * 210u) & 15u;      // (W on 16 bytes)
     float down = 1.f;
@@ -263,85 +241,6 @@ __device__ __forceinline__ void expand_mins(const uint4& h, uint32_t (&w)[4]) {
         const uint32_t mm = kq_mins(h, i != 0);
         w[2 * i] = bits(__hsub2(half_pair<0, 1>(mm), k));
         w[2 * i + 1] = bits(__hsub2(half_pair<2, 3>(mm), k));
-    }
-}
-
-// The epilogue's end of a tile: this CTA's sums of units [seg0, end), 16 tokens of every STEP from `from` on.  A tile that other CTAs have a share of goes to the scratch, and
-// whoever comes last adds the shares in their order.  named barrier 5: the epilogue's threads, two warps to a row where STEP is 32.
-template <int N, int STEP>
-__device__ __forceinline__ void finish_tile(const BlkParams& p, const Place& q, uint64_t (&acc)[N][8], int u0, int seg0, int end, int from, int r, const float* token_scale, uint32_t* last_smem, uint32_t dead) {
-    const int NT = p.NT, live = min(NT, p.T - q.t0), rows = p.mat[q.mi].rows, row = q.row0 + r;
-    bool write = true;
-    if (end - seg0 < p.NB) {                                       // shared: to the scratch; whoever comes last adds
-        write = false;
-        const int tu = q.tile * p.NB, G = gridDim.x;
-        const int c0 = (int)(((long long)(tu + 1) * G - 1) / p.units), c1 = (int)(((long long)(tu + p.NB) * G - 1) / p.units);
-        float* mine = p.part + (size_t)(2 * blockIdx.x + (seg0 == u0 ? 0 : 1)) * 128 * NT + r;
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-            const int n = STEP * i + from;
-            if (n >= live) break;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                float x, y;
-                unpack2(acc[i][j], x, y);
-                __stcg(mine + (n + 2 * j) * 128, x);
-                __stcg(mine + (n + 2 * j + 1) * 128, y);
-            }
-        }
-        __threadfence();
-        named_sync<8 * STEP>(5);
-        if (threadIdx.x == EPI_WARP * 32) {
-            const bool alive = !word_set(dead);
-            const bool is_last = alive && atomicAdd(p.count + c0, 1u) == (unsigned)(c1 - c0);
-            if (is_last) p.count[c0] = 0;
-            __threadfence();
-            *last_smem = is_last;
-        }
-        named_sync<8 * STEP>(5);
-        if (*last_smem) {
-            write = true;
-#pragma unroll
-            for (int i = 0; i < N; i++)
-#pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = 0;
-#pragma unroll 1
-            for (int c = c0; c <= c1; c++) {
-                const float* o = p.part + (size_t)(2 * c + (first_unit(p, c) >= tu ? 0 : 1)) * 128 * NT + r;
-#pragma unroll
-                for (int i = 0; i < N; i++) {
-                    const int n = STEP * i + from;
-                    if (n >= live) break;
-                    float v[16];
-#pragma unroll
-                    for (int j = 0; j < 16; j++) v[j] = __ldcg(o + (n + j) * 128);
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        float x, y;
-                        unpack2(acc[i][j], x, y);
-                        acc[i][j] = pack2(x + v[2 * j], y + v[2 * j + 1]);
-                    }
-                }
-            }
-        }
-    }
-    if (write && row < rows && !word_set(dead)) {                  // a warp stores 128 contiguous bytes for each token
-        float* o = p.mat[q.mi].C + (size_t)(q.t0 + from) * rows + row;
-        const float* ts = token_scale + q.t0 + from;
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                if (STEP * i + from + j >= live) break;
-                float x, y;
-                unpack2(acc[i][j >> 1], x, y);
-                const float v = ((j & 1) ? y : x) * __ldg(ts + STEP * i + j);
-                // adds go to the memory's side (this lane is the element's only writer): nothing is waited for
-                if (p.add) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + (size_t)j * rows), "f"(v) : "memory");
-                else o[(size_t)j * rows] = v;
-            }
-            o += (size_t)STEP * rows;
-        }
     }
 }
 
@@ -523,7 +422,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         uint32_t st = odd, par = 1, rpar = 0;
         Place q = start(p, u0);
         for (int u = u0; u < u1; u++, next(p, q)) {
-            const BlkMat& m = p.mat[q.mi];
+            const DealMat& m = p.mat[q.mi];
             const int fmt = format<MASK>(m.fmt);
             wait_cta(raw_full + slot, rpar, dead);
             float up;
@@ -760,7 +659,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __g
         uint32_t st = 0, par = 1, rpar = 0;
         Place q = start(p, u0);
         for (int u = u0; u < u1; u++, next(p, q)) {
-            const BlkMat& m = p.mat[q.mi];
+            const DealMat& m = p.mat[q.mi];
             const int fmt = format<MASK>(m.fmt);
             wait_cta(raw_full + slot, rpar, dead);
             float up;
@@ -827,9 +726,9 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __g
 // a plain split, which may be the one written to) as F16 hi + lo, the sums of 32 of them
 // (a 32nd part, so that they stay within F16) as hi + lo, FINE: the halves that those two leave of both, and the factor that undoes the token's power of two.  That power takes the largest to 2^13 .. 2^14, where the
 // low halves keep their bits.  Block 0 also clears the product's counts: a launch whose wait ran out leaves some behind.
-// TOK_NORM_ANY: TOK_NORM whose gains do not lie on 16 bytes.
+// TOK_NORM_ANY: TOK_NORM whose gains do not lie on 16 bytes.  BF16: parts in BF16, no power, no sums.
 enum : int { TOK_PLAIN = 0, TOK_NORM = 1, TOK_SILU = 2, TOK_SPLIT = 3, TOK_NORM_ANY = 4 };
-template <int MODE, bool FINE>
+template <int MODE, bool FINE, bool BF16>
 __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* lo, __half* third, __half* __restrict__ sums, __half* __restrict__ third_sums, float* __restrict__ scale, unsigned* __restrict__ count, int counts,
                                                            const float* xin, const float* w, float eps, int K) {
     constexpr int KEEP = 7;                                        // chunks of 2048 held in registers: rows to 14336
@@ -875,26 +774,29 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
     for (int i = 0; i < 16; i++) { tot += red[0][i]; amax = fmaxf(amax, red[1][i]); }
     if (MODE == TOK_NORM || MODE == TOK_NORM_ANY) f = rsqrtf(tot / K + eps);
     const uint32_t e = __float_as_uint(amax * f) >> 23 & 255u;     // not finite, or zero: as it is
-    const uint32_t up = e == 255u || e == 0u ? 127u : min(227u, max(27u, 267u - e));
+    const uint32_t up = BF16 || e == 255u || e == 0u ? 127u : min(227u, max(27u, 267u - e));
     f *= __uint_as_float(up << 23);
     if (tid == 0) scale[blockIdx.x] = __uint_as_float((254u - up) << 23);
     __half* h = hi + (size_t)blockIdx.x * K;
     __half* l = lo + (size_t)blockIdx.x * K;
     const size_t sm = (size_t)blockIdx.x * (K / 16);
     auto rest = [](float v, uint32_t h, uint32_t l, bool upper) {  // what two halves leave of v: exact
+        if (BF16) return upper ? v - __uint_as_float(h & 0xFFFF0000u) - __uint_as_float(l & 0xFFFF0000u) : v - __uint_as_float(h << 16) - __uint_as_float(l << 16);
         const float2 fh = __half22float2(h2(h)), fl = __half22float2(h2(l));
         return upper ? v - fh.y - fl.y : v - fh.x - fl.x;
     };
+    [[maybe_unused]] auto pair = [](float a, float b) { uint32_t h, l; split_pair(a, b, BF16, h, l); return h; };
     auto put = [&](int i, float4 a) {
         a.x *= f; a.y *= f; a.z *= f; a.w *= f;
         uint2 ph, pl;
-        split_pair(a.x, a.y, 0, ph.x, pl.x);
-        split_pair(a.z, a.w, 0, ph.y, pl.y);
+        split_pair(a.x, a.y, BF16, ph.x, pl.x);
+        split_pair(a.z, a.w, BF16, ph.y, pl.y);
         *reinterpret_cast<uint2*>(h + i) = ph;
         *reinterpret_cast<uint2*>(l + i) = pl;
         if (FINE)
             *reinterpret_cast<uint2*>(third + (size_t)blockIdx.x * K + i) =
-                make_uint2(bits(__floats2half2_rn(rest(a.x, ph.x, pl.x, false), rest(a.y, ph.x, pl.x, true))), bits(__floats2half2_rn(rest(a.z, ph.y, pl.y, false), rest(a.w, ph.y, pl.y, true))));
+                make_uint2(pair(rest(a.x, ph.x, pl.x, false), rest(a.y, ph.x, pl.x, true)), pair(rest(a.z, ph.y, pl.y, false), rest(a.w, ph.y, pl.y, true)));
+        if (BF16) return;                                          // (matrices in BF16 have no minima)
         float s = (a.x + a.y) + (a.z + a.w);                       // K is a multiple of 256: whole warps
         s += __shfl_xor_sync(0xFFFFFFFFu, s, 1); s += __shfl_xor_sync(0xFFFFFFFFu, s, 2); s += __shfl_xor_sync(0xFFFFFFFFu, s, 4);
         if ((tid & 7) == 0) {
@@ -975,25 +877,26 @@ BlockTokens block_tokens(void* workspace, int T, int K, bool fine) {
 
 namespace {
 template <int MODE>
-BlockTokens launch_split(void* workspace, const float* x, const float* w, float eps, int T, int K, bool fine, cudaStream_t s) {
+BlockTokens launch_split(void* workspace, const float* x, const float* w, float eps, int T, int K, bool fine, bool bf16, cudaStream_t s) {
     const BlockTokens t = block_tokens(workspace, T, K, fine);
     const size_t part = padded(T) * (size_t)K;
     __half *hi = static_cast<__half*>(t.split), *sums = static_cast<__half*>(t.sums);
-    launch_k_pdl(true, fine ? split_tokens_kernel<MODE, true> : split_tokens_kernel<MODE, false>, dim3(T), dim3(512), 0, s, hi, hi + part, hi + 2 * part, sums, sums + part / 16, t.scale, t.count, sm_count(), x, w, eps, K);
+    const auto kernel = bf16 ? (fine ? split_tokens_kernel<MODE, true, true> : split_tokens_kernel<MODE, false, true>) : fine ? split_tokens_kernel<MODE, true, false> : split_tokens_kernel<MODE, false, false>;
+    launch_k_pdl(true, kernel, dim3(T), dim3(512), 0, s, hi, hi + part, hi + 2 * part, sums, sums + part / 16, t.scale, t.count, sm_count(), x, w, eps, K);
     count_launch();
     return t;
 }
 }  // namespace
 
-BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, float eps, int T, int K, bool fine, cudaStream_t s) {
-    if (!norm_w) return launch_split<TOK_PLAIN>(workspace, x, nullptr, 0.f, T, K, fine, s);
-    return (reinterpret_cast<uintptr_t>(norm_w) & 15) ? launch_split<TOK_NORM_ANY>(workspace, x, norm_w, eps, T, K, fine, s) : launch_split<TOK_NORM>(workspace, x, norm_w, eps, T, K, fine, s);
+BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, float eps, int T, int K, bool fine, cudaStream_t s, bool bf16) {
+    if (!norm_w) return launch_split<TOK_PLAIN>(workspace, x, nullptr, 0.f, T, K, fine, bf16, s);
+    return (reinterpret_cast<uintptr_t>(norm_w) & 15) ? launch_split<TOK_NORM_ANY>(workspace, x, norm_w, eps, T, K, fine, bf16, s) : launch_split<TOK_NORM>(workspace, x, norm_w, eps, T, K, fine, bf16, s);
 }
 BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, bool fine, cudaStream_t s) {
-    return launch_split<TOK_SILU>(workspace, gate, up, 0.f, T, K, fine, s);
+    return launch_split<TOK_SILU>(workspace, gate, up, 0.f, T, K, fine, false, s);
 }
 BlockTokens resplit_tokens(void* workspace, const void* hi, const void* lo, int T, int K, cudaStream_t s) {
-    return launch_split<TOK_SPLIT>(workspace, static_cast<const float*>(hi), static_cast<const float*>(lo), 0.f, T, K, false, s);
+    return launch_split<TOK_SPLIT>(workspace, static_cast<const float*>(hi), static_cast<const float*>(lo), 0.f, T, K, false, false, s);
 }
 // A plain split as it lies, for matrices without minima: it has no sums, and powers of 2^0
 static size_t plain_tokens_bytes(int T) { return padded(T) * sizeof(float) + (size_t)sm_count() * sizeof(unsigned); }
@@ -1020,13 +923,13 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     p.status = wait_status();
     p.n_mat = n_mat; p.T = T; p.NB = K / 256; p.add = add;
     p.Mp = (int)padded(T);
-    p.scale = x.scale;
+    p.scale = x.scale; p.alpha = 1.0f;
     p.kc = x.fine ? 1 : p.NB == 1 ? 2 : 4;
     const int parts = x.fine ? 3 : 2;
     const bool few = x.fine && T <= FEW_TOKENS;
     int tiles = 0, slot = 0, mask = 0;
     for (int i = 0; i < n_mat; i++) {
-        BlkMat& m = p.mat[i];
+        DealMat& m = p.mat[i];
         m.W = static_cast<const uint8_t*>(mats[i].W); m.C = mats[i].y; m.rows = mats[i].out; m.tiles = (m.rows + 127) / 128;
         m.fmt = gemv_kq_format(mats[i].dtype);
         m.pitch = (long long)(mats[i].row_pitch ? mats[i].row_pitch : dtype_row_size(mats[i].dtype, K));
@@ -1066,7 +969,7 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
         !tc_map_f16_rows32(&maps.sums, x.sums, (parts - 1) * (uint64_t)p.Mp, (uint64_t)K / 16, (uint32_t)p.NT))
         return false;
     for (int i = 0; i < n_mat; i++) {
-        const BlkMat& m = p.mat[i];
+        const DealMat& m = p.mat[i];
         if (m.pitch & 15) continue;
         if (!tc_map_words(&maps.w[i], m.W, (uint64_t)m.rows, (uint64_t)p.NB * fmt_bytes(m.fmt), (uint64_t)m.pitch, (uint32_t)raw_pitch(m.fmt))) return false;
         p.tma |= 1 << i;

@@ -429,7 +429,7 @@ bool tc_map_words(CUtensorMap* map, const void* base, uint64_t rows, uint64_t by
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-bool tc_map_f16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) { return make_map(map, base, rows, cols, box_rows); }
+bool tc_map_f16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, bool bf16) { return make_map(map, base, rows, cols, box_rows, bf16); }
 bool tc_map_f16_rows32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) { return make_map(map, base, rows, cols, box_rows, false, true); }
 
 size_t gemm_f16_tc_workspace_bytes(int M, int K) {

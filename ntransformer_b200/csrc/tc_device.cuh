@@ -8,7 +8,7 @@
 namespace nt { namespace b200 {
 
 // prefill_gemm.cu: 2-D F16 tensor [rows][cols] (cols contiguous), box = 64 cols x box_rows rows (<= 256), 128-byte swizzle
-bool tc_map_f16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+bool tc_map_f16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, bool bf16 = false);
 // rows of `bytes`, `pitch` (a multiple of 16) apart, as 32-bit words: box = box_bytes x 128 rows, no swizzle
 bool tc_map_words(CUtensorMap* map, const void* base, uint64_t rows, uint64_t bytes, uint64_t pitch, uint32_t box_bytes);
 // F16 with 16 cols to a box, 32-byte swizzle
@@ -65,6 +65,11 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 __device__ __forceinline__ void umma_ts_by(uint32_t lead, uint32_t d, uint32_t a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
                  ::"r"(d), "r"(a), "l"(db), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
+// the same with both operands in shared memory
+__device__ __forceinline__ void umma_ss_by(uint32_t lead, uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                 ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
 }
 __device__ __forceinline__ void umma_commit_by(uint32_t lead, uint64_t* bar) {
     asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"

@@ -174,14 +174,15 @@ __device__ __forceinline__ int staged_at(int i, int half) { return half ? ((i & 
 
 // The decode GEMV is bound by HBM: every weight is read once.  VEC (16-bit rows in whole 16-byte pieces): a warp streams a row, a lane 4 pieces at a
 // time, and fetches its next pieces (of this row or its next one) before it multiplies the current ones; the staged vector is planar.  So neither the
-// reduction at a row's end nor bank conflicts hold the loads up.  64 registers, so that four CTAs share an SM.  KW = 2 warps share a row where that
-// fills the last round (host).  Before it waits for the producer's grid a warp asks L2 for its first pieces.
+// reduction at a row's end nor bank conflicts hold the loads up.  64 registers, so that four CTAs share an SM.  KW warps share a row where that
+// fills the last round, or where rows are few (host).  Before it waits for the producer's grid a warp asks L2 for its first pieces.
 // BF16 in a graph, before -> now: 14336 + 14336 rows of 4096, gated 49.1 -> 37.7 us (6.2 TB/s), 32000 x 4096 52.4 -> 39.4 (6.7), 4096 x 4096 11.1 -> 8.3,
-// 3000 x 3000 11.1 -> 6.3; F16 4096 x 11008 24.4 -> 17.5.  More warps to a row in general (4 at 4096, 8 at 14336) was slower: 32000 x 4096 55.4.
+// 3000 x 3000 11.1 -> 6.3; F16 4096 x 11008 24.4 -> 17.5.  Where a CTA has more than sixteen rounds its rows lie side by side (128256 x 4096 F16 154.5 -> 149.5 us); with fewer
+// they are spread over all CTAs, whose last rounds then differ by a warp's.
 template <typename T, bool VEC, bool STREAMS>          // STREAMS: the epilogue may be DENSE_STREAMS (its registers are the kernel's without it)
 __global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_dense_kernel(DenseMats m, const float* __restrict__ x, int K, int ep,
                                                                       const float* __restrict__ row_scale, float alpha, int KW, int vec,
-                                                                      const float* __restrict__ norm_w, float eps, StreamsIO sio, int norm_groups) {
+                                                                      const float* __restrict__ norm_w, float eps, StreamsIO sio, int norm_groups, int early) {
     extern __shared__ __align__(16) float xs[];
     __shared__ float red[DV_WARPS];
     __shared__ float inv_g[DENSE_MAX_NORM_GROUPS];
@@ -200,8 +201,9 @@ __global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_d
         int mi; const int row = place(r, mi);
         return m.W[mi] + (size_t)row * m.pitch[mi];
     };
-    int r = blockIdx.x + team * gridDim.x;
-    pdl_launch_dependents();
+    const int teams = DV_WARPS / KW;
+    int r = total > 16 * step ? blockIdx.x * teams + team : blockIdx.x + team * (int)gridDim.x;
+    if (early) pdl_launch_dependents();
     if constexpr (VEC) {
         // lanes 0..15: the lines of the first chunk; lanes 16..31: those of the one after it
         int r1 = r, sub1 = 0, c1 = 0;
@@ -210,6 +212,7 @@ __global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_d
         if (r1 < total && v < nv) asm volatile("prefetch.global.L2 [%0];" ::"l"(row_ptr(r1, sub1) + (size_t)v * 16));
     }
     pdl_wait();
+    x = behind_wait(x);
     float ss = 0.f;
     if (VEC && !sio.X_in && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
 #pragma unroll 4
@@ -330,6 +333,7 @@ __global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_d
             walk(b, a);
         }
     }
+    if (!early) pdl_launch_dependents();
 }
 
 // batch of up to 128 pieces from v0 on, four 16-byte loads in flight per lane
@@ -561,7 +565,7 @@ __global__ void to_f32_kernel(float* __restrict__ out, const T* __restrict__ in,
 bool dense_dtype(DType dt) { return dt == DType::F32 || dt == DType::F16 || dt == DType::BF16; }
 
 void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpilogue ep, const float* row_scale, float alpha, cudaStream_t s,
-                const float* norm_w, float eps, const StreamsIO* sio_p, int norm_groups) {
+                const float* norm_w, float eps, const StreamsIO* sio_p, int norm_groups, bool boundary) {
     NT_CHECK(norm_groups >= 1 && norm_groups <= DENSE_MAX_NORM_GROUPS && K % norm_groups == 0, "gemv_dense: norm groups must be equal parts, at most 256");
     NT_CHECK(n_mat >= 1 && n_mat <= DENSE_MAX_MATS, "gemv_dense: too many matrices for one launch");
     const StreamsIO sio = sio_p ? *sio_p : StreamsIO();
@@ -586,16 +590,29 @@ void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpil
     if (total <= 0) return;
     const size_t smem = (size_t)K * sizeof(float);
     NT_CHECK(smem <= 200 * 1024, "gemv_dense: the activation vector does not fit in shared memory");
-    // 16-bit rows in whole pieces walk with their next pieces under way; F32 rows keep the plain walk, four loads to a lane and trip (1024 x 4096: 6.7 us,
-    // 7.4 in the other form).  Two warps share a row where one to a row would leave a second round nearly empty (4096 x
-    // 14336: 23.4 us, 27.0 with one; 6144 rows of 4096: 10.9 and 11.3).
+    // 16-bit rows in whole pieces walk with their next pieces under way; F32 rows keep the plain walk, four loads to a lane and trip (1024 x 4096: 6.7 us, 7.4 in the other form)
     const bool walk = vec && dt != DType::F32;
     const int per_sm = !walk ? 8 : ep == DENSE_STREAMS ? 2 : 4;
     const int resident = (int)std::max<size_t>(1, std::min<size_t>((size_t)per_sm, (size_t)(220 * 1024) / (smem + (walk ? 3 : 1) * 1024))) * 148;
-    const int kw = walk && total > resident * DV_WARPS && total <= resident * DV_WARPS * 3 / 2 ? 2 : 1, rows_at_once = DV_WARPS / kw;
+    // Warps to a row: what the CTA that ends last takes, its rounds of rows times their pieces of 1024 columns to a warp and 0.4 of one for a row's end; a
+    // single piece takes as long as two, of which one is under way while the other is multiplied (fits 16 shapes from 2048 x 8192 to
+    // 28672 x 4096 with 1, 2, 4 and 8 warps).  F16, us: 4096 x 14336 29.0, 25.3, 24.7, 24.7; 11008 x 4096 18.3, 16.7, 18.6, 28.9; 128256 x 4096 150 with one; 2048 x 8192 9.4, 8.4, 8.5, 8.8.
+    // (With two rows to a warp throughout, F16's form before: 270 x 11776 14.9, now 5.9; 1024 x 4096 7.1, 3.9; 4096 x 4096 9.2, 7.4; 8192 x 28672 142, 128.)
+    int kw = 1;
+    double least = 0;
+    for (int k = 1; walk && k <= DV_WARPS && (k == 1 || k * 64 * per16 < K); k *= 2) {
+        const double cost = (double)(((long long)total * k + resident * DV_WARPS - 1) / (resident * DV_WARPS)) * (std::max(2, (glu ? 2 : 1) * ((K + 128 * per16 * k - 1) / (128 * per16 * k))) + 0.4);
+        if (k == 1 || cost < least) { least = cost; kw = k; }
+    }
+    const int rows_at_once = DV_WARPS / kw;
+    // Behind the launcher boundary several CTAs fit on an SM: where a launch lets the next one start before it has done its part, that one's CTAs gather on the SMs that have room, and
+    // where it does so at its end some still do, which is more than the gap between launches but for small matrices (in F16's form before: 4096 x 14336, call after call, 38 us and
+    // 26.9 against 23.6 launched plainly; 4096 x 4096 6.1, 8.35).  In a step the next launch is another kernel.
+    const bool programmatic = pdl_enabled() || (boundary && (size_t)total * m.pitch[0] <= (size_t)64 << 20);
     const int grid = std::min((total + rows_at_once - 1) / rows_at_once, resident);
 #define NT_DVV(TY, VEC, ST) { static unsigned long long done = 0; if (smem > 40 * 1024) opt_in_dynamic_smem(gemv_dense_kernel<TY, VEC, ST>, 200 * 1024, done); \
-                              launch_k(gemv_dense_kernel<TY, VEC, ST>, dim3(grid), dim3(DV_WARPS * 32), smem, s, m, x, K, (int)ep, row_scale, alpha, kw, vec, norm_w, eps, sio, norm_groups); }
+                              launch_k_pdl(programmatic, gemv_dense_kernel<TY, VEC, ST>, dim3(grid), dim3(DV_WARPS * 32), smem, s, m, x, K, (int)ep, row_scale, alpha, kw, vec, norm_w, eps, sio, norm_groups, \
+                                           pdl_enabled() ? 1 : 0); }
 #define NT_DV(TY) { if (!walk) NT_DVV(TY, false, true) else if (ep == DENSE_STREAMS) NT_DVV(TY, true, true) else NT_DVV(TY, true, false) }
     if (dt == DType::F32) NT_DVV(float, false, true) else if (dt == DType::F16) NT_DV(__half) else NT_DV(__nv_bfloat16)
 #undef NT_DV

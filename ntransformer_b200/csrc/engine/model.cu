@@ -507,6 +507,12 @@ void Model::matvec(const Weight* const* ws, float* const* ys, int n, const float
         gemv_kq(mats, n, K, in, ep, s);
         return;
     }
+    bool f16 = ep != GEMV_PEER && (size_t)K * sizeof(float) <= 200 * 1024 && K % 8 == 0 && (ep != GEMV_SWIGLU || ws[0]->rows == ws[1]->rows);      // norm and epilogue in one launch
+    for (int i = 0; i < n; i++) f16 = f16 && mats[i].dtype == DType::F16 && (reinterpret_cast<uintptr_t>(mats[i].W) & 15) == 0 && mats[i].row_pitch % 16 == 0;
+    if (f16) {
+        gemv_dense(mats, n, K, x, ep == GEMV_ADD ? DENSE_ADD : ep == GEMV_SWIGLU ? DENSE_SWIGLU : DENSE_STORE, nullptr, 1.f, s, norm_w, cfg_.norm_eps);
+        return;
+    }
     const float* xf = x;
     if (norm_w) { rmsnorm(xnorm_, x, norm_w, 1, K, cfg_.norm_eps, s); xf = xnorm_; }
     if (ep == GEMV_SWIGLU) {                   // unfused fallback: gate -> ys[0], up -> ys[1], then silu_mul in place

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(GW * 32) gemv_generic_kernel(float* __restrict
     }
 }
 
-// ---- F16 weights, 16-byte aligned rows (reference K6, gemm.cu:546-610): x staged once per CTA in shared memory, a warp
+// ---- Short F16 rows, 16-byte aligned (reference K6, gemm.cu:546-610): x staged once per CTA in shared memory, a warp
 // streams two rows at a time with four 16-byte loads per row in flight per lane (ld.global.nc, no L1 allocation). ----
 constexpr int F16_WARPS = 8;
 __device__ __forceinline__ uint4 ldg_stream16(const uint4* p) {
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(F16_WARPS * 32) gemv_f16_kernel(float* __restr
     }
     pdl_launch_dependents();
 }
-constexpr int F16_MAX_SMEM = 200 * 1024;
+constexpr int F16_SHORT = 2048;          // columns
 
 }  // namespace
 
@@ -260,16 +260,21 @@ void gemv_generic(float* y, const void* W, const float* x, int out, int in, DTyp
     size_t pitch = row_pitch ? row_pitch : dtype_row_size(dt, (size_t)in);
     const uint8_t* w = static_cast<const uint8_t*>(W);
     if (dt == DType::F16 && in % 8 == 0 && pitch % 16 == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
-        (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (size_t)in * 4 <= (size_t)F16_MAX_SMEM && ep != GEMV_SWIGLU) {
-        static unsigned long long configured = 0;      // bit per device id
-        opt_in_dynamic_smem(gemv_f16_kernel, (int)(F16_MAX_SMEM), configured);
+        (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (size_t)in * 4 <= (size_t)200 * 1024 && ep != GEMV_SWIGLU) {
+        if (in > F16_SHORT) {
+            GemvMat m;
+            m.W = W; m.y = y; m.out = out; m.dtype = dt; m.row_pitch = pitch;
+            gemv_dense(&m, 1, in, x, ep == GEMV_ADD ? DENSE_ADD : DENSE_STORE, nullptr, 1.0f, s, nullptr, 0.f, nullptr, 1, true);
+            return;
+        }
+        // Rows of one or two pieces of gemv_dense's: twice its CTAs to an SM, and two rows to a warp, keep more loads under way (us here, there: 100000 x 1024 34.3, 37.4; 128256 x 2048
+        // 79.7, 83.6; 2000 x 2048 3.43, 3.55; rows of 3072: 900 of them 3.46, 3.57, 20000 23.9, 22.8)
         const int pairs = (out + 1) / 2;
         int grid16 = (pairs + F16_WARPS - 1) / F16_WARPS;
         const int resident = (int)std::min<size_t>(8, (size_t)(220 * 1024) / ((size_t)in * 4 + 1024)) * 148;   // CTAs the chip holds
         if (grid16 > resident && resident > 0) grid16 = resident;
-        // Several CTAs fit on an SM: where this launch lets the next one start before it has done its part, that one's CTAs gather on the SMs that have room (4096 x 14336, call after
-        // call: 38 us, 23.6 launched plainly), where it does so at its end some still do (26.9, 23.7; 14336 x 4096 21.2, 20.4), which is more than the gap between launches
-        // but for small matrices (4096 x 4096 6.1, 8.35).  In a step the next launch is another kernel.
+        // Several CTAs fit on an SM: where this launch lets the next one start before it has done its part, that one's CTAs gather on the SMs that have room, and
+        // where it does so at its end some still do, which is more than the gap between launches but for small matrices.  In a step the next launch is another kernel.
         const bool small = (size_t)out * pitch <= (size_t)64 << 20;
         launch_k_pdl(small || pdl_enabled(), gemv_f16_kernel, dim3(grid16), dim3(F16_WARPS * 32), (size_t)in * 4, s, y, w, x, out, in, pitch, (int)ep, pdl_enabled() ? 1 : 0);
         count_launch();

@@ -209,7 +209,8 @@ bool dense_dtype(DType dt);
 // Up to DENSE_MAX_MATS matrices of one dense dtype sharing the activation vector x[K] (GemvMat::y: each matrix's output rows).
 // norm_w: the kernel's prologue first replaces x by x / sqrt(mean(x^2) + eps) * norm_w (the block's RMS norm, recomputed per CTA).
 void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpilogue ep, const float* row_scale, float alpha, cudaStream_t s,
-                const float* norm_w = nullptr, float eps = 0.f, const StreamsIO* sio = nullptr, int norm_groups = 1);
+                const float* norm_w = nullptr, float eps = 0.f, const StreamsIO* sio = nullptr, int norm_groups = 1,
+                bool boundary = false /* a call of its own behind the launcher boundary */);
 constexpr int DENSE_MAX_NORM_GROUPS = 256;
 // Several matrices with an input vector each, one launch; act is applied to a matrix's own rows.  One 16-bit dtype per launch, F32 matrices
 // (router tables) may stand beside it.

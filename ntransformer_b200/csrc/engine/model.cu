@@ -868,7 +868,7 @@ bool Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
             NT_CHECK(gemm_dense_tc(m, n, K, t, block_scratch_->p, T, ep == GEMV_ADD, s), "GEMM of a few tokens over F16 rejected");
             return ep == GEMV_SWIGLU;
         }
-        if (!gemm_blocks_for_few(m, n, T)) {
+        if (!gemm_blocks_for_few(m, n, K, T)) {
             if (up) silu_mul(const_cast<float*>(x), x, up, T * K, s);
             quantize_rows(sb_.ws, x, norm, cfg_.norm_eps, T, K, s);
             gemv_rows(m, n, K, sb_.ws, T, ep, s);

@@ -587,10 +587,11 @@ BlockTokens resplit_tokens(void* workspace, const void* hi, const void* lo, int 
 // whatever wrote the matrices is done.  No other launch comes between the two.
 size_t block_scratch_bytes(int T);
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, void* scratch, int T, bool add, cudaStream_t s);
-// Whether a few tokens are better served here (fine) than by gemv_rows: from two of its passes on (two layers of an 8B model in Q4_K_M and a head of 32000: 8 tokens
-// 342 us there, about 380 here; 9 tokens 497, 384; 31 tokens 778, 427), and not in Q8_0 and Q4_0, whose weights are pairs of halves here.  Error against 64 bits of a
-// result, K-quants: 1.0e-7 to 1.8e-7 here, 1.3e-7 to 2.6e-7 there
-bool gemm_blocks_for_few(const GemvMat* mats, int n_mat, int tokens);
+// Whether a few tokens are better served here (fine) than by gemv_rows: from two of its passes of 8 on (us there, here; 8, 9, 25 tokens: Q4_K 28672 x 4096 43, 72, 128; 40, 40, 43; 4096 x
+// 14336 29, 45, 76; 30, 30, 31; Q8_0 4096 x 14336 37, 60, 104; 40, 40, 41; Q4_0 28672 x 4096 41, 70, 126; 56, 56, 60), and small matrices in Q8_0 and Q4_0, whose weights are pairs of
+// halves here, from three (2048 x 2048: 12, 13, 15; 14, 14, 15).  Error against 64 bits of a result: K-quants 1.0e-7 to 1.8e-7 here, 1.3e-7 to 2.6e-7 there; Q8_0 and Q4_0 1.2e-7 to
+// 1.6e-7, 1.2e-7 to 2.2e-7
+bool gemm_blocks_for_few(const GemvMat* mats, int n_mat, int K, int tokens);
 // over F32 tokens, or (x null) over split_activations' layout
 bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const float* x, const float* norm_w, float eps, const void* split, bool fine, int T, bool add, cudaStream_t s);
 // prefill_dense.cu: the same over up to three F16 or BF16 matrices (one type, dense rows on 16 bytes, K a multiple of 256): C_i (+)= alpha * col_scale[n] * X . W_i^T.  x as laid out by

@@ -4,7 +4,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 from ntransformer_b200.dtypes import DType  # noqa: E402
-from test_block_products_gpu import FORMATS, activations, matrix, rel  # noqa: E402
+from test_block_products_gpu import FORMATS, activations, matrix, rel, rows_product  # noqa: E402
 from test_block_tokens_gpu import bound, product  # noqa: E402
 
 pytestmark = [pytest.mark.gpu]
@@ -22,3 +22,16 @@ def test_products(dts, tokens, rows, cols):
     product(ys, [m[0] for m in mats], outs, dts, x, fine=True)
     for y, d, (_, W64) in zip(ys, dts, mats):
         assert rel(y[:tokens], x.double() @ W64.T) <= bound(d, 64) and (y[tokens] == 7.0).all()
+
+
+# tokens in blocks whose weights are pairs of halves: together from 9 (large matrices) and 17 tokens on, as exact as gemv_rows' 24-bit integers
+@pytest.mark.parametrize("dt", [DType.Q8_0, DType.Q4_0], ids=lambda d: d.name)
+@pytest.mark.parametrize("tokens,cols", [(9, 4096), (31, 14336)])
+def test_pairs_are_as_exact_as_integers(dt, tokens, cols):
+    W, W64 = matrix(dt, 700, cols, 3)
+    x = activations(tokens, cols, 5, wild=0.01)
+    ys = [torch.zeros(tokens, 700, device="cuda") for _ in range(2)]
+    product(ys[:1], [W], [700], [dt], x, fine=True)
+    rows_product(ys[1:], [W], [700], [dt], x)
+    ref = x.double() @ W64.T
+    assert rel(ys[0], ref) <= 1.05 * rel(ys[1], ref)

@@ -7,7 +7,7 @@
 //     and d joins when the epilogue takes a super-block's sum out of tensor memory.  The minima are a product of their own, m (8 for a super-block) times the sums
 //     of 32 activations.  Q6_K's sc * (q - 32) has up to 14 bits: a pair of halves, the second -1, 0 or 1.  Q8_0 and Q4_0 have a scale for 32 weights: d_i * q as
 //     a pair of halves, exact, under a power of two for the super-block;
-//   * eight warps expand 64 columns of 128 rows at a time, a row to a lane: blocks come into shared memory by TMA (Q6_K rows off 16 bytes by cp.async), two halves cost a PRMT and an HFMA2,
+//   * eight warps (Q6_K: twelve) expand 64 columns of 128 rows at a time, a row to a lane: blocks come into shared memory by TMA (Q6_K rows off 16 bytes by cp.async), two halves cost a PRMT and an HFMA2,
 //     and go to TENSOR MEMORY, from where tcgen05.mma takes its A operand: shared memory's bandwidth is left to B;
 //   * B is the split of the tokens x = hi + lo by TMA: two products for 16 columns (hi, lo), a third with the low half of a pair; in the fine form x = hi + lo + third,
 //     as many bits as the 24-bit integers hold and more (three products, five with a pair);
@@ -35,7 +35,13 @@ namespace {
 constexpr int QBK = 64;                                  // columns of a k-block: a 128-byte swizzle row of F16
 constexpr int NT_MAX = 128, FEW_TOKENS = 32;             // tokens of a tile; of a launch of the form for a few
 constexpr int STAGES_MAX = 4, D_BUFS_MAX = 4, RAW_MAX = 8, SCALE_RING = 8;
-constexpr int EXP_WARP = 12, Q_THREADS = 20 * 32;      // warp 0 tokens, 1 MMA, 2 blocks (2, 3: off 16 bytes), 4-11 epilogue, 12-19 expansion
+constexpr int EXP_WARP = 12;      // warp 0 tokens, 1 MMA, 2 blocks (2, 3: off 16 bytes), 4-11 epilogue, from 12 on expansion
+// Warps of expansion that share 32 rows, k-blocks in turn.  Three where the expansion is what bounds: Q6_K (500 tokens, 4096 x 14336: 178 us with two, 160), and pairs of halves over few
+// tokens (21, 28672 x 4096: Q6_K 71.5, 67.2; Q8_0 63.6, 61.0); products or waits bound the others (Q8_0, 500 tokens 299, 308; Q4_K over few 44.0, 44.3), and formats side by side have
+// no registers for it.  No more of them than stages: a warp waits for the k-block a ring before its own, and knows of the one before that only as long as its last one is no older.
+__host__ __device__ constexpr int groups(int mask) { return mask == 4 ? 3 : 2; }
+__host__ __device__ constexpr int few_groups(int mask) { return mask == 4 || mask == 8 || mask == 16 ? 3 : 2; }
+__host__ __device__ constexpr int threads(int groups) { return (EXP_WARP + 4 * groups) * 32; }
 
 // Bytes between rows of a super-block in shared memory: an odd number of 16-byte units.  Q6_K lies at any even address: the units around it.
 __host__ __device__ constexpr int raw_pitch(int fmt) { return fmt == 2 ? 240 : fmt_bytes(fmt); }
@@ -219,19 +225,22 @@ __device__ __forceinline__ void load_blocks(const BlkMaps& maps, const BlkParams
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// The super-block that this lane's row has in a slot, the power of two that its codes are taken up by, and (first) what its sums are multiplied by
+// The super-block that this lane's row has in a slot, the power of two that its codes are taken up by and its inverse; what its sums and its minima's sum are multiplied by
 template <int MASK>
-__device__ __forceinline__ const uint8_t* find_block(const DealMat& m, const Place& q, int fmt, const uint8_t* slot, int r, float& up, float2& scale) {
+__device__ __forceinline__ const uint8_t* find_block(const DealMat& m, const Place& q, int fmt, const uint8_t* slot, int r, float& up, float& down) {
     const uint8_t* blk = slot + r * raw_pitch(fmt);
     if ((MASK & 4) && fmt == 2) blk += ((uint32_t)min(q.row0 + r, m.rows - 1) * (uint32_t)m.pitch + (uint32_t)q.b * 210u) & 15u;      // (W on 16 bytes)
-    float down = 1.f;
-    up = 1.f;
+    up = down = 1.f;
     if ((MASK & 8) && fmt == 3) up = block_power<3>(blk, down);
     if ((MASK & 16) && fmt == 4) up = block_power<4>(blk, down);
-    scale = make_float2(down, 0.f);
-    if ((MASK & 3) && fmt <= 1) { const uint32_t h = *reinterpret_cast<const uint32_t*>(blk); scale = make_float2(half_bits(h & 0xFFFFu), -32.0f * half_bits(h >> 16)); }
-    if ((MASK & 4) && fmt == 2) scale.x = half_bits(*reinterpret_cast<const uint16_t*>(blk + 208));
     return blk;
+}
+template <int MASK>
+__device__ __forceinline__ float2 block_scale(const uint8_t* blk, int fmt, float down) {
+    float2 s = make_float2(down, 0.f);
+    if ((MASK & 3) && fmt <= 1) { const uint32_t h = *reinterpret_cast<const uint32_t*>(blk); s = make_float2(half_bits(h & 0xFFFFu), -32.0f * half_bits(h >> 16)); }
+    if ((MASK & 4) && fmt == 2) s.x = half_bits(*reinterpret_cast<const uint16_t*>(blk + 208));
+    return s;
 }
 // the minima of a Q4_K / Q5_K super-block as halves
 __device__ __forceinline__ void expand_mins(const uint4& h, uint32_t (&w)[4]) {
@@ -246,8 +255,9 @@ __device__ __forceinline__ void expand_mins(const uint4& h, uint32_t (&w)[4]) {
 
 // MASK: the formats that a launch's matrices have (bits).  PARTS: halves that a token's column is split into
 template <int MASK, int PARTS>
-__global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_constant__ BlkMaps maps, const __grid_constant__ BlkParams p) {
+__global__ void __launch_bounds__(threads(groups(MASK)), 1) gemm_blocks_kernel(const __grid_constant__ BlkMaps maps, const __grid_constant__ BlkParams p) {
     constexpr bool ONE = (MASK & (MASK - 1)) == 0, MINS = (MASK & 3) != 0, PAIRS = (MASK & 28) != 0;
+    constexpr int XG = groups(MASK);                            // warps of expansion that share 32 rows
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     // a stage is a k-block of the tokens (shared memory) and of W (tensor memory) under one pair of barriers
@@ -264,7 +274,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
     if (threadIdx.x == 0) {
         for (int i = 0; i < p.stages; i++) { mbar_init(full + i, 5); mbar_init(empty + i, 1); }      // the tokens' producer and four warps of the expansion
         for (int i = 0; i < p.d_bufs; i++) { mbar_init(d_full + i, 1); mbar_init(d_empty + i, 8); }
-        for (int i = 0; i < p.raw_depth; i++) { mbar_init(raw_full + i, by_tma ? 1 : 65); mbar_init(raw_empty + i, 8); }
+        for (int i = 0; i < p.raw_depth; i++) { mbar_init(raw_full + i, by_tma ? 1 : 65); mbar_init(raw_empty + i, 4 * XG); }
         for (int i = 0; i < SCALE_RING; i++) mbar_init(s_full + i, 4);
         dead_smem = 0;
         mbar_fence_init();
@@ -281,9 +291,10 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
     // tensor memory is this CTA's whole (its address is 0): sums, expanded k-blocks, minima
     const uint32_t a_base = (uint32_t)(p.d_bufs * NT), m_base = a_base + (uint32_t)(p.stages * p.a_cols);
 
-    // registers: 640 threads x 96 at launch; 56 + 2 x 120 + 2 x 88 for the five warpgroups are no more
+    // registers: 640 threads x 96 at launch; 56 + 2 x 120 + 2 x 88 for the five warpgroups are no more (six with 80: 48 + 2 x 96 + 3 x 80)
     if (warp < EPI_WARP) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if constexpr (XG == 3) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 0) {
         if (lane == 0) {                                           // ---- tokens by TMA ----
             uint32_t st = 0, par = 1, filled = 0;
@@ -371,7 +382,8 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         load_blocks<MASK>(maps, p, u0, u1, raw, raw_full, raw_empty, by_tma, dead, warp, lane);      // ---- blocks of W ----
     }
     } else if (warp < EXP_WARP) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
+        if constexpr (XG == 3) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+        else asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
         // ---- epilogue: a lane is a row of W; two warps share a quarter's rows, every other 16 tokens to each ----
         const int quarter = warp & 3, half = (warp - EPI_WARP) >> 2, r = quarter * 32 + lane;
         const uint32_t tq = ((uint32_t)(quarter * 32) << 16) + half * 16;
@@ -415,27 +427,29 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
         }
         if (word_set(dead)) report(p.status);
     } else {                                                       // ---- expansion: two warps share 32 rows; k-blocks 0, 2 or 1, 3 of a super-block to each ----
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-        const int quarter = warp & 3, odd = (warp - EXP_WARP) >> 2;
+        if constexpr (XG == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+        const int quarter = warp & 3, group = (warp - EXP_WARP) >> 2;
         const uint32_t tq = (uint32_t)(quarter * 32) << 16;
         int slot = 0, sslot = 0;
-        uint32_t st = odd, par = 1, rpar = 0;
+        uint32_t st = group, par = 1, rpar = 0;
+        auto wrap = [&] { if (st >= (uint32_t)p.stages) { st -= p.stages; par ^= 1; } };      // (stages >= XG)
+        wrap();
+        int first = group;                                         // of this warp's k-blocks in a super-block: every XG-th of the run is its
         Place q = start(p, u0);
         for (int u = u0; u < u1; u++, next(p, q)) {
             const DealMat& m = p.mat[q.mi];
             const int fmt = format<MASK>(m.fmt);
             wait_cta(raw_full + slot, rpar, dead);
-            float up;
-            float2 scale;
-            const uint8_t* blk = find_block<MASK>(m, q, fmt, raw + (size_t)slot * p.raw_slot, quarter * 32 + lane, up, scale);
-            if (!odd) {
-                scales[sslot][quarter * 32 + lane] = scale;
+            float up, down;
+            const uint8_t* blk = find_block<MASK>(m, q, fmt, raw + (size_t)slot * p.raw_slot, quarter * 32 + lane, up, down);
+            if (group == 0) {
+                scales[sslot][quarter * 32 + lane] = block_scale<MASK>(blk, fmt, down);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(s_full + sslot);
             }
             if (++sslot == SCALE_RING) sslot = 0;
 #pragma unroll 1
-            for (int c = odd; c < 4; c += 2) {
+            for (int c = XG == 2 ? group : first; c < 4; c += XG) {
                 const uint32_t a = tq + a_base + st * p.a_cols;
                 if (MINS && fmt <= 1) {
                     uint32_t v[32];
@@ -453,10 +467,11 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                     }
                 } else if (PAIRS) {
                     uint32_t v[8];
-                    if ((MASK & 4) && fmt == 2) upper_bits(blk, c, v);
+                    if (MASK == 4) upper_bits(blk, c, v);
 #pragma unroll 1
                     for (int hf = 0; hf < 2; hf++) {
                         uint32_t hi[16], lo[16];
+                        if (MASK != 4 && (MASK & 4) && fmt == 2) upper_bits(blk, c, v);      // (formats side by side have no registers to keep them)
                         if ((MASK & 4) && fmt == 2) expand_pair<2>(blk, c, hf, up, v, hi, lo);
                         if ((MASK & 8) && fmt == 3) expand_pair<3>(blk, c, hf, up, v, hi, lo);
                         if ((MASK & 16) && fmt == 4) expand_pair<4>(blk, c, hf, up, v, hi, lo);
@@ -472,9 +487,10 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full + st);
-                st += 2;
-                if (st >= (uint32_t)p.stages) { st -= p.stages; par ^= 1; }
+                st += XG;
+                wrap();
             }
+            if (XG == 3) first = first == 0 ? 2 : first - 1;
             if (lane == 0) mbar_arrive(raw_empty + slot);          // (every lane has read what it stored)
             if (++slot == p.raw_depth) { slot = 0; rpar ^= 1; }
         }
@@ -493,10 +509,11 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_kernel(const __grid_
 // 4096 x 14336 48.5, 46.2.  Sixteen warps of expansion and four of sums in place of eight and eight: 57.6 (the four are then behind, and the issuing warp is starved).
 // Tiles of more than 32 tokens leave room for one stage of it: 40 tokens 60.8, 70.8.
 template <int MASK>
-__global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __grid_constant__ BlkMaps maps, const __grid_constant__ BlkParams p) {
+__global__ void __launch_bounds__(threads(few_groups(MASK)), 1) gemm_blocks_few_kernel(const __grid_constant__ BlkMaps maps, const __grid_constant__ BlkParams p) {
     constexpr bool ONE = (MASK & (MASK - 1)) == 0, MINS = (MASK & 3) != 0, PAIRS = (MASK & 28) != 0;
     // Q8_0, Q4_0: a super-block's sums are added up by themselves first, which keeps small what small numbers are added to (14336 columns, error 1.54e-7 -> 1.39e-7, as gemv_rows')
     constexpr bool APART = MASK == 8 || MASK == 16;
+    constexpr int XG = few_groups(MASK);                            // warps of expansion that share 32 rows
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[STAGES_MAX], done[STAGES_MAX], d_empty[STAGES_MAX];
@@ -511,7 +528,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __g
     const bool by_tma = !(MASK & 4) || p.tma == (1 << p.n_mat) - 1;
     if (threadIdx.x == 0) {
         for (int i = 0; i < p.stages; i++) { mbar_init(full + i, 9); mbar_init(done + i, 1); mbar_init(d_empty + i, 8); }      // the tokens' producer and eight warps of the expansion
-        for (int i = 0; i < p.raw_depth; i++) { mbar_init(raw_full + i, by_tma ? 1 : 65); mbar_init(raw_empty + i, 8); }
+        for (int i = 0; i < p.raw_depth; i++) { mbar_init(raw_full + i, by_tma ? 1 : 65); mbar_init(raw_empty + i, 4 * XG); }
         for (int i = 0; i < SCALE_RING; i++) mbar_init(s_full + i, 4);
         dead_smem = 0;
         mbar_fence_init();
@@ -528,7 +545,8 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __g
     const uint32_t d_cols = (uint32_t)((MINS ? 3 : 2) * NT), a_base = (uint32_t)p.stages * d_cols, m_base = a_base + (uint32_t)(p.stages * 2 * p.a_cols);
 
     if (warp < EPI_WARP) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if constexpr (XG == 3) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 0) {
         if (lane == 0) {                                           // ---- tokens by TMA ----
             uint32_t st = 0, par = 1, filled = 0;
@@ -605,7 +623,8 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __g
         load_blocks<MASK>(maps, p, u0, u1, raw, raw_full, raw_empty, by_tma, dead, warp, lane);      // ---- blocks of W ----
     }
     } else if (warp < EXP_WARP) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
+        if constexpr (XG == 3) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+        else asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
         // ---- epilogue: a lane is a row of W; two warps share a quarter's rows, 16 tokens to each ----
         const int quarter = warp & 3, half = (warp - EPI_WARP) >> 2, r = quarter * 32 + lane;
         const uint32_t tq = ((uint32_t)(quarter * 32) << 16) + half * 16;
@@ -662,28 +681,28 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __g
         }
         if (word_set(dead)) report(p.status);
     } else {                                                       // ---- expansion: two warps share 32 rows; a k-block of a stage to each ----
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-        const int quarter = warp & 3, odd = (warp - EXP_WARP) >> 2;
+        if constexpr (XG == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+        const int quarter = warp & 3, group = (warp - EXP_WARP) >> 2;
         const uint32_t tq = (uint32_t)(quarter * 32) << 16;
         int slot = 0, sslot = 0;
-        uint32_t st = 0, par = 1, rpar = 0;
+        uint32_t st = group >> 1, par = 1, rpar = 0;              // (two stages and more)
+        int first = group;                                         // of this warp's k-blocks in a super-block: every XG-th of the run is its
         Place q = start(p, u0);
         for (int u = u0; u < u1; u++, next(p, q)) {
             const DealMat& m = p.mat[q.mi];
             const int fmt = format<MASK>(m.fmt);
             wait_cta(raw_full + slot, rpar, dead);
-            float up;
-            float2 scale;
-            const uint8_t* blk = find_block<MASK>(m, q, fmt, raw + (size_t)slot * p.raw_slot, quarter * 32 + lane, up, scale);
-            if (!odd) {
-                scales[sslot][quarter * 32 + lane] = scale;
+            float up, down;
+            const uint8_t* blk = find_block<MASK>(m, q, fmt, raw + (size_t)slot * p.raw_slot, quarter * 32 + lane, up, down);
+            if (group == 0) {
+                scales[sslot][quarter * 32 + lane] = block_scale<MASK>(blk, fmt, down);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(s_full + sslot);
             }
             if (++sslot == SCALE_RING) sslot = 0;
 #pragma unroll 1
-            for (int c = odd; c < 4; c += 2) {
-                const uint32_t a = tq + a_base + (2 * st + odd) * p.a_cols;
+            for (int c = XG == 2 ? group : first; c < 4; c += XG) {
+                const uint32_t a = tq + a_base + (2 * st + (c & 1)) * p.a_cols;
                 if (MINS && fmt <= 1) {
                     uint32_t v[32];
                     const uint4 h = lds128(blk);
@@ -700,10 +719,11 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __g
                     }
                 } else if (PAIRS) {
                     uint32_t v[8];
-                    if ((MASK & 4) && fmt == 2) upper_bits(blk, c, v);
+                    if (MASK == 4) upper_bits(blk, c, v);
 #pragma unroll 1
                     for (int hf = 0; hf < 2; hf++) {
                         uint32_t hi[16], lo[16];
+                        if (MASK != 4 && (MASK & 4) && fmt == 2) upper_bits(blk, c, v);      // (formats side by side have no registers to keep them)
                         if ((MASK & 4) && fmt == 2) expand_pair<2>(blk, c, hf, up, v, hi, lo);
                         if ((MASK & 8) && fmt == 3) expand_pair<3>(blk, c, hf, up, v, hi, lo);
                         if ((MASK & 16) && fmt == 4) expand_pair<4>(blk, c, hf, up, v, hi, lo);
@@ -719,8 +739,10 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_blocks_few_kernel(const __g
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full + st);
-                if (++st == (uint32_t)p.stages) { st = 0; par ^= 1; }
+                st += XG == 2 ? 1 : 1 + (c & 1);
+                if (st >= (uint32_t)p.stages) { st -= p.stages; par ^= 1; }
             }
+            if (XG == 3) first = first == 0 ? 2 : first - 1;
             if (lane == 0) mbar_arrive(raw_empty + slot);          // (every lane has read what it stored)
             if (++slot == p.raw_depth) { slot = 0; rpar ^= 1; }
         }
@@ -844,13 +866,13 @@ __global__ void __launch_bounds__(256) silu_split_kernel(uint2* __restrict__ hi,
 template <int MASK>
 void launch_blocks(const BlkMaps& maps, const BlkParams& p, int parts, bool few, int grid, size_t smem, cudaStream_t s) {
     static unsigned long long configured[3] = {};      // bit per device id
-    auto launch = [&](auto kernel, unsigned long long& done) {
+    auto launch = [&](auto kernel, int groups, unsigned long long& done) {
         opt_in_dynamic_smem(kernel, 214 * 1024, done);
-        launch_k_pdl(true, kernel, dim3(grid), dim3(Q_THREADS), smem, s, maps, p);
+        launch_k_pdl(true, kernel, dim3(grid), dim3(threads(groups)), smem, s, maps, p);
     };
-    if (few) launch(gemm_blocks_few_kernel<MASK>, configured[0]);
-    else if (parts == 3) launch(gemm_blocks_kernel<MASK, 3>, configured[1]);
-    else launch(gemm_blocks_kernel<MASK, 2>, configured[2]);
+    if (few) launch(gemm_blocks_few_kernel<MASK>, few_groups(MASK), configured[0]);
+    else if (parts == 3) launch(gemm_blocks_kernel<MASK, 3>, groups(MASK), configured[1]);
+    else launch(gemm_blocks_kernel<MASK, 2>, groups(MASK), configured[2]);
     count_launch();
 }
 
@@ -971,7 +993,7 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
             if (p.d_bufs >= (mins ? 3 : 2) && (size_t)p.stages * p.b_stage + 2 * (size_t)slot <= cap) break;
         }
         p.d_bufs = std::min(D_BUFS_MAX, (512 - p.stages * p.a_cols - (mins ? 8 : 0)) / p.NT);
-        if (p.d_bufs < 2) return false;
+        if (p.d_bufs < 2 || p.stages < groups(mask)) return false;      // (the latter: 3 with tiles of 128 tokens in three parts, otherwise 4)
     }
     p.raw_depth = (int)std::min<size_t>(RAW_MAX, (cap - (size_t)p.stages * p.b_stage) / slot);
     if (p.raw_depth < 1) return false;

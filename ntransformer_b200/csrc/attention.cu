@@ -581,6 +581,28 @@ bool attention_prefill_tc_pays(int seq_len, int start_pos, int n_heads, int hd) 
     const float s64 = (float)((keys + 63) / 64), s128 = (float)((keys + 127) / 128), doubled = log2f((float)((seq_len + 127) / 128));
     return hd == 128 ? 1.9f * s64 - 2.82f * s128 - 0.7f * doubled > 2.75f : 1.22f * s64 - 2.1f * s128 - 0.3f * doubled > 1.25f;
 }
+// How many slices the keys are cut into.  Either form walks a CTA's keys in series, and where the queries give fewer CTAs than there are SMs, the rest idle: slices, at the
+// price of writing their sums and reading them again.  Times as measured (us): the tcgen05 form 8.0 and 1.5 for 64 keys (heads of 64: 4.5 and 1.2), the whole one on
+// mma.sync 5.5 and 2.1 (4.2 and 1.3); slices with their merge 6.0 and 2.3 (1.4) for 64 keys of one, 1.7 (1.5) times that where two CTAs share an SM, and the sums at
+// 0.35 us a megabyte; a slice more costs 0.2.  Whole, in slices: heads of 128, 8 of them, 40 tokens behind 965: 31.2, 13.2; 64, 17 behind 1000: 32.1, 22.8; 2, 1500 behind
+// 1500: 78.3, 39.3; 8, 518 behind 5: 24.2, 21.4; heads of 64, 16 of them, 60 behind 700: 18.8, 10.5.  Not cut: 32 heads of 128, 256 behind 0: 14.4, 18.8 in two;
+// 64 heads, 128 behind 1000: 37.0, 42.5.  Of 110 calls with less than a wave of CTAs none is slower by more than 2 %; half take less than 0.6 of the time.
+// Between programmatic launches the plain one costs 3 to 4 us more: 60 tokens behind 900, 32 heads of 128, two layers of 4096: 443 us whole, 426 in slices.
+int attention_prefill_slices_for(int form, int seq_len, int start_pos, int n_heads, int hd, int max_seq, bool in_chain) {
+    const long long ctas = (long long)((seq_len + 63) / 64) * n_heads, tiles = ((long long)start_pos + seq_len + 63) / 64;
+    if (form == PREFILL_QUERIES || start_pos < 0 || (long long)start_pos + seq_len > max_seq || ctas > 148 || tiles < 4) return 1;
+    const bool wide = hd == 128;
+    const float whole = form == PREFILL_TC ? (wide ? 8.0f + 1.5f * tiles : 4.5f + 1.2f * tiles) : (wide ? 5.5f + 2.1f * tiles : 4.2f + 1.3f * tiles);
+    const float written = 0.35e-6f * 4 * seq_len * n_heads * hd + 0.2f;       // a slice's sums, there and back
+    int best = 1;
+    float least = whole - (in_chain ? 5.0f : 1.5f);
+    for (int n = 2; n <= 16 && n <= tiles; n++) {
+        const long long all = ctas * n, steps = (tiles + n - 1) / n * ((all + 295) / 296);
+        const float t = 6.0f + (wide ? 2.3f : 1.4f) * steps * (all <= 148 ? 1.0f : wide ? 1.7f : 1.5f) + n * written;
+        if (t < least) { least = t; best = n; }
+    }
+    return best;
+}
 // prompt-sized chunks: tiled tensor-core kernels
 int attention_prefill_form(const float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq, bool in_chain) {
     if (!attention_prefill_mma_supported(seq_len, n_heads, n_kv, hd)) return PREFILL_QUERIES;
@@ -592,6 +614,8 @@ void attention_prefill(float* out, const float* Q, const void* kc, const void* v
     if (seq_len <= 0 || n_heads <= 0) return;
     const int form = attention_prefill_form(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq, in_chain);
     if (form != PREFILL_QUERIES) {
+        const int slices = attention_prefill_slices_for(form, seq_len, start_pos, n_heads, hd, max_seq, in_chain);
+        if (slices > 1 && attention_prefill_slices(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq, scale, slices, s)) return;
         if (form == PREFILL_TC && attention_prefill_tc(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, scale, s)) return;
         attention_prefill_mma(out, Q, kc, vc, seq_len, start_pos, n_heads, n_kv, hd, max_seq, scale, s);
         return;

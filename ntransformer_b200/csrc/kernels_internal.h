@@ -155,6 +155,10 @@ bool attention_prefill_tc_takes(const float* out, const float* Q, const void* kc
 bool attention_prefill_tc(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, float scale, cudaStream_t s);
 // attention_prefill_mma.cu: 64-query x 64-key tiles on mma.sync (attention_prefill: seq_len >= 16, hd 64/128, what the form above does not take; windows; BF16 caches)
 bool attention_prefill_mma_supported(int seq_len, int n_heads, int n_kv, int hd);
+// in slices of the keys, joined by a second launch; 1: whole.  false: no memory, nothing launched
+int attention_prefill_slices_for(int form, int seq_len, int start_pos, int n_heads, int hd, int max_seq, bool in_chain);      // attention.cu
+bool attention_prefill_slices(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads, int n_kv, int hd, int max_seq, float scale,
+                              int slices, cudaStream_t s);
 void attention_prefill_mma(float* out, const float* Q, const void* kc, const void* vc, int seq_len, int start_pos, int n_heads,
                            int n_kv, int hd, int max_seq, float scale, cudaStream_t s);
 // A run of a few tokens at start_pos ..., each query with the decode step's F32 arithmetic (slices of the context, merged).

@@ -397,11 +397,24 @@ void launch_decode(float* out, const float* q, const __half* kc, const __half* v
     }
 }
 
-// Slices of a run of `tokens` queries: enough CTAs for the chip, at least 32 keys each.
-int rows_splits(int tokens, int total, int groups) {
-    int n = (2 * 148 + groups * tokens - 1) / (groups * tokens);
-    n = std::min(std::min(n, (total + 31) / 32), MAX_SPLITS);
-    return std::max(1, n);
+// Slices of a run of `tokens` queries over `total` keys, `groups` CTAs to a query and a slice: at least 32 keys each, at most three waves of CTAs, two to an SM.
+int rows_splits_most(int tokens, int total, int groups) { return std::max(1, std::min({888 / (groups * tokens), (total + 31) / 32, MAX_SPLITS})); }
+// A CTA takes 2 us and then, for a key, 10.5 ns and 2.3 ns for each query head that shares it (of 128), 1.75 times that beside another on its SM (half a wave is enough
+// for that: CTAs that wait for the launch before gather two to an SM); a wave begun costs most of one; the merge takes 3.5 us and 6 us for a million of the slices' sums.
+// As many slices as a wave of CTAs and one more, whatever they cost, was what stood here.  21 tokens, 32 heads of 128 over 8, behind 30, 120, 300, 1900 (us, before and
+// now): 10.5, 4.9; 12.6, 7.8; 17.1, 13.3; 56.5, 50.8; 3 tokens, 64 heads, behind 1900: 19.8, 14.4.  Of 225 calls (2 to 31 tokens, 16 to 64 heads, both widths, 30 to 1900
+// keys before) none is slower by more than 2 %, the mean takes 0.79 of the time.
+int rows_splits(int tokens, int total, int groups, int gc, int hd) {
+    const float key = 0.0105f + 0.0023f * gc * hd / 128;
+    int best = 1;
+    float least = 0.f;
+    for (int n = 1, most = rows_splits_most(tokens, total, groups); n <= most; n++) {
+        const int len = (total + n - 1) / n, used = (total + len - 1) / len, ctas = groups * tokens * used;
+        const float waves = ctas <= 296 ? 1.f : 0.7f * ((ctas + 295) / 296) + 0.3f * ctas / 296;
+        const float t = (2.0f + key * len * (ctas <= 74 ? 1.0f : 1.75f)) * waves + (used > 1 ? 3.5f + 6e-6f * used * tokens * groups * gc * hd : 0.f);
+        if (n == 1 || t < least) { least = t; best = used; }
+    }
+    return best;
 }
 // A few consecutive queries (start_pos ...), each with the arithmetic of a decoded token; scratch: attention_rows_scratch_floats().
 template <int DPL, int GC>
@@ -409,7 +422,7 @@ void launch_rows(float* out, const float* q, const __half* kc, const __half* vc,
                  cudaStream_t s) {
     constexpr int HD = DPL * 32;
     const int groups = n_heads / GC, total = start_pos + tokens;
-    int n_splits = rows_splits(tokens, total, groups);
+    int n_splits = rows_splits(tokens, total, groups, GC, HD);
     const int split_len = (total + n_splits - 1) / n_splits;
     n_splits = (total + split_len - 1) / split_len;
     const size_t smem = ((size_t)walk_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
@@ -515,7 +528,7 @@ void attention_decode(float* out, const float* q, const void* kc, const void* vc
 size_t attention_rows_scratch_floats(int tokens, int max_seq, int n_heads, int n_kv, int hd) {
     const int gc = pick_gc(n_heads / n_kv);
     size_t most = 0;                     // fewer tokens are cut into more slices
-    for (int t = 1; t <= tokens; t++) most = std::max(most, (size_t)t * n_heads * rows_splits(t, max_seq, n_heads / gc) * (hd + 2));
+    for (int t = 1; t <= tokens; t++) most = std::max(most, (size_t)t * n_heads * rows_splits_most(t, max_seq, n_heads / gc) * (hd + 2));
     return most;
 }
 void attention_rows_f16(float* out, const float* q, const void* kc, const void* vc, int tokens, int start_pos, int n_heads, int n_kv, int hd, float scale,

@@ -83,7 +83,7 @@ __device__ __forceinline__ void store_row_f16(__half* p, const __half (&h)[DPL])
 // One CTA: GC query heads of one KV head, keys [k_begin, k_end) (attention_walk.cuh).
 // q_base: first of the GC heads' query vectors (contiguous [GC][hd]); out likewise.
 // If part_* != nullptr writes unnormalised partials, else the normalised output.
-template <int DPL, int GC, bool NEW = false>
+template <int DPL, int GC, bool NEW = false, bool APART = true>
 __device__ void attend_group(float* __restrict__ out, const float* __restrict__ q_base, const __half* __restrict__ kc,
                              const __half* __restrict__ vc, int kv_head, int n_kv, int k_begin, int k_end, float scale,
                              float* __restrict__ part_o, float* __restrict__ part_ml, float* smem, const NewToken nt = NewToken{}) {
@@ -91,7 +91,7 @@ __device__ void attend_group(float* __restrict__ out, const float* __restrict__ 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t row_stride = (size_t)n_kv * HD, channel = (size_t)kv_head * HD + (size_t)lane * DPL;
     float rc[DPL], rs[DPL];
-    walk_slice<DPL, GC, NEW>(kc + channel, vc + channel, row_stride, k_begin, k_end, nt.pos, scale, smem, warp, lane,
+    walk_slice<DPL, GC, NEW, APART>(kc + channel, vc + channel, row_stride, k_begin, k_end, nt.pos, scale, smem, warp, lane,
         [&](float (&qr)[GC][DPL]) {
 #pragma unroll
             for (int g = 0; g < GC; g++)
@@ -133,7 +133,7 @@ __device__ void attend_group(float* __restrict__ out, const float* __restrict__ 
 }
 
 // Scratch layout for split decode: [head][split][HD] floats then [head][split][2] (max, sum).
-template <int DPL, int GC>
+template <int DPL, int GC, bool APART = true>
 __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) decode_kernel(float* __restrict__ out, const float* __restrict__ q,
                                                          const __half* __restrict__ kc, const __half* __restrict__ vc,
                                                          int seq_len, int n_heads, int n_kv, float scale, int n_splits,
@@ -159,13 +159,13 @@ __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) decode_kernel
     const int k_begin = split * split_len, k_end = min(seq_len, k_begin + split_len);
     if (k_begin >= k_end) return;
     if (n_splits == 1 && !pos_dev) {
-        attend_group<DPL, GC>(out + (size_t)head0 * HD, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale,
+        attend_group<DPL, GC, false, APART>(out + (size_t)head0 * HD, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale,
                               nullptr, nullptr, smem_dyn);
     } else {
         // partials for head (head0+g) live at scratch[((head0+g) * n_splits + split) * HD]; attend_group strides
         // heads by HD, so hand it a staging area in shared memory and scatter afterwards.
         float* stage = smem_dyn + walk_floats<DPL, GC>();   // [GC][HD] + [GC][2]
-        attend_group<DPL, GC>(nullptr, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale, stage,
+        attend_group<DPL, GC, false, APART>(nullptr, q + (size_t)head0 * HD, kc, vc, kv_head, n_kv, k_begin, k_end, scale, stage,
                               stage + GC * HD, smem_dyn);
         __syncthreads();
         float* ml = scratch + (size_t)n_heads * n_splits * HD;
@@ -362,32 +362,32 @@ __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) prefill_kerne
 
 int pick_gc(int group) { return group % 8 == 0 ? 8 : group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1; }
 
+// Slices of the keys of one query, `groups` CTAs to a slice: at least 32 keys each, and no more CTAs than are resident at once, two to an SM.  (One slice more, to leave no
+// SM with one CTA, began a second wave: 32 heads of 128 with keys of their own, 1000 and 4000 keys, ten slices and nine: 8.9, 7.1; 19.6, 14.6 us; 24 heads over 8, 4000
+// keys, 13 and 12: 15.8, 12.6.)
+int wave_splits(int keys, int groups) { return std::max(1, std::min({2 * 148 / groups, (keys + 31) / 32, MAX_SPLITS})); }
 template <int DPL, int GC>
 void launch_decode(float* out, const float* q, const __half* kc, const __half* vc, int seq_len, int n_heads, int n_kv,
                    float scale, cudaStream_t s) {
     constexpr int HD = DPL * 32;
-    // split so that head-groups x splits covers the chip, with at least 32 keys per split
     int groups = n_heads / GC;
-    int n_splits = 1;
-    if (seq_len > 64) {
-        n_splits = (2 * 148 + groups - 1) / groups;
-        int max_by_len = (seq_len + 31) / 32;
-        if (n_splits > max_by_len) n_splits = max_by_len;
-        if (n_splits > MAX_SPLITS) n_splits = MAX_SPLITS;
-        if (n_splits < 1) n_splits = 1;
-    }
+    int n_splits = seq_len > 64 ? wave_splits(seq_len, groups) : 1;
     int split_len = (seq_len + n_splits - 1) / n_splits;
     n_splits = (seq_len + split_len - 1) / split_len;
     const size_t smem = ((size_t)walk_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
     static unsigned long long configured = 0;      // bit per device id
-    opt_in_dynamic_smem(decode_kernel<DPL, GC>, (int)(ATTN_MAX_DYN_SMEM), configured);
+    // sums apart where the groups do not fill the wave, so that the slices are longer (32 groups, 2000 keys: 1.94e-7 of error, 1.81e-7 so); elsewhere they cost 1 % and nothing calls for them
+    auto kernel = 296 % groups ? decode_kernel<DPL, GC, true> : decode_kernel<DPL, GC, false>;
+    opt_in_dynamic_smem(decode_kernel<DPL, GC, false>, (int)(ATTN_MAX_DYN_SMEM), configured);
+    static unsigned long long configured_apart = 0;
+    opt_in_dynamic_smem(decode_kernel<DPL, GC, true>, (int)(ATTN_MAX_DYN_SMEM), configured_apart);
     // the slices' results: the stream's, so that calls on other streams and devices and by other threads have their own
     std::optional<StreamMemory> memory;
     if (n_splits > 1) memory.emplace((size_t)n_heads * n_splits * (HD + 2) * sizeof(float), s);
     float* scratch = memory ? static_cast<float*>(memory->p) : nullptr;
     if (!scratch) { n_splits = 1; split_len = seq_len; }          // no memory: one slice
     // Programmatic launches outside graphs too: neither kernel reads or writes before its wait, so the merge's launch hides behind the slices
-    launch_k_pdl(true, decode_kernel<DPL, GC>, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, kc, vc, seq_len, n_heads, n_kv, scale, n_splits, split_len,
+    launch_k_pdl(true, kernel, dim3(groups, n_splits), dim3(AW * 32), smem, s, out, q, kc, vc, seq_len, n_heads, n_kv, scale, n_splits, split_len,
                  scratch, (const int*)nullptr);
     count_launch();
     if (n_splits > 1) {
@@ -401,10 +401,11 @@ void launch_decode(float* out, const float* q, const __half* kc, const __half* v
 int rows_splits_most(int tokens, int total, int groups) { return std::max(1, std::min({888 / (groups * tokens), (total + 31) / 32, MAX_SPLITS})); }
 // A CTA takes 2 us and then, for a key, 10.5 ns and 2.3 ns for each query head that shares it (of 128), 1.75 times that beside another on its SM (half a wave is enough
 // for that: CTAs that wait for the launch before gather two to an SM); a wave begun costs most of one; the merge takes 3.5 us and 6 us for a million of the slices' sums.
-// As many slices as a wave of CTAs and one more, whatever they cost, was what stood here.  21 tokens, 32 heads of 128 over 8, behind 30, 120, 300, 1900 (us, before and
-// now): 10.5, 4.9; 12.6, 7.8; 17.1, 13.3; 56.5, 50.8; 3 tokens, 64 heads, behind 1900: 19.8, 14.4.  Of 225 calls (2 to 31 tokens, 16 to 64 heads, both widths, 30 to 1900
-// keys before) none is slower by more than 2 %, the mean takes 0.79 of the time.
+// Before: as many slices as a wave of CTAs and one more, whatever they cost.  21 tokens, 32 heads of 128 over 8, behind 30, 120, 300, 1900 (us, before and now): 10.5, 4.9;
+// 12.6, 7.8; 17.1, 13.3; 56.5, 50.8; 180 calls (2 to 31 tokens, 16 to 32 heads, both widths, 30 to 1900 keys before): the mean takes 0.8 of the time.  Eight heads of
+// 128 to a key head stay with that: their sums are one run (attention_walk.cuh), and longer slices would cost precision (31 queries behind 1000: 2.2e-7, 2.6e-7).
 int rows_splits(int tokens, int total, int groups, int gc, int hd) {
+    if (gc * hd > 512) return std::max(1, std::min({(2 * 148 + groups * tokens - 1) / (groups * tokens), (total + 31) / 32, MAX_SPLITS}));
     const float key = 0.0105f + 0.0023f * gc * hd / 128;
     int best = 1;
     float least = 0.f;
@@ -539,14 +540,7 @@ void attention_rows_f16(float* out, const float* q, const void* kc, const void* 
     NT_DISPATCH_ATTN(launch_rows, out, q, k, v, tokens, start_pos, n_heads, n_kv, scale, scratch, s);
 }
 
-int attention_decode_dyn_splits(int max_seq, int n_heads, int n_kv) {
-    const int groups = n_heads / pick_gc(n_heads / n_kv);
-    int n = (2 * 148 + groups - 1) / groups;
-    int by_len = (max_seq + 31) / 32;
-    if (n > by_len) n = by_len;
-    if (n > MAX_SPLITS) n = MAX_SPLITS;
-    return n < 1 ? 1 : n;
-}
+int attention_decode_dyn_splits(int max_seq, int n_heads, int n_kv) { return wave_splits(max_seq, n_heads / pick_gc(n_heads / n_kv)); }
 size_t attention_decode_dyn_scratch_floats(int max_seq, int n_heads, int n_kv, int hd) {
     return (size_t)n_heads * attention_decode_dyn_splits(max_seq, n_heads, n_kv) * (hd + 2);
 }

@@ -49,11 +49,15 @@ template <int DPL, int GC> __host__ __device__ constexpr int walk_floats() { ret
 
 // Warp `warp` of WALK_WARPS, keys [k_begin, k_end).  kbase, vbase: this lane's DPL channels of cache row 0.  load_q(qr) gives the lane's channels of the
 // queries (after the first rows are under way).  OWN: row `own` is not read from the cache, own_key(f) and own_value(f) give it.
-template <int DPL, int GC, bool OWN, class LoadQ, class OwnKey, class OwnValue>
+// APART: eight keys' sums apart, see below.
+template <int DPL, int GC, bool OWN, bool APART, class LoadQ, class OwnKey, class OwnValue>
 __device__ __forceinline__ void walk_slice(const __half* kbase, const __half* vbase, size_t row_stride, int k_begin, int k_end, int own, float scale, float* smem,
                                            int warp, int lane, LoadQ load_q, OwnKey own_key, OwnValue own_value) {
     constexpr int HD = DPL * 32, LG = 32 / GC;           // lanes that hold a head's score
     using Raw = typename HalfVec<DPL>::T;
+    // Eight keys' sums by themselves before they join the run's, whose length then costs less: 1900 keys in two slices 2.6e-7 of error in one run, 1.8e-7 so.  Not where
+    // the registers do not hold both (64 heads over 8: 4000 keys 12.3 us, 13.6 so; 27 queries behind 1900 85, 102).
+    constexpr bool BLOCKED = APART && DPL * GC <= 16;
     float* pw = smem + (size_t)warp * GC * P_LD;
     float* red = smem + (size_t)WALK_WARPS * GC * P_LD;
     float* ml = red + (size_t)WALK_WARPS * GC * HD;
@@ -106,11 +110,17 @@ __device__ __forceinline__ void walk_slice(const __half* kbase, const __half* vb
         for (int u = 0; u < KU; u++) m2 = fmaxf(m2, s[u]);
         const float corr = expf(mx - m2);                // the first batch: 0, or 1 where no score lies above -FLT_MAX (then the sums are 0)
         mx = m2;
-        sum *= corr;
+        if constexpr (BLOCKED) {
 #pragma unroll
-        for (int u = 0; u < KU; u++) {
-            s[u] = k0 + u < k_end ? expf(s[u] - m2) : 0.f;
-            sum += s[u];
+            for (int u = 0; u < KU; u++) s[u] = k0 + u < k_end ? expf(s[u] - m2) : 0.f;
+            sum = fmaf(sum, corr, ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])));
+        } else {
+            sum *= corr;
+#pragma unroll
+            for (int u = 0; u < KU; u++) {
+                s[u] = k0 + u < k_end ? expf(s[u] - m2) : 0.f;
+                sum += s[u];
+            }
         }
         __syncwarp();                                    // the weights of the batch before have been read
         if ((lane & (LG - 1)) == 0) {
@@ -119,23 +129,46 @@ __device__ __forceinline__ void walk_slice(const __half* kbase, const __half* vb
             pw[KU * GC + lane / LG] = corr;
         }
         __syncwarp();
+        if constexpr (BLOCKED) {
+            float part[2][GC][DPL] = {};
 #pragma unroll
-        for (int g = 0; g < GC; g++) {
-            const float c = pw[KU * GC + g];
+            for (int u = 0; u < KU; u++) {
+                if (k0 + u >= k_end) break;
+                float vf[DPL];
+                to_float(vr[u], vf);
+                if (OWN && k0 + u == own) own_value(vf);
 #pragma unroll
-            for (int i = 0; i < DPL; i++) acc[g][i] *= c;
-        }
+                for (int g = 0; g < GC; g++) {
+                    const float w = pw[u * GC + g];
 #pragma unroll
-        for (int u = 0; u < KU; u++) {
-            if (k0 + u >= k_end) break;
-            float vf[DPL];
-            to_float(vr[u], vf);
-            if (OWN && k0 + u == own) own_value(vf);
+                    for (int i = 0; i < DPL; i++) part[u & 1][g][i] = fmaf(w, vf[i], part[u & 1][g][i]);
+                }
+            }
 #pragma unroll
             for (int g = 0; g < GC; g++) {
-                const float w = pw[u * GC + g];
+                const float c = pw[KU * GC + g];
 #pragma unroll
-                for (int i = 0; i < DPL; i++) acc[g][i] = fmaf(w, vf[i], acc[g][i]);
+                for (int i = 0; i < DPL; i++) acc[g][i] = fmaf(acc[g][i], c, part[0][g][i] + part[1][g][i]);
+            }
+        } else {
+#pragma unroll
+            for (int g = 0; g < GC; g++) {
+                const float c = pw[KU * GC + g];
+#pragma unroll
+                for (int i = 0; i < DPL; i++) acc[g][i] *= c;
+            }
+#pragma unroll
+            for (int u = 0; u < KU; u++) {
+                if (k0 + u >= k_end) break;
+                float vf[DPL];
+                to_float(vr[u], vf);
+                if (OWN && k0 + u == own) own_value(vf);
+#pragma unroll
+                for (int g = 0; g < GC; g++) {
+                    const float w = pw[u * GC + g];
+#pragma unroll
+                    for (int i = 0; i < DPL; i++) acc[g][i] = fmaf(w, vf[i], acc[g][i]);
+                }
             }
         }
         if (k0 + WALK_WARPS * KU < k_end) fetch(vbase, vr, k0 + WALK_WARPS * KU);

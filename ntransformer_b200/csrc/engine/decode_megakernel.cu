@@ -537,7 +537,7 @@ __device__ void attend_unit(const MegaParams& P, Shared& S, const MegaPhase& d, 
     const size_t row_stride = (size_t)n_kv * HD;
     const size_t channel = (size_t)kv_head * HD + (size_t)lane * DPL;
     if (warp < AW)
-        walk_slice<DPL, GC, true>(kc + channel, vc + channel, row_stride, k_begin, k_end, pos, P.attn_scale, smf, warp, lane,
+        walk_slice<DPL, GC, true, true>(kc + channel, vc + channel, row_stride, k_begin, k_end, pos, P.attn_scale, smf, warp, lane,
             [&](float (&qr)[GC][DPL]) {
 #pragma unroll
                 for (int g = 0; g < GC; g++)

@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(threads(groups(MASK)), 1) gemm_blocks_kernel(c
 // alone took 270 of 1050 cycles).  So a stage is half a super-block, with accumulators of its own, and one barrier (done) says that its products are finished, which frees its
 // tokens and weights and hands its sums over.  A super-block of Q4_K takes 2200 cycles where it took 3200; the expansion's instructions bound then, of Q6_K above all (5000).
 // 21 tokens, us with the split of the tokens, before and now: Q4_K 28672 x 4096 56.6, 43.1; 4096 x 14336 39.1, 31.1; 4096 x 4096 21.2, 18.3; Q5_K 14336 x 4096 37.1, 29.8; Q6_K
-// 4096 x 14336 48.5, 46.2.  Sixteen warps of expansion and four of sums in place of eight and eight: 57.6 (the four are then behind, and the issuing warp is starved).
+// 4096 x 14336 48.5, 46.2, and 43.7 with twelve warps of expansion.  Sixteen warps of expansion and four of sums in place of eight and eight: 57.6 (the four are then behind, and the issuing warp is starved).
 // Tiles of more than 32 tokens leave room for one stage of it: 40 tokens 60.8, 70.8.
 template <int MASK>
 __global__ void __launch_bounds__(threads(few_groups(MASK)), 1) gemm_blocks_few_kernel(const __grid_constant__ BlkMaps maps, const __grid_constant__ BlkParams p) {

@@ -50,6 +50,7 @@ __host__ __device__ constexpr bool has_mins(int fmt) { return fmt <= 1; }      /
 struct alignas(64) BlkMaps { CUtensorMap x, sums, w[3]; };      // tokens, their sums, matrices as 32-bit words
 struct BlkParams : Deal {
     int Mp, kc, stages, b_stage, raw_depth, raw_slot, a_cols, d_bufs;
+    int d_cols;                // the form for a few tokens: columns of a stage's sums
     int tma;                   // a matrix's rows come by TMA (bits)
     unsigned* status;          // wait_status.cuh
 };
@@ -541,8 +542,9 @@ __global__ void __launch_bounds__(threads(few_groups(MASK)), 1) gemm_blocks_few_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     pdl_launch_dependents();
-    // tensor memory, stage by stage: sums (two k-blocks, minima), expanded k-blocks, minima
-    const uint32_t d_cols = (uint32_t)((MINS ? 3 : 2) * NT), a_base = (uint32_t)p.stages * d_cols, m_base = a_base + (uint32_t)(p.stages * 2 * p.a_cols);
+    // tensor memory, stage by stage: sums (two k-blocks; minima where a matrix of the launch has them), expanded k-blocks, minima.  Laid out by the host alone: formats side by
+    // side have one kernel, whether any of them has minima or none
+    const uint32_t d_cols = (uint32_t)p.d_cols, a_base = (uint32_t)p.stages * d_cols, m_base = a_base + (uint32_t)(p.stages * 2 * p.a_cols);
 
     if (warp < EPI_WARP) {
     if constexpr (XG == 3) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
@@ -983,9 +985,9 @@ bool gemm_blocks(const GemvMat* mats, int n_mat, int K, const BlockTokens& x, vo
     p.raw_slot = slot;
     const size_t cap = 213 * 1024;
     if (few) {                                                     // a stage is two k-blocks, with sums of its own
-        const int cols = (mins ? 3 : 2) * p.NT + 2 * p.a_cols + (mins ? 8 : 0);
+        p.d_cols = (mins ? 3 : 2) * p.NT;
         p.b_stage = (p.NT * (6 * 128 + (mins ? 64 : 0)) + 1023) / 1024 * 1024;
-        p.stages = std::min(STAGES_MAX, 512 / cols);
+        p.stages = std::min(STAGES_MAX, 512 / (p.d_cols + 2 * p.a_cols + (mins ? 8 : 0)));
     } else {
         p.b_stage = (p.NT * (128 * parts + (mins ? 32 * (parts - 1) : 0)) + 1023) / 1024 * 1024;
         for (p.stages = STAGES_MAX; p.stages > 2; p.stages--) {

@@ -24,6 +24,14 @@ def test_products(dts, tokens, rows, cols):
         assert rel(y[:tokens], x.double() @ W64.T) <= bound(d, 64) and (y[tokens] == 7.0).all()
 
 
+# formats without minima side by side: one kernel with those that have them, but no columns of tensor memory for their sums (3 stages of 16 tokens fill it to 480 of 512)
+@pytest.mark.parametrize("dts", [(DType.Q8_0, DType.Q4_0), (DType.Q4_0, DType.Q6_K), (DType.Q6_K, DType.Q8_0), (DType.Q8_0, DType.Q6_K, DType.Q4_0)], ids=lambda d: "+".join(t.name for t in d))
+@pytest.mark.parametrize("tokens", [1, 9, 16, 17, 32])
+@pytest.mark.parametrize("rows,cols", [(128, 256), (300, 4096), (20000, 512)])
+def test_formats_without_minima_side_by_side(dts, tokens, rows, cols):
+    test_products(dts, tokens, rows, cols)
+
+
 # tokens in blocks whose weights are pairs of halves: together from 9 (large matrices) and 17 tokens on, as exact as gemv_rows' 24-bit integers
 @pytest.mark.parametrize("dt", [DType.Q8_0, DType.Q4_0], ids=lambda d: d.name)
 @pytest.mark.parametrize("tokens,cols", [(9, 4096), (31, 14336)])

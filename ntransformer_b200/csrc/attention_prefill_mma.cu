@@ -65,6 +65,7 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 // Sums as in the form on tcgen05: each addition inside the tensor cores is cut off, so the high halves' products are summed over 64 channels and over a tile's 16 keys x 4
 // at most before F32 takes them, the low halves' apart, and queries go in under a power of two per row.  Error against 64 bits over 40 tokens behind 965, 8 heads of 128:
 // 3e-7; 7e-7 with scores and sums in one run each; 4e-7 on tcgen05.
+__host__ __device__ constexpr int slice_tiles(int tiles, int slices) { return (tiles + slices - 1) / slices; }      // the last slices may have fewer, or none
 template <int HD, int HDV, bool BF, bool SLICED>
 __global__ void __launch_bounds__(128, 2) prefill_mma_kernel(float* __restrict__ out, const float* __restrict__ Q,
                                                              const __half* __restrict__ kc, const __half* __restrict__ vc,
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(128, 2) prefill_mma_kernel(float* __restrict__
     const int first_win = chunk > 0 ? ((start_pos + qb * BQ) / chunk * chunk) / BKV : (window > 0 ? max(0, start_pos + qb * BQ - window + 1) / BKV : 0);
     const int n_keep = (window > 0 && chunk <= 0) ? min((keep + BKV - 1) / BKV, first_win) : 0;
     const int n_tiles = n_keep + (start_pos + last_q) / BKV + 1 - first_win;
-    const int per = SLICED ? (n_tiles + gridDim.z - 1) / gridDim.z : n_tiles, j0 = SLICED ? blockIdx.z * per : 0, j1 = SLICED ? min(n_tiles, j0 + per) : n_tiles;
+    const int per = SLICED ? slice_tiles(n_tiles, gridDim.z) : n_tiles, j0 = SLICED ? blockIdx.z * per : 0, j1 = SLICED ? min(n_tiles, j0 + per) : n_tiles;
     auto tile_of = [&](int j) { return j < n_keep ? j : first_win + (j - n_keep); };
 
     auto load_tile = [&](int j, int st) {
@@ -369,6 +370,9 @@ __global__ void __launch_bounds__(128) prefill_merge_kernel(const __grid_constan
     const int at = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;      // (query, head)
     if (at >= p.rows) return;
     const float2* ml = reinterpret_cast<const float2*>(parts + (size_t)p.slices * p.rows * HD);
+    // Slices that begin behind the query's position are left out, and no others: a weight of zero is none of a NaN or infinite sum of values that the query sees
+    const int row = at / p.n_heads, last = min(row / BQ * BQ + BQ, p.rows / p.n_heads) - 1;
+    const int seen = (p.start_pos + row) / BKV / slice_tiles((p.start_pos + last) / BKV + 1, p.slices) + 1;
     float2 mine = make_float2(-INFINITY, 0.f);
     if (lane < p.slices) mine = ml[(size_t)lane * p.rows + at];
     float o[SLICES][C];
@@ -380,14 +384,14 @@ __global__ void __launch_bounds__(128) prefill_merge_kernel(const __grid_constan
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, d));
     const float w = __expf(mine.x - m);
-    float l = w == 0.f ? 0.f : w * mine.y, sum[C] = {};      // (a slice that the query does not see: maximum -inf)
+    float l = lane < seen ? w * mine.y : 0.f, sum[C] = {};
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, d);
     float odd = 0.f;                                          // NaN where a sum is infinite or NaN
 #pragma unroll
     for (int i = 0; i < SLICES; i++) {
         const float wi = __shfl_sync(0xFFFFFFFFu, w, i);
-        if (wi != 0.f)
+        if (i < seen)
 #pragma unroll
             for (int c = 0; c < C; c++) sum[c] = fmaf(o[i][c], wi, sum[c]);
     }

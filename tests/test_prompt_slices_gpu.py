@@ -48,3 +48,30 @@ def test_values_that_a_row_does_not_see_and_nan():
     keep[60:, :2, 5] = keep[60:, 2:, 100] = False
     assert torch.isfinite(got[keep]).all() and rel(got[keep], want[keep]) <= 1e-6
     assert torch.isinf(got[60:, :2, 5]).all() and torch.isnan(got[60:, 2:, 100]).all()
+
+
+# keys whose scores are NaN, each seen first by the row at its own position: the first of a slice (no other of that slice for the row), one inside, and one whose slice has no weight beside
+# the others'; an infinite value there
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("at", [704, 705, 767])
+def test_keys_that_are_nan_reach_every_row_that_sees_them(dim, at):
+    q, kc, vc = inputs(4, 2, dim, 100, 700)
+    kc[at, 0, 3] = float("nan")
+    got, want = sliced(q, kc, vc, 700, dim ** -0.5), exact(q, torch.where(torch.isfinite(kc), kc, 0), vc, 700, dim ** -0.5)
+    assert torch.isnan(got[at - 700:, :2]).all()                   # heads 0 and 1 share the key head
+    keep = torch.ones_like(want, dtype=torch.bool)
+    keep[at - 700:, :2] = False
+    assert rel(got[keep], want[keep]) <= 1e-6
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+def test_slices_without_weight(dim):
+    q, kc, vc = inputs(4, 2, dim, 100, 700)
+    q, kc = q.abs(), kc.abs() * 0.1
+    kc[1] = 60.0                                                   # every query's weight, all but nothing else's
+    vc[400, 0, 7] = float("inf")
+    kc[401, 1, 2] = float("nan")
+    got = sliced(q, kc, vc, 700, 1.0)
+    assert not torch.isfinite(got[:, :2, 7]).any() and torch.isnan(got[:, 2:]).all()
+    keep = torch.arange(dim, device="cuda") != 7
+    assert rel(got[:, :2][:, :, keep], vc[1, 0].double()[keep].expand(100, 2, dim - 1)) <= 1e-6

@@ -76,7 +76,7 @@ Model::~Model() {
     for (void* p : {pf_arena_, sb_arena_}) if (p) cudaFree(p);
     if (!pf_arena_)                                                // a layer-spec model's
         for (void* p : {(void*)pf_.x, (void*)pf_.q, (void*)pf_.k, (void*)pf_.v, (void*)pf_.attn, pf_.ws, pf_.ws2, (void*)pf_.tok, (void*)pf_.pos, (void*)pf_.g, (void*)pf_.u,
-                        pf_.whi, pf_.wlo})
+                        pf_.whi, pf_.wlo, (void*)pf_.count})
             if (p) cudaFree(p);
     for (size_t i = 0; i < kcs_.size(); i++) if (kcs_[i] && (cache_owned_.empty() || cache_owned_[i])) { cudaFree(kcs_[i]); cudaFree(vcs_[i]); }
     for (void* p : {(void*)pf_.h, (void*)pf_.tmp, pf_.hws, (void*)want_out_, (void*)pf_.xs, (void*)pf_.maps, (void*)pf_.sel, (void*)pf_.work, (void*)pf_.wt,

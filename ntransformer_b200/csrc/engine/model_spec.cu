@@ -632,7 +632,8 @@ bool Model::spec_few_ready(int tokens) {
     return pf_.count && ensure_block_scratch(tokens);
 }
 bool Model::spec_dense(float* const* C, const void* A_split, const Weight* const* w, int n, int T, bool add, const float* row_scale, float alpha, cudaStream_t s) {
-    if (!A_split || !block_scratch_ || !pf_.count) return false;
+    // (the scratch is of the portion's tokens; a product over other rows, as those of the cache, may ask for more)
+    if (!A_split || !block_scratch_ || block_scratch_bytes_ < block_scratch_bytes(T) || !pf_.count) return false;
     int N[3];
     GemvMat m[3];
     for (int i = 0; i < n; i++) {

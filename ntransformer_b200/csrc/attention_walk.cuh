@@ -58,6 +58,9 @@ __device__ __forceinline__ void walk_slice(const __half* kbase, const __half* vb
     // Eight keys' sums by themselves before they join the run's, whose length then costs less: 1900 keys in two slices 2.6e-7 of error in one run, 1.8e-7 so.  Not where
     // the registers do not hold both (64 heads over 8: 4000 keys 12.3 us, 13.6 so; 27 queries behind 1900 85, 102).
     constexpr bool BLOCKED = APART && DPL * GC <= 16;
+    // Two chains of them, even and odd keys; one where two heads of 256 leave no registers for both (8 heads over 4, 15 queries behind 1500: 35.0 us in one run, 45.5 with two
+    // chains, 38.9 with one; 16 over 8, 6000 keys: 13.4, 14.8, 13.7)
+    constexpr int CHAINS = DPL == 8 && GC == 2 ? 1 : 2;
     float* pw = smem + (size_t)warp * GC * P_LD;
     float* red = smem + (size_t)WALK_WARPS * GC * P_LD;
     float* ml = red + (size_t)WALK_WARPS * GC * HD;
@@ -130,7 +133,7 @@ __device__ __forceinline__ void walk_slice(const __half* kbase, const __half* vb
         }
         __syncwarp();
         if constexpr (BLOCKED) {
-            float part[2][GC][DPL] = {};
+            float part[CHAINS][GC][DPL] = {};
 #pragma unroll
             for (int u = 0; u < KU; u++) {
                 if (k0 + u >= k_end) break;
@@ -141,14 +144,14 @@ __device__ __forceinline__ void walk_slice(const __half* kbase, const __half* vb
                 for (int g = 0; g < GC; g++) {
                     const float w = pw[u * GC + g];
 #pragma unroll
-                    for (int i = 0; i < DPL; i++) part[u & 1][g][i] = fmaf(w, vf[i], part[u & 1][g][i]);
+                    for (int i = 0; i < DPL; i++) part[u % CHAINS][g][i] = fmaf(w, vf[i], part[u % CHAINS][g][i]);
                 }
             }
 #pragma unroll
             for (int g = 0; g < GC; g++) {
                 const float c = pw[KU * GC + g];
 #pragma unroll
-                for (int i = 0; i < DPL; i++) acc[g][i] = fmaf(acc[g][i], c, part[0][g][i] + part[1][g][i]);
+                for (int i = 0; i < DPL; i++) acc[g][i] = fmaf(acc[g][i], c, CHAINS == 2 ? part[0][g][i] + part[CHAINS - 1][g][i] : part[0][g][i]);
             }
         } else {
 #pragma unroll

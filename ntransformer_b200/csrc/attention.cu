@@ -362,25 +362,54 @@ __global__ void __launch_bounds__(AW * 32, DPL * GC <= 32 ? 2 : 1) prefill_kerne
 
 int pick_gc(int group) { return group % 8 == 0 ? 8 : group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1; }
 
-// Slices of the keys of one query, `groups` CTAs to a slice: at least 32 keys each, and no more CTAs than are resident at once, two to an SM.  (One slice more, to leave no
-// SM with one CTA, began a second wave: 32 heads of 128 with keys of their own, 1000 and 4000 keys, ten slices and nine: 8.9, 7.1; 19.6, 14.6 us; 24 heads over 8, 4000
-// keys, 13 and 12: 15.8, 12.6.)
+constexpr int wave(int gc, int hd) { return 148 * (hd == 64 && gc <= 2 ? 3 : 2); }      // CTAs of the walk that are resident at once: those of narrow heads have 80 registers
+// Slices of the keys of one query that the scratch of a captured step has room for, `groups` CTAs to a slice: at least 32 keys each, two CTAs to an SM
 int wave_splits(int keys, int groups) { return std::max(1, std::min({2 * 148 / groups, (keys + 31) / 32, MAX_SPLITS})); }
+
+// Slices of a run of `tokens` queries over `total` keys, `groups` CTAs to a query and a slice: at least 32 keys each, at most three waves of CTAs.
+int rows_splits_most(int tokens, int total, int groups, int gc, int hd) { return std::max(1, std::min({3 * wave(gc, hd) / (groups * tokens), (total + 31) / 32, MAX_SPLITS})); }
+// A CTA takes 2 us and then, for a key, 11.9 ns and 1.95 ns for each query head that shares it (of 128), 1.5 times that with another on its SM and 2.2 times with two; a wave
+// begun costs 0.4 of one; the merge takes 2.7 us and 6 us for a million of the slices' sums, two launches 6.5 us at least.  Fitted to 882 calls (2 to 31 tokens, 4 to 48 groups, all widths, 0 to 1900 keys
+// before).  As many slices as two CTAs to an SM and one more, and these, us: 21 tokens, 32 heads of 128 over 8, behind 30, 120, 300, 1900: 10.5, 4.9; 12.6, 7.8; 17.1, 13.3;
+// 56.5, 50.8; 16 heads of 64, 16 behind 1900: 41.3, 37.1; the mean takes 0.89 of the time, a few up to 9 % longer.  (A wave of two CTAs of narrow heads to an SM, and 0.7 for
+// one begun: 56.9 there, and 40 heads of 128 over 8, 11 behind 1000 41.9 in two slices, 38.7 whole.)  Eight heads of 128 to a key head stay with the former: their sums are
+// one run (attention_walk.cuh), and longer slices would cost precision (31 queries behind 1000: 2.2e-7, 2.6e-7).
+int rows_splits(int tokens, int total, int groups, int gc, int hd) {
+    if (gc * hd > 512) return std::max(1, std::min({(2 * 148 + groups * tokens - 1) / (groups * tokens), (total + 31) / 32, MAX_SPLITS}));
+    const float key = 0.0119f + 0.00195f * gc * hd / 128, full = (float)wave(gc, hd);
+    int best = 1;
+    float least = 0.f;
+    for (int n = 1, most = rows_splits_most(tokens, total, groups, gc, hd); n <= most; n++) {
+        const int len = (total + n - 1) / n, used = (total + len - 1) / len, ctas = groups * tokens * used;
+        const float waves = ctas <= full ? 1.f : 0.4f * ceilf(ctas / full) + 0.6f * ctas / full, shared = ctas <= 148 ? 1.0f : full > 296.f ? 2.2f : 1.5f;
+        const float walked = (2.0f + key * len * shared) * waves, t = used > 1 ? std::max(6.5f, walked + 2.7f + 6e-6f * used * tokens * groups * gc * hd) : walked;
+        if (n == 1 || t < least) { least = t; best = used; }
+    }
+    return best;
+}
+// Of a single query.  As many as fit a wave of two CTAs to an SM: one slice more began a second wave (32 heads of 128 with keys of their own, 1000 and 4000 keys, ten slices and
+// nine: 8.9, 7.1; 19.6, 14.6 us; 24 heads over 8, 4000 keys, 13 and 12: 15.8, 12.6).  One more where three fit (64 heads of 64, 2000 and 6000 keys, four and five: 18.5, 16.0;
+// 50.6, 41.9).  Groups of more than half a wave would have one slice however many keys: up to three quarters of one, by what they cost (160 groups of 128, 2000 and 6000 keys,
+// one, two and these: 53.9, 50.9, 42.5; 151, 137, 102; 256 of 64, 2000: 64.7, 51.3, 47.2); beyond, memory is what bounds (240 of 128, 2000 keys, one and two: 55.7, 59.8).
+int decode_splits(int keys, int groups, int gc, int hd) {
+    if (keys <= 64) return 1;
+    if (groups > 148) return groups > wave(gc, hd) * 3 / 4 ? 1 : rows_splits(1, keys, groups, gc, hd);
+    return wave(gc, hd) > 296 ? std::min({(295 + groups) / groups, (keys + 31) / 32, MAX_SPLITS}) : wave_splits(keys, groups);
+}
 template <int DPL, int GC>
 void launch_decode(float* out, const float* q, const __half* kc, const __half* vc, int seq_len, int n_heads, int n_kv,
                    float scale, cudaStream_t s) {
     constexpr int HD = DPL * 32;
     int groups = n_heads / GC;
-    int n_splits = seq_len > 64 ? wave_splits(seq_len, groups) : 1;
+    int n_splits = decode_splits(seq_len, groups, GC, HD);
     int split_len = (seq_len + n_splits - 1) / n_splits;
     n_splits = (seq_len + split_len - 1) / split_len;
     const size_t smem = ((size_t)walk_floats<DPL, GC>() + (size_t)GC * HD + 2 * GC) * sizeof(float);
-    static unsigned long long configured = 0;      // bit per device id
+    static unsigned long long configured[2] = {};      // bit per device id
     // sums apart where the groups do not fill the wave, so that the slices are longer (32 groups, 2000 keys: 1.94e-7 of error, 1.81e-7 so); elsewhere they cost 1 % and nothing calls for them
-    auto kernel = 296 % groups ? decode_kernel<DPL, GC, true> : decode_kernel<DPL, GC, false>;
-    opt_in_dynamic_smem(decode_kernel<DPL, GC, false>, (int)(ATTN_MAX_DYN_SMEM), configured);
-    static unsigned long long configured_apart = 0;
-    opt_in_dynamic_smem(decode_kernel<DPL, GC, true>, (int)(ATTN_MAX_DYN_SMEM), configured_apart);
+    const bool apart = 296 % groups != 0;
+    auto kernel = apart ? decode_kernel<DPL, GC, true> : decode_kernel<DPL, GC, false>;
+    opt_in_dynamic_smem(kernel, (int)(ATTN_MAX_DYN_SMEM), configured[apart]);
     // the slices' results: the stream's, so that calls on other streams and devices and by other threads have their own
     std::optional<StreamMemory> memory;
     if (n_splits > 1) memory.emplace((size_t)n_heads * n_splits * (HD + 2) * sizeof(float), s);
@@ -397,26 +426,6 @@ void launch_decode(float* out, const float* q, const __half* kc, const __half* v
     }
 }
 
-// Slices of a run of `tokens` queries over `total` keys, `groups` CTAs to a query and a slice: at least 32 keys each, at most three waves of CTAs, two to an SM.
-int rows_splits_most(int tokens, int total, int groups) { return std::max(1, std::min({888 / (groups * tokens), (total + 31) / 32, MAX_SPLITS})); }
-// A CTA takes 2 us and then, for a key, 10.5 ns and 2.3 ns for each query head that shares it (of 128), 1.75 times that beside another on its SM (half a wave is enough
-// for that: CTAs that wait for the launch before gather two to an SM); a wave begun costs most of one; the merge takes 3.5 us and 6 us for a million of the slices' sums.
-// Before: as many slices as a wave of CTAs and one more, whatever they cost.  21 tokens, 32 heads of 128 over 8, behind 30, 120, 300, 1900 (us, before and now): 10.5, 4.9;
-// 12.6, 7.8; 17.1, 13.3; 56.5, 50.8; 180 calls (2 to 31 tokens, 16 to 32 heads, both widths, 30 to 1900 keys before): the mean takes 0.8 of the time.  Eight heads of
-// 128 to a key head stay with that: their sums are one run (attention_walk.cuh), and longer slices would cost precision (31 queries behind 1000: 2.2e-7, 2.6e-7).
-int rows_splits(int tokens, int total, int groups, int gc, int hd) {
-    if (gc * hd > 512) return std::max(1, std::min({(2 * 148 + groups * tokens - 1) / (groups * tokens), (total + 31) / 32, MAX_SPLITS}));
-    const float key = 0.0105f + 0.0023f * gc * hd / 128;
-    int best = 1;
-    float least = 0.f;
-    for (int n = 1, most = rows_splits_most(tokens, total, groups); n <= most; n++) {
-        const int len = (total + n - 1) / n, used = (total + len - 1) / len, ctas = groups * tokens * used;
-        const float waves = ctas <= 296 ? 1.f : 0.7f * ((ctas + 295) / 296) + 0.3f * ctas / 296;
-        const float t = (2.0f + key * len * (ctas <= 74 ? 1.0f : 1.75f)) * waves + (used > 1 ? 3.5f + 6e-6f * used * tokens * groups * gc * hd : 0.f);
-        if (n == 1 || t < least) { least = t; best = used; }
-    }
-    return best;
-}
 // A few consecutive queries (start_pos ...), each with the arithmetic of a decoded token; scratch: attention_rows_scratch_floats().
 template <int DPL, int GC>
 void launch_rows(float* out, const float* q, const __half* kc, const __half* vc, int tokens, int start_pos, int n_heads, int n_kv, float scale, float* scratch,
@@ -529,7 +538,7 @@ void attention_decode(float* out, const float* q, const void* kc, const void* vc
 size_t attention_rows_scratch_floats(int tokens, int max_seq, int n_heads, int n_kv, int hd) {
     const int gc = pick_gc(n_heads / n_kv);
     size_t most = 0;                     // fewer tokens are cut into more slices
-    for (int t = 1; t <= tokens; t++) most = std::max(most, (size_t)t * n_heads * rows_splits_most(t, max_seq, n_heads / gc) * (hd + 2));
+    for (int t = 1; t <= tokens; t++) most = std::max(most, (size_t)t * n_heads * rows_splits_most(t, max_seq, n_heads / gc, gc, hd) * (hd + 2));
     return most;
 }
 void attention_rows_f16(float* out, const float* q, const void* kc, const void* vc, int tokens, int start_pos, int n_heads, int n_kv, int hd, float scale,

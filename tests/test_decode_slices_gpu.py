@@ -20,3 +20,10 @@ def test_slices(heads, kv, dim, keys):
     torch.cuda.synchronize()
     # weights to 2^-22, sums of at most keys / 8 of them in a run: sqrt of that many roundings of 2^-24
     assert rel(out, exact(q, kc, vc, keys - 1, dim ** -0.5)) <= 2.0**-22 + (keys / 8) ** 0.5 * 2.0**-24
+
+
+# three CTAs to an SM (narrow heads: as many slices as two of them leave room for, and one more); more groups than half a wave and than three quarters, where slices go by their cost
+@pytest.mark.parametrize("heads,kv,dim", [(64, 64, 64), (40, 20, 64), (16, 8, 256), (210, 210, 128), (320, 160, 128), (256, 256, 64), (340, 340, 64)])
+@pytest.mark.parametrize("keys", [65, 700, 2000])
+def test_slices_by_width_and_cost(heads, kv, dim, keys):
+    test_slices(heads, kv, dim, keys)

@@ -602,7 +602,8 @@ bool attention_prefill_tc_pays(int seq_len, int start_pos, int n_heads, int hd) 
 // mma.sync 5.5 and 2.1 (4.2 and 1.3); slices with their merge 6.0 and 2.3 (1.4) for 64 keys of one, 1.7 (1.5) times that where two CTAs share an SM, and the sums at
 // 0.35 us a megabyte; a slice more costs 0.2.  Whole, in slices: heads of 128, 8 of them, 40 tokens behind 965: 31.2, 13.2; 64, 17 behind 1000: 32.1, 22.8; 2, 1500 behind
 // 1500: 78.3, 39.3; 8, 518 behind 5: 24.2, 21.4; heads of 64, 16 of them, 60 behind 700: 18.8, 10.5.  Not cut: 32 heads of 128, 256 behind 0: 14.4, 18.8 in two;
-// 64 heads, 128 behind 1000: 37.0, 42.5.  Of 110 calls with less than a wave of CTAs none is slower by more than 2 %; half take less than 0.6 of the time.
+// 64 heads, 128 behind 1000: 37.0, 42.5.  Cut only where 2.2 us are gained by that account, which is out by as much where tiles are few (16 heads, 224 behind 0: 12.6, 14.6 in
+// two): of 768 calls with less than a wave of CTAs none is then slower, and the mean takes 0.71 of the time.
 // Between programmatic launches the plain one costs 3 to 4 us more: 60 tokens behind 900, 32 heads of 128, two layers of 4096: 443 us whole, 426 in slices.
 int attention_prefill_slices_for(int form, int seq_len, int start_pos, int n_heads, int hd, int max_seq, bool in_chain) {
     const long long ctas = (long long)((seq_len + 63) / 64) * n_heads, tiles = ((long long)start_pos + seq_len + 63) / 64;
@@ -611,7 +612,7 @@ int attention_prefill_slices_for(int form, int seq_len, int start_pos, int n_hea
     const float whole = form == PREFILL_TC ? (wide ? 8.0f + 1.5f * tiles : 4.5f + 1.2f * tiles) : (wide ? 5.5f + 2.1f * tiles : 4.2f + 1.3f * tiles);
     const float written = 0.35e-6f * 4 * seq_len * n_heads * hd + 0.2f;       // a slice's sums, there and back
     int best = 1;
-    float least = whole - (in_chain ? 5.0f : 1.5f);
+    float least = whole - (in_chain ? 5.0f : 2.2f);
     for (int n = 2; n <= 16 && n <= tiles; n++) {
         const long long all = ctas * n, steps = (tiles + n - 1) / n * ((all + 295) / 296);
         const float t = 6.0f + (wide ? 2.3f : 1.4f) * steps * (all <= 148 ? 1.0f : wide ? 1.7f : 1.5f) + n * written;

@@ -179,10 +179,12 @@ __device__ __forceinline__ int staged_at(int i, int half) { return half ? ((i & 
 // BF16 in a graph, before -> now: 14336 + 14336 rows of 4096, gated 49.1 -> 37.7 us (6.2 TB/s), 32000 x 4096 52.4 -> 39.4 (6.7), 4096 x 4096 11.1 -> 8.3,
 // 3000 x 3000 11.1 -> 6.3; F16 4096 x 11008 24.4 -> 17.5.  Where a CTA has more than sixteen rounds its rows lie side by side (128256 x 4096 F16 154.5 -> 149.5 us); with fewer
 // they are spread over all CTAs, whose last rounds then differ by a warp's.
-template <typename T, bool VEC, bool STREAMS>          // STREAMS: the epilogue may be DENSE_STREAMS (its registers are the kernel's without it)
+// STREAMS: the epilogue may be DENSE_STREAMS (its registers are the kernel's without it).  EARLY: lets the next launch start at once, otherwise at its end (calls behind the launcher
+// boundary alone; by a parameter of the kernel, 8192 x 28672 took 126 us, 122 so)
+template <typename T, bool VEC, bool STREAMS, bool EARLY>
 __global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_dense_kernel(DenseMats m, const float* __restrict__ x, int K, int ep,
                                                                       const float* __restrict__ row_scale, float alpha, int KW, int vec,
-                                                                      const float* __restrict__ norm_w, float eps, StreamsIO sio, int norm_groups, int early) {
+                                                                      const float* __restrict__ norm_w, float eps, StreamsIO sio, int norm_groups) {
     extern __shared__ __align__(16) float xs[];
     __shared__ float red[DV_WARPS];
     __shared__ float inv_g[DENSE_MAX_NORM_GROUPS];
@@ -203,7 +205,7 @@ __global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_d
     };
     const int teams = DV_WARPS / KW;
     int r = total > 16 * step ? blockIdx.x * teams + team : blockIdx.x + team * (int)gridDim.x;
-    if (early) pdl_launch_dependents();
+    if (EARLY) pdl_launch_dependents();
     if constexpr (VEC) {
         // lanes 0..15: the lines of the first chunk; lanes 16..31: those of the one after it
         int r1 = r, sub1 = 0, c1 = 0;
@@ -333,7 +335,7 @@ __global__ void __launch_bounds__(DV_WARPS * 32, VEC && !STREAMS ? 4 : 2) gemv_d
             walk(b, a);
         }
     }
-    if (!early) pdl_launch_dependents();
+    if (!EARLY) pdl_launch_dependents();
 }
 
 // batch of up to 128 pieces from v0 on, four 16-byte loads in flight per lane
@@ -594,14 +596,18 @@ void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpil
     const bool walk = vec && dt != DType::F32;
     const int per_sm = !walk ? 8 : ep == DENSE_STREAMS ? 2 : 4;
     const int resident = (int)std::max<size_t>(1, std::min<size_t>((size_t)per_sm, (size_t)(220 * 1024) / (smem + (walk ? 3 : 1) * 1024))) * 148;
-    // Warps to a row: what the CTA that ends last takes, its rounds of rows times their pieces of 1024 columns to a warp and 0.4 of one for a row's end; a
-    // single piece takes as long as two, of which one is under way while the other is multiplied (fits 16 shapes from 2048 x 8192 to
-    // 28672 x 4096 with 1, 2, 4 and 8 warps).  F16, us: 4096 x 14336 29.0, 25.3, 24.7, 24.7; 11008 x 4096 18.3, 16.7, 18.6, 28.9; 128256 x 4096 150 with one; 2048 x 8192 9.4, 8.4, 8.5, 8.8.
+    // Warps to a row: what the CTA that ends last takes, its rounds of rows times their pieces of 1024 columns to a warp (one and a half at least), 0.2 of one for a row's end and 0.2 for
+    // a meeting of warps; and 0.2 of one for 1024 numbers of the vector, which each of an SM's CTAs lays out for itself (fits 120 shapes from 32 x 2304 to 57344 x 8192, from HBM and from
+    // L2, with 1, 2, 4 and 8 warps, to 0.5 % of the best on average).  F16, us: 4096 x 14336 29.0, 25.3, 24.7, 24.7; 11008 x 4096 18.3, 16.7, 18.6, 28.9; 128256 x 4096 150 with one;
+    // 2048 x 8192 9.4, 8.4, 8.5, 8.8.  BF16 896 x 4864 6.4, 5.6, 6.0, 6.0; 1041 x 9216 9.2, 7.5, 8.7, 9.1; 20858 + 20858 x 1424, gated 23.8, 26.8, 47, 87.
     // (With two rows to a warp throughout, F16's form before: 270 x 11776 14.9, now 5.9; 1024 x 4096 7.1, 3.9; 4096 x 4096 9.2, 7.4; 8192 x 28672 142, 128.)
     int kw = 1;
     double least = 0;
     for (int k = 1; walk && k <= DV_WARPS && (k == 1 || k * 64 * per16 < K); k *= 2) {
-        const double cost = (double)(((long long)total * k + resident * DV_WARPS - 1) / (resident * DV_WARPS)) * (std::max(2, (glu ? 2 : 1) * ((K + 128 * per16 * k - 1) / (128 * per16 * k))) + 0.4);
+        const long long warps = (long long)total * k;
+        const double rounds = (double)((warps + resident * DV_WARPS - 1) / (resident * DV_WARPS)), pieces = (glu ? 2 : 1) * ((K + 128 * per16 * k - 1) / (128 * per16 * k));
+        const double ctas = (double)std::min<long long>((warps + DV_WARPS - 1) / DV_WARPS, resident);
+        const double cost = rounds * (std::max(1.5, pieces) + (k > 1 ? 0.4 : 0.2)) + 0.2 * K / 1024 * std::ceil(ctas / 148);
         if (k == 1 || cost < least) { least = cost; kw = k; }
     }
     const int rows_at_once = DV_WARPS / kw;
@@ -610,11 +616,11 @@ void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpil
     // 26.9 against 23.6 launched plainly; 4096 x 4096 6.1, 8.35).  In a step the next launch is another kernel.
     const bool programmatic = pdl_enabled() || (boundary && (size_t)total * m.pitch[0] <= (size_t)64 << 20);
     const int grid = std::min((total + rows_at_once - 1) / rows_at_once, resident);
-#define NT_DVV(TY, VEC, ST) { static unsigned long long done = 0; if (smem > 40 * 1024) opt_in_dynamic_smem(gemv_dense_kernel<TY, VEC, ST>, 200 * 1024, done); \
-                              launch_k_pdl(programmatic, gemv_dense_kernel<TY, VEC, ST>, dim3(grid), dim3(DV_WARPS * 32), smem, s, m, x, K, (int)ep, row_scale, alpha, kw, vec, norm_w, eps, sio, norm_groups, \
-                                           pdl_enabled() ? 1 : 0); }
-#define NT_DV(TY) { if (!walk) NT_DVV(TY, false, true) else if (ep == DENSE_STREAMS) NT_DVV(TY, true, true) else NT_DVV(TY, true, false) }
-    if (dt == DType::F32) NT_DVV(float, false, true) else if (dt == DType::F16) NT_DV(__half) else NT_DV(__nv_bfloat16)
+#define NT_DVV(TY, VEC, ST, EARLY) { static unsigned long long done = 0; if (smem > 40 * 1024) opt_in_dynamic_smem(gemv_dense_kernel<TY, VEC, ST, EARLY>, 200 * 1024, done); \
+                              launch_k_pdl(programmatic, gemv_dense_kernel<TY, VEC, ST, EARLY>, dim3(grid), dim3(DV_WARPS * 32), smem, s, m, x, K, (int)ep, row_scale, alpha, kw, vec, norm_w, eps, sio, norm_groups); }
+#define NT_DV(TY) { if (!walk) NT_DVV(TY, false, true, true) else if (ep == DENSE_STREAMS) NT_DVV(TY, true, true, true) else NT_DVV(TY, true, false, true) }
+    if (boundary && walk && dt == DType::F16 && ep != DENSE_STREAMS && !pdl_enabled()) NT_DVV(__half, true, false, false)
+    else if (dt == DType::F32) NT_DVV(float, false, true, true) else if (dt == DType::F16) NT_DV(__half) else NT_DV(__nv_bfloat16)
 #undef NT_DV
 #undef NT_DVV
     count_launch();

@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(F16_WARPS * 32) gemv_f16_kernel(float* __restr
     }
     pdl_launch_dependents();
 }
-constexpr int F16_SHORT = 2048;          // columns
+constexpr int F16_SHORT = 2048, F16_SHORT_STORED = 2560;          // columns
 
 }  // namespace
 
@@ -261,14 +261,18 @@ void gemv_generic(float* y, const void* W, const float* x, int out, int in, DTyp
     const uint8_t* w = static_cast<const uint8_t*>(W);
     if (dt == DType::F16 && in % 8 == 0 && pitch % 16 == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (size_t)in * 4 <= (size_t)200 * 1024 && ep != GEMV_SWIGLU) {
-        if (in > F16_SHORT) {
+        // three pieces of a row, which two warps to a row do not halve, and a second round of gemv_dense's rows for less than a fifth of one
+        const bool tail = ep != GEMV_ADD && in <= 3 * 1024 && out > 148 * 32 && out <= 148 * 32 * 6 / 5;
+        if (in > (ep == GEMV_ADD || out < 4096 ? F16_SHORT : F16_SHORT_STORED) && !tail) {
             GemvMat m;
             m.W = W; m.y = y; m.out = out; m.dtype = dt; m.row_pitch = pitch;
             gemv_dense(&m, 1, in, x, ep == GEMV_ADD ? DENSE_ADD : DENSE_STORE, nullptr, 1.0f, s, nullptr, 0.f, nullptr, 1, true);
             return;
         }
         // Rows of one or two pieces of gemv_dense's: twice its CTAs to an SM, and two rows to a warp, keep more loads under way (us here, there: 100000 x 1024 34.3, 37.4; 128256 x 2048
-        // 79.7, 83.6; 2000 x 2048 3.43, 3.55; rows of 3072: 900 of them 3.46, 3.57, 20000 23.9, 22.8)
+        // 79.7, 83.6; 2000 x 2048 3.43, 3.55).  Of three, where nothing is read back: 8192 x 2304 8.5, 8.9, and 6.6, 8.7 from L2; 54683 x 2304 39.5, 43.1; added to what is there 13.0,
+        // 9.1.  Rows of 3072: 900 of them 3.46, 3.57; 4096 7.3, 6.6, and 5.5, 6.2 from L2; 32000 33.3, 32.1; but 5120, a second round there, 7.9, 9.2.  (5120 x 5120
+        // 11.3, 12.4, but 2.4e-7 of error here and 1.8e-7 there, where two warps share a row)
         const int pairs = (out + 1) / 2;
         int grid16 = (pairs + F16_WARPS - 1) / F16_WARPS;
         const int resident = (int)std::min<size_t>(8, (size_t)(220 * 1024) / ((size_t)in * 4 + 1024)) * 148;   // CTAs the chip holds

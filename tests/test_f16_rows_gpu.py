@@ -21,3 +21,15 @@ def test_products(rows, cols, dt, torch_type):
     torch.cuda.synchronize()
     # F32 sums of cols products, 32 lanes of each row by themselves
     assert rel(y[:rows], W.double() @ x.double()) <= (cols / 32) ** 0.5 * 2.0 ** -24 + 2.0 ** -22 and y[rows] == 7.0
+
+
+# rows of three pieces: few, many, and a little more than a round of gemv_dense's, with and without what is there already
+@pytest.mark.parametrize("rows,cols", [(4095, 2304), (4096, 2304), (9000, 2560), (4736, 3072), (4737, 3072), (5684, 3072)])
+def test_rows_of_three_pieces(rows, cols):
+    test_products(rows, cols, DType.F16, torch.float16)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    W, x = (torch.randn(rows, cols, generator=g, device="cuda") * cols ** -0.5).half(), activations(1, cols, cols)[0]
+    y = torch.full((rows + 1,), 3.0, device="cuda")
+    lib().nt_b200_gemv_add(y.data_ptr(), W.data_ptr(), x.data_ptr(), rows, cols, int(DType.F16), stream())
+    torch.cuda.synchronize()
+    assert rel(y[:rows], 3.0 + W.double() @ x.double()) <= (cols / 32) ** 0.5 * 2.0 ** -24 + 2.0 ** -22 and y[rows] == 3.0

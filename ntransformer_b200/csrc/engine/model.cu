@@ -864,7 +864,8 @@ bool Model::prefill_short(const int* tokens, int seq_len, int start_pos) {
         int n = 0;
         for (auto& [w, y] : list) { m[n].W = w->ptr; m[n].y = y; m[n].out = w->rows; m[n].dtype = w->dtype; m[n++].row_pitch = w->pitch; }
         if (dense) {
-            const BlockTokens t = up ? silu_split_tokens(sb_.ws, x, up, T, K, true, s) : split_tokens(sb_.ws, x, norm, cfg_.norm_eps, T, K, true, s);
+            const TokenParts parts = TokenParts::F16_SHORT;
+            const BlockTokens t = up ? silu_split_tokens(sb_.ws, x, up, T, K, true, s, parts) : split_tokens(sb_.ws, x, norm, cfg_.norm_eps, T, K, true, s, parts);
             NT_CHECK(gemm_dense_tc(m, n, K, t, block_scratch_->p, T, ep == GEMV_ADD, s), "GEMM of a few tokens over F16 rejected");
             return ep == GEMV_SWIGLU;
         }

@@ -700,7 +700,7 @@ void Model::prefill_spec(const int* tokens, int seq_len, int start_pos, bool few
             const LayerWeights& L = layer_weights(i);
             if (few) {
                 const int odim = S.heads * S.vdim;
-                const BlockTokens h = split_tokens(pf_.hws, pf_.x, L.attn_norm, cfg_.norm_eps, T, hidden, true, s, true);
+                const BlockTokens h = split_tokens(pf_.hws, pf_.x, L.attn_norm, cfg_.norm_eps, T, hidden, true, s, TokenParts::BF16);
                 const GemvMat qkv[3] = {mat_of(L.wq, pf_.q), mat_of(L.wk, pf_.k), mat_of(L.wv, pf_.v)}, o = mat_of(L.wo, pf_.x), gu[2] = {mat_of(L.gate, pf_.g), mat_of(L.up, pf_.u)},
                               down = mat_of(L.down, pf_.x);
                 auto gemm = [&](const GemvMat* mats, int n, int K, const BlockTokens& t, bool add, const float* ls) {
@@ -711,10 +711,10 @@ void Model::prefill_spec(const int* tokens, int seq_len, int start_pos, bool few
                 qk_norm_kv_write(pf_.q, pf_.k, pf_.v, L.q_norm, L.k_norm, cfg_.norm_eps, kcs_[(size_t)i], vcs_[(size_t)i], cache_dt_, T, nullptr, p0,
                                  S.heads * S.dim, S.kv_heads * S.dim, S.kv_heads * S.vdim, s);
                 attention_window(pf_.attn, pf_.q, kcs_[(size_t)i], vcs_[(size_t)i], cache_dt_, T, nullptr, p0, cfg_.max_seq_len, attn_of(S), s);
-                gemm(&o, 1, odim, split_tokens(pf_.ws, pf_.attn, nullptr, 0.f, T, odim, true, s, true), true, L.ls1);
+                gemm(&o, 1, odim, split_tokens(pf_.ws, pf_.attn, nullptr, 0.f, T, odim, true, s, TokenParts::BF16), true, L.ls1);
                 if (S.ff > 0) {
                     glu_mul(pf_.g, pf_.g, pf_.u, (size_t)T * S.ff, S.act == GluAct::GELU_TANH, s);
-                    gemm(&down, 1, S.ff, split_tokens(pf_.ws2, pf_.g, nullptr, 0.f, T, S.ff, true, s, true), true, L.ls2);
+                    gemm(&down, 1, S.ff, split_tokens(pf_.ws2, pf_.g, nullptr, 0.f, T, S.ff, true, s, TokenParts::BF16), true, L.ls2);
                 }
                 continue;
             }

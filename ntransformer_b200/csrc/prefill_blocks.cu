@@ -760,11 +760,12 @@ __global__ void __launch_bounds__(threads(few_groups(MASK)), 1) gemm_blocks_few_
 // a plain split, which may be the one written to) as F16 hi + lo, the sums of 32 of them
 // (a 32nd part, so that they stay within F16) as hi + lo, FINE: the halves that those two leave of both, and the factor that undoes the token's power of two.  That power takes the largest to 2^13 .. 2^14, where the
 // low halves keep their bits.  Block 0 also clears the product's counts: a launch whose wait ran out leaves some behind.
-// TOK_NORM_ANY: TOK_NORM whose gains do not lie on 16 bytes.  BF16: parts in BF16, no power, no sums.
+// TOK_NORM_ANY: TOK_NORM whose gains do not lie on 16 bytes.  BF16 parts: no power; those for dense matrices: no sums.
 enum : int { TOK_PLAIN = 0, TOK_NORM = 1, TOK_SILU = 2, TOK_SPLIT = 3, TOK_NORM_ANY = 4 };
-template <int MODE, bool FINE, bool BF16>
+template <int MODE, bool FINE, TokenParts PARTS>
 __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* lo, __half* third, __half* __restrict__ sums, __half* __restrict__ third_sums, float* __restrict__ scale, unsigned* __restrict__ count, int counts,
                                                            const float* xin, const float* w, float eps, int K) {
+    constexpr bool BF16 = PARTS == TokenParts::BF16;
     constexpr int KEEP = 7;                                        // chunks of 2048 held in registers: rows to 14336
     __shared__ float red[2][16];
     const int tid = threadIdx.x;
@@ -820,17 +821,25 @@ __global__ void __launch_bounds__(512) split_tokens_kernel(__half* hi, __half* l
         return upper ? v - fh.y - fl.y : v - fh.x - fl.x;
     };
     [[maybe_unused]] auto pair = [](float a, float b) { uint32_t h, l; split_pair(a, b, BF16, h, l); return h; };
+    auto split = [](float a, float b, uint32_t& h, uint32_t& l) {
+        if (PARTS != TokenParts::F16_SHORT) { split_pair(a, b, BF16, h, l); return; }
+        // the nearest numbers of 24 - n bits, c = 2^n + 1 (Dekker's splitting)
+        auto top = [](float a, float b, float c) { const float p = __fmul_rn(a, c), q = __fmul_rn(b, c); return __floats2half2_rn(__fsub_rn(p, __fsub_rn(p, a)), __fsub_rn(q, __fsub_rn(q, b))); };
+        const __half2 p = top(a, b, 1048577.0f);
+        const float2 f = __half22float2(p);
+        h = bits(p); l = bits(top(a - f.x, b - f.y, 65537.0f));
+    };
     auto put = [&](int i, float4 a) {
         a.x *= f; a.y *= f; a.z *= f; a.w *= f;
         uint2 ph, pl;
-        split_pair(a.x, a.y, BF16, ph.x, pl.x);
-        split_pair(a.z, a.w, BF16, ph.y, pl.y);
+        split(a.x, a.y, ph.x, pl.x);
+        split(a.z, a.w, ph.y, pl.y);
         *reinterpret_cast<uint2*>(h + i) = ph;
         *reinterpret_cast<uint2*>(l + i) = pl;
         if (FINE)
             *reinterpret_cast<uint2*>(third + (size_t)blockIdx.x * K + i) =
                 make_uint2(pair(rest(a.x, ph.x, pl.x, false), rest(a.y, ph.x, pl.x, true)), pair(rest(a.z, ph.y, pl.y, false), rest(a.w, ph.y, pl.y, true)));
-        if (BF16) return;                                          // (matrices in BF16 have no minima)
+        if (PARTS != TokenParts::F16) return;                      // (dense matrices have no minima)
         float s = (a.x + a.y) + (a.z + a.w);                       // K is a multiple of 256: whole warps
         s += __shfl_xor_sync(0xFFFFFFFFu, s, 1); s += __shfl_xor_sync(0xFFFFFFFFu, s, 2); s += __shfl_xor_sync(0xFFFFFFFFu, s, 4);
         if ((tid & 7) == 0) {
@@ -911,26 +920,28 @@ BlockTokens block_tokens(void* workspace, int T, int K, bool fine) {
 
 namespace {
 template <int MODE>
-BlockTokens launch_split(void* workspace, const float* x, const float* w, float eps, int T, int K, bool fine, bool bf16, cudaStream_t s) {
+BlockTokens launch_split(void* workspace, const float* x, const float* w, float eps, int T, int K, bool fine, TokenParts parts, cudaStream_t s) {
     const BlockTokens t = block_tokens(workspace, T, K, fine);
     const size_t part = padded(T) * (size_t)K;
     __half *hi = static_cast<__half*>(t.split), *sums = static_cast<__half*>(t.sums);
-    const auto kernel = bf16 ? (fine ? split_tokens_kernel<MODE, true, true> : split_tokens_kernel<MODE, false, true>) : fine ? split_tokens_kernel<MODE, true, false> : split_tokens_kernel<MODE, false, false>;
+    const auto kernel = parts == TokenParts::BF16 ? (fine ? split_tokens_kernel<MODE, true, TokenParts::BF16> : split_tokens_kernel<MODE, false, TokenParts::BF16>)
+                        : !fine                   ? split_tokens_kernel<MODE, false, TokenParts::F16>
+                        : parts == TokenParts::F16 ? split_tokens_kernel<MODE, true, TokenParts::F16> : split_tokens_kernel<MODE, true, TokenParts::F16_SHORT>;
     launch_k_pdl(true, kernel, dim3(T), dim3(512), 0, s, hi, hi + part, hi + 2 * part, sums, sums + part / 16, t.scale, t.count, sm_count(), x, w, eps, K);
     count_launch();
     return t;
 }
 }  // namespace
 
-BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, float eps, int T, int K, bool fine, cudaStream_t s, bool bf16) {
-    if (!norm_w) return launch_split<TOK_PLAIN>(workspace, x, nullptr, 0.f, T, K, fine, bf16, s);
-    return (reinterpret_cast<uintptr_t>(norm_w) & 15) ? launch_split<TOK_NORM_ANY>(workspace, x, norm_w, eps, T, K, fine, bf16, s) : launch_split<TOK_NORM>(workspace, x, norm_w, eps, T, K, fine, bf16, s);
+BlockTokens split_tokens(void* workspace, const float* x, const float* norm_w, float eps, int T, int K, bool fine, cudaStream_t s, TokenParts parts) {
+    if (!norm_w) return launch_split<TOK_PLAIN>(workspace, x, nullptr, 0.f, T, K, fine, parts, s);
+    return (reinterpret_cast<uintptr_t>(norm_w) & 15) ? launch_split<TOK_NORM_ANY>(workspace, x, norm_w, eps, T, K, fine, parts, s) : launch_split<TOK_NORM>(workspace, x, norm_w, eps, T, K, fine, parts, s);
 }
-BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, bool fine, cudaStream_t s) {
-    return launch_split<TOK_SILU>(workspace, gate, up, 0.f, T, K, fine, false, s);
+BlockTokens silu_split_tokens(void* workspace, const float* gate, const float* up, int T, int K, bool fine, cudaStream_t s, TokenParts parts) {
+    return launch_split<TOK_SILU>(workspace, gate, up, 0.f, T, K, fine, parts, s);
 }
 BlockTokens resplit_tokens(void* workspace, const void* hi, const void* lo, int T, int K, cudaStream_t s) {
-    return launch_split<TOK_SPLIT>(workspace, static_cast<const float*>(hi), static_cast<const float*>(lo), 0.f, T, K, false, false, s);
+    return launch_split<TOK_SPLIT>(workspace, static_cast<const float*>(hi), static_cast<const float*>(lo), 0.f, T, K, false, TokenParts::F16, s);
 }
 // A plain split as it lies, for matrices without minima: it has no sums, and powers of 2^0
 static size_t plain_tokens_bytes(int T) { return padded(T) * sizeof(float) + (size_t)sm_count() * sizeof(unsigned); }

@@ -4,13 +4,13 @@
 // projection of an 8B model over 100 tokens has 16 of them.  Here W is A (128 rows to a tile), tokens are B (NT, a multiple of 16 up to 128), and tiles times units of 256
 // columns are dealt out evenly (tile_deal.cuh), so that every SM streams W.
 //   * W and tokens by TMA into a ring of k-blocks of 64 columns, deep enough for HBM's latency (64 to 112 KB of W in flight to an SM);
-//   * tokens as two halves (or two BF16), a unit of 256 columns to an accumulator, added up in F32 registers; or, in the fine form, as three (33 bits of F16, 24 of
-//     BF16) with 64 columns to an accumulator, as exact as F32 products one by one (the tensor cores cut off each addition, which leaves 1.86e-8 of a sum for each);
+//   * tokens as two halves (or two BF16), a unit of 256 columns to an accumulator, added up in F32 registers; or, in the fine form, as three (24 bits
+//     and more, in small first parts: TokenParts) with 64 columns to an accumulator, as exact as F32 products one by one (the tensor cores cut off each addition, which leaves 1.86e-8 of a sum for each);
 //   * the parts of a tile lie one behind the other in shared memory and are ONE operand of parts * NT rows: a product for 16 columns in place of two or three, and the epilogue adds
 //     what the parts gave (21 tokens, 28672 x 4096, fine: 56.9 us with a product for each, 49.8 so).
 // Bound by HBM where tokens are few (21 tokens, F16, with their split: gate and up of an 8B model 28672 x 4096 50 us, 4.7 TB/s; 4096 x 14336 40 us, of which 12 go to start, tail and
 // shares), by L2 from 100 or so on (48 KB to a k-block for 512 cycles of products).  Before: 12 tokens of an F16 model (2 layers of 4096) one by one 3316 us, 379; tiles of 128 x 256
-// over 100 tokens: 4096 x 4096 54 us, 29; 4096 x 14336 177, 50; over 300: 183, 91.  Error against 64 bits, 4096 columns: fine 1.3e-7 (one by one 2.1e-7), otherwise 3.5e-7 (9.7e-6
+// over 100 tokens: 4096 x 4096 54 us, 29; 4096 x 14336 177, 50; over 300: 183, 91.  Error against 64 bits, 4096 columns: fine 1.0e-7 (one by one 1.6e-7), otherwise 3.5e-7 (9.7e-6
 // with 4096 columns to an accumulator); BF16 1.0e-7 and 2.5e-6 (16 bits of an activation).
 #include "kernels_internal.h"
 #include "ring.cuh"
@@ -260,7 +260,7 @@ bool gemm_dense_tc(const GemvMat* mats, int n_mat, int K, const float* x, const 
     for (int t0 = 0; t0 < T; t0 += portion) {
         const int n = std::min(portion, T - t0);
         for (int i = 0; i < n_mat; i++) { m[i] = mats[i]; m[i].y += (size_t)t0 * mats[i].out; }
-        const BlockTokens t = split_tokens(memory.p, x + (size_t)t0 * K, norm_w, eps, n, K, fine, s, mats[0].dtype == DType::BF16);
+        const BlockTokens t = split_tokens(memory.p, x + (size_t)t0 * K, norm_w, eps, n, K, fine, s, mats[0].dtype == DType::BF16 ? TokenParts::BF16 : fine ? TokenParts::F16_SHORT : TokenParts::F16);
         if (!gemm_dense_tc(m, n_mat, K, t, static_cast<uint8_t*>(memory.p) + front(portion), n, add, s, col_scale, alpha)) return false;
     }
     return true;

@@ -65,6 +65,41 @@ def test_what_is_refused():
     assert product([y], [W], x, DType.F32, True) < 0 and (y == 7.0).all()
 
 
+def one_by_one(W, x, dtype):
+    y = torch.zeros(x.shape[0], W.shape[0], device="cuda")
+    for t in range(x.shape[0]):
+        lib().nt_b200_gemv_dense(y[t].data_ptr(), None, None, W.data_ptr(), None, None, W.shape[0], 0, 0, 1, W.shape[1], x[t].data_ptr(), int(dtype), 0, None, 1.0, stream())
+    torch.cuda.synchronize()
+    return y
+
+
+# against the same tokens a GEMV at a time, F32 sums: the form that the fine one took the place of (the plain one is at 2 to 20 times its error).
+# Where one product is most of a short row's sum the order of additions decides: 1024 columns, one number in a thousand 3000 times the others, 1.20e-7 here and 1.05e-7 there.
+@pytest.mark.parametrize("dtype,torch_type", [(DType.F16, torch.float16), (DType.BF16, torch.bfloat16)], ids=["F16", "BF16"])
+@pytest.mark.parametrize("cols,wild,by", [(c, w, b) for c in (512, 1024, 4096, 14336) for w, b in ((0.0, 1.0), (0.01, 10.0))] + [(4096, 0.001, 3000.0), (14336, 0.001, 3000.0)])
+def test_fine_is_as_exact_as_one_by_one(dtype, torch_type, cols, wild, by):
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    W, x = (torch.randn(700, cols, generator=g, device="cuda") * cols ** -0.5).to(torch_type), activations(21, cols, 6, wild, by)
+    y, ref = torch.zeros(21, 700, device="cuda"), x.double() @ W.double().T
+    assert product([y], [W], x, dtype, True) == 0
+    assert rel(y, ref) <= 1.05 * rel(one_by_one(W, x, dtype), ref)
+
+
+# rows with a single weight of 1 give a token's numbers back: all 24 bits of them, but for what lies below 2^-24 of F16 once a token's largest is at 2^13 to 2^14
+@pytest.mark.parametrize("dtype,torch_type", [(DType.F16, torch.float16), (DType.BF16, torch.bfloat16)], ids=["F16", "BF16"])
+def test_fine_keeps_every_bit(dtype, torch_type):
+    x = activations(9, 1024, 8, 0.01, 1000.0)
+    x[1] *= 1e-12
+    x[2] *= 1e12
+    at = torch.randperm(1024, generator=torch.Generator().manual_seed(1))[:300].cuda()
+    W = torch.zeros(300, 1024, device="cuda").to(torch_type)
+    W[torch.arange(300, device="cuda"), at] = 1
+    y = torch.zeros(9, 300, device="cuda")
+    assert product([y], [W], x, dtype, True) == 0
+    left = (y.double() - x[:, at].double()).abs()
+    assert (left <= x.abs().amax(1, keepdim=True).double() * (2.0 ** -37 if dtype == DType.F16 else 0.0)).all()
+
+
 @pytest.mark.parametrize("n,before", [(2, 0), (17, 5), (31, 40)])
 def test_f16_tokens_together_equal_one_by_one(n, before):
     toks = np.random.default_rng(n).integers(0, ODD.vocab_size, size=n + before).tolist()

@@ -368,21 +368,23 @@ int wave_splits(int keys, int groups) { return std::max(1, std::min({2 * 148 / g
 
 // Slices of a run of `tokens` queries over `total` keys, `groups` CTAs to a query and a slice: at least 32 keys each, at most three waves of CTAs.
 int rows_splits_most(int tokens, int total, int groups, int gc, int hd) { return std::max(1, std::min({3 * wave(gc, hd) / (groups * tokens), (total + 31) / 32, MAX_SPLITS})); }
-// A CTA takes 2 us and then, for a key, 11.9 ns and 1.95 ns for each query head that shares it (of 128), 1.5 times that with another on its SM and 2.2 times with two; a wave
-// begun costs 0.4 of one; the merge takes 2.7 us and 6 us for a million of the slices' sums, two launches 6.5 us at least.  Fitted to 882 calls (2 to 31 tokens, 4 to 48 groups, all widths, 0 to 1900 keys
-// before).  As many slices as two CTAs to an SM and one more, and these, us: 21 tokens, 32 heads of 128 over 8, behind 30, 120, 300, 1900: 10.5, 4.9; 12.6, 7.8; 17.1, 13.3;
-// 56.5, 50.8; 16 heads of 64, 16 behind 1900: 41.3, 37.1; the mean takes 0.89 of the time, a few up to 9 % longer.  (A wave of two CTAs of narrow heads to an SM, and 0.7 for
-// one begun: 56.9 there, and 40 heads of 128 over 8, 11 behind 1000 41.9 in two slices, 38.7 whole.)  Eight heads of 128 to a key head stay with the former: their sums are
-// one run (attention_walk.cuh), and longer slices would cost precision (31 queries behind 1000: 2.2e-7, 2.6e-7).
+// A CTA takes 1.25 us and then, for a key, 10.6 ns and 1.5 ns for each query head that shares it (of 128), 1.5 times that beside others on its SM; an SM takes its CTAs two at a time,
+// three where they are narrow (more than 74 CTAs are two to an SM: those that wait for the launch before gather).  The merge takes 3.5 us and 6 us for a million of the slices' sums.
+// Fitted to 784 calls (2 to 31 tokens, 4 to 48 groups, all widths, 0 to 1900 keys before).  As many slices as fill two CTAs to an SM and one more, and
+// these, us: 21 tokens, 32 heads of 128 over 8, behind 30, 120, 300, 1900: 10.5, 4.9; 12.6, 7.8; 17.1, 13.3; 56.5, 50.8; 16 heads of 64, 16 behind 1900: 41.3, 37.1; the mean takes
+// 0.89 of the time.  (By waves of two CTAs to an SM whatever their width, each begun at 0.7 of one: 56.9 there, and 40 heads of 128 over 8, 11 behind 1000 41.9 in two slices, 38.7
+// whole.)  Eight heads of 128 to a key head stay with the former: their sums are one run (attention_walk.cuh), and longer slices would cost precision (31 queries behind 1000:
+// 2.2e-7, 2.6e-7).
 int rows_splits(int tokens, int total, int groups, int gc, int hd) {
     if (gc * hd > 512) return std::max(1, std::min({(2 * 148 + groups * tokens - 1) / (groups * tokens), (total + 31) / 32, MAX_SPLITS}));
-    const float key = 0.0119f + 0.00195f * gc * hd / 128, full = (float)wave(gc, hd);
+    const float key = 0.0106f + 0.0015f * gc * hd / 128;
+    const int at_once = wave(gc, hd) / 148;
     int best = 1;
     float least = 0.f;
     for (int n = 1, most = rows_splits_most(tokens, total, groups, gc, hd); n <= most; n++) {
-        const int len = (total + n - 1) / n, used = (total + len - 1) / len, ctas = groups * tokens * used;
-        const float waves = ctas <= full ? 1.f : 0.4f * ceilf(ctas / full) + 0.6f * ctas / full, shared = ctas <= 148 ? 1.0f : full > 296.f ? 2.2f : 1.5f;
-        const float walked = (2.0f + key * len * shared) * waves, t = used > 1 ? std::max(6.5f, walked + 2.7f + 6e-6f * used * tokens * groups * gc * hd) : walked;
+        const int len = (total + n - 1) / n, used = (total + len - 1) / len, ctas = groups * tokens * used, to_an_sm = ctas > 74 ? std::max(2, (ctas + 147) / 148) : 1, left = to_an_sm % at_once;
+        const float walked = (float)((to_an_sm - left) / at_once + (left > 1)) * (1.25f + 1.5f * key * len) + (left == 1 ? 1.25f + key * len : 0.f);
+        const float t = used > 1 ? walked + 3.5f + 6e-6f * used * tokens * groups * gc * hd : walked;
         if (n == 1 || t < least) { least = t; best = used; }
     }
     return best;

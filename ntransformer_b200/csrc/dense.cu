@@ -597,7 +597,7 @@ void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpil
     const int per_sm = !walk ? 8 : ep == DENSE_STREAMS ? 2 : 4;
     const int resident = (int)std::max<size_t>(1, std::min<size_t>((size_t)per_sm, (size_t)(220 * 1024) / (smem + (walk ? 3 : 1) * 1024))) * 148;
     // Warps to a row: what the CTA that ends last takes, its rounds of rows times their pieces of 1024 columns to a warp (one and a half at least), 0.2 of one for a row's end and 0.15 for
-    // a meeting of warps (twice that where a row has a gate); and 0.2 of one for 1024 numbers of the vector, which each of an SM's CTAs lays out for itself (fits 120 shapes from 32 x 2304 to 57344 x 8192, from HBM and from
+    // a meeting of warps (twice that where a row has a gate); and 0.15 of one for 1024 numbers of the vector, which each of an SM's CTAs lays out for itself (fits 120 shapes from 32 x 2304 to 57344 x 8192, from HBM and from
     // L2, with 1, 2, 4 and 8 warps, to 0.5 % of the best on average).  F16, us: 4096 x 14336 29.0, 25.3, 24.7, 24.7; 11008 x 4096 18.3, 16.7, 18.6, 28.9; 128256 x 4096 150 with one;
     // 2048 x 8192 9.4, 8.4, 8.5, 8.8.  BF16 896 x 4864 6.4, 5.6, 6.0, 6.0; 1041 x 9216 9.2, 7.5, 8.7, 9.1; 20858 + 20858 x 1424, gated 23.8, 26.8, 47, 87.
     // (With two rows to a warp throughout, F16's form before: 270 x 11776 14.9, now 5.9; 1024 x 4096 7.1, 3.9; 4096 x 4096 9.2, 7.4; 8192 x 28672 142, 128.)
@@ -607,7 +607,7 @@ void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpil
         const long long warps = (long long)total * k;
         const double rounds = (double)((warps + resident * DV_WARPS - 1) / (resident * DV_WARPS)), pieces = (glu ? 2 : 1) * ((K + 128 * per16 * k - 1) / (128 * per16 * k));
         const double ctas = (double)std::min<long long>((warps + DV_WARPS - 1) / DV_WARPS, resident);
-        const double cost = rounds * (std::max(1.5, pieces) + (k == 1 ? 0.2 : glu ? 0.5 : 0.35)) + 0.2 * K / 1024 * std::ceil(ctas / 148);
+        const double cost = rounds * (std::max(1.5, pieces) + (k == 1 ? 0.2 : glu ? 0.5 : 0.35)) + 0.15 * K / 1024 * std::ceil(ctas / 148);
         if (k == 1 || cost < least) { least = cost; kw = k; }
     }
     const int rows_at_once = DV_WARPS / kw;

@@ -6,7 +6,7 @@
 
 A "step" is one decoded token (batch 1) of the named Llama-3 shape with synthetic, seeded random GGUF blocks
 generated on the GPU.  N > 1 runs the same model tensor-parallel over N ranks (strong scaling).
-Prints ONE JSON line on rank 0 (see the task contract): value = tok/s with the token already handed to the
+Prints ONE JSON line on rank 0: value = tok/s with the token already handed to the
 device-side step state; e2e = tok/s through the C-ABI with HOST token ids in and HOST logits out every step.
 
 --impl reference times the UNMODIFIED reference (its own CUDA kernels and Transformer::forward, compiled for

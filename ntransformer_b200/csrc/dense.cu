@@ -601,14 +601,16 @@ void gemv_dense(const GemvMat* mats, int n_mat, int K, const float* x, DenseEpil
     // L2, with 1, 2, 4 and 8 warps, to 0.5 % of the best on average).  F16, us: 4096 x 14336 29.0, 25.3, 24.7, 24.7; 11008 x 4096 18.3, 16.7, 18.6, 28.9; 128256 x 4096 150 with one;
     // 2048 x 8192 9.4, 8.4, 8.5, 8.8.  BF16 896 x 4864 6.4, 5.6, 6.0, 6.0; 1041 x 9216 9.2, 7.5, 8.7, 9.1; 20858 + 20858 x 1424, gated 23.8, 26.8, 47, 87.
     // (With two rows to a warp throughout, F16's form before: 270 x 11776 14.9, now 5.9; 1024 x 4096 7.1, 3.9; 4096 x 4096 9.2, 7.4; 8192 x 28672 142, 128.)
+    // In a step the CTAs that wait gather on the SMs that have room, however few they are, and the vector does not count: 1024 x 11264 two warps to a row (256 CTAs) 4 us longer than four.
+    const double staged = pdl_enabled() ? 0.0 : 0.15;
     int kw = 1;
     double least = 0;
     for (int k = 1; walk && k <= DV_WARPS && (k == 1 || k * 64 * per16 < K); k *= 2) {
         const long long warps = (long long)total * k;
         const double rounds = (double)((warps + resident * DV_WARPS - 1) / (resident * DV_WARPS)), pieces = (glu ? 2 : 1) * ((K + 128 * per16 * k - 1) / (128 * per16 * k));
         const double ctas = (double)std::min<long long>((warps + DV_WARPS - 1) / DV_WARPS, resident);
-        const double cost = rounds * (std::max(1.5, pieces) + (k == 1 ? 0.2 : glu ? 0.5 : 0.35)) + 0.15 * K / 1024 * std::ceil(ctas / 148);
-        if (k == 1 || cost < least) { least = cost; kw = k; }
+        const double cost = rounds * (std::max(1.5, pieces) + (k == 1 ? 0.2 : glu ? 0.5 : 0.35)) + staged * K / 1024 * std::ceil(ctas / 148);
+        if (k == 1 || cost <= 1.01 * least) { least = cost; kw = k; }      // as good as equal: more warps, whose sums are shorter and so more exact
     }
     const int rows_at_once = DV_WARPS / kw;
     // Behind the launcher boundary several CTAs fit on an SM: where a launch lets the next one start before it has done its part, that one's CTAs gather on the SMs that have room, and

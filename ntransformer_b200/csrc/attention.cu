@@ -389,14 +389,16 @@ int rows_splits(int tokens, int total, int groups, int gc, int hd) {
     }
     return best;
 }
-// Of a single query.  As many as fit a wave of two CTAs to an SM: one slice more began a second wave (32 heads of 128 with keys of their own, 1000 and 4000 keys, ten slices and
-// nine: 8.9, 7.1; 19.6, 14.6 us; 24 heads over 8, 4000 keys, 13 and 12: 15.8, 12.6).  One more where three fit (64 heads of 64, 2000 and 6000 keys, four and five: 18.5, 16.0;
-// 50.6, 41.9).  Groups of more than half a wave would have one slice however many keys: up to three quarters of one, by what they cost (160 groups of 128, 2000 and 6000 keys,
-// one, two and these: 53.9, 50.9, 42.5; 151, 137, 102; 256 of 64, 2000: 64.7, 51.3, 47.2); beyond, memory is what bounds (240 of 128, 2000 keys, one and two: 55.7, 59.8).
+// Of a single query.  As many as fit a wave of two CTAs to an SM: one slice more began a second wave (32 heads of 128 with keys of their own, 700, 2000 and 6000 keys: 8.4, 7.0;
+// 13.0, 9.8; 30.2, 22.1; 24 heads over 8, 4000 keys, 13 and 12: 15.8, 12.6).  One more where three fit (64 heads of 64, 2000 and 6000 keys, four and five: 18.5, 16.2; 50.6, 41.9).
+// Groups of more than half a wave would have one slice however many keys: up to three quarters of one, by what they cost, narrow ones two at least from 400 keys on (one, two and these:
+// 160 groups of 128, 2000 and 6000 keys 53.9, 50.4, 41.0; 151, 136, 102; 160 of 64, 6000: 141, 96.9, 74.7; 256 of 64, 700 and 2000: 22.3, 18.4, 18.4; 64.7, 50.8, 44.5);
+// beyond, memory is what bounds (240 of 128, 2000 keys, one and two: 55.3, 58.4).
 int decode_splits(int keys, int groups, int gc, int hd) {
     if (keys <= 64) return 1;
-    if (groups > 148) return groups > wave(gc, hd) * 3 / 4 ? 1 : rows_splits(1, keys, groups, gc, hd);
-    return wave(gc, hd) > 296 ? std::min({(295 + groups) / groups, (keys + 31) / 32, MAX_SPLITS}) : wave_splits(keys, groups);
+    const bool narrow = wave(gc, hd) > 296;
+    if (groups > 148) return groups > wave(gc, hd) * 3 / 4 ? 1 : std::max(narrow && keys >= 400 ? 2 : 1, rows_splits(1, keys, groups, gc, hd));
+    return narrow ? std::min({(295 + groups) / groups, (keys + 31) / 32, MAX_SPLITS}) : wave_splits(keys, groups);
 }
 template <int DPL, int GC>
 void launch_decode(float* out, const float* q, const __half* kc, const __half* vc, int seq_len, int n_heads, int n_kv,
